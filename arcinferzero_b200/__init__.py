@@ -1,9 +1,10 @@
 """arcinferzero_b200: the B200 (sm_100a) implementation of inferzero's quantised matrix product.
 
 The product is the CUDA library `libizb200.so` behind the C ABI of include/izb200.h (built in-tree by
-arcinferzero_b200/build.py).  This module is the thin ctypes binding the tests and the benchmark use: it passes raw
-device pointers of torch tensors (torch is only the owner of device memory and streams here) and raises on any non-zero
-status.  There is no CPU path: importing works without a GPU, every call needs one.
+arcinferzero_b200/build.py).  This module is the thin binding the tests and the benchmark use: it passes raw device
+pointers of torch tensors (torch is only the owner of device memory and streams here) and raises on any non-zero status.
+The calls of a decode step or a prompt chunk go through a native module (csrc/izb_py.cpp), the rest through ctypes; both
+call the same C entry points.  There is no CPU path: importing works without a GPU, every call needs one.
 """
 from __future__ import annotations
 
@@ -60,6 +61,27 @@ def _check(rc: int) -> None:
     if rc != 0:
         L = lib()
         raise IzbError(rc, f"{L.izb_status_string(rc).decode()}: {L.izb_last_error().decode()}")
+
+
+_nat = None
+
+
+def _native():
+    """The native side of the hot calls, bound to the loaded library.  Raises if it was never built."""
+    global _nat
+    if _nat is None:
+        import importlib.util
+
+        import torch  # noqa: F401  (its libraries must be loaded first)
+        path = os.path.join(HERE, "_izb_py.so")
+        if not os.path.exists(path):
+            raise ImportError(f"{path} is missing: build it with `python -m arcinferzero_b200.build`")
+        spec = importlib.util.spec_from_file_location("_izb_py", path)
+        m = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(m)
+        m.bind(_check, {n: C.cast(getattr(lib(), n), C.c_void_p).value for n in m.names()})
+        _nat = m
+    return _nat
 
 
 def _p(t) -> C.c_void_p:
@@ -182,105 +204,49 @@ def weight_decode_host(qtype: int, rows: np.ndarray, K: int) -> np.ndarray:
 
 def quantize_act(x, Mp: int | None = None, want_absum: bool = False, out=None):
     """x: [M, K] f32 cuda tensor (row stride may exceed K) -> aq [Mp, K] int8, asc [K/32, Mp] f32, absum or None."""
-    import torch
-    M, K = x.shape
-    Mp = Mp or pad_rows(M)
-    if out is None:
-        aq = torch.empty((Mp, K), dtype=torch.int8, device=x.device)
-        asc = torch.empty((K // 32, Mp), dtype=torch.float32, device=x.device)
-        absum = torch.empty((K // 16, Mp), dtype=torch.int16, device=x.device) if want_absum else None
-    else:
-        aq, asc, absum = out
-    _check(lib().izb_quantize_act(_p(x), x.stride(0), M, Mp, K, _p(aq), _p(asc), _p(absum), _stream()))
-    return aq, asc, absum
+    aq, asc, absum = out if out is not None else (None, None, None)
+    return (_nat or _native()).quantize_act(x, Mp, want_absum, aq, asc, absum)
 
 
 def swiglu_quant(gu, F: int, Mp: int | None = None, want_h: bool = False):
     """gu: [M, 2F] f32 (gate | up) -> quantised h = silu(gate) * up; optionally h itself."""
-    import torch
-    M = gu.shape[0]
-    Mp = Mp or pad_rows(M)
-    aq = torch.empty((Mp, F), dtype=torch.int8, device=gu.device)
-    asc = torch.empty((F // 32, Mp), dtype=torch.float32, device=gu.device)
-    h = torch.empty((M, F), dtype=torch.float32, device=gu.device) if want_h else None
-    _check(lib().izb_swiglu_quant(_p(gu), gu.stride(0), 1, M, Mp, F, _p(h), _p(aq), _p(asc), None, _stream()))
-    return aq, asc, h
+    return (_nat or _native()).swiglu_quant(gu, F, Mp, want_h)
 
 
 def rmsnorm_quant(x, w, eps: float, Mp: int | None = None, want_h: bool = False):
     """x: [M, K] f32, w: [K] f32 -> quantised y = (x * r) * w, r = 1/sqrt(mean(x^2) + eps) per row; optionally y itself."""
-    import torch
-    M, K = x.shape
-    Mp = Mp or pad_rows(M)
-    aq = torch.empty((Mp, K), dtype=torch.int8, device=x.device)
-    asc = torch.empty((K // 32, Mp), dtype=torch.float32, device=x.device)
-    h = torch.empty((M, K), dtype=torch.float32, device=x.device) if want_h else None
-    _check(lib().izb_rmsnorm_quant(_p(x), x.stride(0), _p(w), C.c_float(eps), M, Mp, K, _p(h), _p(aq), _p(asc), None, _stream()))
-    return aq, asc, h
+    return (_nat or _native()).rmsnorm_quant(x, w, eps, Mp, want_h)
 
 
 def add_norm_quant(x, t, w, eps: float, s: float = 1.0, w2=None, Mp: int | None = None):
     """In place x = (x + rmsnorm(t) * w) * s on [M, K] f32 rows, then the quantised next-GEMV input rmsnorm(x) * w2 (or x)."""
-    import torch
-    M, K = x.shape
-    Mp = Mp or pad_rows(M)
-    aq = torch.empty((Mp, K), dtype=torch.int8, device=x.device)
-    asc = torch.empty((K // 32, Mp), dtype=torch.float32, device=x.device)
-    _check(lib().izb_add_norm_quant(_p(x), _p(t), _p(w), C.c_float(eps), C.c_float(s), _p(w2), M, Mp, K, _p(aq), _p(asc), None, _stream()))
-    return aq, asc
+    return (_nat or _native()).add_norm_quant(x, t, w, eps, s, w2, Mp)
 
 
 def softcap_rows(c, rows: int, N: int, cap: float, off: int = 0):
     """In place c[r, off:off+N] = cap * tanh(c[r, off:off+N] / cap) for r < rows (the output head's logit soft-cap)."""
-    _check(lib().izb_softcap_rows(_p(c), rows, c.stride(0), off, N, C.c_float(cap), _stream()))
-    return c
+    return (_nat or _native()).softcap_rows(c, rows, N, cap, off)
 
 
 def matmul(w: Weight, aq, asc, T: int, out=None, c_off: int = 0, acc: int = 0, mat: int = 0):
     """Engine::matmul dispatch: T == 1 GEMV, 2..8 few-row GEMV, else GEMM.  out: [rows, ldc] f32 (default [Mp, N])."""
-    import torch
-    Mp = asc.shape[1]
-    if out is None:
-        out = torch.empty((Mp, w.N), dtype=torch.float32, device=aq.device)
-    _check(lib().izb_matmul(w.handle, mat, _p(aq), _p(asc), None, T, Mp, _p(out), out.stride(0), c_off, acc, _stream()))
-    return out
+    return (_nat or _native()).matmul(w.handle.value, w.N, mat, aq, asc, T, out, c_off, acc)
 
 
 def quant_matmul(w: Weight, x, T: int, Mp: int | None = None, out=None, c_off: int = 0, acc: int = 0, mat: int = 0, qout=None):
     """izb_quant_matmul: quantise x [T, K] f32 and multiply in one call.  Returns (out, aq, asc); qout = (aq, asc) to reuse
     buffers."""
-    import torch
-    Mp = Mp or pad_rows(T)
-    K = w.K
-    if qout is None:
-        aq = torch.empty((Mp, K), dtype=torch.int8, device=x.device)
-        asc = torch.empty((K // 32, Mp), dtype=torch.float32, device=x.device)
-    else:
-        aq, asc = qout
-    if out is None:
-        out = torch.empty((Mp, w.N // 2 if acc == 3 else w.N), dtype=torch.float32, device=x.device)
-    _check(lib().izb_quant_matmul(w.handle, mat, _p(x), x.stride(0), T, Mp, _p(aq), _p(asc), _p(out), out.stride(0), c_off, acc, _stream()))
-    return out, aq, asc
+    aq, asc = qout if qout is not None else (None, None)
+    return (_nat or _native()).quant_matmul(w.handle.value, w.N // 2 if acc == 3 else w.N, w.K, x, T, Mp, out, c_off, acc, mat, aq, asc)
 
 
 def gemv(w: Weight, aq, asc, T: int, out=None, c_off: int = 0, acc: int = 0, mat: int = 0):
-    import torch
-    Mp = asc.shape[1]
-    if out is None:
-        out = torch.empty((T, w.N), dtype=torch.float32, device=aq.device)
-    _check(lib().izb_gemv(w.handle, mat, _p(aq), _p(asc), T, Mp, _p(out), out.stride(0), c_off, acc, _stream()))
-    return out
+    return (_nat or _native()).gemv(w.handle.value, w.N, mat, aq, asc, T, out, c_off, acc)
 
 
 def gemm(w: Weight, aq, asc, M: int | None = None, out=None, c_off: int = 0, acc: int = 0, impl: int = GEMM_AUTO,
          mat: int = 0):
-    import torch
-    Mp = asc.shape[1]
-    M = M or Mp
-    if out is None:
-        out = torch.empty((Mp, w.N // 2 if acc == 3 else w.N), dtype=torch.float32, device=aq.device)
-    _check(lib().izb_gemm(w.handle, mat, _p(aq), _p(asc), M, Mp, _p(out), out.stride(0), c_off, acc, impl, _stream()))
-    return out
+    return (_nat or _native()).gemm(w.handle.value, w.N // 2 if acc == 3 else w.N, mat, aq, asc, M, out, c_off, acc, impl)
 
 
 NOALLOC_SCRATCH_BYTES = 24 << 20
@@ -348,54 +314,26 @@ def matmul_host(w: Weight, x_host, out_host, mat: int = 0) -> None:
 # ---------------------------------------------------------------------------------------------- mixture of experts
 def moe_route(logits, NU: int, shared_gate: bool = False):
     """logits [T, NE] (or [T, NE + 1] with the shared expert's gate logit last) -> ids, wts, counts (, sgate [T])."""
-    import torch
-    T = logits.shape[0]
-    NE = logits.shape[1] - (1 if shared_gate else 0)
-    ids = torch.empty((T, NU), dtype=torch.int32, device=logits.device)
-    wts = torch.empty((T, NU), dtype=torch.float32, device=logits.device)
-    counts = torch.empty((NE,), dtype=torch.int32, device=logits.device)
-    sgate = torch.empty((T,), dtype=torch.float32, device=logits.device) if shared_gate else None
-    _check(lib().izb_moe_route_ex(_p(logits), logits.stride(0), T, NE, NU, _p(ids), _p(wts), _p(counts), _p(sgate), _stream()))
-    return (ids, wts, counts, sgate) if shared_gate else (ids, wts, counts)
+    return (_nat or _native()).moe_route(logits, NU, shared_gate)
 
 
 def moe_sort(ids, wts, counts, TM: int, expert_range: tuple[int, int] | None = None):
-    import torch
-    T, NU = ids.shape
-    NE = counts.shape[0]
-    e0, e1 = expert_range or (0, NE)
-    dev = ids.device
-    max_tiles = (T * NU + TM - 1) // TM + NE
-    offs = torch.empty((NE + 1,), dtype=torch.int32, device=dev)
-    tiles = torch.zeros((1 + 3 * max_tiles,), dtype=torch.int32, device=dev)
-    stok = torch.empty((T * NU,), dtype=torch.int32, device=dev)
-    swt = torch.empty((T * NU,), dtype=torch.float32, device=dev)
-    inv = torch.empty((T * NU,), dtype=torch.int32, device=dev)
-    _check(lib().izb_moe_sort_ex(_p(ids), _p(wts), _p(counts), T, NE, NU, TM, e0, e1, _p(offs), _p(tiles), max_tiles, _p(stok),
-                                 _p(swt), _p(inv), _stream()))
-    return offs, tiles, max_tiles, stok, swt, inv
+    e0, e1 = expert_range or (0, counts.shape[0])
+    return (_nat or _native()).moe_sort(ids, wts, counts, TM, e0, e1)
 
 
 def moe_gateup(wg: Weight, wu: Weight | None, aq, asc, tiles, max_tiles: int, TM: int, stok, S: int):
     """wu = None: wg is an interleaved gate | up stack (gateup_weight) and one grouped GEMM computes both."""
-    import torch
-    h = torch.empty((S, wg.N if wu is not None else wg.N // 2), dtype=torch.float32, device=aq.device)
-    _check(lib().izb_moe_gateup(wg.handle, wu.handle if wu is not None else None, _p(aq), _p(asc), asc.shape[1], _p(tiles), max_tiles, TM, _p(stok), _p(h),
-                                _stream()))
-    return h
+    return (_nat or _native()).moe_gateup(wg.handle.value, wu.handle.value if wu is not None else None, wg.N if wu is not None else wg.N // 2, aq, asc, tiles,
+                                          max_tiles, TM, stok, S)
 
 
 def moe_down(wd: Weight, hq, hsc, tiles, max_tiles: int, TM: int, swt, S: int):
-    import torch
-    y = torch.empty((S, wd.N), dtype=torch.float32, device=hq.device)
-    _check(lib().izb_moe_down(wd.handle, _p(hq), _p(hsc), hsc.shape[1], _p(tiles), max_tiles, TM, _p(swt), _p(y), _stream()))
-    return y
+    return (_nat or _native()).moe_down(wd.handle.value, wd.N, hq, hsc, tiles, max_tiles, TM, swt, S)
 
 
 def moe_combine(x, y, inv, NU: int, sh=None, sgate=None, partial: bool = False):
-    T, E = x.shape
-    _check(lib().izb_moe_combine_ex(_p(x), _p(y), _p(inv), T, NU, E, _p(sh), _p(sgate), int(partial), _stream()))
-    return x
+    return (_nat or _native()).moe_combine(x, y, inv, NU, sh, sgate, partial)
 
 
 # ---------------------------------------------------------------------------------------------- tensor parallel

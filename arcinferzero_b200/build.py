@@ -15,6 +15,7 @@ from concurrent.futures import ThreadPoolExecutor
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "libizb200.so")
+PY_OUT = os.path.join(HERE, "_izb_py.so")  # the Python binding's native side (csrc/izb_py.cpp)
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-fopenmp",
          "-ccbin", "/usr/bin/g++"]
@@ -22,6 +23,24 @@ FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std
 
 def sources():
     return sorted(f for f in os.listdir(CSRC) if f.endswith(".cu"))
+
+
+def build_python_module() -> None:
+    """_izb_py.so: plain C++ against the CPython and torch headers (no CUDA code of its own)."""
+    import sysconfig
+
+    import torch
+    src, hdr = os.path.join(CSRC, "izb_py.cpp"), os.path.join(os.path.dirname(HERE), "include", "izb200.h")
+    if os.path.exists(PY_OUT) and os.path.getmtime(PY_OUT) >= max(os.path.getmtime(src), os.path.getmtime(hdr)):
+        return
+    t = os.path.dirname(torch.__file__)
+    cmd = ["/usr/bin/g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+           "-I" + sysconfig.get_paths()["include"], "-isystem", os.path.join(t, "include"), "-isystem", os.path.join(t, "include/torch/csrc/api/include"),
+           "-isystem", os.path.join(os.path.dirname(os.path.dirname(NVCC)), "include"), src, "-o", PY_OUT, "-L" + os.path.join(t, "lib"), "-ltorch_python",
+           "-ltorch_cuda", "-ltorch_cpu", "-ltorch", "-lc10_cuda", "-lc10"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError("g++ failed:\n" + " ".join(cmd) + "\n" + r.stdout + r.stderr)
 
 
 def build(verbose: bool = False) -> str:
@@ -42,10 +61,12 @@ def build(verbose: bool = False) -> str:
             raise RuntimeError("nvcc failed:\n" + " ".join(cmd) + "\n" + r.stdout + r.stderr)
         return r.stderr
 
-    with ThreadPoolExecutor(max_workers=min(8, max(1, len(jobs)))) as ex:
+    with ThreadPoolExecutor(max_workers=min(8, 1 + len(jobs))) as ex:
+        py = ex.submit(build_python_module)
         for log in ex.map(run, jobs):
             if verbose and log:
                 print(log)
+        py.result()
     if jobs or not os.path.exists(OUT):
         run([NVCC, "-shared", "-o", OUT, *objs, "-lcudart", "-ldl", "-lgomp", "-ccbin", "/usr/bin/g++"])
     return OUT

@@ -123,7 +123,7 @@ extern "C" int izb_profile_stop(char* json, size_t cap) {
 namespace {
 struct DevState {
   std::mutex mu;
-  uint32_t* err_word = nullptr;
+  std::atomic<uint32_t*> err_word{nullptr};
   void* ws[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};  // scratch arenas by user (izb_common.cuh: kWs*)
   size_t ws_bytes[5] = {0, 0, 0, 0, 0};
   void* stage = nullptr;  // staging of the host-buffer call
@@ -206,12 +206,15 @@ extern "C" int izb_set_sm_limit(int device, int sms) {
 // (called with `device` current: every caller has passed izb_require_device or holds a DeviceScope)
 uint32_t* izb_device_error_word(int device) {
   DevState& d = g_dev[device];
+  if (uint32_t* p = d.err_word.load(std::memory_order_acquire)) return p;  // (every GEMV and GEMM call asks: no lock)
   std::lock_guard<std::mutex> lk(d.mu);
-  if (!d.err_word) {
-    if (cudaMalloc(&d.err_word, 256) != cudaSuccess) return nullptr;
-    cudaMemset(d.err_word, 0, 256);
+  uint32_t* p = d.err_word.load(std::memory_order_relaxed);
+  if (!p) {
+    if (cudaMalloc(&p, 256) != cudaSuccess) return nullptr;
+    cudaMemset(p, 0, 256);
+    d.err_word.store(p, std::memory_order_release);
   }
-  return d.err_word;
+  return p;
 }
 
 void izb_note_noalloc_status(int device, uint32_t* status) {
@@ -259,9 +262,11 @@ extern "C" int izb_reserve(int device, int max_rows, int max_K) {
   if (int rc = grow_arena(d, device, kWsGemm, gemm)) return rc;
   if (int rc = grow_arena(d, device, kWsMoe, gemm)) return rc;
   if (int rc = grow_arena(d, device, kWsTp, (size_t)(max_K / 32) * max_rows * 4)) return rc;
-  if (!d.err_word) {
-    if (cudaMalloc(&d.err_word, 256) != cudaSuccess) { cudaGetLastError(); IZB_FAIL(IZB_ERR_NOMEM, "reserve: error word on device %d", device); }
-    IZB_CUDA(cudaMemset(d.err_word, 0, 256));
+  if (!d.err_word.load(std::memory_order_relaxed)) {
+    uint32_t* p = nullptr;
+    if (cudaMalloc(&p, 256) != cudaSuccess) { cudaGetLastError(); IZB_FAIL(IZB_ERR_NOMEM, "reserve: error word on device %d", device); }
+    IZB_CUDA(cudaMemset(p, 0, 256));
+    d.err_word.store(p, std::memory_order_release);
   }
   return IZB_OK;
 }
