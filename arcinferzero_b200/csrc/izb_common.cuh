@@ -131,6 +131,31 @@ uint32_t* izb_device_error_word(int device);
 enum { kWsGemm = 0, kWsTp = 1, kWsMoe = 2, kWsCheck = 3, kWsNorm = 4 };
 int izb_workspace(int device, int slot, size_t bytes, void** out);
 
+// ---------------------------------------------------------------------------------------------- programmatic dependent launch
+// A decode step is a chain of kernels of a few microseconds, each waiting for the one before.  Launched with this attribute
+// a kernel's CTAs move in as soon as every CTA of the kernel before it has called pdl_launch_next() (or ended) and room is
+// free; it may set itself up and touch what no kernel writes (the library's weights), and calls pdl_wait() -- which returns
+// when the kernel before it has completed and its writes are visible -- before it reads or writes anything else.  Every
+// kernel launched this way calls pdl_wait() on every path, so completion stays transitive along the stream.
+#ifdef __CUDACC__
+template <class... P, class... A>
+static inline cudaError_t izb_launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+__device__ __forceinline__ void pdl_launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+#endif
+
 // ---------------------------------------------------------------------------------------------- device helpers
 #ifdef __CUDACC__
 __device__ __forceinline__ uint4 ldg_stream_v4(const void* p) {

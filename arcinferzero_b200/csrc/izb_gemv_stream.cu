@@ -64,6 +64,8 @@ __global__ void __launch_bounds__(stream_warps<T>() * 32, 1) gemv_stream_kernel(
     for (int s = 0; s < slots && s < my_rows; ++s)
       row_copy(s_u32(ring + (size_t)s * slot_bytes), raw + (size_t)(w0 + s * W) * row_bytes, row_bytes, s_u32(&bars[s]));
   }
+  pdl_launch_next();
+  pdl_wait();  // (the ring fill above reads weights only, which no kernel writes: it runs ahead of the wait)
   // ---- stage the T activation rows for all steps: entry (step, t, lane), laid out as in izb_gemv_body.cuh
   for (int i = threadIdx.x; i < nsteps * T * 32; i += blockDim.x) {
     const int l = i & 31, t = (i >> 5) % T, st = (i >> 5) / T;
@@ -239,8 +241,8 @@ __global__ void __launch_bounds__(kRegWarps * 32, 2) gemv_q4k_reg_kernel(const u
   // Programmatic dependent launch: the weights do not depend on the kernel before this one in the stream, so the ring
   // fill above may run while that kernel drains; its results (the activations, and C when accumulating) are read only
   // after griddepcontrol.wait.  launch_dependents lets the next kernel of the stream do the same with this one.
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  pdl_launch_next();
+  pdl_wait();
   // ---- this lane's activations: per step the 2 x 32 int8 values of its block pair, the two block scales (the second one
   // divided by 16, see below) and the two scaled block sums
   uint4 alo[WS][2], ahi[WS][2];
@@ -366,18 +368,8 @@ int launch_q4k_reg(const izb_weight* w, const uint8_t* raw, const int8_t* aq, co
   if (grid > need) grid = need;
   uint32_t* err = izb_device_error_word(w->device);
   if (!err) IZB_FAIL(IZB_ERR_NOMEM, "gemv: no device error word");
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(kRegWarps * 32);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
   const int N = w->N;
-  IZB_LAUNCH("gemv", st, cudaLaunchKernelEx(&cfg, gemv_q4k_reg_kernel<NSTEPS>, raw, N, aq, asc, Mp, C, c_off, acc, slots, slot_bytes, err));
+  IZB_LAUNCH("gemv", st, izb_launch_pdl(gemv_q4k_reg_kernel<NSTEPS>, grid, kRegWarps * 32, smem, st, raw, N, aq, asc, Mp, C, c_off, acc, slots, slot_bytes, err));
   return IZB_OK;
 }
 
@@ -412,8 +404,8 @@ __global__ void __launch_bounds__(kPairWarps * 32, 1) gemv_q4k_pair_kernel(const
     for (int s = 0; s < slots && s < my_rows; ++s)
       row_copy(s_u32(ring + (size_t)s * slot_bytes), raw + (size_t)(w0 + s * W) * row_bytes, row_bytes, s_u32(&bars[s]));
   }
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");  // (see gemv_q4k_reg_kernel: the ring fill above runs ahead of it)
+  pdl_launch_next();
+  pdl_wait();  // (see gemv_q4k_reg_kernel: the ring fill above runs ahead of it)
   // ---- stage the activations: entry (step, token, lane)
   for (int i = threadIdx.x; i < WS * T * 32; i += blockDim.x) {
     const int l = i & 31, t = (i >> 5) % T, st = (i >> 5) / T;
@@ -591,18 +583,8 @@ int launch_q4k_pair(const izb_weight* w, const uint8_t* raw, const int8_t* aq, c
   if (grid > need) grid = need;
   uint32_t* err = izb_device_error_word(w->device);
   if (!err) IZB_FAIL(IZB_ERR_NOMEM, "gemv: no device error word");
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(kPairWarps * 32);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
   const int N = w->N;
-  IZB_LAUNCH("gemv", st, cudaLaunchKernelEx(&cfg, gemv_q4k_pair_kernel<NSB4, T>, raw, N, aq, asc, Mp, C, ldc, c_off, acc, slots, slot_bytes, err));
+  IZB_LAUNCH("gemv", st, izb_launch_pdl(gemv_q4k_pair_kernel<NSB4, T>, grid, kPairWarps * 32, smem, st, raw, N, aq, asc, Mp, C, ldc, c_off, acc, slots, slot_bytes, err));
   return IZB_OK;
 }
 
@@ -660,8 +642,8 @@ __global__ void __launch_bounds__(kPairWarps * 32, 1) gemv_q4k_chunk_kernel(cons
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     for (int n = 0; n < hs && n < total; ++n) issue(n);
   }
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");  // (see gemv_q4k_reg_kernel: the ring fill above runs ahead of it)
+  pdl_launch_next();
+  pdl_wait();  // (see gemv_q4k_reg_kernel: the ring fill above runs ahead of it)
   for (int i = threadIdx.x; i < WS * T * 32; i += blockDim.x) {
     const int l = i & 31, t = (i >> 5) % T, st = (i >> 5) / T;
     const int sb = st < FS ? st * 8 + (l >> 2) : st * 8 + ((l >> 2) & 3), p2 = l & 3;
@@ -791,18 +773,8 @@ int launch_q4k_chunk(const izb_weight* w, const uint8_t* raw, const int8_t* aq, 
   if (grid > need) grid = need;
   uint32_t* err = izb_device_error_word(w->device);
   if (!err) IZB_FAIL(IZB_ERR_NOMEM, "gemv: no device error word");
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(kPairWarps * 32);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
   const int N = w->N, K = w->K;
-  IZB_LAUNCH("gemv", st, cudaLaunchKernelEx(&cfg, gemv_q4k_chunk_kernel<T>, raw, N, K, aq, asc, Mp, C, ldc, c_off, acc, slots, err));
+  IZB_LAUNCH("gemv", st, izb_launch_pdl(gemv_q4k_chunk_kernel<T>, grid, kPairWarps * 32, smem, st, raw, N, K, aq, asc, Mp, C, ldc, c_off, acc, slots, err));
   return IZB_OK;
 }
 
@@ -827,8 +799,7 @@ int launch_stream(const izb_weight* w, const uint8_t* raw, const int8_t* aq, con
   if (grid > need) grid = need;
   uint32_t* err = izb_device_error_word(w->device);
   if (!err) IZB_FAIL(IZB_ERR_NOMEM, "gemv: no device error word");
-  IZB_LAUNCH("gemv", st, gemv_stream_kernel<QT, T><<<grid, kSWarps * 32, smem, st>>>(raw, w->N, w->K, aq, asc, Mp, C, ldc, c_off, acc,
-                                                                                    slots, slot_bytes, err));
+  IZB_LAUNCH("gemv", st, izb_launch_pdl(gemv_stream_kernel<QT, T>, grid, kSWarps * 32, smem, st, raw, w->N, w->K, aq, asc, Mp, C, ldc, c_off, acc, slots, slot_bytes, err));
   return IZB_OK;
 }
 

@@ -23,6 +23,8 @@ __global__ void __launch_bounds__(256) quantize_act_kernel(const float* __restri
   __shared__ int16_t s_sum[16][34];
   const int sb = blockIdx.x, m0 = blockIdx.y * 32, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int col = sb * 256 + lane * 8;
+  pdl_launch_next();
+  pdl_wait();
   float v[4][8];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -104,35 +106,68 @@ __device__ __forceinline__ float cta_sum_ordered(float v, float* s_w) {
   return t;
 }
 
+// rows M..Mp-1 of a quantised activation buffer: zeros with scale 0 (one CTA per row)
+__device__ __forceinline__ void zero_pad_row(int m, int Mp, int K, int8_t* __restrict__ aq, float* __restrict__ asc, int16_t* __restrict__ absum) {
+  for (int i = threadIdx.x; i < K; i += blockDim.x) aq[(size_t)m * K + i] = 0;
+  for (int b = threadIdx.x; b < K / 32; b += blockDim.x) asc[(size_t)b * Mp + m] = 0.0f;
+  if (absum)
+    for (int b = threadIdx.x; b < K / 16; b += blockDim.x) absum[(size_t)b * Mp + m] = 0;
+}
+
 // add_norm_quant (zero/kernels/ops_attn_g.cl:617-680), one CTA of 256 threads per row, K <= 256 * kAnqMax:
 //   x = (x + (t * r) * w) * s with r = 1/sqrt(sum(t^2)/K + eps);  y = w2 ? (x * r2) * w2 : x with r2 from the new x;
 //   y quantised per 32-block.  Thread j owns elements j, j + 256, ...: a warp owns one 32-block per step, so the
 // block maximum is a warp reduction; the new x stays in registers between the two steps.  Both sums of squares are
 // taken in the defined order of cta_sum_ordered over per-thread fused-multiply-add chains.
+// A few decode rows are bound by latency: NK (elements per thread, rounded up) is a compile-time number so that all of a
+// thread's loads are in flight before the first reduction and the chains unroll.  (With a run-time bound over 64 elements
+// the loads were issued one step at a time: 5 rows of 4096 took 35 us.)  Up to 20 elements (K = 5120) the norm weights are
+// requested with the rows; above that they would not fit the registers and come from L2 behind the first reduction.
 constexpr int kAnqMax = 64;
+template <int NK>
 __global__ void __launch_bounds__(256) add_norm_quant_kernel(float* __restrict__ x, const float* __restrict__ t,
                                                              const float* __restrict__ w, int K, float eps, float s,
-                                                             const float* __restrict__ w2, int Mp, int8_t* __restrict__ aq,
+                                                             const float* __restrict__ w2, int M, int Mp, int8_t* __restrict__ aq,
                                                              float* __restrict__ asc, int16_t* __restrict__ absum) {
   __shared__ float s_w[8];
+  constexpr bool kAhead = NK <= 20;
   const int m = blockIdx.x, lane = threadIdx.x & 31;
+  pdl_launch_next();
+  pdl_wait();
+  if (m >= M) {
+    zero_pad_row(m, Mp, K, aq, asc, absum);
+    return;
+  }
   float* xr = x + (size_t)m * K;
   const float* tr = t + (size_t)m * K;
   const int nk = K / 256;
-  float ss = 0.0f;
-  for (int k = 0; k < nk; ++k) {
-    const float v = tr[threadIdx.x + 256 * k];
-    ss = __fmaf_rn(v, v, ss);
+  float tv[NK], xv[NK], wv[kAhead ? NK : 1], w2v[kAhead ? NK : 1];
+#pragma unroll
+  for (int k = 0; k < NK; ++k)
+    if (k < nk) tv[k] = tr[threadIdx.x + 256 * k];
+#pragma unroll
+  for (int k = 0; k < NK; ++k)
+    if (k < nk) xv[k] = xr[threadIdx.x + 256 * k];
+  if (kAhead) {
+#pragma unroll
+    for (int k = 0; k < NK; ++k)
+      if (k < nk) {
+        wv[k] = w[threadIdx.x + 256 * k];
+        if (w2) w2v[k] = w2[threadIdx.x + 256 * k];
+      }
   }
+  float ss = 0.0f;
+#pragma unroll
+  for (int k = 0; k < NK; ++k)
+    if (k < nk) ss = __fmaf_rn(tv[k], tv[k], ss);
   ss = cta_sum_ordered(ss, s_w);
   const float r = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, (float)K), eps)));
-  float xv[kAnqMax];
   float s2 = 0.0f;
 #pragma unroll
-  for (int k = 0; k < kAnqMax; ++k) {
+  for (int k = 0; k < NK; ++k) {
     if (k < nk) {
       const int i = threadIdx.x + 256 * k;
-      const float v = __fmul_rn(__fadd_rn(xr[i], __fmul_rn(__fmul_rn(tr[i], r), w[i])), s);
+      const float v = __fmul_rn(__fadd_rn(xv[k], __fmul_rn(__fmul_rn(tv[k], r), kAhead ? wv[k] : w[i])), s);
       xv[k] = v;
       xr[i] = v;
       s2 = __fmaf_rn(v, v, s2);
@@ -144,10 +179,10 @@ __global__ void __launch_bounds__(256) add_norm_quant_kernel(float* __restrict__
     r2 = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(s2, (float)K), eps)));
   }
 #pragma unroll
-  for (int k = 0; k < kAnqMax; ++k) {
+  for (int k = 0; k < NK; ++k) {
     if (k < nk) {
       const int i = threadIdx.x + 256 * k;
-      const float y = w2 ? __fmul_rn(__fmul_rn(xv[k], r2), w2[i]) : xv[k];
+      const float y = w2 ? __fmul_rn(__fmul_rn(xv[k], r2), kAhead ? w2v[k] : w2[i]) : xv[k];
       float amax = fabsf(y);
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
@@ -155,42 +190,75 @@ __global__ void __launch_bounds__(256) add_norm_quant_kernel(float* __restrict__
       const float p = __fmul_rn(y, inv);
       const int q = fabsf(p) <= 2147483520.0f ? __float2int_rn(p) : 0;  // (see quantize_act_kernel)
       aq[(size_t)m * K + i] = (int8_t)q;
-      int s16 = q;
-#pragma unroll
-      for (int o = 8; o > 0; o >>= 1) s16 += __shfl_xor_sync(0xFFFFFFFFu, s16, o);
       const int b = i >> 5;
       if (lane == 0) asc[(size_t)b * Mp + m] = __fdiv_rn(amax, 127.0f);
-      if (absum && (lane & 15) == 0) absum[(size_t)(2 * b + (lane >> 4)) * Mp + m] = (int16_t)s16;
+      if (absum) {
+        int s16 = q;
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) s16 += __shfl_xor_sync(0xFFFFFFFFu, s16, o);
+        if ((lane & 15) == 0) absum[(size_t)(2 * b + (lane >> 4)) * Mp + m] = (int16_t)s16;
+      }
     }
   }
 }
 
-// rmsnorm_quant (zero/kernels/ops.cl:104-141), one CTA of 256 threads per row: the row is read from HBM once (the second
-// pass finds it in L1 / L2).  Both passes use the quantiser's lane layout: thread j owns the groups of 8 consecutive values
-// j, j + 256, ... .  Pass 1: the sum of squares, a chain of fused multiply-adds over the thread's values in index order,
-// then cta_sum_ordered (this order is part of the definition: the oracle repeats it).  Pass 2: y = (x * r) * w, optional
-// f32 copy, and per 32-block (four adjacent threads) int8 + scale + sums of 16.
+// rmsnorm_quant (zero/kernels/ops.cl:104-141), one CTA of 256 threads per row, in the quantiser's lane layout: thread j owns
+// the groups of 8 consecutive values j, j + 256, ... .  Step 1: the sum of squares, a chain of fused multiply-adds over the
+// thread's values in index order, then cta_sum_ordered (this order is part of the definition: the oracle repeats it).
+// Step 2: y = (x * r) * w, optional f32 copy, and per 32-block (four adjacent threads) int8 + scale + sums of 16.
+// G = groups per thread rounded up: row and norm weights are requested together before the reduction and stay in
+// registers (one pass over the row, one latency instead of two; a row read twice through L1 / L2 measured 56 us at 8192 x
+// 5120 and 5.8 us for one row of 5120).  G = 0: rows too long for that (K > 16384), read twice.
+template <int G>
 __global__ void __launch_bounds__(256) rmsnorm_quant_row_kernel(const float* __restrict__ x, int ldx, const float* __restrict__ w,
-                                                                int K, float eps, int Mp, float* __restrict__ hout,
+                                                                int K, float eps, int M, int Mp, float* __restrict__ hout,
                                                                 int8_t* __restrict__ aq, float* __restrict__ asc,
                                                                 int16_t* __restrict__ absum) {
   __shared__ float s_w[8];
-  const int m = blockIdx.x;
+  constexpr int GR = G > 0 ? G : 1;
+  const int m = blockIdx.x, ng = K / 8;
+  pdl_launch_next();
+  pdl_wait();
+  if (m >= M) {
+    zero_pad_row(m, Mp, K, aq, asc, absum);
+    return;
+  }
   const float* xr = x + (size_t)m * ldx;
+  float4 xa[GR], xb[GR], wa[GR], wb[GR];
   float ss = 0.0f;
-  for (int g = threadIdx.x; g < K / 8; g += 256) {
-    const float4 a = *reinterpret_cast<const float4*>(xr + 8 * g), b = *reinterpret_cast<const float4*>(xr + 8 * g + 4);
+  auto square = [&](const float4& a, const float4& b) {
     ss = __fmaf_rn(a.x, a.x, ss); ss = __fmaf_rn(a.y, a.y, ss); ss = __fmaf_rn(a.z, a.z, ss); ss = __fmaf_rn(a.w, a.w, ss);
     ss = __fmaf_rn(b.x, b.x, ss); ss = __fmaf_rn(b.y, b.y, ss); ss = __fmaf_rn(b.z, b.z, ss); ss = __fmaf_rn(b.w, b.w, ss);
+  };
+  if (G > 0) {
+#pragma unroll
+    for (int k = 0; k < G; ++k) {
+      const int g = threadIdx.x + 256 * k;
+      if (g < ng) {
+        xa[k] = reinterpret_cast<const float4*>(xr)[2 * g];
+        xb[k] = reinterpret_cast<const float4*>(xr)[2 * g + 1];
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < G; ++k) {
+      const int g = threadIdx.x + 256 * k;
+      if (g < ng) {
+        wa[k] = reinterpret_cast<const float4*>(w)[2 * g];
+        wb[k] = reinterpret_cast<const float4*>(w)[2 * g + 1];
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < G; ++k)
+      if (threadIdx.x + 256 * k < ng) square(xa[k], xb[k]);
+  } else {
+    for (int g = threadIdx.x; g < ng; g += 256) square(reinterpret_cast<const float4*>(xr)[2 * g], reinterpret_cast<const float4*>(xr)[2 * g + 1]);
   }
   ss = cta_sum_ordered(ss, s_w);
   const float r = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, (float)K), eps)));
-  for (int g = threadIdx.x; g < K / 8; g += 256) {  // (K / 8 is a multiple of 32: whole warps take part in the shuffles)
+  auto group = [&](int g, const float4& a, const float4& b, const float4& c, const float4& d) {  // (K / 8 is a multiple of 32: whole warps take part in the shuffles)
     const int col = 8 * g;
-    const float4 a = *reinterpret_cast<const float4*>(xr + col), b = *reinterpret_cast<const float4*>(xr + col + 4);
-    const float4 wa = *reinterpret_cast<const float4*>(w + col), wb = *reinterpret_cast<const float4*>(w + col + 4);
     float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-    const float wv[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
+    const float wv[8] = {c.x, c.y, c.z, c.w, d.x, d.y, d.z, d.w};
     float amax = 0.0f;
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
@@ -212,23 +280,25 @@ __global__ void __launch_bounds__(256) rmsnorm_quant_row_kernel(const float* __r
       q[k] = fabsf(p) <= 2147483520.0f ? __float2int_rn(p) : 0;  // (see quantize_act_kernel)
       s8 += q[k];
     }
-    const int s16 = s8 + __shfl_xor_sync(0xFFFFFFFFu, s8, 1);
     uint2 pk;
     pk.x = (q[0] & 0xFF) | ((q[1] & 0xFF) << 8) | ((q[2] & 0xFF) << 16) | ((uint32_t)(q[3] & 0xFF) << 24);
     pk.y = (q[4] & 0xFF) | ((q[5] & 0xFF) << 8) | ((q[6] & 0xFF) << 16) | ((uint32_t)(q[7] & 0xFF) << 24);
     *reinterpret_cast<uint2*>(aq + (size_t)m * K + col) = pk;
     if ((g & 3) == 0) asc[(size_t)(g >> 2) * Mp + m] = __fdiv_rn(amax, 127.0f);
-    if (absum && (g & 1) == 0) absum[(size_t)(g >> 1) * Mp + m] = (int16_t)s16;
+    if (absum) {
+      const int s16 = s8 + __shfl_xor_sync(0xFFFFFFFFu, s8, 1);
+      if ((g & 1) == 0) absum[(size_t)(g >> 1) * Mp + m] = (int16_t)s16;
+    }
+  };
+  if (G > 0) {
+#pragma unroll
+    for (int k = 0; k < G; ++k)
+      if (threadIdx.x + 256 * k < ng) group(threadIdx.x + 256 * k, xa[k], xb[k], wa[k], wb[k]);
+  } else {
+    for (int g = threadIdx.x; g < ng; g += 256)
+      group(g, reinterpret_cast<const float4*>(xr)[2 * g], reinterpret_cast<const float4*>(xr)[2 * g + 1], reinterpret_cast<const float4*>(w)[2 * g],
+            reinterpret_cast<const float4*>(w)[2 * g + 1]);
   }
-}
-
-// rows M..Mp-1 of a quantised activation buffer: zeros with scale 0
-__global__ void zero_pad_rows_kernel(int M, int Mp, int K, int8_t* __restrict__ aq, float* __restrict__ asc, int16_t* __restrict__ absum) {
-  const int m = M + blockIdx.x;
-  for (int i = threadIdx.x; i < K; i += blockDim.x) aq[(size_t)m * K + i] = 0;
-  for (int b = threadIdx.x; b < K / 32; b += blockDim.x) asc[(size_t)b * Mp + m] = 0.0f;
-  if (absum)
-    for (int b = threadIdx.x; b < K / 16; b += blockDim.x) absum[(size_t)b * Mp + m] = 0;
 }
 
 int check_quant_args(const float* x, int ldx, int M, int Mp, int K, const int8_t* aq, const float* asc, int width_needed) {
@@ -247,7 +317,7 @@ extern "C" int izb_quantize_act(const float* d_x, int ldx, int M_valid, int Mp, 
                                 int16_t* d_absum, void* stream) {
   if (int rc = check_quant_args(d_x, ldx, M_valid, Mp, K, d_aq, d_asc, K)) return rc;
   dim3 grid(K / 256, (Mp + 31) / 32);
-  IZB_LAUNCH("quantize_act", (cudaStream_t)stream, quantize_act_kernel<0><<<grid, 256, 0, (cudaStream_t)stream>>>(d_x, ldx, M_valid, Mp, K, d_aq, d_asc, d_absum, nullptr, 0));
+  IZB_LAUNCH("quantize_act", (cudaStream_t)stream, izb_launch_pdl(quantize_act_kernel<0>, grid, 256, 0, (cudaStream_t)stream, d_x, ldx, M_valid, Mp, K, d_aq, d_asc, d_absum, nullptr, 0));
   return IZB_OK;
 }
 
@@ -258,9 +328,9 @@ extern "C" int izb_swiglu_quant(const float* d_gu, int ldgu, int split, int M_va
   dim3 grid(F / 256, (Mp + 31) / 32);
   cudaStream_t st = (cudaStream_t)stream;
   if (split)
-    IZB_LAUNCH("swiglu_quant", st, quantize_act_kernel<1><<<grid, 256, 0, st>>>(d_gu, ldgu, M_valid, Mp, F, d_aq, d_asc, d_absum, d_h, F));
+    IZB_LAUNCH("swiglu_quant", st, izb_launch_pdl(quantize_act_kernel<1>, grid, 256, 0, st, d_gu, ldgu, M_valid, Mp, F, d_aq, d_asc, d_absum, d_h, F));
   else
-    IZB_LAUNCH("quantize_act", st, quantize_act_kernel<0><<<grid, 256, 0, st>>>(d_gu, ldgu, M_valid, Mp, F, d_aq, d_asc, d_absum, nullptr, 0));
+    IZB_LAUNCH("quantize_act", st, izb_launch_pdl(quantize_act_kernel<0>, grid, 256, 0, st, d_gu, ldgu, M_valid, Mp, F, d_aq, d_asc, d_absum, nullptr, 0));
   return IZB_OK;
 }
 
@@ -271,9 +341,11 @@ extern "C" int izb_rmsnorm_quant(const float* d_x, int ldx, const float* d_w, fl
   if (!izb_aligned(d_w, 16) || (d_h && !izb_aligned(d_h, 16))) IZB_FAIL(IZB_ERR_ALIGN, "rmsnorm_quant: w and h must be 16-byte aligned");
   if (!(eps >= 0.0f)) IZB_FAIL(IZB_ERR_ARG, "rmsnorm_quant: eps = %g", (double)eps);
   cudaStream_t st = (cudaStream_t)stream;
-  if (M_valid > 0)
-    IZB_LAUNCH("rmsnorm_quant", st, rmsnorm_quant_row_kernel<<<M_valid, 256, 0, st>>>(d_x, ldx, d_w, K, eps, Mp, d_h, d_aq, d_asc, d_absum));
-  if (Mp > M_valid) IZB_LAUNCH("zero_pad_rows", st, zero_pad_rows_kernel<<<Mp - M_valid, 256, 0, st>>>(M_valid, Mp, K, d_aq, d_asc, d_absum));
+  const int groups = (K / 8 + 255) / 256;  // of 8 values per thread
+  auto kernel = groups <= 1 ? rmsnorm_quant_row_kernel<1> : groups <= 2 ? rmsnorm_quant_row_kernel<2> : groups <= 3 ? rmsnorm_quant_row_kernel<3>
+              : groups <= 4 ? rmsnorm_quant_row_kernel<4> : groups <= 6 ? rmsnorm_quant_row_kernel<6> : groups <= 8 ? rmsnorm_quant_row_kernel<8>
+                                                                                                                 : rmsnorm_quant_row_kernel<0>;
+  IZB_LAUNCH("rmsnorm_quant", st, izb_launch_pdl(kernel, Mp, 256, 0, st, d_x, ldx, d_w, K, eps, M_valid, Mp, d_h, d_aq, d_asc, d_absum));
   return IZB_OK;
 }
 
@@ -284,9 +356,10 @@ extern "C" int izb_add_norm_quant(float* d_x, const float* d_t, const float* d_w
   if (Mp <= 0 || Mp % 16 || M_valid < 0 || M_valid > Mp) IZB_FAIL(IZB_ERR_SHAPE, "add_norm_quant: rows %d of Mp = %d (Mp must be a multiple of 16)", M_valid, Mp);
   if (!(eps >= 0.0f)) IZB_FAIL(IZB_ERR_ARG, "add_norm_quant: eps = %g", (double)eps);
   cudaStream_t st = (cudaStream_t)stream;
-  if (M_valid > 0)
-    IZB_LAUNCH("add_norm_quant", st, add_norm_quant_kernel<<<M_valid, 256, 0, st>>>(d_x, d_t, d_w, K, eps, s, d_w2, Mp, d_aq, d_asc, d_absum));
-  if (Mp > M_valid) IZB_LAUNCH("zero_pad_rows", st, zero_pad_rows_kernel<<<Mp - M_valid, 256, 0, st>>>(M_valid, Mp, K, d_aq, d_asc, d_absum));
+  const int nk = K / 256;  // elements per thread
+  auto kernel = nk <= 4 ? add_norm_quant_kernel<4> : nk <= 8 ? add_norm_quant_kernel<8> : nk <= 16 ? add_norm_quant_kernel<16>
+              : nk <= 20 ? add_norm_quant_kernel<20> : nk <= 32 ? add_norm_quant_kernel<32> : add_norm_quant_kernel<kAnqMax>;
+  IZB_LAUNCH("add_norm_quant", st, izb_launch_pdl(kernel, Mp, 256, 0, st, d_x, d_t, d_w, K, eps, s, d_w2, M_valid, Mp, d_aq, d_asc, d_absum));
   return IZB_OK;
 }
 
@@ -298,6 +371,8 @@ namespace {
 __global__ void __launch_bounds__(256) softcap_rows_kernel(float* __restrict__ C, int ld, int off, int N, float cap, float rcap, int vec) {
   float* p = C + (size_t)blockIdx.y * ld + off;
   const int i = blockIdx.x * 256 + threadIdx.x;
+  pdl_launch_next();
+  pdl_wait();
   if (vec) {
     if (4 * i + 3 < N) {
       float4 v = *reinterpret_cast<float4*>(p + 4 * i);
@@ -325,7 +400,7 @@ extern "C" int izb_softcap_rows(float* d_C, int rows, int ld, int off, int N, fl
   const int vec = izb_aligned(d_C, 16) && ld % 4 == 0 && off % 4 == 0;
   const int per_row = vec ? (N + 3) / 4 : N;
   dim3 grid((per_row + 255) / 256, rows);
-  IZB_LAUNCH("softcap_rows", st, softcap_rows_kernel<<<grid, 256, 0, st>>>(d_C, ld, off, N, cap, 1.0f / cap, vec));
+  IZB_LAUNCH("softcap_rows", st, izb_launch_pdl(softcap_rows_kernel, grid, 256, 0, st, d_C, ld, off, N, cap, 1.0f / cap, vec));
   return IZB_OK;
 }
 

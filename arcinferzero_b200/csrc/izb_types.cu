@@ -170,6 +170,8 @@ __global__ void __launch_bounds__(kGvWarps * 32) gemv_k16_kernel(const uint8_t* 
   const int nb = K >> 5, nsb = K >> 8;
   int8_t* s_a = reinterpret_cast<int8_t*>(smem);                          // [T][K]
   float* s_sc = reinterpret_cast<float*>(smem + (size_t)T * K);           // [T][K/32]
+  pdl_launch_next();
+  pdl_wait();
   for (int i = threadIdx.x; i < T * (K / 16); i += blockDim.x) {
     const int t = i / (K / 16), pc = i % (K / 16);
     reinterpret_cast<uint4*>(s_a)[i] = *reinterpret_cast<const uint4*>(aq + (size_t)t * K + 16 * pc);
@@ -253,6 +255,8 @@ __global__ void __launch_bounds__(kGvWarps * 32, T <= 2 ? 4 : T <= 4 ? 3 : 2) ge
   const int nb = K >> 5, nsb = K >> 8;
   int8_t* s_a = reinterpret_cast<int8_t*>(smem);                          // [T][K]
   float* s_sc = reinterpret_cast<float*>(smem + (size_t)T * K);           // [T][K/32]
+  pdl_launch_next();
+  pdl_wait();
   for (int i = threadIdx.x; i < T * (K / 16); i += blockDim.x) {
     const int t = i / (K / 16), pc = i % (K / 16);
     reinterpret_cast<uint4*>(s_a)[i] = *reinterpret_cast<const uint4*>(aq + (size_t)t * K + 16 * pc);
@@ -322,13 +326,13 @@ int launch_gemv_k16(const izb_weight* w, const uint8_t* raw, const int8_t* aq, c
   if (grid > need) grid = need;
   if (w->packed6) {
     IZB_SMEM_OPTIN((gemv_q6p_kernel<T>), 200 * 1024, w->device);
-    IZB_LAUNCH("gemv_q6p", st, gemv_q6p_kernel<T><<<grid, kGvWarps * 32, smem, st>>>(raw, w->N, w->K, aq, asc, Mp, C, ldc, c_off, acc));
+    IZB_LAUNCH("gemv_q6p", st, izb_launch_pdl(gemv_q6p_kernel<T>, grid, kGvWarps * 32, smem, st, raw, w->N, w->K, aq, asc, Mp, C, ldc, c_off, acc));
   } else if (w->has_min) {
     IZB_SMEM_OPTIN((gemv_k16_kernel<T, true>), 200 * 1024, w->device);
-    IZB_LAUNCH("gemv_k16", st, gemv_k16_kernel<T, true><<<grid, kGvWarps * 32, smem, st>>>(raw, w->N, w->K, aq, asc, Mp, C, ldc, c_off, acc));
+    IZB_LAUNCH("gemv_k16", st, izb_launch_pdl(gemv_k16_kernel<T, true>, grid, kGvWarps * 32, smem, st, raw, w->N, w->K, aq, asc, Mp, C, ldc, c_off, acc));
   } else {
     IZB_SMEM_OPTIN((gemv_k16_kernel<T, false>), 200 * 1024, w->device);
-    IZB_LAUNCH("gemv_k16", st, gemv_k16_kernel<T, false><<<grid, kGvWarps * 32, smem, st>>>(raw, w->N, w->K, aq, asc, Mp, C, ldc, c_off, acc));
+    IZB_LAUNCH("gemv_k16", st, izb_launch_pdl(gemv_k16_kernel<T, false>, grid, kGvWarps * 32, smem, st, raw, w->N, w->K, aq, asc, Mp, C, ldc, c_off, acc));
   }
   return IZB_OK;
 }
