@@ -249,7 +249,7 @@ int izb_workspace(int device, int slot, size_t bytes, void** out) {
   return IZB_OK;
 }
 
-size_t izb_gemm_tc_scratch_bytes(int type, int rows, int K);
+size_t izb_gemm_tc_scratch_bytes(int device, int type, int rows, int K);
 
 extern "C" int izb_reserve(int device, int max_rows, int max_K) {
   if (max_rows < 1 || max_K < 256 || max_K % 256) IZB_FAIL(IZB_ERR_SHAPE, "reserve: rows = %d, K = %d (K in whole superblocks)", max_rows, max_K);
@@ -258,7 +258,7 @@ extern "C" int izb_reserve(int device, int max_rows, int max_K) {
   IZB_CUDA(scope.enter(device));
   DevState& d = g_dev[device];
   std::lock_guard<std::mutex> lk(d.mu);
-  const size_t gemm = izb_gemm_tc_scratch_bytes(IZB_Q4_K, max_rows, max_K);
+  const size_t gemm = izb_gemm_tc_scratch_bytes(device, IZB_Q4_K, max_rows, max_K);
   if (int rc = grow_arena(d, device, kWsGemm, gemm)) return rc;
   if (int rc = grow_arena(d, device, kWsMoe, gemm)) return rc;
   if (int rc = grow_arena(d, device, kWsTp, (size_t)(max_K / 32) * max_rows * 4)) return rc;
@@ -403,7 +403,7 @@ extern "C" int izb_weight_create_slice(int type, const void* h_rows, int n_mats,
     delete w;
     IZB_FAIL(IZB_ERR_CUDA, "weight_create: upload failed: %s", cudaGetErrorString(e));
   }
-  w->has_tmap = w->type != IZB_K16 && izb_make_raw_tensor_map(w) == IZB_OK;
+  w->has_tmap = izb_make_raw_tensor_map(w) == IZB_OK;
   *out = w;
   return IZB_OK;
 }
@@ -543,10 +543,14 @@ extern "C" int izb_gemm(const izb_weight* w, int mat, const int8_t* d_aq, const 
   if (int rc = check_gemm_args(w, mat, d_aq, d_asc, M, Mp, d_C, ldc, c_off, acc)) return rc;
   if (int rc = izb_require_device(w->device, "gemm")) return rc;
   cudaStream_t st = (cudaStream_t)stream;
-  if (w->type == IZB_K16) {  // Q5_K / Q6_K / IQ4_XS: exact per-16 scales, CUDA cores (the reference requantises these for its GEMM)
+  if (w->type == IZB_K16) {  // Q5_K / Q6_K / IQ4_XS: exact per-16 scales (the reference requantises these for its GEMM)
     if (impl == IZB_GEMM_TC) IZB_FAIL(IZB_ERR_TYPE, "gemm: the tensor-core kernel does not take ggml type %d", w->ggml_type);
     if (impl != IZB_GEMM_AUTO && impl != IZB_GEMM_CORE) IZB_FAIL(IZB_ERR_ARG, "gemm: impl %d", impl);
     if (acc == 3) IZB_FAIL(IZB_ERR_TYPE, "gemm: store mode 3 is not built for ggml type %d", w->ggml_type);
+    if (impl == IZB_GEMM_AUTO && g_dev[w->device].tc_ok.load() != 0) {
+      const int rc = izb_gemm_tc_launch(w, mat, d_aq, d_asc, M, Mp, d_C, ldc, c_off, acc, nullptr, st);
+      if (rc <= 0) return rc;
+    }
     return izb_gemm_k16_launch(w, w->raw + (size_t)mat * w->N * w->row_bytes, d_aq, d_asc, M, Mp, d_C, ldc, c_off, acc, nullptr, st);
   }
   if (impl == IZB_GEMM_AUTO || impl == IZB_GEMM_TC) {
@@ -606,7 +610,7 @@ extern "C" int izb_quant_matmul(const izb_weight* w, int mat, const float* d_x, 
   if (!w || !d_x || !d_aq || !d_asc || !d_C) IZB_FAIL(IZB_ERR_ARG, "quant_matmul: null pointer");
   if (T < 1 || T > Mp) IZB_FAIL(IZB_ERR_SHAPE, "quant_matmul: %d rows of Mp = %d", T, Mp);
   // the GEMM with the fused pre-pass: same checks as izb_gemm, then one launch writes aq / asc and the operand images
-  if (T > 8 && (w->type == IZB_Q8_0 || w->type == IZB_Q4_K) && g_dev[w->device < 0 || w->device >= kIzbMaxDev ? 0 : w->device].tc_ok.load() != 0) {
+  if (T > 8 && g_dev[w->device < 0 || w->device >= kIzbMaxDev ? 0 : w->device].tc_ok.load() != 0) {
     if (int rc = check_gemm_args(w, mat, d_aq, d_asc, Mp, Mp, d_C, ldc, c_off, acc)) return rc;
     if (ldx < w->K || ldx % 4 || !izb_aligned(d_x, 16)) IZB_FAIL(IZB_ERR_ALIGN, "quant_matmul: x must be 16-byte aligned with ldx >= K a multiple of 4");
     if (int rc = izb_require_device(w->device, "quant_matmul")) return rc;

@@ -46,20 +46,6 @@ int izb_get_tc_ok(int device);
 int izb_gemm_core_launch(const izb_weight* w, const uint8_t* raw, const int8_t* aq, const float* asc, int M, int Mp, float* C,
                          int ldc, int c_off, int acc, int32_t* dots, cudaStream_t st);
 
-// Build-time experiment switches (defaults = the shipped kernel).
-
-#ifndef IZB_TC_TRACE
-#define IZB_TC_TRACE 0   // diagnostics build: CTA 0 stamps clock64() at the hand-overs of its first blocks into TcParams::trace
-#endif
-#if IZB_TC_TRACE
-#define TRACE(ev, idx)                                                                                      \
-  do {                                                                                                      \
-    if (p.trace && blockIdx.x == 0 && lane == 0 && (idx) >= 0 && (idx) < 2048) p.trace[(ev) * 2048 + (idx)] = clock64(); \
-  } while (0)
-#else
-#define TRACE(ev, idx) do { } while (0)
-#endif
-
 namespace {
 
 constexpr int BM = 128, BN = 128, KS = 64;
@@ -67,50 +53,40 @@ constexpr int ND1 = 3;                    // accumulators of a 32-block in the r
 constexpr int STAGE_BYTES = BM * KS * 2;  // 16 KB: 128 rows x 128 B
 constexpr int kThreads = 512;
 constexpr uint32_t kSpinLimit = 1u << 24;
-constexpr int RAW_Q4 = 128 * 144, RAW_Q8 = 128 * 272;  // 18432, 34816: the raw superblocks of a tile's 128 weight rows
 constexpr int NASC = 3;
 
-// Ring depths.  The two operands of a stage travel through rings of their own: an activation image is a bulk copy from L2
-// whose latency (not its bandwidth) is what has to be covered, so its ring is as deep as shared memory allows; a weight
-// tile is written by the dequantiser warps from a raw tile that is already in shared memory.
-#ifndef IZB_TC_NA4
-#define IZB_TC_NA4 6
-#endif
-#ifndef IZB_TC_NB4
-#define IZB_TC_NB4 4
-#endif
-#ifndef IZB_TC_NR4
-#define IZB_TC_NR4 2
-#endif
-#ifndef IZB_TC_NA8
-#define IZB_TC_NA8 4
-#endif
-#ifndef IZB_TC_NB8
-#define IZB_TC_NB8 4
-#endif
+// ---- what differs between the weight forms
+//   kMin    superblock mins (Q4_K, Q5_K): a fifth operand stage per superblock carries the min term
+//   kTerms  fp16 terms of scale * quant: one where the product fits 11 bits (Q4_K 63 * 15, Q5_K 63 * 31, Q8_0's plain quant);
+//           two where it reaches 4096 (Q6_K, IQ4_XS): scale * quant = hi + lo with hi even and lo in {0, 1}, both exact
+//   kColScale  a scale per block and weight row applied in the combine (Q8_0) instead of one per superblock
+struct FQ4K { static constexpr int SBB = 144, kTerms = 1, NA = 6, NB = 4, NR = 2; static constexpr bool kMin = true, kColScale = false; };
+struct FQ80 { static constexpr int SBB = 272, kTerms = 1, NA = 4, NB = 4, NR = 2; static constexpr bool kMin = false, kColScale = true; };
+struct FQ5K { static constexpr int SBB = kK16SbBytes, kTerms = 1, NA = 4, NB = 4, NR = 2; static constexpr bool kMin = true, kColScale = false; };
+struct FQ6K { static constexpr int SBB = kQ6pSbBytes, kTerms = 2, NA = 3, NB = 3, NR = 2; static constexpr bool kMin = false, kColScale = false; };
+struct FIQ4 { static constexpr int SBB = kK16SbBytes, kTerms = 2, NA = 3, NB = 3, NR = 1; static constexpr bool kMin = false, kColScale = false; };
 
-// shared memory map (bytes from a 1024-aligned base)
-template <int QT>
+// shared memory map (bytes from a 1024-aligned base).  The two operands of a stage travel through rings of their own: an
+// activation image is a bulk copy from L2 whose latency (not its bandwidth) is what has to be covered, so its ring is as
+// deep as shared memory allows; a weight tile is written by the dequantiser warps from a raw tile already in shared memory.
+template <class F>
 struct Map {
-  static constexpr bool q4 = QT == IZB_Q4_K;
-  static constexpr int NA = q4 ? IZB_TC_NA4 : IZB_TC_NA8;  // activation stages
-  static constexpr int NB = q4 ? IZB_TC_NB4 : IZB_TC_NB8;  // weight-operand stages
-  static constexpr int NR = q4 ? IZB_TC_NR4 : 2;           // raw superblock tiles
-  static constexpr int RAW = q4 ? RAW_Q4 : RAW_Q8;
+  static constexpr int NA = F::NA, NB = F::NB, NR = F::NR, RAW = BN * F::SBB;
+  static constexpr int BSTAGE = STAGE_BYTES * F::kTerms;
   static constexpr int OFF_A = 0;
   static constexpr int OFF_B = OFF_A + NA * STAGE_BYTES;
-  static constexpr int OFF_RAW = OFF_B + NB * STAGE_BYTES;
-  static constexpr int OFF_SCL = OFF_RAW + NR * RAW;              // Q4_K: 4 x [128] f32 superblock scales d; Q8_0: 4 x [8][128] f32 block scales
-  static constexpr int OFF_ASC = OFF_SCL + (q4 ? 4 * 512 : 4 * 4096);  // NASC x [8 blocks][128 rows] f32 activation scales
+  static constexpr int OFF_RAW = OFF_B + NB * BSTAGE;
+  static constexpr int OFF_SCL = OFF_RAW + NR * RAW;                          // 4 x [128] f32 superblock scales d; Q8_0: 4 x [8][128] f32 block scales
+  static constexpr int OFF_ASC = OFF_SCL + (F::kColScale ? 4 * 4096 : 4 * 512);  // NASC x [8 blocks][128 rows] f32 activation scales
   static constexpr int OFF_BAR = OFF_ASC + NASC * 4096;
-  static constexpr int SMEM_BYTES = OFF_BAR + 1024 + 1024;        // barriers + alignment slack
+  static constexpr int SMEM_BYTES = OFF_BAR + 1024 + 1024;                    // barriers + alignment slack
   // 8-byte mbarriers
   static constexpr int A_FULL = 0, A_EMPTY = A_FULL + NA, B_FULL = A_EMPTY + NA, B_EMPTY = B_FULL + NB, RAW_FULL = B_EMPTY + NB,
                        RAW_EMPTY = RAW_FULL + NR, D1_FULL = RAW_EMPTY + NR, D1_EMPTY = D1_FULL + ND1, D2_FULL = D1_EMPTY + ND1,
                        D2_EMPTY = D2_FULL + 1, ASC_FULL = D2_EMPTY + 1, ASC_EMPTY = ASC_FULL + NASC, NUM_BARS = ASC_EMPTY + NASC;
   static_assert(SMEM_BYTES <= 232448, "shared memory per CTA");
   static_assert(NUM_BARS * 8 + 16 <= 1024, "barrier area");
-  static_assert(OFF_RAW % 1024 == 0 && OFF_SCL % 16 == 0, "alignment of the TMA destinations");
+  static_assert(OFF_RAW % 1024 == 0 && OFF_SCL % 16 == 0 && RAW % 128 == 0, "alignment of the TMA destinations");
 };
 
 // error-word codes (which wait gave up)
@@ -118,22 +94,23 @@ enum : uint32_t { E_APROD = 1, E_WPROD = 2, E_DEQ = 4, E_MMA = 16, E_EPI = 32 };
 
 struct TcParams {
   const uint16_t* aimg;   // [tiles][stages][128][64] 16-bit operand tiles, rows 128-byte swizzled; stages = K/64, and
-                          // for the Q4_K GEMM one bf16 min-term tile after every four (5 per superblock)
+                          // for weights with mins one bf16 min-term tile after every four (5 per superblock)
   const float* ascimg;    // [tiles][K/32][128] f32: the tile rows' activation scales, gathered
   const int32_t* tiles;   // grouped: [1 + 3*max_tiles]; dense: null
-  const int32_t* rowmap;  // grouped gather of activation rows (slot -> token) or null
   const float* rowscale;  // per output row factor or null
   int M;                  // dense: rows to store
   int n_mtiles;           // dense: row tiles (grouped: tiles[0], read on the device)
   int N, K;               // per matrix
   int mat;                // dense: matrix of the stack
+  int n_split;            // parts the K range of every tile is cut into (dense only)
+  float* part;            // n_split > 1: [n_split][M][N] partial sums, stored instead of C
+  uint32_t* part_bad;     // n_split > 1: set when a wait gave up (split_reduce_kernel then stores nothing)
   float* C;
   int ldc, c_off, acc;
   int32_t* dots;          // verification mode output or null
   uint32_t* err;
   uint32_t spin_limit;    // polls after which a wait gives up
   int skip_stage;         // diagnostics: the operand stage the activation producer leaves out (-1: none)
-  unsigned long long* trace;  // diagnostics build only: [16][2048] clock stamps
 };
 
 // ---------------------------------------------------------------------------------------------- PTX wrappers
@@ -191,12 +168,15 @@ __device__ __forceinline__ void tma_2d(uint32_t dst, const void* tmap, int x, in
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+// MMA and commit are issued by a whole converged warp with one elected lane's predicate inside the statement: the operands
+// then stay in uniform registers.  Behind a lane test they are moved there one by one for every instruction, which
+// measured 98 clk per MMA and per commit; in this form four MMAs and three commits take 168.
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+  asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void tc_mma_f16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "{\n\t.reg .pred p, e;\n\telect.sync _|e, 0xffffffff;\n\tsetp.ne.b32 p, %4, 0;\n\t@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
@@ -315,13 +295,17 @@ __device__ __forceinline__ int q4k_perm8(int p) { return (p & 4) | ((p & 1) << 1
 // v = asc * (float)asum of the superblock's eight blocks as three bf16 terms, laid out as the six 16-byte K-chunks
 // (v1, v1, v2, v1, v2, v3) x eight blocks that meet the weight side's (u1, u2, u1, u3, u2, u1).
 // One thread per (row, 16-byte output chunk).
-template <int QT>
+template <bool kPerm>
 __global__ void __launch_bounds__(256) act_prepare_kernel(const int8_t* __restrict__ aq, const float* __restrict__ asc, int lda,
                                                           int K, int rows_total, const int32_t* __restrict__ tiles,
                                                           const int32_t* __restrict__ rowmap, uint16_t* __restrict__ aimg,
-                                                          float* __restrict__ ascimg, int sps) {
+                                                          float* __restrict__ ascimg, int sps,
+                                                          uint32_t* __restrict__ part_bad) {
   const int tile = blockIdx.y;
   int r0, nr;
+  pdl_launch_next();
+  pdl_wait();
+  if (part_bad && blockIdx.x == 0 && tile == 0 && threadIdx.x == 0) *part_bad = 0;
   if (tiles) {
     if (tile >= tiles[0]) return;
     r0 = tiles[2 + 3 * tile];
@@ -348,7 +332,7 @@ __global__ void __launch_bounds__(256) act_prepare_kernel(const int8_t* __restri
   uint32_t o[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const int e0 = QT == IZB_Q4_K ? q4k_perm8(2 * i) : 2 * i, e1 = QT == IZB_Q4_K ? q4k_perm8(2 * i + 1) : 2 * i + 1;
+    const int e0 = kPerm ? q4k_perm8(2 * i) : 2 * i, e1 = kPerm ? q4k_perm8(2 * i + 1) : 2 * i + 1;
     const __half2 h = __floats2half2_rn((float)a[e0], (float)a[e1]);
     o[i] = *reinterpret_cast<const uint32_t*>(&h);
   }
@@ -364,7 +348,7 @@ __global__ void __launch_bounds__(256) act_prepare_kernel(const int8_t* __restri
       const int b = ch >> 2;
       const float sc = src >= 0 ? asc[(size_t)b * lda + src] : 0.0f;
       ascimg[((size_t)tile * (K / 32) + b) * BM + r] = sc;
-      if (QT == IZB_Q4_K && sps == 5) {
+      if (sps == 5) {
         const float v = __fmul_rn(sc, (float)s);
         const __nv_bfloat16 h1 = __float2bfloat16_rn(v);
         const float r1 = __fsub_rn(v, __bfloat162float(h1));
@@ -386,14 +370,18 @@ __global__ void __launch_bounds__(256) act_prepare_kernel(const int8_t* __restri
 // four lanes a 32-block.  Writes aq / asc exactly as the quantiser does (the caller's buffers stay valid for every other
 // kernel) and, from the same registers, the operand images, the gathered scales and the min-term factors of the dense
 // tensor-core GEMM: the int8 rows are not read back and the second launch is gone.  One CTA = 32 rows x one superblock.
-template <int QT>
+template <bool kPerm>
 __global__ void __launch_bounds__(256) quant_prepare_kernel(const float* __restrict__ x, int ldx, int M, int Mp, int K,
                                                             int8_t* __restrict__ aq, float* __restrict__ asc,
-                                                            uint16_t* __restrict__ aimg, float* __restrict__ ascimg, int sps, int n_tiles) {
+                                                            uint16_t* __restrict__ aimg, float* __restrict__ ascimg, int sps, int n_tiles,
+                                                            uint32_t* __restrict__ part_bad) {
   __shared__ float s_sc[8][33];
   const int sb = blockIdx.x, m0 = blockIdx.y * 32, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int col = sb * 256 + lane * 8;
   const size_t nstages = (size_t)(K / 256) * sps;
+  pdl_launch_next();
+  pdl_wait();
+  if (part_bad && sb == 0 && blockIdx.y == 0 && threadIdx.x == 0) *part_bad = 0;
   float v[4][8];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -442,7 +430,7 @@ __global__ void __launch_bounds__(256) quant_prepare_kernel(const float* __restr
     uint32_t o[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const int e0 = QT == IZB_Q4_K ? q4k_perm8(2 * j) : 2 * j, e1 = QT == IZB_Q4_K ? q4k_perm8(2 * j + 1) : 2 * j + 1;
+      const int e0 = kPerm ? q4k_perm8(2 * j) : 2 * j, e1 = kPerm ? q4k_perm8(2 * j + 1) : 2 * j + 1;
       const __half2 h = __floats2half2_rn((float)q[e0], (float)q[e1]);
       o[j] = *reinterpret_cast<const uint32_t*>(&h);
     }
@@ -451,7 +439,7 @@ __global__ void __launch_bounds__(256) quant_prepare_kernel(const float* __restr
     if ((lane & 3) == 0) {
       const int b = lane >> 2;  // block of the superblock
       ascimg[((size_t)tile * (K / 32) + sb * 8 + b) * BM + r] = sc;
-      if (QT == IZB_Q4_K && sps == 5) {
+      if (sps == 5) {
         const float t = __fmul_rn(sc, (float)s);
         const __nv_bfloat16 h1 = __float2bfloat16_rn(t);
         const float r1 = __fsub_rn(t, __bfloat162float(h1));
@@ -473,50 +461,234 @@ __global__ void __launch_bounds__(256) quant_prepare_kernel(const float* __restr
 }
 
 // ---------------------------------------------------------------------------------------------- the GEMM kernel
-template <int QT, bool kDots>
+// What one superblock of a weight row becomes in shared memory.  Every form offers
+//   load(row)                    the row's superblock header into registers
+//   store_scales(smem, slot, t)  the scales the combine warps apply
+//   load_stage(c, row)           the quants of blocks 2c, 2c + 1 into registers
+//   stage(c, out, t)             those 64 elements as fp16 operand rows, 128-byte swizzled (hi at out, lo 16 KB on)
+//   mins(u)                      -dmin * mn of the eight blocks
+__device__ __forceinline__ uint32_t h2_bits(__half2 h) { return *reinterpret_cast<const uint32_t*>(&h); }
+__device__ __forceinline__ __half2 bits_h2(uint32_t u) { return *reinterpret_cast<const __half2*>(&u); }
+__device__ __forceinline__ __half2 h2_const(unsigned short b) { return __half2half2(__ushort_as_half(b)); }
+__device__ __forceinline__ void put16(unsigned char* orow, int chunk, int t, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  *reinterpret_cast<uint4*>(orow + ((chunk ^ (t & 7)) << 4)) = make_uint4(a, b, c, d);
+}
+
+template <bool kDots>
+struct DeqQ4K {
+  uint4 hdr, q0, q1;
+  // (scale, min) bytes of sub-blocks 2c and 2c + 1 (get_scale_min_k4, src/quants.h:61-69), without a branch on c
+  __device__ __forceinline__ void pair(int c, uint32_t& sc2, uint32_t& mn2) const {
+    const int sh = 16 * (c & 1);
+    const uint32_t a = hdr.y >> sh, b = hdr.z >> sh, d = hdr.w >> sh;
+    sc2 = c >= 2 ? ((d & 0x0F0Fu) | ((a >> 2) & 0x3030u)) : (a & 0x3F3Fu);
+    mn2 = c >= 2 ? (((d >> 4) & 0x0F0Fu) | ((b >> 2) & 0x3030u)) : (b & 0x3F3Fu);
+  }
+  __device__ __forceinline__ void load(const unsigned char* row) { hdr = *reinterpret_cast<const uint4*>(row); }
+  __device__ __forceinline__ void load_stage(int c, const unsigned char* row) {
+    q0 = *reinterpret_cast<const uint4*>(row + 16 + 32 * c);
+    q1 = *reinterpret_cast<const uint4*>(row + 32 + 32 * c);
+  }
+  __device__ __forceinline__ void store_scales(unsigned char* scl, int slot, int t) const {
+    reinterpret_cast<float*>(scl + slot * 512)[t] = half_bits_to_float(hdr.x & 0xFFFFu);
+  }
+  __device__ __forceinline__ void stage(int c, unsigned char* orow, int t) const {
+    const uint32_t w[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+    // the chunk's two 6-bit sub-block scales as half2 pairs (sc, sc) and (-1024 sc, -1024 sc): 0x6400 | sc is the
+    // fp16 number 1024 + sc
+    uint32_t sc2 = 0x0101u, mn_unused;
+    if (!kDots) pair(c, sc2, mn_unused);
+    const __half2 k1024 = h2_const(0x6400), kneg = h2_const(0xE400), k16th = h2_const(0x2C00);
+    const __half2 slo = __hsub2(bits_h2(__byte_perm(sc2, 0x64646464u, 0x4040)), k1024), shi = __hsub2(bits_h2(__byte_perm(sc2, 0x64646464u, 0x4141)), k1024);
+    const __half2 nlo = __hmul2(slo, kneg), nhi16 = __hmul2(__hmul2(shi, kneg), k16th), shi16 = __hmul2(shi, k16th);
+    // High nibbles stay where they are: (word & 0x00F000F0) | 0x6400 is the fp16 number 1024 + 16 q, and
+    // (1024 + 16 q) * (sc / 16) - 64 sc = sc * q exactly (one rounding, of an integer below 2^11).  One shift per
+    // word (for its upper bytes) instead of three.
+    auto cv = [](uint32_t word, uint32_t mask, __half2 scale, __half2 neg) -> uint32_t { return h2_bits(__hfma2(bits_h2((word & mask) | 0x64006400u), scale, neg)); };
+#pragma unroll
+    for (int jj = 0; jj < 4; ++jj) {
+      const uint32_t w0 = w[2 * jj], w1 = w[2 * jj + 1], x0 = w0 >> 8, x1 = w1 >> 8;
+      put16(orow, jj, t, cv(w0, 0x000F000Fu, slo, nlo), cv(x0, 0x000F000Fu, slo, nlo), cv(w1, 0x000F000Fu, slo, nlo), cv(x1, 0x000F000Fu, slo, nlo));
+      put16(orow, 4 + jj, t, cv(w0, 0x00F000F0u, shi16, nhi16), cv(x0, 0x00F000F0u, shi16, nhi16), cv(w1, 0x00F000F0u, shi16, nhi16), cv(x1, 0x00F000F0u, shi16, nhi16));
+    }
+  }
+  __device__ __forceinline__ void mins(float (&u)[8]) const {
+    const float ndmin = -half_bits_to_float(hdr.x >> 16);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      uint32_t sc_unused, mn2;
+      pair(c, sc_unused, mn2);
+      u[2 * c] = __fmul_rn(ndmin, (float)(mn2 & 0xFFu));
+      u[2 * c + 1] = __fmul_rn(ndmin, (float)(mn2 >> 8));
+    }
+  }
+};
+
+// four int8 (offset by 128 into unsigned bytes) of `x` -> two half2, element order kept
+__device__ __forceinline__ __half2 q8_pair(uint32_t x_biased, uint32_t sel) {
+  return __hsub2(bits_h2(__byte_perm(x_biased, 0x64646464u, sel)), h2_const(0x6480));  // (1024 + q + 128) - 1152
+}
+
+struct DeqQ80 {
+  uint4 hdr, qs[4];
+  __device__ __forceinline__ void load(const unsigned char* row) { hdr = *reinterpret_cast<const uint4*>(row); }
+  __device__ __forceinline__ void store_scales(unsigned char* scl, int slot, int t) const {
+    float* d8 = reinterpret_cast<float*>(scl + slot * 4096);
+    const uint32_t hw[4] = {hdr.x, hdr.y, hdr.z, hdr.w};
+#pragma unroll
+    for (int b = 0; b < 8; ++b) d8[b * 128 + t] = half_bits_to_float((b & 1) ? hw[b >> 1] >> 16 : hw[b >> 1] & 0xFFFFu);
+  }
+  __device__ __forceinline__ void load_stage(int c, const unsigned char* row) {
+#pragma unroll
+    for (int jj = 0; jj < 4; ++jj) qs[jj] = *reinterpret_cast<const uint4*>(row + 16 + 64 * c + 16 * jj);
+  }
+  __device__ __forceinline__ void stage(int, unsigned char* orow, int t) const {
+#pragma unroll
+    for (int jj = 0; jj < 4; ++jj) {
+      const uint4 q = qs[jj];
+      const uint32_t x0 = q.x ^ 0x80808080u, x1 = q.y ^ 0x80808080u, x2 = q.z ^ 0x80808080u, x3 = q.w ^ 0x80808080u;
+      put16(orow, 2 * jj, t, h2_bits(q8_pair(x0, 0x4140)), h2_bits(q8_pair(x0, 0x4342)), h2_bits(q8_pair(x1, 0x4140)), h2_bits(q8_pair(x1, 0x4342)));
+      put16(orow, 2 * jj + 1, t, h2_bits(q8_pair(x2, 0x4140)), h2_bits(q8_pair(x2, 0x4342)), h2_bits(q8_pair(x3, 0x4140)), h2_bits(q8_pair(x3, 0x4342)));
+    }
+  }
+  __device__ __forceinline__ void mins(float (&)[8]) const {}
+};
+
+// an integer -128 .. 127 as (s, s)
+__device__ __forceinline__ __half2 small_h2(int s) { return __half2half2(__int2half_rn(s)); }
+// sixteen quants of one 16-element half with its scale: words of four quants q + 128 (biased) -> chunk pair `ch`, `ch` + 1
+template <int kTerms>
+__device__ __forceinline__ void put_half(unsigned char* orow, int ch, int t, const uint32_t (&xb)[4], int sc) {
+  uint32_t hi[8], lo[8];
+  const __half2 s_hi = small_h2(kTerms == 2 ? sc & ~1 : sc), s_lo = small_h2(sc & 1);  // sc = (sc & ~1) + (sc & 1), also below zero
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const __half2 a = q8_pair(xb[k], 0x4140), b = q8_pair(xb[k], 0x4342);
+    hi[2 * k] = h2_bits(__hmul2(a, s_hi));
+    hi[2 * k + 1] = h2_bits(__hmul2(b, s_hi));
+    if (kTerms == 2) {
+      lo[2 * k] = h2_bits(__hmul2(a, s_lo));
+      lo[2 * k + 1] = h2_bits(__hmul2(b, s_lo));
+    }
+  }
+  put16(orow, ch, t, hi[0], hi[1], hi[2], hi[3]);
+  put16(orow, ch + 1, t, hi[4], hi[5], hi[6], hi[7]);
+  if (kTerms == 2) {
+    put16(orow + STAGE_BYTES, ch, t, lo[0], lo[1], lo[2], lo[3]);
+    put16(orow + STAGE_BYTES, ch + 1, t, lo[4], lo[5], lo[6], lo[7]);
+  }
+}
+
+// Q5_K and IQ4_XS in the generic form: f32 d | f32 dmin | int8 scale[16] | uint8 min[16] | pad | int8 quant[256]
+template <int kTerms>
+struct DeqK16 {
+  uint4 h0, h1, h2, qs[4];
+  __device__ __forceinline__ void load(const unsigned char* row) {
+    h0 = *reinterpret_cast<const uint4*>(row);
+    h1 = *reinterpret_cast<const uint4*>(row + 16);
+    h2 = *reinterpret_cast<const uint4*>(row + 32);
+  }
+  __device__ __forceinline__ void store_scales(unsigned char* scl, int slot, int t) const { reinterpret_cast<uint32_t*>(scl + slot * 512)[t] = h0.x; }
+  __device__ __forceinline__ void load_stage(int c, const unsigned char* row) {
+#pragma unroll
+    for (int jj = 0; jj < 4; ++jj) qs[jj] = *reinterpret_cast<const uint4*>(row + 48 + 64 * c + 16 * jj);
+  }
+  __device__ __forceinline__ void stage(int c, unsigned char* orow, int t) const {
+    const uint32_t scw = c == 0 ? h0.z : c == 1 ? h0.w : c == 2 ? h1.x : h1.y;  // the four halves' scales
+#pragma unroll
+    for (int jj = 0; jj < 4; ++jj) {
+      const uint4 q = qs[jj];
+      const uint32_t xb[4] = {q.x ^ 0x80808080u, q.y ^ 0x80808080u, q.z ^ 0x80808080u, q.w ^ 0x80808080u};
+      put_half<kTerms>(orow, 2 * jj, t, xb, (int)(int8_t)(scw >> (8 * jj)));
+    }
+  }
+  __device__ __forceinline__ void mins(float (&u)[8]) const {
+    const float ndmin = -__uint_as_float(h0.y);
+    const uint32_t m[4] = {h1.z, h1.w, h2.x, h2.y};
+#pragma unroll
+    for (int b = 0; b < 8; ++b) u[b] = __fmul_rn(ndmin, (float)((m[b >> 1] >> (16 * (b & 1))) & 0xFFu));  // (both halves of a block share it)
+  }
+};
+
+// Q6_K packed: ql[128] | qh[64] | int8 scale[16] | fp16 d (csrc/izb_types.cu: q6p_word)
+struct DeqQ6K {
+  uint4 sc, h[2], l[4];
+  uint32_t d;
+  __device__ __forceinline__ void load(const unsigned char* row) {
+    sc = *reinterpret_cast<const uint4*>(row + 192);
+    d = *reinterpret_cast<const unsigned short*>(row + 208);
+  }
+  __device__ __forceinline__ void store_scales(unsigned char* scl, int slot, int t) const { reinterpret_cast<float*>(scl + slot * 512)[t] = half_bits_to_float(d); }
+  __device__ __forceinline__ void load_stage(int c, const unsigned char* row) {
+    const unsigned char* pl = row + 64 * (c >> 1);
+    const unsigned char* ph = row + 128 + 32 * (c >> 1);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) l[i] = *reinterpret_cast<const uint4*>(pl + 16 * i);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) h[i] = *reinterpret_cast<const uint4*>(ph + 16 * i);
+  }
+  __device__ __forceinline__ void stage(int c, unsigned char* orow, int t) const {
+    const int up = c & 1;  // blocks 2c, 2c + 1: sub-blocks 2 up, 2 up + 1 of half c / 2
+    const uint32_t scw = c == 0 ? sc.x : c == 1 ? sc.y : c == 2 ? sc.z : sc.w;
+#pragma unroll
+    for (int hl = 0; hl < 2; ++hl) {
+      const uint32_t hw[4] = {h[hl].x, h[hl].y, h[hl].z, h[hl].w};
+#pragma unroll
+      for (int o = 0; o < 2; ++o) {  // sub-block 2 up + o
+        const uint4 lq = l[2 * o + hl];
+        const uint32_t lw[4] = {lq.x, lq.y, lq.z, lq.w};
+        uint32_t xb[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const uint32_t qu = ((lw[k] >> (4 * up)) & 0x0F0F0F0Fu) | (((hw[k] >> (4 * up + 2 * o)) & 0x03030303u) << 4);
+          xb[k] = qu + 0x60606060u;  // 0..63 -> q + 128 (96..159 per byte, no carry)
+        }
+        put_half<2>(orow, 4 * o + 2 * hl, t, xb, (int)(int8_t)(scw >> (8 * (2 * o + hl))));
+      }
+    }
+  }
+  __device__ __forceinline__ void mins(float (&)[8]) const {}
+};
+
+template <class F, bool kDots> struct DeqOf;
+template <bool kDots> struct DeqOf<FQ4K, kDots> { using type = DeqQ4K<kDots>; };
+template <bool kDots> struct DeqOf<FQ80, kDots> { using type = DeqQ80; };
+template <bool kDots> struct DeqOf<FQ5K, kDots> { using type = DeqK16<1>; };
+template <bool kDots> struct DeqOf<FIQ4, kDots> { using type = DeqK16<2>; };
+template <bool kDots> struct DeqOf<FQ6K, kDots> { using type = DeqQ6K; };
+
+// What a hand-over costs (measured on one SM): a satisfied mbarrier test has 54 clk of latency, an arrival is seen by a waiting
+// warp of the same CTA 135 clk later, a tcgen05.commit 182 clk after the last MMA; with three accumulators in the ring
+// that alone allows no block in under 175 clk.  An MMA or commit behind a lane test takes 98 clk to issue, with the elected
+// predicate inside the statement about 25 (6 % of the kernel).  The rest of a block's 550 clk is the combine warps' own
+// chain: test, two 65-clk reads of 32 columns, the packed FMAs and the register copies the compiler puts between the two.
+template <class F, bool kDots>
 __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_constant__ CUtensorMap tmW, const TcParams p) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  using MP = Map<QT>;
-  constexpr int NA = MP::NA, NB = MP::NB, OFF_A = MP::OFF_A, OFF_B = MP::OFF_B, OFF_RAW = MP::OFF_RAW, OFF_DM = MP::OFF_SCL,
-                OFF_D8 = MP::OFF_SCL, OFF_ASC = MP::OFF_ASC, OFF_BAR = MP::OFF_BAR, NUM_BARS = MP::NUM_BARS;
-  constexpr int A_FULL = MP::A_FULL, A_EMPTY = MP::A_EMPTY, B_FULL = MP::B_FULL, B_EMPTY = MP::B_EMPTY, RAW_FULL = MP::RAW_FULL,
-                RAW_EMPTY = MP::RAW_EMPTY, D1_FULL = MP::D1_FULL, D1_EMPTY = MP::D1_EMPTY, D2_FULL = MP::D2_FULL,
-                D2_EMPTY = MP::D2_EMPTY, ASC_FULL = MP::ASC_FULL, ASC_EMPTY = MP::ASC_EMPTY;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BAR);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + OFF_BAR + NUM_BARS * 8);
-  volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(smem + OFF_BAR + NUM_BARS * 8 + 4);
+  using MP = Map<F>;
+  constexpr int NA = MP::NA, NB = MP::NB, NR = MP::NR, RAW = MP::RAW, SBB = F::SBB;
+  constexpr bool kMins = F::kMin && !kDots;
+  constexpr int SPS = kMins ? 5 : 4;  // operand stages per superblock: four of 64 K-elements (+ the min-term stage)
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + MP::OFF_BAR);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + MP::OFF_BAR + MP::NUM_BARS * 8);
+  volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(smem + MP::OFF_BAR + MP::NUM_BARS * 8 + 4);
   const uint32_t bar0 = smem_u32(bars);
   auto bar = [&](int i) -> uint32_t { return bar0 + 8u * (uint32_t)i; };
-
-  // ---- the CTA's work: output tiles blockIdx.x, blockIdx.x + gridDim.x, ... of (row tiles) x (N / 128 column tiles), column
-  // tile fastest.  Every role walks the same list; its ring positions and barrier parities run on from tile to tile, so
-  // the producers, the dequantisers and the MMA issuers are already inside the next tile while the combine warps
-  // store the current one.
-  const int n_ntiles = p.N / BN;
-  const int n_work = (p.tiles ? p.tiles[0] : p.n_mtiles) * n_ntiles;
-  if ((int)blockIdx.x >= n_work) return;  // uniform over the CTA, before any barrier or TMEM use
-  const int nsb = p.K >> 8, nb = p.K >> 5;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  constexpr int SBB = QT == IZB_Q4_K ? 144 : 272;
-  constexpr int RAW = MP::RAW, NR = MP::NR;
-  constexpr bool kMins = QT == IZB_Q4_K && !kDots;
-  constexpr int SPS = kMins ? 5 : 4;  // operand stages per superblock: four of 64 K-elements (+ the min-term stage)
-  const int nstages = SPS * nsb;
 
+  pdl_launch_next();
   if (threadIdx.x == 0) {
-    // Consumers release a buffer with one arrival per THREAD, not per warp: an elected lane costs a divergent branch and a
-    // warp barrier per hand-over, which measured 10 % of the kernel (and one predicated arrival per warp measured no
-    // better than 32).  A_FULL: the activation producer's expect_tx arrival; B_FULL: the 128 dequantiser threads;
-    // A_EMPTY / B_EMPTY: one tcgen05.commit each
-    constexpr int kDeqArr = 128, kCmbArr = 256;
-    for (int i = 0; i < NA; ++i) { mbar_init(bar(A_FULL + i), 1); mbar_init(bar(A_EMPTY + i), 1); }
-    for (int i = 0; i < NB; ++i) { mbar_init(bar(B_FULL + i), kDeqArr); mbar_init(bar(B_EMPTY + i), 1); }
-    for (int i = 0; i < NR; ++i) { mbar_init(bar(RAW_FULL + i), 1); mbar_init(bar(RAW_EMPTY + i), kDeqArr); }
-    for (int i = 0; i < ND1; ++i) { mbar_init(bar(D1_FULL + i), 1); mbar_init(bar(D1_EMPTY + i), kCmbArr); }
-    mbar_init(bar(D2_FULL), 1);
-    mbar_init(bar(D2_EMPTY), kCmbArr);
-    for (int i = 0; i < NASC; ++i) { mbar_init(bar(ASC_FULL + i), 1); mbar_init(bar(ASC_EMPTY + i), kCmbArr); }
+    // Consumers release a buffer with one arrival per THREAD (128 dequantisers, 256 combine threads): one elected arrival per
+    // warp, predicated without a branch, measured 5 % slower (8192 x 17408 x 5120: 3.25 against 3.10 ms).  A_EMPTY / B_EMPTY: one
+    // tcgen05.commit each
+    for (int i = 0; i < NA; ++i) { mbar_init(bar(MP::A_FULL + i), 1); mbar_init(bar(MP::A_EMPTY + i), 1); }
+    for (int i = 0; i < NB; ++i) { mbar_init(bar(MP::B_FULL + i), 128); mbar_init(bar(MP::B_EMPTY + i), 1); }
+    for (int i = 0; i < NR; ++i) { mbar_init(bar(MP::RAW_FULL + i), 1); mbar_init(bar(MP::RAW_EMPTY + i), 128); }
+    for (int i = 0; i < ND1; ++i) { mbar_init(bar(MP::D1_FULL + i), 1); mbar_init(bar(MP::D1_EMPTY + i), 256); }
+    mbar_init(bar(MP::D2_FULL), 1);
+    mbar_init(bar(MP::D2_EMPTY), 256);
+    for (int i = 0; i < NASC; ++i) { mbar_init(bar(MP::ASC_FULL + i), 1); mbar_init(bar(MP::ASC_EMPTY + i), 256); }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -528,23 +700,42 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();
+
+  // ---- the CTA's work: items blockIdx.x, blockIdx.x + gridDim.x, ... of (row tiles) x (column tiles) x (K parts), K part
+  // fastest, then column tile.  Every role walks the same list; its ring positions and barrier parities run on from item to
+  // item, so the producers, the dequantisers and the issuers are already inside the next one while the combine warps store.
+  const int n_ntiles = (p.N + BN - 1) / BN, nsb = p.K >> 8, nb = p.K >> 5;
+  const int n_work = (p.tiles ? p.tiles[0] : p.n_mtiles) * n_ntiles * p.n_split;
+  struct Item { int tile, nt, ks, s0, s1; };
+  auto item = [&](int w) -> Item {
+    Item it;
+    it.ks = 0;
+    int q = w;
+    if (p.n_split > 1) { q = w / p.n_split; it.ks = w - q * p.n_split; }
+    it.tile = q / n_ntiles;
+    it.nt = q - it.tile * n_ntiles;
+    it.s0 = it.ks * nsb / p.n_split;
+    it.s1 = (it.ks + 1) * nsb / p.n_split;
+    return it;
+  };
 
   if (warp < 4) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
-    // Every role loop below is executed by its whole warp (uniform waits, lane 0 issues), so no lane of a role warp
+    // Every role loop below is executed by its whole warp (uniform waits, an elected lane issues), so no lane of a role warp
     // sits at the final CTA barrier while another lane of the same warp is still working.
     if (warp == 0) {
       // ================= activation producer: the tile's stage images lie back to back in global memory
       int sa = 0, pa = 1;
       bool ok = true;
       for (int w = blockIdx.x; w < n_work && ok; w += gridDim.x) {
-        const int tile = w / n_ntiles;
-        const unsigned char* src = reinterpret_cast<const unsigned char*>(p.aimg) + (size_t)tile * nstages * STAGE_BYTES;
-        for (int g = 0; g < nstages; ++g) {
-          if (!mbar_wait(bar(A_EMPTY + sa), pa, abort_flag, p.err, p.spin_limit, E_APROD)) { ok = false; break; }
+        const Item it = item(w);
+        const unsigned char* src = reinterpret_cast<const unsigned char*>(p.aimg) + (size_t)it.tile * nsb * SPS * STAGE_BYTES;
+        for (int g = it.s0 * SPS; g < it.s1 * SPS; ++g) {
+          if (!mbar_wait(bar(MP::A_EMPTY + sa), pa, abort_flag, p.err, p.spin_limit, E_APROD)) { ok = false; break; }
           if (lane == 0 && g != p.skip_stage) {  // (skip_stage: diagnostics only, makes the waits of this stage run out)
-            mbar_expect_tx(bar(A_FULL + sa), STAGE_BYTES);
-            bulk_g2s(smem_u32(smem + OFF_A + sa * STAGE_BYTES), src + (size_t)g * STAGE_BYTES, STAGE_BYTES, bar(A_FULL + sa));
+            mbar_expect_tx(bar(MP::A_FULL + sa), STAGE_BYTES);
+            bulk_g2s(smem_u32(smem + MP::OFF_A + sa * STAGE_BYTES), src + (size_t)g * STAGE_BYTES, STAGE_BYTES, bar(MP::A_FULL + sa));
           }
           __syncwarp();
           if (++sa == NA) { sa = 0; pa ^= 1; }
@@ -556,83 +747,74 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
       int rb = 0, pr = 1, sq = 0, pq = 1;
       bool ok = true;
       for (int w = blockIdx.x; w < n_work && ok; w += gridDim.x) {
-      const int tile = w / n_ntiles;
-      const int wrow = (p.tiles ? p.tiles[1 + 3 * tile] : p.mat) * p.N + (w % n_ntiles) * BN;
-      for (int s = 0; s < nsb; ++s) {
-        if (!mbar_wait(bar(RAW_EMPTY + rb), pr, abort_flag, p.err, p.spin_limit, E_WPROD)) { ok = false; break; }
-        if (lane == 0) {
-          mbar_expect_tx(bar(RAW_FULL + rb), RAW);
-          tma_2d(smem_u32(smem + OFF_RAW + rb * RAW), &tmW, s * (SBB / 4), wrow, bar(RAW_FULL + rb));
-        }
-        if (++rb == NR) { rb = 0; pr ^= 1; }
-        if (!kDots) {
-          if (!mbar_wait(bar(ASC_EMPTY + sq), pq, abort_flag, p.err, p.spin_limit, E_WPROD)) { ok = false; break; }
+        const Item it = item(w);
+        const int wrow = (p.tiles ? p.tiles[1 + 3 * it.tile] : p.mat) * p.N + it.nt * BN;
+        for (int s = it.s0; s < it.s1; ++s) {
+          if (!mbar_wait(bar(MP::RAW_EMPTY + rb), pr, abort_flag, p.err, p.spin_limit, E_WPROD)) { ok = false; break; }
           if (lane == 0) {
-            mbar_expect_tx(bar(ASC_FULL + sq), 4096);
-            bulk_g2s(smem_u32(smem + OFF_ASC + sq * 4096), p.ascimg + ((size_t)tile * nb + 8 * s) * BM, 4096, bar(ASC_FULL + sq));
+            mbar_expect_tx(bar(MP::RAW_FULL + rb), RAW);
+            tma_2d(smem_u32(smem + MP::OFF_RAW + rb * RAW), &tmW, s * (SBB / 4), wrow, bar(MP::RAW_FULL + rb));
           }
-          if (++sq == NASC) { sq = 0; pq ^= 1; }
-        }
-        __syncwarp();
-      }
-      }
-    } else {
-      // ================= MMA issuers.  Of a superblock's stages 0..3 (two 32-blocks each, every block into its own
-      // accumulator buffer: two MMAs of K = 16 + one commit) warp 1 takes 0 and 2, warp 2 takes 1, 3 and the min-term stage 4
-      // (three bf16 MMAs of K = 16 accumulated into the fourth TMEM buffer over the whole of K).  Two issuers because
-      // what a thread pays per block -- barrier polls and commits between MMAs -- is longer than the 128 cycles the two
-      // MMAs run; one issuer for the min term so that its accumulator is updated in program order.
-      bool ok = true;
-      int it = 0;  // tiles done: stage and block counts run on across tiles
-      for (int w = blockIdx.x; w < n_work && ok; w += gridDim.x, ++it) {
-      const int gs = it * nstages, jb = it * nb;
-      for (int s = 0; s < nsb && ok; ++s) {
-        for (int t = warp - 1; t < (warp == 1 ? 4 : SPS) && ok; t += (t == 3 ? 1 : 2)) {
-          const int g = gs + SPS * s + t, sa = g % NA, sb = g % NB;
-          TRACE(10, g);
-          if (!mbar_wait(bar(B_FULL + sb), (g / NB) & 1, abort_flag, p.err, p.spin_limit, E_MMA)) { ok = false; break; }
-          TRACE(11, g);
-          if (!mbar_wait(bar(A_FULL + sa), (g / NA) & 1, abort_flag, p.err, p.spin_limit, E_MMA)) { ok = false; break; }
-          TRACE(12, g);
-          tc_fence_after();
-          const uint32_t a_addr = smem_u32(smem + OFF_A + sa * STAGE_BYTES), b_addr = smem_u32(smem + OFF_B + sb * STAGE_BYTES);
-          if (t < 4) {
-#pragma unroll
-            for (int blk = 0; blk < 2; ++blk) {
-              const int j = jb + 8 * s + 2 * t + blk, d = j % ND1;
-              TRACE(0, j);
-              if (!mbar_wait(bar(D1_EMPTY + d), ((j / ND1) & 1) ^ 1, abort_flag, p.err, p.spin_limit, E_MMA)) { ok = false; break; }
-              TRACE(1, j);
-              tc_fence_after();
-              if (lane == 0) {
-                const uint32_t dt = tmem_base + (uint32_t)(d * BN);
-#pragma unroll
-                for (int k16 = 0; k16 < 2; ++k16)
-                  tc_mma_f16(dt, umma_desc(a_addr + blk * 64 + k16 * 32), umma_desc(b_addr + blk * 64 + k16 * 32), kIdescF16, k16);
-                tc_commit(bar(D1_FULL + d));
-              }
-              TRACE(2, j);
-              __syncwarp();
-            }
-            if (!ok) break;
-          } else {
-            // the min-term accumulator of the tile before must have been read before this tile's first MMA clears it
-            if (s == 0 && it > 0 && !mbar_wait(bar(D2_EMPTY), (it - 1) & 1, abort_flag, p.err, p.spin_limit, E_MMA)) { ok = false; break; }
-            tc_fence_after();
+          if (++rb == NR) { rb = 0; pr ^= 1; }
+          if (!kDots) {
+            if (!mbar_wait(bar(MP::ASC_EMPTY + sq), pq, abort_flag, p.err, p.spin_limit, E_WPROD)) { ok = false; break; }
             if (lane == 0) {
-#pragma unroll
-              for (int k16 = 0; k16 < 3; ++k16)
-                tc_mma_f16(tmem_base + ND1 * BN, umma_desc(a_addr + k16 * 32), umma_desc(b_addr + k16 * 32), kIdescBF16, (s | k16) ? 1u : 0u);
+              mbar_expect_tx(bar(MP::ASC_FULL + sq), 4096);
+              bulk_g2s(smem_u32(smem + MP::OFF_ASC + sq * 4096), p.ascimg + ((size_t)it.tile * nb + 8 * s) * BM, 4096, bar(MP::ASC_FULL + sq));
             }
-          }
-          if (lane == 0) {
-            tc_commit(bar(A_EMPTY + sa));
-            tc_commit(bar(B_EMPTY + sb));
-            if (kMins && t == 4 && s == nsb - 1) tc_commit(bar(D2_FULL));
+            if (++sq == NASC) { sq = 0; pq ^= 1; }
           }
           __syncwarp();
         }
       }
+    } else {
+      // ================= MMA issuers.  Of a superblock's stages 0..3 (two 32-blocks each, every block into its own
+      // accumulator buffer: two MMAs of K = 16 per term + one commit) warp 1 takes 0 and 2, warp 2 takes 1, 3 and the min-term
+      // stage 4 (three bf16 MMAs of K = 16 accumulated into the fourth TMEM buffer over the item's K range).  Two issuers
+      // because what a warp pays per block -- barrier tests and commits between MMAs -- is longer than the 128 cycles the two
+      // MMAs run; one issuer for the min term so that its accumulator is updated in program order.
+      bool ok = true;
+      int n_item = 0, gs = 0, jb = 0;  // items, stages and blocks done: they run on across items
+      for (int w = blockIdx.x; w < n_work && ok; w += gridDim.x, ++n_item) {
+        const Item it = item(w);
+        for (int s = it.s0; s < it.s1 && ok; ++s, gs += SPS, jb += 8) {
+          for (int t = warp - 1; t < (warp == 1 ? 4 : SPS) && ok; t += (t == 3 ? 1 : 2)) {
+            const int g = gs + t, sa = g % NA, sb = g % NB;
+            const uint32_t b_ok = mbar_test(bar(MP::B_FULL + sb), (g / NB) & 1), a_ok = mbar_test(bar(MP::A_FULL + sa), (g / NA) & 1);
+            if (!b_ok && !mbar_wait(bar(MP::B_FULL + sb), (g / NB) & 1, abort_flag, p.err, p.spin_limit, E_MMA)) { ok = false; break; }
+            if (!a_ok && !mbar_wait(bar(MP::A_FULL + sa), (g / NA) & 1, abort_flag, p.err, p.spin_limit, E_MMA)) { ok = false; break; }
+            tc_fence_after();
+            const uint32_t a_addr = smem_u32(smem + MP::OFF_A + sa * STAGE_BYTES), b_addr = smem_u32(smem + MP::OFF_B + sb * MP::BSTAGE);
+            if (t < 4) {
+#pragma unroll
+              for (int blk = 0; blk < 2; ++blk) {
+                const int j = jb + 2 * t + blk, d = j % ND1;
+                if (!mbar_wait(bar(MP::D1_EMPTY + d), ((j / ND1) & 1) ^ 1, abort_flag, p.err, p.spin_limit, E_MMA)) { ok = false; break; }
+                __syncwarp();
+                tc_fence_after();
+                const uint32_t dt = tmem_base + (uint32_t)(d * BN);
+#pragma unroll
+                for (int term = 0; term < F::kTerms; ++term)
+#pragma unroll
+                  for (int k16 = 0; k16 < 2; ++k16)
+                    tc_mma_f16(dt, umma_desc(a_addr + blk * 64 + k16 * 32), umma_desc(b_addr + term * STAGE_BYTES + blk * 64 + k16 * 32), kIdescF16, term | k16);
+                tc_commit(bar(MP::D1_FULL + d));
+              }
+              if (!ok) break;
+            } else {
+              // the min-term accumulator of the item before must have been read before this item's first MMA clears it
+              if (s == it.s0 && n_item > 0 && !mbar_wait(bar(MP::D2_EMPTY), (n_item - 1) & 1, abort_flag, p.err, p.spin_limit, E_MMA)) { ok = false; break; }
+              __syncwarp();
+              tc_fence_after();
+#pragma unroll
+              for (int k16 = 0; k16 < 3; ++k16)
+                tc_mma_f16(tmem_base + ND1 * BN, umma_desc(a_addr + k16 * 32), umma_desc(b_addr + k16 * 32), kIdescBF16, (s > it.s0 || k16) ? 1u : 0u);
+            }
+            tc_commit(bar(MP::A_EMPTY + sa));
+            tc_commit(bar(MP::B_EMPTY + sb));
+            if (kMins && t == 4 && s == it.s1 - 1) tc_commit(bar(MP::D2_FULL));
+          }
+        }
       }
     }
   } else if (warp < 8) {
@@ -642,123 +824,58 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
     bool ok = true;
     int sbq = 0, pbq = 1;  // operand ring position and wait parity
     int rb = 0, pr = 0;    // raw ring
-    int sbc = 0;           // superblocks done (all tiles): position in the 4-deep ring of superblock scales
-    for (int w = blockIdx.x; w < n_work && ok; w += gridDim.x)
-    for (int s = 0; s < nsb && ok; ++s, ++sbc) {
-      if (!mbar_wait(bar(RAW_FULL + rb), pr, abort_flag, p.err, p.spin_limit, E_DEQ)) { ok = false; break; }
-      const unsigned char* rrow = smem + OFF_RAW + rb * RAW + t * SBB;
-      const uint4 hdr = *reinterpret_cast<const uint4*>(rrow);
-      const uint32_t s3[3] = {hdr.y, hdr.z, hdr.w};
-      if (QT == IZB_Q4_K) {
-        if (kMins) reinterpret_cast<float*>(smem + OFF_DM + (sbc & 3) * 512)[t] = half_bits_to_float(hdr.x & 0xFFFFu);
-      } else {
-        float* d8 = reinterpret_cast<float*>(smem + OFF_D8 + (sbc & 3) * 4096);
-        const uint32_t hw[4] = {hdr.x, hdr.y, hdr.z, hdr.w};
-#pragma unroll
-        for (int b = 0; b < 8; ++b) d8[b * 128 + t] = half_bits_to_float((b & 1) ? hw[b >> 1] >> 16 : hw[b >> 1] & 0xFFFFu);
-      }
+    int sbc = 0;           // superblocks done (all items): position in the 4-deep ring of superblock scales
+    for (int w = blockIdx.x; w < n_work && ok; w += gridDim.x) {
+      const Item it = item(w);
+      for (int s = it.s0; s < it.s1 && ok; ++s, ++sbc) {
+        if (!mbar_wait(bar(MP::RAW_FULL + rb), pr, abort_flag, p.err, p.spin_limit, E_DEQ)) { ok = false; break; }
+        const unsigned char* rrow = smem + MP::OFF_RAW + rb * RAW + t * SBB;
+        typename DeqOf<F, kDots>::type dq;
+        dq.load(rrow);
+        if (!kDots) dq.store_scales(smem + MP::OFF_SCL, sbc & 3, t);
+        auto deliver = [&]() {
+          fence_proxy_async();
+          mbar_arrive(bar(MP::B_FULL + sbq));  // (every thread after its own stores and fence)
+          if (++sbq == NB) { sbq = 0; pbq ^= 1; }
+        };
 #pragma unroll 1  // (rolled on purpose: with the role loops resident at once, code size costs more than the loop)
-      for (int c = 0; c < 4; ++c) {
-        if (warp == 4) TRACE(7, sbc * SPS + c);
-        if (!mbar_wait(bar(B_EMPTY + sbq), pbq, abort_flag, p.err, p.spin_limit, E_DEQ)) { ok = false; break; }
-        if (warp == 4) TRACE(8, sbc * SPS + c);
-        unsigned char* orow = smem + OFF_B + sbq * STAGE_BYTES + t * 128;
-        if (QT == IZB_Q4_K) {
-          const uint4 q0 = *reinterpret_cast<const uint4*>(rrow + 16 + 32 * c), q1 = *reinterpret_cast<const uint4*>(rrow + 32 + 32 * c);
-          const uint32_t w[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-          // the chunk's two 6-bit sub-block scales as half2 pairs (sc, sc) and (-1024 sc, -1024 sc): 0x6400 | sc is the
-          // fp16 number 1024 + sc
-          int sc_lo = 1, sc_hi = 1, mn_unused;
-          if (!kDots) {
-            q4k_scale_min(s3, 2 * c, sc_lo, mn_unused);
-            q4k_scale_min(s3, 2 * c + 1, sc_hi, mn_unused);
-          }
-          const __half2 k1024 = __half2half2(__ushort_as_half((unsigned short)0x6400)), kneg = __half2half2(__ushort_as_half((unsigned short)0xE400));
-          const uint32_t blo = 0x64006400u | (uint32_t)sc_lo | ((uint32_t)sc_lo << 16), bhi = 0x64006400u | (uint32_t)sc_hi | ((uint32_t)sc_hi << 16);
-          const __half2 slo = __hsub2(*reinterpret_cast<const __half2*>(&blo), k1024), shi = __hsub2(*reinterpret_cast<const __half2*>(&bhi), k1024);
-          const __half2 nlo = __hmul2(slo, kneg), nhi = __hmul2(shi, kneg);
-          // High nibbles stay where they are: (word & 0x00F000F0) | 0x6400 is the fp16 number 1024 + 16 q, and
-          // (1024 + 16 q) * (sc / 16) - 64 sc = sc * q exactly (one rounding, of an integer below 2^11).  One shift per
-          // word (for its upper bytes) instead of three.
-          const __half2 k16th = __half2half2(__ushort_as_half((unsigned short)0x2C00));  // 1 / 16
-          const __half2 shi16 = __hmul2(shi, k16th), nhi16 = __hmul2(nhi, k16th);
-          auto cv = [](uint32_t word, uint32_t mask, __half2 scale, __half2 neg) -> uint32_t {
-            const uint32_t bitsv = (word & mask) | 0x64006400u;
-            const __half2 r = __hfma2(*reinterpret_cast<const __half2*>(&bitsv), scale, neg);
-            return *reinterpret_cast<const uint32_t*>(&r);
-          };
-#pragma unroll
-          for (int jj = 0; jj < 4; ++jj) {
-            const uint32_t w0 = w[2 * jj], w1 = w[2 * jj + 1], x0 = w0 >> 8, x1 = w1 >> 8;
-            *reinterpret_cast<uint4*>(orow + ((jj ^ (t & 7)) << 4)) =
-                make_uint4(cv(w0, 0x000F000Fu, slo, nlo), cv(x0, 0x000F000Fu, slo, nlo), cv(w1, 0x000F000Fu, slo, nlo), cv(x1, 0x000F000Fu, slo, nlo));
-            *reinterpret_cast<uint4*>(orow + (((4 + jj) ^ (t & 7)) << 4)) =
-                make_uint4(cv(w0, 0x00F000F0u, shi16, nhi16), cv(x0, 0x00F000F0u, shi16, nhi16), cv(w1, 0x00F000F0u, shi16, nhi16), cv(x1, 0x00F000F0u, shi16, nhi16));
-          }
-        } else {
-          const __half2 bias = __half2half2(__int2half_rn(1152));
-          auto cvt = [&](uint32_t x, uint32_t sel) -> uint32_t {
-            const uint32_t bitsv = __byte_perm(x, 0x64646464u, sel);  // (1024 + (q + 128)) in both halves
-            const __half2 r = __hsub2(*reinterpret_cast<const __half2*>(&bitsv), bias);
-            return *reinterpret_cast<const uint32_t*>(&r);
-          };
-#pragma unroll
-          for (int jj = 0; jj < 4; ++jj) {
-            const uint4 q = *reinterpret_cast<const uint4*>(rrow + 16 + 64 * c + 16 * jj);
-            const uint32_t x0 = q.x ^ 0x80808080u, x1 = q.y ^ 0x80808080u, x2 = q.z ^ 0x80808080u, x3 = q.w ^ 0x80808080u;
-            *reinterpret_cast<uint4*>(orow + (((2 * jj) ^ (t & 7)) << 4)) =
-                make_uint4(cvt(x0, 0x4140), cvt(x0, 0x4342), cvt(x1, 0x4140), cvt(x1, 0x4342));
-            *reinterpret_cast<uint4*>(orow + (((2 * jj + 1) ^ (t & 7)) << 4)) =
-                make_uint4(cvt(x2, 0x4140), cvt(x2, 0x4342), cvt(x3, 0x4140), cvt(x3, 0x4342));
-          }
+        for (int c = 0; c < 4; ++c) {
+          dq.load_stage(c, rrow);
+          if (!mbar_wait(bar(MP::B_EMPTY + sbq), pbq, abort_flag, p.err, p.spin_limit, E_DEQ)) { ok = false; break; }
+          dq.stage(c, smem + MP::OFF_B + sbq * MP::BSTAGE + t * 128, t);
+          deliver();
         }
-        fence_proxy_async();
-        mbar_arrive(bar(B_FULL + sbq));  // (every thread after its own stores and fence)
-        if (warp == 4) TRACE(9, sbc * SPS + c);
-        if (++sbq == NB) { sbq = 0; pbq ^= 1; }
-      }
-      if (!ok) break;
-      if (kMins) {
-        // the min-term stage: u[b] = -dmin * mn[b] (exact in f32: 11 x 6 bits) as three bf16 terms u1 + u2 + u3; the
-        // stage's six 16-byte chunks hold (u1, u2, u1, u3, u2, u1) for the eight blocks, against the activation side's
-        // (v1, v1, v2, v1, v2, v3)
-        if (!mbar_wait(bar(B_EMPTY + sbq), pbq, abort_flag, p.err, p.spin_limit, E_DEQ)) { ok = false; break; }
-        const float ndmin = -half_bits_to_float(hdr.x >> 16);
-        uint32_t u1[4], u2[4], u3[4];
+        if (!ok) break;
+        mbar_arrive(bar(MP::RAW_EMPTY + rb));
+        if (++rb == NR) { rb = 0; pr ^= 1; }
+        if (kMins) {
+          // the min-term stage: u[b] = -dmin * mn[b] (exact in f32: 11 x 6 bits) as three bf16 terms u1 + u2 + u3; the
+          // stage's six 16-byte chunks hold (u1, u2, u1, u3, u2, u1) for the eight blocks, against the activation side's
+          // (v1, v1, v2, v1, v2, v3)
+          float u[8];
+          dq.mins(u);
+          uint32_t u1[4], u2[4], u3[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          uint32_t h[2][3];
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            int sc_unused, mn;
-            q4k_scale_min(s3, 2 * k + e, sc_unused, mn);
-            const float u = __fmul_rn(ndmin, (float)mn);
-            const __nv_bfloat16 h1 = __float2bfloat16_rn(u);
-            const float r1 = __fsub_rn(u, __bfloat162float(h1));
-            const __nv_bfloat16 h2 = __float2bfloat16_rn(r1);
-            const __nv_bfloat16 h3 = __float2bfloat16_rn(__fsub_rn(r1, __bfloat162float(h2)));
-            h[e][0] = __bfloat16_as_ushort(h1);
-            h[e][1] = __bfloat16_as_ushort(h2);
-            h[e][2] = __bfloat16_as_ushort(h3);
+          for (int k = 0; k < 4; ++k) {
+            const __nv_bfloat162 h1 = __floats2bfloat162_rn(u[2 * k], u[2 * k + 1]);
+            const float ra = __fsub_rn(u[2 * k], __low2float(h1)), rb2 = __fsub_rn(u[2 * k + 1], __high2float(h1));
+            const __nv_bfloat162 h2 = __floats2bfloat162_rn(ra, rb2);
+            const __nv_bfloat162 h3 = __floats2bfloat162_rn(__fsub_rn(ra, __low2float(h2)), __fsub_rn(rb2, __high2float(h2)));
+            u1[k] = *reinterpret_cast<const uint32_t*>(&h1);
+            u2[k] = *reinterpret_cast<const uint32_t*>(&h2);
+            u3[k] = *reinterpret_cast<const uint32_t*>(&h3);
           }
-          u1[k] = h[0][0] | (h[1][0] << 16);
-          u2[k] = h[0][1] | (h[1][1] << 16);
-          u3[k] = h[0][2] | (h[1][2] << 16);
+          if (!mbar_wait(bar(MP::B_EMPTY + sbq), pbq, abort_flag, p.err, p.spin_limit, E_DEQ)) { ok = false; break; }
+          unsigned char* orow = smem + MP::OFF_B + sbq * MP::BSTAGE + t * 128;
+          put16(orow, 0, t, u1[0], u1[1], u1[2], u1[3]);
+          put16(orow, 1, t, u2[0], u2[1], u2[2], u2[3]);
+          put16(orow, 2, t, u1[0], u1[1], u1[2], u1[3]);
+          put16(orow, 3, t, u3[0], u3[1], u3[2], u3[3]);
+          put16(orow, 4, t, u2[0], u2[1], u2[2], u2[3]);
+          put16(orow, 5, t, u1[0], u1[1], u1[2], u1[3]);
+          deliver();
         }
-        unsigned char* orow = smem + OFF_B + sbq * STAGE_BYTES + t * 128;
-        const uint4 c1 = make_uint4(u1[0], u1[1], u1[2], u1[3]), c2 = make_uint4(u2[0], u2[1], u2[2], u2[3]), c3 = make_uint4(u3[0], u3[1], u3[2], u3[3]);
-        *reinterpret_cast<uint4*>(orow + ((0 ^ (t & 7)) << 4)) = c1;
-        *reinterpret_cast<uint4*>(orow + ((1 ^ (t & 7)) << 4)) = c2;
-        *reinterpret_cast<uint4*>(orow + ((2 ^ (t & 7)) << 4)) = c1;
-        *reinterpret_cast<uint4*>(orow + ((3 ^ (t & 7)) << 4)) = c3;
-        *reinterpret_cast<uint4*>(orow + ((4 ^ (t & 7)) << 4)) = c2;
-        *reinterpret_cast<uint4*>(orow + ((5 ^ (t & 7)) << 4)) = c1;
-        fence_proxy_async();
-        mbar_arrive(bar(B_FULL + sbq));  // (every thread after its own stores and fence)
-        if (++sbq == NB) { sbq = 0; pbq ^= 1; }
       }
-      mbar_arrive(bar(RAW_EMPTY + rb));
-      if (++rb == NR) { rb = 0; pr ^= 1; }
     }
   } else {
     // ================= combine: thread <-> TMEM lane (token row) 32*(warp%4) + lane, 64 of the 128 columns.
@@ -769,120 +886,126 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
     const uint32_t t_lane = tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)(half * 64);
     bool ok = true;
     int d = 0, pd = 0, sq = 0, pq = 0;  // accumulator ring / scale ring positions and wait parities
-    int sbc = 0, it = 0;                // superblocks and tiles done
-    for (int w = blockIdx.x; w < n_work && ok; w += gridDim.x, ++it) {
-    const int tile = w / n_ntiles, n0 = (w % n_ntiles) * BN;
-    const int r0 = p.tiles ? p.tiles[2 + 3 * tile] : tile * BM;
-    const int nr = p.tiles ? p.tiles[3 + 3 * tile] : min(BM, p.M - r0);
-    const bool row_ok = r < nr;
-    const int out_row = r0 + r;
-    unsigned long long res2[32], tq2[32];  // pairs of columns (2i, 2i+1)
+    int sbc = 0, n_item = 0;            // superblocks and items done
+    for (int w = blockIdx.x; w < n_work && ok; w += gridDim.x, ++n_item) {
+      const Item it = item(w);
+      const int n0 = it.nt * BN;
+      const int r0 = p.tiles ? p.tiles[2 + 3 * it.tile] : it.tile * BM;
+      const int nr = p.tiles ? p.tiles[3 + 3 * it.tile] : min(BM, p.M - r0);
+      const bool row_ok = r < nr;
+      const int out_row = r0 + r;
+      unsigned long long res2[32], tq2[32];  // pairs of columns (2i, 2i+1)
 #pragma unroll
-    for (int c = 0; c < 32; ++c) res2[c] = tq2[c] = 0ull;
-    for (int s = 0; s < nsb && ok; ++s, ++sbc) {
-      const float* as = reinterpret_cast<const float*>(smem + OFF_ASC + sq * 4096) + r;  // this row's 8 block scales
-      if (!kDots && !mbar_wait(bar(ASC_FULL + sq), pq, abort_flag, p.err, p.spin_limit, E_EPI)) { ok = false; break; }
+      for (int c = 0; c < 32; ++c) res2[c] = tq2[c] = 0ull;
+      for (int s = it.s0; s < it.s1 && ok; ++s, ++sbc) {
+        const float* as = reinterpret_cast<const float*>(smem + MP::OFF_ASC + sq * 4096) + r;  // this row's 8 block scales
+        if (!kDots && !mbar_wait(bar(MP::ASC_FULL + sq), pq, abort_flag, p.err, p.spin_limit, E_EPI)) { ok = false; break; }
 #pragma unroll
-      for (int b = 0; b < 8; ++b) {
-        const unsigned long long a2 = pack2(kDots ? 0.0f : as[b * BM]);
-        if (warp == 8) TRACE(3, sbc * 8 + b);
-        if (!mbar_wait(bar(D1_FULL + d), pd, abort_flag, p.err, p.spin_limit, E_EPI)) { ok = false; break; }
-        if (warp == 8) TRACE(4, sbc * 8 + b);
-        tc_fence_after();
+        for (int b = 0; b < 8; ++b) {
+          const unsigned long long a2 = pack2(kDots ? 0.0f : as[b * BM]);
+          if (!mbar_wait(bar(MP::D1_FULL + d), pd, abort_flag, p.err, p.spin_limit, E_EPI)) { ok = false; break; }
+          tc_fence_after();
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {  // 32 columns at a time: the block loop's working set stays inside the register budget
-          unsigned long long v[16];
-          tc_ld32_pairs(t_lane + (uint32_t)(d * BN + 32 * h), v);
-          if (h == 1) {
-            tc_fence_before();
-            if (warp == 8) TRACE(5, sbc * 8 + b);
-            mbar_arrive(bar(D1_EMPTY + d));  // the accumulator buffer may be overwritten
-          }
-          if (kDots) {
-            if (row_ok) {
-              int32_t* o = p.dots + ((size_t)out_row * p.N + n0 + half * 64 + 32 * h) * nb + 8 * s + b;
+          for (int h = 0; h < 2; ++h) {  // 32 columns at a time: the block loop's working set stays inside the register budget
+            unsigned long long v[16];
+            tc_ld32_pairs(t_lane + (uint32_t)(d * BN + 32 * h), v);
+            if (h == 1) {
+              tc_fence_before();
+              mbar_arrive(bar(MP::D1_EMPTY + d));  // the accumulator buffer may be overwritten
+            }
+            if (kDots) {
+              if (row_ok) {
+                int32_t* o = p.dots + ((size_t)out_row * p.N + n0 + half * 64 + 32 * h) * nb + 8 * s + b;
 #pragma unroll
-              for (int c = 0; c < 16; ++c) {
-                o[(size_t)(2 * c) * nb] = __float2int_rn(lo_f(v[c]));
-                o[(size_t)(2 * c + 1) * nb] = __float2int_rn(hi_f(v[c]));
+                for (int c = 0; c < 16; ++c)
+                  if (n0 + half * 64 + 32 * h + 2 * c < p.N) {  // (N is a multiple of 16: pairs are whole)
+                    o[(size_t)(2 * c) * nb] = __float2int_rn(lo_f(v[c]));
+                    o[(size_t)(2 * c + 1) * nb] = __float2int_rn(hi_f(v[c]));
+                  }
+              }
+            } else if (!F::kColScale) {
+              if (b == 0) {
+#pragma unroll
+                for (int c = 0; c < 16; ++c) tq2[16 * h + c] = fmul2(a2, v[c]);
+              } else {
+#pragma unroll
+                for (int c = 0; c < 16; ++c) ffma2(tq2[16 * h + c], a2, v[c]);
+              }
+            } else {
+              const ulonglong2* d8 = reinterpret_cast<const ulonglong2*>(smem + MP::OFF_SCL + (sbc & 3) * 4096 + b * 512 + half * 256 + h * 128);
+#pragma unroll
+              for (int c4 = 0; c4 < 8; ++c4) {
+                const ulonglong2 dd = d8[c4];  // four column scales
+                ffma2(res2[16 * h + 2 * c4], fmul2(a2, dd.x), v[2 * c4]);
+                ffma2(res2[16 * h + 2 * c4 + 1], fmul2(a2, dd.y), v[2 * c4 + 1]);
               }
             }
-          } else if (QT == IZB_Q4_K) {
-            if (b == 0) {
+          }
+          if (++d == ND1) { d = 0; pd ^= 1; }
+        }
+        if (!ok) break;
+        if (!kDots) {  // the superblock's scales are read: its ring slot may be refilled
+          mbar_arrive(bar(MP::ASC_EMPTY + sq));
+          if (++sq == NASC) { sq = 0; pq ^= 1; }
+        }
+        if (!kDots && !F::kColScale) {  // res += d * tq
+          const ulonglong2* dv = reinterpret_cast<const ulonglong2*>(smem + MP::OFF_SCL + (sbc & 3) * 512 + half * 256);
 #pragma unroll
-              for (int c = 0; c < 16; ++c) tq2[16 * h + c] = fmul2(a2, v[c]);
-            } else {
-#pragma unroll
-              for (int c = 0; c < 16; ++c) ffma2(tq2[16 * h + c], a2, v[c]);
-            }
-          } else {
-            const ulonglong2* d8 = reinterpret_cast<const ulonglong2*>(smem + OFF_D8 + (sbc & 3) * 4096 + b * 512 + half * 256 + h * 128);
-#pragma unroll
-            for (int c4 = 0; c4 < 8; ++c4) {
-              const ulonglong2 dd = d8[c4];  // four column scales
-              ffma2(res2[16 * h + 2 * c4], fmul2(a2, dd.x), v[2 * c4]);
-              ffma2(res2[16 * h + 2 * c4 + 1], fmul2(a2, dd.y), v[2 * c4 + 1]);
-            }
+          for (int c4 = 0; c4 < 16; ++c4) {
+            const ulonglong2 dd = dv[c4];
+            ffma2(res2[2 * c4], dd.x, tq2[2 * c4]);
+            ffma2(res2[2 * c4 + 1], dd.y, tq2[2 * c4 + 1]);
           }
         }
-        if (warp == 8) TRACE(6, sbc * 8 + b);
-        if (++d == ND1) { d = 0; pd ^= 1; }
       }
-      if (!ok) break;
-      if (!kDots) {  // the superblock's scales are read: its ring slot may be refilled
-        mbar_arrive(bar(ASC_EMPTY + sq));
-        if (++sq == NASC) { sq = 0; pq ^= 1; }
-      }
-      if (kMins) {  // res += d * tq
-        const ulonglong2* dv = reinterpret_cast<const ulonglong2*>(smem + OFF_DM + (sbc & 3) * 512 + half * 256);
+      if (kMins && ok) {  // the min term of the whole K range (already negative)
+        ok = mbar_wait(bar(MP::D2_FULL), n_item & 1, abort_flag, p.err, p.spin_limit, E_EPI);
+        if (ok) {
+          tc_fence_after();
+          unsigned long long v[32];
+          tc_ld64_pairs(t_lane + (uint32_t)(ND1 * BN), v);
+          tc_fence_before();
+          mbar_arrive(bar(MP::D2_EMPTY));  // the next item's min term may start
+          const unsigned long long one2 = pack2(1.0f);
 #pragma unroll
-        for (int c4 = 0; c4 < 16; ++c4) {
-          const ulonglong2 dd = dv[c4];
-          ffma2(res2[2 * c4], dd.x, tq2[2 * c4]);
-          ffma2(res2[2 * c4 + 1], dd.y, tq2[2 * c4 + 1]);
+          for (int c = 0; c < 32; ++c) ffma2(res2[c], one2, v[c]);
         }
       }
-    }
-    if (kMins && ok) {  // the min term of the whole row of K (already negative)
-      ok = mbar_wait(bar(D2_FULL), it & 1, abort_flag, p.err, p.spin_limit, E_EPI);
-      if (ok) {
-        tc_fence_after();
-        unsigned long long v[32];
-        tc_ld64_pairs(t_lane + (uint32_t)(ND1 * BN), v);
-        tc_fence_before();
-        mbar_arrive(bar(D2_EMPTY));  // the next tile's min term may start
-        const unsigned long long one2 = pack2(1.0f);
+      if (!ok || kDots || !row_ok || *abort_flag) continue;
+      const int ncol = min(64, p.N - n0 - half * 64);  // valid columns of this thread (a multiple of 16; <= 0: none)
+      if (ncol <= 0) continue;
+      if (p.acc == 3 && p.n_split == 1) {
+        // Gate and up projections in one weight whose rows alternate in groups of 32 (izb_weight_create_gateup): this
+        // thread's 64 columns are 32 gate outputs followed by the 32 up outputs of the same FFN rows, so the SwiGLU product
+        // up * silu(gate) (zero/kernels/gemm.cl:562-565) is formed in registers and only the F-wide result is stored.
+        float* cp = p.C + (size_t)out_row * p.ldc + p.c_off + (n0 >> 1) + half * 32;
+        const bool wide = ((reinterpret_cast<uintptr_t>(cp) | ((size_t)p.ldc * 4)) & 31) == 0;
 #pragma unroll
-        for (int c = 0; c < 32; ++c) ffma2(res2[c], one2, v[c]);
-      }
-    }
-    if (ok && !kDots && row_ok && !*abort_flag && p.acc == 3) {
-      // Gate and up projections in one weight whose rows alternate in groups of 32 (izb_weight_create_gateup): this
-      // thread's 64 columns are 32 gate outputs followed by the 32 up outputs of the same FFN rows, so the SwiGLU product
-      // up * silu(gate) (zero/kernels/gemm.cl:562-565) is formed in registers and only the F-wide result is stored.
-      float* cp = p.C + (size_t)out_row * p.ldc + p.c_off + (n0 >> 1) + half * 32;
-      const bool wide = ((reinterpret_cast<uintptr_t>(cp) | ((size_t)p.ldc * 4)) & 31) == 0;
+        for (int j = 0; j < 4; ++j) {
+          unsigned long long o[4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        unsigned long long o[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const unsigned long long g2 = res2[4 * j + i], u2 = res2[16 + 4 * j + i];
-          o[i] = pack_pair(swiglu_mul(lo_f(g2), lo_f(u2)), swiglu_mul(hi_f(g2), hi_f(u2)));
+          for (int i = 0; i < 4; ++i) {
+            const unsigned long long g2 = res2[4 * j + i], u2 = res2[16 + 4 * j + i];
+            o[i] = pack_pair(swiglu_mul(lo_f(g2), lo_f(u2)), swiglu_mul(hi_f(g2), hi_f(u2)));
+          }
+          if (wide) {
+            asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(cp + 8 * j), "l"(o[0]), "l"(o[1]), "l"(o[2]), "l"(o[3]) : "memory");
+          } else {
+            reinterpret_cast<float4*>(cp + 8 * j)[0] = make_float4(lo_f(o[0]), hi_f(o[0]), lo_f(o[1]), hi_f(o[1]));
+            reinterpret_cast<float4*>(cp + 8 * j)[1] = make_float4(lo_f(o[2]), hi_f(o[2]), lo_f(o[3]), hi_f(o[3]));
+          }
         }
-        if (wide) {
-          asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(cp + 8 * j), "l"(o[0]), "l"(o[1]), "l"(o[2]), "l"(o[3]) : "memory");
-        } else {
-          reinterpret_cast<float4*>(cp + 8 * j)[0] = make_float4(lo_f(o[0]), hi_f(o[0]), lo_f(o[1]), hi_f(o[1]));
-          reinterpret_cast<float4*>(cp + 8 * j)[1] = make_float4(lo_f(o[2]), hi_f(o[2]), lo_f(o[3]), hi_f(o[3]));
-        }
+        continue;
       }
-    } else if (ok && !kDots && row_ok && !*abort_flag) {
-      float* cp = p.C + (size_t)out_row * p.ldc + p.c_off + n0 + half * 64;
+      // a part of the K range goes to the partial sums as it is (split_reduce_kernel applies the store mode)
+      float* cp = p.n_split > 1 ? p.part + ((size_t)it.ks * p.M + out_row) * p.N + n0 + half * 64
+                                : p.C + (size_t)out_row * p.ldc + p.c_off + n0 + half * 64;
+      const size_t ld = p.n_split > 1 ? (size_t)p.N : (size_t)p.ldc;
+      const int acc = p.n_split > 1 ? 0 : p.acc;
       const float rs = p.rowscale ? p.rowscale[out_row] : 1.0f;
       // plain store (with or without the row factor), 32-byte aligned rows: eight stores of one full 32-byte sector each
       // per thread
-      if (p.acc == 0 && ((reinterpret_cast<uintptr_t>(cp) | ((size_t)p.ldc * 4)) & 31) == 0) {
+      if (acc == 0 && ncol == 64 && ((reinterpret_cast<uintptr_t>(cp) | (ld * 4)) & 31) == 0) {
         if (p.rowscale) {
           const unsigned long long rs2 = pack2(rs);
 #pragma unroll
@@ -893,25 +1016,26 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
           asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(cp + 8 * c8), "l"(res2[4 * c8]), "l"(res2[4 * c8 + 1]),
                        "l"(res2[4 * c8 + 2]), "l"(res2[4 * c8 + 3])
                        : "memory");
-      } else
+      } else {
 #pragma unroll
-      for (int c4 = 0; c4 < 16; ++c4) {
-        float4 v = make_float4(lo_f(res2[2 * c4]), hi_f(res2[2 * c4]), lo_f(res2[2 * c4 + 1]), hi_f(res2[2 * c4 + 1]));
-        if (p.rowscale) { v.x = __fmul_rn(rs, v.x); v.y = __fmul_rn(rs, v.y); v.z = __fmul_rn(rs, v.z); v.w = __fmul_rn(rs, v.w); }
-        float4* dst = reinterpret_cast<float4*>(cp) + c4;
-        if (p.acc == 1) {
-          const float4 o = *dst;
-          v.x = __fadd_rn(v.x, o.x); v.y = __fadd_rn(v.y, o.y); v.z = __fadd_rn(v.z, o.z); v.w = __fadd_rn(v.w, o.w);
-        } else if (p.acc == 2) {  // C holds the gate projection: C = v * silu(C)   (zero/kernels/gemm.cl:562-565)
-          const float4 o = *dst;
-          v.x = swiglu_mul(o.x, v.x);
-          v.y = swiglu_mul(o.y, v.y);
-          v.z = swiglu_mul(o.z, v.z);
-          v.w = swiglu_mul(o.w, v.w);
+        for (int c4 = 0; c4 < 16; ++c4) {
+          if (4 * c4 >= ncol) break;
+          float4 x = make_float4(lo_f(res2[2 * c4]), hi_f(res2[2 * c4]), lo_f(res2[2 * c4 + 1]), hi_f(res2[2 * c4 + 1]));
+          if (p.rowscale) { x.x = __fmul_rn(rs, x.x); x.y = __fmul_rn(rs, x.y); x.z = __fmul_rn(rs, x.z); x.w = __fmul_rn(rs, x.w); }
+          float4* dst = reinterpret_cast<float4*>(cp) + c4;
+          if (acc == 1) {
+            const float4 o = *dst;
+            x.x = __fadd_rn(x.x, o.x); x.y = __fadd_rn(x.y, o.y); x.z = __fadd_rn(x.z, o.z); x.w = __fadd_rn(x.w, o.w);
+          } else if (acc == 2) {  // C holds the gate projection: C = x * silu(C)   (zero/kernels/gemm.cl:562-565)
+            const float4 o = *dst;
+            x.x = swiglu_mul(o.x, x.x);
+            x.y = swiglu_mul(o.y, x.y);
+            x.z = swiglu_mul(o.z, x.z);
+            x.w = swiglu_mul(o.w, x.w);
+          }
+          *dst = x;
         }
-        *dst = v;
       }
-    }
     }
   }
   // ---- teardown
@@ -919,6 +1043,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
   __syncthreads();
   if (*abort_flag) {
     // a wait gave up: let copies and MMAs still in flight land before shared memory and TMEM are released
+    if (p.n_split > 1 && threadIdx.x == 0) atomicOr(p.part_bad, 1u);
     for (int i = 0; i < 64; ++i) __nanosleep(20000);
     __syncthreads();
   }
@@ -926,6 +1051,42 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem_base) : "memory");
   }
+}
+
+// ---------------------------------------------------------------------------------------------- partial sums of a cut K range
+// out (store mode `acc`) = part 0 + part 1 + ... in order.  One thread per four output columns.
+__global__ void __launch_bounds__(256) split_reduce_kernel(const float* __restrict__ part, int n_split, int M, int N, float* __restrict__ C, int ldc, int c_off,
+                                                           int acc, const uint32_t* __restrict__ part_bad) {
+  pdl_launch_next();
+  pdl_wait();
+  if (*part_bad) return;
+  const int n_out = acc == 3 ? N / 2 : N, c = (blockIdx.x * 256 + threadIdx.x) * 4, m = blockIdx.y;
+  if (c >= n_out) return;
+  auto sum = [&](int col) -> float4 {
+    const float* src = part + (size_t)m * N + col;
+    float4 v = *reinterpret_cast<const float4*>(src);
+    for (int k = 1; k < n_split; ++k) {
+      const float4 o = *reinterpret_cast<const float4*>(src + (size_t)k * M * N);
+      v.x = __fadd_rn(v.x, o.x); v.y = __fadd_rn(v.y, o.y); v.z = __fadd_rn(v.z, o.z); v.w = __fadd_rn(v.w, o.w);
+    }
+    return v;
+  };
+  float4* dst = reinterpret_cast<float4*>(C + (size_t)m * ldc + c_off + c);
+  float4 v;
+  if (acc == 3) {  // (groups of 32 gate and 32 up columns, see the GEMM's store mode 3)
+    const float4 g = sum(64 * (c >> 5) + (c & 31)), u = sum(64 * (c >> 5) + 32 + (c & 31));
+    v = make_float4(swiglu_mul(g.x, u.x), swiglu_mul(g.y, u.y), swiglu_mul(g.z, u.z), swiglu_mul(g.w, u.w));
+  } else {
+    v = sum(c);
+    if (acc == 1) {
+      const float4 o = *dst;
+      v.x = __fadd_rn(v.x, o.x); v.y = __fadd_rn(v.y, o.y); v.z = __fadd_rn(v.z, o.z); v.w = __fadd_rn(v.w, o.w);
+    } else if (acc == 2) {
+      const float4 o = *dst;
+      v = make_float4(swiglu_mul(o.x, v.x), swiglu_mul(o.y, v.y), swiglu_mul(o.z, v.z), swiglu_mul(o.w, v.w));
+    }
+  }
+  *dst = v;
 }
 
 // ---------------------------------------------------------------------------------------------- host side
@@ -947,27 +1108,47 @@ EncodeTiledFn get_encode() {
 // producer leaves out, for the NEXT launch only.
 std::atomic<uint32_t> g_test_spin{0};
 std::atomic<int> g_test_skip{-1};
-std::atomic<unsigned long long*> g_test_trace{nullptr};
 
-template <int QT, bool kDots>
+template <class F, bool kDots>
 int launch_tc(const izb_weight* w, TcParams& p, dim3 grid, cudaStream_t st) {
-  constexpr int SMEM_BYTES = Map<QT>::SMEM_BYTES;
-  IZB_SMEM_OPTIN((gemm_tc_kernel<QT, kDots>), SMEM_BYTES, w->device);
+  constexpr int SMEM_BYTES = Map<F>::SMEM_BYTES;
+  IZB_SMEM_OPTIN((gemm_tc_kernel<F, kDots>), SMEM_BYTES, w->device);
   const uint32_t spin = g_test_spin.exchange(0);
   p.spin_limit = spin ? spin : kSpinLimit;
   p.skip_stage = g_test_skip.exchange(-1);
-  p.trace = g_test_trace.load();
   CUtensorMap tm;
   memcpy(&tm, w->tmap_raw, sizeof tm);
-  IZB_LAUNCH("gemm_tc", st, gemm_tc_kernel<QT, kDots><<<grid, kThreads, SMEM_BYTES, st>>>(tm, p));
+  IZB_LAUNCH("gemm_tc", st, izb_launch_pdl(gemm_tc_kernel<F, kDots>, grid, kThreads, SMEM_BYTES, st, tm, p));
   return IZB_OK;
 }
+int launch_tc_of(const izb_weight* w, TcParams& p, dim3 grid, cudaStream_t st) {
+  if (w->type == IZB_Q4_K) return p.dots ? launch_tc<FQ4K, true>(w, p, grid, st) : launch_tc<FQ4K, false>(w, p, grid, st);
+  if (w->type == IZB_Q8_0) return p.dots ? launch_tc<FQ80, true>(w, p, grid, st) : launch_tc<FQ80, false>(w, p, grid, st);
+  if (p.dots) return 1;
+  return w->packed6 ? launch_tc<FQ6K, false>(w, p, grid, st) : w->has_min ? launch_tc<FQ5K, false>(w, p, grid, st) : launch_tc<FIQ4, false>(w, p, grid, st);
+}
 
-// persistent grid: one CTA per SM (shared memory allows no more), fewer when there are fewer tiles
+// operand stages per superblock: weights with mins carry the min term as a fifth one
+int tc_sps(const izb_weight* w, bool dots) { return (w->type == IZB_Q4_K || (w->type == IZB_K16 && w->has_min)) && !dots ? 5 : 4; }
+// does the kernel take this weight at all
+bool tc_takes(const izb_weight* w) { return w->has_tmap && w->N % 16 == 0 && w->K % 256 == 0; }
+
+// persistent grid: one CTA per SM (shared memory allows no more), fewer when there are fewer items
 int tc_grid(int device, int n_work) {
   const int sms = izb_sm_budget(device);
   return n_work < sms ? (n_work > 0 ? n_work : 1) : sms;
 }
+
+// Parts the K range of every output tile is cut into, when the tiles alone would leave more than half the SMs idle: as many
+// as fill them once, each at least one superblock.  The parts' sums are at most one 64 KB tile per SM.
+int tc_split(int device, int n_items, int nsb) {
+  const int s = izb_sm_budget(device) / (n_items > 0 ? n_items : 1);
+  return s < 2 ? 1 : s < nsb ? s : nsb;
+}
+constexpr size_t kSplitBytes = (size_t)BM * BN * 4;  // per SM; the flag of a failed part follows them
+
+size_t split_area(int device) { return kSplitBytes * izb_sm_count(device) + 256; }
+uint32_t* split_flag(float* split_ws, int device) { return split_ws ? (uint32_t*)((unsigned char*)split_ws + kSplitBytes * izb_sm_count(device)) : nullptr; }
 
 // scratch of one call: the operand images (sps stage images of 16 KB per superblock and tile) and the gathered scales
 void tc_scratch_bytes(int n_tiles, int K, int sps, size_t* img_bytes, size_t* asc_bytes) {
@@ -975,27 +1156,25 @@ void tc_scratch_bytes(int n_tiles, int K, int sps, size_t* img_bytes, size_t* as
   *asc_bytes = (size_t)n_tiles * (K / 32) * BM * 4;
 }
 
-// the activation pre-pass + the GEMM on scratch the caller owns (img_bytes + asc_bytes of tc_scratch_bytes)
+// the activation pre-pass + the GEMM on scratch the caller owns (img_bytes + asc_bytes of tc_scratch_bytes, then, where the
+// call may be cut along K, `split_ws`)
 int run_tc_on(const izb_weight* w, int mat, const int8_t* aq, const float* asc, int lda, int rows_total, const int32_t* tiles,
               int n_tiles_grid, const int32_t* rowmap, const float* rowscale, int M_store, float* C, int ldc, int c_off, int acc,
-              int32_t* dots, void* ws, uint32_t* err, cudaStream_t st, bool reuse_images) {
-  const int K = w->K;
-  const int sps = (w->type == IZB_Q4_K && !dots) ? 5 : 4;
+              int32_t* dots, void* ws, float* split_ws, uint32_t* err, cudaStream_t st, bool reuse_images) {
+  const int K = w->K, sps = tc_sps(w, dots != nullptr);
   size_t img_bytes, asc_bytes;
   tc_scratch_bytes(n_tiles_grid, K, sps, &img_bytes, &asc_bytes);
   uint16_t* aimg = (uint16_t*)ws;
   float* ascimg = (float*)((unsigned char*)ws + img_bytes);
-  dim3 pg((BM * (K / 8) + 255) / 256, n_tiles_grid);
-  if (reuse_images) {
-  } else if (w->type == IZB_Q4_K)
-    IZB_LAUNCH("act_prepare", st, act_prepare_kernel<IZB_Q4_K><<<pg, 256, 0, st>>>(aq, asc, lda, K, rows_total, tiles, rowmap, aimg, ascimg, sps));
-  else
-    IZB_LAUNCH("act_prepare", st, act_prepare_kernel<IZB_Q8_0><<<pg, 256, 0, st>>>(aq, asc, lda, K, rows_total, tiles, rowmap, aimg, ascimg, 4));
+  if (!reuse_images) {
+    dim3 pg((BM * (K / 8) + 255) / 256, n_tiles_grid);
+    auto kernel = w->type == IZB_Q4_K ? act_prepare_kernel<true> : act_prepare_kernel<false>;
+    IZB_LAUNCH("act_prepare", st, izb_launch_pdl(kernel, pg, 256, 0, st, aq, asc, lda, K, rows_total, tiles, rowmap, aimg, ascimg, sps, split_flag(split_ws, w->device)));
+  }
   TcParams p;
   p.aimg = aimg;
   p.ascimg = ascimg;
   p.tiles = tiles;
-  p.rowmap = rowmap;
   p.rowscale = rowscale;
   p.M = M_store;
   p.N = w->N;
@@ -1008,9 +1187,17 @@ int run_tc_on(const izb_weight* w, int mat, const int8_t* aq, const float* asc, 
   p.dots = dots;
   p.err = err;
   p.n_mtiles = n_tiles_grid;
-  dim3 grid(tc_grid(w->device, w->N / BN * n_tiles_grid));
-  if (w->type == IZB_Q4_K) return dots ? launch_tc<IZB_Q4_K, true>(w, p, grid, st) : launch_tc<IZB_Q4_K, false>(w, p, grid, st);
-  return dots ? launch_tc<IZB_Q8_0, true>(w, p, grid, st) : launch_tc<IZB_Q8_0, false>(w, p, grid, st);
+  const int n_items = (w->N + BN - 1) / BN * n_tiles_grid;
+  p.n_split = split_ws && !tiles && !dots ? tc_split(w->device, n_items, K / 256) : 1;
+  p.part = split_ws;
+  p.part_bad = split_flag(split_ws, w->device);
+  dim3 grid(tc_grid(w->device, n_items * p.n_split));
+  if (int rc = launch_tc_of(w, p, grid, st)) return rc;
+  if (p.n_split > 1) {
+    dim3 rg(((acc == 3 ? w->N / 2 : w->N) / 4 + 255) / 256, M_store);
+    IZB_LAUNCH("split_reduce", st, izb_launch_pdl(split_reduce_kernel, rg, 256, 0, st, split_ws, p.n_split, M_store, w->N, C, ldc, c_off, acc, p.part_bad));
+  }
+  return IZB_OK;
 }
 
 // the activation pre-pass + the GEMM for one tile set
@@ -1019,32 +1206,26 @@ int run_tc(const izb_weight* w, int mat, const int8_t* aq, const float* asc, int
            int32_t* dots, int ws_slot, cudaStream_t st, bool reuse_images = false) {
   // reuse_images: the call before this one, on the same stream and arena, prepared the same activation rows for a weight
   // of the same type and K (the up projection after the gate projection): its operand images are still there
-  if (!w->has_tmap) return 1;
-  if (w->N % BN || w->K % 256) return 1;
-  const int sps = (w->type == IZB_Q4_K && !dots) ? 5 : 4;
+  if (!tc_takes(w)) return 1;
   size_t img_bytes, asc_bytes;
-  tc_scratch_bytes(n_tiles_grid, w->K, sps, &img_bytes, &asc_bytes);
+  tc_scratch_bytes(n_tiles_grid, w->K, tc_sps(w, dots != nullptr), &img_bytes, &asc_bytes);
+  const size_t split_bytes = tiles || dots ? 0 : split_area(w->device);
   void* ws = nullptr;
-  if (int rc = izb_workspace(w->device, ws_slot, img_bytes + asc_bytes, &ws)) return rc;
+  if (int rc = izb_workspace(w->device, ws_slot, img_bytes + asc_bytes + split_bytes, &ws)) return rc;
   uint32_t* err = izb_device_error_word(w->device);
   if (!err) IZB_FAIL(IZB_ERR_NOMEM, "gemm: no device error word");
-  return run_tc_on(w, mat, aq, asc, lda, rows_total, tiles, n_tiles_grid, rowmap, rowscale, M_store, C, ldc, c_off, acc, dots, ws, err,
+  float* split_ws = split_bytes ? (float*)((unsigned char*)ws + img_bytes + asc_bytes) : nullptr;
+  return run_tc_on(w, mat, aq, asc, lda, rows_total, tiles, n_tiles_grid, rowmap, rowscale, M_store, C, ldc, c_off, acc, dots, ws, split_ws, err,
                    st, reuse_images);
 }
 
 }  // namespace
 
 // scratch bytes of a dense tensor-core GEMM over `rows` activation rows (izb_reserve sizes the arenas with it)
-size_t izb_gemm_tc_scratch_bytes(int type, int rows, int K) {
+size_t izb_gemm_tc_scratch_bytes(int device, int type, int rows, int K) {
   size_t img_bytes, asc_bytes;
   tc_scratch_bytes((rows + BM - 1) / BM, K, type == IZB_Q4_K ? 5 : 4, &img_bytes, &asc_bytes);
-  return img_bytes + asc_bytes;
-}
-
-// diagnostics builds (IZB_TC_TRACE): where CTA 0 of the following launches writes its clock stamps
-extern "C" int izb_debug_set_trace(unsigned long long* d_trace) {
-  g_test_trace.store(d_trace);
-  return IZB_OK;
+  return img_bytes + asc_bytes + split_area(device);
 }
 
 extern "C" int izb_debug_wait_test(uint32_t spin_limit, int skip_stage) {
@@ -1082,23 +1263,22 @@ int izb_gemm_tc_launch(const izb_weight* w, int mat, const int8_t* aq, const flo
 int izb_gemm_tc_quant_launch(const izb_weight* w, int mat, const float* x, int ldx, int M, int Mp, int8_t* aq, float* asc, float* C,
                              int ldc, int c_off, int acc, cudaStream_t st) {
   const int n_tiles = (Mp + BM - 1) / BM;  // (the GEMM runs over the padded rows, as izb_matmul's does)
-  if (n_tiles > 65535 || !w->has_tmap || w->N % BN || w->K % 256) return 1;
-  const int K = w->K, sps = w->type == IZB_Q4_K ? 5 : 4;
+  if (n_tiles > 65535 || !tc_takes(w)) return 1;
+  const int K = w->K, sps = tc_sps(w, false);
   size_t img_bytes, asc_bytes;
   tc_scratch_bytes(n_tiles, K, sps, &img_bytes, &asc_bytes);
   void* ws = nullptr;
-  if (int rc = izb_workspace(w->device, kWsGemm, img_bytes + asc_bytes, &ws)) return rc;
+  if (int rc = izb_workspace(w->device, kWsGemm, img_bytes + asc_bytes + split_area(w->device), &ws)) return rc;
   uint32_t* err = izb_device_error_word(w->device);
   if (!err) IZB_FAIL(IZB_ERR_NOMEM, "gemm: no device error word");
   uint16_t* aimg = (uint16_t*)ws;
   float* ascimg = (float*)((unsigned char*)ws + img_bytes);
+  float* split_ws = (float*)((unsigned char*)ws + img_bytes + asc_bytes);
   const int rows_img = n_tiles * BM > Mp ? n_tiles * BM : Mp;  // every row of every tile is written (rows past M as zeros)
   dim3 grid(K / 256, (rows_img + 31) / 32);
-  if (w->type == IZB_Q4_K)
-    IZB_LAUNCH("quant_prepare", st, quant_prepare_kernel<IZB_Q4_K><<<grid, 256, 0, st>>>(x, ldx, M, Mp, K, aq, asc, aimg, ascimg, sps, n_tiles));
-  else
-    IZB_LAUNCH("quant_prepare", st, quant_prepare_kernel<IZB_Q8_0><<<grid, 256, 0, st>>>(x, ldx, M, Mp, K, aq, asc, aimg, ascimg, sps, n_tiles));
-  return run_tc_on(w, mat, aq, asc, Mp, Mp, nullptr, n_tiles, nullptr, nullptr, Mp, C, ldc, c_off, acc, nullptr, ws, err, st, true);
+  auto kernel = w->type == IZB_Q4_K ? quant_prepare_kernel<true> : quant_prepare_kernel<false>;
+  IZB_LAUNCH("quant_prepare", st, izb_launch_pdl(kernel, grid, 256, 0, st, x, ldx, M, Mp, K, aq, asc, aimg, ascimg, sps, n_tiles, split_flag(split_ws, w->device)));
+  return run_tc_on(w, mat, aq, asc, Mp, Mp, nullptr, n_tiles, nullptr, nullptr, Mp, C, ldc, c_off, acc, nullptr, ws, split_ws, err, st, true);
 }
 
 // MoE on the tensor cores: the slots of each expert are tiles of up to 128 rows (izb_moe_sort with TM = 128); gate then up
@@ -1312,7 +1492,7 @@ extern "C" int izb_gemm_noalloc(const izb_weight* w, int mat, const int8_t* d_aq
   // must start at zero.
   uint32_t* status = d_status ? d_status : dev->status;
   IZB_CUDA(cudaMemsetAsync(status, 0, 4, st));
-  return run_tc_on(w, mat, d_aq, d_asc, Mp, Mp, nullptr, n_tiles, nullptr, nullptr, M, d_C, ldc, c_off, acc, nullptr, dev->scratch, status,
+  return run_tc_on(w, mat, d_aq, d_asc, Mp, Mp, nullptr, n_tiles, nullptr, nullptr, M, d_C, ldc, c_off, acc, nullptr, dev->scratch, nullptr, status,
                    st, false);
 }
 

@@ -1,0 +1,52 @@
+"""The tcgen05 GEMM on every weight form it takes (one and two fp16 terms per weight, with and without mins), on columns that do
+not fill its tiles and on calls whose K range is cut into parts, against the CUDA-core kernel (itself checked against the oracle)."""
+import numpy as np
+import pytest
+
+from arcinferzero_b200 import synth as S
+
+pytestmark = pytest.mark.gpu
+
+
+def extremes(qt, rows):
+    """Largest scales and quants of either sign in some rows: products up to 4096 must stay exact."""
+    v = rows.copy()
+    if qt == 14:
+        v = v.reshape(v.shape[0], -1, 210)
+        v[0, :, 0:192], v[0, :, 192:208] = 0xFF, 0x80   # quant 31, scale -128
+        v[1, :, 0:192], v[1, :, 192:208] = 0x00, 0x80   # quant -32, scale -128: 4096
+        v[2, :, 0:192], v[2, :, 192:208] = 0x00, 0x7F
+    elif qt == 23:
+        v = v.reshape(v.shape[0], -1, 136)
+        v[0, :, 2:8], v[0, :, 8:] = 0x00, 0x00          # scale -32, codebook -127
+        v[1, :, 2:8], v[1, :, 8:] = 0xFF, 0xFF          # scale 31, codebook 113
+    elif qt in (12, 13):
+        v = v.reshape(v.shape[0], -1, 144 if qt == 12 else 176)
+        v[0, :, 4:] = 0xFF
+    return v.reshape(rows.shape)
+
+
+# (16, 16): the smallest call; 144, 272: a part of the last column tile; 40 x 128 x 4096 and 130 x 144 x 2304: K cut into parts;
+# 300 x 2432 x 512: more tiles than half the SMs, not cut
+@pytest.mark.parametrize("qt", [12, 8, 2, 13, 14, 23])
+@pytest.mark.parametrize("M,N,K", [(16, 16, 256), (130, 144, 2304), (40, 128, 4096), (129, 272, 768), (300, 2432, 512)])
+def test_tensor_core_gemm_equals_core_gemm(izb, qt, M, N, K):
+    import torch
+    W = izb.Weight(qt, extremes(qt, S.make_weight(qt, N, K, N + K + qt)), N, K)
+    Mp = izb.pad_rows(M)
+    x = torch.from_numpy(S.make_act(M, K, M + K)).cuda()
+    x[0] = 1.0  # every int8 = 127
+    aq, asc, _ = izb.quantize_act(x, Mp=Mp)
+    for acc in (0, 1, 2):
+        base = torch.from_numpy(np.random.default_rng(acc).standard_normal((Mp, N + 8)).astype(np.float32)).cuda()
+        a, b = base.clone(), base.clone()
+        izb.gemm(W, aq, asc, M=M, out=a, c_off=4, acc=acc)
+        izb.gemm(W, aq, asc, M=M, out=b, c_off=4, acc=acc, impl=izb.GEMM_CORE)
+        ra, rb = a[:M, 4:N + 4].double(), b[:M, 4:N + 4].double()
+        assert float((ra - rb).abs().max() / rb.abs().max()) < 1e-5, acc
+        assert torch.equal(a[:, :4], base[:, :4]) and torch.equal(a[:, N + 4:], base[:, N + 4:]) and torch.equal(a[M:], base[M:])
+    got, _, _ = izb.quant_matmul(W, x, M)
+    want = izb.gemm(W, aq, asc)
+    assert torch.equal(got[:M], want[:M])
+    assert izb.device_status(0) == 0
+    W.close()
