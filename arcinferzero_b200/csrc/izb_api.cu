@@ -18,6 +18,7 @@ int izb_gemm_core_launch(const izb_weight* w, const uint8_t* raw, const int8_t* 
 int izb_gemm_tc_launch(const izb_weight* w, int mat, const int8_t* aq, const float* asc, int M, int Mp, float* C, int ldc,
                        int c_off, int acc, int32_t* dots, cudaStream_t st);
 int izb_make_raw_tensor_map(izb_weight* w);
+int izb_make_rows_tensor_map(izb_weight* w);
 int izb_gemm_k16_launch(const izb_weight* w, const uint8_t* raw, const int8_t* aq, const float* asc, int M, int Mp, float* C, int ldc,
                         int c_off, int acc, int32_t* dots, cudaStream_t st);
 
@@ -404,6 +405,7 @@ extern "C" int izb_weight_create_slice(int type, const void* h_rows, int n_mats,
     IZB_FAIL(IZB_ERR_CUDA, "weight_create: upload failed: %s", cudaGetErrorString(e));
   }
   w->has_tmap = izb_make_raw_tensor_map(w) == IZB_OK;
+  w->has_tmap16 = (w->type != IZB_K16 || w->packed6) && izb_make_rows_tensor_map(w) == IZB_OK;
   *out = w;
   return IZB_OK;
 }

@@ -34,6 +34,8 @@ struct izb_weight {
   uint8_t* raw = nullptr;
   alignas(64) unsigned char tmap_raw[128];  // CUtensorMap over raw: [n_mats*N rows][row_bytes/4 uint32]
   bool has_tmap = false;
+  alignas(64) unsigned char tmap16_raw[128];  // the same view in chunks of 16 rows x one superblock for csrc/izb_rows.cu
+  bool has_tmap16 = false;
 };
 
 static constexpr size_t kRawSlack = 1024;  // zero bytes after the last row (zero/engine_load.h:79-84)

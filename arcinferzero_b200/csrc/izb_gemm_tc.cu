@@ -1234,22 +1234,26 @@ extern "C" int izb_debug_wait_test(uint32_t spin_limit, int skip_stage) {
   return IZB_OK;
 }
 
-int izb_make_raw_tensor_map(izb_weight* w) {
+// Tensor map over the raw rows in boxes of `box_rows` rows x `box_bytes` bytes
+static int make_map(const izb_weight* w, int box_bytes, int box_rows, unsigned char* out) {
   EncodeTiledFn enc = get_encode();
   if (!enc) return IZB_ERR_CUDA;
   const cuuint64_t rows = (cuuint64_t)w->n_mats * w->N;
   if (rows < 1 || w->row_bytes % 16) return IZB_ERR_ALIGN;
   cuuint64_t dims[2] = {(cuuint64_t)(w->row_bytes / 4), rows};
   cuuint64_t strides[1] = {(cuuint64_t)w->row_bytes};
-  cuuint32_t box[2] = {(cuuint32_t)(w->sb_bytes / 4), (cuuint32_t)BN};
+  cuuint32_t box[2] = {(cuuint32_t)(box_bytes / 4), (cuuint32_t)box_rows};
   cuuint32_t estr[2] = {1, 1};
   CUtensorMap tm;
   const CUresult r = enc(&tm, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, w->raw, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                          CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return IZB_ERR_CUDA;
-  memcpy(w->tmap_raw, &tm, sizeof tm);
+  memcpy(out, &tm, sizeof tm);
   return IZB_OK;
 }
+int izb_make_raw_tensor_map(izb_weight* w) { return make_map(w, w->sb_bytes, BN, w->tmap_raw); }
+// chunks of the few-row kernel: a superblock; Q6_K 16 bytes more, for a row pitch its shared-memory reads want
+int izb_make_rows_tensor_map(izb_weight* w) { return make_map(w, w->packed6 ? w->sb_bytes + 16 : w->sb_bytes, 16, w->tmap16_raw); }
 
 int izb_gemm_tc_launch(const izb_weight* w, int mat, const int8_t* aq, const float* asc, int M, int Mp, float* C, int ldc, int c_off,
                        int acc, int32_t* dots, cudaStream_t st) {

@@ -18,6 +18,8 @@ int izb_gemv_k16_launch(const izb_weight* w, const uint8_t* raw, const int8_t* a
 int izb_gemv_stream_launch(const izb_weight* w, const uint8_t* raw, const int8_t* aq, const float* asc, int T, int Mp, float* C,
                            int ldc, int c_off, int acc, cudaStream_t st);
 
+int izb_rows_launch(const izb_weight* w, int mat, const int8_t* aq, const float* asc, int T, int Mp, float* C, int ldc, int c_off, int acc, cudaStream_t st);
+
 namespace {
 using namespace izb_gemvk;
 
@@ -67,6 +69,12 @@ int launch(const izb_weight* w, const uint8_t* raw, const int8_t* aq, const floa
                              : launch_qt<IZB_Q8_0, T>(w, raw, aq, asc, Mp, C, ldc, c_off, acc, st);
 }
 
+#include <stdlib.h>
+bool rows_first(const izb_weight* w, int T) {
+  static const int v = getenv("ROWS_MIN") ? atoi(getenv("ROWS_MIN")) : 2;
+  return T >= v && !(w->type == IZB_Q4_K && T <= 4 && w->K % 1024 == 0 && w->N >= 1024);
+}
+
 }  // namespace
 extern "C" int izb_gemv(const izb_weight* w, int mat, const int8_t* d_aq, const float* d_asc, int T, int Mp, float* d_C,
                         int ldc, int c_off, int acc, void* stream) {
@@ -80,6 +88,10 @@ extern "C" int izb_gemv(const izb_weight* w, int mat, const int8_t* d_aq, const 
   if (int rc = izb_require_device(w->device, "gemv")) return rc;
   const uint8_t* raw = w->raw + (size_t)mat * w->N * w->row_bytes;
   cudaStream_t st = (cudaStream_t)stream;
+  if (rows_first(w, T)) {
+    const int rc = izb_rows_launch(w, mat, d_aq, d_asc, T, Mp, d_C, ldc, c_off, acc, st);
+    if (rc <= 0) return rc;
+  }
   if (w->type == IZB_K16) return izb_gemv_k16_launch(w, raw, d_aq, d_asc, T, Mp, d_C, ldc, c_off, acc, st);
   {  // the streaming kernel takes every call whose staged activations fit in shared memory
     const int rc = izb_gemv_stream_launch(w, raw, d_aq, d_asc, T, Mp, d_C, ldc, c_off, acc, st);

@@ -289,6 +289,9 @@ extern "C" int izb_moe_sort(const int32_t* d_ids, const float* d_wts, const int3
   return izb_moe_sort_ex(d_ids, d_wts, d_counts, T, NE, NU, TM, 0, NE, d_offs, d_tiles, max_tiles, d_stok, d_swt, d_inv, stream);
 }
 
+int izb_moe_rows_launch(const izb_weight* wg, const izb_weight* wu, const int8_t* aq, const float* asc, int Mp, const int32_t* tiles, int max_tiles, const int32_t* stok,
+                        const float* swt, float* out, cudaStream_t st);
+
 int izb_moe_gateup_tiles(const izb_weight* wg, const izb_weight* wu, const int8_t* d_aq, const float* d_asc, int Mp,
                          const int32_t* d_tiles, int max_tiles, const int32_t* d_stok, float* d_h, cudaStream_t st) {
   const int F = wg->N, K = wg->K;
@@ -371,7 +374,10 @@ extern "C" int izb_moe_gateup(const izb_weight* wg, const izb_weight* wu, const 
   if (wg->type == IZB_K16) IZB_FAIL(IZB_ERR_TYPE, "moe_gateup: expert stacks of ggml type %d are not taken (Q8_0, Q4_K, Q4_0)", wg->ggml_type);
   if (wu->device != wg->device) IZB_FAIL(IZB_ERR_ARG, "moe_gateup: gate and up stacks live on different devices");
   if (int rc = izb_require_device(wg->device, "moe_gateup")) return rc;
-  if (TM >= 1 && TM <= 8) return izb_moe_gateup_tiles(wg, wu, d_aq, d_asc, Mp, d_tiles, max_tiles, d_stok, d_h, (cudaStream_t)stream);
+  if (TM >= 1 && TM <= 8) {
+    const int rc = izb_moe_rows_launch(wg, wu, d_aq, d_asc, Mp, d_tiles, max_tiles, d_stok, nullptr, d_h, (cudaStream_t)stream);
+    return rc <= 0 ? rc : izb_moe_gateup_tiles(wg, wu, d_aq, d_asc, Mp, d_tiles, max_tiles, d_stok, d_h, (cudaStream_t)stream);
+  }
   if (TM == 128) {
     const int rc = izb_moe_gateup_tc(wg, wu, d_aq, d_asc, Mp, d_tiles, max_tiles, d_stok, d_h, (cudaStream_t)stream);
     if (rc <= 0) return rc;
@@ -387,7 +393,10 @@ extern "C" int izb_moe_down(const izb_weight* wd, const int8_t* d_hq, const floa
   if (!izb_aligned(d_hq, 16)) IZB_FAIL(IZB_ERR_ALIGN, "moe_down: hq not 16-byte aligned");
   if (wd->type == IZB_K16) IZB_FAIL(IZB_ERR_TYPE, "moe_down: expert stacks of ggml type %d are not taken (Q8_0, Q4_K, Q4_0)", wd->ggml_type);
   if (int rc = izb_require_device(wd->device, "moe_down")) return rc;
-  if (TM >= 1 && TM <= 8) return izb_moe_down_tiles(wd, d_hq, d_hsc, Sp, d_tiles, max_tiles, d_swt, d_y, (cudaStream_t)stream);
+  if (TM >= 1 && TM <= 8) {
+    const int rc = izb_moe_rows_launch(wd, nullptr, d_hq, d_hsc, Sp, d_tiles, max_tiles, nullptr, d_swt, d_y, (cudaStream_t)stream);
+    return rc <= 0 ? rc : izb_moe_down_tiles(wd, d_hq, d_hsc, Sp, d_tiles, max_tiles, d_swt, d_y, (cudaStream_t)stream);
+  }
   if (TM == 128) {
     const int rc = izb_moe_down_tc(wd, d_hq, d_hsc, Sp, d_tiles, max_tiles, d_swt, d_y, (cudaStream_t)stream);
     if (rc <= 0) return rc;

@@ -1,0 +1,577 @@
+// One to eight activation rows against a weight matrix on the warp-level integer matrix instruction (mma.sync, K = 16: int8 x
+// int8 -> int32): decode batches and the per-tile mixture-of-experts products.
+//
+// Such a call is bound by the weights' bytes, but the dot-product kernels (csrc/izb_gemv_stream.cu, csrc/izb_types.cu) spend
+// instructions per weight AND token: at five rows the unpacked nibbles are multiplied five times by dp4a.  One matrix
+// instruction multiplies 16 weight rows x 16 elements with eight tokens at once, so eight tokens cost what one does.  (The
+// tcgen05 kernel wants 128 tokens per tile; at eight it is all latency.)
+//
+// The sums are those of the dot-product kernels bit for bit, so that a batch's results do not depend on which kernel its size
+// selects (a decode step requantises them, and one value that crosses a rounding boundary changes every layer after it): per
+// output the same 32 partial sums -- superblock index modulo kSubs x piece of a superblock -- each added up in superblock order
+// with the same roundings, then the same pairwise tree.  A piece is 16 elements of a block pair (Q4_K), 16 elements (Q8_0) or a
+// 32-block (Q6_K), hence K = 16.  (One sum per output with the min term on a bf16 matrix instruction is a third of the f32
+// work and took 24 us for 34816 x 5120 at five rows, but moved int8 values of the next projection's input.)  Products of the
+// small integers and fp16 scales that those kernels multiply one after the other are exact in f32, so they may be formed once per
+// row and block: P = fma(d * sc, dot, -(dmin * mn) * asum).
+//
+// Lane mapping (g = lane / 4, t = lane % 4): the weight rows are the instruction's M side, the tokens its N side.  A lane supplies
+// bytes 4t .. 4t+3 of a 16-element half of rows g, g + 8 and of token g, and receives rows g, g + 8 against tokens 2t, 2t + 1:
+// register pairs, so all f32 work runs on packed pairs.  Dots reach f32 by starting the accumulator at the bits of 1.5 * 2^23 and
+// subtracting that number (|dot| < 2^22): exact and cheaper than a conversion.  High nibbles are multiplied in place as 16 q.
+//
+// Both operands come from shared memory: each warp has a ring of 16-row x one-superblock chunks filled by TMA (row pitches of 4 mod
+// 8 words: 32-bit reads of eight rows x four words touch every bank once), the activations are staged once per CTA, and what
+// a row's header holds is expanded once per chunk into 16-byte words (per row and block) the whole quad reads.  kSubs warps share
+// a tile, so that neighbouring superblocks of the same rows are in flight together: rings of scattered tiles ran at half the
+// DRAM rate.  The ring's first fill is issued before pdl_wait() (no kernel writes weights).
+#include <cuda.h>
+#include <string.h>
+
+#include "izb_common.cuh"
+
+namespace {
+
+constexpr uint32_t kMagic = 0x4B400000u;  // 1.5 * 2^23
+
+// d = c + rows g (d[0], d[1]) and g + 8 (d[2], d[3]) . tokens 2t, 2t + 1, over 16 elements
+__device__ __forceinline__ void dot16_u8(int (&d)[4], uint32_t w0, uint32_t w1, uint32_t x, uint32_t c0 = kMagic, uint32_t c1 = kMagic) {
+  asm("mma.sync.aligned.m16n8k16.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%8,%7,%8};"
+      : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+      : "r"(w0), "r"(w1), "r"(x), "r"(c0), "r"(c1));
+}
+__device__ __forceinline__ void dot16_s8(int (&d)[4], uint32_t w0, uint32_t w1, uint32_t x) {
+  asm("mma.sync.aligned.m16n8k16.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%7,%7};"
+      : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+      : "r"(w0), "r"(w1), "r"(x), "r"(kMagic));
+}
+
+// f32 pairs (tokens 2t, 2t + 1): two IEEE operations per instruction
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 f2_of(float x, float y) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ f2 f2_add(f2 a, f2 b) {
+  f2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2 f2_mul(f2 a, f2 b) {
+  f2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) {
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ float f2_get(f2 a, int i) { return __uint_as_float((uint32_t)(i ? a >> 32 : a)); }
+// the integer instruction's accumulators of row g + 8 r as f32: minus the number they started from
+__device__ __forceinline__ f2 unmagic(const int (&d)[4], int r) {
+  return f2_add(f2_of(__int_as_float(d[2 * r]), __int_as_float(d[2 * r + 1])), 0xCB400000CB400000ull);
+}
+// unsigned byte k of a word as f32: 0x4B000000 | byte is 2^23 + byte
+__device__ __forceinline__ float byte_f(uint32_t w, int k) { return __fsub_rn(__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440 + k)), 8388608.0f); }
+
+// What the weights are multiplied with, in shared memory (offsets of this lane):
+//   q   token g: words of the first and second 16 elements of a block, `qs` bytes per block
+//   sc  scales of tokens 2t, 2t + 1, four pairs per block
+//   ex  per block and half, four pairs: Q4_K the sum of the 16 values as f32; Q6_K the accumulator's start, kMagic - 32 * that sum
+struct Acts {
+  const unsigned char* q;
+  const f2* sc;
+  const f2* ex;
+  int qs;
+};
+
+// ---- weight forms.  prep() expands the headers of a chunk into `hd` ([block][row] of 16 bytes); mul() multiplies a chunk into
+// the piece sums acc[piece][r]: rows g, g + 8 against tokens 2t, 2t + 1
+struct RQ4K {
+  static constexpr int SBB = 144, kPitch = 144, kSubs = 4, kPieces = 8;
+  static constexpr bool kEx = true, kPrep = true;
+  static __device__ __forceinline__ void prep(const unsigned char* chunk, float4* hd, int lane) {
+    // lane <-> row lane / 2, blocks 4 (lane & 1) .. + 3: (d * sc twice, -dmin * mn twice); the sub-block scales and mins as bytes
+    // (get_scale_min_k4, src/quants.h:61-69).  Odd blocks meet 16 q: their d * sc is divided by 16.
+    const int row = lane >> 1, up = lane & 1;
+    const uint4 h = *reinterpret_cast<const uint4*>(chunk + row * kPitch);
+    const float2 d = __half22float2(*reinterpret_cast<const __half2*>(&h.x));
+    const uint32_t sc = up ? (h.w & 0x0F0F0F0Fu) | ((h.y >> 2) & 0x30303030u) : h.y & 0x3F3F3F3Fu;
+    const uint32_t mn = up ? ((h.w >> 4) & 0x0F0F0F0Fu) | ((h.z >> 2) & 0x30303030u) : h.z & 0x3F3F3F3Fu;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float a = __fmul_rn((k & 1) ? d.x * 0.0625f : d.x, byte_f(sc, k)), b = __fmul_rn(-d.y, byte_f(mn, k));
+      hd[(4 * up + k) * 16 + row] = make_float4(a, a, b, b);
+    }
+  }
+  static __device__ __forceinline__ void mul(const unsigned char* chunk, const float4* hd, const Acts& a, int sb, int g, int t, f2 (&acc)[kPieces][2]) {
+    const unsigned char* p = chunk + g * kPitch + 16 + 4 * t;
+    const unsigned char* xq = a.q + 8 * sb * a.qs;
+    const f2 *xs = a.sc + 32 * sb, *xe = a.ex + 64 * sb;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const uint2 xl = *reinterpret_cast<const uint2*>(xq + 2 * c * a.qs), xh = *reinterpret_cast<const uint2*>(xq + (2 * c + 1) * a.qs);
+      const f2 sl = xs[8 * c], sh = xs[8 * c + 4];
+      f2 hl[2][2], hh[2][2];  // (d * sc, -dmin * mn) of rows g, g + 8: low-nibble and high-nibble block
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const ulonglong2 u = *reinterpret_cast<const ulonglong2*>(hd + 2 * c * 16 + g + 8 * r), v = *reinterpret_cast<const ulonglong2*>(hd + (2 * c + 1) * 16 + g + 8 * r);
+        hl[r][0] = u.x; hl[r][1] = u.y;
+        hh[r][0] = v.x; hh[r][1] = v.y;
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const uint32_t w0 = *reinterpret_cast<const uint32_t*>(p + 32 * c + 16 * h), w1 = *reinterpret_cast<const uint32_t*>(p + 8 * kPitch + 32 * c + 16 * h);
+        const f2 el = xe[16 * c + 4 * h], eh = xe[16 * c + 8 + 4 * h];
+        int dl[4], dh[4];
+        dot16_u8(dl, w0 & 0x0F0F0F0Fu, w1 & 0x0F0F0F0Fu, h ? xl.y : xl.x);
+        dot16_u8(dh, w0 & 0xF0F0F0F0u, w1 & 0xF0F0F0F0u, h ? xh.y : xh.x);
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const f2 P = f2_fma(hl[r][0], unmagic(dl, r), f2_mul(hl[r][1], el)), Q = f2_fma(hh[r][0], unmagic(dh, r), f2_mul(hh[r][1], eh));
+          acc[2 * c + h][r] = f2_add(acc[2 * c + h][r], f2_fma(sl, P, f2_mul(sh, Q)));
+        }
+      }
+    }
+  }
+};
+
+struct RQ80 {
+  static constexpr int SBB = 272, kPitch = 272, kSubs = 2, kPieces = 16;
+  static constexpr bool kEx = false, kPrep = false;
+  static __device__ __forceinline__ void prep(const unsigned char*, float4*, int) {}
+  static __device__ __forceinline__ void mul(const unsigned char* chunk, const float4*, const Acts& a, int sb, int g, int t, f2 (&acc)[kPieces][2]) {
+    const unsigned char* p = chunk + g * kPitch;
+    const uint4 hd[2] = {*reinterpret_cast<const uint4*>(p), *reinterpret_cast<const uint4*>(p + 8 * kPitch)};
+    p += 16 + 4 * t;
+    const unsigned char* xq = a.q + 8 * sb * a.qs;
+    const f2* xs = a.sc + 32 * sb;
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+      const uint2 x = *reinterpret_cast<const uint2*>(xq + b * a.qs);
+      f2 sd[2];
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const uint32_t w = (b >> 1) == 0 ? hd[r].x : (b >> 1) == 1 ? hd[r].y : (b >> 1) == 2 ? hd[r].z : hd[r].w;
+        const float d = half_bits_to_float((b & 1) ? w >> 16 : w & 0xFFFFu);
+        sd[r] = f2_mul(xs[4 * b], f2_of(d, d));
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        int d[4];
+        dot16_s8(d, *reinterpret_cast<const uint32_t*>(p + 32 * b + 16 * h), *reinterpret_cast<const uint32_t*>(p + 8 * kPitch + 32 * b + 16 * h), h ? x.y : x.x);
+#pragma unroll
+        for (int r = 0; r < 2; ++r) acc[2 * b + h][r] = f2_fma(sd[r], unmagic(d, r), acc[2 * b + h][r]);
+      }
+    }
+  }
+};
+
+// Q6_K packed: ql[128] | qh[64] | int8 scale[16] | fp16 d (csrc/izb_types.cu: q6p_word).  The quants' offset of 32 is taken off by the
+// accumulators' start.
+struct RQ6K {
+  static constexpr int SBB = kQ6pSbBytes, kPitch = 240, kSubs = 4, kPieces = 8;
+  static constexpr bool kEx = true, kPrep = true;
+  static __device__ __forceinline__ void prep(const unsigned char* chunk, float4* hd, int lane) {
+    // lane <-> row lane / 2, blocks 4 (lane & 1) .. + 3: (scale of the first half twice, of the second half twice)
+    const int row = lane >> 1, up = lane & 1;
+    const uint2 s = *reinterpret_cast<const uint2*>(chunk + row * kPitch + 192 + 8 * up);
+    const uint32_t w[2] = {s.x ^ 0x80808080u, s.y ^ 0x80808080u};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float a = __fsub_rn(byte_f(w[k >> 1], 2 * (k & 1)), 128.0f), b = __fsub_rn(byte_f(w[k >> 1], 2 * (k & 1) + 1), 128.0f);
+      hd[(4 * up + k) * 16 + row] = make_float4(a, a, b, b);
+    }
+  }
+  static __device__ __forceinline__ uint32_t word(uint32_t ql, uint32_t qh, int sub) {  // 0 .. 63 per byte
+    const uint32_t hi = sub == 0 ? qh << 4 : sub == 1 ? qh << 2 : sub == 2 ? qh : qh >> 2;
+    return (((sub & 2) ? ql >> 4 : ql) & 0x0F0F0F0Fu) | (hi & 0x30303030u);
+  }
+  static __device__ __forceinline__ void mul(const unsigned char* chunk, const float4* hd, const Acts& a, int sb, int g, int t, f2 (&acc)[kPieces][2]) {
+    const unsigned char* p = chunk + g * kPitch;
+    const float d0 = half_bits_to_float(*reinterpret_cast<const unsigned short*>(p + 208)), d1 = half_bits_to_float(*reinterpret_cast<const unsigned short*>(p + 8 * kPitch + 208));
+    const f2 wd[2] = {f2_of(d0, d0), f2_of(d1, d1)};
+    p += 4 * t;
+    const unsigned char* xq = a.q + 8 * sb * a.qs;
+    const f2 *xs = a.sc + 32 * sb, *xe = a.ex + 64 * sb;
+#pragma unroll
+    for (int nh = 0; nh < 2; ++nh) {
+      uint32_t hq[2][2];
+#pragma unroll
+      for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) hq[r][i] = *reinterpret_cast<const uint32_t*>(p + 8 * r * kPitch + 128 + 32 * nh + 16 * i);
+#pragma unroll
+      for (int lo = 0; lo < 2; ++lo) {  // sub-blocks lo and lo + 2 share their low-nibble bytes
+        uint32_t l[2][2];
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+#pragma unroll
+          for (int i = 0; i < 2; ++i) l[r][i] = *reinterpret_cast<const uint32_t*>(p + 8 * r * kPitch + 64 * nh + 32 * lo + 16 * i);
+#pragma unroll
+        for (int up = 0; up < 2; ++up) {
+          const int sub = lo + 2 * up, b = 4 * nh + sub;
+          const uint2 x = *reinterpret_cast<const uint2*>(xq + b * a.qs), c0 = *reinterpret_cast<const uint2*>(xe + 8 * b), c1 = *reinterpret_cast<const uint2*>(xe + 8 * b + 4);
+          int d[4], e[4];
+          dot16_u8(d, word(l[0][0], hq[0][0], sub), word(l[1][0], hq[1][0], sub), x.x, c0.x, c0.y);
+          dot16_u8(e, word(l[0][1], hq[0][1], sub), word(l[1][1], hq[1][1], sub), x.y, c1.x, c1.y);
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            const ulonglong2 s = *reinterpret_cast<const ulonglong2*>(hd + b * 16 + g + 8 * r);
+            // (both products and their sum are integers below 2^24: exact)
+            const f2 v = f2_fma(s.x, unmagic(d, r), f2_mul(s.y, unmagic(e, r)));
+            acc[b][r] = f2_add(acc[b][r], f2_mul(f2_mul(xs[4 * b], wd[r]), v));
+          }
+        }
+      }
+    }
+  }
+};
+
+// ---- a warp's ring of chunks (16 rows x one superblock each), filled by TMA
+__device__ __forceinline__ uint32_t r_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+template <class F>
+struct Ring {
+  static constexpr int kSlot = (16 * F::kPitch + 127) & ~127;
+  static constexpr uint32_t kSpin = 1u << 24;
+  unsigned char* base;
+  uint64_t* bars;
+  int slots, put = 0, get = 0;
+  uint32_t parity = 0;
+  __device__ __forceinline__ void init(int lane) {
+    if (lane == 0) {
+      for (int s = 0; s < slots; ++s) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(r_u32(&bars[s])) : "memory");
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncwarp();
+  }
+  // (every lane keeps the position, lane 0 issues)
+  __device__ __forceinline__ void fill(const void* tmap, int sb, int row, int lane) {
+    if (lane == 0) {
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(r_u32(&bars[put])), "r"(16 * F::kPitch) : "memory");
+      asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(r_u32(base + put * kSlot)),
+                   "l"(tmap), "r"(sb * (F::SBB / 4)), "r"(row), "r"(r_u32(&bars[put]))
+                   : "memory");
+    }
+    if (++put == slots) put = 0;
+  }
+  // the next chunk in order; null when the bounded wait ran out
+  __device__ __forceinline__ const unsigned char* wait() const {
+    for (uint32_t it = 0; it < kSpin; ++it) {
+      uint32_t ok;
+      asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                   : "=r"(ok) : "r"(r_u32(&bars[get])), "r"(parity) : "memory");
+      if (ok) return base + get * kSlot;
+    }
+    return nullptr;
+  }
+  __device__ __forceinline__ void next() {
+    if (++get == slots) { get = 0; parity ^= 1; }
+  }
+};
+
+// ---- shared memory: activations | rings | 4 KB per warp (expanded headers, exchanged sums) | barriers
+template <class F>
+__host__ __device__ __forceinline__ size_t act_bytes(int K, int T) { return ((size_t)(K / 32) * (32 * T + 32 + (F::kEx ? 64 : 0)) + 127) & ~(size_t)127; }
+constexpr int kXch = 4096;
+template <class F>
+__host__ __device__ __forceinline__ size_t rows_smem(int K, int T, int nw, int slots) {
+  return act_bytes<F>(K, T) + (size_t)nw * (slots * (Ring<F>::kSlot + 8) + kXch);
+}
+
+// Activations of T tokens (rows `src(j)` of aq, columns of asc), as Acts describes them.  Four items per thread and pass, so that their
+// loads are in flight together.
+template <class F, class Src>
+__device__ __forceinline__ Acts stage_acts(unsigned char* smem, int K, int T, const int8_t* __restrict__ aq, const float* __restrict__ asc, int Mp, int g, int t, Src src) {
+  const int nb = K / 32, items = nb * T;
+  float* s_sc = reinterpret_cast<float*>(smem + (size_t)nb * 32 * T);
+  float* s_ex = s_sc + nb * 8;
+  constexpr int kBatch = 4;
+  for (int i0 = threadIdx.x; i0 < items; i0 += kBatch * blockDim.x) {
+    uint4 x[kBatch], y[kBatch];
+    float s[kBatch];
+    int bb[kBatch], jj[kBatch];
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      const int i = i0 + u * blockDim.x;
+      bb[u] = i / T;
+      jj[u] = i - bb[u] * T;
+      if (i < items) {
+        const int row = src(jj[u]);
+        const uint4* p = reinterpret_cast<const uint4*>(aq + (size_t)row * K) + 2 * bb[u];
+        x[u] = p[0];
+        y[u] = p[1];
+        s[u] = asc[(size_t)bb[u] * Mp + row];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      const int b = bb[u], j = jj[u];
+      if (i0 + u * (int)blockDim.x >= items) continue;
+      uint4* o = reinterpret_cast<uint4*>(smem + (size_t)(b * T + j) * 32);
+      o[0] = make_uint4(x[u].x, y[u].x, x[u].y, y[u].y);
+      o[1] = make_uint4(x[u].z, y[u].z, x[u].w, y[u].w);
+      s_sc[b * 8 + j] = s[u];
+      if (F::kEx) {
+        const uint32_t w[8] = {x[u].x, x[u].y, x[u].z, x[u].w, y[u].x, y[u].y, y[u].z, y[u].w};
+        int s0 = 0, s1 = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          s0 = __dp4a((int)w[k], 0x01010101, s0);
+          s1 = __dp4a((int)w[4 + k], 0x01010101, s1);
+        }
+        const bool q4 = F::SBB == 144;
+        s_ex[b * 16 + j] = q4 ? (float)s0 : __int_as_float((int)kMagic - 32 * s0);
+        s_ex[b * 16 + 8 + j] = q4 ? (float)s1 : __int_as_float((int)kMagic - 32 * s1);
+      }
+    }
+  }
+  Acts a;
+  a.q = smem + min(g, T - 1) * 32 + 8 * t;  // (lanes past the last token repeat it; their results are not stored)
+  a.sc = reinterpret_cast<const f2*>(s_sc) + t;
+  a.ex = reinterpret_cast<const f2*>(s_ex) + t;
+  a.qs = 32 * T;
+  return a;
+}
+
+// One chunk after the other of this warp's share of a tile (superblocks part, part + kSubs, ...) into acc.  false: a wait ran out.
+template <class F, class Request>
+__device__ __forceinline__ bool accumulate(Ring<F>& ring, float4* hd, const Acts& acts, int part, int nsb, int lane, f2 (&acc)[F::kPieces][2], Request request) {
+  const int g = lane >> 2, t = lane & 3;
+#pragma unroll
+  for (int p = 0; p < F::kPieces; ++p) acc[p][0] = acc[p][1] = 0ull;
+  for (int s = part; s < nsb; s += F::kSubs) {
+    const unsigned char* chunk = ring.wait();
+    if (!chunk) return false;
+    if (F::kPrep) {
+      F::prep(chunk, hd, lane);
+      __syncwarp();
+    }
+    F::mul(chunk, hd, acts, s, g, t, acc);
+    __syncwarp();  // every lane has read the chunk: its slot takes the next request
+    ring.next();
+    request();
+  }
+  return true;
+}
+
+// The tree over a tile's 32 partial sums per output: superblock parts p, p ^ 2, then p ^ 1 (through shared memory: parts 2 and 3
+// hand theirs to 0 and 1, part 1 to 0), then the pieces halves first.  All warps of the CTA call it; the result is valid in part 0.
+// `xch`: this CTA's exchange areas, one per warp.
+template <class F>
+__device__ __forceinline__ void reduce_tile(f2 (&acc)[F::kPieces][2], unsigned char* xch, int warp, int lane) {
+  static_assert(F::kSubs == 4 ? F::kPieces == 8 : F::kSubs == 2 && F::kPieces == 16, "exchange areas: 4 KB per warp");
+  const int part = warp % F::kSubs;
+  auto area = [&](int w) { return reinterpret_cast<ulonglong2*>(xch + (size_t)w * kXch) + lane; };  // [piece][lane] of 16 bytes
+  auto give = [&](int w) {
+#pragma unroll
+    for (int p = 0; p < F::kPieces; ++p) area(w)[32 * p] = make_ulonglong2(acc[p][0], acc[p][1]);
+  };
+  auto take = [&](int w) {
+#pragma unroll
+    for (int p = 0; p < F::kPieces; ++p) {
+      const ulonglong2 v = area(w)[32 * p];
+      acc[p][0] = f2_add(acc[p][0], v.x);
+      acc[p][1] = f2_add(acc[p][1], v.y);
+    }
+  };
+  __syncthreads();  // (the areas hold headers until here, or sums the last tile's readers may still want)
+  if (F::kSubs == 4) {
+    if (part >= 2) give(warp);
+    __syncthreads();
+    if (part < 2) take(warp + 2);
+    if (part == 1) give(warp);
+    __syncthreads();
+    if (part == 0) take(warp + 1);
+  } else {
+    if (part == 1) give(warp - 1);  // (sixteen pieces: the areas of both warps)
+    __syncthreads();
+    if (part == 0) take(warp);
+  }
+#pragma unroll
+  for (int h = F::kPieces / 2; h > 0; h >>= 1)
+#pragma unroll
+    for (int p = 0; p < h; ++p)
+#pragma unroll
+      for (int r = 0; r < 2; ++r) acc[p][r] = f2_add(acc[p][r], acc[p + h][r]);
+  if (F::kPrep) __syncthreads();  // the areas take headers again
+}
+
+// C[token][c_off + row] (= or +=) for T tokens.  The grid walks groups of NW / kSubs row tiles.
+template <class F, int NW>
+__global__ void __launch_bounds__(NW * 32, NW == 8 ? 2 : 1) rows_kernel(const __grid_constant__ CUtensorMap tm, int wrow0, int N, int K, const int8_t* __restrict__ aq,
+                                                                        const float* __restrict__ asc, int T, int Mp, float* __restrict__ C, int ldc, int c_off, int acc_mode,
+                                                                        int slots, uint32_t* err) {
+  extern __shared__ __align__(1024) unsigned char smem[];
+  constexpr int kPer = NW / F::kSubs;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int part = warp % F::kSubs, mine = warp / F::kSubs, nsb = K >> 8, groups = ((N + 15) / 16 + kPer - 1) / kPer;
+  unsigned char* rings = smem + act_bytes<F>(K, T);
+  unsigned char* xch = rings + (size_t)NW * slots * Ring<F>::kSlot;
+  Ring<F> ring;
+  ring.slots = slots;
+  ring.base = rings + (size_t)warp * slots * Ring<F>::kSlot;
+  ring.bars = reinterpret_cast<uint64_t*>(xch + NW * kXch) + warp * slots;
+  ring.init(lane);
+  // chunks still to request: superblock `ps` of the tile in group `pg`
+  int pg = blockIdx.x, ps = part;
+  auto request = [&]() {
+    if (pg >= groups || part >= nsb) return;
+    ring.fill(&tm, ps, wrow0 + (pg * kPer + mine) * 16, lane);
+    if ((ps += F::kSubs) >= nsb) { ps = part; pg += gridDim.x; }
+  };
+  for (int s = 0; s < slots; ++s) request();
+  pdl_launch_next();
+  pdl_wait();
+  const Acts acts = stage_acts<F>(smem, K, T, aq, asc, Mp, g, t, [](int j) { return j; });
+  __syncthreads();
+  bool ok = true;
+  for (int gr = blockIdx.x; gr < groups; gr += gridDim.x) {
+    f2 acc[F::kPieces][2];
+    ok = ok && accumulate<F>(ring, reinterpret_cast<float4*>(xch + (size_t)warp * kXch), acts, part, nsb, lane, acc, request);
+    if (!ok && lane == 0) atomicOr(err, 64u);  // (bounded wait gave up)
+    reduce_tile<F>(acc, xch, warp, lane);
+    ok = __syncthreads_and(ok);
+    if (!ok) break;
+    if (part == 0) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int row = (gr * kPer + mine) * 16 + g + 8 * (i >> 1), tok = 2 * t + (i & 1);
+        if (row < N && tok < T) {
+          float* c = C + (size_t)tok * ldc + c_off + row;
+          const float v = f2_get(acc[0][i >> 1], i & 1);
+          *c = acc_mode ? __fadd_rn(*c, v) : v;
+        }
+      }
+    }
+  }
+}
+
+// Mixture of experts: one CTA = a tile (up to 8 slots of one expert) x a group of row tiles.
+// gate/up (pair): h[slot][N] = silu(x Wg^T) * (x Wu^T), token rows through stok; down: y[slot][N] = swt * (hq Wd^T).
+template <class F, int NW>
+__global__ void __launch_bounds__(NW * 32, NW == 8 ? 2 : 1) moe_rows_kernel(const __grid_constant__ CUtensorMap tg, const __grid_constant__ CUtensorMap tu, int pair, int N, int K,
+                                                                            const int8_t* __restrict__ aq, const float* __restrict__ asc, int Mp,
+                                                                            const int32_t* __restrict__ tiles, const int32_t* __restrict__ stok,
+                                                                            const float* __restrict__ swt, float* __restrict__ out, int slots, uint32_t* err) {
+  extern __shared__ __align__(1024) unsigned char smem[];
+  constexpr int kPer = NW / F::kSubs;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int part = warp % F::kSubs, mine = warp / F::kSubs, nsb = K >> 8;
+  unsigned char* rings = smem + act_bytes<F>(K, 8);
+  unsigned char* xch = rings + (size_t)NW * slots * Ring<F>::kSlot;
+  Ring<F> ring;
+  ring.slots = slots;
+  ring.base = rings + (size_t)warp * slots * Ring<F>::kSlot;
+  ring.bars = reinterpret_cast<uint64_t*>(xch + NW * kXch) + warp * slots;
+  ring.init(lane);
+  pdl_launch_next();
+  pdl_wait();
+  const int ti = blockIdx.y;
+  if (ti >= tiles[0]) return;  // uniform over the CTA
+  const int e = tiles[1 + 3 * ti], s0 = tiles[2 + 3 * ti], T = tiles[3 + 3 * ti];
+  const int tile = blockIdx.x * kPer + mine;
+  int pm = 0, ps = part;  // matrix (gate, up) and superblock still to request
+  auto request = [&]() {
+    if (pm > pair || part >= nsb) return;
+    ring.fill(pm ? &tu : &tg, ps, e * N + tile * 16, lane);
+    if ((ps += F::kSubs) >= nsb) { ps = part; ++pm; }
+  };
+  for (int s = 0; s < slots; ++s) request();
+  const Acts acts = stage_acts<F>(smem, K, T, aq, asc, Mp, g, t, [&](int j) { return stok ? stok[s0 + j] : s0 + j; });
+  __syncthreads();
+  float first[4];
+  for (int m = 0; m <= pair; ++m) {
+    f2 acc[F::kPieces][2];
+    bool ok = accumulate<F>(ring, reinterpret_cast<float4*>(xch + (size_t)warp * kXch), acts, part, nsb, lane, acc, request);
+    if (!ok && lane == 0) atomicOr(err, 64u);  // (bounded wait gave up)
+    reduce_tile<F>(acc, xch, warp, lane);
+    if (!__syncthreads_and(ok)) return;
+    if (m < pair) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) first[i] = f2_get(acc[0][i >> 1], i & 1);
+    } else if (part == 0) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int n = tile * 16 + g + 8 * (i >> 1), slot = 2 * t + (i & 1);
+        if (n < N && slot < T) {
+          const float v = f2_get(acc[0][i >> 1], i & 1);
+          out[(size_t)(s0 + slot) * N + n] = pair ? __fmul_rn(__fdiv_rn(first[i], __fadd_rn(1.0f, expf(-first[i]))), v) : __fmul_rn(swt[s0 + slot], v);
+        }
+      }
+    }
+  }
+}
+
+constexpr size_t kHalfSm = 113 * 1024, kWholeSm = 226 * 1024;
+// most slots (up to four: deeper rings gain nothing) that fit `budget`
+template <class F>
+int rows_slots(int K, int T, int nw, size_t budget) {
+  int s = 4;
+  while (s > 0 && rows_smem<F>(K, T, nw, s) > budget) --s;
+  return s;
+}
+
+template <class F, int NW>
+int launch_rows(const izb_weight* w, int mat, const int8_t* aq, const float* asc, int T, int Mp, float* C, int ldc, int c_off, int acc, int slots, cudaStream_t st) {
+  IZB_SMEM_OPTIN((rows_kernel<F, NW>), kWholeSm, w->device);
+  constexpr int kPer = NW / F::kSubs;
+  const size_t smem = rows_smem<F>(w->K, T, NW, slots);
+  const int groups = ((w->N + 15) / 16 + kPer - 1) / kPer, most = izb_sm_count(w->device) * (smem <= kHalfSm ? 2 : 1), grid = groups < most ? groups : most;
+  uint32_t* err = izb_device_error_word(w->device);
+  if (!err) IZB_FAIL(IZB_ERR_NOMEM, "gemv: no device error word");
+  CUtensorMap tm;
+  memcpy(&tm, w->tmap16_raw, sizeof tm);
+  IZB_LAUNCH("gemv_rows", st, izb_launch_pdl(rows_kernel<F, NW>, grid, NW * 32, smem, st, tm, mat * w->N, w->N, w->K, aq, asc, T, Mp, C, ldc, c_off, acc, slots, err));
+  return IZB_OK;
+}
+// Two CTAs of eight warps per SM where the activations leave room for rings, else one of sixteen, else one of eight; activations that do
+// not fit even there (8 rows of K = 17408) go half the tokens at a time, the second pass finding part of the weights in L2.
+template <class F>
+int rows_of(const izb_weight* w, int mat, const int8_t* aq, const float* asc, int T, int Mp, float* C, int ldc, int c_off, int acc, cudaStream_t st) {
+  if (const int s = rows_slots<F>(w->K, T, 8, kHalfSm); s >= 2) return launch_rows<F, 8>(w, mat, aq, asc, T, Mp, C, ldc, c_off, acc, s, st);
+  if (const int s = rows_slots<F>(w->K, T, 16, kWholeSm); s >= 2) return launch_rows<F, 16>(w, mat, aq, asc, T, Mp, C, ldc, c_off, acc, s, st);
+  if (const int s = rows_slots<F>(w->K, T, 8, kWholeSm); s >= 2) return launch_rows<F, 8>(w, mat, aq, asc, T, Mp, C, ldc, c_off, acc, s, st);
+  if (T < 2) return 1;
+  const int h = (T + 1) / 2;
+  if (const int rc = rows_of<F>(w, mat, aq, asc, h, Mp, C, ldc, c_off, acc, st)) return rc;
+  return rows_of<F>(w, mat, aq + (size_t)h * w->K, asc + h, T - h, Mp, C + (size_t)h * ldc, ldc, c_off, acc, st);
+}
+template <class F>
+int moe_rows_of(const izb_weight* wg, const izb_weight* wu, const int8_t* aq, const float* asc, int Mp, const int32_t* tiles, int max_tiles, const int32_t* stok, const float* swt,
+                float* out, cudaStream_t st) {
+  int slots = rows_slots<F>(wg->K, 8, 8, kHalfSm);
+  if (slots < 2) slots = rows_slots<F>(wg->K, 8, 8, kWholeSm);
+  if (slots < 2) return 1;
+  IZB_SMEM_OPTIN((moe_rows_kernel<F, 8>), kWholeSm, wg->device);
+  constexpr int kPer = 8 / F::kSubs;
+  uint32_t* err = izb_device_error_word(wg->device);
+  if (!err) IZB_FAIL(IZB_ERR_NOMEM, "moe: no device error word");
+  CUtensorMap tg, tu;
+  memcpy(&tg, wg->tmap16_raw, sizeof tg);
+  memcpy(&tu, (wu ? wu : wg)->tmap16_raw, sizeof tu);
+  dim3 grid(((wg->N + 15) / 16 + kPer - 1) / kPer, max_tiles);
+  IZB_LAUNCH(wu ? "moe_gateup" : "moe_down", st, izb_launch_pdl(moe_rows_kernel<F, 8>, grid, 256, rows_smem<F>(wg->K, 8, 8, slots), st, tg, tu, wu ? 1 : 0, wg->N, wg->K, aq, asc, Mp,
+                                                               tiles, stok, swt, out, slots, err));
+  return IZB_OK;
+}
+
+}  // namespace
+
+// up to 8 rows; +1: not taken (another weight form, no tensor map, or activations that do not fit in shared memory)
+int izb_rows_launch(const izb_weight* w, int mat, const int8_t* aq, const float* asc, int T, int Mp, float* C, int ldc, int c_off, int acc, cudaStream_t st) {
+  if (!w->has_tmap16 || T > 8) return 1;
+  if (w->type == IZB_Q4_K) return rows_of<RQ4K>(w, mat, aq, asc, T, Mp, C, ldc, c_off, acc, st);
+  if (w->type == IZB_Q8_0) return rows_of<RQ80>(w, mat, aq, asc, T, Mp, C, ldc, c_off, acc, st);
+  return rows_of<RQ6K>(w, mat, aq, asc, T, Mp, C, ldc, c_off, acc, st);
+}
+
+// gate / up (wu given) or down (wu = null, swt given) over tiles of up to 8 slots; +1: not taken
+int izb_moe_rows_launch(const izb_weight* wg, const izb_weight* wu, const int8_t* aq, const float* asc, int Mp, const int32_t* tiles, int max_tiles, const int32_t* stok,
+                        const float* swt, float* out, cudaStream_t st) {
+  if (!wg->has_tmap16 || (wu && !wu->has_tmap16)) return 1;
+  return wg->type == IZB_Q4_K ? moe_rows_of<RQ4K>(wg, wu, aq, asc, Mp, tiles, max_tiles, stok, swt, out, st)
+                              : moe_rows_of<RQ80>(wg, wu, aq, asc, Mp, tiles, max_tiles, stok, swt, out, st);
+}
