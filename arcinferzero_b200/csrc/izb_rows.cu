@@ -22,7 +22,7 @@
 //
 // Both operands come from shared memory: each warp has a ring of 16-row x one-superblock chunks filled by TMA (row pitches of 4 mod
 // 8 words: 32-bit reads of eight rows x four words touch every bank once), the activations are staged once per CTA, and what
-// a row's header holds is expanded once per chunk into 16-byte words (per row and block) the whole quad reads.  kSubs warps share
+// a row's header holds is expanded once per chunk (per row and block) for the whole quad.  kSubs warps share
 // a tile, so that neighbouring superblocks of the same rows are in flight together: rings of scattered tiles ran at half the
 // DRAM rate.  The ring's first fill is issued before pdl_wait() (no kernel writes weights).
 #include <cuda.h>
@@ -87,13 +87,13 @@ struct Acts {
   int qs;
 };
 
-// ---- weight forms.  prep() expands the headers of a chunk into `hd` ([block][row] of 16 bytes); mul() multiplies a chunk into
+// ---- weight forms.  prep() expands the headers of a chunk into `hd` ([block][row]); mul() multiplies a chunk into
 // the piece sums acc[piece][r]: rows g, g + 8 against tokens 2t, 2t + 1
 struct RQ4K {
   static constexpr int SBB = 144, kPitch = 144, kSubs = 4, kPieces = 8;
   static constexpr bool kEx = true, kPrep = true;
-  static __device__ __forceinline__ void prep(const unsigned char* chunk, float4* hd, int lane) {
-    // lane <-> row lane / 2, blocks 4 (lane & 1) .. + 3: (d * sc twice, -dmin * mn twice); the sub-block scales and mins as bytes
+  static __device__ __forceinline__ void prep(const unsigned char* chunk, float2* hd, int lane) {
+    // lane <-> row lane / 2, blocks 4 (lane & 1) .. + 3: (d * sc, -dmin * mn); the sub-block scales and mins as bytes
     // (get_scale_min_k4, src/quants.h:61-69).  Odd blocks meet 16 q: their d * sc is divided by 16.
     const int row = lane >> 1, up = lane & 1;
     const uint4 h = *reinterpret_cast<const uint4*>(chunk + row * kPitch);
@@ -103,10 +103,10 @@ struct RQ4K {
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const float a = __fmul_rn((k & 1) ? d.x * 0.0625f : d.x, byte_f(sc, k)), b = __fmul_rn(-d.y, byte_f(mn, k));
-      hd[(4 * up + k) * 16 + row] = make_float4(a, a, b, b);
+      hd[(4 * up + k) * 16 + row] = make_float2(a, b);
     }
   }
-  static __device__ __forceinline__ void mul(const unsigned char* chunk, const float4* hd, const Acts& a, int sb, int g, int t, f2 (&acc)[kPieces][2]) {
+  static __device__ __forceinline__ void mul(const unsigned char* chunk, const float2* hd, const Acts& a, int sb, int g, int t, f2 (&acc)[kPieces][2]) {
     const unsigned char* p = chunk + g * kPitch + 16 + 4 * t;
     const unsigned char* xq = a.q + 8 * sb * a.qs;
     const f2 *xs = a.sc + 32 * sb, *xe = a.ex + 64 * sb;
@@ -117,9 +117,9 @@ struct RQ4K {
       f2 hl[2][2], hh[2][2];  // (d * sc, -dmin * mn) of rows g, g + 8: low-nibble and high-nibble block
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
-        const ulonglong2 u = *reinterpret_cast<const ulonglong2*>(hd + 2 * c * 16 + g + 8 * r), v = *reinterpret_cast<const ulonglong2*>(hd + (2 * c + 1) * 16 + g + 8 * r);
-        hl[r][0] = u.x; hl[r][1] = u.y;
-        hh[r][0] = v.x; hh[r][1] = v.y;
+        const float2 u = hd[2 * c * 16 + g + 8 * r], v = hd[(2 * c + 1) * 16 + g + 8 * r];
+        hl[r][0] = f2_of(u.x, u.x); hl[r][1] = f2_of(u.y, u.y);
+        hh[r][0] = f2_of(v.x, v.x); hh[r][1] = f2_of(v.y, v.y);
       }
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
@@ -141,8 +141,8 @@ struct RQ4K {
 struct RQ80 {
   static constexpr int SBB = 272, kPitch = 272, kSubs = 2, kPieces = 16;
   static constexpr bool kEx = false, kPrep = false;
-  static __device__ __forceinline__ void prep(const unsigned char*, float4*, int) {}
-  static __device__ __forceinline__ void mul(const unsigned char* chunk, const float4*, const Acts& a, int sb, int g, int t, f2 (&acc)[kPieces][2]) {
+  static __device__ __forceinline__ void prep(const unsigned char*, float2*, int) {}
+  static __device__ __forceinline__ void mul(const unsigned char* chunk, const float2*, const Acts& a, int sb, int g, int t, f2 (&acc)[kPieces][2]) {
     const unsigned char* p = chunk + g * kPitch;
     const uint4 hd[2] = {*reinterpret_cast<const uint4*>(p), *reinterpret_cast<const uint4*>(p + 8 * kPitch)};
     p += 16 + 4 * t;
@@ -174,22 +174,22 @@ struct RQ80 {
 struct RQ6K {
   static constexpr int SBB = kQ6pSbBytes, kPitch = 240, kSubs = 4, kPieces = 8;
   static constexpr bool kEx = true, kPrep = true;
-  static __device__ __forceinline__ void prep(const unsigned char* chunk, float4* hd, int lane) {
-    // lane <-> row lane / 2, blocks 4 (lane & 1) .. + 3: (scale of the first half twice, of the second half twice)
+  static __device__ __forceinline__ void prep(const unsigned char* chunk, float2* hd, int lane) {
+    // lane <-> row lane / 2, blocks 4 (lane & 1) .. + 3: (scale of the first half, of the second half)
     const int row = lane >> 1, up = lane & 1;
     const uint2 s = *reinterpret_cast<const uint2*>(chunk + row * kPitch + 192 + 8 * up);
     const uint32_t w[2] = {s.x ^ 0x80808080u, s.y ^ 0x80808080u};
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const float a = __fsub_rn(byte_f(w[k >> 1], 2 * (k & 1)), 128.0f), b = __fsub_rn(byte_f(w[k >> 1], 2 * (k & 1) + 1), 128.0f);
-      hd[(4 * up + k) * 16 + row] = make_float4(a, a, b, b);
+      hd[(4 * up + k) * 16 + row] = make_float2(a, b);
     }
   }
   static __device__ __forceinline__ uint32_t word(uint32_t ql, uint32_t qh, int sub) {  // 0 .. 63 per byte
     const uint32_t hi = sub == 0 ? qh << 4 : sub == 1 ? qh << 2 : sub == 2 ? qh : qh >> 2;
     return (((sub & 2) ? ql >> 4 : ql) & 0x0F0F0F0Fu) | (hi & 0x30303030u);
   }
-  static __device__ __forceinline__ void mul(const unsigned char* chunk, const float4* hd, const Acts& a, int sb, int g, int t, f2 (&acc)[kPieces][2]) {
+  static __device__ __forceinline__ void mul(const unsigned char* chunk, const float2* hd, const Acts& a, int sb, int g, int t, f2 (&acc)[kPieces][2]) {
     const unsigned char* p = chunk + g * kPitch;
     const float d0 = half_bits_to_float(*reinterpret_cast<const unsigned short*>(p + 208)), d1 = half_bits_to_float(*reinterpret_cast<const unsigned short*>(p + 8 * kPitch + 208));
     const f2 wd[2] = {f2_of(d0, d0), f2_of(d1, d1)};
@@ -219,10 +219,11 @@ struct RQ6K {
           dot16_u8(e, word(l[0][1], hq[0][1], sub), word(l[1][1], hq[1][1], sub), x.y, c1.x, c1.y);
 #pragma unroll
           for (int r = 0; r < 2; ++r) {
-            const ulonglong2 s = *reinterpret_cast<const ulonglong2*>(hd + b * 16 + g + 8 * r);
+            const float2 s = hd[b * 16 + g + 8 * r];
             // (both products and their sum are integers below 2^24: exact)
-            const f2 v = f2_fma(s.x, unmagic(d, r), f2_mul(s.y, unmagic(e, r)));
-            acc[b][r] = f2_add(acc[b][r], f2_mul(f2_mul(xs[4 * b], wd[r]), v));
+            const f2 v = f2_fma(f2_of(s.x, s.x), unmagic(d, r), f2_mul(f2_of(s.y, s.y), unmagic(e, r)));
+            // (the product as an fma with -0: a multiply would be fused with the addition behind it, one rounding instead of two)
+            acc[b][r] = f2_add(acc[b][r], f2_fma(f2_mul(xs[4 * b], wd[r]), v, 0x8000000080000000ull));
           }
         }
       }
@@ -338,7 +339,7 @@ __device__ __forceinline__ Acts stage_acts(unsigned char* smem, int K, int T, co
 
 // One chunk after the other of this warp's share of a tile (superblocks part, part + kSubs, ...) into acc.  false: a wait ran out.
 template <class F, class Request>
-__device__ __forceinline__ bool accumulate(Ring<F>& ring, float4* hd, const Acts& acts, int part, int nsb, int lane, f2 (&acc)[F::kPieces][2], Request request) {
+__device__ __forceinline__ bool accumulate(Ring<F>& ring, float2* hd, const Acts& acts, int part, int nsb, int lane, f2 (&acc)[F::kPieces][2], Request request) {
   const int g = lane >> 2, t = lane & 3;
 #pragma unroll
   for (int p = 0; p < F::kPieces; ++p) acc[p][0] = acc[p][1] = 0ull;
@@ -358,12 +359,14 @@ __device__ __forceinline__ bool accumulate(Ring<F>& ring, float4* hd, const Acts
 }
 
 // The tree over a tile's 32 partial sums per output: superblock parts p, p ^ 2, then p ^ 1 (through shared memory: parts 2 and 3
-// hand theirs to 0 and 1, part 1 to 0), then the pieces halves first.  All warps of the CTA call it; the result is valid in part 0.
-// `xch`: this CTA's exchange areas, one per warp.
+// hand theirs to 0 and 1, part 1 to 0), then the pieces halves first.  All warps of a tile call it (a named barrier per tile: the
+// tiles of a CTA need not keep step); the result is valid in part 0.  `xch`: this CTA's exchange areas, one per warp.
+template <class F>
+__device__ __forceinline__ void tile_sync(int mine) { asm volatile("bar.sync %0, %1;" ::"r"(1 + mine), "n"(F::kSubs * 32) : "memory"); }
 template <class F>
 __device__ __forceinline__ void reduce_tile(f2 (&acc)[F::kPieces][2], unsigned char* xch, int warp, int lane) {
   static_assert(F::kSubs == 4 ? F::kPieces == 8 : F::kSubs == 2 && F::kPieces == 16, "exchange areas: 4 KB per warp");
-  const int part = warp % F::kSubs;
+  const int part = warp % F::kSubs, mine = warp / F::kSubs;
   auto area = [&](int w) { return reinterpret_cast<ulonglong2*>(xch + (size_t)w * kXch) + lane; };  // [piece][lane] of 16 bytes
   auto give = [&](int w) {
 #pragma unroll
@@ -377,18 +380,19 @@ __device__ __forceinline__ void reduce_tile(f2 (&acc)[F::kPieces][2], unsigned c
       acc[p][1] = f2_add(acc[p][1], v.y);
     }
   };
-  __syncthreads();  // (the areas hold headers until here, or sums the last tile's readers may still want)
   if (F::kSubs == 4) {
-    if (part >= 2) give(warp);
-    __syncthreads();
+    if (part >= 2) give(warp);  // (a warp's own area: only its own headers were there)
+    tile_sync<F>(mine);
     if (part < 2) take(warp + 2);
     if (part == 1) give(warp);
-    __syncthreads();
+    tile_sync<F>(mine);
     if (part == 0) take(warp + 1);
+    tile_sync<F>(mine);  // the areas take headers again
   } else {
     if (part == 1) give(warp - 1);  // (sixteen pieces: the areas of both warps)
-    __syncthreads();
+    tile_sync<F>(mine);
     if (part == 0) take(warp);
+    tile_sync<F>(mine);
   }
 #pragma unroll
   for (int h = F::kPieces / 2; h > 0; h >>= 1)
@@ -396,7 +400,6 @@ __device__ __forceinline__ void reduce_tile(f2 (&acc)[F::kPieces][2], unsigned c
     for (int p = 0; p < h; ++p)
 #pragma unroll
       for (int r = 0; r < 2; ++r) acc[p][r] = f2_add(acc[p][r], acc[p + h][r]);
-  if (F::kPrep) __syncthreads();  // the areas take headers again
 }
 
 // C[token][c_off + row] (= or +=) for T tokens.  The grid walks groups of NW / kSubs row tiles.
@@ -414,6 +417,9 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 2 : 1) rows_kernel(const __
   ring.slots = slots;
   ring.base = rings + (size_t)warp * slots * Ring<F>::kSlot;
   ring.bars = reinterpret_cast<uint64_t*>(xch + NW * kXch) + warp * slots;
+  __shared__ int s_gave_up;
+  volatile int* gave_up = &s_gave_up;
+  if (threadIdx.x == 0) s_gave_up = 0;
   ring.init(lane);
   // chunks still to request: superblock `ps` of the tile in group `pg`
   int pg = blockIdx.x, ps = part;
@@ -430,12 +436,13 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 2 : 1) rows_kernel(const __
   bool ok = true;
   for (int gr = blockIdx.x; gr < groups; gr += gridDim.x) {
     f2 acc[F::kPieces][2];
-    ok = ok && accumulate<F>(ring, reinterpret_cast<float4*>(xch + (size_t)warp * kXch), acts, part, nsb, lane, acc, request);
-    if (!ok && lane == 0) atomicOr(err, 64u);  // (bounded wait gave up)
+    if (ok) ok = accumulate<F>(ring, reinterpret_cast<float2*>(xch + (size_t)warp * kXch), acts, part, nsb, lane, acc, request);
+    if (!ok) {  // (bounded wait gave up: nothing of this CTA is stored any more)
+      if (lane == 0) atomicOr(err, 64u);
+      *gave_up = 1;
+    }
     reduce_tile<F>(acc, xch, warp, lane);
-    ok = __syncthreads_and(ok);
-    if (!ok) break;
-    if (part == 0) {
+    if (part == 0 && !*gave_up) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int row = (gr * kPer + mine) * 16 + g + 8 * (i >> 1), tok = 2 * t + (i & 1);
@@ -466,6 +473,9 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 2 : 1) moe_rows_kernel(cons
   ring.slots = slots;
   ring.base = rings + (size_t)warp * slots * Ring<F>::kSlot;
   ring.bars = reinterpret_cast<uint64_t*>(xch + NW * kXch) + warp * slots;
+  __shared__ int s_gave_up;
+  volatile int* gave_up = &s_gave_up;
+  if (threadIdx.x == 0) s_gave_up = 0;
   ring.init(lane);
   pdl_launch_next();
   pdl_wait();
@@ -483,16 +493,19 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 2 : 1) moe_rows_kernel(cons
   const Acts acts = stage_acts<F>(smem, K, T, aq, asc, Mp, g, t, [&](int j) { return stok ? stok[s0 + j] : s0 + j; });
   __syncthreads();
   float first[4];
+  bool ok = true;
   for (int m = 0; m <= pair; ++m) {
     f2 acc[F::kPieces][2];
-    bool ok = accumulate<F>(ring, reinterpret_cast<float4*>(xch + (size_t)warp * kXch), acts, part, nsb, lane, acc, request);
-    if (!ok && lane == 0) atomicOr(err, 64u);  // (bounded wait gave up)
+    if (ok) ok = accumulate<F>(ring, reinterpret_cast<float2*>(xch + (size_t)warp * kXch), acts, part, nsb, lane, acc, request);
+    if (!ok) {  // (bounded wait gave up: nothing of this CTA is stored any more)
+      if (lane == 0) atomicOr(err, 64u);
+      *gave_up = 1;
+    }
     reduce_tile<F>(acc, xch, warp, lane);
-    if (!__syncthreads_and(ok)) return;
     if (m < pair) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) first[i] = f2_get(acc[0][i >> 1], i & 1);
-    } else if (part == 0) {
+    } else if (part == 0 && !*gave_up) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int n = tile * 16 + g + 8 * (i >> 1), slot = 2 * t + (i & 1);

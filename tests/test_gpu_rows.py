@@ -1,0 +1,64 @@
+"""The few-row kernels (1 .. 8 rows) at the sizes where their tiles, splits and rings end: rows that do not fill a 16-row tile, one
+superblock, superblock counts that do not divide, activations that take one CTA per SM or two passes; dense and per-expert."""
+import numpy as np
+import pytest
+
+from arcinferzero_b200 import synth as S
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-5
+
+
+def rel(a, b):
+    return float(np.abs(a.astype(np.float64) - b).max() / np.abs(b).max())
+
+
+@pytest.mark.parametrize("qt", [12, 8, 14])
+@pytest.mark.parametrize("N,K", [(8, 256), (17, 512), (1000, 768), (4104, 2304), (48, 17408), (3000, 4096)])
+def test_rows_match_oracle(izb, qt, N, K):
+    import torch
+    w = S.make_weight(qt, N, K, N + K + qt)
+    W = izb.Weight(qt, w, N, K)
+    for T in (1, 2, 3, 5, 8):
+        aq, asc, _ = O.quantize_act(S.make_act(T, K, T + K), Mp=16)
+        ref = O.matmul(qt, w, K, aq, asc, T, "f64")
+        base = np.random.default_rng(T).standard_normal((T, N + 8)).astype(np.float32)
+        for acc in (0, 1):
+            out = torch.from_numpy(base).cuda()
+            izb.matmul(W, torch.from_numpy(aq).cuda(), torch.from_numpy(asc).cuda(), T, out=out, c_off=4, acc=acc)
+            got = out.cpu().numpy()
+            assert rel(got[:, 4:N + 4] - (base[:, 4:N + 4] if acc else 0), ref) < (4 * TOL if acc else TOL), (T, acc)
+            assert (got[:, :4] == base[:, :4]).all() and (got[:, N + 4:] == base[:, N + 4:]).all()
+    assert izb.device_status(0) == 0
+    W.close()
+
+
+@pytest.mark.parametrize("qt", [12, 8])
+@pytest.mark.parametrize("T,TM,F,E", [(1, 8, 256, 512), (5, 4, 768, 1024), (40, 8, 256, 2304), (3, 1, 512, 256)])
+def test_expert_rows_equal_dense_rows(izb, qt, T, TM, F, E):
+    """Every slot's expert product against the same product as a dense call on that expert's matrix."""
+    import torch
+    NE, NU = 8, 2
+    g, u, d = (S.make_weight(qt, NE * n, k, i) for i, (n, k) in enumerate(((F, E), (F, E), (E, F))))
+    Wg, Wu, Wd = izb.Weight(qt, g, F, E, n_mats=NE), izb.Weight(qt, u, F, E, n_mats=NE), izb.Weight(qt, d, E, F, n_mats=NE)
+    x = torch.from_numpy(S.make_act(T, E, 9)).cuda() * 0.02
+    aq, asc, _ = izb.quantize_act(x)
+    ids, wts, counts = izb.moe_route(torch.from_numpy(S.make_act(T, NE, 3)).cuda(), NU)
+    offs, tiles, mt, stok, swt, inv = izb.moe_sort(ids, wts, counts, TM)
+    h = izb.moe_gateup(Wg, Wu, aq, asc, tiles, mt, TM, stok, T * NU)
+    hq, hsc, _ = izb.quantize_act(h)
+    y = izb.moe_down(Wd, hq, hsc, tiles, mt, TM, swt, T * NU)
+    for e in range(NE):
+        for s in range(int(offs[e]), int(offs[e + 1])):
+            t = int(stok[s])
+            a, b = aq[t:t + 1].repeat(16, 1).contiguous(), asc[:, t:t + 1].repeat(1, 16).contiguous()
+            gate, up = (izb.gemm(W, a, b, M=1, impl=izb.GEMM_CORE, mat=e)[0].double() for W in (Wg, Wu))
+            want = gate / (1 + torch.exp(-gate)) * up
+            assert float((h[s] - want).abs().max() / want.abs().max()) < TOL
+            a, b = hq[s:s + 1].repeat(16, 1).contiguous(), hsc[:, s:s + 1].repeat(1, 16).contiguous()
+            want = float(swt[s]) * izb.gemm(Wd, a, b, M=1, impl=izb.GEMM_CORE, mat=e)[0].double()
+            assert float((y[s] - want).abs().max() / want.abs().max()) < TOL
+    assert izb.device_status(0) == 0
+    for W in (Wg, Wu, Wd):
+        W.close()
