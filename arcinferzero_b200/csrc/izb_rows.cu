@@ -222,8 +222,9 @@ struct RQ6K {
             const float2 s = hd[b * 16 + g + 8 * r];
             // (both products and their sum are integers below 2^24: exact)
             const f2 v = f2_fma(f2_of(s.x, s.x), unmagic(d, r), f2_mul(f2_of(s.y, s.y), unmagic(e, r)));
-            // (the product as an fma with -0: a multiply would be fused with the addition behind it, one rounding instead of two)
-            acc[b][r] = f2_add(acc[b][r], f2_fma(f2_mul(xs[4 * b], wd[r]), v, 0x8000000080000000ull));
+            // (product and addition on single values: of packed ones ptxas makes one fma, one rounding instead of two)
+            const f2 f = f2_mul(xs[4 * b], wd[r]);
+            acc[b][r] = f2_of(__fadd_rn(f2_get(acc[b][r], 0), __fmul_rn(f2_get(f, 0), f2_get(v, 0))), __fadd_rn(f2_get(acc[b][r], 1), __fmul_rn(f2_get(f, 1), f2_get(v, 1))));
           }
         }
       }
@@ -270,6 +271,13 @@ struct Ring {
   }
   __device__ __forceinline__ void next() {
     if (++get == slots) { get = 0; parity ^= 1; }
+  }
+  // after a wait that ran out: the other requests in flight, with the same limit (their slots must outlive them)
+  __device__ __forceinline__ void drain() {
+    for (int s = 1; s < slots; ++s) {
+      next();
+      wait();
+    }
   }
 };
 
@@ -345,7 +353,10 @@ __device__ __forceinline__ bool accumulate(Ring<F>& ring, float2* hd, const Acts
   for (int p = 0; p < F::kPieces; ++p) acc[p][0] = acc[p][1] = 0ull;
   for (int s = part; s < nsb; s += F::kSubs) {
     const unsigned char* chunk = ring.wait();
-    if (!chunk) return false;
+    if (!chunk) {
+      ring.drain();
+      return false;
+    }
     if (F::kPrep) {
       F::prep(chunk, hd, lane);
       __syncwarp();
@@ -402,13 +413,13 @@ __device__ __forceinline__ void reduce_tile(f2 (&acc)[F::kPieces][2], unsigned c
       for (int r = 0; r < 2; ++r) acc[p][r] = f2_add(acc[p][r], acc[p + h][r]);
 }
 
-// C[token][c_off + row] (= or +=) for T tokens.  The grid walks groups of NW / kSubs row tiles.
-template <class F, int NW>
-__global__ void __launch_bounds__(NW * 32, NW == 8 ? 2 : 1) rows_kernel(const __grid_constant__ CUtensorMap tm, int wrow0, int N, int K, const int8_t* __restrict__ aq,
-                                                                        const float* __restrict__ asc, int T, int Mp, float* __restrict__ C, int ldc, int c_off, int acc_mode,
-                                                                        int slots, uint32_t* err) {
+// C[token][c_off + row] (= or +=) for T tokens.  The grid walks groups of (warps / kSubs) row tiles.
+template <class F>
+__global__ void __launch_bounds__(512, 1) rows_kernel(const __grid_constant__ CUtensorMap tm, int wrow0, int N, int K, const int8_t* __restrict__ aq,
+                                                      const float* __restrict__ asc, int T, int Mp, float* __restrict__ C, int ldc, int c_off, int acc_mode, int slots,
+                                                      uint32_t* err) {
   extern __shared__ __align__(1024) unsigned char smem[];
-  constexpr int kPer = NW / F::kSubs;
+  const int NW = blockDim.x >> 5, kPer = NW / F::kSubs;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int part = warp % F::kSubs, mine = warp / F::kSubs, nsb = K >> 8, groups = ((N + 15) / 16 + kPer - 1) / kPer;
   unsigned char* rings = smem + act_bytes<F>(K, T);
@@ -456,17 +467,19 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 2 : 1) rows_kernel(const __
   }
 }
 
-// Mixture of experts: one CTA = a tile (up to 8 slots of one expert) x a group of row tiles.
+// Mixture of experts: an item is a tile (up to 8 slots of one expert) x a group of row tiles; how many tiles there are is known on the
+// device only.  A CTA takes a run of consecutive items, which mostly share their tile: the activations are staged once per tile, and
+// the rings run on from item to item.  (One CTA per possible item left at once for most of them: 2048 x 768 of 128 experts, 32 slots,
+// 8448 CTAs for some 1800 items: gate/up, quantise and down took 90 us, in this form 64 us.)
 // gate/up (pair): h[slot][N] = silu(x Wg^T) * (x Wu^T), token rows through stok; down: y[slot][N] = swt * (hq Wd^T).
-template <class F, int NW>
-__global__ void __launch_bounds__(NW * 32, NW == 8 ? 2 : 1) moe_rows_kernel(const __grid_constant__ CUtensorMap tg, const __grid_constant__ CUtensorMap tu, int pair, int N, int K,
-                                                                            const int8_t* __restrict__ aq, const float* __restrict__ asc, int Mp,
-                                                                            const int32_t* __restrict__ tiles, const int32_t* __restrict__ stok,
-                                                                            const float* __restrict__ swt, float* __restrict__ out, int slots, uint32_t* err) {
+template <class F>
+__global__ void __launch_bounds__(512, 1) moe_rows_kernel(const __grid_constant__ CUtensorMap tg, const __grid_constant__ CUtensorMap tu, int pair, int N, int K,
+                                                          const int8_t* __restrict__ aq, const float* __restrict__ asc, int Mp, const int32_t* __restrict__ tiles,
+                                                          const int32_t* __restrict__ stok, const float* __restrict__ swt, float* __restrict__ out, int slots, uint32_t* err) {
   extern __shared__ __align__(1024) unsigned char smem[];
-  constexpr int kPer = NW / F::kSubs;
+  const int NW = blockDim.x >> 5, kPer = NW / F::kSubs;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int part = warp % F::kSubs, mine = warp / F::kSubs, nsb = K >> 8;
+  const int part = warp % F::kSubs, mine = warp / F::kSubs, nsb = K >> 8, groups = ((N + 15) / 16 + kPer - 1) / kPer;
   unsigned char* rings = smem + act_bytes<F>(K, 8);
   unsigned char* xch = rings + (size_t)NW * slots * Ring<F>::kSlot;
   Ring<F> ring;
@@ -479,95 +492,123 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 2 : 1) moe_rows_kernel(cons
   ring.init(lane);
   pdl_launch_next();
   pdl_wait();
-  const int ti = blockIdx.y;
-  if (ti >= tiles[0]) return;  // uniform over the CTA
-  const int e = tiles[1 + 3 * ti], s0 = tiles[2 + 3 * ti], T = tiles[3 + 3 * ti];
-  const int tile = blockIdx.x * kPer + mine;
-  int pm = 0, ps = part;  // matrix (gate, up) and superblock still to request
+  const long long items = (long long)tiles[0] * groups;
+  const int lo = (int)(items * blockIdx.x / gridDim.x), hi = (int)(items * (blockIdx.x + 1) / gridDim.x);
+  // chunks still to request: superblock `ps` of matrix `pm` (gate, up) of item `pi`, whose expert is `pe`
+  int pi = lo, pm = 0, ps = part, pe = lo < hi ? tiles[1 + 3 * (lo / groups)] : 0;
   auto request = [&]() {
-    if (pm > pair || part >= nsb) return;
-    ring.fill(pm ? &tu : &tg, ps, e * N + tile * 16, lane);
-    if ((ps += F::kSubs) >= nsb) { ps = part; ++pm; }
+    if (pi >= hi || part >= nsb) return;
+    ring.fill(pm ? &tu : &tg, ps, pe * N + (pi % groups * kPer + mine) * 16, lane);
+    if ((ps += F::kSubs) < nsb) return;
+    ps = part;
+    if (pm++ < pair) return;
+    pm = 0;
+    if (++pi < hi && pi % groups == 0) pe = tiles[1 + 3 * (pi / groups)];
   };
   for (int s = 0; s < slots; ++s) request();
-  const Acts acts = stage_acts<F>(smem, K, T, aq, asc, Mp, g, t, [&](int j) { return stok ? stok[s0 + j] : s0 + j; });
-  __syncthreads();
-  float first[4];
+  Acts acts;
+  int s0 = 0, T = 0;
   bool ok = true;
-  for (int m = 0; m <= pair; ++m) {
-    f2 acc[F::kPieces][2];
-    if (ok) ok = accumulate<F>(ring, reinterpret_cast<float2*>(xch + (size_t)warp * kXch), acts, part, nsb, lane, acc, request);
-    if (!ok) {  // (bounded wait gave up: nothing of this CTA is stored any more)
-      if (lane == 0) atomicOr(err, 64u);
-      *gave_up = 1;
+  for (int it = lo; it < hi; ++it) {
+    if (it == lo || it % groups == 0) {
+      if (it != lo) __syncthreads();  // the last tile's activations have been read
+      s0 = tiles[2 + 3 * (it / groups)];
+      T = tiles[3 + 3 * (it / groups)];
+      acts = stage_acts<F>(smem, K, T, aq, asc, Mp, g, t, [&](int j) { return stok ? stok[s0 + j] : s0 + j; });
+      __syncthreads();
     }
-    reduce_tile<F>(acc, xch, warp, lane);
-    if (m < pair) {
+    float first[4];
+    for (int m = 0; m <= pair; ++m) {
+      f2 acc[F::kPieces][2];
+      if (ok) ok = accumulate<F>(ring, reinterpret_cast<float2*>(xch + (size_t)warp * kXch), acts, part, nsb, lane, acc, request);
+      if (!ok) {  // (bounded wait gave up: nothing of this CTA is stored any more)
+        if (lane == 0) atomicOr(err, 64u);
+        *gave_up = 1;
+      }
+      reduce_tile<F>(acc, xch, warp, lane);
+      if (m < pair) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) first[i] = f2_get(acc[0][i >> 1], i & 1);
-    } else if (part == 0 && !*gave_up) {
+        for (int i = 0; i < 4; ++i) first[i] = f2_get(acc[0][i >> 1], i & 1);
+      } else if (part == 0 && !*gave_up) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int n = tile * 16 + g + 8 * (i >> 1), slot = 2 * t + (i & 1);
-        if (n < N && slot < T) {
-          const float v = f2_get(acc[0][i >> 1], i & 1);
-          out[(size_t)(s0 + slot) * N + n] = pair ? __fmul_rn(__fdiv_rn(first[i], __fadd_rn(1.0f, expf(-first[i]))), v) : __fmul_rn(swt[s0 + slot], v);
+        for (int i = 0; i < 4; ++i) {
+          const int n = (it % groups * kPer + mine) * 16 + g + 8 * (i >> 1), slot = 2 * t + (i & 1);
+          if (n < N && slot < T) {
+            const float v = f2_get(acc[0][i >> 1], i & 1);
+            out[(size_t)(s0 + slot) * N + n] = pair ? __fmul_rn(__fdiv_rn(first[i], __fadd_rn(1.0f, expf(-first[i]))), v) : __fmul_rn(swt[s0 + slot], v);
+          }
         }
       }
     }
   }
 }
 
-constexpr size_t kHalfSm = 113 * 1024, kWholeSm = 226 * 1024;
-// most slots (up to four: deeper rings gain nothing) that fit `budget`
+// Warps per CTA, CTAs per SM and ring slots (2 to 4: deeper rings gain nothing) for `tiles` row tiles.  What hides the latency is chunks
+// in flight and at work, so of all splits that fit: the most warps x (slots + 1) that have work, averaged over the rounds the grid
+// needs; of equals the smaller CTA.  (Four warps suit small matrices -- 1024 x 3072 Q6_K, 5 rows: 4.5 us against 5.2 with eight and
+// 7.9 with sixteen --, sixteen share one copy of large activations: 128000 x 4096 Q4_K, 8 rows: 89 us against 102 with four.)
+constexpr size_t kSmemPerSm = 226 * 1024;
+struct Split {
+  int warps, ctas, slots;  // slots 0: the activations leave no room
+};
 template <class F>
-int rows_slots(int K, int T, int nw, size_t budget) {
-  int s = 4;
-  while (s > 0 && rows_smem<F>(K, T, nw, s) > budget) --s;
-  return s;
+Split pick_split(int K, int T, int tiles, int sms) {
+  Split best = {0, 0, 0};
+  double most = 0;
+  for (int nw = 4; nw <= 16; nw *= 2) {
+    const int groups = (tiles + nw / F::kSubs - 1) / (nw / F::kSubs);
+    for (int c = 1; c * nw <= 16; ++c) {
+      const size_t room = kSmemPerSm / c - (c > 1 ? 1024 : 0);
+      int slots = 4;
+      while (slots >= 2 && rows_smem<F>(K, T, nw, slots) > room) --slots;
+      if (slots < 2) break;
+      const int rounds = (groups + c * sms - 1) / (c * sms);
+      const double at_work = (double)groups * nw * (slots + 1) / rounds;
+      if (at_work > most * 1.001) {
+        most = at_work;
+        best = {nw, c, slots};
+      }
+    }
+  }
+  return best;
 }
 
-template <class F, int NW>
-int launch_rows(const izb_weight* w, int mat, const int8_t* aq, const float* asc, int T, int Mp, float* C, int ldc, int c_off, int acc, int slots, cudaStream_t st) {
-  IZB_SMEM_OPTIN((rows_kernel<F, NW>), kWholeSm, w->device);
-  constexpr int kPer = NW / F::kSubs;
-  const size_t smem = rows_smem<F>(w->K, T, NW, slots);
-  const int groups = ((w->N + 15) / 16 + kPer - 1) / kPer, most = izb_sm_count(w->device) * (smem <= kHalfSm ? 2 : 1), grid = groups < most ? groups : most;
+template <class F>
+int rows_of(const izb_weight* w, int mat, const int8_t* aq, const float* asc, int T, int Mp, float* C, int ldc, int c_off, int acc, cudaStream_t st) {
+  const int sms = izb_sm_count(w->device), tiles = (w->N + 15) / 16;
+  const Split sp = pick_split<F>(w->K, T, tiles, sms);
+  if (!sp.slots) {  // half the tokens at a time, the second pass finding part of the weights in L2
+    if (T < 2) return 1;
+    const int h = (T + 1) / 2;
+    if (const int rc = rows_of<F>(w, mat, aq, asc, h, Mp, C, ldc, c_off, acc, st)) return rc;
+    return rows_of<F>(w, mat, aq + (size_t)h * w->K, asc + h, T - h, Mp, C + (size_t)h * ldc, ldc, c_off, acc, st);
+  }
+  IZB_SMEM_OPTIN((rows_kernel<F>), kSmemPerSm, w->device);
+  const int groups = (tiles + sp.warps / F::kSubs - 1) / (sp.warps / F::kSubs), grid = groups < sms * sp.ctas ? groups : sms * sp.ctas;
   uint32_t* err = izb_device_error_word(w->device);
   if (!err) IZB_FAIL(IZB_ERR_NOMEM, "gemv: no device error word");
   CUtensorMap tm;
   memcpy(&tm, w->tmap16_raw, sizeof tm);
-  IZB_LAUNCH("gemv_rows", st, izb_launch_pdl(rows_kernel<F, NW>, grid, NW * 32, smem, st, tm, mat * w->N, w->N, w->K, aq, asc, T, Mp, C, ldc, c_off, acc, slots, err));
+  IZB_LAUNCH("gemv_rows", st, izb_launch_pdl(rows_kernel<F>, grid, sp.warps * 32, rows_smem<F>(w->K, T, sp.warps, sp.slots), st, tm, mat * w->N, w->N, w->K, aq, asc, T, Mp, C, ldc,
+                                             c_off, acc, sp.slots, err));
   return IZB_OK;
-}
-// Two CTAs of eight warps per SM where the activations leave room for rings, else one of sixteen, else one of eight; activations that do
-// not fit even there (8 rows of K = 17408) go half the tokens at a time, the second pass finding part of the weights in L2.
-template <class F>
-int rows_of(const izb_weight* w, int mat, const int8_t* aq, const float* asc, int T, int Mp, float* C, int ldc, int c_off, int acc, cudaStream_t st) {
-  if (const int s = rows_slots<F>(w->K, T, 8, kHalfSm); s >= 2) return launch_rows<F, 8>(w, mat, aq, asc, T, Mp, C, ldc, c_off, acc, s, st);
-  if (const int s = rows_slots<F>(w->K, T, 16, kWholeSm); s >= 2) return launch_rows<F, 16>(w, mat, aq, asc, T, Mp, C, ldc, c_off, acc, s, st);
-  if (const int s = rows_slots<F>(w->K, T, 8, kWholeSm); s >= 2) return launch_rows<F, 8>(w, mat, aq, asc, T, Mp, C, ldc, c_off, acc, s, st);
-  if (T < 2) return 1;
-  const int h = (T + 1) / 2;
-  if (const int rc = rows_of<F>(w, mat, aq, asc, h, Mp, C, ldc, c_off, acc, st)) return rc;
-  return rows_of<F>(w, mat, aq + (size_t)h * w->K, asc + h, T - h, Mp, C + (size_t)h * ldc, ldc, c_off, acc, st);
 }
 template <class F>
 int moe_rows_of(const izb_weight* wg, const izb_weight* wu, const int8_t* aq, const float* asc, int Mp, const int32_t* tiles, int max_tiles, const int32_t* stok, const float* swt,
                 float* out, cudaStream_t st) {
-  int slots = rows_slots<F>(wg->K, 8, 8, kHalfSm);
-  if (slots < 2) slots = rows_slots<F>(wg->K, 8, 8, kWholeSm);
-  if (slots < 2) return 1;
-  IZB_SMEM_OPTIN((moe_rows_kernel<F, 8>), kWholeSm, wg->device);
-  constexpr int kPer = 8 / F::kSubs;
+  const int sms = izb_sm_count(wg->device), row_tiles = (wg->N + 15) / 16;
+  const long long most = (long long)max_tiles * row_tiles;
+  if (most > (1ll << 30)) return 1;
+  const Split sp = pick_split<F>(wg->K, 8, (int)most, sms);
+  if (!sp.slots) return 1;
+  IZB_SMEM_OPTIN((moe_rows_kernel<F>), kSmemPerSm, wg->device);
   uint32_t* err = izb_device_error_word(wg->device);
   if (!err) IZB_FAIL(IZB_ERR_NOMEM, "moe: no device error word");
   CUtensorMap tg, tu;
   memcpy(&tg, wg->tmap16_raw, sizeof tg);
   memcpy(&tu, (wu ? wu : wg)->tmap16_raw, sizeof tu);
-  dim3 grid(((wg->N + 15) / 16 + kPer - 1) / kPer, max_tiles);
-  IZB_LAUNCH(wu ? "moe_gateup" : "moe_down", st, izb_launch_pdl(moe_rows_kernel<F, 8>, grid, 256, rows_smem<F>(wg->K, 8, 8, slots), st, tg, tu, wu ? 1 : 0, wg->N, wg->K, aq, asc, Mp,
-                                                               tiles, stok, swt, out, slots, err));
+  IZB_LAUNCH(wu ? "moe_gateup" : "moe_down", st, izb_launch_pdl(moe_rows_kernel<F>, sms * sp.ctas, sp.warps * 32, rows_smem<F>(wg->K, 8, sp.warps, sp.slots), st, tg, tu, wu ? 1 : 0,
+                                                               wg->N, wg->K, aq, asc, Mp, tiles, stok, swt, out, sp.slots, err));
   return IZB_OK;
 }
 
