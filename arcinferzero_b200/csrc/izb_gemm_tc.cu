@@ -974,7 +974,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
       if (!ok || kDots || !row_ok || *abort_flag) continue;
       const int ncol = min(64, p.N - n0 - half * 64);  // valid columns of this thread (a multiple of 16; <= 0: none)
       if (ncol <= 0) continue;
-      if (p.acc == 3 && p.n_split == 1) {
+      if (p.acc == 3) {
         // Gate and up projections in one weight whose rows alternate in groups of 32 (izb_weight_create_gateup): this
         // thread's 64 columns are 32 gate outputs followed by the 32 up outputs of the same FFN rows, so the SwiGLU product
         // up * silu(gate) (zero/kernels/gemm.cl:562-565) is formed in registers and only the F-wide result is stored.
@@ -997,11 +997,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
         }
         continue;
       }
-      // a part of the K range goes to the partial sums as it is (split_reduce_kernel applies the store mode)
       float* cp = p.n_split > 1 ? p.part + ((size_t)it.ks * p.M + out_row) * p.N + n0 + half * 64
                                 : p.C + (size_t)out_row * p.ldc + p.c_off + n0 + half * 64;
       const size_t ld = p.n_split > 1 ? (size_t)p.N : (size_t)p.ldc;
-      const int acc = p.n_split > 1 ? 0 : p.acc;
+      const int acc = p.acc;
       const float rs = p.rowscale ? p.rowscale[out_row] : 1.0f;
       // plain store (with or without the row factor), 32-byte aligned rows: eight stores of one full 32-byte sector each
       // per thread
@@ -1054,39 +1053,21 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
 }
 
 // ---------------------------------------------------------------------------------------------- partial sums of a cut K range
-// out (store mode `acc`) = part 0 + part 1 + ... in order.  One thread per four output columns.
+// C = part 0 + part 1 + ... in order.  One thread per four output columns.
 __global__ void __launch_bounds__(256) split_reduce_kernel(const float* __restrict__ part, int n_split, int M, int N, float* __restrict__ C, int ldc, int c_off,
-                                                           int acc, const uint32_t* __restrict__ part_bad) {
+                                                           const uint32_t* __restrict__ part_bad) {
   pdl_launch_next();
   pdl_wait();
   if (*part_bad) return;
-  const int n_out = acc == 3 ? N / 2 : N, c = (blockIdx.x * 256 + threadIdx.x) * 4, m = blockIdx.y;
-  if (c >= n_out) return;
-  auto sum = [&](int col) -> float4 {
-    const float* src = part + (size_t)m * N + col;
-    float4 v = *reinterpret_cast<const float4*>(src);
-    for (int k = 1; k < n_split; ++k) {
-      const float4 o = *reinterpret_cast<const float4*>(src + (size_t)k * M * N);
-      v.x = __fadd_rn(v.x, o.x); v.y = __fadd_rn(v.y, o.y); v.z = __fadd_rn(v.z, o.z); v.w = __fadd_rn(v.w, o.w);
-    }
-    return v;
-  };
-  float4* dst = reinterpret_cast<float4*>(C + (size_t)m * ldc + c_off + c);
-  float4 v;
-  if (acc == 3) {  // (groups of 32 gate and 32 up columns, see the GEMM's store mode 3)
-    const float4 g = sum(64 * (c >> 5) + (c & 31)), u = sum(64 * (c >> 5) + 32 + (c & 31));
-    v = make_float4(swiglu_mul(g.x, u.x), swiglu_mul(g.y, u.y), swiglu_mul(g.z, u.z), swiglu_mul(g.w, u.w));
-  } else {
-    v = sum(c);
-    if (acc == 1) {
-      const float4 o = *dst;
-      v.x = __fadd_rn(v.x, o.x); v.y = __fadd_rn(v.y, o.y); v.z = __fadd_rn(v.z, o.z); v.w = __fadd_rn(v.w, o.w);
-    } else if (acc == 2) {
-      const float4 o = *dst;
-      v = make_float4(swiglu_mul(o.x, v.x), swiglu_mul(o.y, v.y), swiglu_mul(o.z, v.z), swiglu_mul(o.w, v.w));
-    }
+  const int c = (blockIdx.x * 256 + threadIdx.x) * 4, m = blockIdx.y;
+  if (c >= N) return;
+  const float* src = part + (size_t)m * N + c;
+  float4 v = *reinterpret_cast<const float4*>(src);
+  for (int k = 1; k < n_split; ++k) {
+    const float4 o = *reinterpret_cast<const float4*>(src + (size_t)k * M * N);
+    v.x = __fadd_rn(v.x, o.x); v.y = __fadd_rn(v.y, o.y); v.z = __fadd_rn(v.z, o.z); v.w = __fadd_rn(v.w, o.w);
   }
-  *dst = v;
+  *reinterpret_cast<float4*>(C + (size_t)m * ldc + c_off + c) = v;
 }
 
 // ---------------------------------------------------------------------------------------------- host side
@@ -1140,7 +1121,9 @@ int tc_grid(int device, int n_work) {
 }
 
 // Parts the K range of every output tile is cut into, when the tiles alone would leave more than half the SMs idle: as many
-// as fill them once, each at least one superblock.  The parts' sums are at most one 64 KB tile per SM.
+// as fill them once, each at least one superblock.  The parts' sums are at most one 64 KB tile per SM.  Plain stores only: sums cut
+// in parts are rounded in other places, and what the other store modes write (the residual, the SwiGLU product) is quantised to int8
+// next, where a last bit can become a whole step.
 int tc_split(int device, int n_items, int nsb) {
   const int s = izb_sm_budget(device) / (n_items > 0 ? n_items : 1);
   return s < 2 ? 1 : s < nsb ? s : nsb;
@@ -1188,14 +1171,14 @@ int run_tc_on(const izb_weight* w, int mat, const int8_t* aq, const float* asc, 
   p.err = err;
   p.n_mtiles = n_tiles_grid;
   const int n_items = (w->N + BN - 1) / BN * n_tiles_grid;
-  p.n_split = split_ws && !tiles && !dots ? tc_split(w->device, n_items, K / 256) : 1;
+  p.n_split = split_ws && acc == 0 && !tiles && !dots ? tc_split(w->device, n_items, K / 256) : 1;
   p.part = split_ws;
   p.part_bad = split_flag(split_ws, w->device);
   dim3 grid(tc_grid(w->device, n_items * p.n_split));
   if (int rc = launch_tc_of(w, p, grid, st)) return rc;
   if (p.n_split > 1) {
-    dim3 rg(((acc == 3 ? w->N / 2 : w->N) / 4 + 255) / 256, M_store);
-    IZB_LAUNCH("split_reduce", st, izb_launch_pdl(split_reduce_kernel, rg, 256, 0, st, split_ws, p.n_split, M_store, w->N, C, ldc, c_off, acc, p.part_bad));
+    dim3 rg((w->N / 4 + 255) / 256, M_store);
+    IZB_LAUNCH("split_reduce", st, izb_launch_pdl(split_reduce_kernel, rg, 256, 0, st, split_ws, p.n_split, M_store, w->N, C, ldc, c_off, p.part_bad));
   }
   return IZB_OK;
 }
