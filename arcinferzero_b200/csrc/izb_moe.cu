@@ -32,10 +32,18 @@ __device__ __forceinline__ float route_key_value(unsigned long long k) {
   return __uint_as_float((u & 0x80000000u) ? (u & 0x7FFFFFFFu) : ~u);
 }
 
-__global__ void __launch_bounds__(256) moe_route_kernel(const float* __restrict__ logits, int ldl, int T, int NE, int NU,
-                                                        int32_t* __restrict__ ids, float* __restrict__ wts,
-                                                        int32_t* __restrict__ counts, float* __restrict__ sgate) {
-  const int token = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+// `counts` is zeroed here when one CTA takes all tokens (a decode step: a launch less), else before.
+constexpr int kRouteWarps = 16;
+__global__ void __launch_bounds__(kRouteWarps * 32) moe_route_kernel(const float* __restrict__ logits, int ldl, int T, int NE, int NU,
+                                                                     int32_t* __restrict__ ids, float* __restrict__ wts,
+                                                                     int32_t* __restrict__ counts, float* __restrict__ sgate) {
+  const int token = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  pdl_launch_next();
+  pdl_wait();
+  if (gridDim.x == 1) {
+    for (int e = threadIdx.x; e < NE; e += blockDim.x) counts[e] = 0;
+    __syncthreads();
+  }
   if (token >= T) return;
   const float* row = logits + (size_t)token * ldl;
   // the shared expert's gate: the sigmoid of the logit after the experts' (SGATE, zero/kernels/moe.cl:44,88)
@@ -82,63 +90,77 @@ __global__ void __launch_bounds__(256) moe_route_kernel(const float* __restrict_
   }
 }
 
-// One thread per expert: offsets (exclusive scan, serial: NE is a few hundred) and the expert's tiles.
+// The counting sort, one CTA per expert: each sums the slots and tiles of the experts before its own (at most four counts per
+// thread: cheaper than a launch of its own for the scan, which took 18 us of a 4-token step as a serial loop), writes its tiles, and gives
+// its pairs consecutive slots in increasing pair index (a deterministic atomic_inc order).
 // With an expert range [e0, e1) (the expert-parallel split, tp_moe_mask, zero/kernels/tp.cl:61-64) the other experts count
-// as empty and a tile names its expert by its index in this rank's stack, e - e0.
-__global__ void moe_scan_kernel(const int32_t* __restrict__ counts, int NE, int TM, int32_t* __restrict__ offs,
-                                int32_t* __restrict__ tiles, int max_tiles, int e0, int e1) {
-  const int e = threadIdx.x;
-  int off = 0, toff = 0;
-  for (int i = 0; i < e && i < NE; ++i) {
-    const int ci = (i >= e0 && i < e1) ? counts[i] : 0;
-    off += ci;
-    toff += (ci + TM - 1) / TM;
-  }
-  if (e < NE) {
-    const int c = (e >= e0 && e < e1) ? counts[e] : 0, nt = (c + TM - 1) / TM;
-    offs[e] = off;
-    for (int i = 0; i < nt; ++i) {
-      if (toff + i >= max_tiles) break;
-      int32_t* tp = tiles + 1 + 3 * (toff + i);
-      tp[0] = e - e0;
-      tp[1] = off + i * TM;
-      tp[2] = min(TM, c - i * TM);
-    }
-    if (e == NE - 1) {
-      offs[NE] = off + c;
-      tiles[0] = min(toff + nt, max_tiles);
-    }
-  }
-}
-
-// One CTA per expert: its pairs in increasing pair index take consecutive slots (a deterministic atomic_inc order).
-// A thread looks at four consecutive pairs per pass (one 128-bit load), so a pass covers 1024 pairs: an exclusive scan of
-// the per-thread counts over the warp (shuffles) and over the eight warps (shared memory, double-buffered so that one
-// barrier per pass is enough) gives every pair of the expert its slot.
-__global__ void __launch_bounds__(256) moe_scatter_kernel(const int32_t* __restrict__ ids, const float* __restrict__ wts, int n,
-                                                          int NU, const int32_t* __restrict__ offs, int32_t* __restrict__ stok,
-                                                          float* __restrict__ swt, int32_t* __restrict__ inv, int e0, int e1) {
-  __shared__ int s_warp[2][8];
+// as empty and a tile names its expert by its index in this rank's stack, e - e0; their pairs get no slot (tp_moe_scatter,
+// zero/kernels/tp.cl:67-78).  The last CTA also writes the totals and zeroes the unused tail of the tile list.
+//
+// A thread looks at kPairs consecutive pairs per pass, the next pass's loads in flight meanwhile; an exclusive scan of the per-thread
+// counts over the warp (shuffles) and over the eight warps (shared memory, double-buffered so that one barrier per pass is enough)
+// gives every pair of the expert its slot.  (A pass is a chain of load, scan and barrier: with four pairs per thread 32768 pairs
+// were 32 of them, 38 us.)
+constexpr int kPairs = 16;
+__global__ void __launch_bounds__(256) moe_sort_kernel(const int32_t* __restrict__ ids, const float* __restrict__ wts, const int32_t* __restrict__ counts, int n, int NU,
+                                                       int NE, int TM, int32_t* __restrict__ offs, int32_t* __restrict__ tiles, int max_tiles, int32_t* __restrict__ stok,
+                                                       float* __restrict__ swt, int32_t* __restrict__ inv, int e0, int e1) {
+  __shared__ int s_warp[2][8], s_off[8], s_tile[8];
   const int e = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (e < e0 || e >= e1) {  // another rank's expert: its pairs get no slot (tp_moe_scatter, zero/kernels/tp.cl:67-78)
-    for (int i = threadIdx.x; i < n; i += blockDim.x)
-      if (ids[i] == e) inv[i] = -1;
-    return;
-  }
-  int base = offs[e];  // (every thread keeps the running base: no broadcast needed)
-  int buf = 0;
-  for (int i0 = 0; i0 < n; i0 += 1024, buf ^= 1) {
-    const int i = i0 + 4 * threadIdx.x;
-    int4 v = make_int4(-1, -1, -1, -1);
-    if (i + 3 < n) {
-      v = *reinterpret_cast<const int4*>(ids + i);
-    } else {
-      if (i < n) v.x = ids[i];
-      if (i + 1 < n) v.y = ids[i + 1];
-      if (i + 2 < n) v.z = ids[i + 2];
+  pdl_launch_next();
+  pdl_wait();
+  int4 v[kPairs / 4];
+  auto load = [&](int i) {
+#pragma unroll
+    for (int j = 0; j < kPairs / 4; ++j, i += 4) {
+      v[j] = make_int4(-1, -1, -1, -1);
+      if (i + 3 < n) {
+        v[j] = *reinterpret_cast<const int4*>(ids + i);
+      } else {
+        if (i < n) v[j].x = ids[i];
+        if (i + 1 < n) v[j].y = ids[i + 1];
+        if (i + 2 < n) v[j].z = ids[i + 2];
+      }
     }
-    const int m0 = v.x == e, m1 = v.y == e, m2 = v.z == e, m3 = v.w == e;
-    const int cnt = m0 + m1 + m2 + m3;
+  };
+  load(kPairs * threadIdx.x);
+  auto count_of = [&](int i) { return i >= e0 && i < e1 ? counts[i] : 0; };
+  int off = 0, toff = 0;
+  for (int i = threadIdx.x; i < e; i += blockDim.x) {
+    const int c = count_of(i);
+    off += c;
+    toff += (c + TM - 1) / TM;
+  }
+  off = __reduce_add_sync(0xFFFFFFFFu, off);
+  toff = __reduce_add_sync(0xFFFFFFFFu, toff);
+  if (lane == 0) { s_off[warp] = off; s_tile[warp] = toff; }
+  __syncthreads();
+  off = toff = 0;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) { off += s_off[w]; toff += s_tile[w]; }
+  const int mine = count_of(e), nt = (mine + TM - 1) / TM;
+  for (int i = threadIdx.x; i < nt && toff + i < max_tiles; i += blockDim.x) {
+    int32_t* tp = tiles + 1 + 3 * (toff + i);
+    tp[0] = e - e0;
+    tp[1] = off + i * TM;
+    tp[2] = min(TM, mine - i * TM);
+  }
+  if (threadIdx.x == 0) offs[e] = off;
+  if (e == NE - 1) {
+    const int used = min(toff + nt, max_tiles);
+    if (threadIdx.x == 0) { offs[NE] = off + mine; tiles[0] = used; }
+    for (int i = 3 * used + threadIdx.x; i < 3 * max_tiles; i += blockDim.x) tiles[1 + i] = 0;
+  }
+  const bool here = e >= e0 && e < e1;
+  int base = off;  // (every thread keeps the running base: no broadcast needed)
+  for (int i0 = 0, buf = 0; i0 < n; i0 += 256 * kPairs, buf ^= 1) {
+    const int i = i0 + kPairs * threadIdx.x;
+    int id[kPairs], cnt = 0;
+#pragma unroll
+    for (int j = 0; j < kPairs / 4; ++j) { id[4 * j] = v[j].x; id[4 * j + 1] = v[j].y; id[4 * j + 2] = v[j].z; id[4 * j + 3] = v[j].w; }
+#pragma unroll
+    for (int j = 0; j < kPairs; ++j) cnt += id[j] == e;
+    if (i0 + 256 * kPairs < n) load(i + 256 * kPairs);
     int incl = cnt;  // inclusive scan over the warp
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -155,10 +177,15 @@ __global__ void __launch_bounds__(256) moe_scatter_kernel(const int32_t* __restr
       total += c;
     }
     int s = base + before + incl - cnt;
-    if (m0) { stok[s] = i / NU; swt[s] = wts[i]; inv[i] = s; ++s; }
-    if (m1) { stok[s] = (i + 1) / NU; swt[s] = wts[i + 1]; inv[i + 1] = s; ++s; }
-    if (m2) { stok[s] = (i + 2) / NU; swt[s] = wts[i + 2]; inv[i + 2] = s; ++s; }
-    if (m3) { stok[s] = (i + 3) / NU; swt[s] = wts[i + 3]; inv[i + 3] = s; }
+    if (cnt) {
+#pragma unroll
+      for (int j = 0; j < kPairs; ++j)
+        if (id[j] == e) {
+          inv[i + j] = here ? s : -1;
+          if (here) { stok[s] = (i + j) / NU; swt[s] = wts[i + j]; }
+          ++s;
+        }
+    }
     base += total;
   }
 }
@@ -229,6 +256,8 @@ __global__ void __launch_bounds__(kWarps * 32) moe_down_kernel(const uint8_t* __
 __global__ void moe_combine_kernel(float* __restrict__ x, const float* __restrict__ y, const int32_t* __restrict__ inv, int T,
                                    int NU, int E, const float* __restrict__ sh, const float* __restrict__ sgate, int partial) {
   const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 4, t = blockIdx.x;  // (tokens on x: no 65535 limit)
+  pdl_launch_next();
+  pdl_wait();
   if (c >= E) return;
   float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
   for (int k = 0; k < NU; ++k) {
@@ -259,8 +288,9 @@ extern "C" int izb_moe_route_ex(const float* d_logits, int ldl, int T, int NE, i
   if (T < 1 || NE < 1 || NE > 32 * kMaxPerLane || NU < 1 || NU > 32 || NU > NE || ldl < NE + (d_sgate ? 1 : 0))
     IZB_FAIL(IZB_ERR_SHAPE, "moe_route: T=%d NE=%d NU=%d ldl=%d (NE <= 512, NU <= 32, ldl >= NE, + 1 with a shared-expert gate)", T, NE, NU, ldl);
   cudaStream_t st = (cudaStream_t)stream;
-  IZB_CUDA(cudaMemsetAsync(d_counts, 0, (size_t)NE * 4, st));
-  IZB_LAUNCH("moe_route", st, moe_route_kernel<<<(T + 7) / 8, 256, 0, st>>>(d_logits, ldl, T, NE, NU, d_ids, d_wts, d_counts, d_sgate));
+  const int warps = T <= kRouteWarps ? T : 8, grid = (T + warps - 1) / warps;
+  if (grid > 1) IZB_CUDA(cudaMemsetAsync(d_counts, 0, (size_t)NE * 4, st));
+  IZB_LAUNCH("moe_route", st, izb_launch_pdl(moe_route_kernel, grid, warps * 32, 0, st, d_logits, ldl, T, NE, NU, d_ids, d_wts, d_counts, d_sgate));
   return IZB_OK;
 }
 
@@ -278,8 +308,7 @@ extern "C" int izb_moe_sort_ex(const int32_t* d_ids, const float* d_wts, const i
   if (!izb_aligned(d_ids, 16)) IZB_FAIL(IZB_ERR_ALIGN, "moe_sort: ids must be 16-byte aligned (read four at a time)");
   if (max_tiles < (T * NU + TM - 1) / TM + NE) IZB_FAIL(IZB_ERR_LIMIT, "moe_sort: max_tiles = %d < %d (pairs/TM + NE)", max_tiles, (T * NU + TM - 1) / TM + NE);
   cudaStream_t st = (cudaStream_t)stream;
-  IZB_LAUNCH("moe_scan", st, moe_scan_kernel<<<1, 1024, 0, st>>>(d_counts, NE, TM, d_offs, d_tiles, max_tiles, e0, e1));
-  IZB_LAUNCH("moe_scatter", st, moe_scatter_kernel<<<NE, 256, 0, st>>>(d_ids, d_wts, T * NU, NU, d_offs, d_stok, d_swt, d_inv, e0, e1));
+  IZB_LAUNCH("moe_sort", st, izb_launch_pdl(moe_sort_kernel, NE, 256, 0, st, d_ids, d_wts, d_counts, T * NU, NU, NE, TM, d_offs, d_tiles, max_tiles, d_stok, d_swt, d_inv, e0, e1));
   return IZB_OK;
 }
 
@@ -337,7 +366,7 @@ extern "C" int izb_moe_combine_ex(float* d_x, const float* d_y, const int32_t* d
   if ((E / 4 + 127) / 128 > 65535) IZB_FAIL(IZB_ERR_LIMIT, "moe_combine: E = %d too wide", E);
   dim3 grid(T, (E / 4 + 127) / 128);
   IZB_LAUNCH("moe_combine", (cudaStream_t)stream,
-             moe_combine_kernel<<<grid, 128, 0, (cudaStream_t)stream>>>(d_x, d_y, d_inv, T, NU, E, d_sh, d_sgate, partial ? 1 : 0));
+             izb_launch_pdl(moe_combine_kernel, grid, 128, 0, (cudaStream_t)stream, d_x, d_y, d_inv, T, NU, E, d_sh, d_sgate, partial ? 1 : 0));
   return IZB_OK;
 }
 

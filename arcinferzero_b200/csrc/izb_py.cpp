@@ -288,7 +288,7 @@ FN(moe_sort) {
   const c10::Device dev = ids.device();
   const int T = (int)ids.size(0), NU = (int)ids.size(1), NE = (int)tensor(a[2]).size(0), TM = num(a[3]), e0 = num(a[4]), e1 = num(a[5]);
   const int S = T * NU, max_tiles = (TM > 0 ? (S + TM - 1) / TM : 0) + NE;
-  at::Tensor offs = empty({NE + 1}, at::kInt, dev), tiles = at::zeros({1 + 3 * (int64_t)max_tiles}, ids.options()), stok = empty({S}, at::kInt, dev),
+  at::Tensor offs = empty({NE + 1}, at::kInt, dev), tiles = empty({1 + 3 * (int64_t)max_tiles}, at::kInt, dev), stok = empty({S}, at::kInt, dev),
              swt = empty({S}, at::kFloat, dev), inv = empty({S}, at::kInt, dev);
   auto pi = [](at::Tensor& t) { return static_cast<int32_t*>(t.data_ptr()); };
   call(g.izb_moe_sort_ex_, ptr<int32_t>(a[0]), ptr<float>(a[1]), ptr<int32_t>(a[2]), T, NE, NU, TM, e0, e1, pi(offs), pi(tiles), max_tiles, pi(stok),
