@@ -73,6 +73,12 @@ __device__ __forceinline__ float f2_get(f2 a, int i) { return __uint_as_float((u
 __device__ __forceinline__ f2 unmagic(const int (&d)[4], int r) {
   return f2_add(f2_of(__int_as_float(d[2 * r]), __int_as_float(d[2 * r + 1])), 0xCB400000CB400000ull);
 }
+// c + the unsigned bytes of w . the signed bytes of x
+__device__ __forceinline__ int dot_u8(uint32_t w, uint32_t x, int c) {
+  int d;
+  asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(w), "r"(x), "r"(c));
+  return d;
+}
 // unsigned byte k of a word as f32: 0x4B000000 | byte is 2^23 + byte
 __device__ __forceinline__ float byte_f(uint32_t w, int k) { return __fsub_rn(__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440 + k)), 8388608.0f); }
 
@@ -92,18 +98,55 @@ struct Acts {
 struct RQ4K {
   static constexpr int SBB = 144, kPitch = 144, kSubs = 4, kPieces = 8;
   static constexpr bool kEx = true, kPrep = true;
-  static __device__ __forceinline__ void prep(const unsigned char* chunk, float2* hd, int lane) {
-    // lane <-> row lane / 2, blocks 4 (lane & 1) .. + 3: (d * sc, -dmin * mn); the sub-block scales and mins as bytes
-    // (get_scale_min_k4, src/quants.h:61-69).  Odd blocks meet 16 q: their d * sc is divided by 16.
-    const int row = lane >> 1, up = lane & 1;
+  // (d * sc, -dmin * mn) of a row's blocks 4 up .. + 3; the sub-block scales and mins as bytes (get_scale_min_k4,
+  // src/quants.h:61-69).  Odd blocks meet 16 q: their d * sc is divided by 16.
+  static __device__ __forceinline__ void header(const unsigned char* chunk, int row, int up, float2 (&o)[4]) {
     const uint4 h = *reinterpret_cast<const uint4*>(chunk + row * kPitch);
     const float2 d = __half22float2(*reinterpret_cast<const __half2*>(&h.x));
     const uint32_t sc = up ? (h.w & 0x0F0F0F0Fu) | ((h.y >> 2) & 0x30303030u) : h.y & 0x3F3F3F3Fu;
     const uint32_t mn = up ? ((h.w >> 4) & 0x0F0F0F0Fu) | ((h.z >> 2) & 0x30303030u) : h.z & 0x3F3F3F3Fu;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      const float a = __fmul_rn((k & 1) ? d.x * 0.0625f : d.x, byte_f(sc, k)), b = __fmul_rn(-d.y, byte_f(mn, k));
-      hd[(4 * up + k) * 16 + row] = make_float2(a, b);
+      o[k] = make_float2(__fmul_rn((k & 1) ? d.x * 0.0625f : d.x, byte_f(sc, k)), __fmul_rn(-d.y, byte_f(mn, k)));
+    }
+  }
+  static __device__ __forceinline__ void prep(const unsigned char* chunk, float2* hd, int lane) {
+    const int row = lane >> 1, up = lane & 1;
+    float2 h[4];
+    header(chunk, row, up, h);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) hd[(4 * up + k) * 16 + row] = h[k];
+  }
+  // The same products by dp4a: lane <-> row lane % 16 and pieces 4 up .. + 3 of the superblock (up = lane / 16), TT tokens of the T staged
+  template <int TT>
+  static __device__ __forceinline__ void dot(const unsigned char* chunk, const unsigned char* act, int nb, int T, int sb, int lane, float (&acc)[TT][kPieces / 2]) {
+    const int row = lane & 15, up = lane >> 4, b0 = 8 * sb + 4 * up;
+    float2 hd[4];
+    header(chunk, row, up, hd);
+    const float* sc = reinterpret_cast<const float*>(act + (size_t)nb * 32 * T) + b0 * 8;
+    const float* ex = reinterpret_cast<const float*>(act + (size_t)nb * 32 * T) + nb * 8 + b0 * 16;
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const uint4* w = reinterpret_cast<const uint4*>(chunk + row * kPitch + 16 + 64 * up + 32 * c);
+      const uint4 w0 = w[0], w1 = w[1];
+#pragma unroll
+      for (int j = 0; j < TT; ++j) {
+        if (j >= T) break;
+        const uint4 *l = reinterpret_cast<const uint4*>(act + (size_t)((b0 + 2 * c) * T + j) * 32), *h = l + 2 * T;
+        const uint4 l0 = l[0], l1 = l[1], h0 = h[0], h1 = h[1];  // (words of the two halves alternate)
+        const float* e = ex + 32 * c + j;
+        const float sl = sc[16 * c + j], sh = sc[16 * c + 8 + j];
+        int dl0 = 0, dl1 = 0, dh0 = 0, dh1 = 0;
+        dl0 = dot_u8(w0.x & 0x0F0F0F0Fu, l0.x, dl0); dl0 = dot_u8(w0.y & 0x0F0F0F0Fu, l0.z, dl0); dl0 = dot_u8(w0.z & 0x0F0F0F0Fu, l1.x, dl0); dl0 = dot_u8(w0.w & 0x0F0F0F0Fu, l1.z, dl0);
+        dl1 = dot_u8(w1.x & 0x0F0F0F0Fu, l0.y, dl1); dl1 = dot_u8(w1.y & 0x0F0F0F0Fu, l0.w, dl1); dl1 = dot_u8(w1.z & 0x0F0F0F0Fu, l1.y, dl1); dl1 = dot_u8(w1.w & 0x0F0F0F0Fu, l1.w, dl1);
+        dh0 = dot_u8(w0.x & 0xF0F0F0F0u, h0.x, dh0); dh0 = dot_u8(w0.y & 0xF0F0F0F0u, h0.z, dh0); dh0 = dot_u8(w0.z & 0xF0F0F0F0u, h1.x, dh0); dh0 = dot_u8(w0.w & 0xF0F0F0F0u, h1.z, dh0);
+        dh1 = dot_u8(w1.x & 0xF0F0F0F0u, h0.y, dh1); dh1 = dot_u8(w1.y & 0xF0F0F0F0u, h0.w, dh1); dh1 = dot_u8(w1.z & 0xF0F0F0F0u, h1.y, dh1); dh1 = dot_u8(w1.w & 0xF0F0F0F0u, h1.w, dh1);
+        const float2 a = hd[2 * c], b = hd[2 * c + 1];
+        const float p0 = __fmaf_rn(a.x, (float)dl0, __fmul_rn(a.y, e[0])), q0 = __fmaf_rn(b.x, (float)dh0, __fmul_rn(b.y, e[16]));
+        const float p1 = __fmaf_rn(a.x, (float)dl1, __fmul_rn(a.y, e[8])), q1 = __fmaf_rn(b.x, (float)dh1, __fmul_rn(b.y, e[24]));
+        acc[j][2 * c] = __fadd_rn(acc[j][2 * c], __fmaf_rn(sl, p0, __fmul_rn(sh, q0)));
+        acc[j][2 * c + 1] = __fadd_rn(acc[j][2 * c + 1], __fmaf_rn(sl, p1, __fmul_rn(sh, q1)));
+      }
     }
   }
   static __device__ __forceinline__ void mul(const unsigned char* chunk, const float2* hd, const Acts& a, int sb, int g, int t, f2 (&acc)[kPieces][2]) {
@@ -142,6 +185,31 @@ struct RQ80 {
   static constexpr int SBB = 272, kPitch = 272, kSubs = 2, kPieces = 16;
   static constexpr bool kEx = false, kPrep = false;
   static __device__ __forceinline__ void prep(const unsigned char*, float2*, int) {}
+  template <int TT>
+  static __device__ __forceinline__ void dot(const unsigned char* chunk, const unsigned char* act, int nb, int T, int sb, int lane, float (&acc)[TT][kPieces / 2]) {
+    const int row = lane & 15, up = lane >> 4, b0 = 8 * sb + 4 * up;
+    const uint2 hd = *reinterpret_cast<const uint2*>(chunk + row * kPitch + 8 * up);
+    const float* sc = reinterpret_cast<const float*>(act + (size_t)nb * 32 * T) + b0 * 8;
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      const uint4* w = reinterpret_cast<const uint4*>(chunk + row * kPitch + 16 + 128 * up + 32 * b);
+      const uint4 w0 = w[0], w1 = w[1];
+      const uint32_t hw = b < 2 ? hd.x : hd.y;
+      const float d = half_bits_to_float((b & 1) ? hw >> 16 : hw & 0xFFFFu);
+#pragma unroll
+      for (int j = 0; j < TT; ++j) {
+        if (j >= T) break;
+        const uint4* x = reinterpret_cast<const uint4*>(act + (size_t)((b0 + b) * T + j) * 32);
+        const uint4 x0 = x[0], x1 = x[1];  // (words of the two halves alternate)
+        int d0 = 0, d1 = 0;
+        d0 = __dp4a((int)w0.x, (int)x0.x, d0); d0 = __dp4a((int)w0.y, (int)x0.z, d0); d0 = __dp4a((int)w0.z, (int)x1.x, d0); d0 = __dp4a((int)w0.w, (int)x1.z, d0);
+        d1 = __dp4a((int)w1.x, (int)x0.y, d1); d1 = __dp4a((int)w1.y, (int)x0.w, d1); d1 = __dp4a((int)w1.z, (int)x1.y, d1); d1 = __dp4a((int)w1.w, (int)x1.w, d1);
+        const float sd = __fmul_rn(sc[8 * b + j], d);
+        acc[j][2 * b] = __fmaf_rn(sd, (float)d0, acc[j][2 * b]);
+        acc[j][2 * b + 1] = __fmaf_rn(sd, (float)d1, acc[j][2 * b + 1]);
+      }
+    }
+  }
   static __device__ __forceinline__ void mul(const unsigned char* chunk, const float2*, const Acts& a, int sb, int g, int t, f2 (&acc)[kPieces][2]) {
     const unsigned char* p = chunk + g * kPitch;
     const uint4 hd[2] = {*reinterpret_cast<const uint4*>(p), *reinterpret_cast<const uint4*>(p + 8 * kPitch)};
@@ -467,11 +535,62 @@ __global__ void __launch_bounds__(512, 1) rows_kernel(const __grid_constant__ CU
   }
 }
 
-// Mixture of experts: an item is a tile (up to 8 slots of one expert) x a group of row tiles; how many tiles there are is known on the
-// device only.  A CTA takes a run of consecutive items, which mostly share their tile: the activations are staged once per tile, and
-// the rings run on from item to item.  (One CTA per possible item left at once for most of them: 2048 x 768 of 128 experts, 32 slots,
-// 8448 CTAs for some 1800 items: gate/up, quantise and down took 90 us, in this form 64 us.)
+// A warp's whole 16-row tile for TT tokens by dp4a, its chunks in superblock order; the same 32 partial sums per output and the same tree.
+// out[j]: row lane % 16 (both half-warps) against token j.  false: a wait ran out.
+template <class F, int TT, class Request>
+__device__ __forceinline__ bool dot_tile(Ring<F>& ring, const unsigned char* act, int nsb, int T, int lane, float (&out)[4], Request request) {
+  constexpr int kLocal = F::kPieces / 2;
+  float acc[F::kSubs][TT][kLocal];
+#pragma unroll
+  for (int s = 0; s < F::kSubs; ++s)
+#pragma unroll
+    for (int j = 0; j < TT; ++j)
+#pragma unroll
+      for (int p = 0; p < kLocal; ++p) acc[s][j][p] = 0.0f;
+  for (int s0 = 0; s0 < nsb; s0 += F::kSubs) {
+#pragma unroll
+    for (int s = 0; s < F::kSubs; ++s) {
+      if (s0 + s >= nsb) break;
+      const unsigned char* chunk = ring.wait();
+      if (!chunk) {
+        ring.drain();
+        return false;
+      }
+      F::template dot<TT>(chunk, act, nsb * 8, T, s0 + s, lane, acc[s]);
+      __syncwarp();  // every lane has read the chunk: its slot takes the next request
+      ring.next();
+      request();
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < TT; ++j) {
+    float v[kLocal];
+#pragma unroll
+    for (int p = 0; p < kLocal; ++p) {
+      v[p] = F::kSubs == 4 ? __fadd_rn(__fadd_rn(acc[0][j][p], acc[F::kSubs - 2][j][p]), __fadd_rn(acc[1][j][p], acc[F::kSubs - 1][j][p])) : __fadd_rn(acc[0][j][p], acc[1][j][p]);
+      v[p] = __fadd_rn(v[p], __shfl_xor_sync(0xFFFFFFFFu, v[p], 16));
+    }
+#pragma unroll
+    for (int h = kLocal / 2; h > 0; h >>= 1)
+#pragma unroll
+      for (int p = 0; p < h; ++p) v[p] = __fadd_rn(v[p], v[p + h]);
+    out[j] = v[0];
+  }
+  return true;
+}
+template <class F, class Request>
+__device__ __forceinline__ bool dot_tile_of(Ring<F>& ring, const unsigned char* act, int nsb, int T, int lane, float (&out)[4], Request request) {
+  return T == 1 ? dot_tile<F, 1>(ring, act, nsb, T, lane, out, request) : T == 2 ? dot_tile<F, 2>(ring, act, nsb, T, lane, out, request) : dot_tile<F, 4>(ring, act, nsb, T, lane, out, request);
+}
+
+// Mixture of experts: an item is a tile (up to 8 slots of one expert) x as many row tiles as the CTA has warps; how many tiles there are
+// is known on the device only.  A CTA takes a run of consecutive items, which mostly share their tile: the activations are staged once
+// per tile, and the rings run on from item to item.  (One CTA per possible item left at once for most of them: 2048 x 768 of 128
+// experts, 32 slots, 8448 CTAs for some 1800 items: gate/up, quantise and down took 90 us, walked like this 56 us.)
+// A tile of up to kFewSlots slots -- most, while a step has few tokens -- goes by dp4a, each warp a row tile of its own: a third of the
+// matrix instruction's instructions at one slot, and no exchange between warps (@@ us).
 // gate/up (pair): h[slot][N] = silu(x Wg^T) * (x Wu^T), token rows through stok; down: y[slot][N] = swt * (hq Wd^T).
+constexpr int kFewSlots = 4;
 template <class F>
 __global__ void __launch_bounds__(512, 1) moe_rows_kernel(const __grid_constant__ CUtensorMap tg, const __grid_constant__ CUtensorMap tu, int pair, int N, int K,
                                                           const int8_t* __restrict__ aq, const float* __restrict__ asc, int Mp, const int32_t* __restrict__ tiles,
@@ -479,7 +598,7 @@ __global__ void __launch_bounds__(512, 1) moe_rows_kernel(const __grid_constant_
   extern __shared__ __align__(1024) unsigned char smem[];
   const int NW = blockDim.x >> 5, kPer = NW / F::kSubs;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int part = warp % F::kSubs, mine = warp / F::kSubs, nsb = K >> 8, groups = ((N + 15) / 16 + kPer - 1) / kPer;
+  const int part = warp % F::kSubs, mine = warp / F::kSubs, nsb = K >> 8, groups = ((N + 15) / 16 + NW - 1) / NW;
   unsigned char* rings = smem + act_bytes<F>(K, 8);
   unsigned char* xch = rings + (size_t)NW * slots * Ring<F>::kSlot;
   Ring<F> ring;
@@ -494,21 +613,47 @@ __global__ void __launch_bounds__(512, 1) moe_rows_kernel(const __grid_constant_
   pdl_wait();
   const long long items = (long long)tiles[0] * groups;
   const int lo = (int)(items * blockIdx.x / gridDim.x), hi = (int)(items * (blockIdx.x + 1) / gridDim.x);
-  // chunks still to request: superblock `ps` of matrix `pm` (gate, up) of item `pi`, whose expert is `pe`
-  int pi = lo, pm = 0, ps = part, pe = lo < hi ? tiles[1 + 3 * (lo / groups)] : 0;
-  auto request = [&]() {
-    if (pi >= hi || part >= nsb) return;
-    ring.fill(pm ? &tu : &tg, ps, pe * N + (pi % groups * kPer + mine) * 16, lane);
-    if ((ps += F::kSubs) < nsb) return;
-    ps = part;
-    if (pm++ < pair) return;
-    pm = 0;
-    if (++pi < hi && pi % groups == 0) pe = tiles[1 + 3 * (pi / groups)];
+  // Chunks still to request: superblock `ps` of matrix `pm` (gate, up) of this warp's row tile in round `pr` of item `pi`.  Few slots:
+  // one round, every superblock; else kSubs rounds of kPer row tiles, every kSubs-th superblock.
+  int pi = lo, pr = 0, pm = 0, ps = 0, pe = 0;
+  bool few = true;
+  auto enter = [&]() {
+    pe = tiles[1 + 3 * (pi / groups)];
+    few = tiles[3 + 3 * (pi / groups)] <= kFewSlots;
   };
+  auto request = [&]() {
+    while (pi < hi) {
+      const bool any = ps < nsb;
+      if (any) {
+        ring.fill(pm ? &tu : &tg, ps, pe * N + (pi % groups * NW + (few ? warp : pr * kPer + mine)) * 16, lane);
+        if ((ps += few ? 1 : F::kSubs) < nsb) return;
+      }
+      if (pm++ >= pair) {
+        pm = 0;
+        if (++pr >= (few ? 1 : F::kSubs)) {
+          pr = 0;
+          if (++pi < hi && pi % groups == 0) enter();
+        }
+      }
+      ps = few ? 0 : part;
+      if (any) return;
+    }
+  };
+  if (lo < hi) {
+    enter();
+    ps = few ? 0 : part;
+  }
   for (int s = 0; s < slots; ++s) request();
   Acts acts;
   int s0 = 0, T = 0;
   bool ok = true;
+  auto store = [&](int n, int slot, float gate, float v) {
+    if (n < N && slot < T) out[(size_t)(s0 + slot) * N + n] = pair ? __fmul_rn(__fdiv_rn(gate, __fadd_rn(1.0f, expf(-gate))), v) : __fmul_rn(swt[s0 + slot], v);
+  };
+  auto note = [&]() {  // (bounded wait gave up: nothing of this CTA is stored any more)
+    if (lane == 0) atomicOr(err, 64u);
+    *gave_up = 1;
+  };
   for (int it = lo; it < hi; ++it) {
     if (it == lo || it % groups == 0) {
       if (it != lo) __syncthreads();  // the last tile's activations have been read
@@ -517,26 +662,31 @@ __global__ void __launch_bounds__(512, 1) moe_rows_kernel(const __grid_constant_
       acts = stage_acts<F>(smem, K, T, aq, asc, Mp, g, t, [&](int j) { return stok ? stok[s0 + j] : s0 + j; });
       __syncthreads();
     }
-    float first[4];
-    for (int m = 0; m <= pair; ++m) {
-      f2 acc[F::kPieces][2];
-      if (ok) ok = accumulate<F>(ring, reinterpret_cast<float2*>(xch + (size_t)warp * kXch), acts, part, nsb, lane, acc, request);
-      if (!ok) {  // (bounded wait gave up: nothing of this CTA is stored any more)
-        if (lane == 0) atomicOr(err, 64u);
-        *gave_up = 1;
+    const int tile0 = it % groups * NW;
+    if (T <= kFewSlots) {
+      float first[4], v[4];
+      if (ok) ok = dot_tile_of<F>(ring, smem, nsb, T, lane, first, request);
+      if (ok && pair) ok = dot_tile_of<F>(ring, smem, nsb, T, lane, v, request);
+      if (!ok) note();
+      if (!*gave_up && lane < 16) {
+#pragma unroll
+        for (int j = 0; j < kFewSlots; ++j) store((tile0 + warp) * 16 + lane, j, first[j], pair ? v[j] : first[j]);
       }
-      reduce_tile<F>(acc, xch, warp, lane);
-      if (m < pair) {
+      continue;
+    }
+    for (int r = 0; r < F::kSubs; ++r) {
+      float first[4];
+      for (int m = 0; m <= pair; ++m) {
+        f2 acc[F::kPieces][2];
+        if (ok) ok = accumulate<F>(ring, reinterpret_cast<float2*>(xch + (size_t)warp * kXch), acts, part, nsb, lane, acc, request);
+        if (!ok) note();
+        reduce_tile<F>(acc, xch, warp, lane);
+        if (m < pair) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) first[i] = f2_get(acc[0][i >> 1], i & 1);
-      } else if (part == 0 && !*gave_up) {
+          for (int i = 0; i < 4; ++i) first[i] = f2_get(acc[0][i >> 1], i & 1);
+        } else if (part == 0 && !*gave_up) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int n = (it % groups * kPer + mine) * 16 + g + 8 * (i >> 1), slot = 2 * t + (i & 1);
-          if (n < N && slot < T) {
-            const float v = f2_get(acc[0][i >> 1], i & 1);
-            out[(size_t)(s0 + slot) * N + n] = pair ? __fmul_rn(__fdiv_rn(first[i], __fadd_rn(1.0f, expf(-first[i]))), v) : __fmul_rn(swt[s0 + slot], v);
-          }
+          for (int i = 0; i < 4; ++i) store((tile0 + r * kPer + mine) * 16 + g + 8 * (i >> 1), 2 * t + (i & 1), first[i], f2_get(acc[0][i >> 1], i & 1));
         }
       }
     }
@@ -596,19 +746,25 @@ int rows_of(const izb_weight* w, int mat, const int8_t* aq, const float* asc, in
 template <class F>
 int moe_rows_of(const izb_weight* wg, const izb_weight* wu, const int8_t* aq, const float* asc, int Mp, const int32_t* tiles, int max_tiles, const int32_t* stok, const float* swt,
                 float* out, cudaStream_t st) {
-  const int sms = izb_sm_count(wg->device), row_tiles = (wg->N + 15) / 16;
-  const long long most = (long long)max_tiles * row_tiles;
-  if (most > (1ll << 30)) return 1;
-  const Split sp = pick_split<F>(wg->K, 8, (int)most, sms);
-  if (!sp.slots) return 1;
+  // (small CTAs: items are divided among them as they come, and a tile's activations hold up four warps only)
+  constexpr int kWarps = 4;
+  const int sms = izb_sm_count(wg->device);
+  if ((long long)max_tiles * ((wg->N + 15) / 16) > (1ll << 30)) return 1;
+  int ctas = 16 / kWarps, slots = 0;
+  for (; ctas > 0; --ctas) {
+    const size_t room = kSmemPerSm / ctas - (ctas > 1 ? 1024 : 0);
+    for (slots = 4; slots >= 2 && rows_smem<F>(wg->K, 8, kWarps, slots) > room;) --slots;
+    if (slots >= 2) break;
+  }
+  if (ctas == 0) return 1;
   IZB_SMEM_OPTIN((moe_rows_kernel<F>), kSmemPerSm, wg->device);
   uint32_t* err = izb_device_error_word(wg->device);
   if (!err) IZB_FAIL(IZB_ERR_NOMEM, "moe: no device error word");
   CUtensorMap tg, tu;
   memcpy(&tg, wg->tmap16_raw, sizeof tg);
   memcpy(&tu, (wu ? wu : wg)->tmap16_raw, sizeof tu);
-  IZB_LAUNCH(wu ? "moe_gateup" : "moe_down", st, izb_launch_pdl(moe_rows_kernel<F>, sms * sp.ctas, sp.warps * 32, rows_smem<F>(wg->K, 8, sp.warps, sp.slots), st, tg, tu, wu ? 1 : 0,
-                                                               wg->N, wg->K, aq, asc, Mp, tiles, stok, swt, out, sp.slots, err));
+  IZB_LAUNCH(wu ? "moe_gateup" : "moe_down", st, izb_launch_pdl(moe_rows_kernel<F>, sms * ctas, kWarps * 32, rows_smem<F>(wg->K, 8, kWarps, slots), st, tg, tu, wu ? 1 : 0,
+                                                               wg->N, wg->K, aq, asc, Mp, tiles, stok, swt, out, slots, err));
   return IZB_OK;
 }
 
