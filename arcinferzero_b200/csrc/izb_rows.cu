@@ -538,7 +538,7 @@ __global__ void __launch_bounds__(512, 1) rows_kernel(const __grid_constant__ CU
 // A warp's whole 16-row tile for TT tokens by dp4a, its chunks in superblock order; the same 32 partial sums per output and the same tree.
 // out[j]: row lane % 16 (both half-warps) against token j.  false: a wait ran out.
 template <class F, int TT, class Request>
-__device__ __forceinline__ bool dot_tile(Ring<F>& ring, const unsigned char* act, int nsb, int T, int lane, float (&out)[4], Request request) {
+__device__ __forceinline__ bool dot_tile(Ring<F>& ring, const unsigned char* act, int nsb, int T, int lane, float (&out)[2], Request request) {
   constexpr int kLocal = F::kPieces / 2;
   float acc[F::kSubs][TT][kLocal];
 #pragma unroll
@@ -578,11 +578,6 @@ __device__ __forceinline__ bool dot_tile(Ring<F>& ring, const unsigned char* act
   }
   return true;
 }
-template <class F, class Request>
-__device__ __forceinline__ bool dot_tile_of(Ring<F>& ring, const unsigned char* act, int nsb, int T, int lane, float (&out)[4], Request request) {
-  return T == 1 ? dot_tile<F, 1>(ring, act, nsb, T, lane, out, request) : T == 2 ? dot_tile<F, 2>(ring, act, nsb, T, lane, out, request) : dot_tile<F, 4>(ring, act, nsb, T, lane, out, request);
-}
-
 // Mixture of experts: an item is a tile (up to 8 slots of one expert) x as many row tiles as the CTA has warps; how many tiles there are
 // is known on the device only.  A CTA takes a run of consecutive items, which mostly share their tile: the activations are staged once
 // per tile, and the rings run on from item to item.  (One CTA per possible item left at once for most of them: 2048 x 768 of 128
@@ -590,7 +585,7 @@ __device__ __forceinline__ bool dot_tile_of(Ring<F>& ring, const unsigned char* 
 // A tile of up to kFewSlots slots -- most, while a step has few tokens -- goes by dp4a, each warp a row tile of its own: a third of the
 // matrix instruction's instructions at one slot, and no exchange between warps (@@ us).
 // gate/up (pair): h[slot][N] = silu(x Wg^T) * (x Wu^T), token rows through stok; down: y[slot][N] = swt * (hq Wd^T).
-constexpr int kFewSlots = 4;
+constexpr int kFewSlots = 2;
 template <class F>
 __global__ void __launch_bounds__(512, 1) moe_rows_kernel(const __grid_constant__ CUtensorMap tg, const __grid_constant__ CUtensorMap tu, int pair, int N, int K,
                                                           const int8_t* __restrict__ aq, const float* __restrict__ asc, int Mp, const int32_t* __restrict__ tiles,
@@ -664,13 +659,17 @@ __global__ void __launch_bounds__(512, 1) moe_rows_kernel(const __grid_constant_
     }
     const int tile0 = it % groups * NW;
     if (T <= kFewSlots) {
-      float first[4], v[4];
-      if (ok) ok = dot_tile_of<F>(ring, smem, nsb, T, lane, first, request);
-      if (ok && pair) ok = dot_tile_of<F>(ring, smem, nsb, T, lane, v, request);
+      float first[2] = {0.0f, 0.0f}, v[2] = {0.0f, 0.0f};
+#pragma unroll 1
+      for (int m = 0; m <= pair; ++m) {
+        first[0] = v[0];
+        first[1] = v[1];
+        if (ok) ok = T == 1 ? dot_tile<F, 1>(ring, smem, nsb, T, lane, v, request) : dot_tile<F, 2>(ring, smem, nsb, T, lane, v, request);
+      }
       if (!ok) note();
       if (!*gave_up && lane < 16) {
 #pragma unroll
-        for (int j = 0; j < kFewSlots; ++j) store((tile0 + warp) * 16 + lane, j, first[j], pair ? v[j] : first[j]);
+        for (int j = 0; j < kFewSlots; ++j) store((tile0 + warp) * 16 + lane, j, first[j], v[j]);
       }
       continue;
     }
