@@ -399,7 +399,7 @@ __device__ __forceinline__ Acts stage_acts(unsigned char* smem, int K, int T, co
     for (int u = 0; u < kBatch; ++u) {
       const int b = bb[u], j = jj[u];
       if (i0 + u * (int)blockDim.x >= items) continue;
-      if (kFew) {
+      if constexpr (kFew) {
         int s0 = 0, s1 = 0;
         if (F::kEx) {
           s0 = sum16(x[u]);
