@@ -601,13 +601,16 @@ __device__ __forceinline__ bool dot_rows(Ring<F>& ring, const unsigned char* act
 // 16-row chunks of one superblock, 144-byte pieces of 16 rows, the same products took 51 us).
 // gate/up (pair): h[slot][N] = silu(x Wg^T) * (x Wu^T), token rows through stok; down: y[slot][N] = swt * (hq Wd^T).
 constexpr int kFewSlots = 2;
+// (small CTAs: items are divided among them as they come, and a tile's activations hold up four warps only; three per SM leave the two
+// ways 168 registers -- at 128 they spilt, and with the shared memory in use the stacks do not fit in L1: 111 us)
+constexpr int kMoeWarps = 4, kMoeCtas = 3;
 template <class F>
-__global__ void __launch_bounds__(512, 1) moe_rows_kernel(const __grid_constant__ CUtensorMap tg, const __grid_constant__ CUtensorMap tu, const unsigned char* __restrict__ rg,
+__global__ void __launch_bounds__(kMoeWarps * 32, kMoeCtas) moe_rows_kernel(const __grid_constant__ CUtensorMap tg, const __grid_constant__ CUtensorMap tu, const unsigned char* __restrict__ rg,
                                                           const unsigned char* __restrict__ ru, int pair, int N, int K, const int8_t* __restrict__ aq,
                                                           const float* __restrict__ asc, int Mp, const int32_t* __restrict__ tiles,
                                                           const int32_t* __restrict__ stok, const float* __restrict__ swt, float* __restrict__ out, int slots, uint32_t* err) {
   extern __shared__ __align__(1024) unsigned char smem[];
-  const int NW = blockDim.x >> 5, kPer = NW / F::kSubs;
+  constexpr int NW = kMoeWarps, kPer = NW / F::kSubs;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int part = warp % F::kSubs, mine = warp / F::kSubs, nsb = K >> 8, groups = ((N + 15) / 16 + NW - 1) / NW;
   unsigned char* rings = smem + act_bytes<F>(K, 8);
@@ -777,14 +780,12 @@ int rows_of(const izb_weight* w, int mat, const int8_t* aq, const float* asc, in
 template <class F>
 int moe_rows_of(const izb_weight* wg, const izb_weight* wu, const int8_t* aq, const float* asc, int Mp, const int32_t* tiles, int max_tiles, const int32_t* stok, const float* swt,
                 float* out, cudaStream_t st) {
-  // (small CTAs: items are divided among them as they come, and a tile's activations hold up four warps only)
-  constexpr int kWarps = 4;
   const int sms = izb_sm_count(wg->device);
   if ((long long)max_tiles * ((wg->N + 15) / 16) > (1ll << 30)) return 1;
-  int ctas = 16 / kWarps, slots = 0;
+  int ctas = kMoeCtas, slots = 0;
   for (; ctas > 0; --ctas) {
     const size_t room = kSmemPerSm / ctas - (ctas > 1 ? 1024 : 0);
-    for (slots = 4; slots >= 2 && rows_smem<F>(wg->K, 8, kWarps, slots) > room;) --slots;
+    for (slots = 4; slots >= 2 && rows_smem<F>(wg->K, 8, kMoeWarps, slots) > room;) --slots;
     if (slots >= 2) break;
   }
   if (ctas == 0) return 1;
@@ -794,7 +795,7 @@ int moe_rows_of(const izb_weight* wg, const izb_weight* wu, const int8_t* aq, co
   CUtensorMap tg, tu;
   memcpy(&tg, wg->tmap16_raw, sizeof tg);
   memcpy(&tu, (wu ? wu : wg)->tmap16_raw, sizeof tu);
-  IZB_LAUNCH(wu ? "moe_gateup" : "moe_down", st, izb_launch_pdl(moe_rows_kernel<F>, sms * ctas, kWarps * 32, rows_smem<F>(wg->K, 8, kWarps, slots), st, tg, tu, wg->raw, (wu ? wu : wg)->raw, wu ? 1 : 0,
+  IZB_LAUNCH(wu ? "moe_gateup" : "moe_down", st, izb_launch_pdl(moe_rows_kernel<F>, sms * ctas, kMoeWarps * 32, rows_smem<F>(wg->K, 8, kMoeWarps, slots), st, tg, tu, wg->raw, (wu ? wu : wg)->raw, wu ? 1 : 0,
                                                                wg->N, wg->K, aq, asc, Mp, tiles, stok, swt, out, slots, err));
   return IZB_OK;
 }
