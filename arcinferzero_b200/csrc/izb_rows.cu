@@ -125,7 +125,7 @@ struct RQ4K {
   }
   // One row by dp4a: superblocks s0 + lane / 8 (at p: that superblock), lane % 8 the piece; the activations as stage_few lays them out
   template <int TT>
-  static __device__ __forceinline__ void step(const unsigned char* p, const unsigned char* act, int nsb, int sb, int lane, bool in, float (&acc)[TT]) {
+  static __device__ __forceinline__ void step(const unsigned char* p, const unsigned char* act, int nsb, int T, int sb, int lane, bool in, float (&acc)[TT]) {
     const int piece = lane & 7, c = piece >> 1;
     const uint4 h = *reinterpret_cast<const uint4*>(p), w = *reinterpret_cast<const uint4*>(p + 16 + 16 * piece);
     const float2 d = __half22float2(*reinterpret_cast<const __half2*>(&h.x));
@@ -135,9 +135,10 @@ struct RQ4K {
     const float a = __fmul_rn(d.x, byte_f(sc, k)), am = __fmul_rn(-d.y, byte_f(mn, k)), b = __fmul_rn(d.x * 0.0625f, byte_f(sc, k + 1)), bm = __fmul_rn(-d.y, byte_f(mn, k + 1));
 #pragma unroll
     for (int j = 0; j < TT; ++j) {
-      const uint4 xl = *reinterpret_cast<const uint4*>(act + (size_t)(2 * sb * TT + j) * 128 + 16 * piece);
-      const uint4 xh = *reinterpret_cast<const uint4*>(act + (size_t)((2 * sb + 1) * TT + j) * 128 + 16 * piece);
-      const float4 f = *reinterpret_cast<const float4*>(act + (size_t)nsb * 256 * TT + (size_t)(sb * TT + j) * 128 + 16 * piece);
+      if (j >= T) break;
+      const uint4 xl = *reinterpret_cast<const uint4*>(act + (size_t)(2 * sb * T + j) * 128 + 16 * piece);
+      const uint4 xh = *reinterpret_cast<const uint4*>(act + (size_t)((2 * sb + 1) * T + j) * 128 + 16 * piece);
+      const float4 f = *reinterpret_cast<const float4*>(act + (size_t)nsb * 256 * T + (size_t)(sb * T + j) * 128 + 16 * piece);
       int lo = 0, hi = 0;
       lo = dot_u8(w.x & 0x0F0F0F0Fu, xl.x, lo); lo = dot_u8(w.y & 0x0F0F0F0Fu, xl.y, lo); lo = dot_u8(w.z & 0x0F0F0F0Fu, xl.z, lo); lo = dot_u8(w.w & 0x0F0F0F0Fu, xl.w, lo);
       hi = dot_u8(w.x & 0xF0F0F0F0u, xh.x, hi); hi = dot_u8(w.y & 0xF0F0F0F0u, xh.y, hi); hi = dot_u8(w.z & 0xF0F0F0F0u, xh.z, hi); hi = dot_u8(w.w & 0xF0F0F0F0u, xh.w, hi);
@@ -192,14 +193,15 @@ struct RQ80 {
   static constexpr bool kEx = false, kPrep = false;
   static __device__ __forceinline__ void prep(const unsigned char*, float2*, int) {}
   template <int TT>
-  static __device__ __forceinline__ void step(const unsigned char* p, const unsigned char* act, int nsb, int sb, int lane, bool in, float (&acc)[TT]) {
+  static __device__ __forceinline__ void step(const unsigned char* p, const unsigned char* act, int nsb, int T, int sb, int lane, bool in, float (&acc)[TT]) {
     const int piece = lane & 15;
     const float d = half_bits_to_float(*reinterpret_cast<const unsigned short*>(p + (piece & ~1)));
     const uint4 w = *reinterpret_cast<const uint4*>(p + 16 + 16 * piece);
 #pragma unroll
     for (int j = 0; j < TT; ++j) {
-      const uint4 x = *reinterpret_cast<const uint4*>(act + (size_t)(sb * TT + j) * 256 + 16 * piece);
-      const float sa = *reinterpret_cast<const float*>(act + (size_t)nsb * 256 * TT + (size_t)(sb * TT + j) * 32 + 4 * (piece >> 1));
+      if (j >= T) break;
+      const uint4 x = *reinterpret_cast<const uint4*>(act + (size_t)(sb * T + j) * 256 + 16 * piece);
+      const float sa = *reinterpret_cast<const float*>(act + (size_t)nsb * 256 * T + (size_t)(sb * T + j) * 32 + 4 * (piece >> 1));
       int dot = __dp4a((int)w.x, (int)x.x, 0);
       dot = __dp4a((int)w.y, (int)x.y, dot); dot = __dp4a((int)w.z, (int)x.z, dot); dot = __dp4a((int)w.w, (int)x.w, dot);
       if (in) acc[j] = __fmaf_rn(__fmul_rn(sa, d), (float)dot, acc[j]);
@@ -555,7 +557,7 @@ __global__ void __launch_bounds__(512, 1) rows_kernel(const __grid_constant__ CU
 // out[j]: row `lane` against token j.  false: a wait ran out.
 constexpr int kRun = 16;
 template <class F, int TT, class Request>
-__device__ __forceinline__ bool dot_rows(Ring<F>& ring, const unsigned char* act, int nsb, int rows, int lane, float (&out)[2], Request request) {
+__device__ __forceinline__ bool dot_rows(Ring<F>& ring, const unsigned char* act, int nsb, int T, int rows, int lane, float (&out)[4], Request request) {
   const int sub = lane / (32 / F::kSubs);
   int row = 0, sb0 = 0;
   float acc[TT];
@@ -571,7 +573,7 @@ __device__ __forceinline__ bool dot_rows(Ring<F>& ring, const unsigned char* act
       const int n = min(left, nsb - sb0);
       for (int i = 0; i < n; i += F::kSubs) {
         const int k = min(i + sub, n - 1);
-        F::template step<TT>(p + k * F::SBB, act, nsb, sb0 + k, lane, i + sub < n, acc);
+        F::template step<TT>(p + k * F::SBB, act, nsb, TT < 3 ? TT : T, sb0 + k, lane, i + sub < n, acc);
       }
       p += n * F::SBB;
       left -= n;
@@ -600,7 +602,7 @@ __device__ __forceinline__ bool dot_rows(Ring<F>& ring, const unsigned char* act
 // matrix instruction's instructions at one slot, no exchange between warps, and contiguous bytes of the weights per request (@@ us; with
 // 16-row chunks of one superblock, 144-byte pieces of 16 rows, the same products took 51 us).
 // gate/up (pair): h[slot][N] = silu(x Wg^T) * (x Wu^T), token rows through stok; down: y[slot][N] = swt * (hq Wd^T).
-constexpr int kFewSlots = 2;
+constexpr int kFewSlots = 4;
 // (small CTAs: items are divided among them as they come, and a tile's activations hold up four warps only; three per SM leave the two
 // ways 168 registers -- at 128 they spilt, and with the shared memory in use the stacks do not fit in L1: 111 us)
 constexpr int kMoeWarps = 4, kMoeCtas = 3;
@@ -693,13 +695,13 @@ __global__ void __launch_bounds__(kMoeWarps * 32, kMoeCtas) moe_rows_kernel(cons
     }
     const int tile0 = it % groups * NW;
     if (T <= kFewSlots) {
-      float first[2] = {0.0f, 0.0f}, v[2] = {0.0f, 0.0f};
+      float first[4] = {0.0f, 0.0f, 0.0f, 0.0f}, v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll 1
       for (int m = 0; m <= pair; ++m) {
-        first[0] = v[0];
-        first[1] = v[1];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) first[j] = v[j];
         const int rows = min(16, N - (tile0 + warp) * 16);
-        if (ok) ok = T == 1 ? dot_rows<F, 1>(ring, smem, nsb, rows, lane, v, request) : dot_rows<F, 2>(ring, smem, nsb, rows, lane, v, request);
+        if (ok) ok = T == 1 ? dot_rows<F, 1>(ring, smem, nsb, T, rows, lane, v, request) : T == 2 ? dot_rows<F, 2>(ring, smem, nsb, T, rows, lane, v, request) : dot_rows<F, 4>(ring, smem, nsb, T, rows, lane, v, request);
       }
       if (!ok) note();
       if (!*gave_up && lane < 16) {
