@@ -79,13 +79,6 @@ __device__ __forceinline__ int dot_u8(uint32_t w, uint32_t x, int c) {
   asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(w), "r"(x), "r"(c));
   return d;
 }
-// sum of 16 signed bytes
-__device__ __forceinline__ int sum16(const uint4& v) {
-  int s = __dp4a((int)v.x, 0x01010101, 0);
-  s = __dp4a((int)v.y, 0x01010101, s);
-  s = __dp4a((int)v.z, 0x01010101, s);
-  return __dp4a((int)v.w, 0x01010101, s);
-}
 // unsigned byte k of a word as f32: 0x4B000000 | byte is 2^23 + byte
 __device__ __forceinline__ float byte_f(uint32_t w, int k) { return __fsub_rn(__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440 + k)), 8388608.0f); }
 
@@ -105,56 +98,56 @@ struct Acts {
 struct RQ4K {
   static constexpr int SBB = 144, kPitch = 144, kSubs = 4, kPieces = 8;
   static constexpr bool kEx = true, kPrep = true;
-  // the sub-block scales (sc) and mins (mn) of blocks 4 up .. + 3 as bytes (get_scale_min_k4, src/quants.h:61-69)
-  static __device__ __forceinline__ void scales(const uint4& h, int up, uint32_t& sc, uint32_t& mn) {
-    sc = up ? (h.w & 0x0F0F0F0Fu) | ((h.y >> 2) & 0x30303030u) : h.y & 0x3F3F3F3Fu;
-    mn = up ? ((h.w >> 4) & 0x0F0F0F0Fu) | ((h.z >> 2) & 0x30303030u) : h.z & 0x3F3F3F3Fu;
-  }
-  static __device__ __forceinline__ void prep(const unsigned char* chunk, float2* hd, int lane) {
-    // lane <-> row lane / 2, blocks 4 (lane & 1) .. + 3: (d * sc, -dmin * mn).  Odd blocks meet 16 q: their d * sc is divided by 16.
-    const int row = lane >> 1, up = lane & 1;
+  // (d * sc, -dmin * mn) of a row's blocks 4 up .. + 3; the sub-block scales and mins as bytes (get_scale_min_k4,
+  // src/quants.h:61-69).  Odd blocks meet 16 q: their d * sc is divided by 16.
+  static __device__ __forceinline__ void header(const unsigned char* chunk, int row, int up, float2 (&o)[4]) {
     const uint4 h = *reinterpret_cast<const uint4*>(chunk + row * kPitch);
     const float2 d = __half22float2(*reinterpret_cast<const __half2*>(&h.x));
-    uint32_t sc, mn;
-    scales(h, up, sc, mn);
+    const uint32_t sc = up ? (h.w & 0x0F0F0F0Fu) | ((h.y >> 2) & 0x30303030u) : h.y & 0x3F3F3F3Fu;
+    const uint32_t mn = up ? ((h.w >> 4) & 0x0F0F0F0Fu) | ((h.z >> 2) & 0x30303030u) : h.z & 0x3F3F3F3Fu;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      const float a = __fmul_rn((k & 1) ? d.x * 0.0625f : d.x, byte_f(sc, k)), b = __fmul_rn(-d.y, byte_f(mn, k));
-      hd[(4 * up + k) * 16 + row] = make_float2(a, b);
+      o[k] = make_float2(__fmul_rn((k & 1) ? d.x * 0.0625f : d.x, byte_f(sc, k)), __fmul_rn(-d.y, byte_f(mn, k)));
     }
   }
-  // One row by dp4a: superblocks s0 + lane / 8 (at p: that superblock), lane % 8 the piece; the activations as stage_few lays them out
-  template <int TT>
-  static __device__ __forceinline__ void step(const unsigned char* p, const unsigned char* act, int nsb, int T, int sb, int lane, bool in, float (&acc)[TT]) {
-    const int piece = lane & 7, c = piece >> 1;
-    const uint4 h = *reinterpret_cast<const uint4*>(p), w = *reinterpret_cast<const uint4*>(p + 16 + 16 * piece);
-    const float2 d = __half22float2(*reinterpret_cast<const __half2*>(&h.x));
-    uint32_t sc, mn;
-    scales(h, c >> 1, sc, mn);
-    const int k = 2 * (c & 1);
-    const float a = __fmul_rn(d.x, byte_f(sc, k)), am = __fmul_rn(-d.y, byte_f(mn, k)), b = __fmul_rn(d.x * 0.0625f, byte_f(sc, k + 1)), bm = __fmul_rn(-d.y, byte_f(mn, k + 1));
+  static __device__ __forceinline__ void prep(const unsigned char* chunk, float2* hd, int lane) {
+    const int row = lane >> 1, up = lane & 1;
+    float2 h[4];
+    header(chunk, row, up, h);
 #pragma unroll
-    for (int j = 0; j < TT; ++j) {
-      if (j >= T) break;
-      const uint4 xl = *reinterpret_cast<const uint4*>(act + (size_t)(2 * sb * T + j) * 128 + 16 * piece);
-      const uint4 xh = *reinterpret_cast<const uint4*>(act + (size_t)((2 * sb + 1) * T + j) * 128 + 16 * piece);
-      const float4 f = *reinterpret_cast<const float4*>(act + (size_t)nsb * 256 * T + (size_t)(sb * T + j) * 128 + 16 * piece);
-      int lo = 0, hi = 0;
-      lo = dot_u8(w.x & 0x0F0F0F0Fu, xl.x, lo); lo = dot_u8(w.y & 0x0F0F0F0Fu, xl.y, lo); lo = dot_u8(w.z & 0x0F0F0F0Fu, xl.z, lo); lo = dot_u8(w.w & 0x0F0F0F0Fu, xl.w, lo);
-      hi = dot_u8(w.x & 0xF0F0F0F0u, xh.x, hi); hi = dot_u8(w.y & 0xF0F0F0F0u, xh.y, hi); hi = dot_u8(w.z & 0xF0F0F0F0u, xh.z, hi); hi = dot_u8(w.w & 0xF0F0F0F0u, xh.w, hi);
-      const float P = __fmaf_rn(a, (float)lo, __fmul_rn(am, f.z)), Q = __fmaf_rn(b, (float)hi, __fmul_rn(bm, f.w));
-      if (in) acc[j] = __fadd_rn(acc[j], __fmaf_rn(f.x, P, __fmul_rn(f.y, Q)));
-    }
+    for (int k = 0; k < 4; ++k) hd[(4 * up + k) * 16 + row] = h[k];
   }
-  static __device__ __forceinline__ void put_few(unsigned char* smem, int nsb, int T, int b, int j, const uint4& x, const uint4& y, float sa, int s0, int s1) {
-    const int sb = b >> 3, k = b & 7;
-    uint4* q = reinterpret_cast<uint4*>(smem + (size_t)((2 * sb + (k & 1)) * T + j) * 128 + 32 * (k >> 1));
-    q[0] = x;
-    q[1] = y;
-    float* f = reinterpret_cast<float*>(smem + (size_t)nsb * 256 * T + (size_t)(sb * T + j) * 128 + 32 * (k >> 1)) + (k & 1);  // (sl, sh, el, eh) per piece
-    f[0] = f[4] = sa;
-    f[2] = (float)s0;
-    f[6] = (float)s1;
+  // The same products by dp4a: lane <-> row lane % 16 and pieces 4 up .. + 3 of the superblock (up = lane / 16), TT tokens of the T staged
+  template <int TT>
+  static __device__ __forceinline__ void dot(const unsigned char* chunk, const unsigned char* act, int nb, int T, int sb, int lane, float (&acc)[TT][kPieces / 2]) {
+    const int row = lane & 15, up = lane >> 4, b0 = 8 * sb + 4 * up;
+    float2 hd[4];
+    header(chunk, row, up, hd);
+    const float* sc = reinterpret_cast<const float*>(act + (size_t)nb * 32 * T) + b0 * 8;
+    const float* ex = reinterpret_cast<const float*>(act + (size_t)nb * 32 * T) + nb * 8 + b0 * 16;
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const uint4* w = reinterpret_cast<const uint4*>(chunk + row * kPitch + 16 + 64 * up + 32 * c);
+      const uint4 w0 = w[0], w1 = w[1];
+#pragma unroll
+      for (int j = 0; j < TT; ++j) {
+        if (j >= T) break;
+        const uint4 *l = reinterpret_cast<const uint4*>(act + (size_t)((b0 + 2 * c) * T + j) * 32), *h = l + 2 * T;
+        const uint4 l0 = l[0], l1 = l[1], h0 = h[0], h1 = h[1];  // (words of the two halves alternate)
+        const float* e = ex + 32 * c + j;
+        const float sl = sc[16 * c + j], sh = sc[16 * c + 8 + j];
+        int dl0 = 0, dl1 = 0, dh0 = 0, dh1 = 0;
+        dl0 = dot_u8(w0.x & 0x0F0F0F0Fu, l0.x, dl0); dl0 = dot_u8(w0.y & 0x0F0F0F0Fu, l0.z, dl0); dl0 = dot_u8(w0.z & 0x0F0F0F0Fu, l1.x, dl0); dl0 = dot_u8(w0.w & 0x0F0F0F0Fu, l1.z, dl0);
+        dl1 = dot_u8(w1.x & 0x0F0F0F0Fu, l0.y, dl1); dl1 = dot_u8(w1.y & 0x0F0F0F0Fu, l0.w, dl1); dl1 = dot_u8(w1.z & 0x0F0F0F0Fu, l1.y, dl1); dl1 = dot_u8(w1.w & 0x0F0F0F0Fu, l1.w, dl1);
+        dh0 = dot_u8(w0.x & 0xF0F0F0F0u, h0.x, dh0); dh0 = dot_u8(w0.y & 0xF0F0F0F0u, h0.z, dh0); dh0 = dot_u8(w0.z & 0xF0F0F0F0u, h1.x, dh0); dh0 = dot_u8(w0.w & 0xF0F0F0F0u, h1.z, dh0);
+        dh1 = dot_u8(w1.x & 0xF0F0F0F0u, h0.y, dh1); dh1 = dot_u8(w1.y & 0xF0F0F0F0u, h0.w, dh1); dh1 = dot_u8(w1.z & 0xF0F0F0F0u, h1.y, dh1); dh1 = dot_u8(w1.w & 0xF0F0F0F0u, h1.w, dh1);
+        const float2 a = hd[2 * c], b = hd[2 * c + 1];
+        const float p0 = __fmaf_rn(a.x, (float)dl0, __fmul_rn(a.y, e[0])), q0 = __fmaf_rn(b.x, (float)dh0, __fmul_rn(b.y, e[16]));
+        const float p1 = __fmaf_rn(a.x, (float)dl1, __fmul_rn(a.y, e[8])), q1 = __fmaf_rn(b.x, (float)dh1, __fmul_rn(b.y, e[24]));
+        acc[j][2 * c] = __fadd_rn(acc[j][2 * c], __fmaf_rn(sl, p0, __fmul_rn(sh, q0)));
+        acc[j][2 * c + 1] = __fadd_rn(acc[j][2 * c + 1], __fmaf_rn(sl, p1, __fmul_rn(sh, q1)));
+      }
+    }
   }
   static __device__ __forceinline__ void mul(const unsigned char* chunk, const float2* hd, const Acts& a, int sb, int g, int t, f2 (&acc)[kPieces][2]) {
     const unsigned char* p = chunk + g * kPitch + 16 + 4 * t;
@@ -193,26 +186,29 @@ struct RQ80 {
   static constexpr bool kEx = false, kPrep = false;
   static __device__ __forceinline__ void prep(const unsigned char*, float2*, int) {}
   template <int TT>
-  static __device__ __forceinline__ void step(const unsigned char* p, const unsigned char* act, int nsb, int T, int sb, int lane, bool in, float (&acc)[TT]) {
-    const int piece = lane & 15;
-    const float d = half_bits_to_float(*reinterpret_cast<const unsigned short*>(p + (piece & ~1)));
-    const uint4 w = *reinterpret_cast<const uint4*>(p + 16 + 16 * piece);
+  static __device__ __forceinline__ void dot(const unsigned char* chunk, const unsigned char* act, int nb, int T, int sb, int lane, float (&acc)[TT][kPieces / 2]) {
+    const int row = lane & 15, up = lane >> 4, b0 = 8 * sb + 4 * up;
+    const uint2 hd = *reinterpret_cast<const uint2*>(chunk + row * kPitch + 8 * up);
+    const float* sc = reinterpret_cast<const float*>(act + (size_t)nb * 32 * T) + b0 * 8;
 #pragma unroll
-    for (int j = 0; j < TT; ++j) {
-      if (j >= T) break;
-      const uint4 x = *reinterpret_cast<const uint4*>(act + (size_t)(sb * T + j) * 256 + 16 * piece);
-      const float sa = *reinterpret_cast<const float*>(act + (size_t)nsb * 256 * T + (size_t)(sb * T + j) * 32 + 4 * (piece >> 1));
-      int dot = __dp4a((int)w.x, (int)x.x, 0);
-      dot = __dp4a((int)w.y, (int)x.y, dot); dot = __dp4a((int)w.z, (int)x.z, dot); dot = __dp4a((int)w.w, (int)x.w, dot);
-      if (in) acc[j] = __fmaf_rn(__fmul_rn(sa, d), (float)dot, acc[j]);
+    for (int b = 0; b < 4; ++b) {
+      const uint4* w = reinterpret_cast<const uint4*>(chunk + row * kPitch + 16 + 128 * up + 32 * b);
+      const uint4 w0 = w[0], w1 = w[1];
+      const uint32_t hw = b < 2 ? hd.x : hd.y;
+      const float d = half_bits_to_float((b & 1) ? hw >> 16 : hw & 0xFFFFu);
+#pragma unroll
+      for (int j = 0; j < TT; ++j) {
+        if (j >= T) break;
+        const uint4* x = reinterpret_cast<const uint4*>(act + (size_t)((b0 + b) * T + j) * 32);
+        const uint4 x0 = x[0], x1 = x[1];  // (words of the two halves alternate)
+        int d0 = 0, d1 = 0;
+        d0 = __dp4a((int)w0.x, (int)x0.x, d0); d0 = __dp4a((int)w0.y, (int)x0.z, d0); d0 = __dp4a((int)w0.z, (int)x1.x, d0); d0 = __dp4a((int)w0.w, (int)x1.z, d0);
+        d1 = __dp4a((int)w1.x, (int)x0.y, d1); d1 = __dp4a((int)w1.y, (int)x0.w, d1); d1 = __dp4a((int)w1.z, (int)x1.y, d1); d1 = __dp4a((int)w1.w, (int)x1.w, d1);
+        const float sd = __fmul_rn(sc[8 * b + j], d);
+        acc[j][2 * b] = __fmaf_rn(sd, (float)d0, acc[j][2 * b]);
+        acc[j][2 * b + 1] = __fmaf_rn(sd, (float)d1, acc[j][2 * b + 1]);
+      }
     }
-  }
-  static __device__ __forceinline__ void put_few(unsigned char* smem, int nsb, int T, int b, int j, const uint4& x, const uint4& y, float sa, int, int) {
-    const int sb = b >> 3, k = b & 7;
-    uint4* q = reinterpret_cast<uint4*>(smem + (size_t)(sb * T + j) * 256 + 32 * k);
-    q[0] = x;
-    q[1] = y;
-    *reinterpret_cast<float*>(smem + (size_t)nsb * 256 * T + (size_t)(sb * T + j) * 32 + 4 * k) = sa;
   }
   static __device__ __forceinline__ void mul(const unsigned char* chunk, const float2*, const Acts& a, int sb, int g, int t, f2 (&acc)[kPieces][2]) {
     const unsigned char* p = chunk + g * kPitch;
@@ -331,16 +327,6 @@ struct Ring {
     }
     if (++put == slots) put = 0;
   }
-  // `bytes` contiguous bytes (a multiple of 16, at most a slot)
-  __device__ __forceinline__ void fill_run(const unsigned char* src, int bytes, int lane) {
-    if (lane == 0) {
-      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(r_u32(&bars[put])), "r"(bytes) : "memory");
-      asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(r_u32(base + put * kSlot)), "l"(src), "r"(bytes),
-                   "r"(r_u32(&bars[put]))
-                   : "memory");
-    }
-    if (++put == slots) put = 0;
-  }
   // the next chunk in order; null when the bounded wait ran out
   __device__ __forceinline__ const unsigned char* wait() const {
     for (uint32_t it = 0; it < kSpin; ++it) {
@@ -374,7 +360,7 @@ __host__ __device__ __forceinline__ size_t rows_smem(int K, int T, int nw, int s
 
 // Activations of T tokens (rows `src(j)` of aq, columns of asc), as Acts describes them.  Four items per thread and pass, so that their
 // loads are in flight together.
-template <class F, bool kFew = false, class Src>
+template <class F, class Src>
 __device__ __forceinline__ Acts stage_acts(unsigned char* smem, int K, int T, const int8_t* __restrict__ aq, const float* __restrict__ asc, int Mp, int g, int t, Src src) {
   const int nb = K / 32, items = nb * T;
   float* s_sc = reinterpret_cast<float*>(smem + (size_t)nb * 32 * T);
@@ -401,21 +387,18 @@ __device__ __forceinline__ Acts stage_acts(unsigned char* smem, int K, int T, co
     for (int u = 0; u < kBatch; ++u) {
       const int b = bb[u], j = jj[u];
       if (i0 + u * (int)blockDim.x >= items) continue;
-      if constexpr (kFew) {
-        int s0 = 0, s1 = 0;
-        if (F::kEx) {
-          s0 = sum16(x[u]);
-          s1 = sum16(y[u]);
-        }
-        F::put_few(smem, nb >> 3, T, b, j, x[u], y[u], s[u], s0, s1);
-        continue;
-      }
       uint4* o = reinterpret_cast<uint4*>(smem + (size_t)(b * T + j) * 32);
       o[0] = make_uint4(x[u].x, y[u].x, x[u].y, y[u].y);
       o[1] = make_uint4(x[u].z, y[u].z, x[u].w, y[u].w);
       s_sc[b * 8 + j] = s[u];
       if (F::kEx) {
-        const int s0 = sum16(x[u]), s1 = sum16(y[u]);
+        const uint32_t w[8] = {x[u].x, x[u].y, x[u].z, x[u].w, y[u].x, y[u].y, y[u].z, y[u].w};
+        int s0 = 0, s1 = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          s0 = __dp4a((int)w[k], 0x01010101, s0);
+          s1 = __dp4a((int)w[4 + k], 0x01010101, s1);
+        }
         const bool q4 = F::SBB == 144;
         s_ex[b * 16 + j] = q4 ? (float)s0 : __int_as_float((int)kMagic - 32 * s0);
         s_ex[b * 16 + 8 + j] = q4 ? (float)s1 : __int_as_float((int)kMagic - 32 * s1);
@@ -552,46 +535,52 @@ __global__ void __launch_bounds__(512, 1) rows_kernel(const __grid_constant__ CU
   }
 }
 
-// Up to 16 consecutive rows for TT tokens by dp4a, one warp: the rows' bytes come as runs of kRun superblocks (several short rows, or a
-// part of a long one), in order.  Lane <-> superblock modulo kSubs x piece, the 32 partial sums per output as above, and the same tree.
-// out[j]: row `lane` against token j.  false: a wait ran out.
-constexpr int kRun = 16;
+// A warp's whole 16-row tile for TT tokens by dp4a, its chunks in superblock order; the same 32 partial sums per output and the same tree.
+// out[j]: row lane % 16 (both half-warps) against token j.  false: a wait ran out.
 template <class F, int TT, class Request>
-__device__ __forceinline__ bool dot_rows(Ring<F>& ring, const unsigned char* act, int nsb, int T, int rows, int lane, float (&out)[4], Request request) {
-  const int sub = lane / (32 / F::kSubs);
-  int row = 0, sb0 = 0;
-  float acc[TT];
+__device__ __forceinline__ bool dot_tile(Ring<F>& ring, const unsigned char* act, int nsb, int T, int lane, float (&out)[4], Request request) {
+  constexpr int kLocal = F::kPieces / 2;
+  float acc[F::kSubs][TT][kLocal];
 #pragma unroll
-  for (int j = 0; j < TT; ++j) acc[j] = 0.0f;
-  while (row < rows) {
-    const unsigned char* p = ring.wait();
-    if (!p) {
-      ring.drain();
-      return false;
-    }
-    for (int left = nsb <= kRun ? min(kRun / nsb, rows - row) * nsb : min(kRun, nsb - sb0); left > 0;) {  // superblocks of this run
-      const int n = min(left, nsb - sb0);
-      for (int i = 0; i < n; i += F::kSubs) {
-        const int k = min(i + sub, n - 1);
-        F::template step<TT>(p + k * F::SBB, act, nsb, TT < 3 ? TT : T, sb0 + k, lane, i + sub < n, acc);
-      }
-      p += n * F::SBB;
-      left -= n;
-      if ((sb0 += n) < nsb) continue;
+  for (int s = 0; s < F::kSubs; ++s)
 #pragma unroll
-      for (int j = 0; j < TT; ++j) {
-        const float v = warp_sum(acc[j]);
-        if (lane == row) out[j] = v;
-        acc[j] = 0.0f;
+    for (int j = 0; j < TT; ++j)
+#pragma unroll
+      for (int p = 0; p < kLocal; ++p) acc[s][j][p] = 0.0f;
+  for (int s0 = 0; s0 < nsb; s0 += F::kSubs) {
+#pragma unroll
+    for (int s = 0; s < F::kSubs; ++s) {
+      if (s0 + s >= nsb) break;
+      const unsigned char* chunk = ring.wait();
+      if (!chunk) {
+        ring.drain();
+        return false;
       }
-      sb0 = 0;
-      ++row;
+      F::template dot<TT>(chunk, act, nsb * 8, T, s0 + s, lane, acc[s]);
+      __syncwarp();  // every lane has read the chunk: its slot takes the next request
+      ring.next();
+      request();
     }
-    __syncwarp();  // every lane has read the run: its slot takes the next request
-    ring.next();
-    request();
+  }
+#pragma unroll
+  for (int j = 0; j < TT; ++j) {
+    float v[kLocal];
+#pragma unroll
+    for (int p = 0; p < kLocal; ++p) {
+      v[p] = F::kSubs == 4 ? __fadd_rn(__fadd_rn(acc[0][j][p], acc[F::kSubs - 2][j][p]), __fadd_rn(acc[1][j][p], acc[F::kSubs - 1][j][p])) : __fadd_rn(acc[0][j][p], acc[1][j][p]);
+      v[p] = __fadd_rn(v[p], __shfl_xor_sync(0xFFFFFFFFu, v[p], 16));
+    }
+#pragma unroll
+    for (int h = kLocal / 2; h > 0; h >>= 1)
+#pragma unroll
+      for (int p = 0; p < h; ++p) v[p] = __fadd_rn(v[p], v[p + h]);
+    out[j] = v[0];
   }
   return true;
+}
+template <class F, class Request>
+__device__ __forceinline__ bool dot_tile_of(Ring<F>& ring, const unsigned char* act, int nsb, int T, int lane, float (&out)[4], Request request) {
+  return T == 1 ? dot_tile<F, 1>(ring, act, nsb, T, lane, out, request) : T == 2 ? dot_tile<F, 2>(ring, act, nsb, T, lane, out, request) : dot_tile<F, 4>(ring, act, nsb, T, lane, out, request);
 }
 
 // Mixture of experts: an item is a tile (up to 8 slots of one expert) x as many row tiles as the CTA has warps; how many tiles there are
@@ -599,17 +588,15 @@ __device__ __forceinline__ bool dot_rows(Ring<F>& ring, const unsigned char* act
 // per tile, and the rings run on from item to item.  (One CTA per possible item left at once for most of them: 2048 x 768 of 128
 // experts, 32 slots, 8448 CTAs for some 1800 items: gate/up, quantise and down took 90 us, walked like this 56 us.)
 // A tile of up to kFewSlots slots -- most, while a step has few tokens -- goes by dp4a, each warp a row tile of its own: a third of the
-// matrix instruction's instructions at one slot, no exchange between warps, and contiguous bytes of the weights per request (@@ us; with
-// 16-row chunks of one superblock, 144-byte pieces of 16 rows, the same products took 51 us).
+// matrix instruction's instructions at one slot, and no exchange between warps (@@ us).
 // gate/up (pair): h[slot][N] = silu(x Wg^T) * (x Wu^T), token rows through stok; down: y[slot][N] = swt * (hq Wd^T).
 constexpr int kFewSlots = 4;
 // (small CTAs: items are divided among them as they come, and a tile's activations hold up four warps only; three per SM leave the two
-// ways 168 registers -- at 128 they spilt, and with the shared memory in use the stacks do not fit in L1: 111 us)
+// ways 168 registers -- at 128 they spilt, and with the shared memory in use the stacks do not fit in L1)
 constexpr int kMoeWarps = 4, kMoeCtas = 3;
 template <class F>
-__global__ void __launch_bounds__(kMoeWarps * 32, kMoeCtas) moe_rows_kernel(const __grid_constant__ CUtensorMap tg, const __grid_constant__ CUtensorMap tu, const unsigned char* __restrict__ rg,
-                                                          const unsigned char* __restrict__ ru, int pair, int N, int K, const int8_t* __restrict__ aq,
-                                                          const float* __restrict__ asc, int Mp, const int32_t* __restrict__ tiles,
+__global__ void __launch_bounds__(kMoeWarps * 32, kMoeCtas) moe_rows_kernel(const __grid_constant__ CUtensorMap tg, const __grid_constant__ CUtensorMap tu, int pair, int N, int K,
+                                                          const int8_t* __restrict__ aq, const float* __restrict__ asc, int Mp, const int32_t* __restrict__ tiles,
                                                           const int32_t* __restrict__ stok, const float* __restrict__ swt, float* __restrict__ out, int slots, uint32_t* err) {
   extern __shared__ __align__(1024) unsigned char smem[];
   constexpr int NW = kMoeWarps, kPer = NW / F::kSubs;
@@ -629,33 +616,20 @@ __global__ void __launch_bounds__(kMoeWarps * 32, kMoeCtas) moe_rows_kernel(cons
   pdl_wait();
   const long long items = (long long)tiles[0] * groups;
   const int lo = (int)(items * blockIdx.x / gridDim.x), hi = (int)(items * (blockIdx.x + 1) / gridDim.x);
-  // Still to request, of matrix `pm` (gate, up) of item `pi`.  Few slots: the run at superblock `ps` of this warp's rows taken as one line;
-  // else superblock `ps` in round `pr` of kSubs, each kPer row tiles and every kSubs-th superblock per warp.
-  int pi = lo, pr = 0, pm = 0, ps = 0, pe = 0, end = 0;
+  // Chunks still to request: superblock `ps` of matrix `pm` (gate, up) of this warp's row tile in round `pr` of item `pi`.  Few slots:
+  // one round, every superblock; else kSubs rounds of kPer row tiles, every kSubs-th superblock.
+  int pi = lo, pr = 0, pm = 0, ps = 0, pe = 0;
   bool few = true;
-  auto begin = [&]() {  // a matrix of item pi
-    const int rows = min(16, N - (pi % groups * NW + warp) * 16);
-    ps = few ? 0 : part;
-    end = few ? rows * nsb : nsb;
-  };
-  auto enter = [&]() {  // a tile
+  auto enter = [&]() {
     pe = tiles[1 + 3 * (pi / groups)];
     few = tiles[3 + 3 * (pi / groups)] <= kFewSlots;
   };
   auto request = [&]() {
     while (pi < hi) {
-      const bool any = ps < end;
+      const bool any = ps < nsb;
       if (any) {
-        const int tile0 = pi % groups * NW;
-        if (few) {
-          const int n = nsb <= kRun ? min(kRun / nsb * nsb, end - ps) : min(kRun, nsb - ps % nsb);
-          ring.fill_run((pm ? ru : rg) + ((size_t)(pe * N + (tile0 + warp) * 16) * nsb + ps) * F::SBB, n * F::SBB, lane);
-          ps += n;
-        } else {
-          ring.fill(pm ? &tu : &tg, ps, pe * N + (tile0 + pr * kPer + mine) * 16, lane);
-          ps += F::kSubs;
-        }
-        if (ps < end) return;
+        ring.fill(pm ? &tu : &tg, ps, pe * N + (pi % groups * NW + (few ? warp : pr * kPer + mine)) * 16, lane);
+        if ((ps += few ? 1 : F::kSubs) < nsb) return;
       }
       if (pm++ >= pair) {
         pm = 0;
@@ -664,13 +638,13 @@ __global__ void __launch_bounds__(kMoeWarps * 32, kMoeCtas) moe_rows_kernel(cons
           if (++pi < hi && pi % groups == 0) enter();
         }
       }
-      begin();
+      ps = few ? 0 : part;
       if (any) return;
     }
   };
   if (lo < hi) {
     enter();
-    begin();
+    ps = few ? 0 : part;
   }
   for (int s = 0; s < slots; ++s) request();
   Acts acts;
@@ -688,9 +662,7 @@ __global__ void __launch_bounds__(kMoeWarps * 32, kMoeCtas) moe_rows_kernel(cons
       if (it != lo) __syncthreads();  // the last tile's activations have been read
       s0 = tiles[2 + 3 * (it / groups)];
       T = tiles[3 + 3 * (it / groups)];
-      auto src = [&](int j) { return stok ? stok[s0 + j] : s0 + j; };
-      if (T <= kFewSlots) stage_acts<F, true>(smem, K, T, aq, asc, Mp, g, t, src);
-      else acts = stage_acts<F>(smem, K, T, aq, asc, Mp, g, t, src);
+      acts = stage_acts<F>(smem, K, T, aq, asc, Mp, g, t, [&](int j) { return stok ? stok[s0 + j] : s0 + j; });
       __syncthreads();
     }
     const int tile0 = it % groups * NW;
@@ -700,8 +672,7 @@ __global__ void __launch_bounds__(kMoeWarps * 32, kMoeCtas) moe_rows_kernel(cons
       for (int m = 0; m <= pair; ++m) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) first[j] = v[j];
-        const int rows = min(16, N - (tile0 + warp) * 16);
-        if (ok) ok = T == 1 ? dot_rows<F, 1>(ring, smem, nsb, T, rows, lane, v, request) : T == 2 ? dot_rows<F, 2>(ring, smem, nsb, T, rows, lane, v, request) : dot_rows<F, 4>(ring, smem, nsb, T, rows, lane, v, request);
+        if (ok) ok = dot_tile_of<F>(ring, smem, nsb, T, lane, v, request);
       }
       if (!ok) note();
       if (!*gave_up && lane < 16) {
@@ -797,7 +768,7 @@ int moe_rows_of(const izb_weight* wg, const izb_weight* wu, const int8_t* aq, co
   CUtensorMap tg, tu;
   memcpy(&tg, wg->tmap16_raw, sizeof tg);
   memcpy(&tu, (wu ? wu : wg)->tmap16_raw, sizeof tu);
-  IZB_LAUNCH(wu ? "moe_gateup" : "moe_down", st, izb_launch_pdl(moe_rows_kernel<F>, sms * ctas, kMoeWarps * 32, rows_smem<F>(wg->K, 8, kMoeWarps, slots), st, tg, tu, wg->raw, (wu ? wu : wg)->raw, wu ? 1 : 0,
+  IZB_LAUNCH(wu ? "moe_gateup" : "moe_down", st, izb_launch_pdl(moe_rows_kernel<F>, sms * ctas, kMoeWarps * 32, rows_smem<F>(wg->K, 8, kMoeWarps, slots), st, tg, tu, wu ? 1 : 0,
                                                                wg->N, wg->K, aq, asc, Mp, tiles, stok, swt, out, slots, err));
   return IZB_OK;
 }
