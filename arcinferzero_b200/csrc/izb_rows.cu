@@ -547,21 +547,34 @@ __device__ __forceinline__ bool dot_tile(Ring<F>& ring, const unsigned char* act
     for (int j = 0; j < TT; ++j)
 #pragma unroll
       for (int p = 0; p < kLocal; ++p) acc[s][j][p] = 0.0f;
-  for (int s0 = 0; s0 < nsb; s0 += F::kSubs) {
+  // (acc[0] is always the next superblock's: the sums move up by one per chunk, which costs less than the loop body four times over
+  // in the instruction cache; past the last superblock they move on until number 0 is in place)
+  auto turn = [&]() {
 #pragma unroll
-    for (int s = 0; s < F::kSubs; ++s) {
-      if (s0 + s >= nsb) break;
-      const unsigned char* chunk = ring.wait();
-      if (!chunk) {
-        ring.drain();
-        return false;
+    for (int j = 0; j < TT; ++j)
+#pragma unroll
+      for (int p = 0; p < kLocal; ++p) {
+        const float a = acc[0][j][p];
+#pragma unroll
+        for (int s = 0; s + 1 < F::kSubs; ++s) acc[s][j][p] = acc[s + 1][j][p];
+        acc[F::kSubs - 1][j][p] = a;
       }
-      F::template dot<TT>(chunk, act, nsb * 8, T, s0 + s, lane, acc[s]);
-      __syncwarp();  // every lane has read the chunk: its slot takes the next request
-      ring.next();
-      request();
+  };
+#pragma unroll 1
+  for (int sb = 0; sb < nsb; ++sb) {
+    const unsigned char* chunk = ring.wait();
+    if (!chunk) {
+      ring.drain();
+      return false;
     }
+    F::template dot<TT>(chunk, act, nsb * 8, T, sb, lane, acc[0]);
+    __syncwarp();  // every lane has read the chunk: its slot takes the next request
+    ring.next();
+    request();
+    turn();
   }
+#pragma unroll 1
+  for (int sb = nsb; sb % F::kSubs; ++sb) turn();
 #pragma unroll
   for (int j = 0; j < TT; ++j) {
     float v[kLocal];
@@ -618,34 +631,39 @@ __global__ void __launch_bounds__(kMoeWarps * 32, kMoeCtas) moe_rows_kernel(cons
   const int lo = (int)(items * blockIdx.x / gridDim.x), hi = (int)(items * (blockIdx.x + 1) / gridDim.x);
   // Chunks still to request: superblock `ps` of matrix `pm` (gate, up) of this warp's row tile in round `pr` of item `pi`.  Few slots:
   // one round, every superblock; else kSubs rounds of kPer row tiles, every kSubs-th superblock.
-  int pi = lo, pr = 0, pm = 0, ps = 0, pe = 0;
-  bool few = true;
-  auto enter = [&]() {
-    pe = tiles[1 + 3 * (pi / groups)];
-    few = tiles[3 + 3 * (pi / groups)] <= kFewSlots;
+  // (no divisions: a warp asks once per chunk.)
+  int left = hi - lo, pt = lo / groups, pg = lo - pt * groups, row = 0, rounds = 1, pr = 0, pm = 0, ps = 0, by = 1, from = 0;
+  auto enter = [&]() {  // tile pt
+    const bool few = tiles[3 + 3 * pt] <= kFewSlots;
+    row = tiles[1 + 3 * pt] * N + (pg * NW + (few ? warp : mine)) * 16;
+    rounds = few ? 1 : F::kSubs;
+    by = few ? 1 : F::kSubs;
+    ps = from = few ? 0 : part;
   };
   auto request = [&]() {
-    while (pi < hi) {
+    while (left > 0) {
       const bool any = ps < nsb;
       if (any) {
-        ring.fill(pm ? &tu : &tg, ps, pe * N + (pi % groups * NW + (few ? warp : pr * kPer + mine)) * 16, lane);
-        if ((ps += few ? 1 : F::kSubs) < nsb) return;
+        ring.fill(pm ? &tu : &tg, ps, row + pr * kPer * 16, lane);
+        if ((ps += by) < nsb) return;
       }
+      ps = from;
       if (pm++ >= pair) {
         pm = 0;
-        if (++pr >= (few ? 1 : F::kSubs)) {
+        if (++pr >= rounds) {
           pr = 0;
-          if (++pi < hi && pi % groups == 0) enter();
+          row += NW * 16;
+          if (--left > 0 && ++pg == groups) {
+            pg = 0;
+            ++pt;
+            enter();
+          }
         }
       }
-      ps = few ? 0 : part;
       if (any) return;
     }
   };
-  if (lo < hi) {
-    enter();
-    ps = few ? 0 : part;
-  }
+  if (left > 0) enter();
   for (int s = 0; s < slots; ++s) request();
   Acts acts;
   int s0 = 0, T = 0;
@@ -657,15 +675,20 @@ __global__ void __launch_bounds__(kMoeWarps * 32, kMoeCtas) moe_rows_kernel(cons
     if (lane == 0) atomicOr(err, 64u);
     *gave_up = 1;
   };
-  for (int it = lo; it < hi; ++it) {
-    if (it == lo || it % groups == 0) {
-      if (it != lo) __syncthreads();  // the last tile's activations have been read
-      s0 = tiles[2 + 3 * (it / groups)];
-      T = tiles[3 + 3 * (it / groups)];
+  int ti = lo / groups, gi = lo - ti * groups;
+  for (int it = lo; it < hi; ++it, ++gi) {
+    if (it == lo || gi == groups) {
+      if (it != lo) {
+        __syncthreads();  // the last tile's activations have been read
+        gi = 0;
+        ++ti;
+      }
+      s0 = tiles[2 + 3 * ti];
+      T = tiles[3 + 3 * ti];
       acts = stage_acts<F>(smem, K, T, aq, asc, Mp, g, t, [&](int j) { return stok ? stok[s0 + j] : s0 + j; });
       __syncthreads();
     }
-    const int tile0 = it % groups * NW;
+    const int tile0 = gi * NW;
     if (T <= kFewSlots) {
       float first[4] = {0.0f, 0.0f, 0.0f, 0.0f}, v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll 1
