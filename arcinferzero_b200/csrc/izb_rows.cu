@@ -538,7 +538,7 @@ __global__ void __launch_bounds__(512, 1) rows_kernel(const __grid_constant__ CU
 // A warp's whole 16-row tile for TT tokens by dp4a, its chunks in superblock order; the same 32 partial sums per output and the same tree.
 // out[j]: row lane % 16 (both half-warps) against token j.  false: a wait ran out.
 template <class F, int TT, class Request>
-__device__ __forceinline__ bool dot_tile(Ring<F>& ring, const unsigned char* act, int nsb, int T, int lane, float (&out)[4], Request request) {
+__device__ __forceinline__ bool dot_tile(Ring<F>& ring, const unsigned char* act, int nsb, int T, int lane, float (&out)[2], Request request) {
   constexpr int kLocal = F::kPieces / 2;
   float acc[F::kSubs][TT][kLocal];
 #pragma unroll
@@ -591,19 +591,16 @@ __device__ __forceinline__ bool dot_tile(Ring<F>& ring, const unsigned char* act
   }
   return true;
 }
-template <class F, class Request>
-__device__ __forceinline__ bool dot_tile_of(Ring<F>& ring, const unsigned char* act, int nsb, int T, int lane, float (&out)[4], Request request) {
-  return T == 1 ? dot_tile<F, 1>(ring, act, nsb, T, lane, out, request) : T == 2 ? dot_tile<F, 2>(ring, act, nsb, T, lane, out, request) : dot_tile<F, 4>(ring, act, nsb, T, lane, out, request);
-}
-
 // Mixture of experts: an item is a tile (up to 8 slots of one expert) x as many row tiles as the CTA has warps; how many tiles there are
 // is known on the device only.  A CTA takes a run of consecutive items, which mostly share their tile: the activations are staged once
 // per tile, and the rings run on from item to item.  (One CTA per possible item left at once for most of them: 2048 x 768 of 128
-// experts, 32 slots, 8448 CTAs for some 1800 items: gate/up, quantise and down took 90 us, walked like this 56 us.)
+// experts, 32 slots: 8448 CTAs for some 1800 items; a 4-token step took 120 us, walked like this 97.)
 // A tile of up to kFewSlots slots -- most, while a step has few tokens -- goes by dp4a, each warp a row tile of its own: a third of the
-// matrix instruction's instructions at one slot, and no exchange between warps (@@ us).
+// matrix instruction's instructions at one slot and no exchange between warps (the step: 69 -> 50 us; at three slots the two ways
+// are equal).  What bounds it is the latency of a chunk, about 1 us with the three warps per SMSP that fit: contiguous runs of
+// whole rows instead of 16-row chunks wanted four times the header work per weight (94 us).
 // gate/up (pair): h[slot][N] = silu(x Wg^T) * (x Wu^T), token rows through stok; down: y[slot][N] = swt * (hq Wd^T).
-constexpr int kFewSlots = 4;
+constexpr int kFewSlots = 2;
 // (small CTAs: items are divided among them as they come, and a tile's activations hold up four warps only; three per SM leave the two
 // ways 168 registers -- at 128 they spilt, and with the shared memory in use the stacks do not fit in L1)
 constexpr int kMoeWarps = 4, kMoeCtas = 3;
@@ -690,12 +687,12 @@ __global__ void __launch_bounds__(kMoeWarps * 32, kMoeCtas) moe_rows_kernel(cons
     }
     const int tile0 = gi * NW;
     if (T <= kFewSlots) {
-      float first[4] = {0.0f, 0.0f, 0.0f, 0.0f}, v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+      float first[2] = {0.0f, 0.0f}, v[2] = {0.0f, 0.0f};
 #pragma unroll 1
       for (int m = 0; m <= pair; ++m) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) first[j] = v[j];
-        if (ok) ok = dot_tile_of<F>(ring, smem, nsb, T, lane, v, request);
+        for (int j = 0; j < 2; ++j) first[j] = v[j];
+        if (ok) ok = T == 1 ? dot_tile<F, 1>(ring, smem, nsb, T, lane, v, request) : dot_tile<F, 2>(ring, smem, nsb, T, lane, v, request);
       }
       if (!ok) note();
       if (!*gave_up && lane < 16) {
