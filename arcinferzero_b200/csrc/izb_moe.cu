@@ -18,22 +18,19 @@ constexpr int kMaxPerLane = 16;  // experts per lane: NE <= 512
 // not chosen yet, the lower expert id winning a tie; p_k = exp(l_k - l_0) where l_0, the first choice, is the maximum;
 // w_k = p_k / (p_0 + ... + p_{NU-1}), the sum taken in choice order.
 //
-// One warp per token.  A logit and its expert id travel as ONE 64-bit key -- the order-preserving integer image of the
-// float in the high word, the complemented id in the low word -- so a single warp-wide maximum per choice yields the
-// winner and applies the tie rule at once.  Every lane keeps the key of its own best candidate and only the lane that
-// owned the winner rescans its (at most 16) experts.
-__device__ __forceinline__ unsigned long long route_key(float v, int e) {
+// One warp per token.  A lane holds the order-preserving integer images of its logits (kPer: as many as NE needs -- 16 always was
+// four times the work at 128 experts, 17 us for 4096 tokens) and its own best candidate; a choice is one warp-wide maximum of the images and one
+// minimum of the ids that hold it, which is the tie rule.  Only the owner of the winner rescans.
+__device__ __forceinline__ uint32_t route_key(float v) {
   uint32_t u = __float_as_uint(__fadd_rn(v, 0.0f));  // (-0 becomes +0: the two compare equal, so they must tie)
   u = (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-  return ((unsigned long long)u << 32) | (uint32_t)(~(uint32_t)e);
+  return u ? u : 1u;  // (0 is "no candidate"; only a NaN maps there)
 }
-__device__ __forceinline__ float route_key_value(unsigned long long k) {
-  const uint32_t u = (uint32_t)(k >> 32);
-  return __uint_as_float((u & 0x80000000u) ? (u & 0x7FFFFFFFu) : ~u);
-}
+__device__ __forceinline__ float route_key_value(uint32_t u) { return __uint_as_float((u & 0x80000000u) ? (u & 0x7FFFFFFFu) : ~u); }
 
 // `counts` is zeroed here when one CTA takes all tokens (a decode step: a launch less), else before.
 constexpr int kRouteWarps = 16;
+template <int kPer>
 __global__ void __launch_bounds__(kRouteWarps * 32) moe_route_kernel(const float* __restrict__ logits, int ldl, int T, int NE, int NU,
                                                                      int32_t* __restrict__ ids, float* __restrict__ wts,
                                                                      int32_t* __restrict__ counts, float* __restrict__ sgate) {
@@ -48,36 +45,34 @@ __global__ void __launch_bounds__(kRouteWarps * 32) moe_route_kernel(const float
   const float* row = logits + (size_t)token * ldl;
   // the shared expert's gate: the sigmoid of the logit after the experts' (SGATE, zero/kernels/moe.cl:44,88)
   if (sgate && lane == 0) sgate[token] = __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-row[NE])));
-  unsigned long long key[kMaxPerLane];  // 0 = no candidate (past NE, or already chosen)
+  uint32_t key[kPer];  // 0 = no candidate (past NE, or already chosen)
 #pragma unroll
-  for (int i = 0; i < kMaxPerLane; ++i) {
+  for (int i = 0; i < kPer; ++i) {
     const int e = i * 32 + lane;
-    key[i] = e < NE ? route_key(row[e], e) : 0ull;
+    key[i] = e < NE ? route_key(row[e]) : 0u;
   }
-  auto lane_best = [&]() {
-    unsigned long long b = 0ull;
+  uint32_t best = 0u;
+  int at = 0;  // this lane's best candidate is expert 32 at + lane
+  auto rescan = [&]() {
+    best = key[0];
+    at = 0;
 #pragma unroll
-    for (int i = 0; i < kMaxPerLane; ++i) b = key[i] > b ? key[i] : b;
-    return b;
+    for (int i = 1; i < kPer; ++i)
+      if (key[i] > best) { best = key[i]; at = i; }
   };
-  unsigned long long mine = lane_best();
+  rescan();
   float top = 0.0f, denom = 0.0f, p_keep = 0.0f;
   int e_keep = 0;
   for (int k = 0; k < NU; ++k) {
-    unsigned long long win = mine;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const unsigned long long other = __shfl_xor_sync(0xFFFFFFFFu, win, o);
-      win = other > win ? other : win;
-    }
-    const int e = (int)(~(uint32_t)win);
+    const uint32_t win = __reduce_max_sync(0xFFFFFFFFu, best);
+    const int e = (int)__reduce_min_sync(0xFFFFFFFFu, best == win ? (uint32_t)(at * 32 + lane) : 0xFFFFu);
     const float l = route_key_value(win);
     if (k == 0) top = l;
     if ((e & 31) == lane) {  // the owner strikes the winner out and looks for its next candidate
 #pragma unroll
-      for (int i = 0; i < kMaxPerLane; ++i)
-        if (i == (e >> 5)) key[i] = 0ull;
-      mine = lane_best();
+      for (int i = 0; i < kPer; ++i)
+        if (i == (e >> 5)) key[i] = 0u;
+      rescan();
     }
     const float p = expf(l - top);
     denom += p;  // (every lane adds the same terms in choice order)
@@ -100,12 +95,13 @@ __global__ void __launch_bounds__(kRouteWarps * 32) moe_route_kernel(const float
 // A thread looks at kPairs consecutive pairs per pass, the next pass's loads in flight meanwhile; an exclusive scan of the per-thread
 // counts over the warp (shuffles) and over the eight warps (shared memory, double-buffered so that one barrier per pass is enough)
 // gives every pair of the expert its slot.  (A pass is a chain of load, scan and barrier: with four pairs per thread 32768 pairs
-// were 32 of them, 38 us.)
-constexpr int kPairs = 16;
+// were 32 of them, 38 us.)  The pairs found go to a list in shared memory that all threads write out when another pass might not fit:
+// written where they are found, each waits for its weight's load by itself (27 us; @@ us like this).
+constexpr int kPairs = 16, kPairList = 2 * 256 * kPairs;
 __global__ void __launch_bounds__(256) moe_sort_kernel(const int32_t* __restrict__ ids, const float* __restrict__ wts, const int32_t* __restrict__ counts, int n, int NU,
                                                        int NE, int TM, int32_t* __restrict__ offs, int32_t* __restrict__ tiles, int max_tiles, int32_t* __restrict__ stok,
                                                        float* __restrict__ swt, int32_t* __restrict__ inv, int e0, int e1) {
-  __shared__ int s_warp[2][8], s_off[8], s_tile[8];
+  __shared__ int s_warp[2][8], s_off[8], s_tile[8], s_list[kPairList];
   const int e = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   pdl_launch_next();
   pdl_wait();
@@ -152,7 +148,7 @@ __global__ void __launch_bounds__(256) moe_sort_kernel(const int32_t* __restrict
     for (int i = 3 * used + threadIdx.x; i < 3 * max_tiles; i += blockDim.x) tiles[1 + i] = 0;
   }
   const bool here = e >= e0 && e < e1;
-  int base = off;  // (every thread keeps the running base: no broadcast needed)
+  int found = 0;  // pairs in the list (every thread keeps count: no broadcast needed)
   for (int i0 = 0, buf = 0; i0 < n; i0 += 256 * kPairs, buf ^= 1) {
     const int i = i0 + kPairs * threadIdx.x;
     int id[kPairs], cnt = 0;
@@ -176,17 +172,23 @@ __global__ void __launch_bounds__(256) moe_sort_kernel(const int32_t* __restrict
       if (w < warp) before += c;
       total += c;
     }
-    int s = base + before + incl - cnt;
+    int s = found + before + incl - cnt;
     if (cnt) {
 #pragma unroll
       for (int j = 0; j < kPairs; ++j)
-        if (id[j] == e) {
-          inv[i + j] = here ? s : -1;
-          if (here) { stok[s] = (i + j) / NU; swt[s] = wts[i + j]; }
-          ++s;
-        }
+        if (id[j] == e) s_list[s++] = i + j;
     }
-    base += total;
+    found += total;
+    if (i0 + 256 * kPairs < n && found + 256 * kPairs <= kPairList) continue;
+    __syncthreads();
+    for (int k = threadIdx.x; k < found; k += blockDim.x) {
+      const int pair = s_list[k], slot = off + k;
+      inv[pair] = here ? slot : -1;
+      if (here) { stok[slot] = pair / NU; swt[slot] = wts[pair]; }
+    }
+    off += found;
+    found = 0;
+    __syncthreads();
   }
 }
 
@@ -289,8 +291,9 @@ extern "C" int izb_moe_route_ex(const float* d_logits, int ldl, int T, int NE, i
     IZB_FAIL(IZB_ERR_SHAPE, "moe_route: T=%d NE=%d NU=%d ldl=%d (NE <= 512, NU <= 32, ldl >= NE, + 1 with a shared-expert gate)", T, NE, NU, ldl);
   cudaStream_t st = (cudaStream_t)stream;
   const int warps = T <= kRouteWarps ? T : 8, grid = (T + warps - 1) / warps;
+  auto kernel = NE <= 128 ? moe_route_kernel<4> : NE <= 256 ? moe_route_kernel<8> : moe_route_kernel<kMaxPerLane>;
   if (grid > 1) IZB_CUDA(cudaMemsetAsync(d_counts, 0, (size_t)NE * 4, st));
-  IZB_LAUNCH("moe_route", st, izb_launch_pdl(moe_route_kernel, grid, warps * 32, 0, st, d_logits, ldl, T, NE, NU, d_ids, d_wts, d_counts, d_sgate));
+  IZB_LAUNCH("moe_route", st, izb_launch_pdl(kernel, grid, warps * 32, 0, st, d_logits, ldl, T, NE, NU, d_ids, d_wts, d_counts, d_sgate));
   return IZB_OK;
 }
 
