@@ -294,74 +294,98 @@ __device__ __forceinline__ int q4k_perm8(int p) { return (p & 4) | ((p & 1) << 1
 // and, with sps == 5 (the Q4_K GEMM), after every four stages one more 16 KB image: the min-term factor
 // v = asc * (float)asum of the superblock's eight blocks as three bf16 terms, laid out as the six 16-byte K-chunks
 // (v1, v1, v2, v1, v2, v3) x eight blocks that meet the weight side's (u1, u2, u1, u3, u2, u1).
-// One thread per (row, 16-byte output chunk).
+// Bound by its writes, so one CTA = 32 rows x one superblock: the image goes out in whole 128-byte lines, and scales and min terms, whose
+// neighbours in memory belong to other rows, are collected in shared memory first.  (One thread per chunk, rows one after the other, wrote
+// them as 4- and 2-byte pieces: 32768 gathered rows of K = 2048 took 94 us, now @@.)
+struct PrepRows {
+  float sc[8][33], v[8][33];  // [block of the superblock][row]: scale, scale * sum
+};
+// (after a barrier) the scales and, sps == 5, the min-term chunks of the 32 rows from row r0 of the tile on
+__device__ __forceinline__ void put_scales(const PrepRows& p, float* __restrict__ ascimg, uint8_t* tile_img, int tile, int K, int sb, int r0, int sps) {
+  {
+    const int b = threadIdx.x >> 5, r = threadIdx.x & 31;
+    ascimg[((size_t)tile * (K / 32) + sb * 8 + b) * BM + r0 + r] = p.sc[b][r];
+  }
+  if (sps != 5) return;
+  const int r = threadIdx.x >> 3, k = threadIdx.x & 7;
+  if (k >= 6) return;
+  const int term = k == 2 || k == 4 ? 1 : k == 5 ? 2 : 0;
+  uint32_t o[4];
+#pragma unroll
+  for (int b = 0; b < 8; ++b) {
+    const float v = p.v[b][r];
+    const __nv_bfloat16 h1 = __float2bfloat16_rn(v);
+    const float r1 = __fsub_rn(v, __bfloat162float(h1));
+    const __nv_bfloat16 h2 = __float2bfloat16_rn(r1);
+    const __nv_bfloat16 h3 = __float2bfloat16_rn(__fsub_rn(r1, __bfloat162float(h2)));
+    const uint32_t h = __bfloat16_as_ushort(term == 0 ? h1 : term == 1 ? h2 : h3);
+    o[b >> 1] = (b & 1) ? o[b >> 1] | (h << 16) : h;
+  }
+  *reinterpret_cast<uint4*>(tile_img + ((size_t)sb * 5 + 4) * STAGE_BYTES + (r0 + r) * 128 + ((k ^ (r & 7)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
+}
+// the operand chunk of eight int8 values: row r of the tile, chunk `c` (0 .. 31) of superblock sb
+template <bool kPerm>
+__device__ __forceinline__ void put_chunk(uint8_t* tile_img, int sb, int sps, int r, int c, const int (&q)[8]) {
+  uint32_t o[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int e0 = kPerm ? q4k_perm8(2 * j) : 2 * j, e1 = kPerm ? q4k_perm8(2 * j + 1) : 2 * j + 1;
+    const __half2 h = __floats2half2_rn((float)q[e0], (float)q[e1]);
+    o[j] = *reinterpret_cast<const uint32_t*>(&h);
+  }
+  *reinterpret_cast<uint4*>(tile_img + ((size_t)sb * sps + (c >> 3)) * STAGE_BYTES + r * 128 + (((c & 7) ^ (r & 7)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
+}
+
 template <bool kPerm>
 __global__ void __launch_bounds__(256) act_prepare_kernel(const int8_t* __restrict__ aq, const float* __restrict__ asc, int lda,
                                                           int K, int rows_total, const int32_t* __restrict__ tiles,
                                                           const int32_t* __restrict__ rowmap, uint16_t* __restrict__ aimg,
                                                           float* __restrict__ ascimg, int sps,
                                                           uint32_t* __restrict__ part_bad) {
-  const int tile = blockIdx.y;
+  __shared__ PrepRows s;
+  const int sb = blockIdx.y, tile = blockIdx.x >> 2, m0 = (blockIdx.x & 3) * 32, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int r0, nr;
   pdl_launch_next();
   pdl_wait();
-  if (part_bad && blockIdx.x == 0 && tile == 0 && threadIdx.x == 0) *part_bad = 0;
+  if (part_bad && sb == 0 && blockIdx.x == 0 && threadIdx.x == 0) *part_bad = 0;
   if (tiles) {
     if (tile >= tiles[0]) return;
     r0 = tiles[2 + 3 * tile];
     nr = tiles[3 + 3 * tile];
+    if (m0 >= nr) return;  // (rows past the tile's slots reach no result: every accumulator row belongs to one operand row)
   } else {
     r0 = tile * BM;
     nr = min(BM, rows_total - r0);
   }
-  const int nchunk = K / 8;                      // 16-byte output chunks per row
-  const int idx = blockIdx.x * 256 + threadIdx.x;  // over 128 rows x nchunk, chunk fastest
-  if (idx >= BM * nchunk) return;
-  const int r = idx / nchunk, ch = idx % nchunk;
-  const int stage = ch >> 3, c = ch & 7;
-  int src = -1;
-  if (r < nr) src = rowmap ? rowmap[r0 + r] : r0 + r;
-  uint2 v = make_uint2(0, 0);
-  if (src >= 0) v = *reinterpret_cast<const uint2*>(aq + (size_t)src * K + (size_t)ch * 8);
-  int a[8];
+  // this lane's row of the 32, for the scales; the rows a warp copies come from it by shuffle
+  const int src = m0 + lane < nr ? (rowmap ? rowmap[r0 + m0 + lane] : r0 + m0 + lane) : -1;
+  if (asc) s.sc[warp][lane] = src >= 0 ? asc[(size_t)(sb * 8 + warp) * lda + src] : 0.0f;  // (null in the block-dot verification mode)
+  uint2 x[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    a[i] = (int)(int8_t)(v.x >> (8 * i));
-    a[4 + i] = (int)(int8_t)(v.y >> (8 * i));
+    const int from = __shfl_sync(0xFFFFFFFFu, src, warp + 8 * i);
+    x[i] = from >= 0 ? *reinterpret_cast<const uint2*>(aq + (size_t)from * K + sb * 256 + lane * 8) : make_uint2(0, 0);
   }
-  uint32_t o[4];
+  __syncthreads();
+  uint8_t* tile_img = reinterpret_cast<uint8_t*>(aimg) + (size_t)tile * (K / 256) * sps * STAGE_BYTES;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const int e0 = kPerm ? q4k_perm8(2 * i) : 2 * i, e1 = kPerm ? q4k_perm8(2 * i + 1) : 2 * i + 1;
-    const __half2 h = __floats2half2_rn((float)a[e0], (float)a[e1]);
-    o[i] = *reinterpret_cast<const uint32_t*>(&h);
-  }
-  const size_t nstages = (size_t)(K / 256) * sps;
-  uint8_t* tile_img = reinterpret_cast<uint8_t*>(aimg) + (size_t)tile * nstages * STAGE_BYTES;
-  uint8_t* dst = tile_img + ((size_t)(stage >> 2) * sps + (stage & 3)) * STAGE_BYTES + r * 128 + ((c ^ (r & 7)) << 4);
-  *reinterpret_cast<uint4*>(dst) = make_uint4(o[0], o[1], o[2], o[3]);
-  if (asc) {  // (null in the block-dot verification mode: no scales are used)
-    int s = a[0] + a[1] + a[2] + a[3] + a[4] + a[5] + a[6] + a[7];
-    s += __shfl_xor_sync(0xFFFFFFFFu, s, 1);
-    s += __shfl_xor_sync(0xFFFFFFFFu, s, 2);  // the four chunks of a 32-block are four consecutive threads of one row
-    if ((ch & 3) == 0) {
-      const int b = ch >> 2;
-      const float sc = src >= 0 ? asc[(size_t)b * lda + src] : 0.0f;
-      ascimg[((size_t)tile * (K / 32) + b) * BM + r] = sc;
-      if (sps == 5) {
-        const float v = __fmul_rn(sc, (float)s);
-        const __nv_bfloat16 h1 = __float2bfloat16_rn(v);
-        const float r1 = __fsub_rn(v, __bfloat162float(h1));
-        const __nv_bfloat16 h2 = __float2bfloat16_rn(r1);
-        const __nv_bfloat16 h3 = __float2bfloat16_rn(__fsub_rn(r1, __bfloat162float(h2)));
-        uint8_t* row = tile_img + ((size_t)(b >> 3) * 5 + 4) * STAGE_BYTES + r * 128 + 2 * (b & 7);
-        const unsigned short t3[3] = {__bfloat16_as_ushort(h1), __bfloat16_as_ushort(h2), __bfloat16_as_ushort(h3)};
-        constexpr int term[6] = {0, 0, 1, 0, 1, 2};
+    const int rr = warp + 8 * i;
+    int a[8];
 #pragma unroll
-        for (int k = 0; k < 6; ++k) *reinterpret_cast<unsigned short*>(row + ((k ^ (r & 7)) << 4)) = t3[term[k]];
-      }
+    for (int k = 0; k < 4; ++k) {
+      a[k] = (int)(int8_t)(x[i].x >> (8 * k));
+      a[4 + k] = (int)(int8_t)(x[i].y >> (8 * k));
     }
+    put_chunk<kPerm>(tile_img, sb, sps, m0 + rr, lane, a);
+    int sum = a[0] + a[1] + a[2] + a[3] + a[4] + a[5] + a[6] + a[7];
+    sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 1);
+    sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 2);  // the four chunks of a 32-block
+    if ((lane & 3) == 0) s.v[lane >> 2][rr] = __fmul_rn(s.sc[lane >> 2][rr], (float)sum);
   }
+  if (!asc) return;
+  __syncthreads();
+  put_scales(s, ascimg, tile_img, tile, K, sb, m0, sps);
 }
 
 // ---------------------------------------------------------------------------------------------- quantiser + pre-pass in one
@@ -375,10 +399,11 @@ __global__ void __launch_bounds__(256) quant_prepare_kernel(const float* __restr
                                                             int8_t* __restrict__ aq, float* __restrict__ asc,
                                                             uint16_t* __restrict__ aimg, float* __restrict__ ascimg, int sps, int n_tiles,
                                                             uint32_t* __restrict__ part_bad) {
-  __shared__ float s_sc[8][33];
+  __shared__ PrepRows s_rows;
   const int sb = blockIdx.x, m0 = blockIdx.y * 32, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int col = sb * 256 + lane * 8;
-  const size_t nstages = (size_t)(K / 256) * sps;
+  const int tile = m0 >> 7;  // (32 rows lie in one tile)
+  uint8_t* tile_img = reinterpret_cast<uint8_t*>(aimg) + (size_t)tile * (K / 256) * sps * STAGE_BYTES;
   pdl_launch_next();
   pdl_wait();
   if (part_bad && sb == 0 && blockIdx.y == 0 && threadIdx.x == 0) *part_bad = 0;
@@ -422,42 +447,18 @@ __global__ void __launch_bounds__(256) quant_prepare_kernel(const float* __restr
       pk.y = (q[4] & 0xFF) | ((q[5] & 0xFF) << 8) | ((q[6] & 0xFF) << 16) | ((uint32_t)(q[7] & 0xFF) << 24);
       *reinterpret_cast<uint2*>(aq + (size_t)m * K + col) = pk;
     }
-    if ((lane & 3) == 0) s_sc[lane >> 2][rr] = sc;
-    // ---- the operand image of this chunk: tile m / 128, row m % 128, stage lane / 8 of the superblock, chunk lane % 8
-    const int tile = m >> 7, r = m & 127;
-    if (tile >= n_tiles) continue;  // (padding rows past the last tile the GEMM reads: aq / asc only)
-    uint8_t* tile_img = reinterpret_cast<uint8_t*>(aimg) + (size_t)tile * nstages * STAGE_BYTES;
-    uint32_t o[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int e0 = kPerm ? q4k_perm8(2 * j) : 2 * j, e1 = kPerm ? q4k_perm8(2 * j + 1) : 2 * j + 1;
-      const __half2 h = __floats2half2_rn((float)q[e0], (float)q[e1]);
-      o[j] = *reinterpret_cast<const uint32_t*>(&h);
-    }
-    *reinterpret_cast<uint4*>(tile_img + ((size_t)sb * sps + (lane >> 3)) * STAGE_BYTES + r * 128 + (((lane & 7) ^ (r & 7)) << 4)) =
-        make_uint4(o[0], o[1], o[2], o[3]);
     if ((lane & 3) == 0) {
-      const int b = lane >> 2;  // block of the superblock
-      ascimg[((size_t)tile * (K / 32) + sb * 8 + b) * BM + r] = sc;
-      if (sps == 5) {
-        const float t = __fmul_rn(sc, (float)s);
-        const __nv_bfloat16 h1 = __float2bfloat16_rn(t);
-        const float r1 = __fsub_rn(t, __bfloat162float(h1));
-        const __nv_bfloat16 h2 = __float2bfloat16_rn(r1);
-        const __nv_bfloat16 h3 = __float2bfloat16_rn(__fsub_rn(r1, __bfloat162float(h2)));
-        uint8_t* row = tile_img + ((size_t)sb * 5 + 4) * STAGE_BYTES + r * 128 + 2 * b;
-        const unsigned short t3[3] = {__bfloat16_as_ushort(h1), __bfloat16_as_ushort(h2), __bfloat16_as_ushort(h3)};
-        constexpr int term[6] = {0, 0, 1, 0, 1, 2};
-#pragma unroll
-        for (int k = 0; k < 6; ++k) *reinterpret_cast<unsigned short*>(row + ((k ^ (r & 7)) << 4)) = t3[term[k]];
-      }
+      s_rows.sc[lane >> 2][rr] = sc;
+      s_rows.v[lane >> 2][rr] = __fmul_rn(sc, (float)s);
     }
+    if (tile < n_tiles) put_chunk<kPerm>(tile_img, sb, sps, m & 127, lane, q);  // (padding rows past the last tile the GEMM reads: aq / asc only)
   }
   __syncthreads();
   {
     const int b = threadIdx.x >> 5, r = threadIdx.x & 31;
-    if (m0 + r < Mp) asc[(size_t)(sb * 8 + b) * Mp + m0 + r] = s_sc[b][r];
+    if (m0 + r < Mp) asc[(size_t)(sb * 8 + b) * Mp + m0 + r] = s_rows.sc[b][r];
   }
+  if (tile < n_tiles) put_scales(s_rows, ascimg, tile_img, tile, K, sb, m0 & 127, sps);
 }
 
 // ---------------------------------------------------------------------------------------------- the GEMM kernel
@@ -1150,7 +1151,7 @@ int run_tc_on(const izb_weight* w, int mat, const int8_t* aq, const float* asc, 
   uint16_t* aimg = (uint16_t*)ws;
   float* ascimg = (float*)((unsigned char*)ws + img_bytes);
   if (!reuse_images) {
-    dim3 pg((BM * (K / 8) + 255) / 256, n_tiles_grid);
+    dim3 pg(n_tiles_grid * 4, K / 256);
     auto kernel = w->type == IZB_Q4_K ? act_prepare_kernel<true> : act_prepare_kernel<false>;
     IZB_LAUNCH("act_prepare", st, izb_launch_pdl(kernel, pg, 256, 0, st, aq, asc, lda, K, rows_total, tiles, rowmap, aimg, ascimg, sps, split_flag(split_ws, w->device)));
   }

@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(kRouteWarps * 32) moe_route_kernel(const float
 // counts over the warp (shuffles) and over the eight warps (shared memory, double-buffered so that one barrier per pass is enough)
 // gives every pair of the expert its slot.  (A pass is a chain of load, scan and barrier: with four pairs per thread 32768 pairs
 // were 32 of them, 38 us.)  The pairs found go to a list in shared memory that all threads write out when another pass might not fit:
-// written where they are found, each waits for its weight's load by itself (27 us; @@ us like this).
+// written where they are found, each waits for its weight's load by itself (32768 pairs, 128 experts: 27 us against 19).
 constexpr int kPairs = 16, kPairList = 2 * 256 * kPairs;
 __global__ void __launch_bounds__(256) moe_sort_kernel(const int32_t* __restrict__ ids, const float* __restrict__ wts, const int32_t* __restrict__ counts, int n, int NU,
                                                        int NE, int TM, int32_t* __restrict__ offs, int32_t* __restrict__ tiles, int max_tiles, int32_t* __restrict__ stok,
