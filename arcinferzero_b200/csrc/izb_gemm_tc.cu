@@ -1121,13 +1121,15 @@ int tc_grid(int device, int n_work) {
   return n_work < sms ? (n_work > 0 ? n_work : 1) : sms;
 }
 
-// Parts the K range of every output tile is cut into, when the tiles alone would leave more than half the SMs idle: as many
-// as fill them once, each at least one superblock.  The parts' sums are at most one 64 KB tile per SM.  Plain stores only: sums cut
-// in parts are rounded in other places, and what the other store modes write (the residual, the SwiGLU product) is quantised to int8
-// next, where a last bit can become a whole step.
+// Parts the K range of every output tile is cut into, when the tiles alone would leave more than half the SMs idle: as many as fill
+// them once, each at least two superblocks.  The parts' sums are at most one 64 KB tile per SM.  Long K and plain stores only.  Short K:
+// a part's pipeline fill and the summing launch eat the gain (K = 1024: some 10 us uncut).  Other store modes: sums cut in parts are
+// rounded in other places, and what those modes write (the residual, the SwiGLU product) is quantised to int8 next, where a last bit
+// can become a whole step.
 int tc_split(int device, int n_items, int nsb) {
+  if (nsb < 8) return 1;
   const int s = izb_sm_budget(device) / (n_items > 0 ? n_items : 1);
-  return s < 2 ? 1 : s < nsb ? s : nsb;
+  return s < 2 ? 1 : s < nsb / 2 ? s : nsb / 2;
 }
 constexpr size_t kSplitBytes = (size_t)BM * BN * 4;  // per SM; the flag of a failed part follows them
 
