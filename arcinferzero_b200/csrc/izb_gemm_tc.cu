@@ -296,7 +296,7 @@ __device__ __forceinline__ int q4k_perm8(int p) { return (p & 4) | ((p & 1) << 1
 // (v1, v1, v2, v1, v2, v3) x eight blocks that meet the weight side's (u1, u2, u1, u3, u2, u1).
 // Bound by its writes, so one CTA = 32 rows x one superblock: the image goes out in whole 128-byte lines, and scales and min terms, whose
 // neighbours in memory belong to other rows, are collected in shared memory first.  (One thread per chunk, rows one after the other, wrote
-// them as 4- and 2-byte pieces: 32768 gathered rows of K = 2048 took 94 us, now @@.)
+// them as 4- and 2-byte pieces: 32768 gathered rows of K = 2048 took 94 us, now 42.)
 struct PrepRows {
   float sc[8][33], v[8][33];  // [block of the superblock][row]: scale, scale * sum
 };
@@ -678,7 +678,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
   auto bar = [&](int i) -> uint32_t { return bar0 + 8u * (uint32_t)i; };
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-  pdl_launch_next();
   if (threadIdx.x == 0) {
     // Consumers release a buffer with one arrival per THREAD (128 dequantisers, 256 combine threads): one elected arrival per
     // warp, predicated without a branch, measured 5 % slower (8192 x 17408 x 5120: 3.25 against 3.10 ms).  A_EMPTY / B_EMPTY: one
@@ -701,7 +700,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  pdl_wait();
 
   // ---- the CTA's work: items blockIdx.x, blockIdx.x + gridDim.x, ... of (row tiles) x (column tiles) x (K parts), K part
   // fastest, then column tile.  Every role walks the same list; its ring positions and barrier parities run on from item to
@@ -1100,7 +1098,10 @@ int launch_tc(const izb_weight* w, TcParams& p, dim3 grid, cudaStream_t st) {
   p.skip_stage = g_test_skip.exchange(-1);
   CUtensorMap tm;
   memcpy(&tm, w->tmap_raw, sizeof tm);
-  IZB_LAUNCH("gemm_tc", st, izb_launch_pdl(gemm_tc_kernel<F, kDots>, grid, kThreads, SMEM_BYTES, st, tm, p));
+  // No programmatic dependent launch, on either side.  CTAs placed while the pre-pass drains land on the SMs in the order in which these
+  // fall free, and neighbouring items, which share operands, no longer run on neighbours (the down projections of 4096 tokens x 8
+  // experts: 392 us against 345); CTAs of the next kernel that wait beside these cost 10 us when it is a wide one.
+  IZB_LAUNCH("gemm_tc", st, gemm_tc_kernel<F, kDots><<<grid, kThreads, SMEM_BYTES, st>>>(tm, p));
   return IZB_OK;
 }
 int launch_tc_of(const izb_weight* w, TcParams& p, dim3 grid, cudaStream_t st) {
