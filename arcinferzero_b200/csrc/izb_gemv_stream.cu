@@ -607,13 +607,18 @@ int launch_q4k_pair_k(const izb_weight* w, const uint8_t* raw, const int8_t* aq,
 // ONE row per pass (two independent dependency chains), its rows one after the other; the copies of the chunks
 // `slots / 2` passes ahead are in flight, across row boundaries.  K = 1024 * odd ends in a chunk of four superblocks
 // (lanes 16..31 repeat lanes 0..15 there and are dropped).  Activations staged per lane in shared memory (1..4 rows).
+//
+// The rows of the last round, too few for every warp to have one (5120 rows: 384 after two rounds of 2368), would leave most warps idle
+// for a row's whole chain of passes.  They are dealt out pass by pass instead (`tail` rows per CTA): the per-lane sums of a pass
+// go to shared memory, and one warp per row adds them in pass order, the order of the loop.  (5120 x 17408, one row: 17.1 us before,
+// @@ now.)
 constexpr int kChunkBytes = 8 * 144;
 
 template <int T>
 __global__ void __launch_bounds__(kPairWarps * 32, 1) gemv_q4k_chunk_kernel(const uint8_t* __restrict__ raw, int N, int K,
                                                                            const int8_t* __restrict__ aq, const float* __restrict__ asc,
                                                                            int Mp, float* __restrict__ C, int ldc, int c_off, int acc,
-                                                                           int slots, uint32_t* err) {
+                                                                           int slots, int tail, uint32_t* err) {
   extern __shared__ __align__(128) unsigned char smem[];
   const int nsb = K >> 8, FS = nsb >> 3, WS = (nsb + 7) >> 3;  // chunks per row: FS whole ones (+ one of four superblocks)
   const int PP = (WS + 1) >> 1;                                 // passes per row (two chunks each, the last maybe one)
@@ -621,16 +626,42 @@ __global__ void __launch_bounds__(kPairWarps * 32, 1) gemv_q4k_chunk_kernel(cons
   const int act_bytes = WS * T * kPairActBytes;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int W = gridDim.x * kPairWarps, w0 = blockIdx.x * kPairWarps + warp;
-  const int my_rows = w0 < N ? (N - w0 + W - 1) / W : 0;
-  const int total = my_rows * PP;  // passes of this warp, in order (row, pass)
+  // whole rows of this warp, then (tail) its passes of the CTA's last rows: first + k * gridDim.x
+  const int my_rows = tail ? N / W : w0 < N ? (N - w0 + W - 1) / W : 0;
+  const int body = my_rows * PP, first = my_rows * W + blockIdx.x;
+  const int here = tail && first < N ? (N - first + gridDim.x - 1) / gridDim.x : 0;
+  const int total = body + (here * PP > warp ? (here * PP - warp + kPairWarps - 1) / kPairWarps : 0);  // passes of this warp, in order
+  // pass n of them: chunks c0, c0 + 1 of `row`, in slots 2 q, + 1 (stepped, not computed: the divisions were a third of the
+  // loop's instructions)
+  struct Pass {
+    int n, row, c0, q;
+    uint32_t parity;
+  };
+  auto settle = [&](Pass& p) {  // (n == body: over to the last rows)
+    if (p.n == body) { p.row = first; p.c0 = 2 * warp; }
+    if (p.n >= body)
+      while (p.c0 >= 2 * PP) { p.c0 -= 2 * PP; p.row += gridDim.x; }
+  };
+  auto step = [&](Pass& p) {
+    ++p.n;
+    p.c0 += p.n <= body ? 2 : 2 * kPairWarps;
+    if (p.n < body && p.c0 >= 2 * PP) { p.c0 = 0; p.row += W; }
+    if (++p.q == slots >> 1) { p.q = 0; p.parity ^= 1; }
+    settle(p);
+  };
   const int sub = lane >> 2, pp = lane & 3, hs = slots >> 1;
   unsigned char* act = smem;
   unsigned char* ring = smem + act_bytes + (size_t)warp * slots * kChunkBytes;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + act_bytes + (size_t)kPairWarps * slots * kChunkBytes) + warp * slots;
-  // pass n -> copies of chunks 2 * (n % PP), + 1 of row n / PP into slots 2 * (n % hs), + 1
-  auto issue = [&](int n) {
-    const int ri = n / PP, c0 = 2 * (n - ri * PP), q = n % hs;
-    const uint8_t* src = raw + (size_t)(w0 + ri * W) * row_bytes + (size_t)c0 * kChunkBytes;
+  float* part = reinterpret_cast<float*>(smem + act_bytes + (size_t)kPairWarps * slots * kChunkBytes);  // [last row][pass][T][lane]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(part + (size_t)tail * PP * T * 32) + warp * slots;
+  __shared__ int s_gave_up;
+  if (threadIdx.x == 0) s_gave_up = 0;
+  Pass ask = {0, w0, 0, 0, 0}, at = ask;  // (lane 0 asks)
+  settle(ask);
+  settle(at);
+  auto issue = [&]() {
+    const int c0 = ask.c0, q = ask.q;
+    const uint8_t* src = raw + (size_t)ask.row * row_bytes + (size_t)c0 * kChunkBytes;
     row_copy(s_u32(ring + (size_t)(2 * q) * kChunkBytes), src, c0 < FS ? kChunkBytes : kChunkBytes / 2, s_u32(&bars[2 * q]));
     if (c0 + 1 < WS)
       row_copy(s_u32(ring + (size_t)(2 * q + 1) * kChunkBytes), src + kChunkBytes, c0 + 1 < FS ? kChunkBytes : kChunkBytes / 2, s_u32(&bars[2 * q + 1]));
@@ -640,7 +671,7 @@ __global__ void __launch_bounds__(kPairWarps * 32, 1) gemv_q4k_chunk_kernel(cons
   if (lane == 0) {
     for (int s = 0; s < slots; ++s) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(s_u32(&bars[s])) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    for (int n = 0; n < hs && n < total; ++n) issue(n);
+    for (; ask.n < hs && ask.n < total; step(ask)) issue();
   }
   pdl_launch_next();
   pdl_wait();  // (see gemv_q4k_reg_kernel: the ring fill above runs ahead of it)
@@ -675,6 +706,17 @@ __global__ void __launch_bounds__(kPairWarps * 32, 1) gemv_q4k_chunk_kernel(cons
   float accv[T];
 #pragma unroll
   for (int t = 0; t < T; ++t) accv[t] = 0.0f;
+  auto put = [&](int row) {
+#pragma unroll
+    for (int t = 0; t < T; ++t) {
+      const float v = warp_sum(accv[t]);
+      if (lane == 0) {
+        float* cp = C + (size_t)t * ldc + c_off + row;
+        *cp = acc ? *cp + v : v;
+      }
+      accv[t] = 0.0f;
+    }
+  };
   // one chunk against every token: the chunk's nibbles are masked once
   auto chunk = [&](const unsigned char* wp, uint32_t ho, uint32_t qo, const unsigned char* abase, float (&out)[T]) {
     const uint4 h = *reinterpret_cast<const uint4*>(wp + ho);
@@ -709,9 +751,9 @@ __global__ void __launch_bounds__(kPairWarps * 32, 1) gemv_q4k_chunk_kernel(cons
       out[t] = fmaf(df.x, tq, -df.y * tm);
     }
   };
-  for (int n = 0; n < total; ++n) {
-    const int ri = n / PP, c0 = 2 * (n - ri * PP), q = n % hs;
-    const uint32_t parity = (uint32_t)(n / hs) & 1u;
+  for (; at.n < total; step(at)) {
+    const int n = at.n, row = at.row, c0 = at.c0, q = at.q;
+    const uint32_t parity = at.parity;
     const bool two = c0 + 1 < WS;  // (uniform over the warp)
     bool ready = false;
     for (uint32_t it = 0; it < kSpin && !ready; ++it) ready = try_wait(s_u32(&bars[2 * q]), parity);
@@ -721,6 +763,7 @@ __global__ void __launch_bounds__(kPairWarps * 32, 1) gemv_q4k_chunk_kernel(cons
     }
     if (!ready) {  // (bounded wait gave up)
       if (lane == 0) atomicOr(err, 64u);
+      s_gave_up = 1;
       break;
     }
     const unsigned char* wa = ring + (size_t)(2 * q) * kChunkBytes;
@@ -740,19 +783,27 @@ __global__ void __launch_bounds__(kPairWarps * 32, 1) gemv_q4k_chunk_kernel(cons
       for (int t = 0; t < T; ++t) accv[t] += k0 * r0[t];
     }
     __syncwarp();
-    if (lane == 0 && n + hs < total) issue(n + hs);  // the slots are read: the pass `hs` ahead goes into them
-    if (c0 + 2 >= WS) {  // the row is complete
-      const int row = w0 + ri * W;
+    if (lane == 0 && ask.n < total) {  // the slots are read: the pass `hs` ahead goes into them
+      issue();
+      step(ask);
+    }
+    if (n >= body) {  // a pass of a last row
 #pragma unroll
       for (int t = 0; t < T; ++t) {
-        const float v = warp_sum(accv[t]);
-        if (lane == 0) {
-          float* cp = C + (size_t)t * ldc + c_off + row;
-          *cp = acc ? *cp + v : v;
-        }
+        part[((size_t)(warp + kPairWarps * (n - body)) * T + t) * 32 + lane] = accv[t];
         accv[t] = 0.0f;
       }
+    } else if (c0 + 2 >= WS) {  // the row is complete
+      put(row);
     }
+  }
+  if (!tail) return;
+  __syncthreads();
+  if (warp < here && !s_gave_up) {
+    for (int p = 0; p < PP; ++p)
+#pragma unroll
+      for (int t = 0; t < T; ++t) accv[t] += part[((size_t)(warp * PP + p) * T + t) * 32 + lane];
+    put(first + warp * gridDim.x);
   }
 }
 
@@ -763,18 +814,21 @@ int launch_q4k_chunk(const izb_weight* w, const uint8_t* raw, const int8_t* aq, 
   const int nsb = w->K / 256, WS = (nsb + 7) / 8;
   const size_t act = (size_t)WS * T * kPairActBytes;
   if (act + 4096 + (size_t)kPairWarps * 4 * kChunkBytes > kBudget) return 1;
-  int slots = (int)((kBudget - act - 4096) / ((size_t)kPairWarps * kChunkBytes));
+  // the last rows are dealt out by passes where that shortens the longest chain (it is at most half a row) and their sums are small
+  const int sms = izb_sm_count(w->device), PP = (WS + 1) / 2, rest = w->N % (sms * kPairWarps);
+  int tail = (rest + sms - 1) / sms, grid = sms;
+  const size_t part = (size_t)PP * T * 128;  // per row
+  if (tail > kPairWarps / 2 || act + tail * part + 4096 + (size_t)kPairWarps * 6 * kChunkBytes > kBudget) tail = 0;
+  int slots = (int)((kBudget - act - tail * part - 4096) / ((size_t)kPairWarps * kChunkBytes));
   slots = slots > 12 ? 12 : (slots & ~1);
-  const size_t smem = act + (size_t)kPairWarps * slots * kChunkBytes + (size_t)kPairWarps * slots * 8;
+  const size_t smem = act + tail * part + (size_t)kPairWarps * slots * kChunkBytes + (size_t)kPairWarps * slots * 8;
   IZB_SMEM_OPTIN((gemv_q4k_chunk_kernel<T>), kBudget + 8192, w->device);
-  const int sms = izb_sm_count(w->device);
-  int grid = sms;
   const int need = (w->N + kPairWarps - 1) / kPairWarps;
-  if (grid > need) grid = need;
+  if (!tail && grid > need) grid = need;
   uint32_t* err = izb_device_error_word(w->device);
   if (!err) IZB_FAIL(IZB_ERR_NOMEM, "gemv: no device error word");
   const int N = w->N, K = w->K;
-  IZB_LAUNCH("gemv", st, izb_launch_pdl(gemv_q4k_chunk_kernel<T>, grid, kPairWarps * 32, smem, st, raw, N, K, aq, asc, Mp, C, ldc, c_off, acc, slots, err));
+  IZB_LAUNCH("gemv", st, izb_launch_pdl(gemv_q4k_chunk_kernel<T>, grid, kPairWarps * 32, smem, st, raw, N, K, aq, asc, Mp, C, ldc, c_off, acc, slots, tail, err));
   return IZB_OK;
 }
 
