@@ -610,8 +610,8 @@ int launch_q4k_pair_k(const izb_weight* w, const uint8_t* raw, const int8_t* aq,
 //
 // The rows of the last round, too few for every warp to have one (5120 rows: 384 after two rounds of 2368), would leave most warps idle
 // for a row's whole chain of passes.  They are dealt out pass by pass instead (`tail` rows per CTA): the per-lane sums of a pass
-// go to shared memory, and one warp per row adds them in pass order, the order of the loop.  (5120 x 17408, one row: 17.1 us before,
-// @@ now.)
+// go to shared memory, and one warp per row adds them in pass order, the order of the loop.  (5120 x 17408, one to four activation
+// rows: 17.2, 21.2, 25.6, 31.3 us before, 15.8, 18.7, 20.9, 25.3 like this and with stepped positions.)
 constexpr int kChunkBytes = 8 * 144;
 
 template <int T>
@@ -814,11 +814,13 @@ int launch_q4k_chunk(const izb_weight* w, const uint8_t* raw, const int8_t* aq, 
   const int nsb = w->K / 256, WS = (nsb + 7) / 8;
   const size_t act = (size_t)WS * T * kPairActBytes;
   if (act + 4096 + (size_t)kPairWarps * 4 * kChunkBytes > kBudget) return 1;
-  // the last rows are dealt out by passes where that shortens the longest chain (it is at most half a row) and their sums are small
+  // the last rows are dealt out by passes where that shortens the longest chain of passes by more than an eighth (8192 x 8192, seven
+  // for eight, lost 8 % to the exchange) and their sums leave room for rings
   const int sms = izb_sm_count(w->device), PP = (WS + 1) / 2, rest = w->N % (sms * kPairWarps);
   int tail = (rest + sms - 1) / sms, grid = sms;
   const size_t part = (size_t)PP * T * 128;  // per row
-  if (tail > kPairWarps / 2 || act + tail * part + 4096 + (size_t)kPairWarps * 6 * kChunkBytes > kBudget) tail = 0;
+  const int saved = PP - (tail * PP + kPairWarps - 1) / kPairWarps;
+  if (tail > kPairWarps / 2 || saved * 8 <= (w->N / (sms * kPairWarps) + 1) * PP || act + tail * part + 4096 + (size_t)kPairWarps * 6 * kChunkBytes > kBudget) tail = 0;
   int slots = (int)((kBudget - act - tail * part - 4096) / ((size_t)kPairWarps * kChunkBytes));
   slots = slots > 12 ? 12 : (slots & ~1);
   const size_t smem = act + tail * part + (size_t)kPairWarps * slots * kChunkBytes + (size_t)kPairWarps * slots * 8;
