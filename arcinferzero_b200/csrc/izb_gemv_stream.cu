@@ -1,4 +1,5 @@
-// Streaming decode GEMV (1..8 activation rows): the kernel izb_gemv uses whenever its shared-memory plan fits.
+// Streaming decode GEMV (1..8 activation rows) for Q8_0 and Q4_K: what izb_gemv uses where the matrix instruction (csrc/izb_rows.cu) is
+// not faster and the shared-memory plan fits.
 // Same arithmetic as izb_gemv_body.cuh (zero/kernels/decode.cl:913-1034, :1581-1694); different data movement.
 //
 // A decode matrix streams in a few microseconds at HBM speed, so what decides the achieved bandwidth is how many weight

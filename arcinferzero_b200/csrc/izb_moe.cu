@@ -5,8 +5,9 @@
 //   moe_gateup   zero/kernels/decode_moe.cl:92-260   h = silu(x Wg^T) * (x Wu^T) per tile of <= TM slots of one expert
 //   moe_down     zero/kernels/decode_moe.cl:269-449  y = swt * (hq Wd^T)
 //   moe_combine  zero/kernels/moe.cl:344-352   x[t] += sum_k y[inv[t*NU+k]] in choice order
-// The per-tile kernels run the few-row GEMV loop (izb_gemv_body.cuh) over the rows of the tile's expert, with the
-// activation rows gathered through the slot -> token map, as the reference's moe_gateup_q / moe_down_q do.
+// The per-tile products run in csrc/izb_rows.cu; the kernels here (the few-row GEMV loop of izb_gemv_body.cuh over the rows of the tile's
+// expert) take what does not fit there: activations too long for shared memory, weights without a tensor map.  Both gather the
+// activation rows through the slot -> token map, as the reference's moe_gateup_q / moe_down_q do.
 #include "izb_gemv_body.cuh"
 
 namespace {

@@ -17,8 +17,8 @@
 // the same int8 quants -- a decode step over the Q6_K output head streams 0.875 instead of 1.19 bytes per weight.
 //
 // Kernels: a GEMV for 1..8 activation rows (warp per weight row, lane per 32-block, activations staged in shared memory)
-// and a CUDA-core GEMM with the per-superblock combine of the Q4_K kernel.  The tensor-core GEMM does not take K16 (its
-// exact-integer fp16 operand trick needs |scale * quant| < 2048; Q6_K reaches 4096).
+// and a CUDA-core GEMM with the per-superblock combine of the Q4_K kernel.  They serve Q6_K at one row (csrc/izb_rows.cu takes more), the
+// generic form at 1..8 rows, and GEMM calls that the tensor-core kernel (csrc/izb_gemm_tc.cu) does not take.
 #include <string.h>
 
 #include <vector>

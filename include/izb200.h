@@ -118,9 +118,10 @@ int izb_debug_wait_test(uint32_t spin_limit, int skip_stage);
  *   Q6_K (14)                   kept packed: the file's 210-byte superblock (ql | qh | 16 scales | d) in 224 bytes, unpacked
  *                               by the kernels to the same int8 quants (the output head and part of the FFN of the common
  *                               Q4_K_M files are Q6_K: a decode step streams 0.875 instead of 1.19 bytes per weight).
- *                               These three: GEMV for 1..8 rows and a CUDA-core GEMM, both with exact integer dots per
- *                               16-element half (zero/kernels/decode.cl:992-1004); not taken by the tensor-core GEMM, the
- *                               MoE entry points or izb_gemm_noalloc (IZB_ERR_TYPE / IZB_ERR_SHAPE). */
+ *                               These three: GEMV for 1..8 rows, the tensor-core GEMM under IZB_GEMM_AUTO (N % 16 == 0) and a
+ *                               CUDA-core GEMM, all with exact integer dots per 16-element half
+ *                               (zero/kernels/decode.cl:992-1004); not taken by IZB_GEMM_TC, the MoE entry points or
+ *                               izb_gemm_noalloc (IZB_ERR_TYPE / IZB_ERR_SHAPE). */
 int izb_weight_create(int ggml_type, const void* h_gguf_rows, int n_mats, int N, int K, int device, izb_weight** out);
 /* Tensor-parallel shard of a matrix (Engine::tp_slice, zero/mgpu/engine_tp_shard.h:202-234): rows [n0, n1) and input
  * columns [k0, k1) of every matrix; k0, k1 multiples of 256. */

@@ -15,7 +15,8 @@ def rel(a, b):
 
 
 @pytest.mark.parametrize("qt", [12, 8, 14])
-@pytest.mark.parametrize("N,K", [(8, 256), (17, 512), (1000, 768), (4104, 2304), (48, 17408), (3000, 4096)])
+# (48, 17408) and (2400, 6144): Q4_K rows left over after whole rounds, dealt out by passes
+@pytest.mark.parametrize("N,K", [(8, 256), (17, 512), (1000, 768), (4104, 2304), (48, 17408), (3000, 4096), (2400, 6144)])
 def test_rows_match_oracle(izb, qt, N, K):
     import torch
     w = S.make_weight(qt, N, K, N + K + qt)
