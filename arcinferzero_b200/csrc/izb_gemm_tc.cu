@@ -142,7 +142,8 @@ __device__ __forceinline__ uint32_t mbar_test(uint32_t bar, uint32_t parity) {
                : "memory");
   return ok;
 }
-// Bounded wait.  false = gave up (or another thread did): the caller leaves its loop.
+// Bounded wait of one thread.  false = gave up (or another thread did): the caller leaves its loop.  The lanes of a warp may get different
+// answers when the limit runs out: for roles whose threads work by themselves.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag, uint32_t* err,
                                           uint32_t limit, uint32_t code) {
   // (a satisfied wait is the common case: one non-blocking look costs less than the blocking form)
@@ -150,6 +151,22 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   for (uint32_t it = 0; it < limit; ++it) {
     if (mbar_try_wait(bar, parity)) return true;
     if ((it & 255u) == 255u && *abort_flag) return false;
+  }
+  *abort_flag = 1;
+  atomicOr(err, code);
+  return false;
+}
+// Bounded wait of a whole warp: every lane gets the same answer, so no lane leaves for the CTA's last barrier while the others go
+// on to an instruction that needs all 32 (elect.sync under the MMA and the commit, the TMEM reads, __syncwarp).  (A lane that has seen its
+// phase complete sees it again: the phase after it needs this warp.)  The vote costs nothing that shows: 8192 x 17408 x 5120 Q4_K 3.05 ms
+// with and without.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag, uint32_t* err,
+                                               uint32_t limit, uint32_t code) {
+  constexpr uint32_t kAll = 0xFFFFFFFFu;
+  if (__all_sync(kAll, mbar_test(bar, parity))) return true;
+  for (uint32_t it = 0; it < limit; ++it) {
+    if (__all_sync(kAll, mbar_try_wait(bar, parity))) return true;
+    if ((it & 255u) == 255u && __any_sync(kAll, *abort_flag)) return false;
   }
   *abort_flag = 1;
   atomicOr(err, code);
@@ -731,7 +748,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
         const Item it = item(w);
         const unsigned char* src = reinterpret_cast<const unsigned char*>(p.aimg) + (size_t)it.tile * nsb * SPS * STAGE_BYTES;
         for (int g = it.s0 * SPS; g < it.s1 * SPS; ++g) {
-          if (!mbar_wait(bar(MP::A_EMPTY + sa), pa, abort_flag, p.err, p.spin_limit, E_APROD)) { ok = false; break; }
+          if (!mbar_wait_warp(bar(MP::A_EMPTY + sa), pa, abort_flag, p.err, p.spin_limit, E_APROD)) { ok = false; break; }
           if (lane == 0 && g != p.skip_stage) {  // (skip_stage: diagnostics only, makes the waits of this stage run out)
             mbar_expect_tx(bar(MP::A_FULL + sa), STAGE_BYTES);
             bulk_g2s(smem_u32(smem + MP::OFF_A + sa * STAGE_BYTES), src + (size_t)g * STAGE_BYTES, STAGE_BYTES, bar(MP::A_FULL + sa));
@@ -749,14 +766,14 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
         const Item it = item(w);
         const int wrow = (p.tiles ? p.tiles[1 + 3 * it.tile] : p.mat) * p.N + it.nt * BN;
         for (int s = it.s0; s < it.s1; ++s) {
-          if (!mbar_wait(bar(MP::RAW_EMPTY + rb), pr, abort_flag, p.err, p.spin_limit, E_WPROD)) { ok = false; break; }
+          if (!mbar_wait_warp(bar(MP::RAW_EMPTY + rb), pr, abort_flag, p.err, p.spin_limit, E_WPROD)) { ok = false; break; }
           if (lane == 0) {
             mbar_expect_tx(bar(MP::RAW_FULL + rb), RAW);
             tma_2d(smem_u32(smem + MP::OFF_RAW + rb * RAW), &tmW, s * (SBB / 4), wrow, bar(MP::RAW_FULL + rb));
           }
           if (++rb == NR) { rb = 0; pr ^= 1; }
           if (!kDots) {
-            if (!mbar_wait(bar(MP::ASC_EMPTY + sq), pq, abort_flag, p.err, p.spin_limit, E_WPROD)) { ok = false; break; }
+            if (!mbar_wait_warp(bar(MP::ASC_EMPTY + sq), pq, abort_flag, p.err, p.spin_limit, E_WPROD)) { ok = false; break; }
             if (lane == 0) {
               mbar_expect_tx(bar(MP::ASC_FULL + sq), 4096);
               bulk_g2s(smem_u32(smem + MP::OFF_ASC + sq * 4096), p.ascimg + ((size_t)it.tile * nb + 8 * s) * BM, 4096, bar(MP::ASC_FULL + sq));
@@ -780,16 +797,17 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
           for (int t = warp - 1; t < (warp == 1 ? 4 : SPS) && ok; t += (t == 3 ? 1 : 2)) {
             const int g = gs + t, sa = g % NA, sb = g % NB;
             const uint32_t b_ok = mbar_test(bar(MP::B_FULL + sb), (g / NB) & 1), a_ok = mbar_test(bar(MP::A_FULL + sa), (g / NA) & 1);
-            if (!b_ok && !mbar_wait(bar(MP::B_FULL + sb), (g / NB) & 1, abort_flag, p.err, p.spin_limit, E_MMA)) { ok = false; break; }
-            if (!a_ok && !mbar_wait(bar(MP::A_FULL + sa), (g / NA) & 1, abort_flag, p.err, p.spin_limit, E_MMA)) { ok = false; break; }
+            if (!__all_sync(0xFFFFFFFFu, b_ok && a_ok)) {
+              if (!mbar_wait_warp(bar(MP::B_FULL + sb), (g / NB) & 1, abort_flag, p.err, p.spin_limit, E_MMA)) { ok = false; break; }
+              if (!mbar_wait_warp(bar(MP::A_FULL + sa), (g / NA) & 1, abort_flag, p.err, p.spin_limit, E_MMA)) { ok = false; break; }
+            }
             tc_fence_after();
             const uint32_t a_addr = smem_u32(smem + MP::OFF_A + sa * STAGE_BYTES), b_addr = smem_u32(smem + MP::OFF_B + sb * MP::BSTAGE);
             if (t < 4) {
 #pragma unroll
               for (int blk = 0; blk < 2; ++blk) {
                 const int j = jb + 2 * t + blk, d = j % ND1;
-                if (!mbar_wait(bar(MP::D1_EMPTY + d), ((j / ND1) & 1) ^ 1, abort_flag, p.err, p.spin_limit, E_MMA)) { ok = false; break; }
-                __syncwarp();
+                if (!mbar_wait_warp(bar(MP::D1_EMPTY + d), ((j / ND1) & 1) ^ 1, abort_flag, p.err, p.spin_limit, E_MMA)) { ok = false; break; }
                 tc_fence_after();
                 const uint32_t dt = tmem_base + (uint32_t)(d * BN);
 #pragma unroll
@@ -802,8 +820,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
               if (!ok) break;
             } else {
               // the min-term accumulator of the item before must have been read before this item's first MMA clears it
-              if (s == it.s0 && n_item > 0 && !mbar_wait(bar(MP::D2_EMPTY), (n_item - 1) & 1, abort_flag, p.err, p.spin_limit, E_MMA)) { ok = false; break; }
-              __syncwarp();
+              if (s == it.s0 && n_item > 0 && !mbar_wait_warp(bar(MP::D2_EMPTY), (n_item - 1) & 1, abort_flag, p.err, p.spin_limit, E_MMA)) { ok = false; break; }
               tc_fence_after();
 #pragma unroll
               for (int k16 = 0; k16 < 3; ++k16)
@@ -887,6 +904,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
     int d = 0, pd = 0, sq = 0, pq = 0;  // accumulator ring / scale ring positions and wait parities
     int sbc = 0, n_item = 0;            // superblocks and items done
     for (int w = blockIdx.x; w < n_work && ok; w += gridDim.x, ++n_item) {
+      __syncwarp();  // (rows that are not stored come here first)
       const Item it = item(w);
       const int n0 = it.nt * BN;
       const int r0 = p.tiles ? p.tiles[2 + 3 * it.tile] : it.tile * BM;
@@ -898,11 +916,11 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
       for (int c = 0; c < 32; ++c) res2[c] = tq2[c] = 0ull;
       for (int s = it.s0; s < it.s1 && ok; ++s, ++sbc) {
         const float* as = reinterpret_cast<const float*>(smem + MP::OFF_ASC + sq * 4096) + r;  // this row's 8 block scales
-        if (!kDots && !mbar_wait(bar(MP::ASC_FULL + sq), pq, abort_flag, p.err, p.spin_limit, E_EPI)) { ok = false; break; }
+        if (!kDots && !mbar_wait_warp(bar(MP::ASC_FULL + sq), pq, abort_flag, p.err, p.spin_limit, E_EPI)) { ok = false; break; }
 #pragma unroll
         for (int b = 0; b < 8; ++b) {
           const unsigned long long a2 = pack2(kDots ? 0.0f : as[b * BM]);
-          if (!mbar_wait(bar(MP::D1_FULL + d), pd, abort_flag, p.err, p.spin_limit, E_EPI)) { ok = false; break; }
+          if (!mbar_wait_warp(bar(MP::D1_FULL + d), pd, abort_flag, p.err, p.spin_limit, E_EPI)) { ok = false; break; }
           tc_fence_after();
 #pragma unroll
           for (int h = 0; h < 2; ++h) {  // 32 columns at a time: the block loop's working set stays inside the register budget
@@ -958,7 +976,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
         }
       }
       if (kMins && ok) {  // the min term of the whole K range (already negative)
-        ok = mbar_wait(bar(MP::D2_FULL), n_item & 1, abort_flag, p.err, p.spin_limit, E_EPI);
+        ok = mbar_wait_warp(bar(MP::D2_FULL), n_item & 1, abort_flag, p.err, p.spin_limit, E_EPI);
         if (ok) {
           tc_fence_after();
           unsigned long long v[32];
