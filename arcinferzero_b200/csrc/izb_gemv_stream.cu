@@ -28,6 +28,18 @@ __device__ __forceinline__ bool try_wait(uint32_t bar, uint32_t parity) {
                : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
   return ok != 0;
 }
+// Bounded wait of a whole warp for a ring slot.  Every lane gets the same answer: a lane that left alone would be missing in the warp sums,
+// and would wait at a barrier of the CTA for lanes that wait for it.
+__device__ __forceinline__ bool slot_wait(uint32_t bar, uint32_t parity) {
+  for (uint32_t it = 0; it < kSpin; ++it)
+    if (__all_sync(0xFFFFFFFFu, try_wait(bar, parity))) return true;
+  return false;
+}
+// after a wait that ran out: say so, and let copies still in flight land before shared memory is given up
+__device__ __forceinline__ void slot_gave_up(uint32_t* err) {
+  if ((threadIdx.x & 31) == 0) atomicOr(err, 64u);
+  for (int i = 0; i < 64; ++i) __nanosleep(20000);
+}
 __device__ __forceinline__ void row_copy(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src),
@@ -108,10 +120,8 @@ __global__ void __launch_bounds__(stream_warps<T>() * 32, 1) gemv_stream_kernel(
   uint32_t parity = 0;
   for (int i = 0; i < my_rows; ++i) {
     const int row = w0 + i * W;
-    bool ready = false;
-    for (uint32_t it = 0; it < kSpin && !ready; ++it) ready = try_wait(s_u32(&bars[slot]), parity);
-    if (!ready) {  // (bounded wait gave up)
-      if (lane == 0) atomicOr(err, 64u);
+    if (!slot_wait(s_u32(&bars[slot]), parity)) {
+      slot_gave_up(err);
       break;
     }
     const unsigned char* wrow = ring + (size_t)slot * slot_bytes;
@@ -282,14 +292,8 @@ __global__ void __launch_bounds__(kRegWarps * 32, 2) gemv_q4k_reg_kernel(const u
   uint32_t parity = 0;
   for (int i = 0; i < my_rows; i += 2) {
     const bool two = i + 1 < my_rows;  // (uniform over the warp)
-    bool ready = false;
-    for (uint32_t it = 0; it < kSpin && !ready; ++it) ready = try_wait(s_u32(&bars[slot]), parity);
-    if (ready && two) {
-      ready = false;
-      for (uint32_t it = 0; it < kSpin && !ready; ++it) ready = try_wait(s_u32(&bars[slot + 1]), parity);
-    }
-    if (!ready) {  // (bounded wait gave up)
-      if (lane == 0) atomicOr(err, 64u);
+    if (!slot_wait(s_u32(&bars[slot]), parity) || (two && !slot_wait(s_u32(&bars[slot + 1]), parity))) {
+      slot_gave_up(err);
       break;
     }
     const unsigned char* w0p = ring + (size_t)slot * slot_bytes;
@@ -447,14 +451,8 @@ __global__ void __launch_bounds__(kPairWarps * 32, 1) gemv_q4k_pair_kernel(const
   uint32_t parity = 0;
   for (int i = 0; i < my_rows; i += 2) {
     const bool two = i + 1 < my_rows;  // (uniform over the warp)
-    bool ready = false;
-    for (uint32_t it = 0; it < kSpin && !ready; ++it) ready = try_wait(s_u32(&bars[slot]), parity);
-    if (ready && two) {
-      ready = false;
-      for (uint32_t it = 0; it < kSpin && !ready; ++it) ready = try_wait(s_u32(&bars[slot + 1]), parity);
-    }
-    if (!ready) {  // (bounded wait gave up)
-      if (lane == 0) atomicOr(err, 64u);
+    if (!slot_wait(s_u32(&bars[slot]), parity) || (two && !slot_wait(s_u32(&bars[slot + 1]), parity))) {
+      slot_gave_up(err);
       break;
     }
     const unsigned char* wp[2] = {ring + (size_t)slot * slot_bytes, ring + (size_t)(two ? slot + 1 : slot) * slot_bytes};
@@ -756,14 +754,8 @@ __global__ void __launch_bounds__(kPairWarps * 32, 1) gemv_q4k_chunk_kernel(cons
     const int n = at.n, row = at.row, c0 = at.c0, q = at.q;
     const uint32_t parity = at.parity;
     const bool two = c0 + 1 < WS;  // (uniform over the warp)
-    bool ready = false;
-    for (uint32_t it = 0; it < kSpin && !ready; ++it) ready = try_wait(s_u32(&bars[2 * q]), parity);
-    if (ready && two) {
-      ready = false;
-      for (uint32_t it = 0; it < kSpin && !ready; ++it) ready = try_wait(s_u32(&bars[2 * q + 1]), parity);
-    }
-    if (!ready) {  // (bounded wait gave up)
-      if (lane == 0) atomicOr(err, 64u);
+    if (!slot_wait(s_u32(&bars[2 * q]), parity) || (two && !slot_wait(s_u32(&bars[2 * q + 1]), parity))) {
+      slot_gave_up(err);
       s_gave_up = 1;
       break;
     }

@@ -332,13 +332,14 @@ struct Ring {
     }
     if (++put == slots) put = 0;
   }
-  // the next chunk in order; null when the bounded wait ran out
+  // The next chunk in order; null when the bounded wait ran out.  Every lane gets the same answer: a lane that left alone would wait at the
+  // tile's barrier for lanes that wait for it at the next __syncwarp.
   __device__ __forceinline__ const unsigned char* wait() const {
     for (uint32_t it = 0; it < kSpin; ++it) {
       uint32_t ok;
       asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                    : "=r"(ok) : "r"(r_u32(&bars[get])), "r"(parity) : "memory");
-      if (ok) return base + get * kSlot;
+      if (__all_sync(0xFFFFFFFFu, ok)) return base + get * kSlot;
     }
     return nullptr;
   }

@@ -29,6 +29,16 @@ def test_gemm_roles_wait_as_warps():
     assert re.search(r"bool mbar_wait_warp\([^{]*\{.*?__all_sync\(kAll, mbar_test.*?__all_sync\(kAll, mbar_try_wait", s, re.S)
 
 
+@pytest.mark.parametrize("name", ["izb_rows.cu", "izb_gemv_stream.cu"])
+def test_gemv_rings_wait_as_warps(name):
+    """A look at a ring slot's barrier is only ever used through a vote."""
+    s = source(name)
+    looks = [line for line in s.split("\n") if re.search(r"\btry_wait\(", line) and "bool try_wait" not in line]
+    looks += [line for line in s.split("\n") if re.search(r"\bif \(ok\) return base", line)]
+    assert all("__all_sync(" in line for line in looks), looks
+    assert s.count("__all_sync(") >= 1
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("qt,M,N,K", [(12, 300, 272, 1024), (8, 300, 272, 1024), (13, 130, 128, 512), (14, 130, 128, 512), (23, 130, 128, 512), (12, 40, 128, 4096)])
 def test_waits_that_run_out_at_any_moment(izb, qt, M, N, K):
