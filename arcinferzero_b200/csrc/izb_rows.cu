@@ -730,6 +730,8 @@ __global__ void __launch_bounds__(kMoeWarps * 32, kMoeCtas) moe_rows_kernel(cons
 // in flight and at work, so of all splits that fit: the most warps x (slots + 1) that have work, averaged over the rounds the grid
 // needs; of equals the smaller CTA.  (Four warps suit small matrices -- 1024 x 3072 Q6_K, 5 rows: 4.5 us against 5.2 with eight and
 // 7.9 with sixteen --, sixteen share one copy of large activations: 128000 x 4096 Q4_K, 8 rows: 89 us against 102 with four.)
+// Warps past the last tile are not at work: they request and multiply rows that do not exist beside the ones that do (96 x 4096 Q4_K,
+// four rows: 10.5 us in sixteen-warp CTAs, 6.5 in four-warp ones).
 constexpr size_t kSmemPerSm = 226 * 1024;
 struct Split {
   int warps, ctas, slots;  // slots 0: the activations leave no room
@@ -746,7 +748,7 @@ Split pick_split(int K, int T, int tiles, int sms) {
       while (slots >= 2 && rows_smem<F>(K, T, nw, slots) > room) --slots;
       if (slots < 2) break;
       const int rounds = (groups + c * sms - 1) / (c * sms);
-      const double at_work = (double)groups * nw * (slots + 1) / rounds;
+      const double at_work = (double)tiles * F::kSubs * (slots + 1) / rounds;
       if (at_work > most * 1.001) {
         most = at_work;
         best = {nw, c, slots};

@@ -35,6 +35,29 @@ def test_rows_match_oracle(izb, qt, N, K):
     W.close()
 
 
+# Which kernel takes a call depends on its type, rows and sizes; a row's bits must not, since a decode step requantises them (Q4_K with
+# K % 1024 == 0 and N >= 1024 has kernels of its own order up to four rows: there the few-row kernels are compared among themselves).
+# Row tiles that fill no block of any split (16, 48, 96 rows), the borders of the dispatch in K and N, activations that take two passes.
+@pytest.mark.parametrize("qt,N,K", [(14, 16, 512), (14, 48, 2048), (14, 96, 8192), (14, 112, 8448), (14, 144, 8192), (14, 1520, 17408), (14, 1552, 17408), (14, 4096, 1024),
+                                    (12, 16, 4096), (12, 48, 1536), (12, 96, 4096), (12, 1008, 2048), (12, 2544, 18944), (12, 2576, 18944), (12, 16384, 2304), (12, 8192, 5376),
+                                    (12, 4096, 9216), (12, 1024, 2048), (8, 4096, 256), (8, 4096, 8192), (8, 16384, 1024), (8, 4112, 2304), (8, 6144, 512), (8, 16, 1024),
+                                    (13, 64, 768), (23, 64, 768), (2, 4096, 512)])
+def test_rows_do_not_depend_on_their_number(izb, qt, N, K):
+    import torch
+    own_order = qt == 12 and K % 1024 == 0 and N >= 1024
+    W = izb.Weight(qt, np.tile(S.make_weight(qt, 16, K, N + K + qt), (N // 16, 1)), N, K)
+    x = torch.from_numpy(S.make_act(8, K, 5)).cuda()
+    aq, asc, _ = izb.quantize_act(x)
+    first = 5 if own_order else 1
+    want = [izb.gemv(W, aq[j:].contiguous(), asc[:, j:].contiguous(), 1)[0] for j in range(8)] if not own_order else izb.gemv(W, aq, asc, 8)
+    for T in range(first, 9):
+        got = izb.gemv(W, aq, asc, T)
+        for j in range(T):
+            assert torch.equal(got[j], want[j]), (T, j)
+    assert izb.device_status(0) == 0
+    W.close()
+
+
 @pytest.mark.parametrize("qt", [12, 8])
 @pytest.mark.parametrize("T,TM,F,E", [(1, 8, 256, 512), (5, 4, 768, 1024), (40, 8, 256, 2304), (3, 1, 512, 256)])
 def test_expert_rows_equal_dense_rows(izb, qt, T, TM, F, E):
