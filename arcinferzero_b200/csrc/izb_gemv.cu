@@ -70,19 +70,25 @@ int launch(const izb_weight* w, const uint8_t* raw, const int8_t* aq, const floa
 }
 
 // Which of the two ways to the same bits is faster: the matrix instruction's cost does not grow with T, the dot-product kernels' does.
-// Measured (us, matrix instruction / dot products):
-//   Q6_K  32000 x 4096 T=2 28/34, T=8 33/89; 1024 x 3072 T=2 4.1/4.2, T=5 4.5/5.4; T=1 loses everywhere (28.2/27.4)
-//   Q4_K  T >= 4: 3072 x 1536 T=4 4.0/4.3, 1024 x 2048 T=8 4.1/4.2, 34816 x 5120 T=5 34/52, T=8 35/76;
-//         T = 2, 3: 11776 x 2304 8.5/8.6 and 8.6/10, 5376 x 11776 20/30 and 20/26, but 3072 x 1536 4.0/3.3 and 3.9/3.8
+// Measured (us, matrix instruction / dot products, each behind a quantiser and with weights that are not in L2):
+//   Q6_K  32000 x 4096 T=2 36/39, T=8 38/95; 1024 x 2560 T=2 5.9/7.3, T=5 6.8/8.2; T=1 loses everywhere (28.2/27.4, without the quantiser).
+//         Few row tiles leave most of the chip idle over a long K: 96 x 8192 T=2 9.2/8.4, 48 x 17408 T=2 15.6/12.6, but 128 x 8192 T=5 11/11,
+//         48 x 4096 T=5 7.3/7.9
+//   Q4_K  T >= 4: 3072 x 1536 T=4 4.0/4.3, 1024 x 2048 T=8 4.1/4.2, 34816 x 5120 T=5 34/52, T=8 35/76 (without the quantiser);
+//         T = 3: 8192 x 5376 15/19, 16384 x 8448 34/36; small ones lose (3072 x 1536 3.9/3.8);
+//         T = 2: 12288 x 2304 11/13, 12288 x 5376 18/20, 16384 x 3840 19/17, 16384 x 5376 25/22, 12288 x 8448 33/24, 32000 x 8960 61/50; rows above 9216
+//         take the dot-product kernel a second pass over its ring: 16384 x 9472 37/53, 5120 x 13824 26/36
 //         (at up to four rows the kernels for K % 1024 == 0 add in another order: theirs stays)
 //   Q8_0  needs many row tiles (a warp holds half a tile's sums): 1024 x 3072 T=8 6.4/5.0, 2048 x 1024 3.3/3.2, 4096 x 4096 T=3 8.1/7.4,
 //         T=8 8.3/12, 6144 x 1024 T=3 3.6/3.8, T=8 3.9/5.9, 5120 x 5120 T=8 11/17; T <= 2 pays for long K or many short rows:
 //         4096 x 14336 T=1 17.5/22, 32000 x 1024 T=1 8.1/12, 151936 x 2048 T=2 55/60, T=1 54/52, 5120 x 5120 T=2 9.1/8.1
 bool rows_first(const izb_weight* w, int T) {
-  if (w->type == IZB_K16) return T >= 2;
+  if (w->type == IZB_K16) return T >= 2 && (w->N >= 128 || w->K < 8192);
   if (w->type == IZB_Q4_K) {
     if (T <= 4 && w->K % 1024 == 0 && w->N >= 1024) return false;
-    return T >= 4 || (T >= 2 && (size_t)w->N * w->row_bytes >= (size_t)12 << 20);
+    const bool large = (size_t)w->N * w->row_bytes >= (size_t)12 << 20;
+    if (T == 2) return w->K > 9216 || (large && w->K <= (w->N <= 12288 ? 5376 : 3584));
+    return T >= 4 || (T == 3 && large);
   }
   if (w->N < 4096) return false;
   return T >= (w->N < 6144 ? 4 : 3) || w->K >= 8192 || (w->N >= 16384 && w->K <= 1024 * T);

@@ -101,7 +101,7 @@ struct Acts {
 // ---- weight forms.  prep() expands the headers of a chunk into `hd` ([block][row]); mul() multiplies a chunk into
 // the piece sums acc[piece][r]: rows g, g + 8 against tokens 2t, 2t + 1
 struct RQ4K {
-  static constexpr int SBB = 144, kPitch = 144, kSubs = 4, kPieces = 8;
+  static constexpr int SBB = 144, kPitch = 144, kSubs = 4, kPieces = 8, kDotWarps = 16;
   static constexpr bool kEx = true, kPrep = true;
   // (d * sc, -dmin * mn) of a row's blocks 4 up .. + 3; the sub-block scales and mins as bytes (get_scale_min_k4,
   // src/quants.h:61-69).  Odd blocks meet 16 q: their d * sc is divided by 16.
@@ -187,7 +187,7 @@ struct RQ4K {
 };
 
 struct RQ80 {
-  static constexpr int SBB = 272, kPitch = 272, kSubs = 2, kPieces = 16;
+  static constexpr int SBB = 272, kPitch = 272, kSubs = 2, kPieces = 16, kDotWarps = 16;
   static constexpr bool kEx = false, kPrep = false;
   static __device__ __forceinline__ void prep(const unsigned char*, float2*, int) {}
   template <int TT>
@@ -245,7 +245,7 @@ struct RQ80 {
 // Q6_K packed: ql[128] | qh[64] | int8 scale[16] | fp16 d (csrc/izb_types.cu: q6p_word).  The quants' offset of 32 is taken off by the
 // accumulators' start.
 struct RQ6K {
-  static constexpr int SBB = kQ6pSbBytes, kPitch = 240, kSubs = 4, kPieces = 8;
+  static constexpr int SBB = kQ6pSbBytes, kPitch = 240, kSubs = 4, kPieces = 8, kDotWarps = 8;
   static constexpr bool kEx = true, kPrep = true;
   static __device__ __forceinline__ void prep(const unsigned char* chunk, float2* hd, int lane) {
     // lane <-> row lane / 2, blocks 4 (lane & 1) .. + 3: (scale of the first half, of the second half)
@@ -762,8 +762,11 @@ template <class F>
 int rows_of(const izb_weight* w, int mat, const int8_t* aq, const float* asc, int T, int Mp, float* C, int ldc, int c_off, int acc, cudaStream_t st) {
   const int sms = izb_sm_count(w->device), tiles = (w->N + 15) / 16;
   const Split sp = pick_split<F>(w->K, T, tiles, sms);
-  if (!sp.slots) {  // half the tokens at a time, the second pass finding part of the weights in L2
-    if (T < 2) return 1;
+  // Half the tokens at a time, the second pass finding part of the weights in L2; not where the dot-product kernel's warps (kDotWarps per SM)
+  // take every row in one round (us, halves / dot products, eight rows of 17408 Q6_K: 1024 rows 34/28, 1280 rows 34/42; of 18944 Q4_K:
+  // 2304 rows 35/33, 2560 rows 45/60).
+  if (!sp.slots) {
+    if (T < 2 || w->N <= F::kDotWarps * sms) return 1;
     const int h = (T + 1) / 2;
     if (const int rc = rows_of<F>(w, mat, aq, asc, h, Mp, C, ldc, c_off, acc, st)) return rc;
     return rows_of<F>(w, mat, aq + (size_t)h * w->K, asc + h, T - h, Mp, C + (size_t)h * ldc, ldc, c_off, acc, st);
