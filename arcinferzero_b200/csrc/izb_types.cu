@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(kGvWarps * 32) gemv_k16_kernel(const uint8_t* 
   const int nb = K >> 5, nsb = K >> 8;
   int8_t* s_a = reinterpret_cast<int8_t*>(smem);                          // [T][K]
   float* s_sc = reinterpret_cast<float*>(smem + (size_t)T * K);           // [T][K/32]
-  pdl_launch_next();
+  pdl_launch_next();  // (launched plainly, see below; the next kernel may still come early)
   pdl_wait();
   for (int i = threadIdx.x; i < T * (K / 16); i += blockDim.x) {
     const int t = i / (K / 16), pc = i % (K / 16);
@@ -324,15 +324,23 @@ int launch_gemv_k16(const izb_weight* w, const uint8_t* raw, const int8_t* aq, c
   if (w->packed6 && T <= 4 && smem <= 48 * 1024) grid = izb_sm_count(w->device) * (T <= 2 ? 4 : 3);
   const int need = (w->N + kGvWarps - 1) / kGvWarps;
   if (grid > need) grid = need;
+  // Programmatic dependent launch where it pays: blocks placed while the kernel before drains come unevenly, and these kernels, several
+  // blocks to an SM, feel it.  (us with / without, each behind a quantiser: IQ4_XS 12288 x 4096, four rows, 44/29, 1024 x 2048, one row, 5.7/5.7;
+  // Q5_K 12288 x 8192, eight rows, 112/80.  Q6_K, one row: 5120 x 5120 8.1/8.5, 4096 x 4096 9.0/9.6, but 1024 x 17408 18.9/17.1, 1536 x 17408
+  // 19.7/17.3.)
+  const bool ahead = w->K <= 12288;
   if (w->packed6) {
     IZB_SMEM_OPTIN((gemv_q6p_kernel<T>), 200 * 1024, w->device);
-    IZB_LAUNCH("gemv_q6p", st, izb_launch_pdl(gemv_q6p_kernel<T>, grid, kGvWarps * 32, smem, st, raw, w->N, w->K, aq, asc, Mp, C, ldc, c_off, acc));
+    if (ahead)
+      IZB_LAUNCH("gemv_q6p", st, izb_launch_pdl(gemv_q6p_kernel<T>, grid, kGvWarps * 32, smem, st, raw, w->N, w->K, aq, asc, Mp, C, ldc, c_off, acc));
+    else
+      IZB_LAUNCH("gemv_q6p", st, gemv_q6p_kernel<T><<<grid, kGvWarps * 32, smem, st>>>(raw, w->N, w->K, aq, asc, Mp, C, ldc, c_off, acc));
   } else if (w->has_min) {
     IZB_SMEM_OPTIN((gemv_k16_kernel<T, true>), 200 * 1024, w->device);
-    IZB_LAUNCH("gemv_k16", st, izb_launch_pdl(gemv_k16_kernel<T, true>, grid, kGvWarps * 32, smem, st, raw, w->N, w->K, aq, asc, Mp, C, ldc, c_off, acc));
+    IZB_LAUNCH("gemv_k16", st, gemv_k16_kernel<T, true><<<grid, kGvWarps * 32, smem, st>>>(raw, w->N, w->K, aq, asc, Mp, C, ldc, c_off, acc));
   } else {
     IZB_SMEM_OPTIN((gemv_k16_kernel<T, false>), 200 * 1024, w->device);
-    IZB_LAUNCH("gemv_k16", st, izb_launch_pdl(gemv_k16_kernel<T, false>, grid, kGvWarps * 32, smem, st, raw, w->N, w->K, aq, asc, Mp, C, ldc, c_off, acc));
+    IZB_LAUNCH("gemv_k16", st, gemv_k16_kernel<T, false><<<grid, kGvWarps * 32, smem, st>>>(raw, w->N, w->K, aq, asc, Mp, C, ldc, c_off, acc));
   }
   return IZB_OK;
 }
