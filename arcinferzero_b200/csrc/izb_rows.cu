@@ -610,10 +610,59 @@ constexpr int kFewSlots = 2;
 // (small CTAs: items are divided among them as they come, and a tile's activations hold up four warps only; three per SM leave the two
 // ways 168 registers -- at 128 they spilt, and with the shared memory in use the stacks do not fit in L1)
 constexpr int kMoeWarps = 4, kMoeCtas = 3;
+// Where the items are fewer than the blocks that fit, a block takes kPer row tiles of one tile instead of kMoeWarps, its kSubs warps per row
+// tile sharing the superblocks also for few slots: gate / up 1024 x 512 of 8 experts Q4_K, four slots, 10.8 -> 6.0 us, sixteen 16.1 -> 6.9; 4096 x
+// 1536 of 16, two slots, 21.0 -> 11.6.  At most two items per SM: with a third the walk below is faster.  `slots`: the ring's, set up by
+// the caller.  (Out of line: beside the walk in one body it cost that one registers.)
 template <class F>
+__device__ __noinline__ void moe_fine(const CUtensorMap& tg, const CUtensorMap& tu, int pair, int N, int K, const int8_t* aq, const float* asc, int Mp, const int32_t* tiles,
+                                      const int32_t* stok, const float* swt, float* out, int slots, volatile int* gave_up, uint32_t* err) {
+  extern __shared__ __align__(1024) unsigned char smem[];
+  constexpr int NW = kMoeWarps, kPer = NW / F::kSubs;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int part = warp % F::kSubs, mine = warp / F::kSubs, nsb = K >> 8, groups = ((N + 15) / 16 + kPer - 1) / kPer;
+  const int ti = blockIdx.x / groups, row_tile = (blockIdx.x - ti * groups) * kPer + mine;
+  if (ti >= tiles[0]) return;
+  unsigned char* rings = smem + act_bytes<F>(K, 8);
+  unsigned char* xch = rings + (size_t)NW * slots * Ring<F>::kSlot;
+  Ring<F> ring;
+  ring.slots = slots;
+  ring.base = rings + (size_t)warp * slots * Ring<F>::kSlot;
+  ring.bars = reinterpret_cast<uint64_t*>(xch + NW * kXch) + warp * slots;
+  const int row = tiles[1 + 3 * ti] * N + row_tile * 16, s0 = tiles[2 + 3 * ti], T = tiles[3 + 3 * ti];
+  int pm = 0, ps = part;
+  auto request = [&]() {
+    if (pm > pair || part >= nsb) return;
+    ring.fill(pm ? &tu : &tg, ps, row, lane);
+    if ((ps += F::kSubs) >= nsb) { ps = part; ++pm; }
+  };
+  for (int s = 0; s < slots; ++s) request();
+  const Acts acts = stage_acts<F>(smem, K, T, aq, asc, Mp, g, t, [&](int j) { return stok ? stok[s0 + j] : s0 + j; });
+  __syncthreads();
+  bool ok = true;
+  float first[4];
+  for (int m = 0; m <= pair; ++m) {
+    f2 acc[F::kPieces][2];
+    if (ok) ok = accumulate<F>(ring, reinterpret_cast<float2*>(xch + (size_t)warp * kXch), acts, part, nsb, lane, acc, request);
+    if (!ok) {
+      if (lane == 0) atomicOr(err, 64u);
+      *gave_up = 1;
+    }
+    reduce_tile<F>(acc, xch, warp, lane);
+    if (part != 0 || *gave_up) continue;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int n = row_tile * 16 + g + 8 * (i >> 1), slot = 2 * t + (i & 1);
+      const float v = f2_get(acc[0][i >> 1], i & 1);
+      if (m < pair) first[i] = v;
+      else if (n < N && slot < T) out[(size_t)(s0 + slot) * N + n] = pair ? __fmul_rn(__fdiv_rn(first[i], __fadd_rn(1.0f, expf(-first[i]))), v) : __fmul_rn(swt[s0 + slot], v);
+    }
+  }
+}
+template <class F, bool kChoose>
 __global__ void __launch_bounds__(kMoeWarps * 32, kMoeCtas) moe_rows_kernel(const __grid_constant__ CUtensorMap tg, const __grid_constant__ CUtensorMap tu, int pair, int N, int K,
                                                           const int8_t* __restrict__ aq, const float* __restrict__ asc, int Mp, const int32_t* __restrict__ tiles,
-                                                          const int32_t* __restrict__ stok, const float* __restrict__ swt, float* __restrict__ out, int slots, uint32_t* err) {
+                                                          const int32_t* __restrict__ stok, const float* __restrict__ swt, float* __restrict__ out, int slots, int fine_items, uint32_t* err) {
   extern __shared__ __align__(1024) unsigned char smem[];
   constexpr int NW = kMoeWarps, kPer = NW / F::kSubs;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
@@ -630,6 +679,14 @@ __global__ void __launch_bounds__(kMoeWarps * 32, kMoeCtas) moe_rows_kernel(cons
   ring.init(lane);
   pdl_launch_next();
   pdl_wait();
+  if (kChoose) {  // (not for short K and few slots: dp4a without the exchange between warps is as fast there)
+    const int n_tiles = tiles[0], saved = (nsb - (nsb + F::kSubs - 1) / F::kSubs) * (1 + pair);
+    if ((long long)n_tiles * (((N + 15) / 16 + kPer - 1) / kPer) <= fine_items &&
+        (saved > 1 || __any_sync(0xFFFFFFFFu, lane < n_tiles && tiles[3 + 3 * lane] > kFewSlots))) {  // (a look at the first 32 tiles)
+      moe_fine<F>(tg, tu, pair, N, K, aq, asc, Mp, tiles, stok, swt, out, slots, gave_up, err);
+      return;
+    }
+  }
   const long long items = (long long)tiles[0] * groups;
   const int lo = (int)(items * blockIdx.x / gridDim.x), hi = (int)(items * (blockIdx.x + 1) / gridDim.x);
   // Chunks still to request: superblock `ps` of matrix `pm` (gate, up) of this warp's row tile in round `pr` of item `pi`.  Few slots:
@@ -793,14 +850,20 @@ int moe_rows_of(const izb_weight* wg, const izb_weight* wu, const int8_t* aq, co
     if (slots >= 2) break;
   }
   if (ctas == 0) return 1;
-  IZB_SMEM_OPTIN((moe_rows_kernel<F>), kSmemPerSm, wg->device);
   uint32_t* err = izb_device_error_word(wg->device);
   if (!err) IZB_FAIL(IZB_ERR_NOMEM, "moe: no device error word");
   CUtensorMap tg, tu;
   memcpy(&tg, wg->tmap16_raw, sizeof tg);
   memcpy(&tu, (wu ? wu : wg)->tmap16_raw, sizeof tu);
-  IZB_LAUNCH(wu ? "moe_gateup" : "moe_down", st, izb_launch_pdl(moe_rows_kernel<F>, sms * ctas, kMoeWarps * 32, rows_smem<F>(wg->K, 8, kMoeWarps, slots), st, tg, tu, wu ? 1 : 0,
-                                                               wg->N, wg->K, aq, asc, Mp, tiles, stok, swt, out, slots, err));
+  const size_t smem = rows_smem<F>(wg->K, 8, kMoeWarps, slots);
+  const int grid = sms * ctas, fine_items = sms * (ctas < 2 ? ctas : 2);
+  if (wu) {
+    IZB_SMEM_OPTIN((moe_rows_kernel<F, true>), kSmemPerSm, wg->device);
+    IZB_LAUNCH("moe_gateup", st, izb_launch_pdl(moe_rows_kernel<F, true>, grid, kMoeWarps * 32, smem, st, tg, tu, 1, wg->N, wg->K, aq, asc, Mp, tiles, stok, swt, out, slots, fine_items, err));
+  } else {
+    IZB_SMEM_OPTIN((moe_rows_kernel<F, false>), kSmemPerSm, wg->device);
+    IZB_LAUNCH("moe_down", st, izb_launch_pdl(moe_rows_kernel<F, false>, grid, kMoeWarps * 32, smem, st, tg, tu, 0, wg->N, wg->K, aq, asc, Mp, tiles, stok, swt, out, slots, fine_items, err));
+  }
   return IZB_OK;
 }
 

@@ -59,7 +59,7 @@ def test_rows_do_not_depend_on_their_number(izb, qt, N, K):
 
 
 @pytest.mark.parametrize("qt", [12, 8])
-@pytest.mark.parametrize("T,TM,F,E", [(1, 8, 256, 512), (5, 4, 768, 1024), (40, 8, 256, 2304), (3, 1, 512, 256)])
+@pytest.mark.parametrize("T,TM,F,E", [(1, 8, 256, 512), (5, 4, 768, 1024), (40, 8, 256, 2304), (3, 1, 512, 256), (40, 8, 1024, 512), (4, 8, 3072, 256)])
 def test_expert_rows_equal_dense_rows(izb, qt, T, TM, F, E):
     """Every slot's expert product against the same product as a dense call on that expert's matrix."""
     import torch
@@ -83,6 +83,34 @@ def test_expert_rows_equal_dense_rows(izb, qt, T, TM, F, E):
             a, b = hq[s:s + 1].repeat(16, 1).contiguous(), hsc[:, s:s + 1].repeat(1, 16).contiguous()
             want = float(swt[s]) * izb.gemm(Wd, a, b, M=1, impl=izb.GEMM_CORE, mat=e)[0].double()
             assert float((y[s] - want).abs().max() / want.abs().max()) < TOL
+    assert izb.device_status(0) == 0
+    for W in (Wg, Wu, Wd):
+        W.close()
+
+
+@pytest.mark.parametrize("qt", [12, 8])
+@pytest.mark.parametrize("F,E", [(256, 512), (272, 1024), (768, 2304), (1040, 256)])
+def test_expert_rows_do_not_depend_on_the_other_tokens(izb, qt, F, E):
+    """One token's expert products bit for bit in calls of 1 .. 96 tokens: few items and many, tiles of one or two slots and fuller ones,
+    blocks of one row tile and of several."""
+    import torch
+    NE, NU = 8, 2
+    g, u, d = (S.make_weight(qt, NE * n, k, i) for i, (n, k) in enumerate(((F, E), (F, E), (256, E))))
+    Wg, Wu, Wd = izb.Weight(qt, g, F, E, n_mats=NE), izb.Weight(qt, u, F, E, n_mats=NE), izb.Weight(qt, d, 256, E, n_mats=NE)
+    x = torch.from_numpy(S.make_act(96, E, 9)).cuda() * 0.02
+    logits = torch.from_numpy(S.make_act(96, NE, 3)).cuda()
+    def products(T, TM):
+        aq, asc, _ = izb.quantize_act(x[:T])
+        ids, wts, counts = izb.moe_route(logits[:T], NU)
+        _, tiles, mt, stok, swt, inv = izb.moe_sort(ids, wts, counts, TM)
+        h = izb.moe_gateup(Wg, Wu, aq, asc, tiles, mt, TM, stok, T * NU)
+        aq2, asc2 = aq[stok.long()].contiguous(), asc[:, stok.long()].contiguous()  # (the down product's rows are slots)
+        y = izb.moe_down(Wd, aq2, asc2, tiles, mt, TM, swt, T * NU)
+        return h[inv.long()], y[inv.long()]  # by (token, choice)
+    want = products(96, 8)
+    for T, TM in ((1, 8), (2, 8), (3, 1), (5, 4), (9, 8), (24, 8), (48, 2), (96, 1)):
+        for got, ref in zip(products(T, TM), want):
+            assert torch.equal(got, ref[:T * NU]), (T, TM)
     assert izb.device_status(0) == 0
     for W in (Wg, Wu, Wd):
         W.close()
