@@ -659,7 +659,7 @@ __device__ __noinline__ void moe_fine(const CUtensorMap& tg, const CUtensorMap& 
     }
   }
 }
-template <class F, bool kChoose>
+template <class F>
 __global__ void __launch_bounds__(kMoeWarps * 32, kMoeCtas) moe_rows_kernel(const __grid_constant__ CUtensorMap tg, const __grid_constant__ CUtensorMap tu, int pair, int N, int K,
                                                           const int8_t* __restrict__ aq, const float* __restrict__ asc, int Mp, const int32_t* __restrict__ tiles,
                                                           const int32_t* __restrict__ stok, const float* __restrict__ swt, float* __restrict__ out, int slots, int fine_items, uint32_t* err) {
@@ -679,8 +679,8 @@ __global__ void __launch_bounds__(kMoeWarps * 32, kMoeCtas) moe_rows_kernel(cons
   ring.init(lane);
   pdl_launch_next();
   pdl_wait();
-  if (kChoose) {  // (not for short K and few slots: dp4a without the exchange between warps is as fast there)
-    const int n_tiles = tiles[0], saved = (nsb - (nsb + F::kSubs - 1) / F::kSubs) * (1 + pair);
+  {  // (fine_items 0 for the down product; not for short K and few slots: dp4a without the exchange between warps is as fast there)
+    const int n_tiles = tiles[0], saved = 2 * (nsb - (nsb + F::kSubs - 1) / F::kSubs);
     if ((long long)n_tiles * (((N + 15) / 16 + kPer - 1) / kPer) <= fine_items &&
         (saved > 1 || __any_sync(0xFFFFFFFFu, lane < n_tiles && tiles[3 + 3 * lane] > kFewSlots))) {  // (a look at the first 32 tiles)
       moe_fine<F>(tg, tu, pair, N, K, aq, asc, Mp, tiles, stok, swt, out, slots, gave_up, err);
@@ -855,15 +855,10 @@ int moe_rows_of(const izb_weight* wg, const izb_weight* wu, const int8_t* aq, co
   CUtensorMap tg, tu;
   memcpy(&tg, wg->tmap16_raw, sizeof tg);
   memcpy(&tu, (wu ? wu : wg)->tmap16_raw, sizeof tu);
-  const size_t smem = rows_smem<F>(wg->K, 8, kMoeWarps, slots);
-  const int grid = sms * ctas, fine_items = sms * (ctas < 2 ? ctas : 2);
-  if (wu) {
-    IZB_SMEM_OPTIN((moe_rows_kernel<F, true>), kSmemPerSm, wg->device);
-    IZB_LAUNCH("moe_gateup", st, izb_launch_pdl(moe_rows_kernel<F, true>, grid, kMoeWarps * 32, smem, st, tg, tu, 1, wg->N, wg->K, aq, asc, Mp, tiles, stok, swt, out, slots, fine_items, err));
-  } else {
-    IZB_SMEM_OPTIN((moe_rows_kernel<F, false>), kSmemPerSm, wg->device);
-    IZB_LAUNCH("moe_down", st, izb_launch_pdl(moe_rows_kernel<F, false>, grid, kMoeWarps * 32, smem, st, tg, tu, 0, wg->N, wg->K, aq, asc, Mp, tiles, stok, swt, out, slots, fine_items, err));
-  }
+  // (one kernel for both products: as two, the second finds its code out of the instruction cache, 1 us of a 4-token step)
+  IZB_SMEM_OPTIN((moe_rows_kernel<F>), kSmemPerSm, wg->device);
+  IZB_LAUNCH(wu ? "moe_gateup" : "moe_down", st, izb_launch_pdl(moe_rows_kernel<F>, sms * ctas, kMoeWarps * 32, rows_smem<F>(wg->K, 8, kMoeWarps, slots), st, tg, tu, wu ? 1 : 0,
+                                                               wg->N, wg->K, aq, asc, Mp, tiles, stok, swt, out, slots, wu ? sms * (ctas < 2 ? ctas : 2) : 0, err));
   return IZB_OK;
 }
 

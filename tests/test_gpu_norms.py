@@ -1,0 +1,26 @@
+"""The norm producers at the borders of their register plans: elements per thread, and numbers of long rows that change what a block
+holds.  Bit for bit against the oracle."""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def bits(a):
+    return np.ascontiguousarray(a, np.float32).view(np.uint32)
+
+
+# (148 SMs: the number of long rows up to which a block holds both of its rows)
+@pytest.mark.parametrize("M,K", [(3, 1024), (3, 1280), (3, 2304), (3, 4352), (3, 5376), (3, 8192), (3, 8448), (148, 8448), (149, 8448), (300, 16384)])
+def test_add_norm_quant(izb, M, K):
+    import torch
+    rng = np.random.default_rng(M + K)
+    x, t = rng.standard_normal((M, K), dtype=np.float32), rng.standard_normal((M, K), dtype=np.float32) * 3
+    w, w2 = ((1.0 + 0.2 * rng.standard_normal(K)).astype(np.float32) for _ in range(2))
+    for second in (w2, None):
+        xd = torch.from_numpy(x).cuda()
+        aq, asc = izb.add_norm_quant(xd, torch.from_numpy(t).cuda(), torch.from_numpy(w).cuda(), 1e-6, 0.75, None if second is None else torch.from_numpy(second).cuda())
+        rx, raq, rasc, _ = O.add_norm_quant(x, t, w, 1e-6, 0.75, second, Mp=asc.shape[1])
+        assert (bits(xd.cpu().numpy()) == bits(rx)).all() and (aq.cpu().numpy() == raq).all() and (bits(asc.cpu().numpy()) == bits(rasc)).all()
