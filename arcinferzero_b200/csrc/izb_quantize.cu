@@ -123,8 +123,10 @@ __device__ __forceinline__ void zero_pad_row(int m, int Mp, int K, int8_t* __res
 // thread's loads are in flight before the first reduction and the chains unroll.  (With a run-time bound over 64 elements
 // the loads were issued one step at a time: 5 rows of 4096 took 35 us.)  Up to 20 elements (K = 5120) the norm weights are
 // requested with the rows; above that they would not fit the registers and come from L2 behind the first reduction.
+// kHold: t stays in registers from the first sum to the update.  Not for long rows (K > 8192) when there are more of them than SMs: with
+// both rows held one block fills an SM's registers, and the next row waits (16384, 200 rows: 72 us held, 38 read twice; 4096 rows: 1033 and 609).
 constexpr int kAnqMax = 64;
-template <int NK>
+template <int NK, bool kHold>
 __global__ void __launch_bounds__(256) add_norm_quant_kernel(float* __restrict__ x, const float* __restrict__ t,
                                                              const float* __restrict__ w, int K, float eps, float s,
                                                              const float* __restrict__ w2, int M, int Mp, int8_t* __restrict__ aq,
@@ -141,13 +143,15 @@ __global__ void __launch_bounds__(256) add_norm_quant_kernel(float* __restrict__
   float* xr = x + (size_t)m * K;
   const float* tr = t + (size_t)m * K;
   const int nk = K / 256;
-  float tv[NK], xv[NK], wv[kAhead ? NK : 1], w2v[kAhead ? NK : 1];
+  float tv[kHold ? NK : 1], xv[NK], wv[kAhead ? NK : 1], w2v[kAhead ? NK : 1];
+  if (kHold) {
 #pragma unroll
-  for (int k = 0; k < NK; ++k)
-    if (k < nk) tv[k] = tr[threadIdx.x + 256 * k];
+    for (int k = 0; k < NK; ++k)
+      if (k < nk) tv[k] = tr[threadIdx.x + 256 * k];
 #pragma unroll
-  for (int k = 0; k < NK; ++k)
-    if (k < nk) xv[k] = xr[threadIdx.x + 256 * k];
+    for (int k = 0; k < NK; ++k)
+      if (k < nk) xv[k] = xr[threadIdx.x + 256 * k];
+  }
   if (kAhead) {
 #pragma unroll
     for (int k = 0; k < NK; ++k)
@@ -157,9 +161,16 @@ __global__ void __launch_bounds__(256) add_norm_quant_kernel(float* __restrict__
       }
   }
   float ss = 0.0f;
+  if (kHold) {
 #pragma unroll
-  for (int k = 0; k < NK; ++k)
-    if (k < nk) ss = __fmaf_rn(tv[k], tv[k], ss);
+    for (int k = 0; k < NK; ++k)
+      if (k < nk) ss = __fmaf_rn(tv[k], tv[k], ss);
+  } else {
+    for (int k = 0; k < nk; ++k) {
+      const float v = tr[threadIdx.x + 256 * k];
+      ss = __fmaf_rn(v, v, ss);
+    }
+  }
   ss = cta_sum_ordered(ss, s_w);
   const float r = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, (float)K), eps)));
   float s2 = 0.0f;
@@ -167,7 +178,7 @@ __global__ void __launch_bounds__(256) add_norm_quant_kernel(float* __restrict__
   for (int k = 0; k < NK; ++k) {
     if (k < nk) {
       const int i = threadIdx.x + 256 * k;
-      const float v = __fmul_rn(__fadd_rn(xv[k], __fmul_rn(__fmul_rn(tv[k], r), kAhead ? wv[k] : w[i])), s);
+      const float v = __fmul_rn(__fadd_rn(kHold ? xv[k] : xr[i], __fmul_rn(__fmul_rn(kHold ? tv[k] : tr[i], r), kAhead ? wv[k] : w[i])), s);
       xv[k] = v;
       xr[i] = v;
       s2 = __fmaf_rn(v, v, s2);
@@ -357,8 +368,11 @@ extern "C" int izb_add_norm_quant(float* d_x, const float* d_t, const float* d_w
   if (!(eps >= 0.0f)) IZB_FAIL(IZB_ERR_ARG, "add_norm_quant: eps = %g", (double)eps);
   cudaStream_t st = (cudaStream_t)stream;
   const int nk = K / 256;  // elements per thread
-  auto kernel = nk <= 4 ? add_norm_quant_kernel<4> : nk <= 8 ? add_norm_quant_kernel<8> : nk <= 16 ? add_norm_quant_kernel<16>
-              : nk <= 20 ? add_norm_quant_kernel<20> : nk <= 32 ? add_norm_quant_kernel<32> : add_norm_quant_kernel<kAnqMax>;
+  int dev = 0;
+  if (nk > 32) IZB_CUDA(cudaGetDevice(&dev));
+  auto kernel = nk <= 4 ? add_norm_quant_kernel<4, true> : nk <= 8 ? add_norm_quant_kernel<8, true> : nk <= 16 ? add_norm_quant_kernel<16, true>
+              : nk <= 20 ? add_norm_quant_kernel<20, true> : nk <= 32 ? add_norm_quant_kernel<32, true>
+              : M_valid <= izb_sm_count(dev) ? add_norm_quant_kernel<kAnqMax, true> : add_norm_quant_kernel<kAnqMax, false>;
   IZB_LAUNCH("add_norm_quant", st, izb_launch_pdl(kernel, Mp, 256, 0, st, d_x, d_t, d_w, K, eps, s, d_w2, M_valid, Mp, d_aq, d_asc, d_absum));
   return IZB_OK;
 }
