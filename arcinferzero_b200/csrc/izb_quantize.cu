@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(256) add_norm_quant_kernel(float* __restrict__
 // Step 2: y = (x * r) * w, optional f32 copy, and per 32-block (four adjacent threads) int8 + scale + sums of 16.
 // G = groups per thread rounded up: row and norm weights are requested together before the reduction and stay in
 // registers (one pass over the row, one latency instead of two; a row read twice through L1 / L2 measured 56 us at 8192 x
-// 5120 and 5.8 us for one row of 5120).  G = 0: rows too long for that (K > 16384), read twice.
+// 5120 and 5.8 us for one row of 5120).  G = 0: rows too long for that (K > 16384), or many long ones, read twice.
 template <int G>
 __global__ void __launch_bounds__(256) rmsnorm_quant_row_kernel(const float* __restrict__ x, int ldx, const float* __restrict__ w,
                                                                 int K, float eps, int M, int Mp, float* __restrict__ hout,
@@ -353,7 +353,12 @@ extern "C" int izb_rmsnorm_quant(const float* d_x, int ldx, const float* d_w, fl
   if (!(eps >= 0.0f)) IZB_FAIL(IZB_ERR_ARG, "rmsnorm_quant: eps = %g", (double)eps);
   cudaStream_t st = (cudaStream_t)stream;
   const int groups = (K / 8 + 255) / 256;  // of 8 values per thread
-  auto kernel = groups <= 1 ? rmsnorm_quant_row_kernel<1> : groups <= 2 ? rmsnorm_quant_row_kernel<2> : groups <= 3 ? rmsnorm_quant_row_kernel<3>
+  // Rows held in registers cost blocks per SM: many long rows are faster read twice (us, held / read twice: 16384, 296 rows 13.5/12.9, 450 rows
+  // 17.6/15.2, 4096 rows 126/83; 8448, 1000 rows 14.6/16.1, 4096 rows 54/46; 12288, 2000 rows 35/39, 4096 rows 66/63)
+  int dev = 0;
+  if (groups > 4) IZB_CUDA(cudaGetDevice(&dev));
+  const bool hold = groups <= 4 || M_valid <= izb_sm_count(dev) * (groups <= 6 ? 14 : 2);
+  auto kernel = !hold ? rmsnorm_quant_row_kernel<0> : groups <= 1 ? rmsnorm_quant_row_kernel<1> : groups <= 2 ? rmsnorm_quant_row_kernel<2> : groups <= 3 ? rmsnorm_quant_row_kernel<3>
               : groups <= 4 ? rmsnorm_quant_row_kernel<4> : groups <= 6 ? rmsnorm_quant_row_kernel<6> : groups <= 8 ? rmsnorm_quant_row_kernel<8>
                                                                                                                  : rmsnorm_quant_row_kernel<0>;
   IZB_LAUNCH("rmsnorm_quant", st, izb_launch_pdl(kernel, Mp, 256, 0, st, d_x, ldx, d_w, K, eps, M_valid, Mp, d_h, d_aq, d_asc, d_absum));

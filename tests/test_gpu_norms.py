@@ -24,3 +24,14 @@ def test_add_norm_quant(izb, M, K):
         aq, asc = izb.add_norm_quant(xd, torch.from_numpy(t).cuda(), torch.from_numpy(w).cuda(), 1e-6, 0.75, None if second is None else torch.from_numpy(second).cuda())
         rx, raq, rasc, _ = O.add_norm_quant(x, t, w, 1e-6, 0.75, second, Mp=asc.shape[1])
         assert (bits(xd.cpu().numpy()) == bits(rx)).all() and (aq.cpu().numpy() == raq).all() and (bits(asc.cpu().numpy()) == bits(rasc)).all()
+
+
+# (148 SMs: two rows of more than 12288, or fourteen of more than 8192 values per SM are held in registers, more are read twice)
+@pytest.mark.parametrize("M,K", [(3, 2304), (3, 4352), (3, 6400), (3, 8192), (3, 8448), (3, 12544), (3, 16640), (296, 12544), (297, 12544), (2072, 8448), (2073, 8448)])
+def test_rmsnorm_quant(izb, M, K):
+    import torch
+    rng = np.random.default_rng(M + K)
+    x, w = rng.standard_normal((M, K), dtype=np.float32), (1.0 + 0.2 * rng.standard_normal(K)).astype(np.float32)
+    aq, asc, h = izb.rmsnorm_quant(torch.from_numpy(x).cuda(), torch.from_numpy(w).cuda(), 1e-6, want_h=True)
+    ry, raq, rasc, _ = O.rmsnorm_quant(x, w, 1e-6, Mp=asc.shape[1])
+    assert (bits(h.cpu().numpy()) == bits(ry)).all() and (aq.cpu().numpy() == raq).all() and (bits(asc.cpu().numpy()) == bits(rasc)).all()
