@@ -40,6 +40,12 @@ template <class T>
 T* ptr(PyObject* o) {  // None = NULL
   return o == Py_None ? nullptr : static_cast<T*>(tensor(o).data_ptr());
 }
+// rows and columns, as `rows, columns = x.shape` unpacks them: other numbers of dimensions are a ValueError
+const at::Tensor& matrix(PyObject* o) {
+  const at::Tensor& t = tensor(o);
+  TORCH_CHECK_VALUE(t.dim() == 2, "expected two dimensions, got ", t.dim());
+  return t;
+}
 int num(PyObject* o) {
   const long v = PyLong_AsLong(o);
   if (v == -1 && PyErr_Occurred()) throw python_error();
@@ -122,7 +128,7 @@ struct Quantised {
 FN(quantize_act) {
   HANDLE_TH_ERRORS
   count(n, 6);
-  const at::Tensor& x = tensor(a[0]);
+  const at::Tensor& x = matrix(a[0]);
   const int M = (int)x.size(0), K = (int)x.size(1), Mp = rows_or_pad(a[1], M);
   if (a[3] != Py_None) {
     call(g.izb_quantize_act_, ptr<float>(a[0]), (int)x.stride(0), M, Mp, K, ptr<int8_t>(a[3]), ptr<float>(a[4]), ptr<int16_t>(a[5]));
@@ -156,7 +162,7 @@ FN(swiglu_quant) {
 FN(rmsnorm_quant) {
   HANDLE_TH_ERRORS
   count(n, 5);
-  const at::Tensor& x = tensor(a[0]);
+  const at::Tensor& x = matrix(a[0]);
   const int M = (int)x.size(0), K = (int)x.size(1), Mp = rows_or_pad(a[3], M);
   const float eps = real(a[2]);
   Quantised o(Mp, K, x.device());
@@ -172,7 +178,7 @@ FN(rmsnorm_quant) {
 FN(add_norm_quant) {
   HANDLE_TH_ERRORS
   count(n, 7);
-  const at::Tensor& x = tensor(a[0]);
+  const at::Tensor& x = matrix(a[0]);
   const int M = (int)x.size(0), K = (int)x.size(1), Mp = rows_or_pad(a[6], M);
   const float eps = real(a[3]), s = real(a[4]);
   Quantised o(Mp, K, x.device());
@@ -296,7 +302,7 @@ FN(moe_route) {
 FN(moe_sort) {
   HANDLE_TH_ERRORS
   count(n, 6);
-  const at::Tensor& ids = tensor(a[0]);
+  const at::Tensor& ids = matrix(a[0]);
   const c10::Device dev = ids.device();
   const int T = (int)ids.size(0), NU = (int)ids.size(1), NE = (int)tensor(a[2]).size(0), TM = num(a[3]), e0 = num(a[4]), e1 = num(a[5]);
   const int S = T * NU, max_tiles = (TM > 0 ? (S + TM - 1) / TM : 0) + NE;
@@ -339,7 +345,7 @@ FN(moe_down) {
 FN(moe_combine) {
   HANDLE_TH_ERRORS
   count(n, 7);
-  const at::Tensor& x = tensor(a[0]);
+  const at::Tensor& x = matrix(a[0]);
   const int T = (int)x.size(0), E = (int)x.size(1), NU = num(a[3]), partial = PyObject_IsTrue(a[6]) ? 1 : 0;
   call(g.izb_moe_combine_ex_, ptr<float>(a[0]), ptr<float>(a[1]), ptr<int32_t>(a[2]), T, NU, E, ptr<float>(a[4]), ptr<float>(a[5]), partial);
   return own(a[0]);

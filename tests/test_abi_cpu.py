@@ -120,3 +120,14 @@ def test_gateup_interleave_on_the_host():
         izb.gateup_interleave_host(12, g[:96], u[:96], 96, K)          # F % 64
     with pytest.raises(izb.IzbError):
         izb.gateup_interleave_host(99, g, u, F, K, n_mats=n_mats)       # unknown type
+
+
+@pytest.mark.parametrize("shape", [(256,), (2, 256, 3)])
+def test_binding_refuses_what_is_no_matrix(shape):
+    """Calls that unpack `rows, columns = x.shape` raise ValueError for other numbers of dimensions, before any device is asked for."""
+    torch = pytest.importorskip("torch")
+    x, w, i = torch.zeros(shape), torch.zeros(256), torch.zeros(shape, dtype=torch.int32)
+    for call in (lambda: izb.quantize_act(x), lambda: izb.rmsnorm_quant(x, w, 1e-6), lambda: izb.add_norm_quant(x, x, w, 1e-6), lambda: izb.moe_sort(i, w, i[0:1], 8),
+                 lambda: izb.moe_combine(x, x, i, 1)):
+        with pytest.raises(ValueError):
+            call()
