@@ -79,7 +79,7 @@ def _native():
         spec = importlib.util.spec_from_file_location("_izb_py", path)
         m = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(m)
-        m.bind(_check, {n: C.cast(getattr(lib(), n), C.c_void_p).value for n in m.names()})
+        m.bind(_check, lambda o: _p(o).value or 0, {n: C.cast(getattr(lib(), n), C.c_void_p).value for n in m.names()})
         _nat = m
     return _nat
 

@@ -29,7 +29,8 @@ struct Calls {
   IZB_PY_CALLS(X)
 #undef X
 } g;
-PyObject* g_fail = nullptr;  // Python callable(status): raises
+PyObject* g_fail = nullptr;     // Python callable(status): raises
+PyObject* g_address = nullptr;  // Python callable(object): the address of what is no torch tensor (a numpy array over pinned memory, ...)
 
 // ---- arguments
 const at::Tensor& tensor(PyObject* o) {
@@ -38,7 +39,25 @@ const at::Tensor& tensor(PyObject* o) {
 }
 template <class T>
 T* ptr(PyObject* o) {  // None = NULL
-  return o == Py_None ? nullptr : static_cast<T*>(tensor(o).data_ptr());
+  if (o == Py_None) return nullptr;
+  if (THPVariable_Check(o)) return static_cast<T*>(THPVariable_Unpack(o).data_ptr());
+  PyObject* v = PyObject_CallOneArg(g_address, o);
+  if (!v) throw python_error();
+  void* p = PyLong_AsVoidPtr(v);
+  Py_DECREF(v);
+  if (!p && PyErr_Occurred()) throw python_error();
+  return static_cast<T*>(p);
+}
+int extent(PyObject* o, int d) {  // o.shape[d]
+  if (THPVariable_Check(o)) return (int)THPVariable_Unpack(o).size(d);
+  PyObject* shape = PyObject_GetAttrString(o, "shape");
+  PyObject* v = shape ? PySequence_GetItem(shape, d) : nullptr;
+  Py_XDECREF(shape);
+  if (!v) throw python_error();
+  const long n = PyLong_AsLong(v);
+  Py_DECREF(v);
+  if (n == -1 && PyErr_Occurred()) throw python_error();
+  return (int)n;
 }
 // rows and columns, as `rows, columns = x.shape` unpacks them: other numbers of dimensions are a ValueError
 const at::Tensor& matrix(PyObject* o) {
@@ -205,9 +224,9 @@ struct Out {
   PyObject* given;
   float* p;
   int ld;
-  Out(PyObject* o, int rows, int cols, c10::Device dev) : given(o) {
+  Out(PyObject* o, int rows, int cols, PyObject* like) : given(o) {  // (`like`: on whose device)
     if (o == Py_None) {
-      made = empty({rows, cols}, at::kFloat, dev);
+      made = empty({rows, cols}, at::kFloat, tensor(like).device());
       p = static_cast<float*>(made.data_ptr());
       ld = cols;
     } else {
@@ -224,8 +243,8 @@ FN(matmul) {
   HANDLE_TH_ERRORS
   count(n, 9);
   izb_weight* w = weight(a[0]);
-  const int mat = num(a[2]), T = num(a[5]), c_off = num(a[7]), acc = num(a[8]), Mp = (int)tensor(a[4]).size(1);
-  Out o(a[6], Mp, num(a[1]), tensor(a[3]).device());
+  const int mat = num(a[2]), T = num(a[5]), c_off = num(a[7]), acc = num(a[8]), Mp = extent(a[4], 1);
+  Out o(a[6], Mp, num(a[1]), a[3]);
   call(g.izb_matmul_, w, mat, ptr<int8_t>(a[3]), ptr<float>(a[4]), nullptr, T, Mp, o.p, o.ld, c_off, acc);
   return o.result();
   END_HANDLE_TH_ERRORS
@@ -243,13 +262,10 @@ FN(quant_matmul) {
     Quantised q(Mp, K, x.device());
     aq = q.aq;
     asc = q.asc;
-  } else {
-    aq = tensor(a[10]);
-    asc = tensor(a[11]);
   }
-  Out o(a[6], Mp, num(a[1]), x.device());
-  int8_t* pq = static_cast<int8_t*>(aq.data_ptr());
-  float* ps = static_cast<float*>(asc.data_ptr());
+  Out o(a[6], Mp, num(a[1]), a[3]);
+  int8_t* pq = aq.defined() ? static_cast<int8_t*>(aq.data_ptr()) : ptr<int8_t>(a[10]);
+  float* ps = asc.defined() ? static_cast<float*>(asc.data_ptr()) : ptr<float>(a[11]);
   call(g.izb_quant_matmul_, w, mat, ptr<float>(a[3]), (int)x.stride(0), T, Mp, pq, ps, o.p, o.ld, c_off, acc);
   return tuple({o.result(), a[10] == Py_None ? wrap(aq) : own(a[10]), a[10] == Py_None ? wrap(asc) : own(a[11])});
   END_HANDLE_TH_ERRORS
@@ -260,8 +276,8 @@ FN(gemv) {
   HANDLE_TH_ERRORS
   count(n, 9);
   izb_weight* w = weight(a[0]);
-  const int mat = num(a[2]), T = num(a[5]), c_off = num(a[7]), acc = num(a[8]), Mp = (int)tensor(a[4]).size(1);
-  Out o(a[6], T, num(a[1]), tensor(a[3]).device());
+  const int mat = num(a[2]), T = num(a[5]), c_off = num(a[7]), acc = num(a[8]), Mp = extent(a[4], 1);
+  Out o(a[6], T, num(a[1]), a[3]);
   call(g.izb_gemv_, w, mat, ptr<int8_t>(a[3]), ptr<float>(a[4]), T, Mp, o.p, o.ld, c_off, acc);
   return o.result();
   END_HANDLE_TH_ERRORS
@@ -272,9 +288,9 @@ FN(gemm) {
   HANDLE_TH_ERRORS
   count(n, 10);
   izb_weight* w = weight(a[0]);
-  const int mat = num(a[2]), c_off = num(a[7]), acc = num(a[8]), impl = num(a[9]), Mp = (int)tensor(a[4]).size(1);
+  const int mat = num(a[2]), c_off = num(a[7]), acc = num(a[8]), impl = num(a[9]), Mp = extent(a[4], 1);
   const int m = a[5] == Py_None ? 0 : num(a[5]), M = m ? m : Mp;
-  Out o(a[6], Mp, num(a[1]), tensor(a[3]).device());
+  Out o(a[6], Mp, num(a[1]), a[3]);
   call(g.izb_gemm_, w, mat, ptr<int8_t>(a[3]), ptr<float>(a[4]), M, Mp, o.p, o.ld, c_off, acc, impl);
   return o.result();
   END_HANDLE_TH_ERRORS
@@ -304,7 +320,7 @@ FN(moe_sort) {
   count(n, 6);
   const at::Tensor& ids = matrix(a[0]);
   const c10::Device dev = ids.device();
-  const int T = (int)ids.size(0), NU = (int)ids.size(1), NE = (int)tensor(a[2]).size(0), TM = num(a[3]), e0 = num(a[4]), e1 = num(a[5]);
+  const int T = (int)ids.size(0), NU = (int)ids.size(1), NE = extent(a[2], 0), TM = num(a[3]), e0 = num(a[4]), e1 = num(a[5]);
   const int S = T * NU, max_tiles = (TM > 0 ? (S + TM - 1) / TM : 0) + NE;
   at::Tensor offs = empty({NE + 1}, at::kInt, dev), tiles = empty({1 + 3 * (int64_t)max_tiles}, at::kInt, dev), stok = empty({S}, at::kInt, dev),
              swt = empty({S}, at::kFloat, dev), inv = empty({S}, at::kInt, dev);
@@ -320,7 +336,7 @@ FN(moe_gateup) {
   HANDLE_TH_ERRORS
   count(n, 10);
   izb_weight *wg = weight(a[0]), *wu = weight(a[1]);
-  const int N = num(a[2]), Mp = (int)tensor(a[4]).size(1), max_tiles = num(a[6]), TM = num(a[7]), S = num(a[9]);
+  const int N = num(a[2]), Mp = extent(a[4], 1), max_tiles = num(a[6]), TM = num(a[7]), S = num(a[9]);
   at::Tensor h = empty({S, N}, at::kFloat, tensor(a[3]).device());
   float* ph = static_cast<float*>(h.data_ptr());
   call(g.izb_moe_gateup_, wg, wu, ptr<int8_t>(a[3]), ptr<float>(a[4]), Mp, ptr<int32_t>(a[5]), max_tiles, TM, ptr<int32_t>(a[8]), ph);
@@ -333,7 +349,7 @@ FN(moe_down) {
   HANDLE_TH_ERRORS
   count(n, 9);
   izb_weight* w = weight(a[0]);
-  const int N = num(a[1]), Sp = (int)tensor(a[3]).size(1), max_tiles = num(a[5]), TM = num(a[6]), S = num(a[8]);
+  const int N = num(a[1]), Sp = extent(a[3], 1), max_tiles = num(a[5]), TM = num(a[6]), S = num(a[8]);
   at::Tensor y = empty({S, N}, at::kFloat, tensor(a[2]).device());
   float* py = static_cast<float*>(y.data_ptr());
   call(g.izb_moe_down_, w, ptr<int8_t>(a[2]), ptr<float>(a[3]), Sp, ptr<int32_t>(a[4]), max_tiles, TM, ptr<float>(a[7]), py);
@@ -352,13 +368,13 @@ FN(moe_combine) {
   END_HANDLE_TH_ERRORS
 }
 
-// bind(fail, {"izb_...": address})
+// bind(fail, address, {"izb_...": address})
 FN(bind) {
   HANDLE_TH_ERRORS
-  count(n, 2);
+  count(n, 3);
 #define X(name)                                                                    \
   {                                                                                \
-    PyObject* v = PyDict_GetItemString(a[1], #name);                               \
+    PyObject* v = PyDict_GetItemString(a[2], #name);                               \
     if (!v) throw torch::TypeError("bind: no address for " #name);             \
     g.name##_ = reinterpret_cast<decltype(&name)>(PyLong_AsVoidPtr(v));            \
     if (!g.name##_) throw torch::TypeError("bind: null address for " #name);   \
@@ -366,7 +382,9 @@ FN(bind) {
   IZB_PY_CALLS(X)
 #undef X
   Py_INCREF(a[0]);
+  Py_INCREF(a[1]);
   g_fail = a[0];
+  g_address = a[1];
   Py_RETURN_NONE;
   END_HANDLE_TH_ERRORS
 }

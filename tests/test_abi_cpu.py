@@ -131,3 +131,20 @@ def test_binding_refuses_what_is_no_matrix(shape):
                  lambda: izb.moe_combine(x, x, i, 1)):
         with pytest.raises(ValueError):
             call()
+
+
+def test_binding_takes_what_has_an_address():
+    """A buffer may be anything with an address (a numpy array over pinned memory): the calls reach the library, or the search for a device,
+    instead of refusing the type."""
+    torch = pytest.importorskip("torch")
+    x, w = torch.zeros(4, 256), np.zeros(256, np.float32)
+    aq, asc = np.zeros((16, 256), np.int8), np.zeros((8, 16), np.float32)
+    class Handle:
+        handle, N, K = C.c_void_p(0), 64, 256
+    if torch.cuda.is_available():
+        pytest.skip("host buffers that are not pinned: for machines without a device only")
+    for call in (lambda: izb.rmsnorm_quant(x, w, 1e-6), lambda: izb.add_norm_quant(x, w, w, 1e-6), lambda: izb.quantize_act(x, out=(aq, asc, None)),
+                 lambda: izb.matmul(Handle, aq, asc, 2, out=x), lambda: izb.quant_matmul(Handle, x, 2, out=x, qout=(aq, asc))):
+        with pytest.raises(Exception) as e:
+            call()
+        assert not isinstance(e.value, TypeError), e.value
