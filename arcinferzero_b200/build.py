@@ -66,9 +66,9 @@ def build(verbose: bool = False) -> str:
         for log in ex.map(run, jobs):
             if verbose and log:
                 print(log)
-        py.result()
     if jobs or not os.path.exists(OUT):
         run([NVCC, "-shared", "-o", OUT, *objs, "-lcudart", "-ldl", "-lgomp", "-ccbin", "/usr/bin/g++"])
+    py.result()  # (last: the library needs neither torch nor Python headers, and is there for C hosts when the binding cannot be built)
     return OUT
 
 

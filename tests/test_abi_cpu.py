@@ -148,3 +148,16 @@ def test_binding_takes_what_has_an_address():
         with pytest.raises(Exception) as e:
             call()
         assert not isinstance(e.value, TypeError), e.value
+
+
+def test_library_is_linked_when_the_binding_cannot_be_built(monkeypatch, tmp_path):
+    from arcinferzero_b200 import build as B
+    B.build()  # (objects up to date)
+
+    def no_torch():
+        raise RuntimeError("no torch here")
+    monkeypatch.setattr(B, "build_python_module", no_torch)
+    monkeypatch.setattr(B, "OUT", str(tmp_path / "libizb200.so"))
+    with pytest.raises(RuntimeError, match="no torch here"):
+        B.build()
+    assert hasattr(C.CDLL(B.OUT), "izb_gemm")
