@@ -25,14 +25,25 @@ def sources():
     return sorted(f for f in os.listdir(CSRC) if f.endswith(".cu"))
 
 
+def python_module_for() -> str:
+    """What a built binding belongs to: it uses internals of torch and CPython, so another version of either wants another build."""
+    import sysconfig
+
+    import torch
+    return f"{sysconfig.get_config_var('SOABI')} torch {torch.__version__} cxx11abi {int(torch.compiled_with_cxx11_abi())}"
+
+
 def build_python_module() -> None:
     """_izb_py.so: plain C++ against the CPython and torch headers (no CUDA code of its own)."""
     import sysconfig
 
     import torch
     src, hdr = os.path.join(CSRC, "izb_py.cpp"), os.path.join(os.path.dirname(HERE), "include", "izb200.h")
-    if os.path.exists(PY_OUT) and os.path.getmtime(PY_OUT) >= max(os.path.getmtime(src), os.path.getmtime(hdr)):
-        return
+    stamp, made_for = PY_OUT + ".build", python_module_for()
+    if os.path.exists(PY_OUT) and os.path.getmtime(PY_OUT) >= max(os.path.getmtime(src), os.path.getmtime(hdr)) and os.path.exists(stamp):
+        with open(stamp) as f:
+            if f.read() == made_for:
+                return
     t = os.path.dirname(torch.__file__)
     cmd = ["/usr/bin/g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
            "-I" + sysconfig.get_paths()["include"], "-isystem", os.path.join(t, "include"), "-isystem", os.path.join(t, "include/torch/csrc/api/include"),
@@ -41,6 +52,8 @@ def build_python_module() -> None:
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError("g++ failed:\n" + " ".join(cmd) + "\n" + r.stdout + r.stderr)
+    with open(stamp, "w") as f:
+        f.write(made_for)
 
 
 def build(verbose: bool = False) -> str:

@@ -161,3 +161,20 @@ def test_library_is_linked_when_the_binding_cannot_be_built(monkeypatch, tmp_pat
     with pytest.raises(RuntimeError, match="no torch here"):
         B.build()
     assert hasattr(C.CDLL(B.OUT), "izb_gemm")
+
+
+def test_binding_is_rebuilt_for_another_torch(monkeypatch, tmp_path):
+    import subprocess
+    from arcinferzero_b200 import build as B
+    monkeypatch.setattr(B, "PY_OUT", str(tmp_path / "_izb_py.so"))
+    calls = []
+
+    def compiler(cmd, **kw):
+        calls.append(cmd)
+        open(B.PY_OUT, "w").close()
+        return subprocess.CompletedProcess(cmd, 0, "", "")
+    monkeypatch.setattr(B.subprocess, "run", compiler)
+    for made_for, built in (("torch 1", 1), ("torch 1", 1), ("torch 2", 2), ("torch 2", 2)):
+        monkeypatch.setattr(B, "python_module_for", lambda made_for=made_for: made_for, raising=False)
+        B.build_python_module()
+        assert len(calls) == built, (made_for, calls)
