@@ -404,6 +404,14 @@ extern "C" int izb_weight_create_slice(int type, const void* h_rows, int n_mats,
     delete w;
     IZB_FAIL(IZB_ERR_CUDA, "weight_create: upload failed: %s", cudaGetErrorString(e));
   }
+  // Every kernel with a bounded wait reports through the device's error word: made here, so that no product allocates it, in a stream
+  // capture least of all.
+  if (!izb_device_error_word(device)) {
+    cudaGetLastError();
+    cudaFree(w->raw);
+    delete w;
+    IZB_FAIL(IZB_ERR_NOMEM, "weight_create: no device error word");
+  }
   w->has_tmap = izb_make_raw_tensor_map(w) == IZB_OK;
   w->has_tmap16 = (w->type != IZB_K16 || w->packed6) && izb_make_rows_tensor_map(w) == IZB_OK;
   *out = w;

@@ -1,0 +1,46 @@
+"""Products inside a stream capture that are the first of their kind in the process: nothing may allocate there, and a replayed graph
+may rely on no block that a later call gives back.  Each case is a process of its own."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+PRELUDE = """
+import numpy as np, torch
+import arcinferzero_b200 as izb
+from arcinferzero_b200 import synth as S
+
+def captured(call):
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        call()
+    return graph
+
+def rel(a, b):
+    return float((a.double() - b.double()).abs().max() / b.double().abs().max())
+"""
+
+
+def run(body):
+    r = subprocess.run([sys.executable, "-c", PRELUDE + body], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "done" in r.stdout, r.stdout + r.stderr
+
+
+def test_first_call_is_a_captured_gemv():
+    """Q6_K at three rows: a kernel with bounded waits whose first call in the process is in a capture."""
+    run("""
+N, K, T = 256, 768, 3
+W = izb.Weight(14, S.make_weight(14, N, K, 1), N, K)
+aq, asc, _ = izb.quantize_act(torch.from_numpy(S.make_act(T, K, 2)).cuda())
+out = torch.zeros((T, N), device="cuda")
+graph = captured(lambda: izb.gemv(W, aq, asc, T, out=out))
+graph.replay()
+torch.cuda.synchronize()
+got = out.clone()
+assert rel(got, izb.gemm(W, aq, asc, M=T, impl=izb.GEMM_CORE)[:T]) < 1e-5 and izb.device_status(0) == 0
+print("done")
+""")
