@@ -396,8 +396,9 @@ extern "C" int izb_weight_create_slice(int type, const void* h_rows, int n_mats,
     regroup_q8_0_kernel<<<(unsigned)((items + 255) / 256), 256>>>(tmp, w->raw, n_sb);
     g_izb_launches.fetch_add(1);
     e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaDeviceSynchronize();
   }
+  // (a copy from pageable memory may return while its last piece is on the way: the GEMVs of any stream read weights ahead of everything)
+  if (e == cudaSuccess) e = cudaDeviceSynchronize();
   if (tmp) cudaFree(tmp);
   if (e != cudaSuccess) {
     cudaFree(w->raw);

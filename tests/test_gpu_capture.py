@@ -44,3 +44,23 @@ got = out.clone()
 assert rel(got, izb.gemm(W, aq, asc, M=T, impl=izb.GEMM_CORE)[:T]) < 1e-5 and izb.device_status(0) == 0
 print("done")
 """)
+
+
+@pytest.mark.parametrize("qt", [12, 14, 13])
+def test_weights_are_whole_when_created(qt):
+    """A product on another stream right behind the creation of a weight from pageable memory."""
+    run(f"""
+qt, N, K = {qt}, 4096, 4096
+rows = S.make_weight(qt, N, K, 1)
+aq, asc, _ = izb.quantize_act(torch.from_numpy(S.make_act(2, K, 2)).cuda())
+torch.cuda.synchronize()
+stream, got = torch.cuda.Stream(), []
+with torch.cuda.stream(stream):
+    for _ in range(4):
+        W = izb.Weight(qt, rows, N, K)
+        got.append(izb.gemv(W, aq, asc, 2))
+        torch.cuda.synchronize()
+assert all(torch.equal(g, got[-1]) for g in got)
+assert rel(got[0], izb.gemm(W, aq, asc, M=2, impl=izb.GEMM_CORE)[:2]) < 1e-5
+print("done")
+""")
