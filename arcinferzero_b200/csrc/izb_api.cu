@@ -242,10 +242,16 @@ static int grow_arena(DevState& d, int device, int slot, size_t bytes) {
   return IZB_OK;
 }
 
-int izb_workspace(int device, int slot, size_t bytes, void** out) {
+int izb_workspace(int device, int slot, size_t bytes, cudaStream_t st, void** out, bool other_way) {
   DevState& d = g_dev[device];
   std::lock_guard<std::mutex> lk(d.mu);
-  if (int rc = grow_arena(d, device, slot, bytes)) return rc;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) {  // (the legacy stream beside a capture: no place to allocate either)
+    cudaGetLastError();
+    capture = cudaStreamCaptureStatusInvalidated;
+  }
+  if (other_way && bytes > d.ws_bytes[slot] && capture != cudaStreamCaptureStatusNone) return 1;
+  if (int rc = grow_arena(d, device, slot, bytes)) return other_way ? 1 : rc;
   *out = d.ws[slot];
   return IZB_OK;
 }
@@ -576,7 +582,7 @@ extern "C" int izb_gemm(const izb_weight* w, int mat, const int8_t* d_aq, const 
   }
   if (acc == 3) {  // both projections side by side into scratch, then the SwiGLU product of the column groups
     void* ws = nullptr;
-    if (int rc = izb_workspace(w->device, kWsGemm, (size_t)Mp * w->N * 4, &ws)) return rc;
+    if (int rc = izb_workspace(w->device, kWsGemm, (size_t)Mp * w->N * 4, st, &ws)) return rc;
     if (int rc = izb_gemm_core_launch(w, w->raw + (size_t)mat * w->N * w->row_bytes, d_aq, d_asc, M, Mp, (float*)ws, w->N, 0, 0, nullptr, st)) return rc;
     return izb_swiglu_pairs_launch((const float*)ws, w->N, M, w->N / 2, d_C, ldc, c_off, st);
   }

@@ -129,9 +129,10 @@ uint32_t* izb_device_error_word(int device);
 
 // Per-device scratch arenas, one per user so that independent users never share bytes; each is grown on demand
 // (cudaMalloc only when a call needs more than any call before it).  Calls that use the same arena must be ordered on
-// one stream.
+// one stream.  `other_way`: the caller has another kernel; +1 instead of an error where the arena would have to grow and cannot -- in a
+// stream capture, or without memory.
 enum { kWsGemm = 0, kWsTp = 1, kWsMoe = 2, kWsCheck = 3, kWsNorm = 4 };
-int izb_workspace(int device, int slot, size_t bytes, void** out);
+int izb_workspace(int device, int slot, size_t bytes, cudaStream_t st, void** out, bool other_way = false);
 
 // ---------------------------------------------------------------------------------------------- programmatic dependent launch
 // A decode step is a chain of kernels of a few microseconds, each waiting for the one before.  Launched with this attribute

@@ -1131,6 +1131,8 @@ int launch_tc_of(const izb_weight* w, TcParams& p, dim3 grid, cudaStream_t st) {
 
 // operand stages per superblock: weights with mins carry the min term as a fifth one
 int tc_sps(const izb_weight* w, bool dots) { return (w->type == IZB_Q4_K || (w->type == IZB_K16 && w->has_min)) && !dots ? 5 : 4; }
+// Weights that the CUDA-core kernel takes without an arena, and took alone before this kernel did: a call whose arena cannot be had goes there
+bool tc_optional(const izb_weight* w) { return w->type == IZB_K16 || w->N % BN != 0; }
 // does the kernel take this weight at all
 bool tc_takes(const izb_weight* w) { return w->has_tmap && w->N % 16 == 0 && w->K % 256 == 0; }
 
@@ -1216,7 +1218,7 @@ int run_tc(const izb_weight* w, int mat, const int8_t* aq, const float* asc, int
   tc_scratch_bytes(n_tiles_grid, w->K, tc_sps(w, dots != nullptr), &img_bytes, &asc_bytes);
   const size_t split_bytes = tiles || dots ? 0 : split_area(w->device);
   void* ws = nullptr;
-  if (int rc = izb_workspace(w->device, ws_slot, img_bytes + asc_bytes + split_bytes, &ws)) return rc;
+  if (int rc = izb_workspace(w->device, ws_slot, img_bytes + asc_bytes + split_bytes, st, &ws, !tiles && !dots && tc_optional(w))) return rc;
   uint32_t* err = izb_device_error_word(w->device);
   if (!err) IZB_FAIL(IZB_ERR_NOMEM, "gemm: no device error word");
   float* split_ws = split_bytes ? (float*)((unsigned char*)ws + img_bytes + asc_bytes) : nullptr;
@@ -1277,7 +1279,7 @@ int izb_gemm_tc_quant_launch(const izb_weight* w, int mat, const float* x, int l
   size_t img_bytes, asc_bytes;
   tc_scratch_bytes(n_tiles, K, sps, &img_bytes, &asc_bytes);
   void* ws = nullptr;
-  if (int rc = izb_workspace(w->device, kWsGemm, img_bytes + asc_bytes + split_area(w->device), &ws)) return rc;
+  if (int rc = izb_workspace(w->device, kWsGemm, img_bytes + asc_bytes + split_area(w->device), st, &ws, tc_optional(w))) return rc;
   uint32_t* err = izb_device_error_word(w->device);
   if (!err) IZB_FAIL(IZB_ERR_NOMEM, "gemm: no device error word");
   uint16_t* aimg = (uint16_t*)ws;
@@ -1376,7 +1378,7 @@ extern "C" int izb_selfcheck(int device) {
     const size_t n_out = (size_t)Mp * N, n_dots = (size_t)M * N * nb;
     void* ws = nullptr;
     const size_t need = w.bytes + kRawSlack + (size_t)Mp * K + (size_t)nb * Mp * 4 + 2 * n_out * 4 + 2 * n_dots * 4 + 4096;
-    if (int rc = izb_workspace(device, kWsCheck, need, &ws)) return rc;
+    if (int rc = izb_workspace(device, kWsCheck, need, 0, &ws)) return rc;
     uint8_t* base = (uint8_t*)ws;
     w.raw = base; base += (w.bytes + kRawSlack + 255) & ~size_t(255);
     int8_t* aq = (int8_t*)base; base += (size_t)Mp * K;

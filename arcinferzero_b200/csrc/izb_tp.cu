@@ -312,7 +312,7 @@ extern "C" int izb_tp_reduce_quant_gather(izb_tp* tp, const float* d_x, float* d
   //    rank and are re-laid to [E/32][rows] after the gather
   void* ws = nullptr;
   const size_t sc_bytes = (size_t)(E / 32) * rows * 4;
-  if (int rc = izb_workspace(tp->device, kWsTp, sc_bytes, &ws)) return rc;
+  if (int rc = izb_workspace(tp->device, kWsTp, sc_bytes, st, &ws)) return rc;
   float* sc_stage = (float*)ws;  // [R][E/32][own]
   if (int rc = izb_quantize_act(mine, E, own, own, E, d_aq + (size_t)tp->rank * n_own, sc_stage + (size_t)tp->rank * (E / 32) * own, nullptr, st)) return rc;
   if (R > 1) {

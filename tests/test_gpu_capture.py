@@ -64,3 +64,26 @@ assert all(torch.equal(g, got[-1]) for g in got)
 assert rel(got[0], izb.gemm(W, aq, asc, M=2, impl=izb.GEMM_CORE)[:2]) < 1e-5
 print("done")
 """)
+
+
+@pytest.mark.parametrize("qt,N", [(14, 128), (13, 128), (23, 128), (8, 144), (12, 144)])
+def test_first_call_is_a_captured_gemm(qt, N):
+    """Per-16-scale types and part columns: the tensor-core kernel's arena cannot be made in a capture, the CUDA-core kernel needs none."""
+    run(f"""
+qt, N, K, T = {qt}, {N}, 1024, 40
+W = izb.Weight(qt, S.make_weight(qt, N, K, 1), N, K)
+x = torch.from_numpy(S.make_act(T, K, 2)).cuda()
+aq, asc, _ = izb.quantize_act(x)
+a, b = torch.zeros((48, N), device="cuda"), torch.zeros((48, N), device="cuda")
+q = (torch.empty_like(aq), torch.empty_like(asc))
+def call():
+    izb.matmul(W, aq, asc, T, out=a)
+    izb.quant_matmul(W, x, T, out=b, qout=q)
+graph = captured(call)
+graph.replay()
+torch.cuda.synchronize()
+want = izb.gemm(W, aq, asc, impl=izb.GEMM_CORE)
+assert torch.equal(a, want) and torch.equal(b, want) and torch.equal(q[0], aq)
+assert rel(izb.matmul(W, aq, asc, T), want) < 1e-5 and izb.device_status(0) == 0  # (by itself: the arena is made, the tensor cores run)
+print("done")
+""")
