@@ -127,6 +127,7 @@ struct DevState {
   std::atomic<uint32_t*> err_word{nullptr};
   void* ws[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};  // scratch arenas by user (izb_common.cuh: kWs*)
   size_t ws_bytes[5] = {0, 0, 0, 0, 0};
+  bool ws_in_graph[5] = {false, false, false, false, false};  // a capture has seen the block: it stays
   void* stage = nullptr;  // staging of the host-buffer call
   size_t stage_bytes = 0;
   cudaStream_t hs[3] = {nullptr, nullptr, nullptr};  // host-buffer call: copy-in, compute, copy-out streams
@@ -227,19 +228,26 @@ void izb_note_noalloc_status(int device, uint32_t* status) {
 // (work in flight may still read the old block) -- izb_reserve moves that wait out of the hot path.
 static int grow_arena(DevState& d, int device, int slot, size_t bytes) {
   if (bytes <= d.ws_bytes[slot]) return IZB_OK;
-  if (d.ws[slot]) {
+  size_t sizes[2] = {bytes, bytes};  // tried in turn
+  if (d.ws_in_graph[slot]) {  // (the old block is left to the graphs)
+    if (bytes < 2 * d.ws_bytes[slot]) sizes[0] = 2 * d.ws_bytes[slot];
+    d.ws_in_graph[slot] = false;
+  } else if (d.ws[slot]) {
     IZB_CUDA(cudaDeviceSynchronize());
     IZB_CUDA(cudaFree(d.ws[slot]));
-    d.ws[slot] = nullptr;
-    d.ws_bytes[slot] = 0;
   }
-  const size_t want = (bytes + (size_t(1) << 20) - 1) & ~((size_t(1) << 20) - 1);
-  if (cudaMalloc(&d.ws[slot], want) != cudaSuccess) {
+  d.ws[slot] = nullptr;
+  d.ws_bytes[slot] = 0;
+  for (size_t size : sizes) {
+    const size_t want = (size + (size_t(1) << 20) - 1) & ~((size_t(1) << 20) - 1);
+    if (cudaMalloc(&d.ws[slot], want) == cudaSuccess) {
+      d.ws_bytes[slot] = want;
+      return IZB_OK;
+    }
     cudaGetLastError();
-    IZB_FAIL(IZB_ERR_NOMEM, "workspace of %zu bytes on device %d", want, device);
+    d.ws[slot] = nullptr;
   }
-  d.ws_bytes[slot] = want;
-  return IZB_OK;
+  IZB_FAIL(IZB_ERR_NOMEM, "workspace of %zu bytes on device %d", bytes, device);
 }
 
 int izb_workspace(int device, int slot, size_t bytes, cudaStream_t st, void** out, bool other_way) {
@@ -252,6 +260,7 @@ int izb_workspace(int device, int slot, size_t bytes, cudaStream_t st, void** ou
   }
   if (other_way && bytes > d.ws_bytes[slot] && capture != cudaStreamCaptureStatusNone) return 1;
   if (int rc = grow_arena(d, device, slot, bytes)) return other_way ? 1 : rc;
+  if (capture == cudaStreamCaptureStatusActive) d.ws_in_graph[slot] = true;
   *out = d.ws[slot];
   return IZB_OK;
 }

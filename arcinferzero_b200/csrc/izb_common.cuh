@@ -129,8 +129,9 @@ uint32_t* izb_device_error_word(int device);
 
 // Per-device scratch arenas, one per user so that independent users never share bytes; each is grown on demand
 // (cudaMalloc only when a call needs more than any call before it).  Calls that use the same arena must be ordered on
-// one stream.  `other_way`: the caller has another kernel; +1 instead of an error where the arena would have to grow and cannot -- in a
-// stream capture, or without memory.
+// one stream.  A block that a captured graph holds is never given back (the graph may be replayed at any time): the arena then at least
+// doubles where memory allows, so that all such blocks together hold no more than it.  `other_way`: the caller has another kernel; +1 instead
+// of an error where the arena would have to grow and cannot -- in a stream capture, or without memory.
 enum { kWsGemm = 0, kWsTp = 1, kWsMoe = 2, kWsCheck = 3, kWsNorm = 4 };
 int izb_workspace(int device, int slot, size_t bytes, cudaStream_t st, void** out, bool other_way = false);
 

@@ -87,3 +87,29 @@ assert torch.equal(a, want) and torch.equal(b, want) and torch.equal(q[0], aq)
 assert rel(izb.matmul(W, aq, asc, T), want) < 1e-5 and izb.device_status(0) == 0  # (by itself: the arena is made, the tensor cores run)
 print("done")
 """)
+
+
+def test_replays_outlive_the_growth_of_an_arena():
+    run("""
+qt, N, K = 14, 256, 1024
+W = izb.Weight(qt, S.make_weight(qt, N, K, 1), N, K)
+def operands(T):
+    x = torch.from_numpy(S.make_act(T, K, T)).cuda()
+    return izb.quantize_act(x)[:2]
+aq, asc = operands(40)
+out = torch.zeros((48, N), device="cuda")
+izb.matmul(W, aq, asc, 40, out=out)
+want = out.clone()
+graph = captured(lambda: izb.matmul(W, aq, asc, 40, out=out))
+for T in (3000, 9000, 20000):  # the arena grows past the graph's block
+    big = operands(T)
+    izb.matmul(W, *big, T)
+    other = torch.full((64 << 20,), 0xFF, dtype=torch.uint8, device="cuda")  # whatever takes a block given back
+    out.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, want), T
+    assert int(other.min()) == 0xFF
+assert izb.device_status(0) == 0
+print("done")
+""")
