@@ -564,6 +564,16 @@ static int check_gemm_args(const izb_weight* w, int mat, const int8_t* aq, const
   return IZB_OK;
 }
 
+// Is the CUDA-core kernel faster?  Asked where the tensor-core kernel is the newcomer (N % 128 != 0; Q5_K, Q6_K, IQ4_XS): one wave of the
+// other's 64 x 64 tiles over a short K ends before this one's pre-pass and pipeline are through, all the more so where the store reads C
+// (us, CUDA cores / tensor cores: store, Q6_K 1024 rows x 272 x 256 10/12, x 512 19/15; adding, Q6_K 208 x 528 x 512 21/24, Q8_0 208 x 528 x 1024
+// 28/31; SwiGLU, Q6_K 512 x 1040 x 1024 40/45, Q8_0 64 x 272 x 1536 42/48, Q4_K 208 x 528 x 1024 33/40; two waves lose: adding, Q6_K 1024 x 1040 x 512 30/25).
+static bool gemm_core_first(const izb_weight* w, int M, int acc) {
+  if (acc > 2 || (w->type != IZB_K16 && w->N % 128 == 0)) return false;
+  const int max_k = w->type == IZB_K16 ? 256 << acc : w->type == IZB_Q8_0 ? 512 << acc : acc == 0 ? 256 : acc == 1 ? 512 : 1536;
+  return w->K <= max_k && (long long)((M + 63) / 64) * ((w->N + 63) / 64) <= izb_sm_count(w->device);
+}
+
 extern "C" int izb_gemm(const izb_weight* w, int mat, const int8_t* d_aq, const float* d_asc, int M, int Mp, float* d_C, int ldc,
                         int c_off, int acc, int impl, void* stream) {
   if (int rc = check_gemm_args(w, mat, d_aq, d_asc, M, Mp, d_C, ldc, c_off, acc)) return rc;
@@ -573,14 +583,14 @@ extern "C" int izb_gemm(const izb_weight* w, int mat, const int8_t* d_aq, const 
     if (impl == IZB_GEMM_TC) IZB_FAIL(IZB_ERR_TYPE, "gemm: the tensor-core kernel does not take ggml type %d", w->ggml_type);
     if (impl != IZB_GEMM_AUTO && impl != IZB_GEMM_CORE) IZB_FAIL(IZB_ERR_ARG, "gemm: impl %d", impl);
     if (acc == 3) IZB_FAIL(IZB_ERR_TYPE, "gemm: store mode 3 is not built for ggml type %d", w->ggml_type);
-    if (impl == IZB_GEMM_AUTO && g_dev[w->device].tc_ok.load() != 0) {
+    if (impl == IZB_GEMM_AUTO && g_dev[w->device].tc_ok.load() != 0 && !gemm_core_first(w, M, acc)) {
       const int rc = izb_gemm_tc_launch(w, mat, d_aq, d_asc, M, Mp, d_C, ldc, c_off, acc, nullptr, st);
       if (rc <= 0) return rc;
     }
     return izb_gemm_k16_launch(w, w->raw + (size_t)mat * w->N * w->row_bytes, d_aq, d_asc, M, Mp, d_C, ldc, c_off, acc, nullptr, st);
   }
   if (impl == IZB_GEMM_AUTO || impl == IZB_GEMM_TC) {
-    const bool allowed = impl == IZB_GEMM_TC || g_dev[w->device].tc_ok.load() != 0;
+    const bool allowed = impl == IZB_GEMM_TC || (g_dev[w->device].tc_ok.load() != 0 && !gemm_core_first(w, M, acc));
     if (allowed) {
       const int rc = izb_gemm_tc_launch(w, mat, d_aq, d_asc, M, Mp, d_C, ldc, c_off, acc, nullptr, st);
       if (rc <= 0) return rc;
@@ -640,7 +650,7 @@ extern "C" int izb_quant_matmul(const izb_weight* w, int mat, const float* d_x, 
     if (int rc = check_gemm_args(w, mat, d_aq, d_asc, Mp, Mp, d_C, ldc, c_off, acc)) return rc;
     if (ldx < w->K || ldx % 4 || !izb_aligned(d_x, 16)) IZB_FAIL(IZB_ERR_ALIGN, "quant_matmul: x must be 16-byte aligned with ldx >= K a multiple of 4");
     if (int rc = izb_require_device(w->device, "quant_matmul")) return rc;
-    const int rc = izb_gemm_tc_quant_launch(w, mat, d_x, ldx, T, Mp, d_aq, d_asc, d_C, ldc, c_off, acc, (cudaStream_t)stream);
+    const int rc = gemm_core_first(w, Mp, acc) ? 1 : izb_gemm_tc_quant_launch(w, mat, d_x, ldx, T, Mp, d_aq, d_asc, d_C, ldc, c_off, acc, (cudaStream_t)stream);
     if (rc <= 0) return rc;
   }
   if (int rc = izb_quantize_act(d_x, ldx, T, Mp, w->K, d_aq, d_asc, nullptr, stream)) return rc;

@@ -8,6 +8,13 @@ from arcinferzero_b200 import synth as S
 pytestmark = pytest.mark.gpu
 
 
+def kernels_of(izb, call):
+    """Names of the library kernels that `call` launches."""
+    izb.profile_start()
+    call()
+    return set(izb.profile_stop())
+
+
 def extremes(qt, rows):
     """Largest scales and quants of either sign in some rows: products up to 4096 must stay exact."""
     v = rows.copy()
@@ -49,4 +56,26 @@ def test_tensor_core_gemm_equals_core_gemm(izb, qt, M, N, K):
     want = izb.gemm(W, aq, asc)
     assert torch.equal(got[:M], want[:M])
     assert izb.device_status(0) == 0
+    W.close()
+
+
+# One wave of 64 x 64 tiles over a short K goes to the CUDA-core kernel, where the tensor-core kernel is the newcomer (part columns,
+# per-16-scale types); the border in K depends on type and store mode.
+@pytest.mark.parametrize("qt,M,N,K,acc,core", [(14, 64, 128, 256, 0, True), (14, 64, 128, 512, 0, False), (13, 64, 144, 512, 1, True), (23, 64, 144, 768, 1, False),
+                                               (14, 64, 272, 1024, 2, True), (14, 64, 272, 1280, 2, False), (14, 1024, 1040, 256, 0, False), (8, 64, 144, 512, 0, True),
+                                               (8, 64, 144, 768, 0, False), (2, 64, 144, 1024, 1, True), (8, 64, 144, 2048, 2, True), (12, 64, 144, 512, 1, True),
+                                               (12, 64, 144, 512, 0, False), (12, 64, 128, 256, 0, False), (8, 64, 256, 256, 2, False)])
+def test_short_calls_take_the_faster_kernel(izb, qt, M, N, K, acc, core):
+    import torch
+    W = izb.Weight(qt, S.make_weight(qt, N, K, N + K + qt), N, K)
+    x = torch.from_numpy(S.make_act(M, K, M + K)).cuda()
+    aq, asc, _ = izb.quantize_act(x)
+    base = torch.from_numpy(np.random.default_rng(acc).standard_normal((M, N)).astype(np.float32)).cuda()
+    want = izb.gemm(W, aq, asc, out=base.clone(), acc=acc, impl=izb.GEMM_CORE)
+    a, b = base.clone(), base.clone()
+    for out, call in ((a, lambda: izb.matmul(W, aq, asc, M, out=a, acc=acc)), (b, lambda: izb.quant_matmul(W, x, M, out=b, acc=acc))):
+        ran = kernels_of(izb, call)
+        assert ("gemm_tc" not in ran) == core, ran
+        assert torch.equal(out, want) if core else float((out - want).abs().max() / want.abs().max()) < 1e-5
+    assert torch.equal(a, b)
     W.close()
