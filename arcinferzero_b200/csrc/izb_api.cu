@@ -198,6 +198,12 @@ int izb_sm_budget(int device) {
   return lim > 0 && lim < n ? lim : n;
 }
 
+bool izb_one_wave(dim3 grid, int threads) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  return (long long)grid.x * grid.y * threads <= (long long)izb_sm_count(dev) * 2048;
+}
+
 extern "C" int izb_set_sm_limit(int device, int sms) {
   if (device < 0 || device >= kIzbMaxDev) IZB_FAIL(IZB_ERR_ARG, "set_sm_limit: device %d out of range", device);
   if (sms < 0) IZB_FAIL(IZB_ERR_ARG, "set_sm_limit: %d", sms);

@@ -141,6 +141,10 @@ int izb_workspace(int device, int slot, size_t bytes, cudaStream_t st, void** ou
 // free; it may set itself up and touch what no kernel writes (the library's weights), and calls pdl_wait() -- which returns
 // when the kernel before it has completed and its writes are visible -- before it reads or writes anything else.  Every
 // kernel launched this way calls pdl_wait() on every path, so completion stays transitive along the stream.
+//
+// izb_one_wave: does a grid of such blocks fit the current device at once (2048 threads per SM)?  Short blocks of many waves are faster without
+// any of this: each of them pays for the two instructions, and only the last wave has anything to gain.
+bool izb_one_wave(dim3 grid, int threads);
 #ifdef __CUDACC__
 template <class... P, class... A>
 static inline cudaError_t izb_launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {

@@ -35,3 +35,24 @@ def test_rmsnorm_quant(izb, M, K):
     aq, asc, h = izb.rmsnorm_quant(torch.from_numpy(x).cuda(), torch.from_numpy(w).cuda(), 1e-6, want_h=True)
     ry, raq, rasc, _ = O.rmsnorm_quant(x, w, 1e-6, Mp=asc.shape[1])
     assert (bits(h.cpu().numpy()) == bits(ry)).all() and (aq.cpu().numpy() == raq).all() and (bits(asc.cpu().numpy()) == bits(rasc)).all()
+
+
+# (a wave holds 148 x 8 blocks of 1024 logits, 148 x 16 blocks of 512 combined values)
+@pytest.mark.parametrize("rows,N", [(1184, 1024), (1185, 1024), (600, 4100)])
+def test_softcap_of_one_wave_and_more(izb, rows, N):
+    import torch
+    x = torch.randn(rows, N, generator=torch.Generator().manual_seed(N)) * 40
+    got = izb.softcap_rows(x.cuda(), rows, N, 30.0).cpu().double()
+    want = 30.0 * torch.tanh(x.double() / 30.0)
+    # (x / cap, tanhf and the product: a few units in the last place of values up to 30)
+    assert float((got - want).abs().max()) < 8 * 30 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("T,E", [(148, 8192), (149, 8192), (600, 8196)])
+def test_combine_of_one_wave_and_more(izb, T, E):
+    import torch
+    rng = np.random.default_rng(T)
+    x, y = rng.standard_normal((T, E), dtype=np.float32), rng.standard_normal((2 * T, E), dtype=np.float32)
+    inv = rng.permutation(2 * T).astype(np.int32)
+    out = izb.moe_combine(*(torch.from_numpy(a).cuda() for a in (x, y, inv)), 2)
+    assert (bits(out.cpu().numpy()) == bits(O.moe_combine(x, y, inv, 2))).all()
