@@ -1143,13 +1143,14 @@ int tc_grid(int device, int n_work) {
 }
 
 // Parts the K range of every output tile is cut into, when the tiles alone would leave more than half the SMs idle: as many as fill
-// them once, each at least two superblocks.  The parts' sums are at most one 64 KB tile per SM.  Long K and plain stores only.  Short K:
-// a part's pipeline fill and the summing launch eat the gain (K = 1024: some 10 us uncut).  Other store modes: sums cut in parts are
-// rounded in other places, and what those modes write (the residual, the SwiGLU product) is quantised to int8 next, where a last bit
-// can become a whole step.
+// them once, each at least two superblocks.  The parts' sums are at most one 64 KB tile per SM.  The device's SMs count, not the part of them
+// that izb_set_sm_limit leaves: that call caps the grid and changes no result.  Long K and plain stores only.  Short K: a part's pipeline fill
+// and the summing launch eat the gain (K = 1024: some 10 us uncut).  Other store modes: sums cut in parts are rounded in other places, and what
+// those modes write (the residual, the SwiGLU product) is mostly quantised to int8 next, where a last bit can become a whole step.  (A plain
+// store may be quantised next as well; there the cut was taken for its speed.)
 int tc_split(int device, int n_items, int nsb) {
   if (nsb < 8) return 1;
-  const int s = izb_sm_budget(device) / (n_items > 0 ? n_items : 1);
+  const int s = izb_sm_count(device) / (n_items > 0 ? n_items : 1);
   return s < 2 ? 1 : s < nsb / 2 ? s : nsb / 2;
 }
 constexpr size_t kSplitBytes = (size_t)BM * BN * 4;  // per SM; the flag of a failed part follows them

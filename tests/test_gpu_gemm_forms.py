@@ -79,3 +79,22 @@ def test_short_calls_take_the_faster_kernel(izb, qt, M, N, K, acc, core):
         assert torch.equal(out, want) if core else float((out - want).abs().max() / want.abs().max()) < 1e-5
     assert torch.equal(a, b)
     W.close()
+
+
+@pytest.mark.parametrize("qt", [12, 8, 14])
+def test_sm_limit_changes_no_result(izb, qt):
+    """The limit caps the grid of the GEMM; how a long K is cut into parts, and with it where sums are rounded, does not follow it."""
+    import torch
+    M, N, K = 40, 256, 4096
+    W = izb.Weight(qt, S.make_weight(qt, N, K, 5), N, K)
+    aq, asc, _ = izb.quantize_act(torch.from_numpy(S.make_act(M, K, 6)).cuda())
+    want = izb.gemm(W, aq, asc)
+    assert "split_reduce" in kernels_of(izb, lambda: izb.gemm(W, aq, asc))
+    try:
+        for sms in (100, 20, 3, 1):
+            izb.set_sm_limit(0, sms)
+            assert torch.equal(izb.gemm(W, aq, asc), want), sms
+    finally:
+        izb.set_sm_limit(0, 0)
+    assert izb.device_status(0) == 0
+    W.close()
