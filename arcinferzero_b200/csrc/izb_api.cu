@@ -16,7 +16,7 @@ int izb_gemm_core_launch(const izb_weight* w, const uint8_t* raw, const int8_t* 
                          int ldc, int c_off, int acc, int32_t* dots, cudaStream_t st);
 // returns IZB_OK, an error, or +1 when the tensor-core kernel does not take this shape
 int izb_gemm_tc_launch(const izb_weight* w, int mat, const int8_t* aq, const float* asc, int M, int Mp, float* C, int ldc,
-                       int c_off, int acc, int32_t* dots, cudaStream_t st);
+                       int c_off, int acc, int32_t* dots, cudaStream_t st, bool may_cut);
 int izb_make_raw_tensor_map(izb_weight* w);
 int izb_make_rows_tensor_map(izb_weight* w);
 int izb_gemm_k16_launch(const izb_weight* w, const uint8_t* raw, const int8_t* aq, const float* asc, int M, int Mp, float* C, int ldc,
@@ -590,7 +590,7 @@ extern "C" int izb_gemm(const izb_weight* w, int mat, const int8_t* d_aq, const 
     if (impl != IZB_GEMM_AUTO && impl != IZB_GEMM_CORE) IZB_FAIL(IZB_ERR_ARG, "gemm: impl %d", impl);
     if (acc == 3) IZB_FAIL(IZB_ERR_TYPE, "gemm: store mode 3 is not built for ggml type %d", w->ggml_type);
     if (impl == IZB_GEMM_AUTO && g_dev[w->device].tc_ok.load() != 0 && !gemm_core_first(w, M, acc)) {
-      const int rc = izb_gemm_tc_launch(w, mat, d_aq, d_asc, M, Mp, d_C, ldc, c_off, acc, nullptr, st);
+      const int rc = izb_gemm_tc_launch(w, mat, d_aq, d_asc, M, Mp, d_C, ldc, c_off, acc, nullptr, st, true);
       if (rc <= 0) return rc;
     }
     return izb_gemm_k16_launch(w, w->raw + (size_t)mat * w->N * w->row_bytes, d_aq, d_asc, M, Mp, d_C, ldc, c_off, acc, nullptr, st);
@@ -598,7 +598,7 @@ extern "C" int izb_gemm(const izb_weight* w, int mat, const int8_t* d_aq, const 
   if (impl == IZB_GEMM_AUTO || impl == IZB_GEMM_TC) {
     const bool allowed = impl == IZB_GEMM_TC || (g_dev[w->device].tc_ok.load() != 0 && !gemm_core_first(w, M, acc));
     if (allowed) {
-      const int rc = izb_gemm_tc_launch(w, mat, d_aq, d_asc, M, Mp, d_C, ldc, c_off, acc, nullptr, st);
+      const int rc = izb_gemm_tc_launch(w, mat, d_aq, d_asc, M, Mp, d_C, ldc, c_off, acc, nullptr, st, impl == IZB_GEMM_AUTO);
       if (rc <= 0) return rc;
     }
     if (impl == IZB_GEMM_TC) IZB_FAIL(IZB_ERR_SHAPE, "gemm: the tensor-core kernel does not take M=%d Mp=%d N=%d K=%d", M, Mp, w->N, w->K);
@@ -626,7 +626,7 @@ extern "C" int izb_block_dots(const izb_weight* w, int mat, const int8_t* d_aq, 
     return izb_gemm_k16_launch(w, w->raw + (size_t)mat * w->N * w->row_bytes, d_aq, nullptr, M, M, nullptr, 0, 0, 0, d_dots, st);
   }
   if (impl == IZB_GEMM_TC) {
-    const int rc = izb_gemm_tc_launch(w, mat, d_aq, nullptr, M, M, nullptr, 0, 0, 0, d_dots, st);
+    const int rc = izb_gemm_tc_launch(w, mat, d_aq, nullptr, M, M, nullptr, 0, 0, 0, d_dots, st, false);
     if (rc > 0) IZB_FAIL(IZB_ERR_SHAPE, "block_dots: the tensor-core kernel does not take M=%d N=%d K=%d", M, w->N, w->K);
     return rc;
   }

@@ -1211,13 +1211,13 @@ int run_tc_on(const izb_weight* w, int mat, const int8_t* aq, const float* asc, 
 // the activation pre-pass + the GEMM for one tile set
 int run_tc(const izb_weight* w, int mat, const int8_t* aq, const float* asc, int lda, int rows_total, const int32_t* tiles,
            int n_tiles_grid, const int32_t* rowmap, const float* rowscale, int M_store, float* C, int ldc, int c_off, int acc,
-           int32_t* dots, int ws_slot, cudaStream_t st, bool reuse_images = false) {
+           int32_t* dots, int ws_slot, cudaStream_t st, bool reuse_images = false, bool may_cut = true) {
   // reuse_images: the call before this one, on the same stream and arena, prepared the same activation rows for a weight
   // of the same type and K (the up projection after the gate projection): its operand images are still there
   if (!tc_takes(w)) return 1;
   size_t img_bytes, asc_bytes;
   tc_scratch_bytes(n_tiles_grid, w->K, tc_sps(w, dots != nullptr), &img_bytes, &asc_bytes);
-  const size_t split_bytes = tiles || dots ? 0 : split_area(w->device);
+  const size_t split_bytes = tiles || dots || !may_cut ? 0 : split_area(w->device);
   void* ws = nullptr;
   if (int rc = izb_workspace(w->device, ws_slot, img_bytes + asc_bytes + split_bytes, st, &ws, !tiles && !dots && tc_optional(w))) return rc;
   uint32_t* err = izb_device_error_word(w->device);
@@ -1263,11 +1263,12 @@ int izb_make_raw_tensor_map(izb_weight* w) { return make_map(w, w->sb_bytes, BN,
 // chunks of the few-row kernel: a superblock; Q6_K 16 bytes more, for a row pitch its shared-memory reads want
 int izb_make_rows_tensor_map(izb_weight* w) { return make_map(w, w->packed6 ? w->sb_bytes + 16 : w->sb_bytes, 16, w->tmap16_raw); }
 
+// may_cut: the K range may be cut into parts (IZB_GEMM_AUTO); IZB_GEMM_TC names this kernel, and gives the sums of izb_gemm_noalloc
 int izb_gemm_tc_launch(const izb_weight* w, int mat, const int8_t* aq, const float* asc, int M, int Mp, float* C, int ldc, int c_off,
-                       int acc, int32_t* dots, cudaStream_t st) {
+                       int acc, int32_t* dots, cudaStream_t st, bool may_cut) {
   const int n_tiles = (M + BM - 1) / BM;
   if (n_tiles > 65535) return 1;
-  return run_tc(w, mat, aq, asc, Mp, Mp, nullptr, n_tiles, nullptr, nullptr, M, C, ldc, c_off, acc, dots, kWsGemm, st);
+  return run_tc(w, mat, aq, asc, Mp, Mp, nullptr, n_tiles, nullptr, nullptr, M, C, ldc, c_off, acc, dots, kWsGemm, st, false, may_cut);
 }
 
 // quantise + multiply in one call (dense): the fused pre-pass over the M valid rows (rows up to Mp zeroed), then the GEMM on
@@ -1399,7 +1400,7 @@ extern "C" int izb_selfcheck(int device) {
     w.has_tmap = true;
     unsigned int h[3];
     // dots
-    int rc = izb_gemm_tc_launch(&w, 0, aq, nullptr, M, M, nullptr, 0, 0, 0, d_tc, 0);
+    int rc = izb_gemm_tc_launch(&w, 0, aq, nullptr, M, M, nullptr, 0, 0, 0, d_tc, 0, false);
     if (rc == 0) rc = izb_gemm_core_launch(&w, w.raw, aq, nullptr, M, M, nullptr, 0, 0, 0, d_core, 0);
     if (rc != 0) { izb_set_tc_ok(device, 0); return rc < 0 ? rc : IZB_ERR_SELFCHECK; }
     IZB_CUDA(cudaMemset(cmp, 0, 12));
@@ -1409,7 +1410,7 @@ extern "C" int izb_selfcheck(int device) {
     for (int acc = 0; acc < 3 && verdict == IZB_OK; ++acc) {
       fill_scales<<<(unsigned)((n_out + 255) / 256), 256>>>(c_tc, n_out, 3u);
       fill_scales<<<(unsigned)((n_out + 255) / 256), 256>>>(c_core, n_out, 3u);
-      rc = izb_gemm_tc_launch(&w, 0, aq, asc, M, Mp, c_tc, N, 0, acc, nullptr, 0);
+      rc = izb_gemm_tc_launch(&w, 0, aq, asc, M, Mp, c_tc, N, 0, acc, nullptr, 0, true);
       if (rc == 0) rc = izb_gemm_core_launch(&w, w.raw, aq, asc, M, Mp, c_core, N, 0, acc, nullptr, 0);
       if (rc != 0) { izb_set_tc_ok(device, 0); return rc < 0 ? rc : IZB_ERR_SELFCHECK; }
       IZB_CUDA(cudaMemset(cmp, 0, 12));

@@ -62,7 +62,10 @@ extern "C" {
 #define IZB_IQ4_XS 23
 
 /* izb_gemm `impl` */
-#define IZB_GEMM_AUTO 0 /* tensor-core kernel when the shape allows it, else the CUDA-core kernel */
+/* IZB_GEMM_AUTO, and with it izb_matmul and izb_quant_matmul, may cut a long K (2048 and more) of a plain store into parts when there are few
+ * 128 x 128 output tiles, and add the parts' sums afterwards: such sums are rounded in other places, so that a row's last bits may depend on
+ * the number of rows in the call.  Store modes 1, 2 and 3, IZB_GEMM_TC and izb_gemm_noalloc never cut: a row's sums are the same in every call. */
+#define IZB_GEMM_AUTO 0 /* the tensor-core or the CUDA-core kernel, by type and shape */
 #define IZB_GEMM_CORE 1 /* CUDA-core dp4a kernel, f32 combine in the reference's order (zero/kernels/gemm.cl:441-487) */
 #define IZB_GEMM_TC 2   /* tcgen05 kernel (TMEM accumulators), error if the shape is not taken */
 
@@ -139,7 +142,8 @@ int izb_weight_create_stack(int ggml_type, const void* const* h_parts, const int
  * and wu = NULL) one GEMM computes both projections and stores up * silu(gate) [rows][F]: the reference fuses the same
  * product into its up GEMM, which reads the gate GEMM's output back (store mode 2, zero/kernels/gemm.cl:562-565; the
  * `fused` flag of swiglu_quant, zero/kernels/ops.cl:277); here a thread of the GEMM's epilogue holds a gate column and its
- * up column side by side, so the gate projection never goes to memory.  Same operations, same roundings as mode 2. */
+ * up column side by side, so the gate projection never goes to memory.  Same operations, same roundings as mode 2 on a gate
+ * projection whose K was not cut (see IZB_GEMM_AUTO). */
 int izb_weight_create_gateup(int ggml_type, const void* h_gate_rows, const void* h_up_rows, int n_mats, int F, int K, int device,
                              izb_weight** out);
 /* The row order izb_weight_create_gateup uploads, on the host alone (no device needed): h_dst receives n_mats matrices of
@@ -229,7 +233,7 @@ int izb_selfcheck(int device);
  * that it grows with cudaMalloc when a call is larger than any before; this call keeps them in a fixed array of
  * IZB_NOALLOC_SCRATCH_BYTES that lives in the library's device image: every GPU that loads the library holds those
  * bytes until the process exits, and the call itself calls no cudaMalloc, cudaFree or other allocating routine.
- *   - Same arguments and results as izb_gemm with impl = IZB_GEMM_TC (N % 128 == 0 is required here: there is no second
+ *   - Same arguments and results, bit for bit, as izb_gemm with impl = IZB_GEMM_TC (N % 128 == 0 is required here: there is no second
  *     kernel to fall back to), plus d_status.
  *   - Limit: ceil(M/128) * (K/256 * S * 16384 + K/32 * 512) bytes, S = 5 for Q4_K and 4 for Q8_0, must fit in the array (e.g. M = 1024 at K = 5120, or
  *     M = 512 at K = 10240); a larger call returns IZB_ERR_LIMIT and launches nothing.

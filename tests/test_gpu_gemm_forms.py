@@ -98,3 +98,23 @@ def test_sm_limit_changes_no_result(izb, qt):
         izb.set_sm_limit(0, 0)
     assert izb.device_status(0) == 0
     W.close()
+
+
+@pytest.mark.parametrize("qt", [12, 8])
+def test_named_kernel_is_not_cut(izb, qt):
+    """Where IZB_GEMM_AUTO cuts K, IZB_GEMM_TC gives the sums of izb_gemm_noalloc, a row's sums do not depend on the rows beside it, and a
+    gate projection followed by store mode 2 is store mode 3."""
+    import torch
+    M, N, K = 40, 256, 4096
+    g, u = S.make_weight(qt, N, K, 5), S.make_weight(qt, N, K, 6)
+    Wg, Wu, Wgu = izb.Weight(qt, g, N, K), izb.Weight(qt, u, N, K), izb.gateup_weight(qt, g, u, N, K)
+    aq, asc, _ = izb.quantize_act(torch.from_numpy(S.make_act(M, K, 7)).cuda() * 0.02)
+    assert "split_reduce" in kernels_of(izb, lambda: izb.gemm(Wg, aq, asc))
+    named = izb.gemm(Wg, aq, asc, M=M, impl=izb.GEMM_TC)
+    assert torch.equal(izb.gemm_noalloc(Wg, aq, asc, M=M, out=torch.zeros_like(named))[:M], named[:M])
+    many = izb.gemm(Wg, aq.repeat(8, 1), asc.repeat(1, 8), impl=izb.GEMM_TC)
+    assert torch.equal(many[:M], named[:M])
+    assert torch.equal(izb.gemm(Wu, aq, asc, M=M, out=named, acc=2)[:M], izb.gemm(Wgu, aq, asc, M=M, acc=3)[:M])
+    assert izb.device_status(0) == 0
+    for W in (Wg, Wu, Wgu):
+        W.close()
