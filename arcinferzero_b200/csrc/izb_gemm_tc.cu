@@ -36,7 +36,9 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <exception>
 #include <mutex>
+#include <vector>
 
 #include "izb_common.cuh"
 
@@ -1317,32 +1319,18 @@ int izb_moe_down_tc(const izb_weight* wd, const int8_t* d_hq, const float* d_hsc
 }
 
 // ---------------------------------------------------------------------------------------------- start-up check
-// Seeded data, both weight types, all store modes: tensor-core dots == CUDA-core dots bit for bit, outputs within 1e-5
-// of max|ref| (Engine::xmx_check, zero/engine_setup.h:424-622, does the same for its XMX kernel against DP4a).
+// Seeded data, every weight form, all store modes, a part of a column tile, and the plain store with K cut into parts and not:
+// tensor-core dots == CUDA-core dots bit for bit (Q4_K, Q8_0: the forms that have this mode), outputs within 1e-5 of max|ref|
+// (Engine::xmx_check, zero/engine_setup.h:424-622, does the same for its XMX kernel against DP4a).
+int izb_gemm_k16_launch(const izb_weight* w, const uint8_t* raw, const int8_t* aq, const float* asc, int M, int Mp, float* C, int ldc,
+                        int c_off, int acc, int32_t* dots, cudaStream_t st);
 namespace {
-__global__ void fill_kernel(uint8_t* p, size_t n, uint32_t seed, int mode) {
+__global__ void fill_quants(int8_t* p, size_t n, uint32_t seed) {
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   uint32_t x = (uint32_t)i * 2654435761u + seed;
   x ^= x >> 15; x *= 2246822519u; x ^= x >> 13; x *= 3266489917u; x ^= x >> 16;
-  p[i] = mode == 0 ? (uint8_t)x : (uint8_t)(int8_t)((int)(x % 255u) - 127);
-}
-__global__ void fix_q4k_headers(uint8_t* w, size_t n_sb, uint32_t seed) {
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_sb) return;
-  uint32_t x = (uint32_t)i * 747796405u + seed;
-  x ^= x >> 16; x *= 2246822519u; x ^= x >> 13;
-  const __half d = __float2half(0.0001f + (float)(x & 0xFFFF) * (0.0099f / 65535.0f));
-  const __half m = __float2half(0.0001f + (float)(x >> 16) * (0.0099f / 65535.0f));
-  *reinterpret_cast<__half*>(w + i * 144) = d;
-  *reinterpret_cast<__half*>(w + i * 144 + 2) = m;
-}
-__global__ void fix_q8_headers(uint8_t* w, size_t n_sb, uint32_t seed) {
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_sb * 8) return;
-  uint32_t x = (uint32_t)i * 747796405u + seed;
-  x ^= x >> 16; x *= 2246822519u; x ^= x >> 13;
-  *reinterpret_cast<__half*>(w + (i / 8) * 272 + 2 * (i % 8)) = __float2half(0.001f + (float)(x & 0xFFFF) * (0.019f / 65535.0f));
+  p[i] = (int8_t)((int)(x % 255u) - 127);
 }
 __global__ void fill_scales(float* p, size_t n, uint32_t seed) {
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1364,67 +1352,102 @@ __global__ void compare_kernel(const float* a, const float* b, size_t n, int as_
     atomicMax(&out[2], __float_as_uint(fabsf(b[i])));
   }
 }
+// file rows: random bytes, the fp16 factors of each superblock (Q8_0: block) between 0.0002 and 0.005
+std::vector<uint8_t> seeded_rows(int type, size_t n_sb) {
+  const size_t sb = type == IZB_Q4_K ? 144 : type == IZB_Q5_K ? 176 : type == IZB_Q6_K ? 210 : type == IZB_IQ4_XS ? 136 : 272;
+  std::vector<uint8_t> rows(n_sb * sb);
+  uint32_t x = 17u + (uint32_t)type;
+  auto next = [&]() { x = x * 1664525u + 1013904223u; return x >> 16; };
+  for (uint8_t& v : rows) v = (uint8_t)next();
+  auto factor = [&](size_t at) {
+    const unsigned short h = __half_as_ushort(__float2half(0.0002f + (float)next() * (0.0048f / 65535.0f)));
+    rows[at] = (uint8_t)h;
+    rows[at + 1] = (uint8_t)(h >> 8);
+  };
+  for (size_t i = 0; i < n_sb; ++i) {
+    if (type == IZB_Q8_0) {
+      for (int b = 0; b < 8; ++b) factor(i * sb + 34 * b);
+    } else {
+      factor(i * sb + (type == IZB_Q6_K ? 208 : 0));
+      if (type == IZB_Q4_K || type == IZB_Q5_K) factor(i * sb + 2);
+    }
+  }
+  return rows;
+}
+struct WeightHolder {
+  izb_weight* w = nullptr;
+  ~WeightHolder() { if (w) izb_weight_destroy(w); }
+};
+
+// one weight form; IZB_ERR_SELFCHECK: the kernels disagree, other errors: the check could not run
+int check_form(int device, int type) {
+  constexpr int M = 200, Mp = 256, N = 272, K = 2048, nb = K / 32;
+  WeightHolder h;
+  try {
+    const std::vector<uint8_t> rows = seeded_rows(type, (size_t)N * (K / 256));
+    if (int rc = izb_weight_create(type, rows.data(), 1, N, K, device, &h.w)) return rc;
+  } catch (const std::exception&) {
+    IZB_FAIL(IZB_ERR_NOMEM, "selfcheck: host memory for the seeded rows");
+  }
+  const izb_weight* w = h.w;
+  if (!w->has_tmap) IZB_FAIL(IZB_ERR_SELFCHECK, "selfcheck: cannot encode a tensor map");
+  const bool k16 = w->type == IZB_K16;
+  auto core = [&](const int8_t* aq, const float* asc, int mp, float* C, int acc, int32_t* dots) {
+    return k16 ? izb_gemm_k16_launch(w, w->raw, aq, asc, M, mp, C, N, 0, acc, dots, 0) : izb_gemm_core_launch(w, w->raw, aq, asc, M, mp, C, N, 0, acc, dots, 0);
+  };
+  const size_t n_out = (size_t)Mp * N, n_dots = (size_t)M * N * nb;
+  void* ws = nullptr;
+  if (int rc = izb_workspace(device, kWsCheck, (size_t)Mp * K + (size_t)nb * Mp * 4 + 2 * n_out * 4 + 2 * n_dots * 4 + 4096, 0, &ws)) return rc;
+  int8_t* aq = (int8_t*)ws;
+  float* asc = (float*)(aq + (size_t)Mp * K);
+  float *c_tc = asc + (size_t)nb * Mp, *c_core = c_tc + n_out;
+  int32_t *d_tc = (int32_t*)(c_core + n_out), *d_core = d_tc + n_dots;
+  unsigned int* cmp = (unsigned int*)(d_core + n_dots);
+  unsigned int out[3];
+  auto blocks = [](size_t n) { return (unsigned)((n + 255) / 256); };
+  fill_quants<<<blocks((size_t)Mp * K), 256>>>(aq, (size_t)Mp * K, 99u);
+  fill_scales<<<blocks((size_t)nb * Mp), 256>>>(asc, (size_t)nb * Mp, 7u);
+  IZB_CUDA(cudaGetLastError());
+  if (!k16) {
+    int rc = izb_gemm_tc_launch(w, 0, aq, nullptr, M, M, nullptr, 0, 0, 0, d_tc, 0, false);
+    if (rc == 0) rc = core(aq, nullptr, M, nullptr, 0, d_core);
+    if (rc != 0) return rc < 0 ? rc : IZB_ERR_SELFCHECK;
+    IZB_CUDA(cudaMemset(cmp, 0, 12));
+    compare_kernel<<<blocks(n_dots), 256>>>((const float*)d_tc, (const float*)d_core, n_dots, 1, cmp);
+    IZB_CUDA(cudaMemcpy(out, cmp, 12, cudaMemcpyDeviceToHost));
+    if (out[0]) IZB_FAIL(IZB_ERR_SELFCHECK, "selfcheck: type %d: %u block dots differ between the tensor-core and CUDA-core kernels", type, out[0]);
+  }
+  for (int mode = 0; mode < 4; ++mode) {  // 3: the plain store again, K not cut
+    const int acc = mode % 3;
+    fill_scales<<<blocks(n_out), 256>>>(c_tc, n_out, 3u);
+    fill_scales<<<blocks(n_out), 256>>>(c_core, n_out, 3u);
+    int rc = izb_gemm_tc_launch(w, 0, aq, asc, M, Mp, c_tc, N, 0, acc, nullptr, 0, mode < 3);
+    if (rc == 0) rc = core(aq, asc, Mp, c_core, acc, nullptr);
+    if (rc != 0) return rc < 0 ? rc : IZB_ERR_SELFCHECK;
+    IZB_CUDA(cudaMemset(cmp, 0, 12));
+    compare_kernel<<<blocks(n_out), 256>>>(c_tc, c_core, n_out, 0, cmp);
+    IZB_CUDA(cudaMemcpy(out, cmp, 12, cudaMemcpyDeviceToHost));
+    float err, ref;
+    memcpy(&err, &out[1], 4);
+    memcpy(&ref, &out[2], 4);
+    if (out[0] || !(err <= 1e-5f * ref))
+      IZB_FAIL(IZB_ERR_SELFCHECK, "selfcheck: type %d store mode %d%s: max|err| %g vs max|ref| %g (%u NaN)", type, acc, mode == 0 ? ", K cut" : "", err, ref, out[0]);
+  }
+  return IZB_OK;
+}
 }  // namespace
 
 extern "C" int izb_selfcheck(int device) {
   if (izb_get_tc_ok(device) == 1) return IZB_OK;
   IZB_CUDA(cudaSetDevice(device));
-  const int M = 200, Mp = 256, N = 256, K = 1024, nb = K / 32;
   int verdict = IZB_OK;
-  for (int type : {IZB_Q4_K, IZB_Q8_0}) {
-    izb_weight w;
-    w.type = type; w.n_mats = 1; w.N = N; w.K = K; w.device = device;
-    w.sb_bytes = type == IZB_Q4_K ? 144 : 272;
-    w.row_bytes = (size_t)(K / 256) * w.sb_bytes;
-    w.bytes = (size_t)N * w.row_bytes;
-    const size_t n_out = (size_t)Mp * N, n_dots = (size_t)M * N * nb;
-    void* ws = nullptr;
-    const size_t need = w.bytes + kRawSlack + (size_t)Mp * K + (size_t)nb * Mp * 4 + 2 * n_out * 4 + 2 * n_dots * 4 + 4096;
-    if (int rc = izb_workspace(device, kWsCheck, need, 0, &ws)) return rc;
-    uint8_t* base = (uint8_t*)ws;
-    w.raw = base; base += (w.bytes + kRawSlack + 255) & ~size_t(255);
-    int8_t* aq = (int8_t*)base; base += (size_t)Mp * K;
-    float* asc = (float*)base; base += (size_t)nb * Mp * 4;
-    float* c_tc = (float*)base; base += n_out * 4;
-    float* c_core = (float*)base; base += n_out * 4;
-    int32_t* d_tc = (int32_t*)base; base += n_dots * 4;
-    int32_t* d_core = (int32_t*)base; base += n_dots * 4;
-    unsigned int* cmp = (unsigned int*)base;
-    fill_kernel<<<(unsigned)((w.bytes + 255) / 256), 256>>>(w.raw, w.bytes, 17u + type, type == IZB_Q4_K ? 0 : 1);
-    if (type == IZB_Q4_K) fix_q4k_headers<<<(unsigned)((w.bytes / 144 + 255) / 256), 256>>>(w.raw, w.bytes / 144, 5u);
-    else fix_q8_headers<<<(unsigned)((w.bytes / 272 * 8 + 255) / 256), 256>>>(w.raw, w.bytes / 272, 5u);
-    fill_kernel<<<(unsigned)(((size_t)Mp * K + 255) / 256), 256>>>((uint8_t*)aq, (size_t)Mp * K, 99u, 1);
-    fill_scales<<<(unsigned)(((size_t)nb * Mp + 255) / 256), 256>>>(asc, (size_t)nb * Mp, 7u);
-    IZB_CUDA(cudaGetLastError());
-    if (izb_make_raw_tensor_map(&w) != IZB_OK) { izb_set_tc_ok(device, 0); IZB_FAIL(IZB_ERR_SELFCHECK, "selfcheck: cannot encode a tensor map"); }
-    w.has_tmap = true;
-    unsigned int h[3];
-    // dots
-    int rc = izb_gemm_tc_launch(&w, 0, aq, nullptr, M, M, nullptr, 0, 0, 0, d_tc, 0, false);
-    if (rc == 0) rc = izb_gemm_core_launch(&w, w.raw, aq, nullptr, M, M, nullptr, 0, 0, 0, d_core, 0);
-    if (rc != 0) { izb_set_tc_ok(device, 0); return rc < 0 ? rc : IZB_ERR_SELFCHECK; }
-    IZB_CUDA(cudaMemset(cmp, 0, 12));
-    compare_kernel<<<(unsigned)((n_dots + 255) / 256), 256>>>((const float*)d_tc, (const float*)d_core, n_dots, 1, cmp);
-    IZB_CUDA(cudaMemcpy(h, cmp, 12, cudaMemcpyDeviceToHost));
-    if (h[0]) { verdict = IZB_ERR_SELFCHECK; izb_set_error("selfcheck: type %d: %u block dots differ between the tensor-core and CUDA-core kernels", type, h[0]); break; }
-    for (int acc = 0; acc < 3 && verdict == IZB_OK; ++acc) {
-      fill_scales<<<(unsigned)((n_out + 255) / 256), 256>>>(c_tc, n_out, 3u);
-      fill_scales<<<(unsigned)((n_out + 255) / 256), 256>>>(c_core, n_out, 3u);
-      rc = izb_gemm_tc_launch(&w, 0, aq, asc, M, Mp, c_tc, N, 0, acc, nullptr, 0, true);
-      if (rc == 0) rc = izb_gemm_core_launch(&w, w.raw, aq, asc, M, Mp, c_core, N, 0, acc, nullptr, 0);
-      if (rc != 0) { izb_set_tc_ok(device, 0); return rc < 0 ? rc : IZB_ERR_SELFCHECK; }
-      IZB_CUDA(cudaMemset(cmp, 0, 12));
-      compare_kernel<<<(unsigned)((n_out + 255) / 256), 256>>>(c_tc, c_core, n_out, 0, cmp);
-      IZB_CUDA(cudaMemcpy(h, cmp, 12, cudaMemcpyDeviceToHost));
-      float err, ref;
-      memcpy(&err, &h[1], 4);
-      memcpy(&ref, &h[2], 4);
-      if (h[0] || !(err <= 1e-5f * ref)) {
-        verdict = IZB_ERR_SELFCHECK;
-        izb_set_error("selfcheck: type %d store mode %d: max|err| %g vs max|ref| %g (%u NaN)", type, acc, err, ref, h[0]);
-      }
-    }
+  for (int type : {IZB_Q4_K, IZB_Q8_0, IZB_Q5_K, IZB_Q6_K, IZB_IQ4_XS}) {
+    verdict = check_form(device, type);
     if (verdict != IZB_OK) break;
+  }
+  if (verdict != IZB_OK && verdict != IZB_ERR_SELFCHECK) {
+    izb_set_tc_ok(device, 0);
+    return verdict;
   }
   uint32_t word = 0;
   const int st = izb_device_status(device, &word);

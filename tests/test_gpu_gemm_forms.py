@@ -118,3 +118,24 @@ def test_named_kernel_is_not_cut(izb, qt):
     assert izb.device_status(0) == 0
     for W in (Wg, Wu, Wgu):
         W.close()
+
+
+def test_selfcheck_runs_every_form():
+    """The start-up check switches the tensor-core kernel for all weight forms, part columns and cut K: it must run them all.  (In a process
+    of its own: the verdict is kept.)"""
+    import os
+    import subprocess
+    import sys
+    body = """
+import torch, arcinferzero_b200 as izb
+izb.profile_start()
+izb.selfcheck(0)
+ran = izb.profile_stop()
+# five forms x (plain cut, adding, SwiGLU, plain uncut), two with block dots
+assert ran["gemm_tc"]["launches"] == 22 and ran["split_reduce"]["launches"] == 5, ran
+assert sum(ran[k]["launches"] for k in ran if k.startswith("gemm_k16")) == 12, ran
+assert izb.device_status(0) == 0
+print("done")
+"""
+    r = subprocess.run([sys.executable, "-c", body], cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))), capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "done" in r.stdout, r.stdout + r.stderr
