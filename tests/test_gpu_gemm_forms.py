@@ -1,5 +1,6 @@
 """The tcgen05 GEMM on every weight form it takes (one and two fp16 terms per weight, with and without mins), on columns that do
-not fill its tiles and on calls whose K range is cut into parts, against the CUDA-core kernel (itself checked against the oracle)."""
+not fill its tiles and on calls whose K range is cut into parts, against the CUDA-core kernel (itself checked against the oracle); which
+calls take it, and which of them are cut."""
 import numpy as np
 import pytest
 
@@ -33,28 +34,67 @@ def extremes(qt, rows):
     return v.reshape(rows.shape)
 
 
-# (16, 16): the smallest call; 144, 272: a part of the last column tile; 40 x 128 x 4096 and 130 x 144 x 2304: K cut into parts;
+# (16, 16): the smallest calls; 144, 272: a part of the last column tile; 40 x 128 x 4096 and 130 x 144 x 2304: K cut into parts;
 # 300 x 2432 x 512: more tiles than half the SMs, not cut
 @pytest.mark.parametrize("qt", [12, 8, 2, 13, 14, 23])
-@pytest.mark.parametrize("M,N,K", [(16, 16, 256), (130, 144, 2304), (40, 128, 4096), (129, 272, 768), (300, 2432, 512)])
+@pytest.mark.parametrize("M,N,K", [(16, 16, 256), (16, 16, 1280), (130, 144, 2304), (40, 128, 4096), (129, 272, 768), (300, 2432, 512)])
 def test_tensor_core_gemm_equals_core_gemm(izb, qt, M, N, K):
+    """Which kernel ran is looked at: IZB_GEMM_AUTO may take the other one, and would then be compared with itself."""
     import torch
     W = izb.Weight(qt, extremes(qt, S.make_weight(qt, N, K, N + K + qt)), N, K)
     Mp = izb.pad_rows(M)
     x = torch.from_numpy(S.make_act(M, K, M + K)).cuda()
     x[0] = 1.0  # every int8 = 127
     aq, asc, _ = izb.quantize_act(x, Mp=Mp)
+    impls = [izb.GEMM_AUTO, izb.GEMM_TC] if qt in (12, 8, 2) else [izb.GEMM_AUTO]  # (the per-16-scale types cannot name the kernel)
     for acc in (0, 1, 2):
         base = torch.from_numpy(np.random.default_rng(acc).standard_normal((Mp, N + 8)).astype(np.float32)).cuda()
-        a, b = base.clone(), base.clone()
-        izb.gemm(W, aq, asc, M=M, out=a, c_off=4, acc=acc)
+        b = base.clone()
         izb.gemm(W, aq, asc, M=M, out=b, c_off=4, acc=acc, impl=izb.GEMM_CORE)
-        ra, rb = a[:M, 4:N + 4].double(), b[:M, 4:N + 4].double()
-        assert float((ra - rb).abs().max() / rb.abs().max()) < 1e-5, acc
-        assert torch.equal(a[:, :4], base[:, :4]) and torch.equal(a[:, N + 4:], base[:, N + 4:]) and torch.equal(a[M:], base[M:])
-    got, _, _ = izb.quant_matmul(W, x, M)
+        for impl in impls:
+            a = base.clone()
+            ran = kernels_of(izb, lambda: izb.gemm(W, aq, asc, M=M, out=a, c_off=4, acc=acc, impl=impl))
+            short = impl == izb.GEMM_AUTO and (qt not in (12, 8, 2) or N % 128 != 0) and K <= 512 << acc  # (may go to the CUDA cores, below)
+            assert "gemm_tc" in ran or short, (acc, impl, ran)
+            assert ("split_reduce" in ran) == (impl == izb.GEMM_AUTO and acc == 0 and K >= 2048), (acc, impl, ran)
+            ra, rb = a[:M, 4:N + 4].double(), b[:M, 4:N + 4].double()
+            assert float((ra - rb).abs().max() / rb.abs().max()) < 1e-5, (acc, impl)
+            assert torch.equal(a[:, :4], base[:, :4]) and torch.equal(a[:, N + 4:], base[:, N + 4:]) and torch.equal(a[M:], base[M:])
     want = izb.gemm(W, aq, asc)
-    assert torch.equal(got[:M], want[:M])
+    got = []
+    ran = kernels_of(izb, lambda: got.append(izb.quant_matmul(W, x, M)[0]))
+    assert "quant_prepare" in ran or K <= 512, ran
+    assert torch.equal(got[0][:M], want[:M])
+    assert izb.device_status(0) == 0
+    W.close()
+
+
+@pytest.mark.parametrize("qt", [13, 14, 23])
+def test_scaled_products_are_exact(izb, qt):
+    """scale * quant reaches 4096 and travels as one or two fp16 terms.  With unit factors and one block's activation scale at 1, the others at
+    0, an output is that block's integer: equal to the CUDA-core kernel's (itself equal to the oracle's) bit for bit."""
+    import torch
+    M, N, K = 130, 144, 1280
+    w = extremes(qt, S.make_weight(qt, N, K, qt)).copy()
+    sb = w.reshape(N, K // 256, -1)
+    at = 208 if qt == 14 else 0
+    sb[:, :, at:at + 2] = np.frombuffer(np.float16(1.0).tobytes(), np.uint8)
+    if qt == 13:
+        sb[:, :, 2:4] = 0
+    W = izb.Weight(qt, w, N, K)
+    Mp = izb.pad_rows(M)
+    x = torch.from_numpy(S.make_act(M, K, 7)).cuda()
+    x[0], x[1] = 1.0, -1.0
+    aq, asc, _ = izb.quantize_act(x, Mp=Mp)
+    assert "gemm_tc" in kernels_of(izb, lambda: izb.gemm(W, aq, asc, M=M))
+    largest = 0.0
+    for b in range(K // 32):
+        one = torch.zeros_like(asc)
+        one[b] = 1.0
+        got, want = izb.gemm(W, aq, one, M=M)[:M], izb.gemm(W, aq, one, M=M, impl=izb.GEMM_CORE)[:M]
+        assert torch.equal(got, want) and torch.equal(got, got.round()), b
+        largest = max(largest, float(got.abs().max()))
+    assert largest > (2.0 ** 23 if qt != 13 else 2.0 ** 20)
     assert izb.device_status(0) == 0
     W.close()
 

@@ -114,3 +114,32 @@ def test_expert_rows_do_not_depend_on_the_other_tokens(izb, qt, F, E):
     assert izb.device_status(0) == 0
     for W in (Wg, Wu, Wd):
         W.close()
+
+
+def test_rows_too_long_for_the_rings(izb):
+    """Activations that leave no room for a ring go to the kernels that take them in pieces: expert rows of K = 20480, Q6_K rows of 65536."""
+    import torch
+    NE, NU, T, N, K = 2, 1, 5, 64, 20480
+    for qt in (12, 8):
+        g, u = S.make_weight(qt, NE * N, K, 1), S.make_weight(qt, NE * N, K, 2)
+        Wg, Wu = izb.Weight(qt, g, N, K, n_mats=NE), izb.Weight(qt, u, N, K, n_mats=NE)
+        aq, asc, _ = izb.quantize_act(torch.from_numpy(S.make_act(T, K, 9)).cuda() * 0.01)
+        ids, wts, counts = izb.moe_route(torch.from_numpy(S.make_act(T, NE, 3)).cuda(), NU)
+        _, tiles, mt, stok, swt, inv = izb.moe_sort(ids, wts, counts, 8)
+        h = izb.moe_gateup(Wg, Wu, aq, asc, tiles, mt, 8, stok, T * NU)[inv.long()]
+        y = izb.moe_down(Wg, aq[stok.long()].contiguous(), asc[:, stok.long()].contiguous(), tiles, mt, 8, swt, T * NU)[inv.long()]
+        for t in range(T):
+            e = int(ids[t, 0])
+            gate, up = (izb.gemm(W, aq, asc, impl=izb.GEMM_CORE, mat=e)[t].double() for W in (Wg, Wu))
+            for got, want in ((h[t], gate / (1 + torch.exp(-gate)) * up), (y[t], gate * float(wts[t, 0]))):
+                assert float((got - want).abs().max() / want.abs().max()) < TOL
+        Wg.close()
+        Wu.close()
+    W = izb.Weight(14, S.make_weight(14, N, 65536, 4), N, 65536)
+    aq, asc, _ = izb.quantize_act(torch.from_numpy(S.make_act(2, 65536, 5)).cuda())
+    want = izb.gemm(W, aq, asc, impl=izb.GEMM_CORE)[:2].double()
+    for t in (1, 2):
+        got = izb.gemv(W, aq, asc, t)
+        assert float((got - want[:t]).abs().max() / want.abs().max()) < TOL
+    assert izb.device_status(0) == 0
+    W.close()
