@@ -681,7 +681,7 @@ template <bool kDots> struct DeqOf<FQ6K, kDots> { using type = DeqQ6K; };
 // warp of the same CTA 135 clk later, a tcgen05.commit 182 clk after the last MMA; with three accumulators in the ring
 // that alone allows no block in under 175 clk.  An MMA or commit behind a lane test takes 98 clk to issue, with the elected
 // predicate inside the statement about 25 (6 % of the kernel).  The rest of a block's 550 clk is the combine warps' own
-// chain: test, two 65-clk reads of 32 columns, the packed FMAs and the register copies the compiler puts between the two.
+// chain: test, two 65-clk reads of 32 columns and the packed FMAs (64-column reads of the same chain were no faster).
 template <class F, bool kDots>
 __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_constant__ CUtensorMap tmW, const TcParams p) {
   extern __shared__ unsigned char smem_raw[];

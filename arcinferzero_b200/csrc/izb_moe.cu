@@ -421,7 +421,7 @@ extern "C" int izb_moe_gateup(const izb_weight* wg, const izb_weight* wu, const 
   if (TM == 128) {
     const int rc = izb_moe_gateup_tc(wg, wu, d_aq, d_asc, Mp, d_tiles, max_tiles, d_stok, d_h, (cudaStream_t)stream);
     if (rc <= 0) return rc;
-    IZB_FAIL(IZB_ERR_SHAPE, "moe_gateup: the grouped tensor-core GEMM needs F %% 128 == 0 and a weight with a tensor map (F = %d, K = %d); use TM <= 8", wg->N, wg->K);
+    IZB_FAIL(IZB_ERR_SHAPE, "moe_gateup: the grouped tensor-core GEMM needs F %% 16 == 0 and a weight with a tensor map (F = %d, K = %d); use TM <= 8", wg->N, wg->K);
   }
   IZB_FAIL(IZB_ERR_SHAPE, "moe_gateup: tiles of %d slots (1..8: per-tile GEMV kernels; 128: grouped tensor-core GEMM)", TM);
 }
@@ -440,7 +440,7 @@ extern "C" int izb_moe_down(const izb_weight* wd, const int8_t* d_hq, const floa
   if (TM == 128) {
     const int rc = izb_moe_down_tc(wd, d_hq, d_hsc, Sp, d_tiles, max_tiles, d_swt, d_y, (cudaStream_t)stream);
     if (rc <= 0) return rc;
-    IZB_FAIL(IZB_ERR_SHAPE, "moe_down: the grouped tensor-core GEMM needs E %% 128 == 0 and a weight with a tensor map (E = %d, F = %d); use TM <= 8", wd->N, wd->K);
+    IZB_FAIL(IZB_ERR_SHAPE, "moe_down: the grouped tensor-core GEMM needs E %% 16 == 0 and a weight with a tensor map (E = %d, F = %d); use TM <= 8", wd->N, wd->K);
   }
   IZB_FAIL(IZB_ERR_SHAPE, "moe_down: tiles of %d slots (1..8: per-tile GEMV kernels; 128: grouped tensor-core GEMM)", TM);
 }

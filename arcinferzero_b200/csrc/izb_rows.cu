@@ -6,8 +6,10 @@
 // instruction multiplies 16 weight rows x 16 elements with eight tokens at once, so eight tokens cost what one does.  (The
 // tcgen05 kernel wants 128 tokens per tile; at eight it is all latency.)
 //
-// The sums are those of the dot-product kernels bit for bit, so that a batch's results do not depend on which kernel its size
-// selects (a decode step requantises them, and one value that crosses a rounding boundary changes every layer after it): per
+// The sums are those of gemv_stream_kernel, gemv_q6p_kernel and the per-tile expert kernels bit for bit, so that a row's result does not
+// depend on which of these its call's size selects (a decode step requantises it, and one value that crosses a rounding boundary changes
+// every layer after it).  Not those of the Q4_K kernels for one to four rows of K % 1024 == 0, N >= 1024 (gemv_q4k_*), which add in an order of
+// their own: there four and five rows differ in last bits.  Per
 // output the same 32 partial sums -- superblock index modulo kSubs x piece of a superblock -- each added up in superblock order
 // with the same roundings, then the same pairwise tree.  A piece is 16 elements of a block pair (Q4_K), 16 elements (Q8_0) or a
 // 32-block (Q6_K), hence K = 16.  (One sum per output with the min term on a bf16 matrix instruction is a third of the f32
@@ -295,7 +297,7 @@ struct RQ6K {
             const float2 s = hd[b * 16 + g + 8 * r];
             // (both products and their sum are integers below 2^24: exact)
             const f2 v = f2_fma(f2_of(s.x, s.x), unmagic(d, r), f2_mul(f2_of(s.y, s.y), unmagic(e, r)));
-            // (product and addition on single values: of packed ones ptxas makes one fma, one rounding instead of two)
+            // (product and addition on single values: written as packed ones the results differed in their last bits, as of one rounding)
             const f2 f = f2_mul(xs[4 * b], wd[r]);
             acc[b][r] = f2_of(__fadd_rn(f2_get(acc[b][r], 0), __fmul_rn(f2_get(f, 0), f2_get(v, 0))), __fadd_rn(f2_get(acc[b][r], 1), __fmul_rn(f2_get(f, 1), f2_get(v, 1))));
           }
@@ -608,7 +610,7 @@ __device__ __forceinline__ bool dot_tile(Ring<F>& ring, const unsigned char* act
 // gate/up (pair): h[slot][N] = silu(x Wg^T) * (x Wu^T), token rows through stok; down: y[slot][N] = swt * (hq Wd^T).
 constexpr int kFewSlots = 2;
 // (small CTAs: items are divided among them as they come, and a tile's activations hold up four warps only; three per SM leave the two
-// ways 168 registers -- at 128 they spilt, and with the shared memory in use the stacks do not fit in L1)
+// ways 168 registers, which do not hold everything either: 100 bytes a thread are spilt for Q4_K, 176 for Q8_0)
 constexpr int kMoeWarps = 4, kMoeCtas = 3;
 // Where the items are fewer than the blocks that fit, a block takes kPer row tiles of one tile instead of kMoeWarps, its kSubs warps per row
 // tile sharing the superblocks also for few slots: gate / up 1024 x 512 of 8 experts Q4_K, four slots, 10.8 -> 6.0 us, sixteen 16.1 -> 6.9; 4096 x
