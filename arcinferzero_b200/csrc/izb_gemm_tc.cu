@@ -1,4 +1,5 @@
-// Prefill GEMM on the 5th-generation tensor cores (tcgen05, TMEM accumulators), exact per-32-block semantics.
+// Prefill GEMM on the 5th-generation tensor cores (tcgen05, TMEM accumulators), exact per-32-block semantics; the host side of this kernel and of
+// the folded one (csrc/izb_gemm_fold.cu), which takes plain stores of Q4_K and Q5_K products of long K under IZB_GEMM_AUTO.
 //
 // Problem: C[m][n] = sum over 32-blocks b of asc[m][b] * wscale[n][b] * dot_b[m][n]  (- the Q4_K min term), where dot_b
 // is an exact integer.  Both operands carry a scale per block, so a block's dot product must leave the tensor core
@@ -36,11 +37,12 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <algorithm>
 #include <exception>
 #include <mutex>
 #include <vector>
 
-#include "izb_common.cuh"
+#include "izb_fold.cuh"
 
 void izb_set_tc_ok(int device, int ok);
 void izb_note_noalloc_status(int device, uint32_t* status);
@@ -1166,6 +1168,12 @@ void tc_scratch_bytes(int n_tiles, int K, int sps, size_t* img_bytes, size_t* as
   *asc_bytes = (size_t)n_tiles * (K / 32) * BM * 4;
 }
 
+int launch_split_reduce(const float* part, int n_split, int M, int N, float* C, int ldc, int c_off, const uint32_t* part_bad, cudaStream_t st) {
+  dim3 grid((N / 4 + 255) / 256, M);
+  IZB_LAUNCH("split_reduce", st, izb_launch_pdl(split_reduce_kernel, grid, 256, 0, st, part, n_split, M, N, C, ldc, c_off, part_bad));
+  return IZB_OK;
+}
+
 // the activation pre-pass + the GEMM on scratch the caller owns (img_bytes + asc_bytes of tc_scratch_bytes, then, where the
 // call may be cut along K, `split_ws`)
 int run_tc_on(const izb_weight* w, int mat, const int8_t* aq, const float* asc, int lda, int rows_total, const int32_t* tiles,
@@ -1203,11 +1211,7 @@ int run_tc_on(const izb_weight* w, int mat, const int8_t* aq, const float* asc, 
   p.part_bad = split_flag(split_ws, w->device);
   dim3 grid(tc_grid(w->device, n_items * p.n_split));
   if (int rc = launch_tc_of(w, p, grid, st)) return rc;
-  if (p.n_split > 1) {
-    dim3 rg((w->N / 4 + 255) / 256, M_store);
-    IZB_LAUNCH("split_reduce", st, izb_launch_pdl(split_reduce_kernel, rg, 256, 0, st, split_ws, p.n_split, M_store, w->N, C, ldc, c_off, p.part_bad));
-  }
-  return IZB_OK;
+  return p.n_split > 1 ? launch_split_reduce(split_ws, p.n_split, M_store, w->N, C, ldc, c_off, p.part_bad, st) : IZB_OK;
 }
 
 // the activation pre-pass + the GEMM for one tile set
@@ -1229,13 +1233,52 @@ int run_tc(const izb_weight* w, int mat, const int8_t* aq, const float* asc, int
                    st, reuse_images);
 }
 
+// A plain store with the scales folded into the operands (csrc/izb_gemm_fold.cu), of long K as with tc_split, and for the same reasons: short K
+// gains little (a tile is mostly fill and drain), and keeps the sums of the other store modes; x: the quantiser's input (aq and asc are written), or
+// null where aq and asc are there.  +1: not taken, or its arena (1.6 times the other kernel's) cannot be had in a capture or without memory:
+// the caller goes on with the other kernel.
+int run_fold(const izb_weight* w, int mat, const float* x, int ldx, int T, int8_t* aq, float* asc, int Mp, int M_store, float* C, int ldc, int c_off, cudaStream_t st) {
+  if (!tc_takes(w) || !izb_fold_takes(w) || w->K < 2048) return 1;
+  FoldParams p;
+  p.tt = izb_fold_tile_rows(w->device, M_store, w->N);
+  p.n_mtiles = (M_store + p.tt - 1) / p.tt;
+  const int rows = p.n_mtiles * p.tt;
+  if ((rows + 31) / 32 > 65535) return 1;
+  const size_t img_bytes = izb_fold_img_bytes(rows, w->K), tail_bytes = izb_fold_tail_bytes(rows, w->K);
+  void* ws = nullptr;
+  if (int rc = izb_workspace(w->device, kWsGemm, img_bytes + tail_bytes + split_area(w->device), st, &ws, true)) return rc;
+  uint32_t* err = izb_device_error_word(w->device);
+  if (!err) IZB_FAIL(IZB_ERR_NOMEM, "gemm: no device error word");
+  p.img = (unsigned char*)ws;
+  p.tail = p.img + img_bytes;
+  p.part = (float*)(p.tail + tail_bytes);
+  p.part_bad = split_flag(p.part, w->device);
+  p.M = M_store;
+  p.N = w->N;
+  p.K = w->K;
+  p.mat = mat;
+  p.C = C;
+  p.ldc = ldc;
+  p.c_off = c_off;
+  p.err = err;
+  const uint32_t spin = g_test_spin.exchange(0);
+  p.spin_limit = spin ? spin : kSpinLimit;
+  p.skip_stage = g_test_skip.exchange(-1);
+  const int n_items = (w->N + BN - 1) / BN * p.n_mtiles;
+  p.n_split = tc_split(w->device, n_items, w->K / 256);
+  if (int rc = x ? izb_fold_quant_prepare(w, x, ldx, T, Mp, aq, asc, p, st) : izb_fold_prepare(w, aq, asc, Mp, Mp, p, st)) return rc;
+  if (int rc = izb_fold_gemm(w, p, tc_grid(w->device, n_items * p.n_split), st)) return rc;
+  return p.n_split > 1 ? launch_split_reduce(p.part, p.n_split, M_store, w->N, C, ldc, c_off, p.part_bad, st) : IZB_OK;
+}
+
 }  // namespace
 
 // scratch bytes of a dense tensor-core GEMM over `rows` activation rows (izb_reserve sizes the arenas with it)
 size_t izb_gemm_tc_scratch_bytes(int device, int type, int rows, int K) {
   size_t img_bytes, asc_bytes;
   tc_scratch_bytes((rows + BM - 1) / BM, K, type == IZB_Q4_K ? 5 : 4, &img_bytes, &asc_bytes);
-  return img_bytes + asc_bytes + split_area(device);
+  const size_t fold = izb_fold_img_bytes(rows + BM, K) + izb_fold_tail_bytes(rows + BM, K);  // (tiles round the rows up by less than one)
+  return std::max(img_bytes + asc_bytes, fold) + split_area(device);
 }
 
 extern "C" int izb_debug_wait_test(uint32_t spin_limit, int skip_stage) {
@@ -1265,9 +1308,14 @@ int izb_make_raw_tensor_map(izb_weight* w) { return make_map(w, w->sb_bytes, BN,
 // chunks of the few-row kernel: a superblock; Q6_K 16 bytes more, for a row pitch its shared-memory reads want
 int izb_make_rows_tensor_map(izb_weight* w) { return make_map(w, w->packed6 ? w->sb_bytes + 16 : w->sb_bytes, 16, w->tmap16_raw); }
 
-// may_cut: the K range may be cut into parts (IZB_GEMM_AUTO); IZB_GEMM_TC names this kernel, and gives the sums of izb_gemm_noalloc
+// may_cut: the K range may be cut into parts, and scales be folded into the operands (IZB_GEMM_AUTO); IZB_GEMM_TC names this kernel, and gives the
+// sums of izb_gemm_noalloc
 int izb_gemm_tc_launch(const izb_weight* w, int mat, const int8_t* aq, const float* asc, int M, int Mp, float* C, int ldc, int c_off,
                        int acc, int32_t* dots, cudaStream_t st, bool may_cut) {
+  if (may_cut && acc == 0 && !dots) {
+    const int rc = run_fold(w, mat, nullptr, 0, 0, const_cast<int8_t*>(aq), const_cast<float*>(asc), Mp, M, C, ldc, c_off, st);
+    if (rc <= 0) return rc;
+  }
   const int n_tiles = (M + BM - 1) / BM;
   if (n_tiles > 65535) return 1;
   return run_tc(w, mat, aq, asc, Mp, Mp, nullptr, n_tiles, nullptr, nullptr, M, C, ldc, c_off, acc, dots, kWsGemm, st, false, may_cut);
@@ -1277,6 +1325,10 @@ int izb_gemm_tc_launch(const izb_weight* w, int mat, const int8_t* aq, const flo
 // its images.  +1 = shape not taken.
 int izb_gemm_tc_quant_launch(const izb_weight* w, int mat, const float* x, int ldx, int M, int Mp, int8_t* aq, float* asc, float* C,
                              int ldc, int c_off, int acc, cudaStream_t st) {
+  if (acc == 0) {
+    const int rc = run_fold(w, mat, x, ldx, M, aq, asc, Mp, Mp, C, ldc, c_off, st);
+    if (rc <= 0) return rc;
+  }
   const int n_tiles = (Mp + BM - 1) / BM;  // (the GEMM runs over the padded rows, as izb_matmul's does)
   if (n_tiles > 65535 || !tc_takes(w)) return 1;
   const int K = w->K, sps = tc_sps(w, false);

@@ -64,7 +64,9 @@ extern "C" {
 /* izb_gemm `impl` */
 /* IZB_GEMM_AUTO, and with it izb_matmul and izb_quant_matmul, may cut a long K (2048 and more) of a plain store into parts when there are few
  * 128 x 128 output tiles, and add the parts' sums afterwards: such sums are rounded in other places, so that a row's last bits may depend on
- * the number of rows in the call.  Store modes 1, 2 and 3, IZB_GEMM_TC and izb_gemm_noalloc never cut: a row's sums are the same in every call. */
+ * the number of rows in the call.  Plain stores of long K of Q4_K and Q5_K weights run on a kernel that folds the block scales into its operands and
+ * sums in an order of its own (nearer to 64 bits than the other one's).  Store modes 1, 2 and 3, IZB_GEMM_TC and izb_gemm_noalloc do
+ * neither: a row's sums are the same in every call. */
 #define IZB_GEMM_AUTO 0 /* the tensor-core or the CUDA-core kernel, by type and shape */
 #define IZB_GEMM_CORE 1 /* CUDA-core dp4a kernel, f32 combine in the reference's order (zero/kernels/gemm.cl:441-487) */
 #define IZB_GEMM_TC 2   /* tcgen05 kernel (TMEM accumulators), error if the shape is not taken */

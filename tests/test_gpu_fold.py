@@ -1,0 +1,144 @@
+"""The folded GEMM (plain stores of Q4_K and Q5_K products of K >= 2048 under GEMM_AUTO): tiles of any number of token rows, part columns, K cut and not, extreme
+and non-finite scales."""
+import numpy as np
+import pytest
+
+from arcinferzero_b200 import synth as S
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def weights64(qt, rows, K):
+    """The weights in 64 bits, exactly."""
+    n, nsb = rows.shape[0], K // 256
+    w, out = rows.reshape(n, nsb, -1), np.empty((n, nsb, 16, 16))
+    for i in range(n):
+        for s in range(nsb):
+            if qt == 12:
+                d, dmin, sc, mn, q = O.decode_q4k_sb(w[i, s])
+                sc, mn = sc.repeat(2), mn.repeat(2)
+            else:
+                d, dmin, sc, mn, _, q = O.decode_generic_sb(qt, w[i, s])
+            out[i, s] = d * sc[:, None].astype(np.float64) * q.reshape(16, 16) - dmin * mn[:, None].astype(np.float64)
+    return out.reshape(n, K)
+
+
+def exact(qt, rows, K, aq, asc):
+    a = aq.astype(np.float64).reshape(len(aq), K // 32, 32) * asc.T[:, :, None].astype(np.float64)
+    return a.reshape(len(aq), K) @ weights64(qt, rows, K).T
+
+
+def run(izb, W, aq, asc, M, N, Mp):
+    import torch
+    out = torch.full((Mp, N + 8), float("nan"), device="cuda")
+    izb.gemm(W, aq, asc, M=M, out=out, c_off=4)
+    assert izb.device_status(0) == 0
+    got = out.cpu().numpy()
+    assert np.isnan(got[:, :4]).all() and np.isnan(got[:, N + 4:]).all() and np.isnan(got[M:]).all()
+    return got[:M, 4:N + 4]
+
+
+# 9 .. 145 rows: one tile of each height, two tiles of unequal ones; 144: a part column tile; 20000 columns: more than one round, K not cut
+@pytest.mark.parametrize("qt", [12, 13])
+@pytest.mark.parametrize("M,N,K", [(9, 128, 2048), (16, 128, 2304), (33, 128, 2048), (64, 256, 2560), (97, 128, 2048), (128, 128, 2048), (129, 256, 2048), (145, 128, 4096),
+                                   (300, 144, 2304), (40, 20000, 2048), (700, 4096, 2048)])
+def test_fold_against_64_bits(izb, qt, M, N, K):
+    """Bound: the activations keep 22 bits of a superblock's largest, the superblock's sum is cut once below 2^-23 of itself, and K / 256 such sums are
+    added in f32: some 2e-7 of the result's norm; 4e-7 leaves room for the spread."""
+    import torch
+    w = S.make_weight(qt, N, K, N + K)
+    W = izb.Weight(qt, w, N, K)
+    Mp = izb.pad_rows(M)
+    x = S.make_act(M, K, M + K)
+    x.reshape(M, -1, 32)[:, ::3] *= 40.0  # superblocks whose blocks differ in scale
+    aq, asc, _ = izb.quantize_act(torch.from_numpy(x).cuda(), Mp=Mp)
+    got = run(izb, W, aq, asc, M, N, Mp)
+    cols = np.unique(np.linspace(0, N - 1, 96).astype(int))
+    ref = exact(qt, w[cols], K, aq[:M].cpu().numpy(), asc[:, :M].cpu().numpy())
+    err = np.linalg.norm(got[:, cols] - ref) / np.linalg.norm(ref)
+    assert err < 4e-7, err
+    core = izb.gemm(W, aq, asc, M=M, impl=izb.GEMM_CORE).cpu().numpy()[:M]
+    assert np.abs(got - core).max() / np.abs(core).max() < 1e-5
+    both, q, _ = izb.quant_matmul(W, torch.from_numpy(x).cuda(), M)
+    assert torch.equal(q, aq) and (both.cpu().numpy()[:M] == got).all()  # the pre-pass with the quantiser in it
+    W.close()
+
+
+def test_rows_do_not_depend_on_the_tile(izb):
+    import torch
+    N, K = 10240, 2048  # (80 column tiles: K is not cut)
+    W = izb.Weight(12, np.tile(S.make_weight(12, 256, K, 1), (N // 256, 1)), N, K)
+    aq, asc, _ = izb.quantize_act(torch.from_numpy(S.make_act(400, K, 2)).cuda())
+    want = izb.gemm(W, aq, asc, M=400)[:400]
+    for M in (16, 48, 80, 112, 128, 160, 272):
+        assert torch.equal(izb.gemm(W, aq[:M].contiguous(), asc[:, :M].contiguous(), M=M)[:M], want[:M]), M
+    W.close()
+
+
+@pytest.mark.parametrize("qt", [12, 13])
+def test_fold_scales_at_the_ends_of_their_range(izb, qt):
+    """Activation scales of 0, denormal, next to overflow and of either sign; weights at their largest.  Against the CUDA-core kernel, row by row."""
+    import torch
+    M, N, K = 48, 128, 2048
+    w = S.make_weight(qt, N, K, 3).reshape(N, K // 256, -1).copy()
+    w[0, :, 4:] = 0xFF
+    w[1, :, 0:4] = 0
+    W = izb.Weight(qt, w.reshape(N, -1), N, K)
+    aq, asc, _ = izb.quantize_act(torch.from_numpy(S.make_act(M, K, 4)).cuda())
+    aq[0], aq[1] = 127, -128
+    f = torch.ones_like(asc)
+    for row, v in enumerate([1.0, 1.0, 0.0, 1e-45, 1e-40, 2.0 ** -126, 1e-36, 1e-30, 1e28, 1e31, -1.0]):
+        f[:, row] = v
+    f[5, 11], f[6, 12], f[7, 13], f[8, 14] = 0.0, 1e-20, -1.0, 1e20
+    asc = torch.where(f.abs() < 1e-25, f, asc * f)
+    got, core = izb.gemm(W, aq, asc, M=M)[:M].double(), izb.gemm(W, aq, asc, M=M, impl=izb.GEMM_CORE)[:M].double()
+    assert torch.isfinite(core).all() and torch.isfinite(got).all()
+    for row in range(M):
+        big = core[row].abs().max()
+        # (a sum of denormal terms is rounded to 2^-149 once per block in one kernel, once per superblock in the other)
+        assert float((got[row] - core[row]).abs().max()) <= 1e-5 * float(big) + K / 32 * 2.0 ** -149, row
+    assert float(core[3].abs().max()) > 0
+    W.close()
+
+
+def test_fold_scales_that_are_no_numbers(izb):
+    """An infinite or undefined scale reaches what it reaches in the CUDA-core kernel's results, its own row, and no other row."""
+    import torch
+    M, N, K = 48, 128, 2048
+    W = izb.Weight(12, S.make_weight(12, N, K, 5), N, K)
+    aq, asc, _ = izb.quantize_act(torch.from_numpy(S.make_act(M, K, 6)).cuda())
+    want = izb.gemm(W, aq, asc, M=M)[:M]
+    asc[3, 2], asc[9, 20], asc[32, 33] = float("inf"), float("nan"), float("-inf")
+    got, core = izb.gemm(W, aq, asc, M=M)[:M], izb.gemm(W, aq, asc, M=M, impl=izb.GEMM_CORE)[:M]
+    assert torch.equal(torch.isfinite(got), torch.isfinite(core))
+    keep = [r for r in range(M) if r not in (2, 20, 33)]
+    assert torch.equal(got[keep], want[keep])
+    W.close()
+
+
+def test_fold_in_a_capture_without_its_arena(izb):
+    """Where the folded kernel's arena would have to grow inside a capture, the call goes to the other kernel."""
+    import os
+    import subprocess
+    import sys
+    body = """
+import torch, arcinferzero_b200 as izb
+from arcinferzero_b200 import synth as S
+N, K, M = 1024, 2048, 4096
+W = izb.Weight(12, S.make_weight(12, N, K, 1), N, K)
+aq, asc, _ = izb.quantize_act(torch.from_numpy(S.make_act(M, K, 2)).cuda())
+izb.gemm(W, aq, asc, out=torch.zeros(M, N, device="cuda"), acc=1)  # the arena of the other kernel
+want = izb.gemm(W, aq, asc, impl=izb.GEMM_TC)
+out = torch.zeros(M, N, device="cuda")
+torch.cuda.synchronize()
+g = torch.cuda.CUDAGraph()
+with torch.cuda.graph(g):
+    izb.gemm(W, aq, asc, out=out)
+g.replay()
+torch.cuda.synchronize()
+assert torch.equal(out, want) and izb.device_status(0) == 0
+print("done")
+"""
+    r = subprocess.run([sys.executable, "-c", body], cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))), capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "done" in r.stdout, r.stdout + r.stderr
