@@ -28,8 +28,14 @@
 //               operand layout, the min-term operand, block scales to shared memory;
 //   warps 1-2   issue tcgen05.mma (one thread each, alternating stages) into a ring of three 128-column accumulators +
 //               the min-term accumulator (always warp 2, so that one thread orders all updates of it);
-//   warps 8-15  combine: tcgen05.ld of 64 columns at a time, one fma per element, final store with the reference's
+//   warps 8-15  combine: tcgen05.ld of 16 rows x 64 columns at a time, one fma per element, final store with the reference's
 //               store modes.
+// The combine warps read accumulators as fragments: a thread meets 4 token rows x 8 column pairs, not 1 x 64 columns.  With a lane per row the
+// column scales (Q8_0: 64 per block) were 16-byte reads of one address by the whole warp, four passes each: the shared-memory pipe stood at 86 %
+// of its peak for Q8_0.  Together with role branches the compiler knows to be warp-uniform, and SwiGLU products two at a time (us, before and
+// now): 300 x 5120 x 17408 Q6_K 235 / 216, 512 x 4096 x 4096 Q8_0 67.6 / 64.9, feed-forward block of 1000 x 5120 x 17408 Q4_K 1387 / 1297, of
+// 94 x 2048 x 7168 123 / 111, 4096 tokens x 8 of 128 experts 1163 / 1148.  Tried: sixteen combine warps of 16 rows x 64 columns and two groups of
+// dequantisers (28 warps, 72 registers at launch): Q8_0 62, but the feed-forward block 1482 and the experts 1200.
 // All waits are bounded: a wait that gives up sets a CTA-wide abort flag and a device error word, the CTA drains and
 // returns without storing (izb_device_status reports it).
 #include <cuda.h>
@@ -125,6 +131,9 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
+__device__ __forceinline__ void mbar_arrive_if(uint32_t bar, bool pred) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, 0;\n\t@p mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}" ::"r"(bar), "r"((uint32_t)pred) : "memory");
+}
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
@@ -201,55 +210,12 @@ __device__ __forceinline__ void tc_mma_f16(uint32_t d_tmem, uint64_t adesc, uint
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// tcgen05.ld of 64 columns + wait, delivered as 32 register pairs (columns 2i, 2i+1) for the f32x2 arithmetic.  The
-// load, the wait and the moves are one asm block: nothing that uses the values can be scheduled before the wait.
-__device__ __forceinline__ void tc_ld64_pairs(uint32_t taddr, unsigned long long (&r)[32]) {
-  asm volatile(
-      "{\n\t.reg .b32 t<64>;\n\t"
-      "tcgen05.ld.sync.aligned.32x32b.x64.b32 {t0,t1,t2,t3,t4,t5,t6,t7,t8,t9,t10,t11,t12,t13,t14,t15,t16,t17,t18,t19,t20,t21,t22,t23,t24,t25,t26,t27,t28,t29,t30,t31,t32,t33,t34,t35,t36,t37,t38,t39,t40,t41,t42,t43,t44,t45,t46,t47,t48,t49,t50,t51,t52,t53,t54,t55,t56,t57,t58,t59,t60,t61,t62,t63}, [%32];\n\t"
-      "tcgen05.wait::ld.sync.aligned;\n\t"
-      "mov.b64 %0, {t0,t1};\n\t"
-      "mov.b64 %1, {t2,t3};\n\t"
-      "mov.b64 %2, {t4,t5};\n\t"
-      "mov.b64 %3, {t6,t7};\n\t"
-      "mov.b64 %4, {t8,t9};\n\t"
-      "mov.b64 %5, {t10,t11};\n\t"
-      "mov.b64 %6, {t12,t13};\n\t"
-      "mov.b64 %7, {t14,t15};\n\t"
-      "mov.b64 %8, {t16,t17};\n\t"
-      "mov.b64 %9, {t18,t19};\n\t"
-      "mov.b64 %10, {t20,t21};\n\t"
-      "mov.b64 %11, {t22,t23};\n\t"
-      "mov.b64 %12, {t24,t25};\n\t"
-      "mov.b64 %13, {t26,t27};\n\t"
-      "mov.b64 %14, {t28,t29};\n\t"
-      "mov.b64 %15, {t30,t31};\n\t"
-      "mov.b64 %16, {t32,t33};\n\t"
-      "mov.b64 %17, {t34,t35};\n\t"
-      "mov.b64 %18, {t36,t37};\n\t"
-      "mov.b64 %19, {t38,t39};\n\t"
-      "mov.b64 %20, {t40,t41};\n\t"
-      "mov.b64 %21, {t42,t43};\n\t"
-      "mov.b64 %22, {t44,t45};\n\t"
-      "mov.b64 %23, {t46,t47};\n\t"
-      "mov.b64 %24, {t48,t49};\n\t"
-      "mov.b64 %25, {t50,t51};\n\t"
-      "mov.b64 %26, {t52,t53};\n\t"
-      "mov.b64 %27, {t54,t55};\n\t"
-      "mov.b64 %28, {t56,t57};\n\t"
-      "mov.b64 %29, {t58,t59};\n\t"
-      "mov.b64 %30, {t60,t61};\n\t"
-      "mov.b64 %31, {t62,t63};\n\t"
-      "}"
-      : "=l"(r[0]), "=l"(r[1]), "=l"(r[2]), "=l"(r[3]), "=l"(r[4]), "=l"(r[5]), "=l"(r[6]), "=l"(r[7]), "=l"(r[8]), "=l"(r[9]), "=l"(r[10]), "=l"(r[11]), "=l"(r[12]), "=l"(r[13]), "=l"(r[14]), "=l"(r[15]), "=l"(r[16]), "=l"(r[17]), "=l"(r[18]), "=l"(r[19]), "=l"(r[20]), "=l"(r[21]), "=l"(r[22]), "=l"(r[23]), "=l"(r[24]), "=l"(r[25]), "=l"(r[26]), "=l"(r[27]), "=l"(r[28]), "=l"(r[29]), "=l"(r[30]), "=l"(r[31])
-      : "r"(taddr)
-      : "memory");
-}
-// the same for 32 columns (16 register pairs): for readers that are short of registers
-__device__ __forceinline__ void tc_ld32_pairs(uint32_t taddr, unsigned long long (&r)[16]) {
+// tcgen05.ld of 16 TMEM lanes x 64 columns + wait as matrix fragments: register pair 2g + r holds lane 8 r + threadlane / 4, columns
+// 8 g + 2 (threadlane % 4) and the one after
+__device__ __forceinline__ void tc_ld_frag64(uint32_t taddr, unsigned long long (&r)[16]) {
   asm volatile(
       "{\n\t.reg .b32 t<32>;\n\t"
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {t0,t1,t2,t3,t4,t5,t6,t7,t8,t9,t10,t11,t12,t13,t14,t15,t16,t17,t18,t19,t20,t21,t22,t23,t24,t25,t26,t27,t28,t29,t30,t31}, [%16];\n\t"
+      "tcgen05.ld.sync.aligned.16x256b.x8.b32 {t0,t1,t2,t3,t4,t5,t6,t7,t8,t9,t10,t11,t12,t13,t14,t15,t16,t17,t18,t19,t20,t21,t22,t23,t24,t25,t26,t27,t28,t29,t30,t31}, [%16];\n\t"
       "tcgen05.wait::ld.sync.aligned;\n\t"
       "mov.b64 %0, {t0,t1};\n\t"
       "mov.b64 %1, {t2,t3};\n\t"
@@ -286,11 +252,10 @@ __device__ __forceinline__ unsigned long long pack2(float x) {
   asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x));
   return r;
 }
-// up * silu(gate) (zero/kernels/gemm.cl:562-565).  Out of line on purpose: the epilogues call it 64 and 32 times per
-// thread, and the role loops of the kernel compete for the instruction cache.
-__device__ __noinline__ float swiglu_mul(float g, float u) { return __fmul_rn(u, __fdiv_rn(g, __fadd_rn(1.0f, expf(-g)))); }
-__device__ __forceinline__ unsigned long long pack_pair(float lo, float hi) {
-  return (unsigned long long)__float_as_uint(lo) | ((unsigned long long)__float_as_uint(hi) << 32);
+// up * silu(gate) (zero/kernels/gemm.cl:562-565).  Two at a time, for their latency; out of line on purpose:
+// the epilogues call it 32 and 16 times per thread, and the role loops of the kernel compete for the instruction cache.
+__device__ __noinline__ float2 swiglu_mul2(float2 g, float2 u) {
+  return make_float2(__fmul_rn(u.x, __fdiv_rn(g.x, __fadd_rn(1.0f, expf(-g.x)))), __fmul_rn(u.y, __fdiv_rn(g.y, __fadd_rn(1.0f, expf(-g.y)))));
 }
 __device__ __forceinline__ float lo_f(unsigned long long a) { return __uint_as_float((uint32_t)a); }
 __device__ __forceinline__ float hi_f(unsigned long long a) { return __uint_as_float((uint32_t)(a >> 32)); }
@@ -682,8 +647,8 @@ template <bool kDots> struct DeqOf<FQ6K, kDots> { using type = DeqQ6K; };
 // What a hand-over costs (measured on one SM): a satisfied mbarrier test has 54 clk of latency, an arrival is seen by a waiting
 // warp of the same CTA 135 clk later, a tcgen05.commit 182 clk after the last MMA; with three accumulators in the ring
 // that alone allows no block in under 175 clk.  An MMA or commit behind a lane test takes 98 clk to issue, with the elected
-// predicate inside the statement about 25 (6 % of the kernel).  The rest of a block's 550 clk is the combine warps' own
-// chain: test, two 65-clk reads of 32 columns and the packed FMAs (64-column reads of the same chain were no faster).
+// predicate inside the statement about 25 (6 % of the kernel).  The rest of a block's time is the combine warps' own
+// chain: test, two TMEM reads and the packed FMAs; in calls of a millisecond the board is at its 1000 W as well.
 template <class F, bool kDots>
 __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_constant__ CUtensorMap tmW, const TcParams p) {
   extern __shared__ unsigned char smem_raw[];
@@ -697,7 +662,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
   volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(smem + MP::OFF_BAR + MP::NUM_BARS * 8 + 4);
   const uint32_t bar0 = smem_u32(bars);
   auto bar = [&](int i) -> uint32_t { return bar0 + 8u * (uint32_t)i; };
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // (through a shuffle: the compiler then knows it to be the same for the whole warp and keeps what follows from it in uniform registers)
+  const int warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     // Consumers release a buffer with one arrival per THREAD (128 dequantisers, 256 combine threads): one elected arrival per
@@ -706,9 +672,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
     for (int i = 0; i < NA; ++i) { mbar_init(bar(MP::A_FULL + i), 1); mbar_init(bar(MP::A_EMPTY + i), 1); }
     for (int i = 0; i < NB; ++i) { mbar_init(bar(MP::B_FULL + i), 128); mbar_init(bar(MP::B_EMPTY + i), 1); }
     for (int i = 0; i < NR; ++i) { mbar_init(bar(MP::RAW_FULL + i), 1); mbar_init(bar(MP::RAW_EMPTY + i), 128); }
-    for (int i = 0; i < ND1; ++i) { mbar_init(bar(MP::D1_FULL + i), 1); mbar_init(bar(MP::D1_EMPTY + i), 256); }
+    for (int i = 0; i < ND1; ++i) { mbar_init(bar(MP::D1_FULL + i), 1); mbar_init(bar(MP::D1_EMPTY + i), 8); }
     mbar_init(bar(MP::D2_FULL), 1);
-    mbar_init(bar(MP::D2_EMPTY), 256);
+    mbar_init(bar(MP::D2_EMPTY), 8);
     for (int i = 0; i < NASC; ++i) { mbar_init(bar(MP::ASC_FULL + i), 1); mbar_init(bar(MP::ASC_EMPTY + i), 256); }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -720,7 +686,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xFFFFFFFFu, *tmem_slot, 0);
 
   // ---- the CTA's work: items blockIdx.x, blockIdx.x + gridDim.x, ... of (row tiles) x (column tiles) x (K parts), K part
   // fastest, then column tile.  Every role walks the same list; its ring positions and barrier parities run on from item to
@@ -898,11 +864,11 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
       }
     }
   } else {
-    // ================= combine: thread <-> TMEM lane (token row) 32*(warp%4) + lane, 64 of the 128 columns.
+    // ================= combine: a warp holds 32 token rows (TMEM lanes 32 * (warp % 4) ..) x 64 of the 128 columns as fragments (tc_ld_frag64).
     // All f32 arithmetic is done on register pairs (fma.rn.f32x2): half the instructions for the same IEEE results.
     asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
     const int q = warp & 3, half = (warp - 8) >> 2;
-    const int r = 32 * q + lane;
+    const int row0 = 32 * q + (lane >> 2), cl = 64 * half + 2 * (lane & 3);  // this thread's rows row0 + 8 k, k < 4; columns cl + 8 g, + 1, g < 8
     const uint32_t t_lane = tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)(half * 64);
     bool ok = true;
     int d = 0, pd = 0, sq = 0, pq = 0;  // accumulator ring / scale ring positions and wait parities
@@ -910,55 +876,55 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
     for (int w = blockIdx.x; w < n_work && ok; w += gridDim.x, ++n_item) {
       __syncwarp();  // (rows that are not stored come here first)
       const Item it = item(w);
-      const int n0 = it.nt * BN;
+      const int n0 = it.nt * BN + cl;
       const int r0 = p.tiles ? p.tiles[2 + 3 * it.tile] : it.tile * BM;
       const int nr = p.tiles ? p.tiles[3 + 3 * it.tile] : min(BM, p.M - r0);
-      const bool row_ok = r < nr;
-      const int out_row = r0 + r;
-      unsigned long long res2[32], tq2[32];  // pairs of columns (2i, 2i+1)
+      unsigned long long res2[4][8], tq2[4][8];  // [row][column pair]
 #pragma unroll
-      for (int c = 0; c < 32; ++c) res2[c] = tq2[c] = 0ull;
+      for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int g = 0; g < 8; ++g) res2[k][g] = tq2[k][g] = 0ull;
       for (int s = it.s0; s < it.s1 && ok; ++s, ++sbc) {
-        const float* as = reinterpret_cast<const float*>(smem + MP::OFF_ASC + sq * 4096) + r;  // this row's 8 block scales
+        const float* as = reinterpret_cast<const float*>(smem + MP::OFF_ASC + sq * 4096) + row0;  // the rows' eight block scales
         if (!kDots && !mbar_wait_warp(bar(MP::ASC_FULL + sq), pq, abort_flag, p.err, p.spin_limit, E_EPI)) { ok = false; break; }
 #pragma unroll
         for (int b = 0; b < 8; ++b) {
-          const unsigned long long a2 = pack2(kDots ? 0.0f : as[b * BM]);
+          unsigned long long a2[4];
+          if (!kDots) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) a2[k] = pack2(as[b * BM + 8 * k]);
+          }
           if (!mbar_wait_warp(bar(MP::D1_FULL + d), pd, abort_flag, p.err, p.spin_limit, E_EPI)) { ok = false; break; }
           tc_fence_after();
+          unsigned long long dd[8];
+          if (F::kColScale && !kDots) {
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {  // 32 columns at a time: the block loop's working set stays inside the register budget
+            for (int g = 0; g < 8; ++g) dd[g] = *reinterpret_cast<const unsigned long long*>(smem + MP::OFF_SCL + (sbc & 3) * 4096 + b * 512 + (cl + 8 * g) * 4);
+          }
+#pragma unroll
+          for (int hr = 0; hr < 2; ++hr) {  // 16 rows at a time: the block loop's working set stays inside the register budget
             unsigned long long v[16];
-            tc_ld32_pairs(t_lane + (uint32_t)(d * BN + 32 * h), v);
-            if (h == 1) {
+            tc_ld_frag64(t_lane + ((uint32_t)(16 * hr) << 16) + (uint32_t)(d * BN), v);
+            if (hr == 1) {
               tc_fence_before();
-              mbar_arrive(bar(MP::D1_EMPTY + d));  // the accumulator buffer may be overwritten
+              mbar_arrive_if(bar(MP::D1_EMPTY + d), lane == 0);  // the accumulator buffer may be overwritten (the loads were the whole warp's)
             }
-            if (kDots) {
-              if (row_ok) {
-                int32_t* o = p.dots + ((size_t)out_row * p.N + n0 + half * 64 + 32 * h) * nb + 8 * s + b;
 #pragma unroll
-                for (int c = 0; c < 16; ++c)
-                  if (n0 + half * 64 + 32 * h + 2 * c < p.N) {  // (N is a multiple of 16: pairs are whole)
-                    o[(size_t)(2 * c) * nb] = __float2int_rn(lo_f(v[c]));
-                    o[(size_t)(2 * c + 1) * nb] = __float2int_rn(hi_f(v[c]));
-                  }
-              }
-            } else if (!F::kColScale) {
-              if (b == 0) {
-#pragma unroll
-                for (int c = 0; c < 16; ++c) tq2[16 * h + c] = fmul2(a2, v[c]);
+            for (int j = 0; j < 16; ++j) {
+              const int k = 2 * hr + (j & 1), g = j >> 1;
+              if (kDots) {
+                const int row = row0 + 8 * k;
+                if (row < nr && n0 + 8 * g < p.N) {  // (N is a multiple of 16: pairs are whole)
+                  int32_t* o = p.dots + ((size_t)(r0 + row) * p.N + n0 + 8 * g) * nb + 8 * s + b;
+                  o[0] = __float2int_rn(lo_f(v[j]));
+                  o[nb] = __float2int_rn(hi_f(v[j]));
+                }
+              } else if (F::kColScale) {
+                ffma2(res2[k][g], fmul2(a2[k], dd[g]), v[j]);
+              } else if (b == 0) {
+                tq2[k][g] = fmul2(a2[k], v[j]);
               } else {
-#pragma unroll
-                for (int c = 0; c < 16; ++c) ffma2(tq2[16 * h + c], a2, v[c]);
-              }
-            } else {
-              const ulonglong2* d8 = reinterpret_cast<const ulonglong2*>(smem + MP::OFF_SCL + (sbc & 3) * 4096 + b * 512 + half * 256 + h * 128);
-#pragma unroll
-              for (int c4 = 0; c4 < 8; ++c4) {
-                const ulonglong2 dd = d8[c4];  // four column scales
-                ffma2(res2[16 * h + 2 * c4], fmul2(a2, dd.x), v[2 * c4]);
-                ffma2(res2[16 * h + 2 * c4 + 1], fmul2(a2, dd.y), v[2 * c4 + 1]);
+                ffma2(tq2[k][g], a2[k], v[j]);
               }
             }
           }
@@ -970,12 +936,11 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
           if (++sq == NASC) { sq = 0; pq ^= 1; }
         }
         if (!kDots && !F::kColScale) {  // res += d * tq
-          const ulonglong2* dv = reinterpret_cast<const ulonglong2*>(smem + MP::OFF_SCL + (sbc & 3) * 512 + half * 256);
 #pragma unroll
-          for (int c4 = 0; c4 < 16; ++c4) {
-            const ulonglong2 dd = dv[c4];
-            ffma2(res2[2 * c4], dd.x, tq2[2 * c4]);
-            ffma2(res2[2 * c4 + 1], dd.y, tq2[2 * c4 + 1]);
+          for (int g = 0; g < 8; ++g) {
+            const unsigned long long dd = *reinterpret_cast<const unsigned long long*>(smem + MP::OFF_SCL + (sbc & 3) * 512 + (cl + 8 * g) * 4);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) ffma2(res2[k][g], dd, tq2[k][g]);
           }
         }
       }
@@ -983,77 +948,57 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
         ok = mbar_wait_warp(bar(MP::D2_FULL), n_item & 1, abort_flag, p.err, p.spin_limit, E_EPI);
         if (ok) {
           tc_fence_after();
-          unsigned long long v[32];
-          tc_ld64_pairs(t_lane + (uint32_t)(ND1 * BN), v);
-          tc_fence_before();
-          mbar_arrive(bar(MP::D2_EMPTY));  // the next item's min term may start
           const unsigned long long one2 = pack2(1.0f);
 #pragma unroll
-          for (int c = 0; c < 32; ++c) ffma2(res2[c], one2, v[c]);
+          for (int hr = 0; hr < 2; ++hr) {
+            unsigned long long v[16];
+            tc_ld_frag64(t_lane + ((uint32_t)(16 * hr) << 16) + (uint32_t)(ND1 * BN), v);
+            if (hr == 1) {
+              tc_fence_before();
+              mbar_arrive_if(bar(MP::D2_EMPTY), lane == 0);  // the next item's min term may start
+            }
+#pragma unroll
+            for (int j = 0; j < 16; ++j) ffma2(res2[2 * hr + (j & 1)][j >> 1], one2, v[j]);
+          }
         }
       }
-      if (!ok || kDots || !row_ok || *abort_flag) continue;
-      const int ncol = min(64, p.N - n0 - half * 64);  // valid columns of this thread (a multiple of 16; <= 0: none)
-      if (ncol <= 0) continue;
+      if (!ok || kDots || *abort_flag) continue;
       if (p.acc == 3) {
         // Gate and up projections in one weight whose rows alternate in groups of 32 (izb_weight_create_gateup): this
-        // thread's 64 columns are 32 gate outputs followed by the 32 up outputs of the same FFN rows, so the SwiGLU product
+        // thread's columns are gate outputs (g < 4) and the up outputs of the same FFN rows (g + 4), so the SwiGLU product
         // up * silu(gate) (zero/kernels/gemm.cl:562-565) is formed in registers and only the F-wide result is stored.
-        float* cp = p.C + (size_t)out_row * p.ldc + p.c_off + (n0 >> 1) + half * 32;
-        const bool wide = ((reinterpret_cast<uintptr_t>(cp) | ((size_t)p.ldc * 4)) & 31) == 0;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          unsigned long long o[4];
+        for (int k = 0; k < 4; ++k) {
+          if (row0 + 8 * k >= nr) break;
+          float* cp = p.C + (size_t)(r0 + row0 + 8 * k) * p.ldc + p.c_off + ((it.nt * BN) >> 1) + half * 32 + 2 * (lane & 3);
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const unsigned long long g2 = res2[4 * j + i], u2 = res2[16 + 4 * j + i];
-            o[i] = pack_pair(swiglu_mul(lo_f(g2), lo_f(u2)), swiglu_mul(hi_f(g2), hi_f(u2)));
-          }
-          if (wide) {
-            asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(cp + 8 * j), "l"(o[0]), "l"(o[1]), "l"(o[2]), "l"(o[3]) : "memory");
-          } else {
-            reinterpret_cast<float4*>(cp + 8 * j)[0] = make_float4(lo_f(o[0]), hi_f(o[0]), lo_f(o[1]), hi_f(o[1]));
-            reinterpret_cast<float4*>(cp + 8 * j)[1] = make_float4(lo_f(o[2]), hi_f(o[2]), lo_f(o[3]), hi_f(o[3]));
+          for (int g = 0; g < 4; ++g) {
+            const unsigned long long g2 = res2[k][g], u2 = res2[k][g + 4];
+            *reinterpret_cast<float2*>(cp + 8 * g) = swiglu_mul2(make_float2(lo_f(g2), hi_f(g2)), make_float2(lo_f(u2), hi_f(u2)));
           }
         }
         continue;
       }
-      float* cp = p.n_split > 1 ? p.part + ((size_t)it.ks * p.M + out_row) * p.N + n0 + half * 64
-                                : p.C + (size_t)out_row * p.ldc + p.c_off + n0 + half * 64;
-      const size_t ld = p.n_split > 1 ? (size_t)p.N : (size_t)p.ldc;
       const int acc = p.acc;
-      const float rs = p.rowscale ? p.rowscale[out_row] : 1.0f;
-      // plain store (with or without the row factor), 32-byte aligned rows: eight stores of one full 32-byte sector each
-      // per thread
-      if (acc == 0 && ncol == 64 && ((reinterpret_cast<uintptr_t>(cp) | (ld * 4)) & 31) == 0) {
-        if (p.rowscale) {
-          const unsigned long long rs2 = pack2(rs);
 #pragma unroll
-          for (int c = 0; c < 32; ++c) res2[c] = fmul2(rs2, res2[c]);
+      for (int k = 0; k < 4; ++k) {
+        const int out_row = r0 + row0 + 8 * k;
+        if (row0 + 8 * k >= nr) break;
+        float* cp = p.n_split > 1 ? p.part + ((size_t)it.ks * p.M + out_row) * p.N + n0 : p.C + (size_t)out_row * p.ldc + p.c_off + n0;
+        const float rs = p.rowscale ? p.rowscale[out_row] : 1.0f;
+        float2 old[8];
+        if (acc != 0) {
+#pragma unroll
+          for (int g = 0; g < 8; ++g) old[g] = n0 + 8 * g < p.N ? *reinterpret_cast<const float2*>(cp + 8 * g) : make_float2(0.0f, 0.0f);
         }
 #pragma unroll
-        for (int c8 = 0; c8 < 8; ++c8)
-          asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(cp + 8 * c8), "l"(res2[4 * c8]), "l"(res2[4 * c8 + 1]),
-                       "l"(res2[4 * c8 + 2]), "l"(res2[4 * c8 + 3])
-                       : "memory");
-      } else {
-#pragma unroll
-        for (int c4 = 0; c4 < 16; ++c4) {
-          if (4 * c4 >= ncol) break;
-          float4 x = make_float4(lo_f(res2[2 * c4]), hi_f(res2[2 * c4]), lo_f(res2[2 * c4 + 1]), hi_f(res2[2 * c4 + 1]));
-          if (p.rowscale) { x.x = __fmul_rn(rs, x.x); x.y = __fmul_rn(rs, x.y); x.z = __fmul_rn(rs, x.z); x.w = __fmul_rn(rs, x.w); }
-          float4* dst = reinterpret_cast<float4*>(cp) + c4;
-          if (acc == 1) {
-            const float4 o = *dst;
-            x.x = __fadd_rn(x.x, o.x); x.y = __fadd_rn(x.y, o.y); x.z = __fadd_rn(x.z, o.z); x.w = __fadd_rn(x.w, o.w);
-          } else if (acc == 2) {  // C holds the gate projection: C = x * silu(C)   (zero/kernels/gemm.cl:562-565)
-            const float4 o = *dst;
-            x.x = swiglu_mul(o.x, x.x);
-            x.y = swiglu_mul(o.y, x.y);
-            x.z = swiglu_mul(o.z, x.z);
-            x.w = swiglu_mul(o.w, x.w);
-          }
-          *dst = x;
+        for (int g = 0; g < 8; ++g) {
+          if (n0 + 8 * g >= p.N) break;
+          float2 y = make_float2(lo_f(res2[k][g]), hi_f(res2[k][g]));
+          if (p.rowscale) y = make_float2(__fmul_rn(rs, y.x), __fmul_rn(rs, y.y));
+          if (acc == 1) y = make_float2(__fadd_rn(y.x, old[g].x), __fadd_rn(y.y, old[g].y));
+          else if (acc == 2) y = swiglu_mul2(old[g], y);  // C holds the gate projection: C = y * silu(C)   (zero/kernels/gemm.cl:562-565)
+          *reinterpret_cast<float2*>(cp + 8 * g) = y;
         }
       }
     }
