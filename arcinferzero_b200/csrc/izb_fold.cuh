@@ -17,6 +17,7 @@ struct FoldParams {
   int ldc, c_off;
   uint32_t* err;
   uint32_t spin_limit;    // polls after which a wait gives up
+  int pdl;                // programmatic dependent launch (csrc/izb_gemm_tc.cu: tc_pdl)
   int skip_stage;         // diagnostics: the unit of the activation ring that its producer leaves out (-1: none)
 };
 

@@ -604,6 +604,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fold_kernel(const __grid_con
     // sits at the final CTA barrier while another lane of the same warp is still working.
     if (warp == 16) {
       // ================= activation producer: the tile's stage images lie back to back in global memory
+      pdl_wait();  // (the pre-pass; the weights depend on no kernel and are on their way by then)
       int sa = 0, pa = 1;
       bool ok = true;
       for (int w = blockIdx.x; w < n_work && ok; w += gridDim.x) {
@@ -629,6 +630,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fold_kernel(const __grid_con
       }
     } else if (warp == 17) {
       // ================= per superblock: row scales and the min term's activation side
+      pdl_wait();
       int sq = 0, pq = 1;
       bool ok = true;
       for (int w = blockIdx.x; w < n_work && ok; w += gridDim.x) {
@@ -776,6 +778,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fold_kernel(const __grid_con
     // ================= combine: a warp holds 32 weight rows (TMEM lanes 32 * (warp % 4) ..) x one or two groups of 32 tokens as fragments (tc_ld_frag2).
     // All f32 arithmetic is done on register pairs (fma.rn.f32x2): half the instructions for the same IEEE results.
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsComb));
+    pdl_wait();  // (C belongs to kernels before this one until they are done)
     const int q = warp & 3, grp = (warp - 8) >> 2;
     const int row0 = 32 * q + (lane >> 2), cl = 2 * (lane & 3);  // this thread's rows row0 + 8 k, k < 4; tokens column(i) + 8 g + cl, + 1
     const uint32_t t_lane = tmem_base + ((uint32_t)(32 * q) << 16);
@@ -851,6 +854,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fold_kernel(const __grid_con
   __syncthreads();
   if (*abort_flag) {
     // a wait gave up: let copies and MMAs still in flight land before shared memory and TMEM are released
+    pdl_wait();  // (the pre-pass clears the flag)
     if (p.n_split > 1 && threadIdx.x == 0) atomicOr(p.part_bad, 1u);
     for (int i = 0; i < 64; ++i) __nanosleep(20000);
     __syncthreads();
@@ -875,7 +879,10 @@ int launch(const izb_weight* w, const FoldParams& p, int grid, cudaStream_t st) 
     return rc;
   CUtensorMap tm;
   memcpy(&tm, w->tmap_raw, sizeof tm);
-  IZB_LAUNCH("gemm_tc", st, gemm_fold_kernel<F><<<grid, kThreads, SMEM_BYTES, st>>>(tm, p));
+  if (p.pdl)
+    IZB_LAUNCH("gemm_tc", st, izb_launch_pdl(gemm_fold_kernel<F>, dim3(grid), dim3(kThreads), SMEM_BYTES, st, tm, p));
+  else
+    IZB_LAUNCH("gemm_tc", st, gemm_fold_kernel<F><<<grid, kThreads, SMEM_BYTES, st>>>(tm, p));
   return IZB_OK;
 }
 

@@ -121,6 +121,7 @@ struct TcParams {
   uint32_t* err;
   uint32_t spin_limit;    // polls after which a wait gives up
   int skip_stage;         // diagnostics: the operand stage the activation producer leaves out (-1: none)
+  int pdl;                // programmatic dependent launch (tc_pdl)
 };
 
 // ---------------------------------------------------------------------------------------------- PTX wrappers
@@ -712,6 +713,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
     // sits at the final CTA barrier while another lane of the same warp is still working.
     if (warp == 0) {
       // ================= activation producer: the tile's stage images lie back to back in global memory
+      pdl_wait();  // (the pre-pass; the weights depend on no kernel and are on their way by then)
       int sa = 0, pa = 1;
       bool ok = true;
       for (int w = blockIdx.x; w < n_work && ok; w += gridDim.x) {
@@ -744,6 +746,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
           if (++rb == NR) { rb = 0; pr ^= 1; }
           if (!kDots) {
             if (!mbar_wait_warp(bar(MP::ASC_EMPTY + sq), pq, abort_flag, p.err, p.spin_limit, E_WPROD)) { ok = false; break; }
+            pdl_wait();  // (the scales are the pre-pass's; the first weights are on their way; later calls return at once)
             if (lane == 0) {
               mbar_expect_tx(bar(MP::ASC_FULL + sq), 4096);
               bulk_g2s(smem_u32(smem + MP::OFF_ASC + sq * 4096), p.ascimg + ((size_t)it.tile * nb + 8 * s) * BM, 4096, bar(MP::ASC_FULL + sq));
@@ -867,6 +870,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
     // ================= combine: a warp holds 32 token rows (TMEM lanes 32 * (warp % 4) ..) x 64 of the 128 columns as fragments (tc_ld_frag64).
     // All f32 arithmetic is done on register pairs (fma.rn.f32x2): half the instructions for the same IEEE results.
     asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
+    pdl_wait();  // (C belongs to kernels before this one until they are done)
     const int q = warp & 3, half = (warp - 8) >> 2;
     const int row0 = 32 * q + (lane >> 2), cl = 64 * half + 2 * (lane & 3);  // this thread's rows row0 + 8 k, k < 4; columns cl + 8 g, + 1, g < 8
     const uint32_t t_lane = tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)(half * 64);
@@ -1008,6 +1012,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
   __syncthreads();
   if (*abort_flag) {
     // a wait gave up: let copies and MMAs still in flight land before shared memory and TMEM are released
+    pdl_wait();  // (the pre-pass clears the flag)
     if (p.n_split > 1 && threadIdx.x == 0) atomicOr(p.part_bad, 1u);
     for (int i = 0; i < 64; ++i) __nanosleep(20000);
     __syncthreads();
@@ -1065,10 +1070,10 @@ int launch_tc(const izb_weight* w, TcParams& p, dim3 grid, cudaStream_t st) {
   p.skip_stage = g_test_skip.exchange(-1);
   CUtensorMap tm;
   memcpy(&tm, w->tmap_raw, sizeof tm);
-  // No programmatic dependent launch, on either side.  CTAs placed while the pre-pass drains land on the SMs in the order in which these
-  // fall free, and neighbouring items, which share operands, no longer run on neighbours (the down projections of 4096 tokens x 8
-  // experts: 392 us against 345); CTAs of the next kernel that wait beside these cost 10 us when it is a wide one.
-  IZB_LAUNCH("gemm_tc", st, gemm_tc_kernel<F, kDots><<<grid, kThreads, SMEM_BYTES, st>>>(tm, p));
+  if (p.pdl)
+    IZB_LAUNCH("gemm_tc", st, izb_launch_pdl(gemm_tc_kernel<F, kDots>, grid, dim3(kThreads), SMEM_BYTES, st, tm, p));
+  else
+    IZB_LAUNCH("gemm_tc", st, gemm_tc_kernel<F, kDots><<<grid, kThreads, SMEM_BYTES, st>>>(tm, p));
   return IZB_OK;
 }
 int launch_tc_of(const izb_weight* w, TcParams& p, dim3 grid, cudaStream_t st) {
@@ -1090,6 +1095,13 @@ int tc_grid(int device, int n_work) {
   const int sms = izb_sm_budget(device);
   return n_work < sms ? (n_work > 0 ? n_work : 1) : sms;
 }
+
+// Programmatic dependent launch behind the pre-pass, for dense calls of one wave: barriers, TMEM and the first weights are there when it ends (us
+// without / with: 37 x 5120 x 5120 Q4_K 22.6/18.9, 18 x 512 x 768 Q6_K 18.6/14.5, 512 x 4096 x 4096 Q8_0 63.6/61.3).  Not for more items: CTAs placed while the
+// pre-pass drains land on the SMs in the order in which these fall free, and neighbouring items, which share operands, no longer run on neighbours
+// (the down projections of 4096 tokens x 8 experts: 392 us against 345).  The GEMM itself lets no kernel in before its end: what waits beside it
+// takes issue slots and power (the first of these calls 21.9, 300 x 5120 x 17408 Q6_K 211 -> 225).
+bool tc_pdl(bool grouped, int grid, int n_work) { return !grouped && n_work <= grid; }
 
 // Parts the K range of every output tile is cut into, when the tiles alone would leave more than half the SMs idle: as many as fill
 // them once, each at least two superblocks.  The parts' sums are at most one 64 KB tile per SM.  The device's SMs count, not the part of them
@@ -1154,8 +1166,9 @@ int run_tc_on(const izb_weight* w, int mat, const int8_t* aq, const float* asc, 
   p.n_split = split_ws && acc == 0 && !tiles && !dots ? tc_split(w->device, n_items, K / 256) : 1;
   p.part = split_ws;
   p.part_bad = split_flag(split_ws, w->device);
-  dim3 grid(tc_grid(w->device, n_items * p.n_split));
-  if (int rc = launch_tc_of(w, p, grid, st)) return rc;
+  const int grid = tc_grid(w->device, n_items * p.n_split);
+  p.pdl = tc_pdl(tiles != nullptr, grid, n_items * p.n_split);
+  if (int rc = launch_tc_of(w, p, dim3(grid), st)) return rc;
   return p.n_split > 1 ? launch_split_reduce(split_ws, p.n_split, M_store, w->N, C, ldc, c_off, p.part_bad, st) : IZB_OK;
 }
 
@@ -1212,7 +1225,9 @@ int run_fold(const izb_weight* w, int mat, const float* x, int ldx, int T, int8_
   const int n_items = (w->N + BN - 1) / BN * p.n_mtiles;
   p.n_split = tc_split(w->device, n_items, w->K / 256);
   if (int rc = x ? izb_fold_quant_prepare(w, x, ldx, T, Mp, aq, asc, p, st) : izb_fold_prepare(w, aq, asc, Mp, Mp, p, st)) return rc;
-  if (int rc = izb_fold_gemm(w, p, tc_grid(w->device, n_items * p.n_split), st)) return rc;
+  const int grid = tc_grid(w->device, n_items * p.n_split);
+  p.pdl = tc_pdl(false, grid, n_items * p.n_split);
+  if (int rc = izb_fold_gemm(w, p, grid, st)) return rc;
   return p.n_split > 1 ? launch_split_reduce(p.part, p.n_split, M_store, w->N, C, ldc, c_off, p.part_bad, st) : IZB_OK;
 }
 
