@@ -98,6 +98,7 @@ struct Acts {
   const f2* sc;
   const f2* ex;
   int qs;
+  f2 neg_zero;  // (-0, -0), from a number that only the launch knows
 };
 
 // ---- weight forms.  prep() expands the headers of a chunk into `hd` ([block][row]); mul() multiplies a chunk into
@@ -297,9 +298,9 @@ struct RQ6K {
             const float2 s = hd[b * 16 + g + 8 * r];
             // (both products and their sum are integers below 2^24: exact)
             const f2 v = f2_fma(f2_of(s.x, s.x), unmagic(d, r), f2_mul(f2_of(s.y, s.y), unmagic(e, r)));
-            // (product and addition on single values: written as packed ones the results differed in their last bits, as of one rounding)
-            const f2 f = f2_mul(xs[4 * b], wd[r]);
-            acc[b][r] = f2_of(__fadd_rn(f2_get(acc[b][r], 0), __fmul_rn(f2_get(f, 0), f2_get(v, 0))), __fadd_rn(f2_get(acc[b][r], 1), __fmul_rn(f2_get(f, 1), f2_get(v, 1))));
+            // the product is rounded before it is added: fma(x, y, -0) with a -0 that the compiler does not know (a packed product and a packed addition
+            // came out as of one rounding, also as a fma with the constant; single values take a seventh more instructions)
+            acc[b][r] = f2_add(acc[b][r], f2_fma(f2_mul(xs[4 * b], wd[r]), v, a.neg_zero));
           }
         }
       }
@@ -418,6 +419,8 @@ __device__ __forceinline__ Acts stage_acts(unsigned char* smem, int K, int T, co
   a.sc = reinterpret_cast<const f2*>(s_sc) + t;
   a.ex = reinterpret_cast<const f2*>(s_ex) + t;
   a.qs = 32 * T;
+  const uint32_t nz = 0x80000000u | (uint32_t)(K >> 31);  // (K > 0)
+  a.neg_zero = (f2)nz << 32 | nz;
   return a;
 }
 
