@@ -18,6 +18,7 @@ int izb_gemv_k16_launch(const izb_weight* w, const uint8_t* raw, const int8_t* a
 int izb_gemv_stream_launch(const izb_weight* w, const uint8_t* raw, const int8_t* aq, const float* asc, int T, int Mp, float* C,
                            int ldc, int c_off, int acc, cudaStream_t st);
 
+bool izb_gemv_stream_fits(const izb_weight* w, int T);
 int izb_rows_launch(const izb_weight* w, int mat, const int8_t* aq, const float* asc, int T, int Mp, float* C, int ldc, int c_off, int acc, cudaStream_t st);
 
 namespace {
@@ -69,29 +70,35 @@ int launch(const izb_weight* w, const uint8_t* raw, const int8_t* aq, const floa
                              : launch_qt<IZB_Q8_0, T>(w, raw, aq, asc, Mp, C, ldc, c_off, acc, st);
 }
 
-// Which of the two ways to the same bits is faster: the matrix instruction's cost does not grow with T, the dot-product kernels' does.
-// Measured (us, matrix instruction / dot products, each behind a quantiser and with weights that are not in L2):
-//   Q6_K  32000 x 4096 T=2 36/39, T=8 38/95; 1024 x 2560 T=2 5.9/7.3, T=5 6.8/8.2; T=1 loses everywhere (28.2/27.4, without the quantiser).
-//         Few row tiles leave most of the chip idle over a long K: 96 x 8192 T=2 9.2/8.4, 48 x 17408 T=2 15.6/12.6, but 128 x 8192 T=5 11/11,
-//         48 x 4096 T=5 7.3/7.9
-//   Q4_K  T >= 4: 3072 x 1536 T=4 4.0/4.3, 1024 x 2048 T=8 4.1/4.2, 34816 x 5120 T=5 34/52, T=8 35/76 (without the quantiser);
-//         T = 3: 8192 x 5376 15/19, 16384 x 8448 34/36; small ones lose (3072 x 1536 3.9/3.8);
-//         T = 2: 12288 x 2304 11/13, 12288 x 5376 18/20, 16384 x 3840 19/17, 16384 x 5376 25/22, 12288 x 8448 33/24, 32000 x 8960 61/50; rows above 9216
-//         take the dot-product kernel a second pass over its ring: 16384 x 9472 37/53, 5120 x 13824 26/36
+// Which of the two ways to the same bits is faster: the matrix instruction's cost does not grow with T but at T = 5, the dot-product kernels' does.
+// Measured (us, matrix instruction / dot products, calls back to back with weights that are not in L2; five rows and more behind a quantiser):
+//   Q6_K  32000 x 4096 T=1 22/27, T=4 24/52, T=8 38/95; 1024 x 1024 T=1 2.3/2.7, 5120 x 17408 T=1 26/27.  Few row tiles leave most of the chip idle
+//         over a long K: 256 x 8192 T=1 5.8/4.9, T=4 6.9/6.4, 256 x 4096 T=1 3.6/3.2, T=2 3.7/3.8, 384 x 8192 T=1 5.8/7.0; 128 x 8192 T=5 11/11, 48 x
+//         4096 T=5 7.3/7.9
+//   Q4_K  rows that are too long for the dot product's ring: 1024 x 10496 T=1 8.0/13, 4096 x 9472 T=1 8.6/8.2 (fits), T=2 9.4/14, 512 x 12544 T=4 10/14;
+//         T = 1 pays in a middle range: 12288 x 2304 7.0/8.3, 12288 x 3328 8.6/11, 16384 x 3840 12/12, 16384 x 8448 23/20, 4096 x 2816 4.4/3.8;
+//         T = 2: 8192 x 3328 6.7/8.1, 4096 x 5376 6.1/6.6, 4096 x 2816 4.5/4.4; T = 3: 4096 x 2816 4.9/5.0, 3072 x 2816 4.7/4.5; T = 4: 2560 x 2816
+//         4.9/5.1, 2048 x 2304 3.9/3.5; T >= 5: 1024 x 2048 T=8 4.1/4.2, 34816 x 5120 T=5 34/52, T=8 35/76
 //         (at up to four rows the kernels for K % 1024 == 0 add in another order: theirs stays)
-//   Q8_0  needs many row tiles (a warp holds half a tile's sums): 1024 x 3072 T=8 6.4/5.0, 2048 x 1024 3.3/3.2, 4096 x 4096 T=3 8.1/7.4,
-//         T=8 8.3/12, 6144 x 1024 T=3 3.6/3.8, T=8 3.9/5.9, 5120 x 5120 T=8 11/17; T <= 2 pays for long K or many short rows:
-//         4096 x 14336 T=1 17.5/22, 32000 x 1024 T=1 8.1/12, 151936 x 2048 T=2 55/60, T=1 54/52, 5120 x 5120 T=2 9.1/8.1
+//   Q8_0  rows that are too long for the ring: 512 x 8192 T=1 7.5/13, T=8 13/21, 1024 x 6144 T=4 7.0/13, 2048 x 5120 T=4 6.7/11; else many row tiles: T = 1 12288 x
+//         2048 5.7/8.0, 151936 x 1024 27/38, 151936 x 2048 51/49, 5120 x 2560 4.4/4.5, 5120 x 5120 7.4/6.8, 4096 x 2048 3.7/3.3; T = 2: 6144 x 4096
+//         6.8/6.8, 8192 x 4096 7.6/8.2, 64000 x 5120 55/53, 5120 x 4096 6.5/6.1; T = 3: 4096 x 4096 6.0/6.4, 3072 x 3072 4.8/4.7; T = 4: 3072 x
+//         1024 2.8/3.0, 2048 x 1024 2.5/2.3; T >= 5 (a warp holds twice the sums): 1024 x 3072 T=8 6.4/5.0, 4096 x 4096 T=8 8.3/12
 bool rows_first(const izb_weight* w, int T) {
-  if (w->type == IZB_K16) return T >= 2 && (w->N >= 128 || w->K < 8192);
-  if (w->type == IZB_Q4_K) {
-    if (T <= 4 && w->K % 1024 == 0 && w->N >= 1024) return false;
-    const bool large = (size_t)w->N * w->row_bytes >= (size_t)12 << 20;
-    if (T == 2) return w->K > 9216 || (large && w->K <= (w->N <= 12288 ? 5376 : 3584));
-    return T >= 4 || (T == 3 && large);
+  const int N = w->N, K = w->K;
+  if (w->type == IZB_K16) return T > 4 ? N >= 128 || K < 8192 : N > 256 || K <= (T == 1 ? 2048 : 4096);
+  if (w->type == IZB_Q4_K && T <= 4 && K % 1024 == 0 && N >= 1024) return false;
+  if (T > 4 && w->type == IZB_Q4_K) return true;
+  if (!izb_gemv_stream_fits(w, T)) return N >= 512;
+  if (w->type == IZB_Q4_K)
+    return T == 1 ? N >= 12288 && K <= 3328 : T == 2 ? (size_t)N * w->row_bytes >= (size_t)12 << 20 : N >= (T == 3 ? 4096 : 2560);
+  switch (T) {
+    case 1: return N >= 5120 && (K <= 1024 || (K <= 2560 && N <= 40960));
+    case 2: return N >= 6144 && (K <= 4096 || N <= 32768);
+    case 3: return N >= 4096;
+    case 4: return N >= 3072;
+    default: return N >= 4096;
   }
-  if (w->N < 4096) return false;
-  return T >= (w->N < 6144 ? 4 : 3) || w->K >= 8192 || (w->N >= 16384 && w->K <= 1024 * T);
 }
 
 }  // namespace

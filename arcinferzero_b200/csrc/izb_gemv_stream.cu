@@ -47,10 +47,10 @@ __device__ __forceinline__ void row_copy(uint32_t dst, const void* src, uint32_t
 }
 
 // warps per CTA (32 with half the ring slots measured slower for every shape but one)
-template <int T> __host__ __device__ constexpr int stream_warps() { return 16; }
+constexpr int kStreamWarps = 16;
 
 template <int QT, int T>
-__global__ void __launch_bounds__(stream_warps<T>() * 32, 1) gemv_stream_kernel(const uint8_t* __restrict__ raw, int N, int K,
+__global__ void __launch_bounds__(kStreamWarps * 32, 1) gemv_stream_kernel(const uint8_t* __restrict__ raw, int N, int K,
                                                                       const int8_t* __restrict__ aq, const float* __restrict__ asc,
                                                                       int Mp, float* __restrict__ C, int ldc, int c_off, int acc,
                                                                       int slots, int slot_bytes, uint32_t* err) {
@@ -58,10 +58,9 @@ __global__ void __launch_bounds__(stream_warps<T>() * 32, 1) gemv_stream_kernel(
   constexpr int SBS = QT == IZB_Q4_K ? 4 : 2;  // superblocks per step
   constexpr int SBB = QT == IZB_Q4_K ? 144 : 272;
   constexpr int STEP = QT == IZB_Q4_K ? kQ4StepBytes : kQ8StepBytes;
-  constexpr int kSWarps = stream_warps<T>();
-  const int nsb = K >> 8, nsteps = (nsb + SBS - 1) / SBS;
+    const int nsb = K >> 8, nsteps = (nsb + SBS - 1) / SBS;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int W = gridDim.x * kSWarps, w0 = blockIdx.x * kSWarps + warp;
+  const int W = gridDim.x * kStreamWarps, w0 = blockIdx.x * kStreamWarps + warp;
   const uint32_t row_bytes = (uint32_t)nsb * SBB;
   const int my_rows = w0 < N ? (N - w0 + W - 1) / W : 0;
   const int sub = QT == IZB_Q4_K ? lane >> 3 : lane >> 4;   // superblock of the step
@@ -70,7 +69,7 @@ __global__ void __launch_bounds__(stream_warps<T>() * 32, 1) gemv_stream_kernel(
   unsigned char* act = smem;
   unsigned char* ring = smem + (((size_t)nsteps * T * STEP + 127) & ~(size_t)127) + (size_t)warp * slots * slot_bytes;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + (((size_t)nsteps * T * STEP + 127) & ~(size_t)127) +
-                                               (size_t)kSWarps * slots * slot_bytes) + warp * slots;
+                                               (size_t)kStreamWarps * slots * slot_bytes) + warp * slots;
   if (lane == 0) {
     for (int s = 0; s < slots; ++s) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(s_u32(&bars[s])) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -827,32 +826,41 @@ int launch_q4k_chunk(const izb_weight* w, const uint8_t* raw, const int8_t* aq, 
   return IZB_OK;
 }
 
+// shared memory of gemv_stream_kernel: the activations, and slots of whole rows per warp (fewer than two: it does not take the call)
+constexpr size_t kStreamBudget = 200 * 1024;
+struct StreamPlan {
+  size_t act;
+  int slots, slot_bytes;
+};
+StreamPlan stream_plan(const izb_weight* w, int T) {
+  const int nsb = w->K / 256, nsteps = w->type == IZB_Q4_K ? (nsb + 3) / 4 : (nsb + 1) / 2;
+  StreamPlan p = {((size_t)nsteps * T * (w->type == IZB_Q4_K ? kQ4StepBytes : kQ8StepBytes) + 127) & ~(size_t)127, 0, (int)((w->row_bytes + 127) & ~(size_t)127)};
+  if (p.act + 4096 < kStreamBudget) p.slots = (int)((kStreamBudget - p.act - 4096) / ((size_t)kStreamWarps * p.slot_bytes));
+  if (p.slots > 8) p.slots = 8;
+  return p;
+}
+
 template <int QT, int T>
 int launch_stream(const izb_weight* w, const uint8_t* raw, const int8_t* aq, const float* asc, int Mp, float* C, int ldc,
                   int c_off, int acc, cudaStream_t st) {
-  constexpr int STEP = QT == IZB_Q4_K ? kQ4StepBytes : kQ8StepBytes;
-  constexpr size_t kBudget = 200 * 1024;
-  constexpr int kSWarps = stream_warps<T>();
-  const int nsb = w->K / 256, nsteps = QT == IZB_Q4_K ? (nsb + 3) / 4 : (nsb + 1) / 2;
-  const size_t act = ((size_t)nsteps * T * STEP + 127) & ~(size_t)127;
-  const int slot_bytes = (int)((w->row_bytes + 127) & ~(size_t)127);
-  if (act + 4096 >= kBudget) return 1;
-  int slots = (int)((kBudget - act - 4096) / ((size_t)kSWarps * slot_bytes));
-  if (slots < 2) return 1;  // (rows too long for a ring: the chunked kernel takes the call)
-  if (slots > 8) slots = 8;
-  const size_t smem = act + (size_t)kSWarps * slots * slot_bytes + (size_t)kSWarps * slots * 8;
-  IZB_SMEM_OPTIN((gemv_stream_kernel<QT, T>), kBudget + 8192, w->device);
+  const StreamPlan p = stream_plan(w, T);
+  if (p.slots < 2) return 1;  // (rows too long for a ring: the chunked kernel takes the call)
+  const size_t smem = p.act + (size_t)kStreamWarps * p.slots * (p.slot_bytes + 8);
+  IZB_SMEM_OPTIN((gemv_stream_kernel<QT, T>), kStreamBudget + 8192, w->device);
   const int sms = izb_sm_count(w->device);
   int grid = sms;
-  const int need = (w->N + kSWarps - 1) / kSWarps;
+  const int need = (w->N + kStreamWarps - 1) / kStreamWarps;
   if (grid > need) grid = need;
   uint32_t* err = izb_device_error_word(w->device);
   if (!err) IZB_FAIL(IZB_ERR_NOMEM, "gemv: no device error word");
-  IZB_LAUNCH("gemv", st, izb_launch_pdl(gemv_stream_kernel<QT, T>, grid, kSWarps * 32, smem, st, raw, w->N, w->K, aq, asc, Mp, C, ldc, c_off, acc, slots, slot_bytes, err));
+  IZB_LAUNCH("gemv", st, izb_launch_pdl(gemv_stream_kernel<QT, T>, grid, kStreamWarps * 32, smem, st, raw, w->N, w->K, aq, asc, Mp, C, ldc, c_off, acc, p.slots, p.slot_bytes, err));
   return IZB_OK;
 }
 
 }  // namespace
+
+// rings of whole rows fit (Q4_K, Q8_0: else izb_gemv.cu's kernel takes what no other kernel here does)
+bool izb_gemv_stream_fits(const izb_weight* w, int T) { return stream_plan(w, T).slots >= 2; }
 
 // +1: the shared-memory plan does not fit (the chunked kernel of izb_gemv.cu takes the call)
 template <int T>

@@ -28,8 +28,15 @@
 // a tile, so that neighbouring superblocks of the same rows are in flight together: rings of scattered tiles ran at half the
 // DRAM rate.  The ring's first fill is issued before pdl_wait() (no kernel writes weights).
 //
-// Measured (us, dot-product kernels before / now; the time at the copy's bandwidth): Q4_K 34816 x 5120 five rows 52.3 / 34.4 (15.3), eight
-// 75.7 / 35.1; 128000 x 4096 eight 218 / 89 (45); Q8_0 151936 x 2048 eight 136 / 57 (51); Q6_K 32000 x 4096 three 44 / 29 (17).  The
+// Up to four tokens would leave half of the instruction's columns empty, and with them half of every lane's f32 work.  There one instruction
+// takes 32 elements, two pieces: columns 0-3 are the tokens with zeros for the second piece, columns 4-7 the same tokens with zeros for
+// the first, so that each lane has half of the pieces and all of its work counts (mul4; the K = 32 instruction takes the tensor pipe's 8 clk like
+// the K = 16 one).  The sums are the same and in the same order; half as many accumulators also halve what the warps of a tile exchange.
+// (us before / now: Q6_K 151936 x 5120 three rows 149 / 118, 32000 x 4096 three 30 / 24; Q4_K 16384 x 5376 three 20.8 / 16.5, 5120 x 13824 four 27 /
+// 19; Q8_0 4096 x 14336 one 17.2 / 13.2, 8192 x 4096 four 8.8 / 7.8.)
+//
+// Measured (us, dot-product kernels / this one; the time at the copy's bandwidth): Q4_K 34816 x 5120 five rows 52.3 / 34.4 (15.3), eight
+// 75.7 / 35.1; 128000 x 4096 eight 218 / 89 (45); Q8_0 151936 x 2048 eight 136 / 57 (51); Q6_K 32000 x 4096 three 44 / 24 (17).  The
 // Q4_K case is bound by instruction issue (56 % of the cycles) and shared-memory latency: about 450 warp instructions per chunk, of
 // which 128 are the 32 partial sums' f32 work that the other kernels' order asks for.
 #include <cuda.h>
@@ -51,6 +58,19 @@ __device__ __forceinline__ void dot16_s8(int (&d)[4], uint32_t w0, uint32_t w1, 
   asm("mma.sync.aligned.m16n8k16.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%7,%7};"
       : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
       : "r"(w0), "r"(w1), "r"(x), "r"(kMagic));
+}
+
+// The same with up to four tokens: 32 elements, of which columns 0-3 meet the first 16 (their words of the other 16 are zero) and
+// columns 4-7, the same tokens again, the last 16.
+__device__ __forceinline__ void dot32_u8(int (&d)[4], uint32_t w0, uint32_t w1, uint32_t v0, uint32_t v1, uint32_t x, uint32_t y, uint32_t c0 = kMagic, uint32_t c1 = kMagic) {
+  asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%10,%11};"
+      : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+      : "r"(w0), "r"(w1), "r"(v0), "r"(v1), "r"(x), "r"(y), "r"(c0), "r"(c1));
+}
+__device__ __forceinline__ void dot32_s8(int (&d)[4], uint32_t w0, uint32_t w1, uint32_t v0, uint32_t v1, uint32_t x, uint32_t y) {
+  asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+      : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+      : "r"(w0), "r"(w1), "r"(v0), "r"(v1), "r"(x), "r"(y), "r"(kMagic));
 }
 
 // f32 pairs (tokens 2t, 2t + 1): two IEEE operations per instruction
@@ -93,16 +113,19 @@ __device__ __forceinline__ float byte_f(uint32_t w, int k) { return __fsub_rn(__
 //   q   token g: words of the first and second 16 elements of a block, `qs` bytes per block
 //   sc  scales of tokens 2t, 2t + 1, four pairs per block
 //   ex  per block and half, four pairs: Q4_K the sum of the 16 values as f32; Q6_K the accumulator's start, kMagic - 32 * that sum
+// For mul4 token g % 4, tokens 2 (t % 2), + 1, and of two pieces the one that the column meets.
 struct Acts {
   const unsigned char* q;
   const f2* sc;
   const f2* ex;
   int qs;
   f2 neg_zero;  // (-0, -0), from a number that only the launch knows
+  uint32_t first, last;  // mul4: masks, all ones in lanes whose column g meets the first / the last 16 elements
 };
 
 // ---- weight forms.  prep() expands the headers of a chunk into `hd` ([block][row]); mul() multiplies a chunk into
-// the piece sums acc[piece][r]: rows g, g + 8 against tokens 2t, 2t + 1
+// the piece sums acc[piece][r]: rows g, g + 8 against tokens 2t, 2t + 1.  mul4(), for up to four tokens: rows g, g + 8 against tokens
+// 2 (t % 2), + 1, and the half of the pieces whose number has t / 2 at bit kLaneBit.
 struct RQ4K {
   static constexpr int SBB = 144, kPitch = 144, kSubs = 4, kPieces = 8, kDotWarps = 16;
   static constexpr bool kEx = true, kPrep = true;
@@ -187,6 +210,29 @@ struct RQ4K {
       }
     }
   }
+  // lane's pieces: 2c + t / 2
+  static constexpr int kLaneBit = 0;
+  static __device__ __forceinline__ void mul4(const unsigned char* chunk, const float2* hd, const Acts& a, int sb, int g, int t, f2 (&acc)[kPieces / 2][2]) {
+    const unsigned char* p = chunk + g * kPitch + 16 + 4 * t;
+    const unsigned char* xq = a.q + 8 * sb * a.qs;
+    const f2 *xs = a.sc + 32 * sb, *xe = a.ex + 64 * sb;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const uint32_t xl = *reinterpret_cast<const uint32_t*>(xq + 2 * c * a.qs), xh = *reinterpret_cast<const uint32_t*>(xq + (2 * c + 1) * a.qs);
+      const f2 sl = xs[8 * c], sh = xs[8 * c + 4], el = xe[16 * c], eh = xe[16 * c + 8];
+      const uint32_t w0 = *reinterpret_cast<const uint32_t*>(p + 32 * c), w1 = *reinterpret_cast<const uint32_t*>(p + 8 * kPitch + 32 * c);
+      const uint32_t v0 = *reinterpret_cast<const uint32_t*>(p + 32 * c + 16), v1 = *reinterpret_cast<const uint32_t*>(p + 8 * kPitch + 32 * c + 16);
+      int dl[4], dh[4];
+      dot32_u8(dl, w0 & 0x0F0F0F0Fu, w1 & 0x0F0F0F0Fu, v0 & 0x0F0F0F0Fu, v1 & 0x0F0F0F0Fu, xl & a.first, xl & a.last);
+      dot32_u8(dh, w0 & 0xF0F0F0F0u, w1 & 0xF0F0F0F0u, v0 & 0xF0F0F0F0u, v1 & 0xF0F0F0F0u, xh & a.first, xh & a.last);
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const float2 u = hd[2 * c * 16 + g + 8 * r], v = hd[(2 * c + 1) * 16 + g + 8 * r];
+        const f2 P = f2_fma(f2_of(u.x, u.x), unmagic(dl, r), f2_mul(f2_of(u.y, u.y), el)), Q = f2_fma(f2_of(v.x, v.x), unmagic(dh, r), f2_mul(f2_of(v.y, v.y), eh));
+        acc[c][r] = f2_add(acc[c][r], f2_fma(sl, P, f2_mul(sh, Q)));
+      }
+    }
+  }
 };
 
 struct RQ80 {
@@ -240,6 +286,28 @@ struct RQ80 {
         dot16_s8(d, *reinterpret_cast<const uint32_t*>(p + 32 * b + 16 * h), *reinterpret_cast<const uint32_t*>(p + 8 * kPitch + 32 * b + 16 * h), h ? x.y : x.x);
 #pragma unroll
         for (int r = 0; r < 2; ++r) acc[2 * b + h][r] = f2_fma(sd[r], unmagic(d, r), acc[2 * b + h][r]);
+      }
+    }
+  }
+  // lane's pieces: 2b + t / 2
+  static constexpr int kLaneBit = 0;
+  static __device__ __forceinline__ void mul4(const unsigned char* chunk, const float2*, const Acts& a, int sb, int g, int t, f2 (&acc)[kPieces / 2][2]) {
+    const unsigned char* p = chunk + g * kPitch;
+    const uint4 hd[2] = {*reinterpret_cast<const uint4*>(p), *reinterpret_cast<const uint4*>(p + 8 * kPitch)};
+    p += 16 + 4 * t;
+    const unsigned char* xq = a.q + 8 * sb * a.qs;
+    const f2* xs = a.sc + 32 * sb;
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+      const uint32_t x = *reinterpret_cast<const uint32_t*>(xq + b * a.qs);
+      int d[4];
+      dot32_s8(d, *reinterpret_cast<const uint32_t*>(p + 32 * b), *reinterpret_cast<const uint32_t*>(p + 8 * kPitch + 32 * b), *reinterpret_cast<const uint32_t*>(p + 32 * b + 16),
+               *reinterpret_cast<const uint32_t*>(p + 8 * kPitch + 32 * b + 16), x & a.first, x & a.last);
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const uint32_t w = (b >> 1) == 0 ? hd[r].x : (b >> 1) == 1 ? hd[r].y : (b >> 1) == 2 ? hd[r].z : hd[r].w;
+        const float s = half_bits_to_float((b & 1) ? w >> 16 : w & 0xFFFFu);
+        acc[b][r] = f2_fma(f2_mul(xs[4 * b], f2_of(s, s)), unmagic(d, r), acc[b][r]);
       }
     }
   }
@@ -306,6 +374,45 @@ struct RQ6K {
       }
     }
   }
+  // lane's pieces, the blocks of a superblock: 4 nh + lo + 2 (t / 2)
+  static constexpr int kLaneBit = 1;
+  static __device__ __forceinline__ void mul4(const unsigned char* chunk, const float2* hd, const Acts& a, int sb, int g, int t, f2 (&acc)[kPieces / 2][2]) {
+    const unsigned char* p = chunk + g * kPitch;
+    const float d0 = half_bits_to_float(*reinterpret_cast<const unsigned short*>(p + 208)), d1 = half_bits_to_float(*reinterpret_cast<const unsigned short*>(p + 8 * kPitch + 208));
+    const f2 wd[2] = {f2_of(d0, d0), f2_of(d1, d1)};
+    p += 4 * t;
+    const unsigned char* xq = a.q + 8 * sb * a.qs;
+    const f2 *xs = a.sc + 32 * sb, *xe = a.ex + 64 * sb;
+    hd += (t >> 1) * 32 + g;
+#pragma unroll
+    for (int nh = 0; nh < 2; ++nh) {
+      uint32_t hq[2][2];
+#pragma unroll
+      for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) hq[r][i] = *reinterpret_cast<const uint32_t*>(p + 8 * r * kPitch + 128 + 32 * nh + 16 * i);
+#pragma unroll
+      for (int lo = 0; lo < 2; ++lo) {  // sub-blocks lo and lo + 2 share their low-nibble bytes
+        const int b = 4 * nh + lo;
+        const uint2 x = *reinterpret_cast<const uint2*>(xq + b * a.qs), c0 = *reinterpret_cast<const uint2*>(xe + 8 * b), c1 = *reinterpret_cast<const uint2*>(xe + 8 * b + 4);
+        int d[2][4];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          uint32_t l[2];
+#pragma unroll
+          for (int r = 0; r < 2; ++r) l[r] = *reinterpret_cast<const uint32_t*>(p + 8 * r * kPitch + 64 * nh + 32 * lo + 16 * i);
+          const uint32_t v = i ? x.y : x.x;
+          dot32_u8(d[i], word(l[0], hq[0][i], lo), word(l[1], hq[1][i], lo), word(l[0], hq[0][i], lo + 2), word(l[1], hq[1][i], lo + 2), v & a.first, v & a.last, i ? c1.x : c0.x, i ? c1.y : c0.y);
+        }
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const float2 s = hd[b * 16 + 8 * r];
+          const f2 v = f2_fma(f2_of(s.x, s.x), unmagic(d[0], r), f2_mul(f2_of(s.y, s.y), unmagic(d[1], r)));
+          acc[2 * nh + lo][r] = f2_add(acc[2 * nh + lo][r], f2_fma(f2_mul(xs[4 * b], wd[r]), v, a.neg_zero));  // (see mul)
+        }
+      }
+    }
+  }
 };
 
 // ---- a warp's ring of chunks (16 rows x one superblock each), filled by TMA
@@ -358,18 +465,19 @@ struct Ring {
   }
 };
 
-// ---- shared memory: activations | rings | 4 KB per warp (expanded headers, exchanged sums) | barriers
+// ---- shared memory: activations | rings | 4 KB per warp, 2 KB with half the sums (expanded headers, exchanged sums) | barriers
 template <class F>
 __host__ __device__ __forceinline__ size_t act_bytes(int K, int T) { return ((size_t)(K / 32) * (32 * T + 32 + (F::kEx ? 64 : 0)) + 127) & ~(size_t)127; }
-constexpr int kXch = 4096;
-template <class F>
+template <bool kFour>
+constexpr int kXch = kFour ? 2048 : 4096;
+template <class F, bool kFour>
 __host__ __device__ __forceinline__ size_t rows_smem(int K, int T, int nw, int slots) {
-  return act_bytes<F>(K, T) + (size_t)nw * (slots * (Ring<F>::kSlot + 8) + kXch);
+  return act_bytes<F>(K, T) + (size_t)nw * (slots * (Ring<F>::kSlot + 8) + kXch<kFour>);
 }
 
 // Activations of T tokens (rows `src(j)` of aq, columns of asc), as Acts describes them.  Four items per thread and pass, so that their
 // loads are in flight together.
-template <class F, class Src>
+template <class F, bool kFour, class Src>
 __device__ __forceinline__ Acts stage_acts(unsigned char* smem, int K, int T, const int8_t* __restrict__ aq, const float* __restrict__ asc, int Mp, int g, int t, Src src) {
   const int nb = K / 32, items = nb * T;
   float* s_sc = reinterpret_cast<float*>(smem + (size_t)nb * 32 * T);
@@ -415,21 +523,33 @@ __device__ __forceinline__ Acts stage_acts(unsigned char* smem, int K, int T, co
     }
   }
   Acts a;
-  a.q = smem + min(g, T - 1) * 32 + 8 * t;  // (lanes past the last token repeat it; their results are not stored)
-  a.sc = reinterpret_cast<const f2*>(s_sc) + t;
-  a.ex = reinterpret_cast<const f2*>(s_ex) + t;
   a.qs = 32 * T;
+  a.first = g < 4 ? 0xFFFFFFFFu : 0u;
+  a.last = ~a.first;
+  a.q = smem + min(kFour ? g & 3 : g, T - 1) * 32 + 8 * t;  // (lanes past the last token repeat it; their results are not stored)
+  a.sc = reinterpret_cast<const f2*>(s_sc) + (kFour ? t & 1 : t);
+  a.ex = reinterpret_cast<const f2*>(s_ex) + (kFour ? t & 1 : t);
+  if (kFour && F::kLaneBit == 0) {  // columns 4-7: the second half of a block
+    a.q += 4 * (g >> 2);
+    a.ex += 4 * (t >> 1);
+  } else if (kFour) {  // ... the block after the next
+    a.q += 2 * a.qs * (g >> 2);
+    a.sc += 8 * (t >> 1);
+    a.ex += 16 * (t >> 1);
+  }
   const uint32_t nz = 0x80000000u | (uint32_t)(K >> 31);  // (K > 0)
   a.neg_zero = (f2)nz << 32 | nz;
   return a;
 }
 
 // One chunk after the other of this warp's share of a tile (superblocks part, part + kSubs, ...) into acc.  false: a wait ran out.
-template <class F, class Request>
-__device__ __forceinline__ bool accumulate(Ring<F>& ring, float2* hd, const Acts& acts, int part, int nsb, int lane, f2 (&acc)[F::kPieces][2], Request request) {
+template <class F, bool kFour>
+constexpr int kLanePieces = kFour ? F::kPieces / 2 : F::kPieces;
+template <class F, bool kFour, class Request>
+__device__ __forceinline__ bool accumulate(Ring<F>& ring, float2* hd, const Acts& acts, int part, int nsb, int lane, f2 (&acc)[kLanePieces<F, kFour>][2], Request request) {
   const int g = lane >> 2, t = lane & 3;
 #pragma unroll
-  for (int p = 0; p < F::kPieces; ++p) acc[p][0] = acc[p][1] = 0ull;
+  for (int p = 0; p < kLanePieces<F, kFour>; ++p) acc[p][0] = acc[p][1] = 0ull;
   for (int s = part; s < nsb; s += F::kSubs) {
     const unsigned char* chunk = ring.wait();
     if (!chunk) {
@@ -440,7 +560,8 @@ __device__ __forceinline__ bool accumulate(Ring<F>& ring, float2* hd, const Acts
       F::prep(chunk, hd, lane);
       __syncwarp();
     }
-    F::mul(chunk, hd, acts, s, g, t, acc);
+    if constexpr (kFour) F::mul4(chunk, hd, acts, s, g, t, acc);
+    else F::mul(chunk, hd, acts, s, g, t, acc);
     __syncwarp();  // every lane has read the chunk: its slot takes the next request
     ring.next();
     request();
@@ -448,23 +569,37 @@ __device__ __forceinline__ bool accumulate(Ring<F>& ring, float2* hd, const Acts
   return true;
 }
 
+// the pieces of a lane into acc[0], pairs `H` apart and then nearer ones (mul4: the step over the bit kLaneBit is between lanes)
+template <class F, bool kFour, int H>
+__device__ __forceinline__ void fold_pieces(f2 (&acc)[kLanePieces<F, kFour>][2]) {
+  constexpr bool kLanes = kFour && H == 1 << F::kLaneBit;
+  constexpr int kHave = kFour && H >= 1 << F::kLaneBit ? H : 2 * H, kLeft = kLanes ? kHave : kHave / 2;  // the lane's pieces before and after
+#pragma unroll
+  for (int p = 0; p < kLeft; ++p)
+#pragma unroll
+    for (int r = 0; r < 2; ++r) acc[p][r] = f2_add(acc[p][r], kLanes ? __shfl_xor_sync(0xFFFFFFFFu, acc[p][r], 2) : acc[p + kLeft][r]);
+  if constexpr (H > 1) fold_pieces<F, kFour, H / 2>(acc);
+}
+
 // The tree over a tile's 32 partial sums per output: superblock parts p, p ^ 2, then p ^ 1 (through shared memory: parts 2 and 3
 // hand theirs to 0 and 1, part 1 to 0), then the pieces halves first.  All warps of a tile call it (a named barrier per tile: the
 // tiles of a CTA need not keep step); the result is valid in part 0.  `xch`: this CTA's exchange areas, one per warp.
 template <class F>
 __device__ __forceinline__ void tile_sync(int mine) { asm volatile("bar.sync %0, %1;" ::"r"(1 + mine), "n"(F::kSubs * 32) : "memory"); }
-template <class F>
-__device__ __forceinline__ void reduce_tile(f2 (&acc)[F::kPieces][2], unsigned char* xch, int warp, int lane) {
+// (mul4: lanes t and t + 2 both have the result.)
+template <class F, bool kFour>
+__device__ __forceinline__ void reduce_tile(f2 (&acc)[kLanePieces<F, kFour>][2], unsigned char* xch, int warp, int lane) {
+  constexpr int kMine = kLanePieces<F, kFour>;
   static_assert(F::kSubs == 4 ? F::kPieces == 8 : F::kSubs == 2 && F::kPieces == 16, "exchange areas: 4 KB per warp");
   const int part = warp % F::kSubs, mine = warp / F::kSubs;
-  auto area = [&](int w) { return reinterpret_cast<ulonglong2*>(xch + (size_t)w * kXch) + lane; };  // [piece][lane] of 16 bytes
+  auto area = [&](int w) { return reinterpret_cast<ulonglong2*>(xch + (size_t)w * kXch<kFour>) + lane; };  // [piece][lane] of 16 bytes
   auto give = [&](int w) {
 #pragma unroll
-    for (int p = 0; p < F::kPieces; ++p) area(w)[32 * p] = make_ulonglong2(acc[p][0], acc[p][1]);
+    for (int p = 0; p < kMine; ++p) area(w)[32 * p] = make_ulonglong2(acc[p][0], acc[p][1]);
   };
   auto take = [&](int w) {
 #pragma unroll
-    for (int p = 0; p < F::kPieces; ++p) {
+    for (int p = 0; p < kMine; ++p) {
       const ulonglong2 v = area(w)[32 * p];
       acc[p][0] = f2_add(acc[p][0], v.x);
       acc[p][1] = f2_add(acc[p][1], v.y);
@@ -484,16 +619,11 @@ __device__ __forceinline__ void reduce_tile(f2 (&acc)[F::kPieces][2], unsigned c
     if (part == 0) take(warp);
     tile_sync<F>(mine);
   }
-#pragma unroll
-  for (int h = F::kPieces / 2; h > 0; h >>= 1)
-#pragma unroll
-    for (int p = 0; p < h; ++p)
-#pragma unroll
-      for (int r = 0; r < 2; ++r) acc[p][r] = f2_add(acc[p][r], acc[p + h][r]);
+  fold_pieces<F, kFour, F::kPieces / 2>(acc);
 }
 
 // C[token][c_off + row] (= or +=) for T tokens.  The grid walks groups of (warps / kSubs) row tiles.
-template <class F>
+template <class F, bool kFour>
 __global__ void __launch_bounds__(512, 1) rows_kernel(const __grid_constant__ CUtensorMap tm, int wrow0, int N, int K, const int8_t* __restrict__ aq,
                                                       const float* __restrict__ asc, int T, int Mp, float* __restrict__ C, int ldc, int c_off, int acc_mode, int slots,
                                                       uint32_t* err) {
@@ -506,7 +636,7 @@ __global__ void __launch_bounds__(512, 1) rows_kernel(const __grid_constant__ CU
   Ring<F> ring;
   ring.slots = slots;
   ring.base = rings + (size_t)warp * slots * Ring<F>::kSlot;
-  ring.bars = reinterpret_cast<uint64_t*>(xch + NW * kXch) + warp * slots;
+  ring.bars = reinterpret_cast<uint64_t*>(xch + NW * kXch<kFour>) + warp * slots;
   __shared__ int s_gave_up;
   volatile int* gave_up = &s_gave_up;
   if (threadIdx.x == 0) s_gave_up = 0;
@@ -521,21 +651,22 @@ __global__ void __launch_bounds__(512, 1) rows_kernel(const __grid_constant__ CU
   for (int s = 0; s < slots; ++s) request();
   pdl_launch_next();
   pdl_wait();
-  const Acts acts = stage_acts<F>(smem, K, T, aq, asc, Mp, g, t, [](int j) { return j; });
+  const Acts acts = stage_acts<F, kFour>(smem, K, T, aq, asc, Mp, g, t, [](int j) { return j; });
   __syncthreads();
   bool ok = true;
   for (int gr = blockIdx.x; gr < groups; gr += gridDim.x) {
-    f2 acc[F::kPieces][2];
-    if (ok) ok = accumulate<F>(ring, reinterpret_cast<float2*>(xch + (size_t)warp * kXch), acts, part, nsb, lane, acc, request);
+    f2 acc[kLanePieces<F, kFour>][2];
+    if (ok) ok = accumulate<F, kFour>(ring, reinterpret_cast<float2*>(xch + (size_t)warp * kXch<kFour>), acts, part, nsb, lane, acc, request);
     if (!ok) {  // (bounded wait gave up: nothing of this CTA is stored any more)
       if (lane == 0) atomicOr(err, 64u);
       *gave_up = 1;
     }
-    reduce_tile<F>(acc, xch, warp, lane);
+    reduce_tile<F, kFour>(acc, xch, warp, lane);
     if (part == 0 && !*gave_up) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const int row = (gr * kPer + mine) * 16 + g + 8 * (i >> 1), tok = 2 * t + (i & 1);
+        const int row = (gr * kPer + mine) * 16 + g + 8 * (i >> 1), tok = 2 * (kFour ? t & 1 : t) + (i & 1);
+        if (kFour && (t >> 1) != i >> 1) continue;  // (both pairs of lanes have the sums: one stores rows g, the other g + 8)
         if (row < N && tok < T) {
           float* c = C + (size_t)tok * ldc + c_off + row;
           const float v = f2_get(acc[0][i >> 1], i & 1);
@@ -633,7 +764,7 @@ __device__ __noinline__ void moe_fine(const CUtensorMap& tg, const CUtensorMap& 
   Ring<F> ring;
   ring.slots = slots;
   ring.base = rings + (size_t)warp * slots * Ring<F>::kSlot;
-  ring.bars = reinterpret_cast<uint64_t*>(xch + NW * kXch) + warp * slots;
+  ring.bars = reinterpret_cast<uint64_t*>(xch + NW * kXch<false>) + warp * slots;
   const int row = tiles[1 + 3 * ti] * N + row_tile * 16, s0 = tiles[2 + 3 * ti], T = tiles[3 + 3 * ti];
   int pm = 0, ps = part;
   auto request = [&]() {
@@ -642,18 +773,18 @@ __device__ __noinline__ void moe_fine(const CUtensorMap& tg, const CUtensorMap& 
     if ((ps += F::kSubs) >= nsb) { ps = part; ++pm; }
   };
   for (int s = 0; s < slots; ++s) request();
-  const Acts acts = stage_acts<F>(smem, K, T, aq, asc, Mp, g, t, [&](int j) { return stok ? stok[s0 + j] : s0 + j; });
+  const Acts acts = stage_acts<F, false>(smem, K, T, aq, asc, Mp, g, t, [&](int j) { return stok ? stok[s0 + j] : s0 + j; });
   __syncthreads();
   bool ok = true;
   float first[4];
   for (int m = 0; m <= pair; ++m) {
     f2 acc[F::kPieces][2];
-    if (ok) ok = accumulate<F>(ring, reinterpret_cast<float2*>(xch + (size_t)warp * kXch), acts, part, nsb, lane, acc, request);
+    if (ok) ok = accumulate<F, false>(ring, reinterpret_cast<float2*>(xch + (size_t)warp * kXch<false>), acts, part, nsb, lane, acc, request);
     if (!ok) {
       if (lane == 0) atomicOr(err, 64u);
       *gave_up = 1;
     }
-    reduce_tile<F>(acc, xch, warp, lane);
+    reduce_tile<F, false>(acc, xch, warp, lane);
     if (part != 0 || *gave_up) continue;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -677,7 +808,7 @@ __global__ void __launch_bounds__(kMoeWarps * 32, kMoeCtas) moe_rows_kernel(cons
   Ring<F> ring;
   ring.slots = slots;
   ring.base = rings + (size_t)warp * slots * Ring<F>::kSlot;
-  ring.bars = reinterpret_cast<uint64_t*>(xch + NW * kXch) + warp * slots;
+  ring.bars = reinterpret_cast<uint64_t*>(xch + NW * kXch<false>) + warp * slots;
   __shared__ int s_gave_up;
   volatile int* gave_up = &s_gave_up;
   if (threadIdx.x == 0) s_gave_up = 0;
@@ -750,7 +881,7 @@ __global__ void __launch_bounds__(kMoeWarps * 32, kMoeCtas) moe_rows_kernel(cons
       }
       s0 = tiles[2 + 3 * ti];
       T = tiles[3 + 3 * ti];
-      acts = stage_acts<F>(smem, K, T, aq, asc, Mp, g, t, [&](int j) { return stok ? stok[s0 + j] : s0 + j; });
+      acts = stage_acts<F, false>(smem, K, T, aq, asc, Mp, g, t, [&](int j) { return stok ? stok[s0 + j] : s0 + j; });
       __syncthreads();
     }
     const int tile0 = gi * NW;
@@ -773,9 +904,9 @@ __global__ void __launch_bounds__(kMoeWarps * 32, kMoeCtas) moe_rows_kernel(cons
       float first[4];
       for (int m = 0; m <= pair; ++m) {
         f2 acc[F::kPieces][2];
-        if (ok) ok = accumulate<F>(ring, reinterpret_cast<float2*>(xch + (size_t)warp * kXch), acts, part, nsb, lane, acc, request);
+        if (ok) ok = accumulate<F, false>(ring, reinterpret_cast<float2*>(xch + (size_t)warp * kXch<false>), acts, part, nsb, lane, acc, request);
         if (!ok) note();
-        reduce_tile<F>(acc, xch, warp, lane);
+        reduce_tile<F, false>(acc, xch, warp, lane);
         if (m < pair) {
 #pragma unroll
           for (int i = 0; i < 4; ++i) first[i] = f2_get(acc[0][i >> 1], i & 1);
@@ -798,7 +929,7 @@ constexpr size_t kSmemPerSm = 226 * 1024;
 struct Split {
   int warps, ctas, slots;  // slots 0: the activations leave no room
 };
-template <class F>
+template <class F, bool kFour>
 Split pick_split(int K, int T, int tiles, int sms) {
   Split best = {0, 0, 0};
   double most = 0;
@@ -807,7 +938,7 @@ Split pick_split(int K, int T, int tiles, int sms) {
     for (int c = 1; c * nw <= 16; ++c) {
       const size_t room = kSmemPerSm / c - (c > 1 ? 1024 : 0);
       int slots = 4;
-      while (slots >= 2 && rows_smem<F>(K, T, nw, slots) > room) --slots;
+      while (slots >= 2 && rows_smem<F, kFour>(K, T, nw, slots) > room) --slots;
       if (slots < 2) break;
       const int rounds = (groups + c * sms - 1) / (c * sms);
       const double at_work = (double)tiles * F::kSubs * (slots + 1) / rounds;
@@ -820,26 +951,26 @@ Split pick_split(int K, int T, int tiles, int sms) {
   return best;
 }
 
-template <class F>
+template <class F, bool kFour>
 int rows_of(const izb_weight* w, int mat, const int8_t* aq, const float* asc, int T, int Mp, float* C, int ldc, int c_off, int acc, cudaStream_t st) {
   const int sms = izb_sm_count(w->device), tiles = (w->N + 15) / 16;
-  const Split sp = pick_split<F>(w->K, T, tiles, sms);
+  const Split sp = pick_split<F, kFour>(w->K, T, tiles, sms);
   // Half the tokens at a time, the second pass finding part of the weights in L2; not where the dot-product kernel's warps (kDotWarps per SM)
   // take every row in one round (us, halves / dot products, eight rows of 17408 Q6_K: 1024 rows 34/28, 1280 rows 34/42; of 18944 Q4_K:
   // 2304 rows 35/33, 2560 rows 45/60).
   if (!sp.slots) {
     if (T < 2 || w->N <= F::kDotWarps * sms) return 1;
     const int h = (T + 1) / 2;
-    if (const int rc = rows_of<F>(w, mat, aq, asc, h, Mp, C, ldc, c_off, acc, st)) return rc;
-    return rows_of<F>(w, mat, aq + (size_t)h * w->K, asc + h, T - h, Mp, C + (size_t)h * ldc, ldc, c_off, acc, st);
+    if (const int rc = rows_of<F, true>(w, mat, aq, asc, h, Mp, C, ldc, c_off, acc, st)) return rc;
+    return rows_of<F, true>(w, mat, aq + (size_t)h * w->K, asc + h, T - h, Mp, C + (size_t)h * ldc, ldc, c_off, acc, st);
   }
-  IZB_SMEM_OPTIN((rows_kernel<F>), kSmemPerSm, w->device);
+  IZB_SMEM_OPTIN((rows_kernel<F, kFour>), kSmemPerSm, w->device);
   const int groups = (tiles + sp.warps / F::kSubs - 1) / (sp.warps / F::kSubs), grid = groups < sms * sp.ctas ? groups : sms * sp.ctas;
   uint32_t* err = izb_device_error_word(w->device);
   if (!err) IZB_FAIL(IZB_ERR_NOMEM, "gemv: no device error word");
   CUtensorMap tm;
   memcpy(&tm, w->tmap16_raw, sizeof tm);
-  IZB_LAUNCH("gemv_rows", st, izb_launch_pdl(rows_kernel<F>, grid, sp.warps * 32, rows_smem<F>(w->K, T, sp.warps, sp.slots), st, tm, mat * w->N, w->N, w->K, aq, asc, T, Mp, C, ldc,
+  IZB_LAUNCH("gemv_rows", st, izb_launch_pdl(rows_kernel<F, kFour>, grid, sp.warps * 32, rows_smem<F, kFour>(w->K, T, sp.warps, sp.slots), st, tm, mat * w->N, w->N, w->K, aq, asc, T, Mp, C, ldc,
                                              c_off, acc, sp.slots, err));
   return IZB_OK;
 }
@@ -851,7 +982,7 @@ int moe_rows_of(const izb_weight* wg, const izb_weight* wu, const int8_t* aq, co
   int ctas = kMoeCtas, slots = 0;
   for (; ctas > 0; --ctas) {
     const size_t room = kSmemPerSm / ctas - (ctas > 1 ? 1024 : 0);
-    for (slots = 4; slots >= 2 && rows_smem<F>(wg->K, 8, kMoeWarps, slots) > room;) --slots;
+    for (slots = 4; slots >= 2 && rows_smem<F, false>(wg->K, 8, kMoeWarps, slots) > room;) --slots;
     if (slots >= 2) break;
   }
   if (ctas == 0) return 1;
@@ -862,7 +993,7 @@ int moe_rows_of(const izb_weight* wg, const izb_weight* wu, const int8_t* aq, co
   memcpy(&tu, (wu ? wu : wg)->tmap16_raw, sizeof tu);
   // (one kernel for both products: as two, the second finds its code out of the instruction cache, 1 us of a 4-token step)
   IZB_SMEM_OPTIN((moe_rows_kernel<F>), kSmemPerSm, wg->device);
-  IZB_LAUNCH(wu ? "moe_gateup" : "moe_down", st, izb_launch_pdl(moe_rows_kernel<F>, sms * ctas, kMoeWarps * 32, rows_smem<F>(wg->K, 8, kMoeWarps, slots), st, tg, tu, wu ? 1 : 0,
+  IZB_LAUNCH(wu ? "moe_gateup" : "moe_down", st, izb_launch_pdl(moe_rows_kernel<F>, sms * ctas, kMoeWarps * 32, rows_smem<F, false>(wg->K, 8, kMoeWarps, slots), st, tg, tu, wu ? 1 : 0,
                                                                wg->N, wg->K, aq, asc, Mp, tiles, stok, swt, out, slots, wu ? sms * (ctas < 2 ? ctas : 2) : 0, err));
   return IZB_OK;
 }
@@ -872,9 +1003,9 @@ int moe_rows_of(const izb_weight* wg, const izb_weight* wu, const int8_t* aq, co
 // up to 8 rows; +1: not taken (another weight form, no tensor map, or activations that do not fit in shared memory)
 int izb_rows_launch(const izb_weight* w, int mat, const int8_t* aq, const float* asc, int T, int Mp, float* C, int ldc, int c_off, int acc, cudaStream_t st) {
   if (!w->has_tmap16 || T > 8) return 1;
-  if (w->type == IZB_Q4_K) return rows_of<RQ4K>(w, mat, aq, asc, T, Mp, C, ldc, c_off, acc, st);
-  if (w->type == IZB_Q8_0) return rows_of<RQ80>(w, mat, aq, asc, T, Mp, C, ldc, c_off, acc, st);
-  return rows_of<RQ6K>(w, mat, aq, asc, T, Mp, C, ldc, c_off, acc, st);
+  auto of = w->type == IZB_Q4_K ? (T <= 4 ? rows_of<RQ4K, true> : rows_of<RQ4K, false>) : w->type == IZB_Q8_0 ? (T <= 4 ? rows_of<RQ80, true> : rows_of<RQ80, false>)
+          : T <= 4 ? rows_of<RQ6K, true> : rows_of<RQ6K, false>;
+  return of(w, mat, aq, asc, T, Mp, C, ldc, c_off, acc, st);
 }
 
 // gate / up (wu given) or down (wu = null, swt given) over tiles of up to 8 slots; +1: not taken

@@ -58,6 +58,33 @@ def test_rows_do_not_depend_on_their_number(izb, qt, N, K):
     W.close()
 
 
+# The matrix instruction's kernel for up to four rows (two pieces of a row per instruction) against the dot-product kernel: the first 16 weight
+# rows alone make a matrix that is too small for the former.  Rows that do not fill a tile, fewer superblocks than warps share, odd counts of them,
+# both sides of the K up to which the dot product's rings hold whole rows, and of the bounds in N.
+@pytest.mark.parametrize("qt,N,K,Ts", [(14, 257, 4352, "1234"), (14, 1000, 8448, "1234"), (14, 4100, 4608, "1234"), (12, 12288, 256, "134"), (12, 12290, 3328, "1234"), (12, 2561, 768, "4"),
+                                       (12, 4100, 2304, "34"), (12, 520, 10496, "1234"), (12, 520, 12288, "1234"), (12, 512, 17664, "1234"), (8, 5128, 2560, "134"), (8, 40968, 256, "1234"),
+                                       (8, 6152, 1280, "1234"), (8, 3080, 768, "4"), (8, 520, 5888, "1234"), (8, 4104, 5120, "34"), (8, 1000, 8448, "1234"), (8, 512, 17152, "1234")])
+def test_four_rows_equal_dot_products(izb, qt, N, K, Ts):
+    import torch
+    rows = S.make_weight(qt, 16, K, N + K + qt)
+    W, head = izb.Weight(qt, np.tile(rows, ((N + 15) // 16, 1))[:N], N, K), izb.Weight(qt, rows, 16, K)
+    x = S.make_act(4, K, 7)
+    x[1] *= 1e4
+    aq, asc, _ = izb.quantize_act(torch.from_numpy(x).cuda())
+    for T in map(int, Ts):
+        izb.profile_start()
+        got = izb.gemv(W, aq, asc, T)
+        ran = set(izb.profile_stop())
+        izb.profile_start()
+        want = izb.gemv(head, aq, asc, T)
+        ran_head = set(izb.profile_stop())
+        assert ran == {"gemv_rows"} and "gemv_rows" not in ran_head, (T, ran, ran_head)
+        for n in range(0, N, 16):
+            assert torch.equal(got[:T, n:n + 16], want[:T, :min(16, N - n)]), (T, n)
+    assert izb.device_status(0) == 0
+    W.close(), head.close()
+
+
 @pytest.mark.parametrize("qt", [12, 8])
 @pytest.mark.parametrize("T,TM,F,E", [(1, 8, 256, 512), (5, 4, 768, 1024), (40, 8, 256, 2304), (3, 1, 512, 256), (40, 8, 1024, 512), (4, 8, 3072, 256)])
 def test_expert_rows_equal_dense_rows(izb, qt, T, TM, F, E):
