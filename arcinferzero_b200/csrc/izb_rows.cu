@@ -919,31 +919,32 @@ __global__ void __launch_bounds__(kMoeWarps * 32, kMoeCtas) moe_rows_kernel(cons
   }
 }
 
-// Warps per CTA, CTAs per SM and ring slots (2 to 4: deeper rings gain nothing) for `tiles` row tiles.  What hides the latency is chunks
-// in flight and at work, so of all splits that fit: the most warps x (slots + 1) that have work, averaged over the rounds the grid
-// needs; of equals the smaller CTA.  (Four warps suit small matrices -- 1024 x 3072 Q6_K, 5 rows: 4.5 us against 5.2 with eight and
-// 7.9 with sixteen --, sixteen share one copy of large activations: 128000 x 4096 Q4_K, 8 rows: 89 us against 102 with four.)
-// Warps past the last tile are not at work: they request and multiply rows that do not exist beside the ones that do (96 x 4096 Q4_K,
-// four rows: 10.5 us in sixteen-warp CTAs, 6.5 in four-warp ones).
+// Warps per CTA, CTAs per SM and ring slots (2 to 4) for `tiles` row tiles.  The fewest rounds of the grid, weighted by what a round of
+// fewer slots takes longer (three for two 1.15; four for three 1.04, up to eight warps per SM: with twelve three are enough); of equals
+// the smaller CTA, which spreads the tiles of a single round over more SMs.  (us, 16 warps / 12: Q4_K 5120 x 13824, one row, 17.5 / 14.9,
+// 6144 x 4096, five, 9.3 / 8.6; Q6_K 5120 x 17408, three, 27.8 / 20.5 with eight in two rounds.  One CTA of twelve / three of four: Q6_K 5120 x 5120, one row,
+// 7.9 / 7.0; of sixteen / two of eight: Q4_K 16384 x 5376, three, 17.0 / 15.4.  Two of four, three slots / one of eight, four: Q8_0 8192 x 4096, eight,
+// 10.9 / 9.7.)
 constexpr size_t kSmemPerSm = 226 * 1024;
 struct Split {
   int warps, ctas, slots;  // slots 0: the activations leave no room
 };
 template <class F, bool kFour>
 Split pick_split(int K, int T, int tiles, int sms) {
+  constexpr double kDepth[5] = {0, 0, 1.0, 1.15, 1.2};
   Split best = {0, 0, 0};
-  double most = 0;
-  for (int nw = 4; nw <= 16; nw *= 2) {
+  double least = 0;
+  for (int nw = 4; nw <= 16; nw += 4) {
     const int groups = (tiles + nw / F::kSubs - 1) / (nw / F::kSubs);
-    for (int c = 1; c * nw <= 16; ++c) {
+    for (int c = 1; c * nw <= 16 && (c - 1) * sms < groups; ++c) {
       const size_t room = kSmemPerSm / c - (c > 1 ? 1024 : 0);
       int slots = 4;
       while (slots >= 2 && rows_smem<F, kFour>(K, T, nw, slots) > room) --slots;
       if (slots < 2) break;
       const int rounds = (groups + c * sms - 1) / (c * sms);
-      const double at_work = (double)tiles * F::kSubs * (slots + 1) / rounds;
-      if (at_work > most * 1.001) {
-        most = at_work;
+      const double time = rounds / kDepth[slots == 4 && c * nw >= 12 ? 3 : slots];
+      if (best.slots == 0 || time < least * 0.999) {
+        least = time;
         best = {nw, c, slots};
       }
     }
