@@ -4,7 +4,7 @@
 // The divisions and the product are written with the round-to-nearest intrinsics so no contraction or reciprocal
 // approximation can change a bit.
 //
-// One CTA covers 32 token rows x 256 columns: every lane owns 8 consecutive values (two 128-bit loads), four lanes make
+// (Many rows.)  One CTA covers 32 token rows x 256 columns: every lane owns 8 consecutive values (two 128-bit loads), four lanes make
 // a 32-block.  The int8 row stores are 256 contiguous bytes per warp; the scales, whose layout is block-major
 // ([K/32][Mp]), go through shared memory so that each block's 32 token scales leave as one 128-byte line.
 #include "izb_common.cuh"
@@ -89,6 +89,45 @@ __global__ void __launch_bounds__(256) quantize_act_kernel(const float* __restri
         absum[(size_t)(sb * 16 + 8 + b) * Mp + m0 + r] = s_sum[8 + b][r];
       }
     }
+  }
+}
+
+// The same for few rows: one thread per value, a warp per 32-block, a CTA per row and 256 columns (one CTA more for the padding rows).  What bounds
+// a decode step's quantiser is the latency of one thread's values: eight of them, each with an exponential and two divisions (SwiGLU).
+template <int kMode>
+__global__ void __launch_bounds__(256) quantize_few_kernel(const float* __restrict__ x, int ldx, int M, int Mp, int K, int8_t* __restrict__ aq, float* __restrict__ asc,
+                                                           int16_t* __restrict__ absum, float* __restrict__ hout, int F) {
+  const int sb = blockIdx.x, row = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, col = sb * 256 + threadIdx.x;
+  pdl_launch_next();
+  pdl_wait();
+  if (row == M) {
+    for (int i = threadIdx.x; i < (Mp - M) * 16; i += 256) {
+      const int m = M + (i >> 4), c = i & 15;
+      *reinterpret_cast<uint4*>(aq + (size_t)m * K + sb * 256 + 16 * c) = make_uint4(0, 0, 0, 0);
+      if (c < 8) asc[(size_t)(sb * 8 + c) * Mp + m] = 0.0f;
+      if (absum) absum[(size_t)(sb * 16 + c) * Mp + m] = 0;
+    }
+    return;
+  }
+  float v = x[(size_t)row * ldx + col];
+  if (kMode == 1) {
+    const float u = x[(size_t)row * ldx + F + col];
+    v = __fmul_rn(__fdiv_rn(v, __fadd_rn(1.0f, expf(-v))), u);
+    if (hout) hout[(size_t)row * F + col] = v;
+  }
+  float amax = fmaxf(0.0f, fabsf(v));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
+  const float inv = amax > 0.0f ? __fdiv_rn(127.0f, amax) : 0.0f;
+  const float p = __fmul_rn(v, inv);
+  const int q = fabsf(p) <= 2147483520.0f ? __float2int_rn(p) : 0;  // (see quantize_act_kernel)
+  aq[(size_t)row * K + col] = (int8_t)q;
+  if (lane == 0) asc[(size_t)(sb * 8 + warp) * Mp + row] = __fdiv_rn(amax, 127.0f);
+  if (absum) {
+    int s16 = q;
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) s16 += __shfl_xor_sync(0xFFFFFFFFu, s16, o);
+    if ((lane & 15) == 0) absum[(size_t)(sb * 16 + 2 * warp + (lane >> 4)) * Mp + row] = (int16_t)s16;
   }
 }
 
@@ -324,25 +363,34 @@ int check_quant_args(const float* x, int ldx, int M, int Mp, int K, const int8_t
 
 }  // namespace
 
+// Few rows -- blocks of one row that fit the device at once, four times as many with the SwiGLU product -- take a thread per value.  (us, a thread
+// per eight values / per value: quantise 1 x 5120 2.2 / 1.2, 32 x 768 2.1 / 1.2, 128 x 2048 2.1 / 2.0, 64 x 5120 2.2 / 2.3, 256 x 5120 3.7 / 5.9; SwiGLU 1 x
+// 17408 2.9 / 1.4, 32 x 5120 4.7 / 2.0, 64 x 17408 7.5 / 5.8, 100 x 17408 7.8 / 8.3, 512 x 5120 8.5 / 11.9.)
+template <int kMode>
+static int launch_quantize(const char* what, const float* x, int ldx, int M, int Mp, int K, int8_t* aq, float* asc, int16_t* absum, float* hout, cudaStream_t st) {
+  const dim3 few(K / 256, M + (Mp > M ? 1 : 0));
+  if (izb_one_wave(dim3(few.x, kMode == 1 ? (few.y + 3) / 4 : few.y), 256)) {
+    IZB_LAUNCH(what, st, izb_launch_pdl(quantize_few_kernel<kMode>, few, 256, 0, st, x, ldx, M, Mp, K, aq, asc, absum, hout, K));
+  } else {
+    dim3 grid(K / 256, (Mp + 31) / 32);
+    IZB_LAUNCH(what, st, izb_launch_pdl(quantize_act_kernel<kMode>, grid, 256, 0, st, x, ldx, M, Mp, K, aq, asc, absum, hout, K));
+  }
+  return IZB_OK;
+}
+
 extern "C" int izb_quantize_act(const float* d_x, int ldx, int M_valid, int Mp, int K, int8_t* d_aq, float* d_asc,
                                 int16_t* d_absum, void* stream) {
   if (int rc = check_quant_args(d_x, ldx, M_valid, Mp, K, d_aq, d_asc, K)) return rc;
-  dim3 grid(K / 256, (Mp + 31) / 32);
-  IZB_LAUNCH("quantize_act", (cudaStream_t)stream, izb_launch_pdl(quantize_act_kernel<0>, grid, 256, 0, (cudaStream_t)stream, d_x, ldx, M_valid, Mp, K, d_aq, d_asc, d_absum, nullptr, 0));
-  return IZB_OK;
+  return launch_quantize<0>("quantize_act", d_x, ldx, M_valid, Mp, K, d_aq, d_asc, d_absum, nullptr, (cudaStream_t)stream);
 }
 
 extern "C" int izb_swiglu_quant(const float* d_gu, int ldgu, int split, int M_valid, int Mp, int F, float* d_h, int8_t* d_aq,
                                 float* d_asc, int16_t* d_absum, void* stream) {
   if (int rc = check_quant_args(d_gu, ldgu, M_valid, Mp, F, d_aq, d_asc, split ? 2 * F : F)) return rc;
   if (d_h && !izb_aligned(d_h, 16)) IZB_FAIL(IZB_ERR_ALIGN, "swiglu_quant: h not 16-byte aligned");
-  dim3 grid(F / 256, (Mp + 31) / 32);
   cudaStream_t st = (cudaStream_t)stream;
-  if (split)
-    IZB_LAUNCH("swiglu_quant", st, izb_launch_pdl(quantize_act_kernel<1>, grid, 256, 0, st, d_gu, ldgu, M_valid, Mp, F, d_aq, d_asc, d_absum, d_h, F));
-  else
-    IZB_LAUNCH("quantize_act", st, izb_launch_pdl(quantize_act_kernel<0>, grid, 256, 0, st, d_gu, ldgu, M_valid, Mp, F, d_aq, d_asc, d_absum, nullptr, 0));
-  return IZB_OK;
+  return split ? launch_quantize<1>("swiglu_quant", d_gu, ldgu, M_valid, Mp, F, d_aq, d_asc, d_absum, d_h, st)
+               : launch_quantize<0>("quantize_act", d_gu, ldgu, M_valid, Mp, F, d_aq, d_asc, d_absum, nullptr, st);
 }
 
 extern "C" int izb_rmsnorm_quant(const float* d_x, int ldx, const float* d_w, float eps, int M_valid, int Mp, int K, float* d_h,

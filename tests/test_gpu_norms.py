@@ -37,6 +37,28 @@ def test_rmsnorm_quant(izb, M, K):
     assert (bits(h.cpu().numpy()) == bits(ry)).all() and (aq.cpu().numpy() == raq).all() and (bits(asc.cpu().numpy()) == bits(rasc)).all()
 
 
+# Few rows go by a thread per value (148 x 8 blocks of one row and 256 columns, with the SwiGLU product four times as many), more by a thread per
+# eight: the same bits, also for zeros, infinities, NaN and blocks whose 127 / amax overflows.
+@pytest.mark.parametrize("M,K", [(1, 256), (16, 512), (17, 768), (147, 2048), (148, 2048), (591, 2048), (592, 2048)])
+def test_quantisers_do_not_depend_on_the_number_of_rows(izb, M, K):
+    import torch
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(M + K)
+    x = torch.randn((2500, 2 * K), generator=gen, device="cuda")
+    x[0, :32] = 0.0
+    x[0, 40], x[0, 70], x[0, 100] = float("inf"), float("nan"), -0.0
+    x[0, 128:160] = 1e-44
+    x[0, 160:192] = float("nan")
+    def same(a, b):
+        return torch.equal(a.contiguous().view(torch.int8), b.contiguous().view(torch.int8))
+    few, many = izb.quantize_act(x[:M, :K], want_absum=True), izb.quantize_act(x[:, :K], want_absum=True)
+    hfew, hmany = izb.swiglu_quant(x[:M], K, want_h=True), izb.swiglu_quant(x, K, want_h=True)
+    for f, m in ((few, many), (hfew, hmany)):
+        assert same(f[0][:M], m[0][:M]) and not f[0][M:].any()
+        assert same(f[1][:, :M], m[1][:, :M]) and f[1].shape[1] == izb.pad_rows(M) and not f[1][:, M:].any()
+    assert same(few[2][:, :M], many[2][:, :M]) and not few[2][:, M:].any() and same(hfew[2][:M], hmany[2][:M])
+
+
 # (a wave holds 148 x 8 blocks of 1024 logits, 148 x 16 blocks of 512 combined values)
 @pytest.mark.parametrize("rows,N", [(1184, 1024), (1185, 1024), (600, 4100)])
 def test_softcap_of_one_wave_and_more(izb, rows, N):
