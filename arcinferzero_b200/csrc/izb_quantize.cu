@@ -92,12 +92,31 @@ __global__ void __launch_bounds__(256) quantize_act_kernel(const float* __restri
   }
 }
 
+// One value per thread, a warp per 32-block: the block's scale and sums from the warp.
+__device__ __forceinline__ void quantize_value(float v, int row, int col, int Mp, int K, int8_t* __restrict__ aq, float* __restrict__ asc, int16_t* __restrict__ absum) {
+  const int lane = threadIdx.x & 31;
+  float amax = fmaxf(0.0f, fabsf(v));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
+  const float inv = amax > 0.0f ? __fdiv_rn(127.0f, amax) : 0.0f;
+  const float p = __fmul_rn(v, inv);
+  const int q = fabsf(p) <= 2147483520.0f ? __float2int_rn(p) : 0;  // (see quantize_act_kernel)
+  aq[(size_t)row * K + col] = (int8_t)q;
+  if (lane == 0) asc[(size_t)(col >> 5) * Mp + row] = __fdiv_rn(amax, 127.0f);
+  if (absum) {
+    int s16 = q;
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) s16 += __shfl_xor_sync(0xFFFFFFFFu, s16, o);
+    if ((lane & 15) == 0) absum[(size_t)(col >> 4) * Mp + row] = (int16_t)s16;
+  }
+}
+
 // The same for few rows: one thread per value, a warp per 32-block, a CTA per row and 256 columns (one CTA more for the padding rows).  What bounds
 // a decode step's quantiser is the latency of one thread's values: eight of them, each with an exponential and two divisions (SwiGLU).
 template <int kMode>
 __global__ void __launch_bounds__(256) quantize_few_kernel(const float* __restrict__ x, int ldx, int M, int Mp, int K, int8_t* __restrict__ aq, float* __restrict__ asc,
                                                            int16_t* __restrict__ absum, float* __restrict__ hout, int F) {
-  const int sb = blockIdx.x, row = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, col = sb * 256 + threadIdx.x;
+  const int sb = blockIdx.x, row = blockIdx.y, col = sb * 256 + threadIdx.x;
   pdl_launch_next();
   pdl_wait();
   if (row == M) {
@@ -115,20 +134,7 @@ __global__ void __launch_bounds__(256) quantize_few_kernel(const float* __restri
     v = __fmul_rn(__fdiv_rn(v, __fadd_rn(1.0f, expf(-v))), u);
     if (hout) hout[(size_t)row * F + col] = v;
   }
-  float amax = fmaxf(0.0f, fabsf(v));
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
-  const float inv = amax > 0.0f ? __fdiv_rn(127.0f, amax) : 0.0f;
-  const float p = __fmul_rn(v, inv);
-  const int q = fabsf(p) <= 2147483520.0f ? __float2int_rn(p) : 0;  // (see quantize_act_kernel)
-  aq[(size_t)row * K + col] = (int8_t)q;
-  if (lane == 0) asc[(size_t)(sb * 8 + warp) * Mp + row] = __fdiv_rn(amax, 127.0f);
-  if (absum) {
-    int s16 = q;
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) s16 += __shfl_xor_sync(0xFFFFFFFFu, s16, o);
-    if ((lane & 15) == 0) absum[(size_t)(sb * 16 + 2 * warp + (lane >> 4)) * Mp + row] = (int16_t)s16;
-  }
+  quantize_value(v, row, col, Mp, K, aq, asc, absum);
 }
 
 // Sum over the CTA's 256 threads in the defined order: xor butterfly 16, 8, 4, 2, 1 inside every warp, then the eight
@@ -145,12 +151,16 @@ __device__ __forceinline__ float cta_sum_ordered(float v, float* s_w) {
   return t;
 }
 
-// rows M..Mp-1 of a quantised activation buffer: zeros with scale 0 (one CTA per row)
+// rows M..Mp-1 of a quantised activation buffer: zeros with scale 0 (one CTA per row, or columns c0 .. c1 - 1 of a row)
+__device__ __forceinline__ void zero_pad_cols(int m, int c0, int c1, int Mp, int K, int8_t* __restrict__ aq, float* __restrict__ asc, int16_t* __restrict__ absum) {
+  for (int i = c0 / 16 + threadIdx.x; i < c1 / 16; i += blockDim.x) {
+    reinterpret_cast<uint4*>(aq + (size_t)m * K)[i] = make_uint4(0, 0, 0, 0);
+    if (!(i & 1)) asc[(size_t)(i >> 1) * Mp + m] = 0.0f;
+    if (absum) absum[(size_t)i * Mp + m] = 0;
+  }
+}
 __device__ __forceinline__ void zero_pad_row(int m, int Mp, int K, int8_t* __restrict__ aq, float* __restrict__ asc, int16_t* __restrict__ absum) {
-  for (int i = threadIdx.x; i < K; i += blockDim.x) aq[(size_t)m * K + i] = 0;
-  for (int b = threadIdx.x; b < K / 32; b += blockDim.x) asc[(size_t)b * Mp + m] = 0.0f;
-  if (absum)
-    for (int b = threadIdx.x; b < K / 16; b += blockDim.x) absum[(size_t)b * Mp + m] = 0;
+  zero_pad_cols(m, 0, K, Mp, K, aq, asc, absum);
 }
 
 // add_norm_quant (zero/kernels/ops_attn_g.cl:617-680), one CTA of 256 threads per row, K <= 256 * kAnqMax:
@@ -252,6 +262,80 @@ __global__ void __launch_bounds__(256) add_norm_quant_kernel(float* __restrict__
   }
 }
 
+// The same for few rows of 1280 to 5120: a cluster of up to eight CTAs per row.  Every CTA takes both sums over the whole row, in the same order, and then
+// updates and quantises its share of it (up to three steps of 256): one SM's issue slots, not its loads, are what a row took its time for.
+// The new x goes over the old one that the other CTAs read: they store behind the cluster's barrier.
+constexpr int kFewSteps = 3;
+template <int NK>
+__global__ void __launch_bounds__(256) add_norm_few_kernel(float* __restrict__ x, const float* __restrict__ t, const float* __restrict__ w, int K, float eps, float s,
+                                                           const float* __restrict__ w2, int M, int Mp, int8_t* __restrict__ aq, float* __restrict__ asc,
+                                                           int16_t* __restrict__ absum, int steps) {
+  __shared__ float s_w[8];
+  const int m = blockIdx.y, first = blockIdx.x * steps, nk = K / 256;
+  pdl_launch_next();
+  pdl_wait();
+  if (m >= M) {
+    zero_pad_cols(m, 256 * first, min(256 * (first + steps), K), Mp, K, aq, asc, absum);
+    return;
+  }
+  float* xr = x + (size_t)m * K;
+  const float* tr = t + (size_t)m * K;
+  float tv[NK], xv[NK], wv[NK], to[kFewSteps], xo[kFewSteps], wo[kFewSteps], w2o[kFewSteps];
+#pragma unroll
+  for (int k = 0; k < NK; ++k)
+    if (k < nk) tv[k] = tr[threadIdx.x + 256 * k];
+  if (w2) {
+#pragma unroll
+    for (int k = 0; k < NK; ++k)
+      if (k < nk) {
+        xv[k] = xr[threadIdx.x + 256 * k];
+        wv[k] = w[threadIdx.x + 256 * k];
+      }
+  }
+#pragma unroll
+  for (int k = 0; k < kFewSteps; ++k)
+    if (k < steps && first + k < nk) {
+      const int i = threadIdx.x + 256 * (first + k);
+      to[k] = tr[i];
+      xo[k] = xr[i];
+      wo[k] = w[i];
+      if (w2) w2o[k] = w2[i];
+    }
+  float ss = 0.0f;
+#pragma unroll
+  for (int k = 0; k < NK; ++k)
+    if (k < nk) ss = __fmaf_rn(tv[k], tv[k], ss);
+  ss = cta_sum_ordered(ss, s_w);
+  const float r = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, (float)K), eps)));
+  auto updated = [&](float xe, float te, float we) { return __fmul_rn(__fadd_rn(xe, __fmul_rn(__fmul_rn(te, r), we)), s); };
+  float s2 = 0.0f;
+  if (w2) {
+#pragma unroll
+    for (int k = 0; k < NK; ++k)
+      if (k < nk) {
+        const float v = updated(xv[k], tv[k], wv[k]);
+        s2 = __fmaf_rn(v, v, s2);
+      }
+  }
+#pragma unroll
+  for (int k = 0; k < kFewSteps; ++k)
+    if (k < steps && first + k < nk) xo[k] = updated(xo[k], to[k], wo[k]);
+  asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");  // this CTA has read the row
+  float r2 = 1.0f;
+  if (w2) {
+    s2 = cta_sum_ordered(s2, s_w);
+    r2 = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(s2, (float)K), eps)));
+  }
+  asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+#pragma unroll
+  for (int k = 0; k < kFewSteps; ++k)
+    if (k < steps && first + k < nk) {
+      const int i = threadIdx.x + 256 * (first + k);
+      xr[i] = xo[k];
+      quantize_value(w2 ? __fmul_rn(__fmul_rn(xo[k], r2), w2o[k]) : xo[k], m, i, Mp, K, aq, asc, absum);
+    }
+}
+
 // rmsnorm_quant (zero/kernels/ops.cl:104-141), one CTA of 256 threads per row, in the quantiser's lane layout: thread j owns
 // the groups of 8 consecutive values j, j + 256, ... .  Step 1: the sum of squares, a chain of fused multiply-adds over the
 // thread's values in index order, then cta_sum_ordered (this order is part of the definition: the oracle repeats it).
@@ -351,6 +435,49 @@ __global__ void __launch_bounds__(256) rmsnorm_quant_row_kernel(const float* __r
   }
 }
 
+// The same for few rows: several CTAs per row, each with the whole row's sum in the same order and two steps of 256 values to quantise (see
+// add_norm_few_kernel; nothing is written over what another CTA reads).
+template <int G>
+__global__ void __launch_bounds__(256) rmsnorm_few_kernel(const float* __restrict__ x, int ldx, const float* __restrict__ w, int K, float eps, int M, int Mp, float* __restrict__ hout,
+                                                          int8_t* __restrict__ aq, float* __restrict__ asc, int16_t* __restrict__ absum) {
+  __shared__ float s_w[8];
+  const int m = blockIdx.y, ng = K / 8, i0 = blockIdx.x * 512 + threadIdx.x, i1 = i0 + 256;
+  pdl_launch_next();
+  pdl_wait();
+  if (m >= M) {
+    zero_pad_cols(m, blockIdx.x * 512, min(blockIdx.x * 512 + 512, K), Mp, K, aq, asc, absum);
+    return;
+  }
+  const float* xr = x + (size_t)m * ldx;
+  float4 xa[G], xb[G];
+#pragma unroll
+  for (int k = 0; k < G; ++k) {
+    const int g = threadIdx.x + 256 * k;
+    if (g < ng) {
+      xa[k] = reinterpret_cast<const float4*>(xr)[2 * g];
+      xb[k] = reinterpret_cast<const float4*>(xr)[2 * g + 1];
+    }
+  }
+  const bool two = i1 < K;  // (uniform over the CTA, as K is a multiple of 256)
+  const float x0 = xr[i0], w0 = w[i0], x1 = two ? xr[i1] : 0.0f, w1 = two ? w[i1] : 0.0f;
+  float ss = 0.0f;
+#pragma unroll
+  for (int k = 0; k < G; ++k)
+    if (threadIdx.x + 256 * k < ng) {
+      ss = __fmaf_rn(xa[k].x, xa[k].x, ss); ss = __fmaf_rn(xa[k].y, xa[k].y, ss); ss = __fmaf_rn(xa[k].z, xa[k].z, ss); ss = __fmaf_rn(xa[k].w, xa[k].w, ss);
+      ss = __fmaf_rn(xb[k].x, xb[k].x, ss); ss = __fmaf_rn(xb[k].y, xb[k].y, ss); ss = __fmaf_rn(xb[k].z, xb[k].z, ss); ss = __fmaf_rn(xb[k].w, xb[k].w, ss);
+    }
+  ss = cta_sum_ordered(ss, s_w);
+  const float r = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, (float)K), eps)));
+  const float v0 = __fmul_rn(__fmul_rn(x0, r), w0), v1 = __fmul_rn(__fmul_rn(x1, r), w1);
+  if (hout) hout[(size_t)m * K + i0] = v0;
+  quantize_value(v0, m, i0, Mp, K, aq, asc, absum);
+  if (two) {
+    if (hout) hout[(size_t)m * K + i1] = v1;
+    quantize_value(v1, m, i1, Mp, K, aq, asc, absum);
+  }
+}
+
 int check_quant_args(const float* x, int ldx, int M, int Mp, int K, const int8_t* aq, const float* asc, int width_needed) {
   if (!x || !aq || !asc) IZB_FAIL(IZB_ERR_ARG, "quantize: null pointer");
   if (K <= 0 || K % 256) IZB_FAIL(IZB_ERR_SHAPE, "quantize: K = %d is not a positive multiple of 256", K);
@@ -401,6 +528,13 @@ extern "C" int izb_rmsnorm_quant(const float* d_x, int ldx, const float* d_w, fl
   if (!(eps >= 0.0f)) IZB_FAIL(IZB_ERR_ARG, "rmsnorm_quant: eps = %g", (double)eps);
   cudaStream_t st = (cudaStream_t)stream;
   const int groups = (K / 8 + 255) / 256;  // of 8 values per thread
+  // decode steps over long rows (us, a CTA per row / several: 4096, one row 2.0/1.8, eight 2.1/2.1; 5120, one 2.3/1.9, eight 2.4/2.2, sixteen 2.4/3.0; 12288, one
+  // 3.6/2.7, eight 3.6/3.4; 2048, one 1.5/1.6)
+  if (M_valid <= 8 && K >= 4096 && groups <= 8) {
+    auto kernel = groups <= 2 ? rmsnorm_few_kernel<2> : groups <= 3 ? rmsnorm_few_kernel<3> : groups <= 4 ? rmsnorm_few_kernel<4> : rmsnorm_few_kernel<8>;
+    IZB_LAUNCH("rmsnorm_quant", st, izb_launch_pdl(kernel, dim3((K + 511) / 512, Mp), 256, 0, st, d_x, ldx, d_w, K, eps, M_valid, Mp, d_h, d_aq, d_asc, d_absum));
+    return IZB_OK;
+  }
   // Rows held in registers cost blocks per SM: many long rows are faster read twice (us, held / read twice: 16384, 296 rows 13.5/12.9, 450 rows
   // 17.6/15.2, 4096 rows 126/83; 8448, 1000 rows 14.6/16.1, 4096 rows 54/46; 12288, 2000 rows 35/39, 4096 rows 66/63)
   int dev = 0;
@@ -422,7 +556,15 @@ extern "C" int izb_add_norm_quant(float* d_x, const float* d_t, const float* d_w
   cudaStream_t st = (cudaStream_t)stream;
   const int nk = K / 256;  // elements per thread
   int dev = 0;
-  if (nk > 32) IZB_CUDA(cudaGetDevice(&dev));
+  IZB_CUDA(cudaGetDevice(&dev));
+  // A cluster per row while there are up to three CTAs per SM (us, a CTA per row / a cluster: 2048, one row 4.0/2.6, 100 rows 5.3/4.3; 4096, one 6.6/3.0,
+  // 32 6.9/4.2, 64 7.4/7.3, 100 7.6/9.6; 5120, one 8.2/3.5, 100 9.4/11; 1024, one 2.7/2.5, 100 3.0/3.1)
+  const int cl = nk <= 16 ? (nk + 1) / 2 : 7, steps = (nk + cl - 1) / cl;
+  if (nk > 4 && nk <= 20 && (long long)cl * Mp <= 3 * izb_sm_count(dev)) {
+    auto kernel = nk <= 8 ? add_norm_few_kernel<8> : nk <= 16 ? add_norm_few_kernel<16> : add_norm_few_kernel<20>;
+    IZB_LAUNCH("add_norm_quant", st, izb_launch_pdl_cluster(kernel, cl, dim3(cl, Mp), 256, 0, st, d_x, d_t, d_w, K, eps, s, d_w2, M_valid, Mp, d_aq, d_asc, d_absum, steps));
+    return IZB_OK;
+  }
   auto kernel = nk <= 4 ? add_norm_quant_kernel<4, true> : nk <= 8 ? add_norm_quant_kernel<8, true> : nk <= 16 ? add_norm_quant_kernel<16, true>
               : nk <= 20 ? add_norm_quant_kernel<20, true> : nk <= 32 ? add_norm_quant_kernel<32, true>
               : M_valid <= izb_sm_count(dev) ? add_norm_quant_kernel<kAnqMax, true> : add_norm_quant_kernel<kAnqMax, false>;

@@ -37,6 +37,26 @@ def test_rmsnorm_quant(izb, M, K):
     assert (bits(h.cpu().numpy()) == bits(ry)).all() and (aq.cpu().numpy() == raq).all() and (bits(asc.cpu().numpy()) == bits(rasc)).all()
 
 
+# Few rows are shared by several CTAs (with the residual addition up to 3 x 148 CTAs in clusters of up to eight; without up to eight rows of 4096 and
+# more): shares that do not divide, rows without a second norm, sums and padding, a step of a row that runs on from the one before.
+@pytest.mark.parametrize("M,K", [(1, 1280), (1, 1536), (5, 2304), (2, 3840), (8, 4096), (48, 4096), (64, 4096), (3, 4352), (5, 4608), (1, 4864), (8, 5120), (63, 5120)])
+def test_norms_of_few_rows(izb, M, K):
+    import torch
+    rng = np.random.default_rng(M + K)
+    x, w, w2 = (rng.standard_normal(n, dtype=np.float32) for n in ((M, K), K, K))
+    for second in (w2, None):
+        xd, rx = torch.from_numpy(x).cuda(), x
+        for step in range(3):
+            t = rng.standard_normal((M, K), dtype=np.float32) * 3
+            aq, asc = izb.add_norm_quant(xd, torch.from_numpy(t).cuda(), torch.from_numpy(w).cuda(), 1e-6, 0.75, None if second is None else torch.from_numpy(second).cuda())
+            rx, raq, rasc, _ = O.add_norm_quant(rx, t, w, 1e-6, 0.75, second, Mp=asc.shape[1])
+            assert (bits(xd.cpu().numpy()) == bits(rx)).all() and (aq.cpu().numpy() == raq).all() and (bits(asc.cpu().numpy()) == bits(rasc)).all(), step
+    wide = torch.from_numpy(np.concatenate([x, x], 1)).cuda()  # (a row stride of its own)
+    aq, asc, h = izb.rmsnorm_quant(wide[:, :K], torch.from_numpy(w).cuda(), 1e-6, want_h=True)
+    ry, raq, rasc, _ = O.rmsnorm_quant(x, w, 1e-6, Mp=asc.shape[1])
+    assert (bits(h.cpu().numpy()) == bits(ry)).all() and (aq.cpu().numpy() == raq).all() and (bits(asc.cpu().numpy()) == bits(rasc)).all()
+
+
 # Few rows go by a thread per value (148 x 8 blocks of one row and 256 columns, with the SwiGLU product four times as many), more by a thread per
 # eight: the same bits, also for zeros, infinities, NaN and blocks whose 127 / amax overflows.
 @pytest.mark.parametrize("M,K", [(1, 256), (16, 512), (17, 768), (147, 2048), (148, 2048), (591, 2048), (592, 2048)])
