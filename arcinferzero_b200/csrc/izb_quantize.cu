@@ -153,8 +153,12 @@ __device__ __forceinline__ float cta_sum_ordered(float v, float* s_w) {
 
 // rows M..Mp-1 of a quantised activation buffer: zeros with scale 0 (one CTA per row, or columns c0 .. c1 - 1 of a row)
 __device__ __forceinline__ void zero_pad_cols(int m, int c0, int c1, int Mp, int K, int8_t* __restrict__ aq, float* __restrict__ asc, int16_t* __restrict__ absum) {
+  int8_t* row = aq + (size_t)m * K;
+  const bool wide = (reinterpret_cast<uintptr_t>(row) & 15) == 0;  // (add_norm_quant takes any alignment)
   for (int i = c0 / 16 + threadIdx.x; i < c1 / 16; i += blockDim.x) {
-    reinterpret_cast<uint4*>(aq + (size_t)m * K)[i] = make_uint4(0, 0, 0, 0);
+    if (wide) reinterpret_cast<uint4*>(row)[i] = make_uint4(0, 0, 0, 0);
+    else
+      for (int j = 0; j < 16; ++j) row[16 * i + j] = 0;
     if (!(i & 1)) asc[(size_t)(i >> 1) * Mp + m] = 0.0f;
     if (absum) absum[(size_t)i * Mp + m] = 0;
   }
@@ -490,13 +494,19 @@ int check_quant_args(const float* x, int ldx, int M, int Mp, int K, const int8_t
 
 }  // namespace
 
+// two byte ranges share memory
+static bool overlap(const void* a, size_t na, const void* b, size_t nb) {
+  const uintptr_t x = (uintptr_t)a, y = (uintptr_t)b;
+  return x < y + nb && y < x + na;
+}
+
 // Few rows -- blocks of one row that fit the device at once, four times as many with the SwiGLU product -- take a thread per value.  (us, a thread
 // per eight values / per value: quantise 1 x 5120 2.2 / 1.2, 32 x 768 2.1 / 1.2, 128 x 2048 2.1 / 2.0, 64 x 5120 2.2 / 2.3, 256 x 5120 3.7 / 5.9; SwiGLU 1 x
 // 17408 2.9 / 1.4, 32 x 5120 4.7 / 2.0, 64 x 17408 7.5 / 5.8, 100 x 17408 7.8 / 8.3, 512 x 5120 8.5 / 11.9.)
 template <int kMode>
 static int launch_quantize(const char* what, const float* x, int ldx, int M, int Mp, int K, int8_t* aq, float* asc, int16_t* absum, float* hout, cudaStream_t st) {
   const dim3 few(K / 256, M + (Mp > M ? 1 : 0));
-  if (izb_one_wave(dim3(few.x, kMode == 1 ? (few.y + 3) / 4 : few.y), 256)) {
+  if (izb_one_wave(dim3(few.x, kMode == 1 ? (few.y + 3) / 4 : few.y), 256) && Mp - M <= 256) {
     IZB_LAUNCH(what, st, izb_launch_pdl(quantize_few_kernel<kMode>, few, 256, 0, st, x, ldx, M, Mp, K, aq, asc, absum, hout, K));
   } else {
     dim3 grid(K / 256, (Mp + 31) / 32);
@@ -530,7 +540,11 @@ extern "C" int izb_rmsnorm_quant(const float* d_x, int ldx, const float* d_w, fl
   const int groups = (K / 8 + 255) / 256;  // of 8 values per thread
   // decode steps over long rows (us, a CTA per row / several: 4096, one row 2.0/1.8, eight 2.1/2.1; 5120, one 2.3/1.9, eight 2.4/2.2, sixteen 2.4/3.0; 12288, one
   // 3.6/2.7, eight 3.6/3.4; 2048, one 1.5/1.6)
-  if (M_valid <= 8 && K >= 4096 && groups <= 8) {
+  // (not over its own input, which other blocks still read)
+  const size_t xb = M_valid > 0 ? ((size_t)(M_valid - 1) * ldx + K) * 4 : 0;
+  const bool apart = !(d_h && overlap(d_x, xb, d_h, (size_t)M_valid * K * 4)) && !overlap(d_x, xb, d_aq, (size_t)Mp * K) && !overlap(d_x, xb, d_asc, (size_t)Mp * (K / 8)) &&
+                     !(d_absum && overlap(d_x, xb, d_absum, (size_t)Mp * (K / 8)));
+  if (M_valid <= 8 && K >= 4096 && groups <= 8 && Mp <= 65535 && apart) {
     auto kernel = groups <= 2 ? rmsnorm_few_kernel<2> : groups <= 3 ? rmsnorm_few_kernel<3> : groups <= 4 ? rmsnorm_few_kernel<4> : rmsnorm_few_kernel<8>;
     IZB_LAUNCH("rmsnorm_quant", st, izb_launch_pdl(kernel, dim3((K + 511) / 512, Mp), 256, 0, st, d_x, ldx, d_w, K, eps, M_valid, Mp, d_h, d_aq, d_asc, d_absum));
     return IZB_OK;

@@ -57,6 +57,45 @@ def test_norms_of_few_rows(izb, M, K):
     assert (bits(h.cpu().numpy()) == bits(ry)).all() and (aq.cpu().numpy() == raq).all() and (bits(asc.cpu().numpy()) == bits(rasc)).all()
 
 
+# The residual addition's outputs may lie anywhere (padding rows are zeroed 16 bytes at a time where they are aligned).
+@pytest.mark.parametrize("M,K,off", [(1, 1024, 1), (3, 2048, 4), (3, 2048, 0), (5, 5376, 8)])
+def test_add_norm_quant_unaligned_output(izb, M, K, off):
+    import ctypes as C
+    import torch
+    rng = np.random.default_rng(M + K)
+    x, t, w = (rng.standard_normal(n, dtype=np.float32) for n in ((M, K), (M, K), K))
+    xd, td, wd = (torch.from_numpy(a).cuda() for a in (x, t, w))
+    Mp = izb.pad_rows(M)
+    buf, asc = torch.full((Mp * K + 32,), 7, dtype=torch.int8, device="cuda"), torch.full((K // 32, Mp), 7.0, device="cuda")
+    p = lambda a, o=0: C.c_void_p(a.data_ptr() + o)
+    rc = izb.lib().izb_add_norm_quant(p(xd), p(td), p(wd), C.c_float(1e-6), C.c_float(1.0), p(wd), M, Mp, K, p(buf, off), p(asc), None, C.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0
+    _, raq, rasc, _ = O.add_norm_quant(x, t, w, 1e-6, 1.0, w, Mp=Mp)
+    got = buf.cpu().numpy()
+    assert (got[off:off + Mp * K].reshape(Mp, K) == raq).all() and (got[:off] == 7).all() and (got[off + Mp * K:] == 7).all()
+    assert (bits(asc.cpu().numpy()) == bits(rasc)).all()
+
+
+# The normalised rows may be written over the input (one block per row then), and a few rows may have any number of padding rows.
+@pytest.mark.parametrize("M,K", [(1, 5120), (5, 4096), (8, 12288)])
+def test_rmsnorm_quant_in_place(izb, M, K):
+    import ctypes as C
+    import torch
+    rng = np.random.default_rng(M + K)
+    x, w = rng.standard_normal((M, K), dtype=np.float32), rng.standard_normal(K, dtype=np.float32)
+    p = lambda a: C.c_void_p(a.data_ptr())
+    for Mp in (16, 1024):
+        xd, wd = torch.from_numpy(x).cuda(), torch.from_numpy(w).cuda()
+        aq, asc = torch.full((Mp, K), 7, dtype=torch.int8, device="cuda"), torch.full((K // 32, Mp), 7.0, device="cuda")
+        st = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+        assert izb.lib().izb_rmsnorm_quant(p(xd), K, p(wd), C.c_float(1e-6), M, Mp, K, p(xd), p(aq), p(asc), None, st) == 0
+        ry, raq, rasc, _ = O.rmsnorm_quant(x, w, 1e-6, Mp=Mp)
+        assert (bits(xd.cpu().numpy()) == bits(ry)).all() and (aq.cpu().numpy() == raq).all() and (bits(asc.cpu().numpy()) == bits(rasc)).all()
+        assert izb.lib().izb_quantize_act(p(xd), K, M, Mp, K, p(aq), p(asc), None, st) == 0
+        qaq, qasc, _ = O.quantize_act(ry, Mp=Mp)
+        assert (aq.cpu().numpy() == qaq).all() and (bits(asc.cpu().numpy()) == bits(qasc)).all()
+
+
 # Few rows go by a thread per value (148 x 8 blocks of one row and 256 columns, with the SwiGLU product four times as many), more by a thread per
 # eight: the same bits, also for zeros, infinities, NaN and blocks whose 127 / amax overflows.
 @pytest.mark.parametrize("M,K", [(1, 256), (16, 512), (17, 768), (147, 2048), (148, 2048), (591, 2048), (592, 2048)])
