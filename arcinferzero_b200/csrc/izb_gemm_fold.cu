@@ -18,7 +18,7 @@
 //
 // What bounds it: in long calls power.  The MMAs take 256 clk of a block and the whole 390, but at 1000 W the SM clock falls to some 1.45 GHz
 // (the kernel with one MMA per block keeps 1.94).  Measured, us with the quantiser, before and now: 8192 x 17408 x 5120 3079 / 2740,
-// 3401 x 4528 x 3584 275 / 242, 1108 x 4560 x 2048 76 / 56, 37 x 5120 x 5120 30.5 / 22.5, Q5_K 14 x 3920 x 16896 57 / 34.  Two-term weights
+// 3401 x 4528 x 3584 275 / 242, 1108 x 4560 x 2048 76 / 56, 37 x 5120 x 5120 30.5 / 18.9, Q5_K 14 x 3920 x 16896 57 / 30.  Two-term weights
 // (Q8_0, Q6_K) would need four MMAs per block and end up where the other kernel is (512 x 4096 x 4096 Q8_0 65 us at 1.75 GHz against 67 at 1.96).
 //
 // Plain stores of long K under IZB_GEMM_AUTO only, as with the cut of K: what the other store modes write is mostly quantised to int8 next, where a last

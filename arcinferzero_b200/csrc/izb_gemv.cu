@@ -72,7 +72,7 @@ int launch(const izb_weight* w, const uint8_t* raw, const int8_t* aq, const floa
 
 // Which of the two ways to the same bits is faster: the matrix instruction's cost does not grow with T but at T = 5, the dot-product kernels' does.
 // Measured (us, matrix instruction / dot products, calls back to back with weights that are not in L2; five rows and more behind a quantiser):
-//   Q6_K  32000 x 4096 T=1 22/27, T=4 24/52, T=8 38/95; 1024 x 1024 T=1 2.3/2.7, 5120 x 17408 T=1 26/27.  Few row tiles leave most of the chip idle
+//   Q6_K  32000 x 4096 T=1 22/27, T=4 24/52, T=8 38/95; 1024 x 1024 T=1 2.3/2.7, 5120 x 17408 T=1 19/27.  Few row tiles leave most of the chip idle
 //         over a long K: 256 x 8192 T=1 5.8/4.9, T=4 6.9/6.4, 256 x 4096 T=1 3.6/3.2, T=2 3.7/3.8, 384 x 8192 T=1 5.8/7.0; 128 x 8192 T=5 11/11, 48 x
 //         4096 T=5 7.3/7.9
 //   Q4_K  rows that are too long for the dot product's ring: 1024 x 10496 T=1 8.0/13, 4096 x 9472 T=1 8.6/8.2 (fits), T=2 9.4/14, 512 x 12544 T=4 10/14;

@@ -33,7 +33,7 @@
 // the first, so that each lane has half of the pieces and all of its work counts (mul4; the K = 32 instruction takes the tensor pipe's 8 clk like
 // the K = 16 one).  The sums are the same and in the same order; half as many accumulators also halve what the warps of a tile exchange.
 // (us before / now: Q6_K 151936 x 5120 three rows 149 / 118, 32000 x 4096 three 30 / 24; Q4_K 16384 x 5376 three 20.8 / 16.5, 5120 x 13824 four 27 /
-// 19; Q8_0 4096 x 14336 one 17.2 / 13.2, 8192 x 4096 four 8.8 / 7.8.)
+// 19; Q8_0 4096 x 14336 one 17.2 / 15.1, 8192 x 4096 four 8.8 / 7.8.)
 //
 // Measured (us, dot-product kernels / this one; the time at the copy's bandwidth): Q4_K 34816 x 5120 five rows 52.3 / 34.4 (15.3), eight
 // 75.7 / 35.1; 128000 x 4096 eight 218 / 89 (45); Q8_0 151936 x 2048 eight 136 / 57 (51); Q6_K 32000 x 4096 three 44 / 24 (17).  The

@@ -36,7 +36,7 @@ QT = 12
 SEED = 20261125
 WORKLOAD = "config2: Q4_K prefill GEMM M=8192 N=17408 K=5120 (quantiser + GEMM per step: one izb_quant_matmul call)"
 NOMINAL_INT8_TOPS = 4500.0
-NCU_TRAFFIC_BYTES_PER_TILE = (127.5e6 + 115.6e6) / (16 * 136)       # gemm_tc: ncu capture of 16 x 136 tiles of 128 x 128
+NCU_TRAFFIC_BYTES_PER_TILE = (159.7e6 + 121.0e6) / (16 * 136)       # gemm_tc (the folded kernel): ncu capture of 16 x 136 tiles of 128 x 128
 
 
 def peaks():
@@ -667,8 +667,8 @@ def main() -> None:
             "dtype": "int8",
             "data": "synthetic",
             "config": {"workload": WORKLOAD,
-                       "arithmetic": ("exact integer dot products per 32-block (int8 x 4-bit; operands fed to the tensor cores as fp16 "
-                                      "holding exact integers, f32 TMEM accumulators), f32 combine"),
+                       "arithmetic": ("int8 x 4-bit dot products per 32-block with the block scales in the operands (activations as two fp16 terms, 22 to 24 bits; "
+                                      "weight sub-scale x quant exact in fp16; f32 TMEM accumulators per 256 of K), f32 combine"),
                        "parallelism": f"weight rows split over {world} rank(s), no exchange",
                        "l2": "per step 168 MB of f32 activations in and 570 MB of outputs written: larger than the 126 MB L2",
                        "rows_per_rank": Nr},
@@ -678,7 +678,7 @@ def main() -> None:
                          "frac_of_measured_int8": achieved / tc_peaks["i8"]["burst_tops"], "frac_of_measured_f16_mma": achieved / tc_peaks["f16"]["burst_tops"],
                          "measured_tcgen05_peaks": dict(tc_peaks, method="izb_tensor_peak: tcgen05.mma 128x256 loop, operands in shared memory, accumulators in TMEM, all SMs"),
                          # DRAM bytes per launch: one ncu capture of the same kernel at 2048 token rows and all weight rows
-                         # (read 132.1 MB + written 116.6 MB), scaled by the 128x128 tiles this launch runs
+                         # (read 159.7 MB + written 121.0 MB), scaled by the 128x128 tiles this launch runs
                          "traffic": per_tile * ((M + 127) // 128) * (Nr // 128),
                          "traffic_source": f"ncu dram__bytes_read+write of {kname} at M=2048, N=17408 (profiles/), per 128x128 tile x tiles",
                          "ms_per_launch": ms_kernel, "launches": g["launches"],
