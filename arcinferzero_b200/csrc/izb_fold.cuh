@@ -30,4 +30,6 @@ size_t izb_fold_tail_bytes(int rows, int K);
 // pre-pass over rows already quantised (rows past `rows` count as zeros), or with the quantiser in it
 int izb_fold_prepare(const izb_weight* w, const int8_t* aq, const float* asc, int lda, int rows, const FoldParams& p, cudaStream_t st);
 int izb_fold_quant_prepare(const izb_weight* w, const float* x, int ldx, int M, int Mp, int8_t* aq, float* asc, const FoldParams& p, cudaStream_t st);
+// Do the kernels that quantise and prepare `rows` rows at once take one row per warp (blocks of 8 rows) instead of four?
+bool izb_one_row_per_warp(int rows, int K);
 int izb_fold_gemm(const izb_weight* w, const FoldParams& p, int grid, cudaStream_t st);

@@ -18,7 +18,7 @@
 //
 // What bounds it: in long calls power.  The MMAs take 256 clk of a block and the whole 390, but at 1000 W the SM clock falls to some 1.45 GHz
 // (the kernel with one MMA per block keeps 1.94).  Measured, us with the quantiser, before and now: 8192 x 17408 x 5120 3079 / 2740,
-// 3401 x 4528 x 3584 275 / 242, 1108 x 4560 x 2048 76 / 56, 37 x 5120 x 5120 30.5 / 18.9, Q5_K 14 x 3920 x 16896 57 / 30.  Two-term weights
+// 3401 x 4528 x 3584 275 / 242, 1108 x 4560 x 2048 76 / 56, 37 x 5120 x 5120 30.5 / 17.9, Q5_K 14 x 3920 x 16896 57 / 30.  Two-term weights
 // (Q8_0, Q6_K) would need four MMAs per block and end up where the other kernel is (512 x 4096 x 4096 Q8_0 65 us at 1.75 GHz against 67 at 1.96).
 //
 // Plain stores of long K under IZB_GEMM_AUTO only, as with the cut of K: what the other store modes write is mostly quantised to int8 next, where a last
@@ -381,21 +381,21 @@ __global__ void __launch_bounds__(256) fold_prepare_kernel(const int8_t* __restr
 // fold_prepare_kernel above in one pass over the f32 rows: a lane owns 8 consecutive values (= one 16-byte operand chunk),
 // four lanes a 32-block.  Writes aq / asc exactly as the quantiser does (the caller's buffers stay valid for every other
 // kernel) and, from the same registers, the operand images and what goes beside them: the int8 rows are not read back and the
-// second launch is gone.  One CTA = 32 rows x one superblock.
-template <bool kPerm>
+// second launch is gone.  One CTA = 8 kR rows x one superblock: four rows a warp, or one where that leaves SMs without work.
+template <bool kPerm, int kR>
 __global__ void __launch_bounds__(256) fold_quant_prepare_kernel(const float* __restrict__ x, int ldx, int M, int Mp, int K,
                                                             int8_t* __restrict__ aq, float* __restrict__ asc,
                                                             unsigned char* __restrict__ img, unsigned char* __restrict__ tail, int tt, int n_tiles,
                                                             uint32_t* __restrict__ part_bad) {
   __shared__ PrepRows s;
-  const int sb = blockIdx.x, nsb = K >> 8, m0 = blockIdx.y * 32, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int sb = blockIdx.x, nsb = K >> 8, m0 = blockIdx.y * (8 * kR), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int col = sb * 256 + lane * 8;
   pdl_launch_next();
   pdl_wait();
   if (part_bad && sb == 0 && blockIdx.y == 0 && threadIdx.x == 0) *part_bad = 0;
-  float v[4][8];
+  float v[kR][8];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < kR; ++i) {
     const int m = m0 + warp + 8 * i;
     if (m < M) {
       const float4* p = reinterpret_cast<const float4*>(x + (size_t)m * ldx + col);
@@ -408,7 +408,7 @@ __global__ void __launch_bounds__(256) fold_quant_prepare_kernel(const float* __
     }
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < kR; ++i) {
     const int rr = warp + 8 * i, m = m0 + rr;
     float amax = 0.0f;
 #pragma unroll
@@ -436,6 +436,7 @@ __global__ void __launch_bounds__(256) fold_quant_prepare_kernel(const float* __
       put_row<kPerm>(s, img + ((size_t)tile * nsb + sb) * kImgRow * tt, tt, m - tile * tt, rr, lane, sc, q);
   }
   __syncthreads();
+  if (lane >= 8 * kR) return;
   if (m0 + lane < Mp) asc[(size_t)(sb * 8 + warp) * Mp + m0 + lane] = s.sc[warp][lane];
   const int tile = (m0 + lane) / tt;
   if (tile < n_tiles) put_tail(s, tail + ((size_t)tile * nsb + sb) * kTailRow * tt, tt, m0 + lane - tile * tt, warp, lane);
@@ -917,8 +918,11 @@ int izb_fold_prepare(const izb_weight* w, const int8_t* aq, const float* asc, in
 
 int izb_fold_quant_prepare(const izb_weight* w, const float* x, int ldx, int M, int Mp, int8_t* aq, float* asc, const FoldParams& p, cudaStream_t st) {
   const int rows = p.n_mtiles * p.tt;  // (every row of every tile is written, rows past M as zeros)
-  dim3 grid(w->K / 256, ((rows > Mp ? rows : Mp) + 31) / 32);
-  auto kernel = w->type == IZB_Q4_K ? fold_quant_prepare_kernel<true> : fold_quant_prepare_kernel<false>;
+  const int all = rows > Mp ? rows : Mp;
+  const bool one = izb_one_row_per_warp(all, w->K);
+  dim3 grid(w->K / 256, one ? (all + 7) / 8 : (all + 31) / 32);
+  auto kernel = w->type == IZB_Q4_K ? (one ? fold_quant_prepare_kernel<true, 1> : fold_quant_prepare_kernel<true, 4>)
+                                    : one ? fold_quant_prepare_kernel<false, 1> : fold_quant_prepare_kernel<false, 4>;
   IZB_LAUNCH("quant_prepare", st, izb_launch_pdl(kernel, grid, 256, 0, st, x, ldx, M, Mp, w->K, aq, asc, p.img, p.tail, p.tt, p.n_mtiles, p.part_bad));
   return IZB_OK;
 }

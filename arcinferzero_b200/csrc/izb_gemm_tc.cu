@@ -287,15 +287,16 @@ __device__ __forceinline__ int q4k_perm8(int p) { return (p & 4) | ((p & 1) << 1
 struct PrepRows {
   float sc[8][33], v[8][33];  // [block of the superblock][row]: scale, scale * sum
 };
-// (after a barrier) the scales and, sps == 5, the min-term chunks of the 32 rows from row r0 of the tile on
+// (after a barrier) the scales and, sps == 5, the min-term chunks of the kN rows from row r0 of the tile on
+template <int kN>
 __device__ __forceinline__ void put_scales(const PrepRows& p, float* __restrict__ ascimg, uint8_t* tile_img, int tile, int K, int sb, int r0, int sps) {
   {
     const int b = threadIdx.x >> 5, r = threadIdx.x & 31;
-    ascimg[((size_t)tile * (K / 32) + sb * 8 + b) * BM + r0 + r] = p.sc[b][r];
+    if (r < kN) ascimg[((size_t)tile * (K / 32) + sb * 8 + b) * BM + r0 + r] = p.sc[b][r];
   }
   if (sps != 5) return;
   const int r = threadIdx.x >> 3, k = threadIdx.x & 7;
-  if (k >= 6) return;
+  if (k >= 6 || r >= kN) return;
   const int term = k == 2 || k == 4 ? 1 : k == 5 ? 2 : 0;
   uint32_t o[4];
 #pragma unroll
@@ -372,7 +373,7 @@ __global__ void __launch_bounds__(256) act_prepare_kernel(const int8_t* __restri
   }
   if (!asc) return;
   __syncthreads();
-  put_scales(s, ascimg, tile_img, tile, K, sb, m0, sps);
+  put_scales<32>(s, ascimg, tile_img, tile, K, sb, m0, sps);
 }
 
 // ---------------------------------------------------------------------------------------------- quantiser + pre-pass in one
@@ -380,23 +381,24 @@ __global__ void __launch_bounds__(256) act_prepare_kernel(const int8_t* __restri
 // act_prepare_kernel above in one pass over the f32 rows: a lane owns 8 consecutive values (= one 16-byte operand chunk),
 // four lanes a 32-block.  Writes aq / asc exactly as the quantiser does (the caller's buffers stay valid for every other
 // kernel) and, from the same registers, the operand images, the gathered scales and the min-term factors of the dense
-// tensor-core GEMM: the int8 rows are not read back and the second launch is gone.  One CTA = 32 rows x one superblock.
-template <bool kPerm>
+// tensor-core GEMM: the int8 rows are not read back and the second launch is gone.  One CTA = 8 kR rows x one superblock: four rows a
+// warp, or one where that leaves SMs without work.
+template <bool kPerm, int kR>
 __global__ void __launch_bounds__(256) quant_prepare_kernel(const float* __restrict__ x, int ldx, int M, int Mp, int K,
                                                             int8_t* __restrict__ aq, float* __restrict__ asc,
                                                             uint16_t* __restrict__ aimg, float* __restrict__ ascimg, int sps, int n_tiles,
                                                             uint32_t* __restrict__ part_bad) {
   __shared__ PrepRows s_rows;
-  const int sb = blockIdx.x, m0 = blockIdx.y * 32, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int sb = blockIdx.x, m0 = blockIdx.y * (8 * kR), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int col = sb * 256 + lane * 8;
-  const int tile = m0 >> 7;  // (32 rows lie in one tile)
+  const int tile = m0 >> 7;  // (the rows lie in one tile)
   uint8_t* tile_img = reinterpret_cast<uint8_t*>(aimg) + (size_t)tile * (K / 256) * sps * STAGE_BYTES;
   pdl_launch_next();
   pdl_wait();
   if (part_bad && sb == 0 && blockIdx.y == 0 && threadIdx.x == 0) *part_bad = 0;
-  float v[4][8];
+  float v[kR][8];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < kR; ++i) {
     const int m = m0 + warp + 8 * i;
     if (m < M) {
       const float4* p = reinterpret_cast<const float4*>(x + (size_t)m * ldx + col);
@@ -409,7 +411,7 @@ __global__ void __launch_bounds__(256) quant_prepare_kernel(const float* __restr
     }
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < kR; ++i) {
     const int rr = warp + 8 * i, m = m0 + rr;
     float amax = 0.0f;
 #pragma unroll
@@ -443,9 +445,9 @@ __global__ void __launch_bounds__(256) quant_prepare_kernel(const float* __restr
   __syncthreads();
   {
     const int b = threadIdx.x >> 5, r = threadIdx.x & 31;
-    if (m0 + r < Mp) asc[(size_t)(sb * 8 + b) * Mp + m0 + r] = s_rows.sc[b][r];
+    if (r < 8 * kR && m0 + r < Mp) asc[(size_t)(sb * 8 + b) * Mp + m0 + r] = s_rows.sc[b][r];
   }
-  if (tile < n_tiles) put_scales(s_rows, ascimg, tile_img, tile, K, sb, m0 & 127, sps);
+  if (tile < n_tiles) put_scales<8 * kR>(s_rows, ascimg, tile_img, tile, K, sb, m0 & 127, sps);
 }
 
 // ---------------------------------------------------------------------------------------------- the GEMM kernel
@@ -1302,11 +1304,17 @@ int izb_gemm_tc_quant_launch(const izb_weight* w, int mat, const float* x, int l
   float* ascimg = (float*)((unsigned char*)ws + img_bytes);
   float* split_ws = (float*)((unsigned char*)ws + img_bytes + asc_bytes);
   const int rows_img = n_tiles * BM > Mp ? n_tiles * BM : Mp;  // every row of every tile is written (rows past M as zeros)
-  dim3 grid(K / 256, (rows_img + 31) / 32);
-  auto kernel = w->type == IZB_Q4_K ? quant_prepare_kernel<true> : quant_prepare_kernel<false>;
+  const bool one = izb_one_row_per_warp(rows_img, K);
+  dim3 grid(K / 256, one ? (rows_img + 7) / 8 : (rows_img + 31) / 32);
+  auto kernel = w->type == IZB_Q4_K ? (one ? quant_prepare_kernel<true, 1> : quant_prepare_kernel<true, 4>) : one ? quant_prepare_kernel<false, 1> : quant_prepare_kernel<false, 4>;
   IZB_LAUNCH("quant_prepare", st, izb_launch_pdl(kernel, grid, 256, 0, st, x, ldx, M, Mp, K, aq, asc, aimg, ascimg, sps, n_tiles, split_flag(split_ws, w->device)));
   return run_tc_on(w, mat, aq, asc, Mp, Mp, nullptr, n_tiles, nullptr, nullptr, Mp, C, ldc, c_off, acc, nullptr, ws, split_ws, err, st, true);
 }
+
+// Up to one wave of the smaller blocks: in a short call a warp's four rows come one after the other while most SMs are idle (us, quantise + GEMM, four
+// rows a warp / one: Q4_K 37 x 5120 x 5120 18.4 / 17.4, 64 x 1024 x 2304 13.0 / 11.3, 256 x 1024 x 2304 14.6 / 13.6, Q6_K 37 x 2048 x 8192 22.5 / 21.9; 512 x 1024 x 1024
+// Q8_0 18.9 / 19.4).
+bool izb_one_row_per_warp(int rows, int K) { return izb_one_wave(dim3(K / 256, (rows + 7) / 8), 256); }
 
 // MoE on the tensor cores: the slots of each expert are tiles of up to 128 rows (izb_moe_sort with TM = 128); gate then up
 // with the fused-SwiGLU store mode (h = up * silu(gate)), down with the routing weight as row scale.

@@ -142,3 +142,19 @@ print("done")
 """
     r = subprocess.run([sys.executable, "-c", body], cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))), capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "done" in r.stdout, r.stdout + r.stderr
+
+
+# The quantiser that prepares the operands as it goes takes one row per warp up to one wave of such blocks (148 x 8), else four: the same bytes and products
+# as the quantiser and the pre-pass one after the other.
+@pytest.mark.parametrize("qt,N,K", [(12, 256, 2048), (13, 272, 2304), (8, 256, 2048), (14, 256, 2304)])
+@pytest.mark.parametrize("M", [9, 37, 100, 129, 1000, 1180, 1300])
+def test_quantising_pre_pass_equals_two_steps(izb, qt, N, K, M):
+    import torch
+    W = izb.Weight(qt, S.make_weight(qt, N, K, N + K), N, K)
+    x = torch.from_numpy(S.make_act(M, K, M)).cuda()
+    out, aq, asc = izb.quant_matmul(W, x, M)
+    bq, bsc, _ = izb.quantize_act(x)
+    assert torch.equal(aq, bq) and torch.equal(asc.view(torch.int32), bsc.view(torch.int32))
+    assert torch.equal(out[:M], izb.matmul(W, bq, bsc, M)[:M])
+    assert izb.device_status(0) == 0
+    W.close()
