@@ -4,7 +4,10 @@
 
 struct FoldParams {
   unsigned char* img;     // operand images: per token tile and superblock [lo, hi][4 stages of 64][tt rows][128 B], rows 128-byte swizzled
-  unsigned char* tail;    // per token tile and superblock [tt rows][16] fp16 min-term factors, [tt] f32 row scales s
+  unsigned char* fine;    // ... [4 stages of 64][tt rows][128 B], swizzled alike: the third term, of the rows that have one
+  unsigned char* tail;    // ... [tt rows][16] fp16 min-term factors, [tt] f32 row scales s, [tt] bytes: kinds of the rows
+  const float* asc;       // the activations' scales [K / 32][lda], read again for rows whose kind is wide
+  int lda;
   int tt;                 // token rows of a tile (a multiple of 16, at most 128)
   int n_mtiles;           // token tiles
   int M;                  // rows to store
@@ -26,6 +29,7 @@ static inline bool izb_fold_takes(const izb_weight* w) { return w->type == IZB_Q
 int izb_fold_tile_rows(int device, int M, int N);
 // scratch for n_mtiles * tt rows
 size_t izb_fold_img_bytes(int rows, int K);
+size_t izb_fold_fine_bytes(int rows, int K);
 size_t izb_fold_tail_bytes(int rows, int K);
 // pre-pass over rows already quantised (rows past `rows` count as zeros), or with the quantiser in it
 int izb_fold_prepare(const izb_weight* w, const int8_t* aq, const float* asc, int lda, int rows, const FoldParams& p, cudaStream_t st);

@@ -5,25 +5,30 @@
 // is an exact integer.  Both operands carry a scale per block.  Left out of the operands, the scales force every block's 128 x 128 dot products
 // through TMEM reads and an fma on the CUDA cores before the next block may be added: that, not the MMA, bounds such a kernel (550 clk per
 // 128 x 128 x 32 block).  Here they are folded into the operands and the accumulators leave TMEM once per superblock (256 of K):
-//   * activations: asc[m][b] * a as TWO fp16 terms.  Per row and superblock asc[m][b] = r[m][b] * s[m], s a 16th of the largest |asc|, so
-//     |r * a| <= 2^11; r * a = hi + lo, hi a multiple of 1/2 (of 1 from 2^10 on), lo = fp16(r * a - hi): 22 to 24 bits of the largest.
+//   * activations: asc[m][b] * a as TWO fp16 terms.  Per row and superblock asc[m][b] = r[m][b] * s[m], s a 128th of the largest |asc|, so
+//     |r * a| <= 2^14; r * a = hi + lo, hi a multiple of 4 or 8, lo = fp16(r * a - hi): 23 to 24 bits of the largest value.
 //     s is applied in f32.
 //   * weights: sub-scale * quant <= 1953, exact in one fp16 term.
 //   * so a block costs two MMAs (a_lo, a_hi), 256 clk of a 128 x 128 x 32 block, and the CUDA cores per superblock and element:
 //     res += s[m] * (d[n] * D - dmin[n] * D2).
 //   * D2[m][n] = sum_b (r * asum)[m][b] * mn[n][b]: one more MMA of K = 16 per superblock, the eight blocks' hi and lo terms.
+// Where a row's scales lie more than 4 : 1 apart inside a superblock, 24 bits of the largest block's values are too few of the smallest's: the large block's
+// weights may be zeros.  Such rows have a third term, on 16 more MMAs into an accumulator of its own; beyond 4096 : 1, and where a scale is no finite
+// number, the blocks are multiplied one by one (split_scale).  A tile whose rows are all plain in its part of K runs the loops of plain rows, and a
+// row's sums do not depend on what the others are.  (Two terms alone: 1.4e-6 of the result at 40 : 1, 2e-4 at 2^13 : 1.)
 // The tensor core adds in f32 but rounds towards zero, which would shrink every sum a little with every MMA (6e-7 of the result over a
-// superblock's 32).  Hence the order of a superblock's MMAs: first all with a_lo, on sums some 2^11 times smaller; then a_hi, whose products
-// and sums are halves of integers mostly below 2^23 and lose nothing but, once, the fraction that they found.
+// superblock's 32).  Hence the order of a superblock's MMAs: first all with a_lo, on sums some 2^12 times smaller; then a_hi, whose products
+// and sums are multiples of 4 or 8, mostly of less than 24 bits, and lose nothing but, once, the fraction that they found.
 //
 // What bounds it: in long calls power.  The MMAs take 256 clk of a block and the whole 390, but at 1000 W the SM clock falls to some 1.45 GHz
 // (the kernel with one MMA per block keeps 1.94).  Measured, us with the quantiser, before and now: 8192 x 17408 x 5120 3079 / 2740,
 // 3401 x 4528 x 3584 275 / 242, 1108 x 4560 x 2048 76 / 56, 37 x 5120 x 5120 30.5 / 17.9, Q5_K 14 x 3920 x 16896 57 / 30.  Two-term weights
 // (Q8_0, Q6_K) would need four MMAs per block and end up where the other kernel is (512 x 4096 x 4096 Q8_0 65 us at 1.75 GHz against 67 at 1.96).
+// With one block of every superblock 40 (2^15) times the others, all rows, us against the other kernel now: 8192 x 17408 x 5120 4126 (12207) / 2920, 1108 x
+// 4560 x 2048 87 (238) / 74, 300 x 5120 x 5120 69 (217) / 55, 37 x 5120 x 5120 26.8 (61) / 26.4, Q5_K 14 x 3920 x 16896 51 (116) / 51.
 //
 // Plain stores of long K under IZB_GEMM_AUTO only, as with the cut of K: what the other store modes write is mostly quantised to int8 next, where a last
-// bit can become a whole step, and they keep the sums that they had.  (These here lie nearer to 64 bits: relative error 1.3e-7 against 2e-7
-// to 1e-6 at K = 5120, where the other kernel's min term runs through the accumulator, rounded towards zero, over all of K.)
+// bit can become a whole step, and they keep the sums that they had.
 //
 // The weight rows are the MMA's M (TMEM lanes), the token rows its N (TMEM columns): a dequantiser thread owns a weight row and writes its
 // operand straight from registers to its TMEM lane (no shared-memory round trip, no swizzle), a short token tile costs a short MMA, and a
@@ -33,7 +38,7 @@
 //   warps 0-7    dequantisers, two groups of four: one thread per weight row; raw superblock -> fp16 operand in TMEM (four slots
 //                of 64 K-elements; group g fills slots g and g + 2), scales and mins to shared memory;
 //   warps 8-15   combine: once per superblock tcgen05.ld and the f32 arithmetic above; final store;
-//   warp 16      activation producer: cp.async.bulk of pre-swizzled operand images (made by the pre-pass) into a ring;
+//   warp 16      activation producer: cp.async.bulk of pre-swizzled operand images (made by the pre-pass) into a ring; finds out what rows are not plain;
 //   warp 17      producer of the row scales s and the min-term images;
 //   warp 18      weight producer: TMA (cp.async.bulk.tensor.2d) of the raw GGUF superblocks of 128 rows into a ring;
 //   warp 19      issues tcgen05.mma (one elected thread).
@@ -41,6 +46,8 @@
 // returns without storing (izb_device_status reports it).
 #include <cuda.h>
 #include <string.h>
+
+#include <type_traits>
 
 #include "izb_fold.cuh"
 
@@ -194,6 +201,11 @@ __device__ __forceinline__ unsigned long long pack2(float x) {
   asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x));
   return r;
 }
+__device__ __forceinline__ unsigned long long pair(float lo, float hi) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
 __device__ __forceinline__ float lo_f(unsigned long long a) { return __uint_as_float((uint32_t)a); }
 __device__ __forceinline__ float hi_f(unsigned long long a) { return __uint_as_float((uint32_t)(a >> 32)); }
 
@@ -244,7 +256,7 @@ struct Map {
   static constexpr int OFF_W2 = OFF_RAW + NR * RAW;                // 2 x [128 rows][16] fp16, the weights' side of the min term
   static constexpr int OFF_MIN = OFF_W2 + 2 * 4096;                // NM x [tokens][16] fp16, the activations' side
   static constexpr int OFF_S = OFF_MIN + NM * 4096;                // NM x [tokens] f32 row scales s
-  static constexpr int OFF_SCL = OFF_S + NM * 512;                 // 4 x 128 weight rows: f32 d, then f32 -2 dmin
+  static constexpr int OFF_SCL = OFF_S + NM * 512;                 // 4 x 128 weight rows: f32 d, then f32 -16 dmin
   static constexpr int SCL = 1024;
   static constexpr int OFF_BAR = OFF_SCL + 4 * SCL;
   static constexpr int SMEM_BYTES = OFF_BAR + 512 + 1024;          // barriers + alignment slack
@@ -253,12 +265,12 @@ struct Map {
                        RAW_EMPTY = RAW_FULL + NR, S_FULL = RAW_EMPTY + NR, S_EMPTY = S_FULL + NM, W2_FULL = S_EMPTY + NM, W2_EMPTY = W2_FULL + 2,
                        D_FULL = W2_EMPTY + 2, D_EMPTY = D_FULL + 2, D2_EMPTY = D_EMPTY + 2, NUM_BARS = D2_EMPTY + 1;
   static_assert(SMEM_BYTES <= 232448, "shared memory per CTA");
-  static_assert(NUM_BARS * 8 + 16 <= 512, "barrier area");
+  static_assert(NUM_BARS * 8 + 56 + 4 * NM <= 512, "barrier area");
   static_assert(OFF_RAW % 1024 == 0 && RAW % 1024 == 0 && OFF_W2 % 1024 == 0, "alignment of the operand and TMA areas");
 };
 
-// bytes per token row and superblock of the operand images, and of what goes beside them (min-term factors, s)
-constexpr int kImgRow = 1024, kTailRow = 36;
+// bytes per token row and superblock of the operand images, of the third term's, and of what goes beside them (min-term factors, s; kind)
+constexpr int kImgRow = 1024, kFineRow = 512, kTailCopy = 36, kTailRow = kTailCopy + 1;
 
 // position p (0..7) inside a 16-byte chunk of the Q4_K operand row holds element perm8[p] of that group of eight:
 // the order in which the dequantiser's two-nibbles-per-word extraction delivers them
@@ -269,52 +281,78 @@ __device__ __forceinline__ int q4k_perm8(int p) { return (p & 4) | ((p & 1) << 1
 // a lane per eight values (= one 16-byte chunk of an image); the images go out in whole 128-byte lines, what belongs to a row or block only
 // once is collected in shared memory first.
 struct PrepRows {
-  float sc[8][33], v[8][33];  // [block of the superblock][row]: activation scale, r * (sum of the quants) / 2
+  float sc[8][33], v[8][33];  // [block of the superblock][row]: activation scale, r * (sum of the quants) / 16
   float s[32];
+  unsigned char kind[32];
 };
-// asc = r * s for the eight blocks of a row's superblock; the whole warp calls it, lane l with block l / 4.  s is a 16th of the largest
-// |asc| (down at 2^-118 that itself, which would lose bits), or, where a scale is no finite number, that number: r is then 1 for the blocks
-// that have it and 0 for the others, whose part is lost beside it in any order of sums.
-struct RowScale { float r, s; };
+// asc = r * s for the eight blocks of a row's superblock; the whole warp calls it, lane l with block l / 4.  s is a 128th of the largest
+// |asc| (down at 2^-118 that itself, which would lose bits).  `kind`, for scales that differ more and more:
+//   kPlain   all r that are not 0 at least 32: hi + lo keep 21 to 22 bits of the smallest block's largest value
+//   kSpread  at least 2^-5: a third term, all three on grids that the blocks share.  (Finer grids for smaller blocks would do with two terms, but
+//            sums that larger blocks make long then lose those bits MMA by MMA and always towards zero: 5e-7 of the result for 256 : 1.)  s is negative.
+//   kWide    all else, also scales that are no finite numbers: r = 1 and s = 0, and the GEMM takes the blocks one by one
+enum : uint32_t { kPlain = 0, kSpread = 1, kWide = 2 };
+struct RowScale {
+  float r, s;
+  uint32_t kind;
+};
 __device__ __forceinline__ RowScale split_scale(float asc) {
+  constexpr uint32_t kAll = 0xFFFFFFFFu;
   const uint32_t mag = __float_as_uint(asc) & 0x7FFFFFFFu;
-  uint32_t mx = max(mag, __shfl_xor_sync(0xFFFFFFFFu, mag, 4));
-  mx = max(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, 8));
-  mx = max(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, 16));
+  uint32_t mx = max(mag, __shfl_xor_sync(kAll, mag, 4));
+  mx = max(mx, __shfl_xor_sync(kAll, mx, 8));
+  mx = max(mx, __shfl_xor_sync(kAll, mx, 16));
   const float m = __uint_as_float(mx);
-  RowScale o;
-  if (mx < 0x7F800000u) {
-    const bool tiny = m < 0x1p-118f;
-    o.s = tiny ? m : 0.0625f * m;
-    o.r = mx == 0 ? 0.0f : __fmul_rn(tiny ? 1.0f : 16.0f, __fdiv_rn(asc, m));
-  } else {
-    o.s = m;
-    o.r = mag >= 0x7F800000u ? copysignf(1.0f, asc) : 0.0f;
+  const bool tiny = m < 0x1p-118f;
+  RowScale o = {mag == 0 ? 0.0f : __fmul_rn(tiny ? 1.0f : 128.0f, __fdiv_rn(asc, m)), tiny ? m : 0.0078125f * m, kPlain};
+  if (__any_sync(kAll, mag != 0 && !(fabsf(o.r) >= 32.0f))) {
+    if (__any_sync(kAll, mx >= 0x7F800000u || (mag != 0 && !(fabsf(o.r) >= 0x1p-5f)))) o = {1.0f, 0.0f, kWide};
+    else o.s = -o.s, o.kind = kSpread;
   }
   return o;
 }
-// the chunk of eight values r * q: row `row` of a tile of tt rows, chunk `c` (0 .. 31) of a superblock
-template <bool kPerm>
-__device__ __forceinline__ void put_chunk(unsigned char* sb_img, int tt, int row, int c, float r, const int (&q)[8]) {
-  uint32_t hi[4], lo[4];
+// where a row's chunks go: the images of its tile and superblock, and the third term's
+struct RowImg {
+  unsigned char *img, *fine;
+  int tt, row;
+};
+__device__ __forceinline__ RowImg row_img(unsigned char* img, unsigned char* fine, size_t sb, int tt, int row) {
+  return {img + sb * kImgRow * tt, fine + sb * kFineRow * tt, tt, row};
+}
+// the chunk of eight values r * q, chunk `c` (0 .. 31) of a superblock: hi a multiple of 4, of 8 from 2^13 on; a spread row's lo a multiple of 2^-9; a wide row's
+// hi all of q.  Q5_K, whose weights have a bit more, hi a multiple of 8 (plain rows' of 4 while r is below 64): of two errors that grow in opposite
+// directions, the bits that the tensor core's sums lose and lo's own, the smaller sum (K = 2048 and 5120: 1.2e-7, multiples of 4 1.5e-7; Q4_K 1.1e-7).
+template <bool kQ4K>
+__device__ __forceinline__ void put_chunk(const RowImg& o, int c, const RowScale& rs, const int (&q)[8]) {
+  uint32_t hi[4], lo[4], fine[4];
+  // x + round - round: x as a multiple of round / (1.5 * 2^23)
+  const float round = rs.kind == kWide ? 0x1.8p23f : kQ4K || (rs.kind == kPlain && fabsf(rs.r) < 64.0f) ? 0x1.8p25f : 0x1.8p26f;
+  constexpr float kRoundLo = 0x1.8p14f;
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    const float x = (float)q[kPerm ? q4k_perm8(2 * j) : 2 * j], y = (float)q[kPerm ? q4k_perm8(2 * j + 1) : 2 * j + 1];
-    constexpr float kRound = 6291456.0f;  // 1.5 * 2^22: the sum's last place is 1/2
-    const __half2 h = __floats2half2_rn(__fsub_rn(__fmaf_rn(r, x, kRound), kRound), __fsub_rn(__fmaf_rn(r, y, kRound), kRound));
+    const float x = (float)q[kQ4K ? q4k_perm8(2 * j) : 2 * j], y = (float)q[kQ4K ? q4k_perm8(2 * j + 1) : 2 * j + 1];
+    const __half2 h = __floats2half2_rn(__fsub_rn(__fmaf_rn(rs.r, x, round), round), __fsub_rn(__fmaf_rn(rs.r, y, round), round));
     const float2 hf = __half22float2(h);
+    float2 rest = make_float2(__fmaf_rn(rs.r, x, -hf.x), __fmaf_rn(rs.r, y, -hf.y));
     hi[j] = h2_bits(h);
-    lo[j] = h2_bits(__floats2half2_rn(__fmaf_rn(r, x, -hf.x), __fmaf_rn(r, y, -hf.y)));
+    if (rs.kind == kSpread) {
+      const float2 l = make_float2(__fsub_rn(__fadd_rn(rest.x, kRoundLo), kRoundLo), __fsub_rn(__fadd_rn(rest.y, kRoundLo), kRoundLo));
+      fine[j] = h2_bits(__floats2half2_rn(__fsub_rn(rest.x, l.x), __fsub_rn(rest.y, l.y)));
+      rest = l;
+    }
+    lo[j] = h2_bits(__floats2half2_rn(rest.x, rest.y));
   }
-  unsigned char* o = sb_img + (size_t)(c >> 3) * 128 * tt + row * 128 + (((c & 7) ^ (row & 7)) << 4);
-  *reinterpret_cast<uint4*>(o) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-  *reinterpret_cast<uint4*>(o + 512 * tt) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+  const size_t at = (size_t)(c >> 3) * 128 * o.tt + o.row * 128 + (((c & 7) ^ (o.row & 7)) << 4);
+  *reinterpret_cast<uint4*>(o.img + at) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+  *reinterpret_cast<uint4*>(o.img + at + 512 * o.tt) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+  if (rs.kind == kSpread) *reinterpret_cast<uint4*>(o.fine + at) = make_uint4(fine[0], fine[1], fine[2], fine[3]);
 }
 // (after a barrier, the whole CTA) what goes beside the images, for the lane's row: row r of a tile
 __device__ __forceinline__ void put_tail(const PrepRows& p, unsigned char* sb_tail, int tt, int r, int warp, int lane) {
   if (warp > 2) return;
   if (warp == 2) {
     reinterpret_cast<float*>(sb_tail + 32 * tt)[r] = p.s[lane];
+    sb_tail[36 * tt + r] = p.kind[lane];
     return;
   }
   uint32_t o[4];  // warp 0: the eight hi terms, warp 1: the eight lo terms
@@ -332,19 +370,19 @@ __device__ __forceinline__ void put_tail(const PrepRows& p, unsigned char* sb_ta
 }
 // one row's images from its int8 values and their block's scale (this lane's eight and its block's)
 template <bool kPerm>
-__device__ __forceinline__ void put_row(PrepRows& p, unsigned char* sb_img, int tt, int r, int row, int lane, float asc, const int (&q)[8]) {
+__device__ __forceinline__ void put_row(PrepRows& p, const RowImg& o, int row, int lane, float asc, const int (&q)[8]) {
   const RowScale rs = split_scale(asc);
-  put_chunk<kPerm>(sb_img, tt, r, lane, rs.r, q);
+  put_chunk<kPerm>(o, lane, rs, q);
   int sum = q[0] + q[1] + q[2] + q[3] + q[4] + q[5] + q[6] + q[7];
   sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 1);
   sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 2);  // the four chunks of a 32-block
-  if ((lane & 3) == 0) p.v[lane >> 2][row] = __fmul_rn(rs.r, 0.5f * (float)sum);  // (at most 2^15)
-  if (lane == 0) p.s[row] = rs.s;
+  if ((lane & 3) == 0) p.v[lane >> 2][row] = __fmul_rn(rs.r, 0.0625f * (float)sum);  // (at most 2^15)
+  if (lane == 0) p.s[row] = rs.s, p.kind[row] = (unsigned char)rs.kind;
 }
 
 template <bool kPerm>
 __global__ void __launch_bounds__(256) fold_prepare_kernel(const int8_t* __restrict__ aq, const float* __restrict__ asc, int lda, int K, int rows_total,
-                                                           unsigned char* __restrict__ img, unsigned char* __restrict__ tail, int tt, int n_rows,
+                                                           unsigned char* __restrict__ img, unsigned char* __restrict__ fine, unsigned char* __restrict__ tail, int tt, int n_rows,
                                                            uint32_t* __restrict__ part_bad) {
   __shared__ PrepRows s;
   const int sb = blockIdx.y, nsb = K >> 8, m0 = blockIdx.x * 32, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -369,7 +407,7 @@ __global__ void __launch_bounds__(256) fold_prepare_kernel(const int8_t* __restr
       a[k] = (int)(int8_t)(x[i].x >> (8 * k));
       a[4 + k] = (int)(int8_t)(x[i].y >> (8 * k));
     }
-    put_row<kPerm>(s, img + ((size_t)tile * nsb + sb) * kImgRow * tt, tt, m - tile * tt, rr, lane, s.sc[lane >> 2][rr], a);
+    put_row<kPerm>(s, row_img(img, fine, (size_t)tile * nsb + sb, tt, m - tile * tt), rr, lane, s.sc[lane >> 2][rr], a);
   }
   __syncthreads();
   const int m = m0 + lane, tile = m / tt;
@@ -385,7 +423,7 @@ __global__ void __launch_bounds__(256) fold_prepare_kernel(const int8_t* __restr
 template <bool kPerm, int kR>
 __global__ void __launch_bounds__(256) fold_quant_prepare_kernel(const float* __restrict__ x, int ldx, int M, int Mp, int K,
                                                             int8_t* __restrict__ aq, float* __restrict__ asc,
-                                                            unsigned char* __restrict__ img, unsigned char* __restrict__ tail, int tt, int n_tiles,
+                                                            unsigned char* __restrict__ img, unsigned char* __restrict__ fine, unsigned char* __restrict__ tail, int tt, int n_tiles,
                                                             uint32_t* __restrict__ part_bad) {
   __shared__ PrepRows s;
   const int sb = blockIdx.x, nsb = K >> 8, m0 = blockIdx.y * (8 * kR), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -433,7 +471,7 @@ __global__ void __launch_bounds__(256) fold_quant_prepare_kernel(const float* __
     if ((lane & 3) == 0) s.sc[lane >> 2][rr] = sc;
     const int tile = m / tt;
     if (tile < n_tiles)  // (padding rows past the last tile the GEMM reads: aq / asc only)
-      put_row<kPerm>(s, img + ((size_t)tile * nsb + sb) * kImgRow * tt, tt, m - tile * tt, rr, lane, sc, q);
+      put_row<kPerm>(s, row_img(img, fine, (size_t)tile * nsb + sb, tt, m - tile * tt), rr, lane, sc, q);
   }
   __syncthreads();
   if (lane >= 8 * kR) return;
@@ -465,7 +503,7 @@ struct DeqQ4K {
   }
   __device__ __forceinline__ void put_scales(unsigned char* scl, int t) const {
     reinterpret_cast<float*>(scl)[t] = half_bits_to_float(hdr.x & 0xFFFFu);
-    reinterpret_cast<float*>(scl)[128 + t] = -2.0f * half_bits_to_float(hdr.x >> 16);
+    reinterpret_cast<float*>(scl)[128 + t] = -16.0f * half_bits_to_float(hdr.x >> 16);
   }
   template <int kH>
   __device__ __forceinline__ void half(int c, uint32_t (&o)[16]) const {
@@ -506,7 +544,7 @@ struct DeqQ5K {
   }
   __device__ __forceinline__ void put_scales(unsigned char* scl, int t) const {
     reinterpret_cast<float*>(scl)[t] = __uint_as_float(h0.x);
-    reinterpret_cast<float*>(scl)[128 + t] = -2.0f * __uint_as_float(h0.y);
+    reinterpret_cast<float*>(scl)[128 + t] = -16.0f * __uint_as_float(h0.y);
   }
   __device__ __forceinline__ void load_stage(int c, const unsigned char* row) {
 #pragma unroll
@@ -551,6 +589,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fold_kernel(const __grid_con
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + MP::OFF_BAR);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + MP::OFF_BAR + MP::NUM_BARS * 8);
   volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(smem + MP::OFF_BAR + MP::NUM_BARS * 8 + 4);
+  uint32_t* unit_kinds = reinterpret_cast<uint32_t*>(smem + MP::OFF_BAR + MP::NUM_BARS * 8 + 8);  // [4], items with rows that are not plain: superblocks in turn
+  uint32_t* s_kinds = unit_kinds + 4;                                                                // [NM], with the ring of scales
+  uint32_t *unit_item = s_kinds + NM, *s_item = unit_item + 4;                                       // [4] each, items in turn
   const uint32_t bar0 = smem_u32(bars);
   auto bar = [&](int i) -> uint32_t { return bar0 + 8u * (uint32_t)i; };
   // (through a shuffle: the compiler then knows that the role branches and what follows from them are the same for the whole warp, and keeps
@@ -599,6 +640,23 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fold_kernel(const __grid_con
     return it;
   };
 
+  // Kinds of a tile's rows.  Both producers of the token side look them up, the issuer and the combine warps find them in shared memory: for an item, whose
+  // loops then are those for plain rows alone or the longer ones, and in the latter for a superblock (`sb` of all tiles').
+  auto load_kinds = [&](size_t sb, int n) -> uint32_t {
+    return 4 * lane < n ? *reinterpret_cast<const uint32_t*>(p.tail + sb * kTailRow * p.tt + kTailCopy * p.tt + 4 * lane) : 0u;
+  };
+  auto all_kinds = [&](uint32_t k) -> uint32_t {
+    k = __reduce_or_sync(0xFFFFFFFFu, k);
+    k |= k >> 16;
+    return (k | k >> 8) & 3u;
+  };
+  auto item_kinds = [&](const Item& it) -> uint32_t {
+    uint32_t k = 0;
+#pragma unroll 8
+    for (int s = it.s0; s < it.s1; ++s) k |= load_kinds((size_t)it.tile * nsb + s, it.n);
+    return all_kinds(k);
+  };
+
   if (warp >= 16) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsOther));
     // Every role loop below is executed by its whole warp (uniform waits, an elected lane issues), so no lane of a role warp
@@ -606,43 +664,84 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fold_kernel(const __grid_con
     if (warp == 16) {
       // ================= activation producer: the tile's stage images lie back to back in global memory
       pdl_wait();  // (the pre-pass; the weights depend on no kernel and are on their way by then)
-      int sa = 0, pa = 1;
+      int sa = 0, pa = 1, sbc = 0, n_item = 0;
       bool ok = true;
-      for (int w = blockIdx.x; w < n_work && ok; w += gridDim.x) {
+      for (int w = blockIdx.x; w < n_work && ok; w += gridDim.x, ++n_item) {
         const Item it = item(w);
         const uint32_t half = (uint32_t)it.n * 128;  // bytes of a stage; a unit of the ring is two of them
-        const unsigned char* src = p.img + (size_t)it.tile * nsb * kImgRow * p.tt;
-        for (int g = it.s0 * UNITS; g < it.s1 * UNITS; ++g) {
-          if (!mbar_wait_warp(bar(MP::A_EMPTY + sa), pa, abort_flag, p.err, p.spin_limit, E_APROD)) { ok = false; break; }
-          if (lane == 0 && g != p.skip_stage) {  // (skip_stage: diagnostics only, makes the waits of this unit run out)
-            const uint32_t dst = smem_u32(smem + MP::OFF_A + sa * UNIT_BYTES);
-            const unsigned char* s = src + (size_t)g * 256 * p.tt;
+        const int step = 256 * p.tt;
+        auto copy = [&](const unsigned char* src) {
+          const uint32_t dst = smem_u32(smem + MP::OFF_A + sa * UNIT_BYTES);
+          if (it.n == p.tt) {
+            bulk_g2s(dst, src, 2 * half, bar(MP::A_FULL + sa));
+          } else {
+            bulk_g2s(dst, src, half, bar(MP::A_FULL + sa));
+            bulk_g2s(dst + half, src + 128 * p.tt, half, bar(MP::A_FULL + sa));
+          }
+        };
+        auto next = [&]() { if (++sa == NA) { sa = 0; pa ^= 1; } };
+        auto unit = [&](const unsigned char* src, bool skip) -> bool {
+          if (!mbar_wait_warp(bar(MP::A_EMPTY + sa), pa, abort_flag, p.err, p.spin_limit, E_APROD)) return false;
+          if (lane == 0 && !skip) {
             mbar_expect_tx(bar(MP::A_FULL + sa), 2 * half);
-            if (it.n == p.tt) {
-              bulk_g2s(dst, s, 2 * half, bar(MP::A_FULL + sa));
-            } else {
-              bulk_g2s(dst, s, half, bar(MP::A_FULL + sa));
-              bulk_g2s(dst + half, s + 128 * p.tt, half, bar(MP::A_FULL + sa));
-            }
+            copy(src);
           }
           __syncwarp();
-          if (++sa == NA) { sa = 0; pa ^= 1; }
+          next();
+          return true;
+        };
+        const size_t sb0 = (size_t)it.tile * nsb;
+        const unsigned char* src = p.img + sb0 * kImgRow * p.tt;
+        // the item's first unit: its bytes are on their way while the kinds are looked up, and count as arrived with this thread's arrival
+        if (!mbar_wait_warp(bar(MP::A_EMPTY + sa), pa, abort_flag, p.err, p.spin_limit, E_APROD)) break;
+        const bool skip = it.s0 * UNITS == p.skip_stage;  // (skip_stage: diagnostics only, makes the waits of this unit run out)
+        if (lane == 0 && !skip) copy(src + (size_t)(it.s0 * UNITS) * step);
+        __syncwarp();
+        const uint32_t any = item_kinds(it);
+        uint32_t more = any ? all_kinds(load_kinds(sb0 + it.s0, it.n)) : 0u;
+        if (lane == 0) {
+          unit_item[n_item & 3] = any;
+          unit_kinds[sbc & 3] = more;
+          if (!skip) mbar_expect_tx(bar(MP::A_FULL + sa), 2 * half);
+        }
+        __syncwarp();
+        next();
+        if (!any) {
+          for (int g = it.s0 * UNITS + 1; g < it.s1 * UNITS && ok; ++g) ok = unit(src + (size_t)g * step, g == p.skip_stage);
+          sbc += it.s1 - it.s0;
+          continue;
+        }
+        for (int s = it.s0; s < it.s1 && ok; ++s, ++sbc) {
+          const uint32_t ahead = s + 1 < it.s1 ? load_kinds(sb0 + s + 1, it.n) : 0u;
+          const unsigned char *u = src + (size_t)(s * UNITS) * step, *fine = p.fine + (sb0 + s) * kFineRow * p.tt;
+          if (s > it.s0) {
+            if (lane == 0) unit_kinds[sbc & 3] = more;  // (before this thread's arrival for the unit)
+            ok = unit(u, s * UNITS == p.skip_stage);
+          }
+          if (ok && (more & kSpread)) ok = unit(fine, false) && unit(fine + step, false);
+          for (int i = 1; i < UNITS && ok; ++i) ok = unit(u + i * step, s * UNITS + i == p.skip_stage);
+          more = all_kinds(ahead);
         }
       }
     } else if (warp == 17) {
       // ================= per superblock: row scales and the min term's activation side
       pdl_wait();
-      int sq = 0, pq = 1;
+      int sq = 0, pq = 1, n_item = 0;
       bool ok = true;
-      for (int w = blockIdx.x; w < n_work && ok; w += gridDim.x) {
+      for (int w = blockIdx.x; w < n_work && ok; w += gridDim.x, ++n_item) {
         const Item it = item(w);
         const size_t sb_bytes = (size_t)kTailRow * p.tt;
         const unsigned char* src = p.tail + ((size_t)it.tile * nsb + it.s0) * sb_bytes;
+        const uint32_t any = item_kinds(it);
         for (int s = it.s0; s < it.s1; ++s, src += sb_bytes) {
+          uint32_t more = 0;
+          if (any) more = all_kinds(load_kinds((size_t)it.tile * nsb + s, it.n));
           if (!mbar_wait_warp(bar(MP::S_EMPTY + sq), pq, abort_flag, p.err, p.spin_limit, E_WPROD)) { ok = false; break; }
           const uint32_t dst = smem_u32(smem + MP::OFF_S + sq * 512), full = bar(MP::S_FULL + sq);
           if (lane == 0) {
-            mbar_expect_tx(full, it.n * kTailRow);
+            if (s == it.s0) s_item[n_item & 3] = any;  // (before this thread's arrival)
+            s_kinds[sq] = more;
+            mbar_expect_tx(full, it.n * kTailCopy);
             bulk_g2s(smem_u32(smem + MP::OFF_MIN + sq * 4096), src, it.n * 32, full);
             bulk_g2s(dst, src + 32 * p.tt, it.n * 4, full);
           }
@@ -671,8 +770,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fold_kernel(const __grid_con
       // ================= MMA issuer
       bool ok = true;
       const bool leader = elect_one();
-      int sa = 0, pa = 0, sq = 0, pq = 0, d = 0, pd = 1, sbc = 0;  // ring positions and wait parities, superblocks done: they run on across items
-      for (int w = blockIdx.x; w < n_work && ok; w += gridDim.x) {
+      int sa = 0, pa = 0, sq = 0, pq = 0, d = 0, pd = 1, sbc = 0, n_item = 0;  // ring positions and wait parities, superblocks and items done: they run on across items
+      for (int w = blockIdx.x; w < n_work && ok; w += gridDim.x, ++n_item) {
         const Item it = item(w);
         const uint32_t idesc = umma_idesc(it.n), half = (uint32_t)it.n * 128;
         // K = 16 step k of stage c's weights x an activation stage
@@ -681,6 +780,132 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fold_kernel(const __grid_con
         };
         auto a_base = [&](int u) -> uint32_t { return smem_u32(smem + MP::OFF_A + u * UNIT_BYTES); };
         auto next = [&]() { if (++sa == NA) { sa = 0; pa ^= 1; } };
+        // (the item's first unit tells which of the two loops)
+        if (!mbar_wait_warp(bar(MP::A_FULL + sa), pa, abort_flag, p.err, p.spin_limit, E_MMA)) break;
+        if (__shfl_sync(0xFFFFFFFFu, unit_item[n_item & 3], 0)) {  // (a shuffle: see `warp`)
+          // with rows that are not plain
+          auto wait = [&](int b, int parity) -> bool { return mbar_wait_warp(bar(b), (uint32_t)parity, abort_flag, p.err, p.spin_limit, E_MMA); };
+          auto next_d = [&]() { if (++d == ND) { d = 0; pd ^= 1; } };
+          struct Place { int u, parity; };  // in the ring of units, `ahead` places on
+          auto place = [&](int ahead) -> Place {
+            Place o = {sa, pa};
+            for (int i = 0; i < ahead; ++i)
+              if (++o.u == NA) { o.u = 0; o.parity ^= 1; }
+            return o;
+          };
+          auto unit = [&](Place at) -> Wait { return {bar(MP::A_FULL + at.u), (uint32_t)at.parity}; };
+          // (the leader) eight K steps, half h of the superblock
+          auto issue = [&](int u, uint32_t dt, int h, bool fresh, bool last) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              mma(dt, 2 * h + (e >> 2), e & 3, a_base(u) + (e >> 2) * half, fresh && e == 0 ? 0u : 1u);
+              if ((e & 3) == 3 && last) tc_commit(bar(MP::W_EMPTY + 2 * h + (e >> 2)));
+            }
+          };
+          // one superblock.  Compiled for each of the common combinations of kinds: tests of them between its MMAs cost these their uniform registers
+          // (1108 x 4560 x 2048: 66 us with all rows plain in this loop, 51 in the one below)
+          auto superblock = [&](auto spread_known, auto wide_known) -> bool {
+            const bool spread = decltype(spread_known)::value, wide = decltype(wide_known)::value;
+            const int b = sbc & 1;
+            const uint32_t pw = b;
+            const Place lo0 = place(0);
+            const Wait w2{bar(MP::W_FULL + 2), pw}, w3{bar(MP::W_FULL + 3), pw};
+            const int at = spread ? 3 : 1;
+            if (spread) {
+              // the third term, into an accumulator of its own.  Before the others, although the first of those lies before it in the ring: the combine
+              // warps take it while these run, and the next superblock's while they take these
+              const Place f0 = place(1), f1 = place(2);
+              const Wait need[4] = {unit(f0), unit(f1), w2, w3};
+              if (!mbar_wait_warp(need, abort_flag, p.err, p.spin_limit, E_MMA)) return false;
+              tc_fence_after();
+              if (leader) {
+                const uint32_t dt = tmem_base + (uint32_t)(TM_D + d * BT);
+                issue(f0.u, dt, 0, true, false);
+                tc_commit(bar(MP::A_EMPTY + f0.u));
+                issue(f1.u, dt, 1, false, false);
+                tc_commit(bar(MP::A_EMPTY + f1.u));
+                tc_commit(bar(MP::D_FULL + d));
+              }
+              __syncwarp();
+              next_d();
+            }
+            const Place lo1 = place(at), hi0 = place(at + 1), hi1 = place(at + 2);
+            const uint32_t dt = tmem_base + (uint32_t)(TM_D + d * BT);
+            const Wait need[4] = {{bar(MP::D_EMPTY + d), (uint32_t)pd}, unit(lo1), w2, w3};
+            if (!mbar_wait_warp(need, abort_flag, p.err, p.spin_limit, E_MMA)) return false;
+            tc_fence_after();
+            if (leader) {
+              issue(lo0.u, dt, 0, true, false);
+              tc_commit(bar(MP::A_EMPTY + lo0.u));
+              issue(lo1.u, dt, 1, false, false);
+              tc_commit(bar(MP::A_EMPTY + lo1.u));
+            }
+            __syncwarp();
+#pragma unroll 1
+            for (int h = 0; h < 2; ++h) {
+              const Place hi = h ? hi1 : hi0;
+              if (!wait(MP::A_FULL + hi.u, hi.parity)) return false;
+              tc_fence_after();
+              if (leader) {
+                issue(hi.u, dt, h, false, !wide);
+                if (!wide) tc_commit(bar(MP::A_EMPTY + hi.u));
+              }
+              __syncwarp();
+            }
+            const Wait w2_full{bar(MP::W2_FULL + b), (uint32_t)(sbc >> 1) & 1u}, s_full{bar(MP::S_FULL + sq), (uint32_t)pq};
+            const Wait min_term[4] = {w2_full, s_full, {bar(MP::D2_EMPTY), pw ^ 1u}, s_full};
+            if (!mbar_wait_warp(min_term, abort_flag, p.err, p.spin_limit, E_MMA)) return false;
+            tc_fence_after();
+            if (leader) {
+              tc_mma_ss(tmem_base + TM_D2, umma_desc32(smem_u32(smem + MP::OFF_W2 + b * 4096)), umma_desc32(smem_u32(smem + MP::OFF_MIN + sq * 4096)), idesc, 0);
+              if (!wide) tc_commit(bar(MP::W2_EMPTY + b));
+              tc_commit(bar(MP::S_EMPTY + sq));
+              tc_commit(bar(MP::D_FULL + d));
+            }
+            __syncwarp();
+            if (++sq == NM) { sq = 0; pq ^= 1; }
+            next_d();
+            if (wide) {
+              // the hi images once more, whose wide rows are whole numbers (their lo images are zeros): block by block, each into an accumulator of its own
+#pragma unroll 1
+              for (int blk = 0; blk < 8; ++blk) {
+                if (!wait(MP::D_EMPTY + d, pd)) return false;
+                tc_fence_after();
+                if (leader) {
+                  const uint32_t a = a_base(blk < 4 ? hi0.u : hi1.u) + (blk >> 1 & 1) * half, to = tmem_base + (uint32_t)(TM_D + d * BT);
+                  mma(to, blk >> 1, 2 * (blk & 1), a, 0u);
+                  mma(to, blk >> 1, 2 * (blk & 1) + 1, a, 1u);
+                  tc_commit(bar(MP::D_FULL + d));
+                }
+                __syncwarp();
+                next_d();
+              }
+              if (leader) {
+#pragma unroll
+                for (int c = 0; c < 4; ++c) tc_commit(bar(MP::W_EMPTY + c));
+                tc_commit(bar(MP::A_EMPTY + hi0.u));
+                tc_commit(bar(MP::A_EMPTY + hi1.u));
+              }
+              __syncwarp();
+              // (the combine warps read the weights' side of the min term: it is free when they are done with the last block's accumulator)
+              const int e = d + 1 < ND ? d + 1 : 0;
+              if (!wait(MP::D_EMPTY + e, e ? pd : pd ^ 1)) return false;
+              mbar_arrive_if(bar(MP::W2_EMPTY + b), lane == 0);
+            }
+            for (int i = 0; i < at + 3; ++i) next();
+            return true;
+          };
+          using Yes = std::true_type;
+          using No = std::false_type;
+          for (int s = it.s0; s < it.s1 && ok; ++s, ++sbc) {
+            const Wait first[4] = {unit(place(0)), {bar(MP::W_FULL), (uint32_t)(sbc & 1)}, {bar(MP::W_FULL + 1), (uint32_t)(sbc & 1)}, {bar(MP::D_EMPTY + d), (uint32_t)pd}};
+            ok = mbar_wait_warp(first, abort_flag, p.err, p.spin_limit, E_MMA);
+            if (!ok) break;
+            const uint32_t more = __shfl_sync(0xFFFFFFFFu, unit_kinds[sbc & 3], 0);
+            ok = more == 0 ? superblock(No{}, No{}) : more == kSpread ? superblock(Yes{}, No{}) : more == kWide ? superblock(No{}, Yes{}) : superblock(Yes{}, Yes{});
+          }
+          continue;
+        }
         for (int s = it.s0; s < it.s1 && ok; ++s, ++sbc) {
           const uint32_t pw = sbc & 1;
           // a superblock: the lo images (two units of two stages), then the hi images, all into one accumulator; the min term into its own
@@ -785,8 +1010,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fold_kernel(const __grid_con
     const uint32_t t_lane = tmem_base + ((uint32_t)(32 * q) << 16);
     auto column = [&](int i) -> int { return 32 * (grp + 2 * i); };
     bool ok = true;
-    int d = 0, pd = 0, sq = 0, pq = 0, sbc = 0;
-    for (int w = blockIdx.x; w < n_work && ok; w += gridDim.x) {
+    int d = 0, pd = 0, sq = 0, pq = 0, sbc = 0, n_item = 0;
+    for (int w = blockIdx.x; w < n_work && ok; w += gridDim.x, ++n_item) {
       __syncwarp();
       const Item it = item(w);
       unsigned long long res[NCH][2][8];  // [group][rows 16 hr ..][2 g + r]: row 16 hr + 8 r, token pair 8 g
@@ -794,7 +1019,144 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fold_kernel(const __grid_con
       for (int i = 0; i < NCH; ++i)
 #pragma unroll
         for (int j = 0; j < 16; ++j) res[i][j >> 3][j & 7] = 0ull;
-      for (int s = it.s0; s < it.s1 && ok; ++s, ++sbc) {
+      if (!mbar_wait_warp(bar(MP::S_FULL + sq), pq, abort_flag, p.err, p.spin_limit, E_EPI)) break;
+      int s = it.s0;
+      if (__shfl_sync(0xFFFFFFFFu, s_item[n_item & 3], 0)) {
+        // with rows that are not plain
+        auto wait = [&](int b, int parity) -> bool { return mbar_wait_warp(bar(b), (uint32_t)parity, abort_flag, p.err, p.spin_limit, E_EPI); };
+        auto done = [&]() {  // with an accumulator
+          tc_fence_before();
+          __syncwarp();
+          mbar_arrive_if(bar(MP::D_EMPTY + d), lane == 0);
+          if (++d == ND) { d = 0; pd ^= 1; }
+        };
+        for (; s < it.s1 && ok; ++s, ++sbc) {
+          ok = false;  // (until the superblock is through)
+          if (!wait(MP::S_FULL + sq, pq)) break;
+          const uint32_t more = __shfl_sync(0xFFFFFFFFu, s_kinds[sq], 0);
+          const unsigned char* scl = smem + MP::OFF_SCL + (sbc & 3) * MP::SCL;
+          const float* sv = reinterpret_cast<const float*>(smem + MP::OFF_S + sq * 512) + cl;
+          if (!wait(MP::D_FULL + d, pd)) break;
+          tc_fence_after();
+          unsigned long long d2[4], nd2[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            d2[k] = pack2(reinterpret_cast<const float*>(scl)[row0 + 8 * k]);
+            nd2[k] = pack2(reinterpret_cast<const float*>(scl)[128 + row0 + 8 * k]);
+          }
+          if (more & kSpread) {  // the third term; what comes of rows without one may be anything (their image is what was there) and is not taken
+#pragma unroll
+            for (int i = 0; i < NCH; ++i) {
+              const int col = column(i);
+              if (col >= it.n) break;
+              unsigned long long v[8], x[8];
+              const uint32_t at = t_lane + (uint32_t)(col + TM_D + d * BT);
+              tc_ld_frag2(at, at + (16u << 16), v, x);
+#pragma unroll
+              for (int g = 0; g < 4; ++g) {
+                const unsigned long long ss = *reinterpret_cast<const unsigned long long*>(sv + col + 8 * g);
+                const unsigned long long t2 = ss ^ 0x8000000080000000ull;
+                const float s0 = lo_f(ss), s1 = hi_f(ss);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                  const unsigned long long y = (k >> 1 ? x : v)[2 * g + (k & 1)];
+                  ffma2(res[i][k >> 1][2 * g + (k & 1)], t2, fmul2(d2[k], pair(s0 < 0.0f ? lo_f(y) : 0.0f, s1 < 0.0f ? hi_f(y) : 0.0f)));
+                }
+              }
+            }
+            done();
+            if (!wait(MP::D_FULL + d, pd)) break;
+            tc_fence_after();
+          }
+#pragma unroll
+          for (int i = 0; i < NCH; ++i) {  // the first two terms, as for plain rows (s of wide ones is 0)
+            const int col = column(i);
+            if (col >= it.n) break;
+            unsigned long long ss[4];
+#pragma unroll
+            for (int g = 0; g < 4; ++g) ss[g] = *reinterpret_cast<const unsigned long long*>(sv + col + 8 * g) & 0x7FFFFFFF7FFFFFFFull;
+#pragma unroll
+            for (int hr = 0; hr < 2; ++hr) {
+              unsigned long long v[8], x[8];
+              const uint32_t at = t_lane + ((uint32_t)(16 * hr) << 16) + (uint32_t)col;
+              tc_ld_frag2(at + (uint32_t)(TM_D + d * BT), at + (uint32_t)TM_D2, v, x);
+#pragma unroll
+              for (int j = 0; j < 8; ++j) {
+                unsigned long long a = fmul2(d2[2 * hr + (j & 1)], v[j]);
+                ffma2(a, nd2[2 * hr + (j & 1)], x[j]);
+                ffma2(res[i][hr][j], ss[j >> 1], a);
+              }
+            }
+          }
+          done();
+          mbar_arrive_if(bar(MP::D2_EMPTY), lane == 0);
+          if (more & kWide) {
+            // Wide rows, block by block: the sums are whole numbers, the scales come from memory, the min term is taken on the CUDA cores.  A lane holds the
+            // factors of one row per group, and every lane takes those of its tokens from there.
+            if (!wait(MP::W2_FULL + (sbc & 1), sbc >> 1 & 1)) break;
+            const unsigned char* mnp = smem + MP::OFF_W2 + (sbc & 1) * 4096 + row0 * 32;
+            const unsigned char* kp = p.tail + ((size_t)it.tile * nsb + s) * kTailRow * p.tt + kTailCopy * p.tt;
+            bool mine[NCH], any[NCH];
+            float tr[NCH], ar[NCH];
+#pragma unroll
+            for (int i = 0; i < NCH; ++i) {
+              const int row = column(i) + lane;
+              mine[i] = row < it.n && __ldcg(kp + row) == kWide;
+              any[i] = __any_sync(0xFFFFFFFFu, mine[i]);
+            }
+            auto fetch = [&](int b) {
+#pragma unroll
+              for (int i = 0; i < NCH; ++i) {
+                const int row = column(i) + lane;
+                tr[i] = ar[i] = 0.0f;
+                if (mine[i]) {
+                  tr[i] = __ldcg(p.asc + (size_t)(8 * s + b) * p.lda + it.r0 + row);
+                  const unsigned char* vr = smem + MP::OFF_MIN + sq * 4096 + row * 32 + 2 * b;
+                  const int sw = (row >> 2 & 1) << 4;
+                  ar[i] = __fadd_rn(__half2float(*reinterpret_cast<const __half*>(vr + sw)), __half2float(*reinterpret_cast<const __half*>(vr + (sw ^ 16))));
+                }
+              }
+            };
+            fetch(0);
+            int b = 0;
+#pragma unroll 1
+            for (; b < 8; ++b) {
+              const float t_now[NCH] = {tr[0], tr[1]}, a_now[NCH] = {ar[0], ar[1]};
+              if (b < 7) fetch(b + 1);
+              if (!wait(MP::D_FULL + d, pd)) break;
+              tc_fence_after();
+              unsigned long long mn[4];
+#pragma unroll
+              for (int k = 0; k < 4; ++k) mn[k] = fmul2(nd2[k], pack2(__half2float(*reinterpret_cast<const __half*>(mnp + 256 * k + 2 * b))));
+#pragma unroll
+              for (int i = 0; i < NCH; ++i) {
+                if (!any[i]) continue;
+                unsigned long long v[8], x[8];
+                const uint32_t at = t_lane + (uint32_t)(column(i) + TM_D + d * BT);
+                tc_ld_frag2(at, at + (16u << 16), v, x);
+#pragma unroll
+                for (int g = 0; g < 4; ++g) {
+                  const int row = 8 * g + cl;
+                  const unsigned long long t2 = pair(__shfl_sync(0xFFFFFFFFu, t_now[i], row), __shfl_sync(0xFFFFFFFFu, t_now[i], row + 1));
+                  const unsigned long long a2 = pair(__shfl_sync(0xFFFFFFFFu, a_now[i], row), __shfl_sync(0xFFFFFFFFu, a_now[i], row + 1));
+#pragma unroll
+                  for (int k = 0; k < 4; ++k) {
+                    unsigned long long y = fmul2(d2[k], (k >> 1 ? x : v)[2 * g + (k & 1)]);
+                    ffma2(y, mn[k], a2);
+                    ffma2(res[i][k >> 1][2 * g + (k & 1)], t2, y);
+                  }
+                }
+              }
+              done();
+            }
+            if (b < 8) break;
+          }
+          mbar_arrive(bar(MP::S_EMPTY + sq));
+          if (++sq == NM) { sq = 0; pq ^= 1; }
+          ok = true;
+        }
+      }
+      for (; s < it.s1 && ok; ++s, ++sbc) {
         if (!mbar_wait_warp(bar(MP::S_FULL + sq), pq, abort_flag, p.err, p.spin_limit, E_EPI)) { ok = false; break; }
         const unsigned char* scl = smem + MP::OFF_SCL + (sbc & 3) * MP::SCL;
         const float* sv = reinterpret_cast<const float*>(smem + MP::OFF_S + sq * 512) + cl;
@@ -906,13 +1268,14 @@ int izb_fold_tile_rows(int device, int M, int N) {
 }
 
 size_t izb_fold_img_bytes(int rows, int K) { return (size_t)rows * (K / 256) * kImgRow; }
+size_t izb_fold_fine_bytes(int rows, int K) { return (size_t)rows * (K / 256) * kFineRow; }
 size_t izb_fold_tail_bytes(int rows, int K) { return ((size_t)rows * (K / 256) * kTailRow + 255) & ~(size_t)255; }
 
 int izb_fold_prepare(const izb_weight* w, const int8_t* aq, const float* asc, int lda, int rows, const FoldParams& p, cudaStream_t st) {
   const int n_rows = p.n_mtiles * p.tt;
   dim3 grid((n_rows + 31) / 32, w->K / 256);
   auto kernel = w->type == IZB_Q4_K ? fold_prepare_kernel<true> : fold_prepare_kernel<false>;
-  IZB_LAUNCH("act_prepare", st, izb_launch_pdl(kernel, grid, 256, 0, st, aq, asc, lda, w->K, rows, p.img, p.tail, p.tt, n_rows, p.part_bad));
+  IZB_LAUNCH("act_prepare", st, izb_launch_pdl(kernel, grid, 256, 0, st, aq, asc, lda, w->K, rows, p.img, p.fine, p.tail, p.tt, n_rows, p.part_bad));
   return IZB_OK;
 }
 
@@ -923,7 +1286,7 @@ int izb_fold_quant_prepare(const izb_weight* w, const float* x, int ldx, int M, 
   dim3 grid(w->K / 256, one ? (all + 7) / 8 : (all + 31) / 32);
   auto kernel = w->type == IZB_Q4_K ? (one ? fold_quant_prepare_kernel<true, 1> : fold_quant_prepare_kernel<true, 4>)
                                     : one ? fold_quant_prepare_kernel<false, 1> : fold_quant_prepare_kernel<false, 4>;
-  IZB_LAUNCH("quant_prepare", st, izb_launch_pdl(kernel, grid, 256, 0, st, x, ldx, M, Mp, w->K, aq, asc, p.img, p.tail, p.tt, p.n_mtiles, p.part_bad));
+  IZB_LAUNCH("quant_prepare", st, izb_launch_pdl(kernel, grid, 256, 0, st, x, ldx, M, Mp, w->K, aq, asc, p.img, p.fine, p.tail, p.tt, p.n_mtiles, p.part_bad));
   return IZB_OK;
 }
 

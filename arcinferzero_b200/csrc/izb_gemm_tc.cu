@@ -1195,7 +1195,7 @@ int run_tc(const izb_weight* w, int mat, const int8_t* aq, const float* asc, int
 
 // A plain store with the scales folded into the operands (csrc/izb_gemm_fold.cu), of long K as with tc_split, and for the same reasons: short K
 // gains little (a tile is mostly fill and drain), and keeps the sums of the other store modes; x: the quantiser's input (aq and asc are written), or
-// null where aq and asc are there.  +1: not taken, or its arena (1.6 times the other kernel's) cannot be had in a capture or without memory:
+// null where aq and asc are there.  +1: not taken, or its arena (2.3 times the other kernel's) cannot be had in a capture or without memory:
 // the caller goes on with the other kernel.
 int run_fold(const izb_weight* w, int mat, const float* x, int ldx, int T, int8_t* aq, float* asc, int Mp, int M_store, float* C, int ldc, int c_off, cudaStream_t st) {
   if (!tc_takes(w) || !izb_fold_takes(w) || w->K < 2048) return 1;
@@ -1204,15 +1204,18 @@ int run_fold(const izb_weight* w, int mat, const float* x, int ldx, int T, int8_
   p.n_mtiles = (M_store + p.tt - 1) / p.tt;
   const int rows = p.n_mtiles * p.tt;
   if ((rows + 31) / 32 > 65535) return 1;
-  const size_t img_bytes = izb_fold_img_bytes(rows, w->K), tail_bytes = izb_fold_tail_bytes(rows, w->K);
+  const size_t img_bytes = izb_fold_img_bytes(rows, w->K), fine_bytes = izb_fold_fine_bytes(rows, w->K), tail_bytes = izb_fold_tail_bytes(rows, w->K);
   void* ws = nullptr;
-  if (int rc = izb_workspace(w->device, kWsGemm, img_bytes + tail_bytes + split_area(w->device), st, &ws, true)) return rc;
+  if (int rc = izb_workspace(w->device, kWsGemm, img_bytes + fine_bytes + tail_bytes + split_area(w->device), st, &ws, true)) return rc;
   uint32_t* err = izb_device_error_word(w->device);
   if (!err) IZB_FAIL(IZB_ERR_NOMEM, "gemm: no device error word");
   p.img = (unsigned char*)ws;
-  p.tail = p.img + img_bytes;
+  p.fine = p.img + img_bytes;
+  p.tail = p.fine + fine_bytes;
   p.part = (float*)(p.tail + tail_bytes);
   p.part_bad = split_flag(p.part, w->device);
+  p.asc = asc;
+  p.lda = Mp;
   p.M = M_store;
   p.N = w->N;
   p.K = w->K;
@@ -1239,7 +1242,7 @@ int run_fold(const izb_weight* w, int mat, const float* x, int ldx, int T, int8_
 size_t izb_gemm_tc_scratch_bytes(int device, int type, int rows, int K) {
   size_t img_bytes, asc_bytes;
   tc_scratch_bytes((rows + BM - 1) / BM, K, type == IZB_Q4_K ? 5 : 4, &img_bytes, &asc_bytes);
-  const size_t fold = izb_fold_img_bytes(rows + BM, K) + izb_fold_tail_bytes(rows + BM, K);  // (tiles round the rows up by less than one)
+  const size_t fold = izb_fold_img_bytes(rows + BM, K) + izb_fold_fine_bytes(rows + BM, K) + izb_fold_tail_bytes(rows + BM, K);  // (tiles round the rows up by less than one)
   return std::max(img_bytes + asc_bytes, fold) + split_area(device);
 }
 

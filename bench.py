@@ -667,7 +667,7 @@ def main() -> None:
             "dtype": "int8",
             "data": "synthetic",
             "config": {"workload": WORKLOAD,
-                       "arithmetic": ("int8 x 4-bit dot products per 32-block with the block scales in the operands (activations as two fp16 terms, 22 to 24 bits; "
+                       "arithmetic": ("int8 x 4-bit dot products per 32-block with the block scales in the operands (activations as two fp16 terms, 23 to 24 bits; "
                                       "weight sub-scale x quant exact in fp16; f32 TMEM accumulators per 256 of K), f32 combine"),
                        "parallelism": f"weight rows split over {world} rank(s), no exchange",
                        "l2": "per step 168 MB of f32 activations in and 570 MB of outputs written: larger than the 126 MB L2",

@@ -117,6 +117,91 @@ def test_fold_scales_that_are_no_numbers(izb):
     W.close()
 
 
+# Up to 4 : 1 two terms, up to 4096 : 1 three, beyond that block by block; 40 token rows, and tiles whose rows differ in kind
+RATIOS = [1.0, 3.0, 5.0, 40.0, 2.0 ** 10, 2.0 ** 11.8, 2.0 ** 12.4, 2.0 ** 14, 2.0 ** 28, 2.0 ** 40]
+
+
+@pytest.mark.parametrize("qt", [12, 13])
+@pytest.mark.parametrize("K", [2048, 5120])
+@pytest.mark.parametrize("zero", [False, True])
+def test_fold_small_blocks_beside_a_large_one(izb, qt, K, zero):
+    """One block of every superblock is many times the others; with `zero` its weights are zeros, and the small blocks' products are all there is.
+    Bound: as in test_fold_against_64_bits, of the norm of every row."""
+    import torch
+    M, N = 40, 256
+    w = S.make_weight(qt, N, K, K).copy()
+    if zero:
+        v = w.reshape(N, K // 256, -1)
+        v[:, :, 4] &= 0xC0  # sub-scale and min of block 0
+        v[:, :, 8] &= 0xC0
+    W = izb.Weight(qt, w, N, K)
+    w64 = weights64(qt, w, K)
+    for ratio in RATIOS + [None]:
+        x = S.make_act(M, K, K)
+        f = np.float32(ratio) if ratio else np.array([RATIOS[m % len(RATIOS)] for m in range(M)], np.float32)[:, None, None]
+        x.reshape(M, K // 256, 8, 32)[:, :, 0] *= f
+        aq, asc, _ = izb.quantize_act(torch.from_numpy(x).cuda())
+        got = izb.gemm(W, aq, asc, M=M).cpu().numpy()[:M]
+        assert izb.device_status(0) == 0
+        a = aq[:M].cpu().numpy().astype(np.float64).reshape(M, K // 32, 32) * asc[:, :M].cpu().numpy().T[:, :, None].astype(np.float64)
+        ref = a.reshape(M, K) @ w64.T
+        err = np.linalg.norm(got - ref, axis=1) / np.linalg.norm(ref, axis=1)
+        assert err.max() < 4e-7, (ratio, err.max())
+    W.close()
+
+
+@pytest.mark.parametrize("qt,M,N,K", [(12, 130, 256, 2048), (13, 100, 144, 2304), (12, 40, 20000, 2048), (13, 40, 20000, 2048)])
+def test_rows_do_not_depend_on_the_kinds_of_others(izb, qt, M, N, K):
+    """Rows with two terms, with three and with blocks one by one, alone and beside each other in a superblock."""
+    import torch
+    W = izb.Weight(qt, np.tile(S.make_weight(qt, 16, K, 1), (N // 16, 1)), N, K)
+
+    def run_with(kinds):
+        x = S.make_act(M, K, 2)
+        for sb in range(K // 256):
+            for m in range(M):
+                x[m, 256 * sb + 32 * (m % 8):256 * sb + 32 * (m % 8) + 32] *= np.float32(kinds(m, sb))
+        aq, asc, _ = izb.quantize_act(torch.from_numpy(x).cuda())
+        out = izb.gemm(W, aq, asc, M=M)[:M]
+        assert izb.device_status(0) == 0
+        return out
+    plain, spread, wide = (run_with(lambda m, sb, f=f: f) for f in (1.0, 100.0, 2.0 ** 20))
+    for a, b in ((1.0, 100.0), (1.0, 2.0 ** 20), (100.0, 2.0 ** 20)):
+        of = {1.0: plain, 100.0: spread, 2.0 ** 20: wide}
+        mixed = run_with(lambda m, sb: a if m % 3 else b)
+        for m in range(M):
+            assert torch.equal(mixed[m], of[a if m % 3 else b][m]), (a, b, m)
+    W.close()
+
+
+@pytest.mark.parametrize("qt,M,N,K", [(12, 40, 256, 2048), (13, 40, 256, 2048), (12, 40, 20000, 2048), (13, 40, 20000, 2048)])
+@pytest.mark.parametrize("ratio", [1.0, 100.0, 2.0 ** 20])
+def test_fold_waits_that_run_out(izb, qt, M, N, K, ratio):
+    """Every element is the right one or was left alone, with K cut and not; the next call is whole again."""
+    import torch
+    W = izb.Weight(qt, np.tile(S.make_weight(qt, 16, K, 1), (N // 16, 1)), N, K)
+    x = S.make_act(M, K, 2)
+    x.reshape(M, K // 256, 8, 32)[M // 2:, :, 3] *= np.float32(ratio)
+    Mp = izb.pad_rows(M)
+    aq, asc, _ = izb.quantize_act(torch.from_numpy(x).cuda(), Mp=Mp)
+    want = izb.gemm(W, aq, asc, M=M)[:M]
+    assert izb.device_status(0) == 0
+    gave_up = 0
+    for limit, skip in ((1, -1), (2, -1), (3, -1), (5, -1), (8, -1), (2000, 0), (2000, 5), (2000, 30)):  # (skip: a unit of the activations that is left out)
+        izb.debug_wait_test(limit, skip)
+        out = torch.full((Mp, N), float("nan"), device="cuda")
+        izb.gemm(W, aq, asc, M=M, out=out)
+        status = izb.device_status(0)
+        kept = torch.isnan(out[:M])
+        assert torch.equal(out[:M][~kept], want[~kept]), (limit, skip)
+        assert status != 0 or not bool(kept.any())
+        assert skip < 0 or status != 0
+        gave_up += status != 0
+    assert gave_up >= 3
+    assert torch.equal(izb.gemm(W, aq, asc, M=M)[:M], want) and izb.device_status(0) == 0
+    W.close()
+
+
 def test_fold_in_a_capture_without_its_arena(izb):
     """Where the folded kernel's arena would have to grow inside a capture, the call goes to the other kernel."""
     import os
