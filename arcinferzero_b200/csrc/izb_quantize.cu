@@ -92,10 +92,12 @@ __global__ void __launch_bounds__(256) quantize_act_kernel(const float* __restri
   }
 }
 
-// One value per thread, a warp per 32-block: the block's scale and sums from the warp.
+// One value per thread, a warp per 32-block: the block's scale and sums from the warp.  kNan: a block that is all NaN has the scale NaN, as the residual
+// addition's rows have it, else 0, as the quantisers' and the other norm's have it.
+template <bool kNan>
 __device__ __forceinline__ void quantize_value(float v, int row, int col, int Mp, int K, int8_t* __restrict__ aq, float* __restrict__ asc, int16_t* __restrict__ absum) {
   const int lane = threadIdx.x & 31;
-  float amax = fmaxf(0.0f, fabsf(v));
+  float amax = kNan ? fabsf(v) : fmaxf(0.0f, fabsf(v));
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
   const float inv = amax > 0.0f ? __fdiv_rn(127.0f, amax) : 0.0f;
@@ -134,7 +136,7 @@ __global__ void __launch_bounds__(256) quantize_few_kernel(const float* __restri
     v = __fmul_rn(__fdiv_rn(v, __fadd_rn(1.0f, expf(-v))), u);
     if (hout) hout[(size_t)row * F + col] = v;
   }
-  quantize_value(v, row, col, Mp, K, aq, asc, absum);
+  quantize_value<false>(v, row, col, Mp, K, aq, asc, absum);
 }
 
 // Sum over the CTA's 256 threads in the defined order: xor butterfly 16, 8, 4, 2, 1 inside every warp, then the eight
@@ -336,7 +338,7 @@ __global__ void __launch_bounds__(256) add_norm_few_kernel(float* __restrict__ x
     if (k < steps && first + k < nk) {
       const int i = threadIdx.x + 256 * (first + k);
       xr[i] = xo[k];
-      quantize_value(w2 ? __fmul_rn(__fmul_rn(xo[k], r2), w2o[k]) : xo[k], m, i, Mp, K, aq, asc, absum);
+      quantize_value<true>(w2 ? __fmul_rn(__fmul_rn(xo[k], r2), w2o[k]) : xo[k], m, i, Mp, K, aq, asc, absum);
     }
 }
 
@@ -475,10 +477,10 @@ __global__ void __launch_bounds__(256) rmsnorm_few_kernel(const float* __restric
   const float r = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, (float)K), eps)));
   const float v0 = __fmul_rn(__fmul_rn(x0, r), w0), v1 = __fmul_rn(__fmul_rn(x1, r), w1);
   if (hout) hout[(size_t)m * K + i0] = v0;
-  quantize_value(v0, m, i0, Mp, K, aq, asc, absum);
+  quantize_value<false>(v0, m, i0, Mp, K, aq, asc, absum);
   if (two) {
     if (hout) hout[(size_t)m * K + i1] = v1;
-    quantize_value(v1, m, i1, Mp, K, aq, asc, absum);
+    quantize_value<false>(v1, m, i1, Mp, K, aq, asc, absum);
   }
 }
 

@@ -57,6 +57,26 @@ def test_norms_of_few_rows(izb, M, K):
     assert (bits(h.cpu().numpy()) == bits(ry)).all() and (aq.cpu().numpy() == raq).all() and (bits(asc.cpu().numpy()) == bits(rasc)).all()
 
 
+# ... and the same bits as in many rows where values are no finite numbers: a row with one NaN is NaN throughout behind the norm.
+@pytest.mark.parametrize("K", [1280, 2048, 4096, 5120])
+def test_add_norm_quant_of_no_numbers(izb, K):
+    import torch
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(K)
+    x, t = (torch.randn((600, K), generator=gen, device="cuda") for _ in range(2))
+    w, w2 = (torch.randn(K, generator=gen, device="cuda") for _ in range(2))
+    t[1, 5], t[2, 40], x[3, 700], x[4, 64:96], t[5, 0] = float("nan"), float("inf"), float("nan"), float("nan"), float("-inf")
+    t[6], x[6] = 0.0, 0.0
+    x[7, 32:64] = float("inf")
+    same = lambda a, b: torch.equal(a.contiguous().view(torch.uint8), b.contiguous().view(torch.uint8))
+    for second in (w2, None):
+        xm, xf = x.clone(), x[:8].clone()
+        aqm, ascm = izb.add_norm_quant(xm, t, w, 1e-6, 0.75, second)
+        aqf, ascf = izb.add_norm_quant(xf, t[:8].contiguous(), w, 1e-6, 0.75, second)
+        assert same(xm[:8], xf) and same(aqm[:8], aqf[:8]) and same(ascm[:, :8], ascf[:, :8])
+        assert bool(torch.isnan(ascf[:, 1]).all())
+
+
 # The residual addition's outputs may lie anywhere (padding rows are zeroed 16 bytes at a time where they are aligned).
 @pytest.mark.parametrize("M,K,off", [(1, 1024, 1), (3, 2048, 4), (3, 2048, 0), (5, 5376, 8)])
 def test_add_norm_quant_unaligned_output(izb, M, K, off):
