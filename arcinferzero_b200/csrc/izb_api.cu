@@ -128,6 +128,7 @@ struct DevState {
   void* ws[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};  // scratch arenas by user (izb_common.cuh: kWs*)
   size_t ws_bytes[5] = {0, 0, 0, 0, 0};
   bool ws_in_graph[5] = {false, false, false, false, false};  // a capture has seen the block: it stays
+  int ws_no_try[5] = {0, 0, 0, 0, 0};                           // kWsOrBlock: calls that do not try to grow, since one was without memory
   void* stage = nullptr;  // staging of the host-buffer call
   size_t stage_bytes = 0;
   cudaStream_t hs[3] = {nullptr, nullptr, nullptr};  // host-buffer call: copy-in, compute, copy-out streams
@@ -232,31 +233,49 @@ void izb_note_noalloc_status(int device, uint32_t* status) {
 
 // An arena never shrinks and is only replaced when a call needs more than it holds.  Replacing waits for the device
 // (work in flight may still read the old block) -- izb_reserve moves that wait out of the hot path.
-static int grow_arena(DevState& d, int device, int slot, size_t bytes) {
+// `keep`: the new block first, and without memory for it the old one stays; else the old one makes room.
+static int grow_arena(DevState& d, int device, int slot, size_t bytes, bool keep = false) {
   if (bytes <= d.ws_bytes[slot]) return IZB_OK;
   size_t sizes[2] = {bytes, bytes};  // tried in turn
+  void* old = d.ws[slot];
   if (d.ws_in_graph[slot]) {  // (the old block is left to the graphs)
     if (bytes < 2 * d.ws_bytes[slot]) sizes[0] = 2 * d.ws_bytes[slot];
-    d.ws_in_graph[slot] = false;
-  } else if (d.ws[slot]) {
-    IZB_CUDA(cudaDeviceSynchronize());
-    IZB_CUDA(cudaFree(d.ws[slot]));
+    old = nullptr;
   }
-  d.ws[slot] = nullptr;
-  d.ws_bytes[slot] = 0;
+  auto give_back = [&]() -> int {
+    if (old) {
+      IZB_CUDA(cudaDeviceSynchronize());
+      IZB_CUDA(cudaFree(old));
+    }
+    old = nullptr;
+    d.ws[slot] = nullptr;
+    d.ws_bytes[slot] = 0;
+    d.ws_in_graph[slot] = false;
+    return IZB_OK;
+  };
+  if (!keep)
+    if (int rc = give_back()) return rc;
   for (size_t size : sizes) {
     const size_t want = (size + (size_t(1) << 20) - 1) & ~((size_t(1) << 20) - 1);
-    if (cudaMalloc(&d.ws[slot], want) == cudaSuccess) {
+    void* block = nullptr;
+    if (cudaMalloc(&block, want) == cudaSuccess) {
+      if (keep) {
+        if (int rc = give_back()) {
+          cudaFree(block);
+          return rc;
+        }
+      }
+      d.ws[slot] = block;
       d.ws_bytes[slot] = want;
+      d.ws_no_try[slot] = 0;
       return IZB_OK;
     }
     cudaGetLastError();
-    d.ws[slot] = nullptr;
   }
   IZB_FAIL(IZB_ERR_NOMEM, "workspace of %zu bytes on device %d", bytes, device);
 }
 
-int izb_workspace(int device, int slot, size_t bytes, cudaStream_t st, void** out, bool other_way) {
+int izb_workspace(int device, int slot, size_t bytes, cudaStream_t st, void** out, IzbNeed need) {
   DevState& d = g_dev[device];
   std::lock_guard<std::mutex> lk(d.mu);
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
@@ -264,8 +283,15 @@ int izb_workspace(int device, int slot, size_t bytes, cudaStream_t st, void** ou
     cudaGetLastError();
     capture = cudaStreamCaptureStatusInvalidated;
   }
-  if (other_way && bytes > d.ws_bytes[slot] && capture != cudaStreamCaptureStatusNone) return 1;
-  if (int rc = grow_arena(d, device, slot, bytes)) return other_way ? 1 : rc;
+  if (need != kWsMust && bytes > d.ws_bytes[slot] && capture != cudaStreamCaptureStatusNone) return 1;
+  if (need == kWsOrBlock && bytes > d.ws_bytes[slot] && d.ws_no_try[slot] > 0) {
+    --d.ws_no_try[slot];
+    return 1;
+  }
+  if (int rc = grow_arena(d, device, slot, bytes, need == kWsOrBlock)) {
+    if (need == kWsOrBlock) d.ws_no_try[slot] = 255;  // (a failing cudaMalloc takes longer than most calls)
+    return need == kWsMust ? rc : 1;
+  }
   if (capture == cudaStreamCaptureStatusActive) d.ws_in_graph[slot] = true;
   *out = d.ws[slot];
   return IZB_OK;
@@ -281,6 +307,7 @@ extern "C" int izb_reserve(int device, int max_rows, int max_K) {
   DevState& d = g_dev[device];
   std::lock_guard<std::mutex> lk(d.mu);
   const size_t gemm = izb_gemm_tc_scratch_bytes(device, IZB_Q4_K, max_rows, max_K);
+  for (int& n : d.ws_no_try) n = 0;
   if (int rc = grow_arena(d, device, kWsGemm, gemm)) return rc;
   if (int rc = grow_arena(d, device, kWsMoe, gemm)) return rc;
   if (int rc = grow_arena(d, device, kWsTp, (size_t)(max_K / 32) * max_rows * 4)) return rc;

@@ -130,10 +130,12 @@ uint32_t* izb_device_error_word(int device);
 // Per-device scratch arenas, one per user so that independent users never share bytes; each is grown on demand
 // (cudaMalloc only when a call needs more than any call before it).  Calls that use the same arena must be ordered on
 // one stream.  A block that a captured graph holds is never given back (the graph may be replayed at any time): the arena then at least
-// doubles where memory allows, so that all such blocks together hold no more than it.  `other_way`: the caller has another kernel; +1 instead
-// of an error where the arena would have to grow and cannot -- in a stream capture, or without memory.
+// doubles where memory allows, so that all such blocks together hold no more than it.  `need`: a caller with another kernel gets +1 instead
+// of an error where the arena would have to grow and cannot -- in a stream capture, or without memory.  Where that kernel works in the arena as it
+// is (kWsOrBlock), the block there is only given up for a larger one, and after an attempt without memory the next calls do not try.
+enum IzbNeed { kWsMust, kWsOrElse, kWsOrBlock };
 enum { kWsGemm = 0, kWsTp = 1, kWsMoe = 2, kWsCheck = 3, kWsNorm = 4 };
-int izb_workspace(int device, int slot, size_t bytes, cudaStream_t st, void** out, bool other_way = false);
+int izb_workspace(int device, int slot, size_t bytes, cudaStream_t st, void** out, IzbNeed need = kWsMust);
 
 // ---------------------------------------------------------------------------------------------- programmatic dependent launch
 // A decode step is a chain of kernels of a few microseconds, each waiting for the one before.  Launched with this attribute

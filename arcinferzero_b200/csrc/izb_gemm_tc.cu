@@ -1185,7 +1185,7 @@ int run_tc(const izb_weight* w, int mat, const int8_t* aq, const float* asc, int
   tc_scratch_bytes(n_tiles_grid, w->K, tc_sps(w, dots != nullptr), &img_bytes, &asc_bytes);
   const size_t split_bytes = tiles || dots || !may_cut ? 0 : split_area(w->device);
   void* ws = nullptr;
-  if (int rc = izb_workspace(w->device, ws_slot, img_bytes + asc_bytes + split_bytes, st, &ws, !tiles && !dots && tc_optional(w))) return rc;
+  if (int rc = izb_workspace(w->device, ws_slot, img_bytes + asc_bytes + split_bytes, st, &ws, !tiles && !dots && tc_optional(w) ? kWsOrElse : kWsMust)) return rc;
   uint32_t* err = izb_device_error_word(w->device);
   if (!err) IZB_FAIL(IZB_ERR_NOMEM, "gemm: no device error word");
   float* split_ws = split_bytes ? (float*)((unsigned char*)ws + img_bytes + asc_bytes) : nullptr;
@@ -1206,7 +1206,7 @@ int run_fold(const izb_weight* w, int mat, const float* x, int ldx, int T, int8_
   if ((rows + 31) / 32 > 65535) return 1;
   const size_t img_bytes = izb_fold_img_bytes(rows, w->K), fine_bytes = izb_fold_fine_bytes(rows, w->K), tail_bytes = izb_fold_tail_bytes(rows, w->K);
   void* ws = nullptr;
-  if (int rc = izb_workspace(w->device, kWsGemm, img_bytes + fine_bytes + tail_bytes + split_area(w->device), st, &ws, true)) return rc;
+  if (int rc = izb_workspace(w->device, kWsGemm, img_bytes + fine_bytes + tail_bytes + split_area(w->device), st, &ws, kWsOrBlock)) return rc;
   uint32_t* err = izb_device_error_word(w->device);
   if (!err) IZB_FAIL(IZB_ERR_NOMEM, "gemm: no device error word");
   p.img = (unsigned char*)ws;
@@ -1300,7 +1300,7 @@ int izb_gemm_tc_quant_launch(const izb_weight* w, int mat, const float* x, int l
   size_t img_bytes, asc_bytes;
   tc_scratch_bytes(n_tiles, K, sps, &img_bytes, &asc_bytes);
   void* ws = nullptr;
-  if (int rc = izb_workspace(w->device, kWsGemm, img_bytes + asc_bytes + split_area(w->device), st, &ws, tc_optional(w))) return rc;
+  if (int rc = izb_workspace(w->device, kWsGemm, img_bytes + asc_bytes + split_area(w->device), st, &ws, tc_optional(w) ? kWsOrElse : kWsMust)) return rc;
   uint32_t* err = izb_device_error_word(w->device);
   if (!err) IZB_FAIL(IZB_ERR_NOMEM, "gemm: no device error word");
   uint16_t* aimg = (uint16_t*)ws;

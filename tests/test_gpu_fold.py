@@ -229,6 +229,58 @@ print("done")
     assert r.returncode == 0 and "done" in r.stdout, r.stdout + r.stderr
 
 
+def test_fold_without_memory_for_its_arena(izb):
+    """On a full GPU a call whose folded arena cannot be had keeps the arena that is there, here one that a graph holds, and goes to the other kernel, as often as
+    it is made; with memory again, the folded kernel has its own."""
+    import os
+    import subprocess
+    import sys
+    body = """
+import torch, arcinferzero_b200 as izb
+from arcinferzero_b200 import synth as S
+N, K, M = 1024, 17408, 4096  # (arenas: 190 and 450 MB; K is not cut)
+W = izb.Weight(12, S.make_weight(12, N, K, 1), N, K)
+aq, asc, _ = izb.quantize_act(torch.from_numpy(S.make_act(M, K, 2)).cuda())
+out = torch.zeros(M, N, device="cuda")
+izb.gemm(W, aq, asc, out=out, acc=1)
+want = izb.gemm(W, aq, asc, impl=izb.GEMM_TC)
+q = (torch.empty((M, K), dtype=torch.int8, device="cuda"), torch.empty((K // 32, M), dtype=torch.float32, device="cuda"))
+x = torch.zeros(M, K, device="cuda")
+izb.quant_matmul(W, x[:64], 64)
+again = torch.zeros(M, N, device="cuda")
+torch.cuda.synchronize()
+g = torch.cuda.CUDAGraph()
+with torch.cuda.graph(g):
+    izb.gemm(W, aq, asc, out=again, acc=1)
+g.replay()
+assert torch.equal(again, want)
+assert torch.equal(out, want) and out.any()  # (what torch allocates for these is there then)
+torch.cuda.synchronize()
+full = torch.empty(torch.cuda.mem_get_info()[0] - (96 << 20), dtype=torch.uint8, device="cuda")
+free = torch.cuda.mem_get_info()[0]
+for i in range(5):
+    out.zero_()
+    izb.gemm(W, aq, asc, out=out)
+    torch.cuda.synchronize()
+    assert torch.equal(out, want), float((out - want).abs().max())
+    assert torch.cuda.mem_get_info()[0] == free, (i, torch.cuda.mem_get_info()[0] - free)
+izb.quant_matmul(W, x, M, out=out, qout=q)
+torch.cuda.synchronize()
+assert not out.any() and torch.cuda.mem_get_info()[0] == free and izb.device_status(0) == 0
+del full
+torch.cuda.empty_cache()
+for i in range(300):
+    izb.gemm(W, aq, asc, out=out)
+assert not torch.equal(out, want) and float((out - want).abs().max()) <= 1e-5 * float(want.abs().max())
+again.zero_()
+g.replay()
+assert torch.equal(again, want) and izb.device_status(0) == 0
+print("done")
+"""
+    r = subprocess.run([sys.executable, "-c", body], cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))), capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "done" in r.stdout, r.stdout + r.stderr
+
+
 # The quantiser that prepares the operands as it goes takes one row per warp up to one wave of such blocks (148 x 8), else four: the same bytes and products
 # as the quantiser and the pre-pass one after the other.
 @pytest.mark.parametrize("qt,N,K", [(12, 256, 2048), (13, 272, 2304), (8, 256, 2048), (14, 256, 2304)])
