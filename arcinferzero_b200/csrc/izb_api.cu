@@ -297,7 +297,7 @@ int izb_workspace(int device, int slot, size_t bytes, cudaStream_t st, void** ou
   return IZB_OK;
 }
 
-size_t izb_gemm_tc_scratch_bytes(int device, int type, int rows, int K);
+size_t izb_gemm_tc_scratch_bytes(int device, int type, int rows, int K, bool folded);
 
 extern "C" int izb_reserve(int device, int max_rows, int max_K) {
   if (max_rows < 1 || max_K < 256 || max_K % 256) IZB_FAIL(IZB_ERR_SHAPE, "reserve: rows = %d, K = %d (K in whole superblocks)", max_rows, max_K);
@@ -306,11 +306,13 @@ extern "C" int izb_reserve(int device, int max_rows, int max_K) {
   IZB_CUDA(scope.enter(device));
   DevState& d = g_dev[device];
   std::lock_guard<std::mutex> lk(d.mu);
-  const size_t gemm = izb_gemm_tc_scratch_bytes(device, IZB_Q4_K, max_rows, max_K);
+  const size_t gemm = izb_gemm_tc_scratch_bytes(device, IZB_Q4_K, max_rows, max_K, false), folded = izb_gemm_tc_scratch_bytes(device, IZB_Q4_K, max_rows, max_K, true);
   for (int& n : d.ws_no_try) n = 0;
-  if (int rc = grow_arena(d, device, kWsGemm, gemm)) return rc;
-  if (int rc = grow_arena(d, device, kWsMoe, gemm)) return rc;
+  if (int rc = grow_arena(d, device, kWsMoe, gemm)) return rc;  // (expert calls never run the folded kernel)
   if (int rc = grow_arena(d, device, kWsTp, (size_t)(max_K / 32) * max_rows * 4)) return rc;
+  // (dense calls have another one where its arena, 2.3 times that one's, cannot be had)
+  if (grow_arena(d, device, kWsGemm, folded, d.ws_bytes[kWsGemm] >= gemm))
+    if (int rc = grow_arena(d, device, kWsGemm, gemm)) return rc;
   if (!d.err_word.load(std::memory_order_relaxed)) {
     uint32_t* p = nullptr;
     if (cudaMalloc(&p, 256) != cudaSuccess) { cudaGetLastError(); IZB_FAIL(IZB_ERR_NOMEM, "reserve: error word on device %d", device); }

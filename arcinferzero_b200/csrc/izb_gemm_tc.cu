@@ -1238,10 +1238,12 @@ int run_fold(const izb_weight* w, int mat, const float* x, int ldx, int T, int8_
 
 }  // namespace
 
-// scratch bytes of a dense tensor-core GEMM over `rows` activation rows (izb_reserve sizes the arenas with it)
-size_t izb_gemm_tc_scratch_bytes(int device, int type, int rows, int K) {
+// scratch bytes of a tensor-core GEMM over `rows` activation rows (izb_reserve sizes the arenas with it); folded: of dense calls, which may run the
+// folded kernel
+size_t izb_gemm_tc_scratch_bytes(int device, int type, int rows, int K, bool folded) {
   size_t img_bytes, asc_bytes;
   tc_scratch_bytes((rows + BM - 1) / BM, K, type == IZB_Q4_K ? 5 : 4, &img_bytes, &asc_bytes);
+  if (!folded) return img_bytes + asc_bytes + split_area(device);
   const size_t fold = izb_fold_img_bytes(rows + BM, K) + izb_fold_fine_bytes(rows + BM, K) + izb_fold_tail_bytes(rows + BM, K);  // (tiles round the rows up by less than one)
   return std::max(img_bytes + asc_bytes, fold) + split_area(device);
 }

@@ -191,6 +191,51 @@ def test_reserve_then_calls_do_not_allocate(izb, torch):
     W.close()
 
 
+def test_reserve_sizes_each_arena_for_its_kernels(izb):
+    """What izb_reserve takes: the folded kernel's arena once (1024 + 512 + 37 bytes per row and superblock), the other kernel's (5 stages of 16 KB per 128 rows and
+    superblock) for the experts.  Dense calls up to the reserved size then allocate nothing; on a full GPU the reserve gets by with the other kernel's size."""
+    import os
+    import subprocess
+    import sys
+    body = """
+import torch, arcinferzero_b200 as izb
+from arcinferzero_b200 import synth as S
+rows, K, N = 8192, 8192, 256
+torch.zeros(1, device="cuda")
+W = izb.Weight(12, S.make_weight(12, N, K, 5), N, K)
+def buffers(M):
+    Mp = izb.pad_rows(M)
+    return M, torch.ones((M, K), device="cuda"), torch.empty((Mp, N), device="cuda"), (torch.empty((Mp, K), dtype=torch.int8, device="cuda"), torch.empty((K // 32, Mp), device="cuda"))
+def call(M, x, out, q):
+    izb.quant_matmul(W, x, M, out=out, qout=q)
+    izb.gemm(W, *q, M=M, out=out)
+def free():
+    torch.cuda.synchronize()
+    return torch.cuda.mem_get_info()[0]
+for M in (9, 100): call(*buffers(M))  # (the kernels are loaded)
+pad = torch.empty(torch.cuda.mem_get_info()[0] - (500 << 20), dtype=torch.uint8, device="cuda")
+f0 = free()
+izb.reserve(0, rows, K)  # (both arenas: 2 x 180 MB; the folded kernel's, 420 MB, does not fit beside the experts')
+few = f0 - free()
+other = rows // 128 * (K // 256) * 5 * 16384 + rows * K // 32 * 4 + 148 * 65536
+assert 2 * other - (16 << 20) <= few <= 2 * other + (16 << 20) + rows * K // 32 * 4, (few, other)
+del pad
+torch.cuda.empty_cache()
+f0 = free()
+izb.reserve(0, rows, K)
+more, folded = f0 - free(), (rows + 128) * (K // 256) * 1573 + 148 * 65536
+assert 0 < more + other <= folded + (4 << 20), (more, other, folded)
+todo = [buffers(M) for M in (16, 33, 700, 1000, 2047, 5000, 8192)]
+f0 = free()
+for t in todo: call(*t)
+assert free() == f0
+assert izb.device_status(0) == 0
+print("done")
+"""
+    r = subprocess.run([sys.executable, "-c", body], cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))), capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "done" in r.stdout, r.stdout + r.stderr
+
+
 def test_two_devices_from_two_threads_of_one_process(izb, torch):
     """The reference drives its GPUs from one process, one thread per GPU (zero/mgpu/engine_tp.h:825).  Two threads, each
     bound to its own device, run the whole dispatch (GEMV, few-row GEMV, tensor-core GEMM, MoE tiles) at once; both must
