@@ -1243,9 +1243,9 @@ int launch(const izb_weight* w, const FoldParams& p, int grid, cudaStream_t st) 
   CUtensorMap tm;
   memcpy(&tm, w->tmap_raw, sizeof tm);
   if (p.pdl)
-    IZB_LAUNCH("gemm_tc", st, izb_launch_pdl(gemm_fold_kernel<F>, dim3(grid), dim3(kThreads), SMEM_BYTES, st, tm, p));
+    IZB_LAUNCH("gemm_fold", st, izb_launch_pdl(gemm_fold_kernel<F>, dim3(grid), dim3(kThreads), SMEM_BYTES, st, tm, p));
   else
-    IZB_LAUNCH("gemm_tc", st, gemm_fold_kernel<F><<<grid, kThreads, SMEM_BYTES, st>>>(tm, p));
+    IZB_LAUNCH("gemm_fold", st, gemm_fold_kernel<F><<<grid, kThreads, SMEM_BYTES, st>>>(tm, p));
   return IZB_OK;
 }
 

@@ -653,7 +653,7 @@ def main() -> None:
 
     if rank == 0:
         hbm, tc_burst, tc_sus, src = peaks()
-        kname = next((k for k in ("gemm_tc", "gemm_core") if k in prof), "gemm_tc")
+        kname = next((k for k in ("gemm_fold", "gemm_tc", "gemm_core") if k in prof), "gemm_tc")
         g = prof.get(kname) or {"launches": 0, "ms": 0.0}
         per_tile = NCU_TRAFFIC_BYTES_PER_TILE
         ms_kernel = g["ms"] / max(1, g["launches"])

@@ -32,8 +32,10 @@ def exact(qt, rows, K, aq, asc):
 def run(izb, W, aq, asc, M, N, Mp):
     import torch
     out = torch.full((Mp, N + 8), float("nan"), device="cuda")
+    izb.profile_start()
     izb.gemm(W, aq, asc, M=M, out=out, c_off=4)
-    assert izb.device_status(0) == 0
+    ran = izb.profile_stop()
+    assert izb.device_status(0) == 0 and "gemm_fold" in ran and "gemm_tc" not in ran, ran
     got = out.cpu().numpy()
     assert np.isnan(got[:, :4]).all() and np.isnan(got[:, N + 4:]).all() and np.isnan(got[M:]).all()
     return got[:M, 4:N + 4]

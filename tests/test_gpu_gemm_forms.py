@@ -55,7 +55,9 @@ def test_tensor_core_gemm_equals_core_gemm(izb, qt, M, N, K):
             a = base.clone()
             ran = kernels_of(izb, lambda: izb.gemm(W, aq, asc, M=M, out=a, c_off=4, acc=acc, impl=impl))
             short = impl == izb.GEMM_AUTO and (qt not in (12, 8, 2) or N % 128 != 0) and K <= 512 << acc  # (may go to the CUDA cores, below)
-            assert "gemm_tc" in ran or short, (acc, impl, ran)
+            folded = qt in (12, 13) and impl == izb.GEMM_AUTO and acc == 0 and K >= 2048
+            assert ("gemm_fold" if folded else "gemm_tc") in ran or short, (acc, impl, ran)
+            assert ("gemm_fold" in ran) + ("gemm_tc" in ran) <= 1, (acc, impl, ran)
             assert ("split_reduce" in ran) == (impl == izb.GEMM_AUTO and acc == 0 and K >= 2048), (acc, impl, ran)
             ra, rb = a[:M, 4:N + 4].double(), b[:M, 4:N + 4].double()
             assert float((ra - rb).abs().max() / rb.abs().max()) < 1e-5, (acc, impl)
@@ -64,6 +66,7 @@ def test_tensor_core_gemm_equals_core_gemm(izb, qt, M, N, K):
     got = []
     ran = kernels_of(izb, lambda: got.append(izb.quant_matmul(W, x, M)[0]))
     assert "quant_prepare" in ran or K <= 512, ran
+    assert ("gemm_fold" in ran) == (qt in (12, 13) and K >= 2048), ran
     assert torch.equal(got[0][:M], want[:M])
     assert izb.device_status(0) == 0
     W.close()
@@ -171,8 +174,8 @@ import torch, arcinferzero_b200 as izb
 izb.profile_start()
 izb.selfcheck(0)
 ran = izb.profile_stop()
-# five forms x (plain cut, adding, SwiGLU, plain uncut), two with block dots
-assert ran["gemm_tc"]["launches"] == 22 and ran["split_reduce"]["launches"] == 5, ran
+# five forms x (plain cut, adding, SwiGLU, plain uncut), two with block dots; two forms' plain cut in the folded kernel
+assert ran["gemm_tc"]["launches"] == 20 and ran["gemm_fold"]["launches"] == 2 and ran["split_reduce"]["launches"] == 5, ran
 assert sum(ran[k]["launches"] for k in ran if k.startswith("gemm_k16")) == 12, ran
 assert izb.device_status(0) == 0
 print("done")
