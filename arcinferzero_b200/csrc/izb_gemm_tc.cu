@@ -1197,7 +1197,7 @@ int run_tc(const izb_weight* w, int mat, const int8_t* aq, const float* asc, int
 // gains little (a tile is mostly fill and drain), and keeps the sums of the other store modes; x: the quantiser's input (aq and asc are written), or
 // null where aq and asc are there.  +1: not taken, or its arena (2.3 times the other kernel's) cannot be had in a capture or without memory:
 // the caller goes on with the other kernel.
-int run_fold(const izb_weight* w, int mat, const float* x, int ldx, int T, int8_t* aq, float* asc, int Mp, int M_store, float* C, int ldc, int c_off, cudaStream_t st) {
+int run_fold(const izb_weight* w, int mat, const float* x, int ldx, int T, int8_t* aq, float* asc, int Mp, int M_store, float* C, int ldc, int c_off, cudaStream_t st, bool may_cut = true) {
   if (!tc_takes(w) || !izb_fold_takes(w) || w->K < 2048) return 1;
   FoldParams p;
   p.tt = izb_fold_tile_rows(w->device, M_store, w->N);
@@ -1228,7 +1228,7 @@ int run_fold(const izb_weight* w, int mat, const float* x, int ldx, int T, int8_
   p.spin_limit = spin ? spin : kSpinLimit;
   p.skip_stage = g_test_skip.exchange(-1);
   const int n_items = (w->N + BN - 1) / BN * p.n_mtiles;
-  p.n_split = tc_split(w->device, n_items, w->K / 256);
+  p.n_split = may_cut ? tc_split(w->device, n_items, w->K / 256) : 1;
   if (int rc = x ? izb_fold_quant_prepare(w, x, ldx, T, Mp, aq, asc, p, st) : izb_fold_prepare(w, aq, asc, Mp, Mp, p, st)) return rc;
   const int grid = tc_grid(w->device, n_items * p.n_split);
   p.pdl = tc_pdl(false, grid, n_items * p.n_split);
@@ -1344,7 +1344,8 @@ int izb_moe_down_tc(const izb_weight* wd, const int8_t* d_hq, const float* d_hsc
 }
 
 // ---------------------------------------------------------------------------------------------- start-up check
-// Seeded data, every weight form, all store modes, a part of a column tile, and the plain store with K cut into parts and not:
+// Seeded data, every weight form, all store modes, a part of a column tile, and the plain store with K cut into parts and not, in this kernel and, of the
+// forms it takes, in the folded one (whose rows are of all its kinds):
 // tensor-core dots == CUDA-core dots bit for bit (Q4_K, Q8_0: the forms that have this mode), outputs within 1e-5 of max|ref|
 // (Engine::xmx_check, zero/engine_setup.h:424-622, does the same for its XMX kernel against DP4a).
 int izb_gemm_k16_launch(const izb_weight* w, const uint8_t* raw, const int8_t* aq, const float* asc, int M, int Mp, float* C, int ldc,
@@ -1357,12 +1358,13 @@ __global__ void fill_quants(int8_t* p, size_t n, uint32_t seed) {
   x ^= x >> 15; x *= 2246822519u; x ^= x >> 13; x *= 3266489917u; x ^= x >> 16;
   p[i] = (int8_t)((int)(x % 255u) - 127);
 }
-__global__ void fill_scales(float* p, size_t n, uint32_t seed) {
+// (few_small: one of 64 is 2^-15 of that)
+__global__ void fill_scales(float* p, size_t n, uint32_t seed, bool few_small) {
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   uint32_t x = (uint32_t)i * 2654435761u + seed;
   x ^= x >> 15; x *= 2246822519u; x ^= x >> 13;
-  p[i] = 0.005f + (float)(x & 0xFFFF) * (0.03f / 65535.0f);
+  p[i] = (0.005f + (float)(x & 0xFFFF) * (0.03f / 65535.0f)) * (few_small && (x >> 26) == 0 ? 0x1p-15f : 1.0f);
 }
 // out[0] = count of differing ints, out[1] = max|a-b| bits, out[2] = max|b| bits
 __global__ void compare_kernel(const float* a, const float* b, size_t n, int as_int, unsigned int* out) {
@@ -1431,7 +1433,7 @@ int check_form(int device, int type) {
   unsigned int out[3];
   auto blocks = [](size_t n) { return (unsigned)((n + 255) / 256); };
   fill_quants<<<blocks((size_t)Mp * K), 256>>>(aq, (size_t)Mp * K, 99u);
-  fill_scales<<<blocks((size_t)nb * Mp), 256>>>(asc, (size_t)nb * Mp, 7u);
+  fill_scales<<<blocks((size_t)nb * Mp), 256>>>(asc, (size_t)nb * Mp, 7u, true);
   IZB_CUDA(cudaGetLastError());
   if (!k16) {
     int rc = izb_gemm_tc_launch(w, 0, aq, nullptr, M, M, nullptr, 0, 0, 0, d_tc, 0, false);
@@ -1442,11 +1444,20 @@ int check_form(int device, int type) {
     IZB_CUDA(cudaMemcpy(out, cmp, 12, cudaMemcpyDeviceToHost));
     if (out[0]) IZB_FAIL(IZB_ERR_SELFCHECK, "selfcheck: type %d: %u block dots differ between the tensor-core and CUDA-core kernels", type, out[0]);
   }
-  for (int mode = 0; mode < 4; ++mode) {  // 3: the plain store again, K not cut
-    const int acc = mode % 3;
-    fill_scales<<<blocks(n_out), 256>>>(c_tc, n_out, 3u);
-    fill_scales<<<blocks(n_out), 256>>>(c_core, n_out, 3u);
-    int rc = izb_gemm_tc_launch(w, 0, aq, asc, M, Mp, c_tc, N, 0, acc, nullptr, 0, mode < 3);
+  constexpr struct {
+    const char* what;
+    int acc;
+    bool folded, cut;
+  } modes[] = {{"plain store, K cut", 0, false, true}, {"adding store", 1, false, false}, {"SwiGLU store", 2, false, false}, {"plain store", 0, false, false},
+               {"plain store, folded, K cut", 0, true, true}, {"plain store, folded", 0, true, false}};
+  for (const auto& mode : modes) {
+    if (mode.folded && !izb_fold_takes(w)) continue;
+    const int acc = mode.acc;
+    fill_scales<<<blocks(n_out), 256>>>(c_tc, n_out, 3u, false);
+    fill_scales<<<blocks(n_out), 256>>>(c_core, n_out, 3u, false);
+    int rc = mode.folded ? run_fold(w, 0, nullptr, 0, 0, aq, asc, Mp, M, c_tc, N, 0, 0, mode.cut)
+                         : run_tc(w, 0, aq, asc, Mp, Mp, nullptr, (M + BM - 1) / BM, nullptr, nullptr, M, c_tc, N, 0, acc, nullptr, kWsGemm, 0, false, mode.cut);
+    if (mode.folded && rc > 0) continue;  // (without memory for its arena: its calls go to this kernel)
     if (rc == 0) rc = core(aq, asc, Mp, c_core, acc, nullptr);
     if (rc != 0) return rc < 0 ? rc : IZB_ERR_SELFCHECK;
     IZB_CUDA(cudaMemset(cmp, 0, 12));
@@ -1456,7 +1467,7 @@ int check_form(int device, int type) {
     memcpy(&err, &out[1], 4);
     memcpy(&ref, &out[2], 4);
     if (out[0] || !(err <= 1e-5f * ref))
-      IZB_FAIL(IZB_ERR_SELFCHECK, "selfcheck: type %d store mode %d%s: max|err| %g vs max|ref| %g (%u NaN)", type, acc, mode == 0 ? ", K cut" : "", err, ref, out[0]);
+      IZB_FAIL(IZB_ERR_SELFCHECK, "selfcheck: type %d, %s: max|err| %g vs max|ref| %g (%u NaN)", type, mode.what, err, ref, out[0]);
   }
   return IZB_OK;
 }

@@ -225,9 +225,9 @@ int izb_gemm(const izb_weight* w, int mat, const int8_t* d_aq, const float* d_as
  * kernel's accumulators before any scaling (impl = IZB_GEMM_TC).  Both must equal the CPU values bit for bit. */
 int izb_block_dots(const izb_weight* w, int mat, const int8_t* d_aq, int M, int32_t* d_dots, int impl, void* stream);
 /* Start-up check in the manner of Engine::xmx_check: runs the tensor-core kernel and the CUDA-core kernels on seeded
- * data for every weight form and store mode, with a part of a column tile and with K cut into parts, and compares (dots of Q4_K and
- * Q8_0 bit for bit, outputs within 1e-5 of max|ref|).  Synchronous.  IZB_ERR_SELFCHECK on disagreement; izb_matmul then keeps to the
- * CUDA-core kernels on that device. */
+ * data for every weight form and store mode, with a part of a column tile, with K cut into parts and not, plain stores of Q4_K and Q5_K in both
+ * of their kernels, and compares (dots of Q4_K and Q8_0 bit for bit, outputs within 1e-5 of max|ref|).  Synchronous.  IZB_ERR_SELFCHECK on
+ * disagreement; izb_matmul then keeps to the CUDA-core kernels on that device. */
 int izb_selfcheck(int device);
 
 /* izb_gemm for callers that cannot allocate device memory while they run.  It has no counterpart in the reference.

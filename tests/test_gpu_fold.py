@@ -204,19 +204,21 @@ def test_fold_waits_that_run_out(izb, qt, M, N, K, ratio):
     W.close()
 
 
-def test_fold_in_a_capture_without_its_arena(izb):
-    """Where the folded kernel's arena would have to grow inside a capture, the call goes to the other kernel."""
+# (256 tiles, and four, whose K is cut)
+@pytest.mark.parametrize("qt,N,K,M,cut", [(12, 1024, 2048, 4096, False), (12, 128, 4096, 512, True), (13, 128, 4096, 512, True)])
+def test_fold_in_a_capture_without_its_arena(izb, qt, N, K, M, cut):
+    """Where the folded kernel's arena would have to grow inside a capture, the call goes to the other kernel, which may cut K as well."""
     import os
     import subprocess
     import sys
-    body = """
+    body = f"""qt, N, K, M, cut = {qt}, {N}, {K}, {M}, {cut}
 import torch, arcinferzero_b200 as izb
 from arcinferzero_b200 import synth as S
-N, K, M = 1024, 2048, 4096
-W = izb.Weight(12, S.make_weight(12, N, K, 1), N, K)
+W = izb.Weight(qt, S.make_weight(qt, N, K, 1), N, K)
 aq, asc, _ = izb.quantize_act(torch.from_numpy(S.make_act(M, K, 2)).cuda())
 izb.gemm(W, aq, asc, out=torch.zeros(M, N, device="cuda"), acc=1)  # the arena of the other kernel
-want = izb.gemm(W, aq, asc, impl=izb.GEMM_TC)
+want = izb.gemm(W, aq, asc, out=torch.zeros(M, N, device="cuda"), acc=1)
+core = izb.gemm(W, aq, asc, impl=izb.GEMM_CORE)
 out = torch.zeros(M, N, device="cuda")
 torch.cuda.synchronize()
 g = torch.cuda.CUDAGraph()
@@ -224,7 +226,10 @@ with torch.cuda.graph(g):
     izb.gemm(W, aq, asc, out=out)
 g.replay()
 torch.cuda.synchronize()
-assert torch.equal(out, want) and izb.device_status(0) == 0
+assert torch.equal(out, want) != cut and float((out - core).abs().max()) <= 1e-5 * float(core.abs().max())
+got = out.clone()
+izb.gemm(W, aq, asc, out=out)  # (the folded kernel)
+assert not torch.equal(out, got) and izb.device_status(0) == 0
 print("done")
 """
     r = subprocess.run([sys.executable, "-c", body], cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))), capture_output=True, text=True, timeout=300)

@@ -174,9 +174,9 @@ import torch, arcinferzero_b200 as izb
 izb.profile_start()
 izb.selfcheck(0)
 ran = izb.profile_stop()
-# five forms x (plain cut, adding, SwiGLU, plain uncut), two with block dots; two forms' plain cut in the folded kernel
-assert ran["gemm_tc"]["launches"] == 20 and ran["gemm_fold"]["launches"] == 2 and ran["split_reduce"]["launches"] == 5, ran
-assert sum(ran[k]["launches"] for k in ran if k.startswith("gemm_k16")) == 12, ran
+# five forms x (plain cut, adding, SwiGLU, plain uncut), two with block dots; two forms in the folded kernel, cut and uncut
+assert ran["gemm_tc"]["launches"] == 22 and ran["gemm_fold"]["launches"] == 4 and ran["split_reduce"]["launches"] == 7, ran
+assert sum(ran[k]["launches"] for k in ran if k.startswith("gemm_k16")) == 14, ran
 assert izb.device_status(0) == 0
 print("done")
 """
