@@ -76,14 +76,17 @@ int launch(const izb_weight* w, const uint8_t* raw, const int8_t* aq, const floa
 //         over a long K: 256 x 8192 T=1 5.8/4.9, T=4 6.9/6.4, 256 x 4096 T=1 3.6/3.2, T=2 3.7/3.8, 384 x 8192 T=1 5.8/7.0; 128 x 8192 T=5 11/11, 48 x
 //         4096 T=5 7.3/7.9
 //   Q4_K  rows that are too long for the dot product's ring: 1024 x 10496 T=1 8.0/13, 4096 x 9472 T=1 8.6/8.2 (fits), T=2 9.4/14, 512 x 12544 T=4 10/14;
-//         T = 1 pays in a middle range: 12288 x 2304 7.0/8.3, 12288 x 3328 8.6/11, 16384 x 3840 12/12, 16384 x 8448 23/20, 4096 x 2816 4.4/3.8;
-//         T = 2: 8192 x 3328 6.7/8.1, 4096 x 5376 6.1/6.6, 4096 x 2816 4.5/4.4; T = 3: 4096 x 2816 4.9/5.0, 3072 x 2816 4.7/4.5; T = 4: 2560 x 2816
-//         4.9/5.1, 2048 x 2304 3.9/3.5; T >= 5: 1024 x 2048 T=8 4.1/4.2, 34816 x 5120 T=5 34/52, T=8 35/76
+//         T = 1 pays in a middle range: 12288 x 2304 7.6/8.3, 12288 x 3840 9.3/10.7, 24576 x 3840 15.3/16.4, 24576 x 5376 21.1/20.2, 8192 x 2816 7.7/6.1;
+//         T = 2: 5120 x 1280 3.6/4.0, 5120 x 5376 7.3/8.3, 4096 x 1280 3.5/3.2, 4096 x 2816 4.5/4.4, 4096 x 5376 7.0/6.8, 4096 x 6912 7.1/7.7, 3072 x 8448 8.5/8.2;
+//         T = 3: 4096 x 2304 4.4/4.8, 3072 x 2816 4.7/4.5; T = 4: 2560 x 2304 4.4/5.1, 2048 x 2304 3.9/3.5; T >= 5: 1024 x 2048 T=8 4.1/4.2, 34816 x 5120 T=5
+//         34/52, T=8 35/76
 //         (at up to four rows the kernels for K % 1024 == 0 add in another order: theirs stays)
-//   Q8_0  rows that are too long for the ring: 512 x 8192 T=1 7.5/13, T=8 13/21, 1024 x 6144 T=4 7.0/13, 2048 x 5120 T=4 6.7/11; else many row tiles: T = 1 12288 x
-//         2048 5.7/8.0, 151936 x 1024 27/38, 151936 x 2048 51/49, 5120 x 2560 4.4/4.5, 5120 x 5120 7.4/6.8, 4096 x 2048 3.7/3.3; T = 2: 6144 x 4096
-//         6.8/6.8, 8192 x 4096 7.6/8.2, 64000 x 5120 55/53, 5120 x 4096 6.5/6.1; T = 3: 4096 x 4096 6.0/6.4, 3072 x 3072 4.8/4.7; T = 4: 3072 x
-//         1024 2.8/3.0, 2048 x 1024 2.5/2.3; T >= 5 (a warp holds twice the sums): 1024 x 3072 T=8 6.4/5.0, 4096 x 4096 T=8 8.3/12
+//   Q8_0  rows that are too long for the ring: 512 x 8192 T=1 7.5/13, T=8 13/21, 1024 x 6144 T=4 7.0/13, 2048 x 5120 T=4 6.7/11; else many row tiles, and while
+//         latency, not the copy's rate, is what both take their time for: T = 1 131072 x 1536 35/39, 65536 x 2048 23.5/23.5, 131072 x 2048 45/43, 20480 x
+//         2560 10.3/10.9, 32768 x 2560 15.7/15.1, 5120 x 2560 4.4/4.5, 4096 x 2048 3.7/3.3; T = 2: 131072 x 2048 46/50, 32768 x 3072 18.9/19.5 (102 MiB of weights),
+//         65536 x 3072 35/34, 16384 x 4096 12.7/13.4 (68), 32768 x 4096 24/23 (136), 24576 x 4352 20.0/20.3 (108), 24576 x 4608 20.8/20.6 (115), 6144 x 4096
+//         6.8/6.8; T = 3: 131072 x 5120 112/115, 4096 x 5120 7.2/7.5, 3072 x 4096 5.8/5.6; T = 4: 3072 x 2048 3.6/4.0, 2048 x 1024 2.5/2.3; T >= 5 (a warp holds
+//         twice the sums): 1024 x 3072 T=8 6.4/5.0, 4096 x 4096 T=8 8.3/12
 bool rows_first(const izb_weight* w, int T) {
   const int N = w->N, K = w->K;
   if (w->type == IZB_K16) return T > 4 ? N >= 128 || K < 8192 : N > 256 || K <= (T == 1 ? 2048 : 4096);
@@ -91,10 +94,10 @@ bool rows_first(const izb_weight* w, int T) {
   if (T > 4 && w->type == IZB_Q4_K) return true;
   if (!izb_gemv_stream_fits(w, T)) return N >= 512;
   if (w->type == IZB_Q4_K)
-    return T == 1 ? N >= 12288 && K <= 3328 : T == 2 ? (size_t)N * w->row_bytes >= (size_t)12 << 20 : N >= (T == 3 ? 4096 : 2560);
+    return T == 1 ? N >= 12288 && K <= 3840 : T == 2 ? N >= (K <= 6400 ? 5120 : 4096) : N >= (T == 3 ? 4096 : 2560);
   switch (T) {
-    case 1: return N >= 5120 && (K <= 1024 || (K <= 2560 && N <= 40960));
-    case 2: return N >= 6144 && (K <= 4096 || N <= 32768);
+    case 1: return N >= 5120 && (K <= 1536 || (K <= 2048 && N <= 65536) || (K <= 2560 && N <= 24576));
+    case 2: return N >= 6144 && (K <= 2560 || (size_t)N * w->row_bytes <= (size_t)108 << 20);
     case 3: return N >= 4096;
     case 4: return N >= 3072;
     default: return N >= 4096;

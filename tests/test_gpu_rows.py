@@ -41,6 +41,8 @@ def test_rows_match_oracle(izb, qt, N, K):
 @pytest.mark.parametrize("qt,N,K", [(14, 16, 512), (14, 48, 2048), (14, 96, 8192), (14, 112, 8448), (14, 144, 8192), (14, 1184, 17408), (14, 1200, 17408), (14, 4096, 1024),
                                     (12, 16, 4096), (12, 48, 1536), (12, 96, 4096), (12, 1008, 2048), (12, 2368, 18944), (12, 2384, 18944), (12, 16384, 2304), (12, 8192, 5376),
                                     (12, 4096, 8960), (12, 4096, 9472), (12, 12304, 5376), (12, 16384, 3840), (12, 1024, 2048), (8, 4096, 256), (8, 4096, 8192), (8, 16384, 1024), (8, 4112, 2304), (8, 6144, 512), (8, 16, 1024),
+                                    (12, 5104, 5376), (12, 5120, 5376), (12, 4080, 6656), (12, 4096, 6656), (12, 12288, 3840), (12, 12288, 4352), (8, 24576, 2560), (8, 24592, 2560), (8, 65552, 1792),
+                                    (8, 24576, 4352), (8, 24592, 4352),
                                     (13, 64, 768), (23, 64, 768), (2, 4096, 512)])
 def test_rows_do_not_depend_on_their_number(izb, qt, N, K):
     import torch
