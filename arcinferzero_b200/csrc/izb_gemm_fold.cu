@@ -1252,7 +1252,8 @@ int launch(const izb_weight* w, const FoldParams& p, int grid, cudaStream_t st) 
 }  // namespace
 
 // The cut of M whose rounds of tiles over the SMs cost least.  A tile's time follows its rows while its MMAs set the pace, and stops following
-// them below 64 rows, where the dequantisers do; every tile has a fill and a drain.  (The rows' results do not depend on it.)
+// them below 64 rows, where the dequantisers do; every tile has a fill and a drain.  (The rows' results do not depend on it while K is not cut; the number of
+// tiles has a part in how it is.)
 int izb_fold_tile_rows(int device, int M, int N) {
   const int sms = izb_sm_count(device), n_ntiles = (N + BN - 1) / BN;
   int best = BT;

@@ -58,7 +58,7 @@ __global__ void __launch_bounds__(kStreamWarps * 32, 1) gemv_stream_kernel(const
   constexpr int SBS = QT == IZB_Q4_K ? 4 : 2;  // superblocks per step
   constexpr int SBB = QT == IZB_Q4_K ? 144 : 272;
   constexpr int STEP = QT == IZB_Q4_K ? kQ4StepBytes : kQ8StepBytes;
-    const int nsb = K >> 8, nsteps = (nsb + SBS - 1) / SBS;
+  const int nsb = K >> 8, nsteps = (nsb + SBS - 1) / SBS;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int W = gridDim.x * kStreamWarps, w0 = blockIdx.x * kStreamWarps + warp;
   const uint32_t row_bytes = (uint32_t)nsb * SBB;

@@ -574,7 +574,8 @@ extern "C" int izb_add_norm_quant(float* d_x, const float* d_t, const float* d_w
   int dev = 0;
   IZB_CUDA(cudaGetDevice(&dev));
   // A cluster per row while there are up to three CTAs per SM (us, a CTA per row / a cluster: 2048, one row 4.0/2.6, 100 rows 5.3/4.3; 4096, one 6.6/3.0,
-  // 32 6.9/4.2, 64 7.4/7.3, 100 7.6/9.6; 5120, one 8.2/3.5, 100 9.4/11; 1024, one 2.7/2.5, 100 3.0/3.1)
+  // 32 6.9/4.2, 64 7.4/7.3, 100 7.6/9.6; 5120, one 8.2/3.5, 100 9.4/11; 1024, one 2.7/2.5, 100 3.0/3.1).  It ends at 5120 because every CTA holds the whole of three
+  // rows in registers, 60 per thread there; it is not written for longer rows, of which a CTA takes 18 us for eight of 8192
   const int cl = nk <= 16 ? (nk + 1) / 2 : 7, steps = (nk + cl - 1) / cl;
   if (nk > 4 && nk <= 20 && (long long)cl * Mp <= 3 * izb_sm_count(dev)) {
     auto kernel = nk <= 8 ? add_norm_few_kernel<8> : nk <= 16 ? add_norm_few_kernel<16> : add_norm_few_kernel<20>;

@@ -29,6 +29,15 @@ def test_gemm_roles_wait_as_warps():
     assert re.search(r"bool mbar_wait_warp\([^{]*\{.*?__all_sync\(kAll, mbar_test.*?__all_sync\(kAll, mbar_try_wait", s, re.S)
 
 
+def test_folded_gemm_waits_as_warps():
+    """Every role of the folded GEMM issues something warp-wide: there is no wait but the voting ones."""
+    s = source("izb_gemm_fold.cu")
+    kernel = s[s.index("gemm_fold_kernel(const __grid_constant__"):s.index("int launch(const izb_weight")]
+    assert len(re.findall(r"\bmbar_wait_warp\(", kernel)) >= 12 and not re.findall(r"\bmbar_(wait|test|try_wait)\(", kernel)
+    assert re.search(r"bool mbar_wait_warp\([^{]*\{.*?__all_sync\(kAll, mbar_test.*?__all_sync\(kAll, mbar_try_wait", s, re.S)
+    assert not re.findall(r"\bmbar_(test|try_wait)\(", re.sub(r"__all_sync\(kAll, mbar_(test|try_wait)\(", "", s[s.index("bool mbar_wait_warp("):]).replace("ok &= mbar_test(w[i]", ""))
+
+
 @pytest.mark.parametrize("name", ["izb_rows.cu", "izb_gemv_stream.cu"])
 def test_gemv_rings_wait_as_warps(name):
     """A look at a ring slot's barrier is only ever used through a vote."""
@@ -40,7 +49,7 @@ def test_gemv_rings_wait_as_warps(name):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("qt,M,N,K", [(12, 300, 272, 1024), (8, 300, 272, 1024), (13, 130, 128, 512), (14, 130, 128, 512), (23, 130, 128, 512), (12, 40, 128, 4096)])
+@pytest.mark.parametrize("qt,M,N,K", [(12, 300, 272, 1024), (8, 300, 272, 1024), (13, 130, 128, 512), (14, 130, 128, 512), (23, 130, 128, 512), (12, 40, 128, 4096), (8, 40, 128, 4096), (14, 40, 128, 4096)])
 def test_waits_that_run_out_at_any_moment(izb, qt, M, N, K):
     """Every element is the right one or was left alone; the next call is whole again."""
     import torch
