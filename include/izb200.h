@@ -24,7 +24,8 @@
  *     device must be ordered (same stream, or events between streams); calls on different devices are independent.
  *     An arena grows when a call needs more than any call before it, which waits for the device and calls
  *     cudaFree / cudaMalloc: call izb_reserve once at start-up to keep that out of the hot path (and out of stream
- *     capture).
+ *     capture).  A plain store of Q4_K or Q5_K whose arena would have to grow in a capture, or cannot for lack of memory, runs on the
+ *     other tensor-core kernel, whose arena is smaller: the graph then has other last bits and takes longer than the same call outside.
  *
  * Buffer layouts are the reference engine's (zero/engine_alloc.h:10,39,41):
  *   aq     int8  [Mp][K]      quantised activations, row-major
