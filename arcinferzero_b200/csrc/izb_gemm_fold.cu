@@ -652,8 +652,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fold_kernel(const __grid_con
   };
   auto item_kinds = [&](const Item& it) -> uint32_t {
     uint32_t k = 0;
-#pragma unroll 8
-    for (int s = it.s0; s < it.s1; ++s) k |= load_kinds((size_t)it.tile * nsb + s, it.n);
+    for (int s = it.s0; s < it.s1; s += 8) {  // (eight at a time, so that their loads overlap: one by one they took 0.7 us of a call's 18)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) k |= load_kinds((size_t)it.tile * nsb + min(s + i, it.s1 - 1), it.n);
+    }
     return all_kinds(k);
   };
 
