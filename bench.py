@@ -36,7 +36,7 @@ QT = 12
 SEED = 20261125
 WORKLOAD = "config2: Q4_K prefill GEMM M=8192 N=17408 K=5120 (quantiser + GEMM per step: one izb_quant_matmul call)"
 NOMINAL_INT8_TOPS = 4500.0
-NCU_TRAFFIC_BYTES_PER_TILE = (159.7e6 + 121.0e6) / (16 * 136)       # gemm_tc (the folded kernel): ncu capture of 16 x 136 tiles of 128 x 128
+NCU_TRAFFIC_BYTES_PER_TILE = (159.7e6 + 121.0e6) / (16 * 136)       # gemm_fold: ncu capture of 16 x 136 tiles of 128 x 128
 
 
 def peaks():
