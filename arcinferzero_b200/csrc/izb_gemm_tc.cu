@@ -1229,7 +1229,8 @@ int run_fold(const izb_weight* w, int mat, const float* x, int ldx, int T, int8_
   p.skip_stage = g_test_skip.exchange(-1);
   const int n_items = (w->N + BN - 1) / BN * p.n_mtiles;
   p.n_split = may_cut ? tc_split(w->device, n_items, w->K / 256) : 1;
-  if (int rc = x ? izb_fold_quant_prepare(w, x, ldx, T, Mp, aq, asc, p, st) : izb_fold_prepare(w, aq, asc, Mp, Mp, p, st)) return rc;
+  // (rows that are not stored count as zeros: what is in them must not send a tile through the longer loops)
+  if (int rc = x ? izb_fold_quant_prepare(w, x, ldx, T, Mp, aq, asc, p, st) : izb_fold_prepare(w, aq, asc, Mp, M_store, p, st)) return rc;
   const int grid = tc_grid(w->device, n_items * p.n_split);
   p.pdl = tc_pdl(false, grid, n_items * p.n_split);
   if (int rc = izb_fold_gemm(w, p, grid, st)) return rc;

@@ -176,6 +176,20 @@ def test_rows_do_not_depend_on_the_kinds_of_others(izb, qt, M, N, K):
     W.close()
 
 
+@pytest.mark.parametrize("M", [9, 40, 130])
+def test_fold_rows_that_are_not_stored(izb, M):
+    """What the padding rows hold (here no numbers, and scales far apart) reaches no result and is not written to."""
+    import torch
+    N, K = 256, 2048
+    W = izb.Weight(12, S.make_weight(12, N, K, 3), N, K)
+    Mp = izb.pad_rows(M) + 16
+    aq, asc, _ = izb.quantize_act(torch.from_numpy(S.make_act(M, K, 4)).cuda(), Mp=Mp)
+    want = run(izb, W, aq, asc, M, N, Mp)
+    aq[M:], asc[:, M:], asc[::3, M:], asc[::8, M + 1:] = 77, 1e30, 1e-20, float("nan")
+    assert (run(izb, W, aq, asc, M, N, Mp) == want).all()
+    W.close()
+
+
 @pytest.mark.parametrize("qt,M,N,K", [(12, 40, 256, 2048), (13, 40, 256, 2048), (12, 40, 20000, 2048), (13, 40, 20000, 2048)])
 @pytest.mark.parametrize("ratio", [1.0, 100.0, 2.0 ** 20])
 def test_fold_waits_that_run_out(izb, qt, M, N, K, ratio):
