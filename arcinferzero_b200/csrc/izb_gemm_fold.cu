@@ -650,13 +650,19 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_fold_kernel(const __grid_con
     k |= k >> 16;
     return (k | k >> 8) & 3u;
   };
-  auto item_kinds = [&](const Item& it) -> uint32_t {
-    uint32_t k = 0;
-    for (int s = it.s0; s < it.s1; s += 8) {  // (eight at a time, so that their loads overlap: one by one they took 0.7 us of a call's 18)
+  auto item_kinds = [&](const Item& it) -> uint32_t {  // a lane 16 rows: four superblocks a load, kAhead loads in flight
+    constexpr int kAhead = 8;
+    const unsigned char* k = p.tail + (size_t)it.tile * nsb * kTailRow * p.tt + kTailCopy * p.tt + 16 * (lane & 7);
+    uint32_t any = 0;
+    for (int s = it.s0 + (lane >> 3); 16 * (lane & 7) < it.n && s < it.s1; s += 4 * kAhead) {
+      uint4 v[kAhead];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) k |= load_kinds((size_t)it.tile * nsb + min(s + i, it.s1 - 1), it.n);
+      for (int i = 0; i < kAhead; ++i) v[i] = *reinterpret_cast<const uint4*>(k + (size_t)min(s + 4 * i, it.s1 - 1) * kTailRow * p.tt);
+#pragma unroll
+      for (int i = 0; i < kAhead; ++i) any |= v[i].x | v[i].y | v[i].z | v[i].w;
     }
-    return all_kinds(k);
+    __syncwarp();
+    return all_kinds(any);
   };
 
   if (warp >= 16) {
